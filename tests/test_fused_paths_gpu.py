@@ -1,0 +1,88 @@
+"""Kernels that fold several passes into one, at the sizes where their dispatch or their tiling changes, against plain
+PyTorch in fp32 or fp64 (tolerances: the rounding of the result's type, times the length of a sum where there is one)."""
+import math
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda", 0)
+EPS = {torch.float32: 2 ** -23, torch.bfloat16: 2 ** -8}
+
+
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+def _cl(*shape, dtype=torch.bfloat16):
+    n, c, h, w = shape
+    return torch.randn(n, h, w, c, device=DEV).to(dtype).permute(0, 3, 1, 2)
+
+
+# ---- losses -------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,c", [(3, 7), (5, 8), (4, 776), (3, 1001), (2, 4104), (2, 16400)])
+def test_kd_ce_rows_vectorised_and_not(n, c, dtype):
+    """Row lengths on both sides of every block size, 8 elements per access or one; a masked row, rows without a label,
+    classes switched off by the type's lowest value, and by -inf under cross-entropy alone."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(0)
+    s = (torch.randn(n, c, device=DEV) * 3).to(dtype)
+    t = (torch.randn(n, c, device=DEV) * 3).to(dtype)
+    s[0, : c // 2] = torch.finfo(dtype).min
+    t[0, : c // 2] = torch.finfo(dtype).min
+    y = torch.randint(c // 2 + 1, c, (n,), device=DEV)
+    y[1] = -100
+    on = torch.ones(n, dtype=torch.bool, device=DEV)
+    on[-1] = n < 3
+    s = s.requires_grad_()
+    loss = fused.kd_ce_loss(s, t, y, 2.0, 0.5, 0.25, row_mask=on)
+    (g,) = torch.autograd.grad(loss * 3.0, s)
+    r = s.detach().double().requires_grad_()
+    ls, lt = F.log_softmax(r / 2, 1), F.log_softmax(t.double() / 2, 1)
+    term = torch.where(lt.exp() > 0, lt.exp() * (lt - ls), torch.zeros_like(ls))
+    ref = 0.25 * 4 * term[on].sum() + 0.5 * F.cross_entropy(r[on], y[on], ignore_index=-100, reduction="sum")
+    (gr,) = torch.autograd.grad(ref * 3.0, r)
+    assert abs(float(loss.detach()) - float(ref.detach())) <= 1e-5 * abs(float(ref.detach()))
+    assert _rel(g, gr) < max(2 * EPS[dtype], 1e-5)
+    assert not g[~on].any()
+    s = s.detach().clone()
+    s[0, : c // 2] = -math.inf
+    s.requires_grad_()
+    (g,) = torch.autograd.grad(fused.kd_ce_loss(s, None, y, 1.0, 1.0, 0.0), s)
+    r = s.detach().double().requires_grad_()
+    (gr,) = torch.autograd.grad(F.cross_entropy(r, y, ignore_index=-100, reduction="sum"), r)
+    assert _rel(g, gr) < max(2 * EPS[dtype], 1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,d", [(1, 8), (7, 256), (130, 100)])
+def test_byol_pair_equals_two_single_losses(n, d, dtype):
+    from tspipe_b200.ops import fused
+    torch.manual_seed(1)
+    o1, o2, t1, t2 = (torch.randn(n, d, device=DEV).to(dtype) for _ in range(4))
+    o1, o2 = o1.requires_grad_(), o2.requires_grad_()
+    gs = torch.autograd.grad(fused.byol_loss(o1, o2, t1, t2), [o1, o2])
+    ref = fused.byol_pair_loss(o1, t2, 1.0 / n) + fused.byol_pair_loss(o2, t1, 1.0 / n)
+    for a, b in zip(gs, torch.autograd.grad(ref, [o1, o2])):
+        assert torch.equal(a, b)
+    # a recorded or batched product goes through plain ops
+    (g,) = torch.autograd.grad(fused.byol_loss(o1, o2, t1, t2), o1, torch.ones((), device=DEV, requires_grad=True),
+                               create_graph=True)
+    assert g.requires_grad and torch.equal(g.detach(), gs[0])
+
+
+def test_loss_gradient_scaling_in_place_and_not():
+    """A retained graph gives the same gradient again, with any factor; a freed one takes the buffer over."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(15)
+    s = torch.randn(9, 1000, device=DEV).bfloat16().requires_grad_()
+    y = torch.randint(0, 1000, (9,), device=DEV)
+    loss = fused.cross_entropy(s, y)
+    one = torch.autograd.grad(loss, s, retain_graph=True)[0].clone()
+    (half,) = torch.autograd.grad(loss, s, torch.tensor(0.5, device=DEV), retain_graph=True)
+    (again,) = torch.autograd.grad(loss, s, retain_graph=True)
+    assert torch.equal(one, again) and torch.equal(half.float(), one.float() * 0.5)
+    (last,) = torch.autograd.grad(loss, s, torch.tensor(2.0, device=DEV))
+    assert torch.equal(last.float(), one.float() * 2)

@@ -197,6 +197,29 @@ def sgd_step_(p, g, buf, chunks, seg_hp, grad_scale=1.0, teacher=None, ema_m=0.0
 # ---------------------------------------------------------------------------------------------
 # losses: forward computes value AND gradient; backward only scales
 # ---------------------------------------------------------------------------------------------
+def _plain(t: torch.Tensor) -> bool:
+    """A tensor whose memory a kernel can read: not a batched or otherwise wrapped stand-in (vmap, tracing)."""
+    return type(t) is torch.Tensor and not (torch._C._functorch.is_legacy_batchedtensor(t)
+                                            or torch._C._functorch.is_functorch_wrapped_tensor(t))
+
+
+def _scaled(g: torch.Tensor, gout: torch.Tensor) -> torch.Tensor:
+    """``g * gout`` for a gradient ``g`` that the forward has computed and saved and the loss's gradient ``gout`` (a scalar).
+    As plain ops where the product is recorded itself (``create_graph``) or ``gout`` is no plain fp32 scalar.  In place where
+    the graph is freed behind this backward, so that nobody else will read ``g`` (a CUDA graph may be replayed: not
+    there); then ``gout = 1``, a loss that is differentiated as it is, costs no pass over the gradient."""
+    if (torch.is_grad_enabled() or not (_plain(g) and _plain(gout)) or gout.dtype != torch.float32 or gout.dim() != 0
+            or gout.device != g.device or not g.is_contiguous() or g.data_ptr() % 16):
+        return g * gout.to(g.dtype)
+    own = not torch._C._autograd._get_current_graph_task_keep_graph() and not torch.cuda.is_current_stream_capturing()
+    out = g if own else torch.empty_like(g)
+    with on_device(g.device):
+        _check(lib().tsp_scale(_ptr(g), _ptr(gout), _ptr(out), _c.c_int64(g.numel()), _c.c_int(_dt(g)), _stream()),
+               "tsp_scale")
+    _count()
+    return out
+
+
 class _ByolPair(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, y, scale):
@@ -215,7 +238,7 @@ class _ByolPair(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         (gx,) = ctx.saved_tensors
-        return gx * gout.to(gx.dtype), None, None
+        return _scaled(gx, gout), None, None
 
 
 def byol_pair_loss(x: torch.Tensor, y: torch.Tensor, scale: float) -> torch.Tensor:
@@ -224,8 +247,35 @@ def byol_pair_loss(x: torch.Tensor, y: torch.Tensor, scale: float) -> torch.Tens
     return _ByolPair.apply(x, y, scale)
 
 
+class _ByolBoth(torch.autograd.Function):
+    """Both directions of the symmetric loss from one launch, their gradients scaled by another."""
+
+    @staticmethod
+    def forward(ctx, x1, x2, y1, y2, scale):
+        n, d = x1.shape
+        loss = torch.empty((), dtype=torch.float32, device=x1.device)
+        gx = torch.empty((2, n, d), dtype=x1.dtype, device=x1.device)
+        with on_device(x1.device):
+            _check(lib().tsp_byol_loss_pair(_ptr(x1), _ptr(y1), _ptr(x2), _ptr(y2), _c.c_int(n), _c.c_int(d),
+                                            _c.c_int(_dt(x1)), _c.c_float(scale), _ptr(loss), _ptr(gx), _stream()),
+                   "tsp_byol_loss_pair")
+        _count()
+        ctx.save_for_backward(gx)
+        return loss
+
+    @staticmethod
+    def backward(ctx, gout):
+        (gx,) = ctx.saved_tensors
+        g1, g2 = _scaled(gx, gout).unbind(0)
+        need = ctx.needs_input_grad
+        return g1 if need[0] else None, g2 if need[1] else None, None, None, None
+
+
 def byol_loss(o1, o2, t1, t2) -> torch.Tensor:
     n = o1.shape[0]
+    if all(t.dim() == 2 and t.shape == o1.shape and t.dtype == o1.dtype and t.device == o1.device
+           and t.is_contiguous() for t in (o1, o2, t1, t2)) and o1.dtype in (torch.float32, torch.bfloat16) and n > 0:
+        return _ByolBoth.apply(o1, o2, t2.detach(), t1.detach(), 1.0 / n)
     return byol_pair_loss(o1, t2, 1.0 / n) + byol_pair_loss(o2, t1, 1.0 / n)
 
 
@@ -255,7 +305,7 @@ class _KdCe(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         (gs,) = ctx.saved_tensors
-        return (gs * gout.to(gs.dtype)).view(ctx.shape), None, None, None, None, None, None
+        return _scaled(gs, gout).view(ctx.shape), None, None, None, None, None, None
 
 
 def kd_ce_loss(s, t, labels, temp: float, w_ce: float, w_kd: float, row_mask=None) -> torch.Tensor:
@@ -295,7 +345,7 @@ class _Cosine(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         (gx,) = ctx.saved_tensors
-        return (gx * gout.to(gx.dtype)).view(ctx.shape), None, None, None
+        return _scaled(gx, gout).view(ctx.shape), None, None, None
 
 
 def cosine_embedding_loss(x, y, scale: float, row_mask=None) -> torch.Tensor:
