@@ -59,6 +59,13 @@ __device__ __forceinline__ ChunkView load_chunk(const int64_t* __restrict__ chun
   return v;
 }
 
+// How many 16-byte vectors of a chunk can be updated at once: all of its body when the chunk starts on a vector, every
+// buffer does (`bits`: their addresses or-ed) and the teacher's end does not cut a vector; none otherwise.  AdamW over 86.6 M
+// parameters with the EMA teacher, 3.1 GB: 700 us with 4-byte accesses, 495 (6.3 TB/s) with 16-byte ones.
+__device__ __forceinline__ int vec4_body(const ChunkView& c, uintptr_t bits, bool has_t, int64_t teacher_n) {
+  return ((c.begin & 3) == 0 && (bits & 15) == 0 && !(has_t && (teacher_n & 3) != 0)) ? c.len >> 2 : 0;
+}
+
 // norms[2*seg] += sum p^2 ; norms[2*seg+1] += sum (grad_scale*g + wd*p)^2   (only segments with adapt != 0)
 __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __restrict__ p, const float* __restrict__ g,
                                                               const int64_t* __restrict__ chunks,
@@ -75,6 +82,7 @@ __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __res
     const float4* p4 = reinterpret_cast<const float4*>(p + c.begin);
     const float4* g4 = reinterpret_cast<const float4*>(g + c.begin);
     const int n4 = c.len >> 2;
+#pragma unroll 4
     for (int i = threadIdx.x; i < n4; i += kThreads) {
       const float4 a = p4[i], b = g4[i];
       float u;
@@ -104,14 +112,17 @@ __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __res
 
 // LARS apply (+ optional fused momentum-teacher update for segments that have a local teacher copy):
 //   dp = adapt ? q*(gs*g + wd*p) : gs*g ; mu = mom*mu + dp ; p -= lr*mu ; [t = m*t + (1-m)*p]
+// `last_first`: the chunks are walked from the last one back, right behind lars_norms_kernel, which has left the end of
+// p and g in L2 (up to 126 MB of them); the buffers that only this kernel touches pass L2 with evict-first hints.  Both passes
+// over 25.6 M parameters: 163.6 us walked in the same order, 161.3 this way.
 __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict__ p, const float* __restrict__ g,
                                                               float* __restrict__ mu,
                                                               const int64_t* __restrict__ chunks,
                                                               const float* __restrict__ seg_hp, float grad_scale,
                                                               const float* __restrict__ norms,
                                                               float* __restrict__ teacher, int64_t teacher_n,
-                                                              float ema_m) {
-  const ChunkView c = load_chunk(chunks, blockIdx.x);
+                                                              float ema_m, int last_first) {
+  const ChunkView c = load_chunk(chunks, last_first ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
   const float* hp = seg_hp + 5 * (int64_t)c.seg;
   const float lr = hp[0], wd = hp[1], mom = hp[2], trust = hp[3];
   const bool adapt = hp[4] != 0.f;
@@ -129,11 +140,12 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
   const float4* g4 = reinterpret_cast<const float4*>(g + c.begin);
   float4* m4 = reinterpret_cast<float4*>(mu + c.begin);
   float4* t4 = has_t ? reinterpret_cast<float4*>(teacher + c.begin) : nullptr;
+#pragma unroll 2
   for (int i = threadIdx.x; i < n4; i += kThreads) {
-    float4 pv = p4[i], mv = m4[i];
-    const float4 gv = g4[i];
+    float4 pv = p4[i], mv = __ldcs(m4 + i);
+    const float4 gv = __ldcs(g4 + i);
     const bool t_ok = has_t && (c.begin + 4 * (int64_t)i + 3 < teacher_n);
-    float4 tv = t_ok ? t4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 tv = t_ok ? __ldcs(t4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #define TSP_LARS1(X)                                                   \
     {                                                                  \
       const float dp = q * (grad_scale * gv.X + wd_eff * pv.X);        \
@@ -144,8 +156,8 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
     TSP_LARS1(x) TSP_LARS1(y) TSP_LARS1(z) TSP_LARS1(w)
 #undef TSP_LARS1
     p4[i] = pv;
-    m4[i] = mv;
-    if (t_ok) t4[i] = tv;
+    __stcs(m4 + i, mv);
+    if (t_ok) __stcs(t4 + i, tv);
   }
   for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += kThreads) {
     const int64_t k = c.begin + i;
@@ -171,16 +183,45 @@ __global__ void __launch_bounds__(kThreads) adamw_kernel(float* __restrict__ p, 
   const float om = 1.f - ema_m;
   const float step = lr / bc1;
   const float inv_sqrt_bc2 = rsqrtf(bc2);
-  for (int i = threadIdx.x; i < c.len; i += kThreads) {
-    const int64_t k = c.begin + i;
-    const float gv = grad_scale * g[k];
-    float pv = p[k] * (1.f - lr * wd);
-    const float mv = b1 * m[k] + (1.f - b1) * gv;
-    const float vv = b2 * v[k] + (1.f - b2) * gv * gv;
-    m[k] = mv; v[k] = vv;
+  const bool has_t = teacher != nullptr;
+  auto one = [&](float& pv, float gv, float& mv, float& vv, float& tv) {
+    gv *= grad_scale;
+    pv *= 1.f - lr * wd;
+    mv = b1 * mv + (1.f - b1) * gv;
+    vv = b2 * vv + (1.f - b2) * gv * gv;
     pv -= step * mv / (sqrtf(vv) * inv_sqrt_bc2 + eps);
+    tv = ema_m * tv + om * pv;
+  };
+  // 16-byte vectors over the aligned body (up to five loads in flight per thread and trip), scalars for the tail
+  const int n4 = vec4_body(c, (uintptr_t)p | (uintptr_t)g | (uintptr_t)m | (uintptr_t)v | (uintptr_t)teacher, has_t, teacher_n);
+  float4* p4 = reinterpret_cast<float4*>(p + c.begin);
+  const float4* g4 = reinterpret_cast<const float4*>(g + c.begin);
+  float4* m4 = reinterpret_cast<float4*>(m + c.begin);
+  float4* v4 = reinterpret_cast<float4*>(v + c.begin);
+  float4* t4 = has_t ? reinterpret_cast<float4*>(teacher + c.begin) : nullptr;
+  for (int i = threadIdx.x; i < n4; i += kThreads) {
+    float4 pv = p4[i], mv = m4[i], vv = v4[i];
+    const float4 gv = g4[i];
+    const bool t_ok = has_t && (c.begin + 4 * (int64_t)i + 3 < teacher_n);
+    float4 tv = t_ok ? t4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    one(pv.x, gv.x, mv.x, vv.x, tv.x);
+    one(pv.y, gv.y, mv.y, vv.y, tv.y);
+    one(pv.z, gv.z, mv.z, vv.z, tv.z);
+    one(pv.w, gv.w, mv.w, vv.w, tv.w);
+    p4[i] = pv;
+    m4[i] = mv;
+    v4[i] = vv;
+    if (t_ok) t4[i] = tv;
+  }
+  for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += kThreads) {
+    const int64_t k = c.begin + i;
+    const bool t_ok = has_t && k < teacher_n;
+    float pv = p[k], mv = m[k], vv = v[k], tv = t_ok ? teacher[k] : 0.f;
+    one(pv, g[k], mv, vv, tv);
     p[k] = pv;
-    if (teacher != nullptr && k < teacher_n) teacher[k] = ema_m * teacher[k] + om * pv;
+    m[k] = mv;
+    v[k] = vv;
+    if (t_ok) teacher[k] = tv;
   }
 }
 
@@ -194,18 +235,44 @@ __global__ void __launch_bounds__(kThreads) sgd_kernel(float* __restrict__ p, co
   const float lr = hp[0], mom = hp[1], damp = hp[2], wd = hp[3];
   const bool nesterov = hp[4] != 0.f, first = hp[5] != 0.f;
   const float om = 1.f - ema_m;
-  for (int i = threadIdx.x; i < c.len; i += kThreads) {
-    const int64_t k = c.begin + i;
-    const float pv = p[k];
-    float d = grad_scale * g[k] + wd * pv;
-    if (mom != 0.f) {
-      const float b = first ? d : mom * buf[k] + (1.f - damp) * d;
-      buf[k] = b;
-      d = nesterov ? d + mom * b : b;
+  const bool has_t = teacher != nullptr, has_b = mom != 0.f;
+  auto one = [&](float& pv, float gv, float& bv, float& tv) {
+    float d = grad_scale * gv + wd * pv;
+    if (has_b) {
+      bv = first ? d : mom * bv + (1.f - damp) * d;
+      d = nesterov ? d + mom * bv : bv;
     }
-    const float np = pv - lr * d;
-    p[k] = np;
-    if (teacher != nullptr && k < teacher_n) teacher[k] = ema_m * teacher[k] + om * np;
+    pv -= lr * d;
+    tv = ema_m * tv + om * pv;
+  };
+  const int n4 = vec4_body(c, (uintptr_t)p | (uintptr_t)g | (uintptr_t)buf | (uintptr_t)teacher, has_t, teacher_n);
+  float4* p4 = reinterpret_cast<float4*>(p + c.begin);
+  const float4* g4 = reinterpret_cast<const float4*>(g + c.begin);
+  float4* b4 = reinterpret_cast<float4*>(buf + c.begin);
+  float4* t4 = has_t ? reinterpret_cast<float4*>(teacher + c.begin) : nullptr;
+#pragma unroll 2
+  for (int i = threadIdx.x; i < n4; i += kThreads) {
+    float4 pv = p4[i];
+    const float4 gv = g4[i];
+    const bool t_ok = has_t && (c.begin + 4 * (int64_t)i + 3 < teacher_n);
+    float4 bv = has_b && !first ? b4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 tv = t_ok ? t4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    one(pv.x, gv.x, bv.x, tv.x);
+    one(pv.y, gv.y, bv.y, tv.y);
+    one(pv.z, gv.z, bv.z, tv.z);
+    one(pv.w, gv.w, bv.w, tv.w);
+    p4[i] = pv;
+    if (has_b) b4[i] = bv;
+    if (t_ok) t4[i] = tv;
+  }
+  for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += kThreads) {
+    const int64_t k = c.begin + i;
+    const bool t_ok = has_t && k < teacher_n;
+    float pv = p[k], bv = has_b && !first ? buf[k] : 0.f, tv = t_ok ? teacher[k] : 0.f;
+    one(pv, g[k], bv, tv);
+    p[k] = pv;
+    if (has_b) buf[k] = bv;
+    if (t_ok) teacher[k] = tv;
   }
 }
 
@@ -238,7 +305,7 @@ int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, in
   if (e != cudaSuccess) return (int)e;
   lars_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, chunks, seg_hp, grad_scale, norms);
   lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, seg_hp, grad_scale, norms, teacher,
-                                                       teacher_n, ema_m);
+                                                       teacher_n, ema_m, 1);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -256,7 +323,7 @@ int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, i
                    cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
   lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, seg_hp, grad_scale, norms, teacher,
-                                                       teacher_n, ema_m);
+                                                       teacher_n, ema_m, 0);
   return TSP_LAUNCH_CHECK();
 }
 

@@ -104,7 +104,14 @@ class _FlatMixin:
     def _hp_table(self, rows: List[List[float]]) -> torch.Tensor:
         key = tuple(tuple(r) for r in rows)
         if self._hp_cache is None or self._hp_cache[0] != key:
-            self._hp_cache = (key, torch.tensor(rows, dtype=torch.float32, device=self.flat.device))
+            dev = self.flat.device
+            if dev.type == "cuda" and not torch.cuda.is_current_stream_capturing():
+                # a copy from pinned memory (kept by the host allocator until the copy is done) is ordered on the stream;
+                # one from pageable memory would first wait on the host for everything enqueued before it
+                table = torch.tensor(rows, dtype=torch.float32).pin_memory().to(dev, non_blocking=True)
+            else:
+                table = torch.tensor(rows, dtype=torch.float32, device=dev)
+            self._hp_cache = (key, table)
         return self._hp_cache[1]
 
     def flat_state_dict(self) -> Dict[str, Any]:
