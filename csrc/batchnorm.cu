@@ -16,6 +16,21 @@ namespace {
 
 constexpr int kBlock = 256;
 
+// ---------------------------------------------------------------------------------------------
+// per-channel sums:  out[c] += sum_rows a(r,c),  out[C + c] += sum_rows b(r,c)
+//   MODE 0 (forward statistics): a = x, b = x*x
+//   MODE 1 (backward reduction): a = dy', b = dy' * (x - mean) * rstd with dy' = dy masked by the ReLU:
+//          mask from y > 0 when `y` is given (residual case), else recomputed as scale*x + shift > 0 when
+//          `relu` is set (no extra tensor read); optionally stores dy' to dres.
+//   MODE 2 (bias gradients): a = x, no b
+//
+// For what the streaming kernel below does not take: fp32, widths that are no power of two, tensors of at most a
+// megabyte or so.  Those are bound by latency, so a block is 32 channel vectors (512 contiguous bytes of a row) by 8
+// rows, every thread has 4 or 8 rows in flight, and the rows are split over as many blocks as fill the chip - down to
+// one trip per thread.  The backward reduction of [2 x 128, 4096] bf16 and the bias gradients of 12608 rows (768 - 3072 columns, each), B200:
+// 17.4 and 20 us with fewer rows in flight and additions that share sectors, 4.2 and 8 this way.
+// grid = (row blocks, channel slabs, segments).
+// ---------------------------------------------------------------------------------------------
 struct Tile {
   int tx_n;   // threads along the channel-vector axis
   int ty_n;   // rows processed in parallel by a block
@@ -23,27 +38,20 @@ struct Tile {
 
 __host__ __device__ inline Tile make_tile(int cpv) {
   Tile t;
-  t.tx_n = cpv < kBlock ? cpv : kBlock;
+  t.tx_n = cpv < 32 ? cpv : 32;
   t.ty_n = kBlock / t.tx_n;
-  if (t.ty_n < 1) t.ty_n = 1;
   return t;
 }
 
-// ---------------------------------------------------------------------------------------------
-// per-channel sums:  out[c] += sum_rows a(r,c),  out[C + c] += sum_rows b(r,c)
-//   MODE 0 (forward statistics): a = x, b = x*x
-//   MODE 1 (backward reduction): a = dy', b = dy' * (x - mean) * rstd with dy' = dy masked by the ReLU:
-//          mask from y > 0 when `y` is given (residual case), else recomputed as scale*x + shift > 0 when
-//          `relu` is set (no extra tensor read); optionally stores dy' to dres.
-// grid = (row blocks, channel slabs); block = tx_n * ty_n threads; smem = ty_n * tx_n * 16 floats.
-// ---------------------------------------------------------------------------------------------
+template <typename T, int MODE> struct ColsumRows { static constexpr int value = MODE == 1 ? (sizeof(T) == 2 ? 3 : 2) : (sizeof(T) == 2 ? 8 : 4); };
+
 template <typename T, int MODE>
-__global__ void __launch_bounds__(kBlock, MODE == 0 ? 5 : 2) bn_colsum_kernel(const T* __restrict__ x, const T* __restrict__ dy,
+__global__ void __launch_bounds__(kBlock, 2) bn_colsum_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                            const T* __restrict__ y, T* __restrict__ dres,
                                                            const float* __restrict__ mean_rstd,
                                                            const float* __restrict__ w, const float* __restrict__ bias,
                                                            int relu, int64_t m, int c, float* __restrict__ out) {
-  extern __shared__ float sm[];
+  __shared__ float sm[(kBlock + 4) * 16];
   {   // blockIdx.z = segment: an independent group of m rows with its own statistics
     const int64_t so = (int64_t)blockIdx.z * m * c;
     x += so;
@@ -53,6 +61,7 @@ __global__ void __launch_bounds__(kBlock, MODE == 0 ? 5 : 2) bn_colsum_kernel(co
     if (mean_rstd != nullptr) mean_rstd += (int64_t)blockIdx.z * 2 * c;
     out += (int64_t)blockIdx.z * 2 * c;
   }
+  constexpr int U = ColsumRows<T, MODE>::value;
   const int cpv = c >> 3;
   const Tile tl = make_tile(cpv);
   const int tx = threadIdx.x % tl.tx_n, ty = threadIdx.x / tl.tx_n;
@@ -61,96 +70,88 @@ __global__ void __launch_bounds__(kBlock, MODE == 0 ? 5 : 2) bn_colsum_kernel(co
   float a[8], b[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) { a[e] = 0.f; b[e] = 0.f; }
-  float mu[8], rs[8], sc[8], sh[8];
-  const bool recompute_mask = (MODE == 1) && relu && (y == nullptr);
-  if (MODE == 1 && active) {
-    tsp::ld8(mean_rstd, (int64_t)cg * 8, mu);
-    tsp::ld8(mean_rstd + c, (int64_t)cg * 8, rs);
-    if (recompute_mask) {
-      float wv[8], bv[8];
-      tsp::ld8(w, (int64_t)cg * 8, wv);
-      tsp::ld8(bias, (int64_t)cg * 8, bv);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { sc[e] = wv[e] * rs[e]; sh[e] = bv[e] - mu[e] * sc[e]; }
-    }
-  }
   if (active) {
-    // each block owns one contiguous range of rows: consecutive iterations stream consecutive memory
+    // each block owns one contiguous range of rows
     const int64_t rows_per_block = (m + gridDim.x - 1) / gridDim.x;
     const int64_t r_begin = (int64_t)blockIdx.x * rows_per_block;
     const int64_t r_end = r_begin + rows_per_block < m ? r_begin + rows_per_block : m;
-    const int64_t step = tl.ty_n;
-    const int64_t col = (int64_t)cg * 8;
-    int64_t r = r_begin + ty;
-    if (MODE == 0) {
-      // eight independent 16/32-byte loads in flight per thread before any arithmetic (raw registers)
-      for (; r + 7 * step < r_end; r += 8 * step) {
-        tsp::Raw8<T> raw[8];
+    const int64_t step = tl.ty_n, col = (int64_t)cg * 8;
+    float mu[8], rs[8], sc[8], sh[8];
+    const bool recompute_mask = (MODE == 1) && relu && (y == nullptr);
+    if (MODE == 1) {
+      tsp::ld8(mean_rstd, col, mu);
+      tsp::ld8(mean_rstd + c, col, rs);
+      if (recompute_mask) {
+        float wv[8], bv[8];
+        tsp::ld8(w, col, wv);
+        tsp::ld8(bias, col, bv);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) tsp::ldraw(x, (r + u * step) * c + col, raw[u]);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          float v[8];
-          tsp::cvt8(raw[u], v);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) { a[e] += v[e]; b[e] += v[e] * v[e]; }
-        }
+        for (int e = 0; e < 8; ++e) { sc[e] = wv[e] * rs[e]; sh[e] = bv[e] - mu[e] * sc[e]; }
       }
-      for (; r < r_end; r += step) {
-        float v0[8];
-        tsp::ld8(x, r * c + col, v0);
+    }
+    for (int64_t r = r_begin + ty; r < r_end; r += U * step) {
+      // the loads of a trip are all issued before the first use; rows past the end are skipped
+      tsp::Raw8<T> xr[U], gr[MODE == 1 ? U : 1], yr[MODE == 1 ? U : 1];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) { a[e] += v0[e]; b[e] += v0[e] * v0[e]; }
-      }
-    } else {
-      for (; r < r_end; r += 2 * step) {
-        const bool two = r + step < r_end;
-        const int64_t off0 = r * c + col, off1 = (r + step) * c + col;
-        float x0[8], x1[8], g0[8], g1[8], y0[8], y1[8];
-        tsp::ld8(x, off0, x0);
-        tsp::ld8(dy, off0, g0);
-        if (y != nullptr) tsp::ld8(y, off0, y0);
-        if (two) {
-          tsp::ld8(x, off1, x1);
-          tsp::ld8(dy, off1, g1);
-          if (y != nullptr) tsp::ld8(y, off1, y1);
-        }
-        if (y != nullptr) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) { g0[e] = y0[e] > 0.f ? g0[e] : 0.f; if (two) g1[e] = y1[e] > 0.f ? g1[e] : 0.f; }
-        } else if (recompute_mask) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            g0[e] = (x0[e] * sc[e] + sh[e]) > 0.f ? g0[e] : 0.f;
-            if (two) g1[e] = (x1[e] * sc[e] + sh[e]) > 0.f ? g1[e] : 0.f;
+      for (int u = 0; u < U; ++u)
+        if (r + u * step < r_end) {
+          const int64_t off = (r + u * step) * c + col;
+          tsp::ldraw(x, off, xr[u]);
+          if constexpr (MODE == 1) {
+            tsp::ldraw(dy, off, gr[u]);
+            if (y != nullptr) tsp::ldraw(y, off, yr[u]);
           }
         }
-        if (dres != nullptr) { tsp::st8(dres, off0, g0); if (two) tsp::st8(dres, off1, g1); }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          a[e] += g0[e]; b[e] += g0[e] * (x0[e] - mu[e]) * rs[e];
-          if (two) { a[e] += g1[e]; b[e] += g1[e] * (x1[e] - mu[e]) * rs[e]; }
+      for (int u = 0; u < U; ++u)
+        if (r + u * step < r_end) {
+          float v[8];
+          tsp::cvt8(xr[u], v);
+          if constexpr (MODE == 0) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { a[e] += v[e]; b[e] += v[e] * v[e]; }
+          } else if constexpr (MODE == 2) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) a[e] += v[e];
+          } else {
+            float g[8];
+            tsp::cvt8(gr[u], g);
+            if (y != nullptr) {
+              float yv[8];
+              tsp::cvt8(yr[u], yv);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) g[e] = yv[e] > 0.f ? g[e] : 0.f;
+            } else if (recompute_mask) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) g[e] = (v[e] * sc[e] + sh[e]) > 0.f ? g[e] : 0.f;
+            }
+            if (dres != nullptr) tsp::st8(dres, (r + u * step) * c + col, g);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { a[e] += g[e]; b[e] += g[e] * (v[e] - mu[e]) * rs[e]; }
+          }
         }
-      }
     }
   }
-  // reduce over ty through shared memory, then one atomic per channel per block
-  float* mine = sm + ((int64_t)ty * tl.tx_n + tx) * 16;
+  // sum over ty through shared memory, then one addition per channel and block, lane = channel: a warp's additions go out
+  // as whole sectors.  (Additions to one sector are serialised at some 15 ns each; with eight lanes' worth of
+  // instructions per sector that was the whole time of the kernel.)
+  constexpr int kVals = MODE == 2 ? 8 : 16;
+  constexpr int pitch = kBlock + 4;                  // values 4 banks apart: the reads below are conflict-free
   if (ty < tl.ty_n) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) { mine[e] = a[e]; mine[8 + e] = b[e]; }
+    for (int e = 0; e < 8; ++e) {
+      sm[e * pitch + threadIdx.x] = a[e];
+      if (MODE != 2) sm[(8 + e) * pitch + threadIdx.x] = b[e];
+    }
   }
   __syncthreads();
-  if (ty == 0 && cg < cpv) {
-    for (int k = 1; k < tl.ty_n; ++k) {
-      const float* o = sm + ((int64_t)k * tl.tx_n + tx) * 16;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { a[e] += o[e]; b[e] += o[8 + e]; }
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      atomicAdd(out + cg * 8 + e, a[e]);
-      atomicAdd(out + c + cg * 8 + e, b[e]);
+  for (int p = threadIdx.x; p < kVals * tl.tx_n; p += kBlock) {
+    const int half = p >= 8 * tl.tx_n ? 1 : 0, q = p - half * 8 * tl.tx_n;
+    const int e = q & 7, px = q >> 3, ch = blockIdx.y * tl.tx_n * 8 + q;
+    if (ch < c) {
+      float acc = 0.f;
+      for (int k = 0; k < tl.ty_n; ++k) acc += sm[(half * 8 + e) * pitch + k * tl.tx_n + px];
+      atomicAdd(out + half * c + ch, acc);
     }
   }
 }
@@ -372,14 +373,20 @@ bn_colsum_stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 
 // ---------------------------------------------------------------------------------------------
 // forward apply: y = act(scale*x + shift [+ res]).
-//   training: mean/var from `sums` (sum, sum of squares over m rows); block 0 saves mean / rstd and folds the
+//   training: mean/var from `sums` (sum, sum of squares over m rows); the first threads save mean / rstd and fold the
 //             sums into the deferred accumulators (acc_sum, acc_sumsq) when given.
 //   eval:     mean/var from `fixed` ([mean | var]).
-// dynamic smem: 2*c floats (scale | shift).  A thread's channel group is loop-invariant whenever the grid
-// stride is a multiple of c/8 (all power-of-two widths), so scale/shift then stay in registers.
+// The grid stride is a multiple of c/8 (apply_blocks), so a thread meets one channel vector only and derives its scale
+// and shift itself, in registers, while its first activations are on their way.  (A table of all channels per block,
+// behind a barrier, cost more than the pass itself on the small tensors: [2 x 128, 4096] took 27.6 us with it and takes 8.0.)
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(kBlock) bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res,
+// vectors in flight per thread and array (64 - 80 registers)
+template <typename T> struct ApplyVecs {
+  static constexpr int fwd = sizeof(T) == 2 ? 4 : 2, fwd_res = sizeof(T) == 2 ? 3 : 1, bwd = sizeof(T) == 2 ? 2 : 1;
+};
+
+template <typename T, bool RES>
+__global__ void __launch_bounds__(kBlock, 3) bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res,
                                                           T* __restrict__ y, const float* __restrict__ sums,
                                                           const float* __restrict__ fixed,
                                                           const float* __restrict__ w, const float* __restrict__ b,
@@ -387,67 +394,78 @@ __global__ void __launch_bounds__(kBlock) bn_apply_kernel(const T* __restrict__ 
                                                           float* __restrict__ acc_sum, float* __restrict__ acc_sumsq,
                                                           float* __restrict__ acc_count, int64_t acc_seg_stride,
                                                           int64_t m, int c, float eps, int relu) {
-  extern __shared__ float sm[];
   {   // blockIdx.y = segment: m rows with their own statistics (and their own set of accumulators)
     const int64_t so = (int64_t)blockIdx.y * m * c;
     x += so;
     y += so;
-    if (res != nullptr) res += so;
+    if (RES) res += so;
     if (sums != nullptr) sums += (int64_t)blockIdx.y * 2 * c;
     if (save_mean_rstd != nullptr) save_mean_rstd += (int64_t)blockIdx.y * 2 * c;
     if (acc_sum != nullptr) { acc_sum += blockIdx.y * acc_seg_stride; acc_sumsq += blockIdx.y * acc_seg_stride; }
     if (acc_count != nullptr) acc_count += blockIdx.y * acc_seg_stride;
   }
-  float* scale = sm;
-  float* shift = sm + c;
-  const float inv_m = 1.f / (float)m;
-  for (int i = threadIdx.x; i < c; i += blockDim.x) {
-    float mean, var;
-    if (fixed != nullptr) {
-      mean = fixed[i]; var = fixed[c + i];
-    } else {
-      const float s = sums[i], q = sums[c + i];
-      mean = s * inv_m;
-      var = fmaxf(q * inv_m - mean * mean, 0.f);
-      if (blockIdx.x == 0) {
-        if (acc_sum != nullptr) { acc_sum[i] += s; acc_sumsq[i] += q; }
-        if (acc_count != nullptr) acc_count[i] += (float)m;
-      }
-    }
-    const float rstd = rsqrtf(var + eps);
-    if (blockIdx.x == 0 && save_mean_rstd != nullptr) { save_mean_rstd[i] = mean; save_mean_rstd[c + i] = rstd; }
-    const float sc = (w ? w[i] : 1.f) * rstd;
-    scale[i] = sc;
-    shift[i] = (b ? b[i] : 0.f) - mean * sc;
-  }
-  __syncthreads();
+  constexpr int U = RES ? ApplyVecs<T>::fwd_res : ApplyVecs<T>::fwd;
   const int cpv = c >> 3;
   const int64_t nvec = m * cpv;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * kBlock;
+  const int first = blockIdx.x * kBlock + threadIdx.x;
+  int64_t i = first;
   if (i >= nvec) return;
-  int cg = (int)(i % cpv);
-  const int dcg = (int)(stride % cpv);
-  float sc[8], sh[8];
+  const int ch = (first % cpv) * 8;
+  tsp::Raw8<T> xr[U], rr[RES ? U : 1];
+  auto load = [&](int64_t at) {
 #pragma unroll
-  for (int e = 0; e < 8; ++e) { sc[e] = scale[cg * 8 + e]; sh[e] = shift[cg * 8 + e]; }
-  if (dcg == 0) {
-    // four independent vectors per thread and trip: all loads are issued before the first use
-    for (; i + 3 * stride < nvec; i += 4 * stride) {
-      tsp::Raw8<T> xr[4], rr[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) tsp::ldraw(x, (i + u * stride) * 8, xr[u]);
-      if (res != nullptr) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) tsp::ldraw(res, (i + u * stride) * 8, rr[u]);
+    for (int u = 0; u < U; ++u)
+      if (at + u * stride < nvec) {
+        tsp::ldraw(x, (at + u * stride) * 8, xr[u]);
+        if constexpr (RES) tsp::ldraw(res, (at + u * stride) * 8, rr[u]);
       }
+  };
+  load(i);
+  float sc[8], sh[8];
+  {
+    float mean[8], var[8];
+    if (fixed != nullptr) {
+      tsp::ld8(fixed, ch, mean);
+      tsp::ld8(fixed + c, ch, var);
+    } else {
+      const float inv_m = 1.f / (float)m;
+      float s[8], q[8];
+      tsp::ld8(sums, ch, s);
+      tsp::ld8(sums + c, ch, q);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float v[8], o[8];
-        tsp::cvt8(xr[u], v);
+      for (int e = 0; e < 8; ++e) {
+        mean[e] = s[e] * inv_m;
+        var[e] = fmaxf(q[e] * inv_m - mean[e] * mean[e], 0.f);
+      }
+      if (first < cpv) {                                  // the first c/8 threads own the channels' bookkeeping
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = v[e] * sc[e] + sh[e];
-        if (res != nullptr) {
+        for (int e = 0; e < 8; ++e) {
+          if (acc_sum != nullptr) { acc_sum[ch + e] += s[e]; acc_sumsq[ch + e] += q[e]; }
+          if (acc_count != nullptr) acc_count[ch + e] += (float)m;
+        }
+      }
+    }
+    float wv[8], bv[8];
+    if (w != nullptr) tsp::ld8(w, ch, wv);
+    if (b != nullptr) tsp::ld8(b, ch, bv);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float rstd = rsqrtf(var[e] + eps);
+      if (first < cpv && save_mean_rstd != nullptr) { save_mean_rstd[ch + e] = mean[e]; save_mean_rstd[c + ch + e] = rstd; }
+      sc[e] = (w != nullptr ? wv[e] : 1.f) * rstd;
+      sh[e] = (b != nullptr ? bv[e] : 0.f) - mean[e] * sc[e];
+    }
+  }
+  while (true) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * stride < nvec) {
+        float o[8];
+        tsp::cvt8(xr[u], o);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = o[e] * sc[e] + sh[e];
+        if constexpr (RES) {
           float r[8];
           tsp::cvt8(rr[u], r);
 #pragma unroll
@@ -459,108 +477,85 @@ __global__ void __launch_bounds__(kBlock) bn_apply_kernel(const T* __restrict__ 
         }
         tsp::st8(y, (i + u * stride) * 8, o);
       }
-    }
-  }
-  for (; i < nvec; i += stride) {
-    float v[8], o[8];
-    tsp::ld8(x, i * 8, v);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = v[e] * sc[e] + sh[e];
-    if (res != nullptr) {
-      float r[8];
-      tsp::ld8(res, i * 8, r);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] += r[e];
-    }
-    if (relu) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = fmaxf(o[e], 0.f);
-    }
-    tsp::st8(y, i * 8, o);
-    if (dcg != 0) {
-      cg += dcg;
-      if (cg >= cpv) cg -= cpv;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { sc[e] = scale[cg * 8 + e]; sh[e] = shift[cg * 8 + e]; }
-    }
+    i += U * stride;
+    if (i >= nvec) break;
+    load(i);
   }
 }
 
 // ---------------------------------------------------------------------------------------------
 // backward apply: dx = w*rstd * (dy' - sum(dy')/m - xhat * sum(dy'*xhat)/m), dy' masked as in the reduction
 // (by y > 0 when `y` is given, by scale*x + shift > 0 when `relu` is set and y is null).
-// Per element: dx = A*dy' + B*x + D with A = w*rstd, B = -A*rstd*k2, D = -A*k1 - B*mean.
-// dynamic smem: 5*c floats (A | B | D | scale | shift)
+// Per element: dx = A*dy' + B*x + D with A = w*rstd, B = -A*rstd*k2, D = -A*k1 - B*mean, in registers as above.
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(kBlock) bn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+// MASK: 0 none, 1 recomputed from x, 2 from y
+template <typename T, int MASK>
+__global__ void __launch_bounds__(kBlock, 3) bn_bwd_apply_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                               const T* __restrict__ y,
                                                               const float* __restrict__ mean_rstd,
                                                               const float* __restrict__ w,
-                                                              const float* __restrict__ bias, int relu,
+                                                              const float* __restrict__ bias,
                                                               const float* __restrict__ sums, T* __restrict__ dx,
                                                               int64_t m, int c) {
-  extern __shared__ float sm[];
   {   // blockIdx.y = segment
     const int64_t so = (int64_t)blockIdx.y * m * c;
     dy += so;
     x += so;
     dx += so;
-    if (y != nullptr) y += so;
+    if (MASK == 2) y += so;
     mean_rstd += (int64_t)blockIdx.y * 2 * c;
     sums += (int64_t)blockIdx.y * 2 * c;
   }
-  float* s_a = sm;
-  float* s_b = sm + c;
-  float* s_d = sm + 2 * c;
-  float* s_sc = sm + 3 * c;
-  float* s_sh = sm + 4 * c;
-  const float inv_m = 1.f / (float)m;
-  const bool recompute_mask = relu && (y == nullptr);
-  for (int i = threadIdx.x; i < c; i += blockDim.x) {
-    const float mean = mean_rstd[i], rs = mean_rstd[c + i];
-    const float k1 = sums[i] * inv_m, k2 = sums[c + i] * inv_m;
-    const float wv = w ? w[i] : 1.f;
-    const float A = wv * rs;
-    const float B = -A * rs * k2;
-    s_a[i] = A;
-    s_b[i] = B;
-    s_d[i] = -A * k1 - B * mean;
-    s_sc[i] = A;
-    s_sh[i] = (bias ? bias[i] : 0.f) - mean * A;
-  }
-  __syncthreads();
+  constexpr int U = ApplyVecs<T>::bwd;
   const int cpv = c >> 3;
   const int64_t nvec = m * cpv;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * kBlock;
+  const int first = blockIdx.x * kBlock + threadIdx.x;
+  int64_t i = first;
   if (i >= nvec) return;
-  int cg = (int)(i % cpv);
-  const int dcg = (int)(stride % cpv);
-  float A[8], B[8], D[8], sh[8];
+  const int ch = (first % cpv) * 8;
+  tsp::Raw8<T> gr[U], xr[U], yr[MASK == 2 ? U : 1];
+  auto load = [&](int64_t at) {
 #pragma unroll
-  for (int e = 0; e < 8; ++e) { A[e] = s_a[cg * 8 + e]; B[e] = s_b[cg * 8 + e]; D[e] = s_d[cg * 8 + e]; sh[e] = s_sh[cg * 8 + e]; }
-  if (dcg == 0) {
-    // two independent vectors per thread and trip (4 - 6 loads in flight)
-    for (; i + stride < nvec; i += 2 * stride) {
-      tsp::Raw8<T> gr[2], xr[2], yr[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) { tsp::ldraw(dy, (i + u * stride) * 8, gr[u]); tsp::ldraw(x, (i + u * stride) * 8, xr[u]); }
-      if (y != nullptr) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) tsp::ldraw(y, (i + u * stride) * 8, yr[u]);
+    for (int u = 0; u < U; ++u)
+      if (at + u * stride < nvec) {
+        tsp::ldraw(dy, (at + u * stride) * 8, gr[u]);
+        tsp::ldraw(x, (at + u * stride) * 8, xr[u]);
+        if constexpr (MASK == 2) tsp::ldraw(y, (at + u * stride) * 8, yr[u]);
       }
+  };
+  load(i);
+  float A[8], B[8], D[8], sh[8];
+  {
+    const float inv_m = 1.f / (float)m;
+    float mean[8], rs[8], k1[8], k2[8], wv[8], bv[8];
+    tsp::ld8(mean_rstd, ch, mean);
+    tsp::ld8(mean_rstd + c, ch, rs);
+    tsp::ld8(sums, ch, k1);
+    tsp::ld8(sums + c, ch, k2);
+    if (w != nullptr) tsp::ld8(w, ch, wv);
+    if (bias != nullptr) tsp::ld8(bias, ch, bv);
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+    for (int e = 0; e < 8; ++e) {
+      A[e] = (w != nullptr ? wv[e] : 1.f) * rs[e];
+      B[e] = -A[e] * rs[e] * (k2[e] * inv_m);
+      D[e] = -A[e] * (k1[e] * inv_m) - B[e] * mean[e];
+      sh[e] = (bias != nullptr ? bv[e] : 0.f) - mean[e] * A[e];
+    }
+  }
+  while (true) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * stride < nvec) {
         float g[8], xv[8], o[8];
         tsp::cvt8(gr[u], g);
         tsp::cvt8(xr[u], xv);
-        if (y != nullptr) {
+        if constexpr (MASK == 2) {
           float yv[8];
           tsp::cvt8(yr[u], yv);
 #pragma unroll
           for (int e = 0; e < 8; ++e) g[e] = yv[e] > 0.f ? g[e] : 0.f;
-        } else if (recompute_mask) {
+        } else if constexpr (MASK == 1) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) g[e] = (xv[e] * A[e] + sh[e]) > 0.f ? g[e] : 0.f;
         }
@@ -568,49 +563,25 @@ __global__ void __launch_bounds__(kBlock) bn_bwd_apply_kernel(const T* __restric
         for (int e = 0; e < 8; ++e) o[e] = A[e] * g[e] + B[e] * xv[e] + D[e];
         tsp::st8(dx, (i + u * stride) * 8, o);
       }
-    }
-  }
-  for (; i < nvec; i += stride) {
-    float g[8], xv[8], o[8];
-    tsp::ld8(dy, i * 8, g);
-    tsp::ld8(x, i * 8, xv);
-    if (y != nullptr) {
-      float yv[8];
-      tsp::ld8(y, i * 8, yv);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) g[e] = yv[e] > 0.f ? g[e] : 0.f;
-    } else if (recompute_mask) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) g[e] = (xv[e] * A[e] + sh[e]) > 0.f ? g[e] : 0.f;
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = A[e] * g[e] + B[e] * xv[e] + D[e];
-    tsp::st8(dx, i * 8, o);
-    if (dcg != 0) {
-      cg += dcg;
-      if (cg >= cpv) cg -= cpv;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { A[e] = s_a[cg * 8 + e]; B[e] = s_b[cg * 8 + e]; D[e] = s_d[cg * 8 + e]; sh[e] = s_sh[cg * 8 + e]; }
-    }
+    i += U * stride;
+    if (i >= nvec) break;
+    load(i);
   }
 }
 
-inline int row_blocks(int64_t m, int ty_n, int slabs) {
-  int64_t want = (m + ty_n - 1) / ty_n;
-  int64_t cap = (148 * 8) / (slabs > 0 ? slabs : 1);
-  if (cap < 1) cap = 1;
-  // keep at least ~32 rows per thread-row so that the atomics stay a small part of the work
-  int64_t by_work = (m + (int64_t)ty_n * 32 - 1) / ((int64_t)ty_n * 32);
-  if (by_work < 1) by_work = 1;
-  int64_t g = want < cap ? want : cap;
-  if (g > by_work) g = by_work;
+// Row blocks of bn_colsum_kernel: enough to fill the chip four times over all slabs and segments, but at least one trip of
+// `rows` rows per thread.
+inline int row_blocks(int64_t m, int ty_n, int rows, int slabs, int segs) {
+  const int64_t most = (m + (int64_t)ty_n * rows - 1) / ((int64_t)ty_n * rows);
+  int64_t g = (148 * 4) / (slabs * segs);
+  if (g > most) g = most;
   return (int)(g < 1 ? 1 : g);
 }
 
-inline int elem_blocks(int64_t nvec) {
-  int64_t b = (nvec + kBlock - 1) / kBlock;
-  if (b > 148 * 16) b = 148 * 16;
-  return (int)(b < 1 ? 1 : b);
+// Blocks of the apply passes for one of `segs` groups: two blocks per SM over all groups before a thread takes a second
+// vector, at most eight.
+inline int apply_blocks(int64_t nvec, int cpv, int per_thread, int segs) {
+  return tsp::row_stride_blocks(nvec, cpv, kBlock, per_thread, 148 * 2 / segs, 148 * 8 / segs);
 }
 
 // Streaming kernel eligibility: bf16, c/8 a power of two in [8, 256], enough rows to give every CTA work.
@@ -683,14 +654,31 @@ int tsp_bn_stats(const void* x, int64_t m, int c, int dtype, float* sums, int se
   const int cpv = c / 8;
   const Tile tl = make_tile(cpv);
   const int slabs = (cpv + tl.tx_n - 1) / tl.tx_n;
-  dim3 grid(row_blocks(m, tl.ty_n, slabs), slabs, segs);
-  const size_t smem = sizeof(float) * 16 * (size_t)tl.tx_n * tl.ty_n;
+  const dim3 grid(row_blocks(m, tl.ty_n, (dtype == TSP_DTYPE_BF16 ? ColsumRows<__nv_bfloat16, 0>::value : ColsumRows<float, 0>::value), slabs, segs), slabs, segs);
   if (dtype == TSP_DTYPE_BF16)
-    bn_colsum_kernel<__nv_bfloat16, 0><<<grid, kBlock, smem, stream>>>((const __nv_bfloat16*)x, nullptr, nullptr, nullptr,
+    bn_colsum_kernel<__nv_bfloat16, 0><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, nullptr, nullptr, nullptr,
                                                                        nullptr, nullptr, nullptr, 0, m, c, sums);
   else
-    bn_colsum_kernel<float, 0><<<grid, kBlock, smem, stream>>>((const float*)x, nullptr, nullptr, nullptr, nullptr, nullptr,
+    bn_colsum_kernel<float, 0><<<grid, kBlock, 0, stream>>>((const float*)x, nullptr, nullptr, nullptr, nullptr, nullptr,
                                                                nullptr, 0, m, c, sums);
+  return TSP_LAUNCH_CHECK();
+}
+
+// sums [c] fp32 = column sums of x [m, c] (the gradient of a bias).
+int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, cudaStream_t stream) {
+  if (m <= 0) return 0;
+  if (c % 8 != 0 || c > 8192) return -3;
+  cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(float) * (size_t)c, stream);
+  if (e != cudaSuccess) return (int)e;
+  const Tile tl = make_tile(c / 8);
+  const int slabs = (c / 8 + tl.tx_n - 1) / tl.tx_n;
+  const dim3 grid(row_blocks(m, tl.ty_n, (dtype == TSP_DTYPE_BF16 ? ColsumRows<__nv_bfloat16, 2>::value : ColsumRows<float, 2>::value), slabs, 1), slabs, 1);
+  if (dtype == TSP_DTYPE_BF16)
+    bn_colsum_kernel<__nv_bfloat16, 2><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, nullptr, nullptr, nullptr,
+                                                                    nullptr, nullptr, nullptr, 0, m, c, sums);
+  else
+    bn_colsum_kernel<float, 2><<<grid, kBlock, 0, stream>>>((const float*)x, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                                            nullptr, 0, m, c, sums);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -703,19 +691,14 @@ int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, con
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 4096 || segs < 1 || m % segs != 0) return -3;
   m /= segs;
-  const size_t smem = sizeof(float) * 2 * (size_t)c;
-  int gx = elem_blocks(m * (c / 8));
-  if (segs > 1 && gx > (148 * 16) / segs) gx = (148 * 16) / segs;
-  const dim3 grid(gx, segs);
-  if (dtype == TSP_DTYPE_BF16)
-    bn_apply_kernel<__nv_bfloat16><<<grid, kBlock, smem, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res,
-                                                                   (__nv_bfloat16*)y, sums, fixed_mean_var, w, b,
-                                                                   save_mean_rstd, acc_sum, acc_sumsq, acc_count,
-                                                                   acc_seg_stride, m, c, eps, relu);
-  else
-    bn_apply_kernel<float><<<grid, kBlock, smem, stream>>>((const float*)x, (const float*)res, (float*)y, sums,
-                                                           fixed_mean_var, w, b, save_mean_rstd, acc_sum, acc_sumsq,
-                                                           acc_count, acc_seg_stride, m, c, eps, relu);
+#define TSP_BN_APPLY(T, RES)                                                                                            \
+  bn_apply_kernel<T, RES><<<dim3(apply_blocks(m * (c / 8), c / 8, RES ? ApplyVecs<T>::fwd_res : ApplyVecs<T>::fwd, segs), \
+                                 segs), kBlock, 0, stream>>>(                                                            \
+      (const T*)x, (const T*)res, (T*)y, sums, fixed_mean_var, w, b, save_mean_rstd, acc_sum, acc_sumsq, acc_count,      \
+      acc_seg_stride, m, c, eps, relu)
+  if (dtype == TSP_DTYPE_BF16) { if (res) TSP_BN_APPLY(__nv_bfloat16, true); else TSP_BN_APPLY(__nv_bfloat16, false); }
+  else { if (res) TSP_BN_APPLY(float, true); else TSP_BN_APPLY(float, false); }
+#undef TSP_BN_APPLY
   return TSP_LAUNCH_CHECK();
 }
 
@@ -734,14 +717,13 @@ int tsp_bn_bwd_reduce(const void* dy, const void* x, const void* y, void* dres, 
   const int cpv = c / 8;
   const Tile tl = make_tile(cpv);
   const int slabs = (cpv + tl.tx_n - 1) / tl.tx_n;
-  dim3 grid(row_blocks(m, tl.ty_n, slabs), slabs, segs);
-  const size_t smem = sizeof(float) * 16 * (size_t)tl.tx_n * tl.ty_n;
+  const dim3 grid(row_blocks(m, tl.ty_n, (dtype == TSP_DTYPE_BF16 ? ColsumRows<__nv_bfloat16, 1>::value : ColsumRows<float, 1>::value), slabs, segs), slabs, segs);
   if (dtype == TSP_DTYPE_BF16)
-    bn_colsum_kernel<__nv_bfloat16, 1><<<grid, kBlock, smem, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy,
+    bn_colsum_kernel<__nv_bfloat16, 1><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy,
                                                                        (const __nv_bfloat16*)y, (__nv_bfloat16*)dres,
                                                                        mean_rstd, w, bias, relu, m, c, sums);
   else
-    bn_colsum_kernel<float, 1><<<grid, kBlock, smem, stream>>>((const float*)x, (const float*)dy, (const float*)y,
+    bn_colsum_kernel<float, 1><<<grid, kBlock, 0, stream>>>((const float*)x, (const float*)dy, (const float*)y,
                                                                (float*)dres, mean_rstd, w, bias, relu, m, c, sums);
   return TSP_LAUNCH_CHECK();
 }
@@ -752,21 +734,17 @@ int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* 
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 4096 || segs < 1 || m % segs != 0) return -3;
   m /= segs;
-  const size_t smem = sizeof(float) * 5 * (size_t)c;
-  if (smem > 48 * 1024) {      // opt in to more than the default dynamic shared memory
-    cudaFuncSetAttribute(bn_bwd_apply_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-    cudaFuncSetAttribute(bn_bwd_apply_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  }
-  int gx = elem_blocks(m * (c / 8));
-  if (segs > 1 && gx > (148 * 16) / segs) gx = (148 * 16) / segs;
-  const dim3 grid(gx, segs);
-  if (dtype == TSP_DTYPE_BF16)
-    bn_bwd_apply_kernel<__nv_bfloat16><<<grid, kBlock, smem, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
-                                                                       (const __nv_bfloat16*)y, mean_rstd, w, bias, relu,
-                                                                       sums, (__nv_bfloat16*)dx, m, c);
-  else
-    bn_bwd_apply_kernel<float><<<grid, kBlock, smem, stream>>>((const float*)dy, (const float*)x, (const float*)y,
-                                                               mean_rstd, w, bias, relu, sums, (float*)dx, m, c);
+  const int mask = y != nullptr ? 2 : (relu ? 1 : 0);
+#define TSP_BN_BWD(T, MASK)                                                                                             \
+  bn_bwd_apply_kernel<T, MASK>                                                                                          \
+      <<<dim3(apply_blocks(m * (c / 8), c / 8, ApplyVecs<T>::bwd, segs), segs), kBlock, 0, stream>>>(                   \
+          (const T*)dy, (const T*)x, (const T*)y, mean_rstd, w, bias, sums, (T*)dx, m, c)
+#define TSP_BN_BWD_MASK(T)                                                                                              \
+  do { if (mask == 2) TSP_BN_BWD(T, 2); else if (mask == 1) TSP_BN_BWD(T, 1); else TSP_BN_BWD(T, 0); } while (0)
+  if (dtype == TSP_DTYPE_BF16) TSP_BN_BWD_MASK(__nv_bfloat16);
+  else TSP_BN_BWD_MASK(float);
+#undef TSP_BN_BWD_MASK
+#undef TSP_BN_BWD
   return TSP_LAUNCH_CHECK();
 }
 

@@ -5,6 +5,7 @@ import math
 import pytest
 import torch
 import torch.nn.functional as F
+from torch import nn
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0)
@@ -71,6 +72,34 @@ def test_byol_pair_equals_two_single_losses(n, d, dtype):
     (g,) = torch.autograd.grad(fused.byol_loss(o1, o2, t1, t2), o1, torch.ones((), device=DEV, requires_grad=True),
                                create_graph=True)
     assert g.requires_grad and torch.equal(g.detach(), gs[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,c,res", [(16, 4096, False), (64, 4096, True), (37, 24, True), (515, 1000, False),
+                                     (4099, 64, True), (9, 2056, False)])
+def test_batchnorm_passes_at_odd_widths(m, c, res, dtype):
+    """Channel counts whose vectors do and do not divide a block, from one row per thread to several trips."""
+    from tspipe_b200.ops import bn as fbn
+    torch.manual_seed(5)
+    mod = nn.BatchNorm1d(c).to(DEV)
+    with torch.no_grad():
+        mod.weight.normal_(1, 0.2)
+        mod.bias.normal_(0.3, 0.2)
+    x = (torch.randn(m, c, device=DEV) + 0.5).to(dtype).requires_grad_()
+    r = torch.randn(m, c, device=DEV).to(dtype).requires_grad_() if res else None
+    g = torch.randn(m, c, device=DEV).to(dtype)
+    y = fbn.bn_act(mod, x, r, True)
+    got = torch.autograd.grad(y, [x, mod.weight, mod.bias] + ([r] if res else []), g)
+    x6, w6, b6 = x.detach().double().requires_grad_(), mod.weight.detach().double().requires_grad_(), \
+        mod.bias.detach().double().requires_grad_()
+    r6 = r.detach().double().requires_grad_() if res else None
+    z = F.batch_norm(x6, None, None, w6, b6, True)
+    z = z + r6 if res else z
+    assert _rel(y, F.relu(z)) < 2 * EPS[dtype] + 1e-6
+    z = z * (y.double() > 0)                           # the kernel's own mask: roundings at the corner are not at issue
+    want = torch.autograd.grad(z, [x6, w6, b6] + ([r6] if res else []), g.double())
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 4 * EPS[dtype] + 2e-5
 
 
 def test_loss_gradient_scaling_in_place_and_not():

@@ -432,7 +432,10 @@ class _Gelu(torch.autograd.Function):
             _check(lib().tsp_gelu_bwd(_ptr(dy), _ptr(x), _ptr(bf if ctx.has_bias else None), _ptr(dx),
                                       _c.c_int64(x.numel()), _c.c_int(d), _c.c_int(_dt(x)), _stream()), "tsp_gelu_bwd")
         _count()
-        db = dx.reshape(-1, d).sum(0).to(ctx.bdtype) if ctx.has_bias else None
+        db = None
+        if ctx.has_bias:
+            from .gemm import _column_sums
+            db = _column_sums(dx.reshape(-1, d)).to(ctx.bdtype)
         return dx, db
 
 

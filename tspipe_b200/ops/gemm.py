@@ -135,19 +135,18 @@ def _w16_t(weight: torch.Tensor) -> torch.Tensor:
     return hit[2]
 
 
-def _column_sums(dy2: torch.Tensor) -> torch.Tensor:
-    """fp32 column sums of a bf16 matrix (the bias gradient) on the streaming statistics kernel."""
+def _column_sums(dy2: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """fp32 column sums of a matrix (the bias gradient) on the column-sum kernel."""
     m, n = dy2.shape
-    if n % 8 or n > 4096 or m < 2:
-        return dy2.float().sum(0)
-    sums = torch.empty(2 * n, dtype=torch.float32, device=dy2.device)
+    sums = torch.empty(n, dtype=torch.float32, device=dy2.device) if out is None else out
+    if n % 8 or n > 8192 or m < 2:
+        return torch.sum(dy2, 0, dtype=torch.float32, out=sums)
     L = _f.lib()
-    L.tsp_bn_stats.restype = _c.c_int
     with _f.on_device(dy2.device):
-        _f._check(L.tsp_bn_stats(_f._ptr(dy2), _c.c_int64(m), _c.c_int(n), _c.c_int(_f._dt(dy2)), _f._ptr(sums),
-                                 _c.c_int(1), _f._stream()), "tsp_bn_stats")
-    _f._count(2)
-    return sums[:n]
+        _f._check(L.tsp_col_sums(_f._ptr(dy2), _c.c_int64(m), _c.c_int(n), _c.c_int(_f._dt(dy2)), _f._ptr(sums),
+                                 _f._stream()), "tsp_col_sums")
+    _f._count()
+    return sums
 
 
 # dX = dY @ W: on the CTA-pair GEMM against a cached transposed bf16 copy of W (True), or on the implicit-GEMM
