@@ -569,6 +569,261 @@ __global__ void __launch_bounds__(kBlock, 3) bn_bwd_apply_kernel(const T* __rest
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// BatchNorm + ReLU + 3x3 / stride 2 / pad 1 max-pool (the ResNet stem) without the normalised activation in memory.
+//
+// Forward: one pass reads x and writes the pooled rows and the winning tap (0..8) of every output, a byte; values are
+// rounded to T before they are compared and the first maximum in (row, column) order wins, so the result is that of
+// the two separate passes.  A thread walks kPoolRows output rows of one column and 4 channels and forms each input
+// row's maximum over the three columns once (an odd row is the last of one window and the first of the next); the next
+// row is on its way meanwhile.
+// Backward: dy' of an input pixel is gathered from the <= 4 windows it belongs to where it is needed, in the reduction
+// and again in the pass for dx, instead of being scattered to an activation-sized tensor that both would read.  A
+// thread takes a 2 x 2 block of input pixels, which meets exactly the four windows (a, b) .. (a + 1, b + 1).
+// Four channels per thread: the arithmetic (nine taps per block) needs more warps than eight would leave registers for.
+// 256 images of 112 x 112 x 64 bf16 (205 MB), B200: forward 178 us as two passes, 139 as one; backward 410 as three, 320 as two.
+// ---------------------------------------------------------------------------------------------
+constexpr int kPoolRows = 4;
+
+struct PoolGeom {
+  int n, h, w, c, ho, wo;      // images of one segment, extents
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_kernel(const T* __restrict__ x, T* __restrict__ y,
+                                                              uint8_t* __restrict__ idx, const float* __restrict__ sums,
+                                                              const float* __restrict__ wgt,
+                                                              const float* __restrict__ bias,
+                                                              float* __restrict__ save_mean_rstd,
+                                                              float* __restrict__ acc_sum, float* __restrict__ acc_sumsq,
+                                                              float* __restrict__ acc_count, int64_t acc_seg_stride,
+                                                              const PoolGeom g, float eps) {
+  {   // blockIdx.y = segment
+    const int64_t seg = blockIdx.y;
+    x += seg * g.n * g.h * g.w * g.c;
+    y += seg * g.n * g.ho * g.wo * g.c;
+    if (idx != nullptr) idx += seg * g.n * g.ho * g.wo * g.c;
+    sums += seg * 2 * g.c;
+    save_mean_rstd += seg * 2 * g.c;
+    if (acc_sum != nullptr) { acc_sum += seg * acc_seg_stride; acc_sumsq += seg * acc_seg_stride; }
+    if (acc_count != nullptr) acc_count += seg * acc_seg_stride;
+  }
+  const int c = g.c, cpv = c >> 2, strips = (g.ho + kPoolRows - 1) / kPoolRows;
+  const int64_t total = (int64_t)g.n * strips * g.wo * cpv;
+  const int64_t stride = (int64_t)gridDim.x * kBlock;
+  const int first = blockIdx.x * kBlock + threadIdx.x;
+  if (first >= total) return;
+  const int ch = (first % cpv) * 4;             // the grid stride is a multiple of c/4
+  float sc[4], sh[4];
+  {
+    const float rows = (float)((int64_t)g.n * g.h * g.w), inv_m = 1.f / rows;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float s = sums[ch + e], q = sums[c + ch + e];
+      const float mean = s * inv_m, rstd = rsqrtf(fmaxf(q * inv_m - mean * mean, 0.f) + eps);
+      if (first < cpv) {
+        if (acc_sum != nullptr) { acc_sum[ch + e] += s; acc_sumsq[ch + e] += q; }
+        if (acc_count != nullptr) acc_count[ch + e] += rows;
+        save_mean_rstd[ch + e] = mean;
+        save_mean_rstd[c + ch + e] = rstd;
+      }
+      sc[e] = wgt[ch + e] * rstd;
+      sh[e] = bias[ch + e] - mean * sc[e];
+    }
+  }
+  for (int64_t i = first; i < total; i += stride) {
+    uint32_t p = (uint32_t)(i / cpv);
+    const int ox = (int)(p % (uint32_t)g.wo);
+    p /= (uint32_t)g.wo;
+    const int oy0 = (int)(p % (uint32_t)strips) * kPoolRows;
+    const int img = (int)(p / (uint32_t)strips);
+    const int ix0 = 2 * ox - 1, iy0 = 2 * oy0 - 1;
+    const bool left = ix0 >= 0, right = ix0 + 2 < g.w;
+    const T* xi = x + (int64_t)img * g.h * g.w * c + ch;
+    const int64_t o0 = (((int64_t)img * g.ho + oy0) * g.wo + ox) * c + ch;
+    // input rows iy0 .. iy0 + 2 kPoolRows that exist and that a window of this strip needs
+    const int rows = min(g.h - iy0, 2 * min(kPoolRows, g.ho - oy0) + 1);
+    auto load = [&](int r, tsp::Raw4<T> (&raw)[3]) {
+      const T* row = xi + ((int64_t)(iy0 + r) * g.w + ix0) * c;
+      if (left) tsp::ldraw(row, 0, raw[0]);
+      tsp::ldraw(row, c, raw[1]);
+      if (right) tsp::ldraw(row, 2 * (int64_t)c, raw[2]);
+    };
+    tsp::Raw4<T> cur[3], nxt[3];
+    float best[4], m[4];                         // maximum of the current window and of the current row
+    uint32_t arg = 0, col = 0;                   // their taps and columns, a byte per channel
+#pragma unroll
+    for (int e = 0; e < 4; ++e) best[e] = -INFINITY;
+    if (iy0 >= 0) load(0, cur);
+    load(1, nxt);                                // (row 2 * oy0 always exists)
+#pragma unroll
+    for (int r = 0; r <= 2 * kPoolRows; ++r) {
+      if (r > 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cur[k] = nxt[k];
+        if (r + 1 < rows) load(r + 1, nxt);
+      }
+      const bool have = r < rows && (r > 0 || iy0 >= 0);
+      if (have) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) m[e] = -INFINITY;
+        col = 0;
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx)
+          if (kx == 1 || (kx == 0 ? left : right)) {
+            float v[4];
+            tsp::cvt4(cur[kx], v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = fmaxf(v[e] * sc[e] + sh[e], 0.f);
+            tsp::round_as<T>(v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (v[e] > m[e]) { m[e] = v[e]; col = (col & ~(0xffu << (8 * e))) | ((uint32_t)kx << (8 * e)); }
+          }
+        const uint32_t tap = r == 0 ? 0u : (r & 1) ? 3u : 6u;              // first tap of this row in the current window
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (m[e] > best[e]) {
+            best[e] = m[e];
+            arg = (arg & ~(0xffu << (8 * e))) | ((col & (0xffu << (8 * e))) + (tap << (8 * e)));
+          }
+      }
+      if (r > 0 && (r & 1) == 0 && r - 1 < rows) {                         // the window's last row (which may not exist)
+        const int64_t o = o0 + (int64_t)(r / 2 - 1) * g.wo * c;
+        tsp::st4(y, o, best);
+        if (idx != nullptr) *reinterpret_cast<uint32_t*>(idx + o) = arg;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) best[e] = m[e];                        // the odd row opens the next window
+        arg = col;
+      }
+    }
+  }
+}
+
+// APPLY false: sums[seg] += (sum dy', sum dy' * xhat).  APPLY true: dx from those sums.
+template <typename T, bool APPLY>
+__global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_bwd_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ idx,
+                                                                  const T* __restrict__ x,
+                                                                  const float* __restrict__ mean_rstd,
+                                                                  const float* __restrict__ wgt,
+                                                                  const float* __restrict__ bias,
+                                                                  float* __restrict__ sums, T* __restrict__ dx,
+                                                                  const PoolGeom g) {
+  constexpr int pitch = kBlock + 8;
+  __shared__ float sm[APPLY ? 1 : 8 * pitch];
+  const int c = g.c, cpv = c >> 2;
+  {   // blockIdx.y = segment
+    const int64_t seg = blockIdx.y, in = seg * g.n * g.h * g.w * c, outs = seg * g.n * g.ho * g.wo * c;
+    x += in;
+    if (APPLY) dx += in;
+    dy += outs;
+    idx += outs;
+    mean_rstd += seg * 2 * c;
+    sums += seg * 2 * c;
+  }
+  const int64_t total = (int64_t)g.n * g.ho * g.wo * cpv;
+  const int64_t stride = (int64_t)gridDim.x * kBlock;
+  const int first = blockIdx.x * kBlock + threadIdx.x;
+  const int ch = (first % cpv) * 4;
+  float A[4], B[4], D[4], sh[4];                // APPLY: dx = A g + B x + D; else xhat = (x - D) * B; mask: x * A + sh > 0
+  {
+    const float inv_m = 1.f / (float)((int64_t)g.n * g.h * g.w);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float mean = mean_rstd[ch + e], rs = mean_rstd[c + ch + e];
+      A[e] = wgt[ch + e] * rs;
+      sh[e] = bias[ch + e] - mean * A[e];
+      if constexpr (APPLY) {
+        B[e] = -A[e] * rs * (sums[c + ch + e] * inv_m);
+        D[e] = -A[e] * (sums[ch + e] * inv_m) - B[e] * mean;
+      } else {
+        B[e] = rs;
+        D[e] = mean;
+      }
+    }
+  }
+  float a[4], b[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) { a[e] = 0.f; b[e] = 0.f; }
+  for (int64_t i = first; i < total; i += stride) {
+    uint32_t p = (uint32_t)(i / cpv);
+    const int wb = (int)(p % (uint32_t)g.wo);
+    p /= (uint32_t)g.wo;
+    const int wa = (int)(p % (uint32_t)g.ho);
+    const int img = (int)(p / (uint32_t)g.ho);
+    const bool down = wa + 1 < g.ho, right = wb + 1 < g.wo;             // windows below and to the right
+    const bool row1 = 2 * wa + 1 < g.h, col1 = 2 * wb + 1 < g.w;        // second input row and column
+    const T* dyi = dy + (((int64_t)img * g.ho + wa) * g.wo + wb) * c + ch;
+    const uint8_t* ti = idx + (((int64_t)img * g.ho + wa) * g.wo + wb) * c + ch;
+    const int64_t q = (((int64_t)img * g.h + 2 * wa) * g.w + 2 * wb) * c + ch;
+    tsp::Raw4<T> gr[4], xr[4];
+    uint32_t tap[4];
+    const bool have[4] = {true, right, down, down && right};
+    const bool pix[4] = {true, col1, row1, row1 && col1};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int oo = ((k >> 1) * g.wo + (k & 1)) * c;
+      tap[k] = 0xffffffffu;                                             // no tap: a window that does not exist wins nothing
+      if (have[k]) {
+        tsp::ldraw(dyi, oo, gr[k]);
+        tap[k] = *reinterpret_cast<const uint32_t*>(ti + oo);
+      }
+      if (pix[k]) tsp::ldraw(x + q, ((k >> 1) * g.w + (k & 1)) * c, xr[k]);
+    }
+    float gv[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (have[k]) tsp::cvt4(gr[k], gv[k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (!pix[k]) continue;
+      const int dr = k >> 1, dc = k & 1;                                // pixel (2 wa + dr, 2 wb + dc)
+      float d[4], xv[4];
+      tsp::cvt4(xr[k], xv);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d[e] = 0.f;
+#pragma unroll
+      for (int kw = 0; kw < 4; ++kw) {                                  // window (wa + kw / 2, wb + kw % 2)
+        const int ky = dr + 1 - 2 * (kw >> 1), kx = dc + 1 - 2 * (kw & 1);
+        if (ky < 0 || kx < 0) continue;
+        const uint32_t want = (uint32_t)(ky * 3 + kx);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (((tap[kw] >> (8 * e)) & 0xffu) == want) d[e] += gv[kw][e];
+      }
+      tsp::round_as<T>(d);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) d[e] = (xv[e] * A[e] + sh[e]) > 0.f ? d[e] : 0.f;
+      if constexpr (APPLY) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[e] = A[e] * d[e] + B[e] * xv[e] + D[e];
+        tsp::st4(dx + q, (dr * g.w + dc) * c, d);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { a[e] += d[e]; b[e] += d[e] * (xv[e] - D[e]) * B[e]; }
+      }
+    }
+  }
+  if constexpr (!APPLY) {
+    // threads that are cpv apart hold the same channels when cpv divides the block (one addition per channel and block,
+    // lane = channel, as in bn_colsum_kernel), else every thread adds its own
+    if (kBlock % cpv == 0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { sm[e * pitch + threadIdx.x] = a[e]; sm[(4 + e) * pitch + threadIdx.x] = b[e]; }
+      __syncthreads();
+      for (int p = threadIdx.x; p < 2 * c; p += kBlock) {
+        const int half = p >= c ? 1 : 0, cc = p - half * c;
+        float acc = 0.f;
+        for (int k = cc >> 2; k < kBlock; k += cpv) acc += sm[(half * 4 + (cc & 3)) * pitch + k];
+        atomicAdd(sums + p, acc);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { atomicAdd(sums + ch + e, a[e]); atomicAdd(sums + c + ch + e, b[e]); }
+    }
+  }
+}
+
 // Row blocks of bn_colsum_kernel: enough to fill the chip four times over all slabs and segments, but at least one trip of
 // `rows` rows per thread.
 inline int row_blocks(int64_t m, int ty_n, int rows, int slabs, int segs) {
@@ -745,6 +1000,60 @@ int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* 
   else TSP_BN_BWD_MASK(float);
 #undef TSP_BN_BWD_MASK
 #undef TSP_BN_BWD
+  return TSP_LAUNCH_CHECK();
+}
+
+// Training-mode BatchNorm + ReLU + 3x3 / 2 / 1 max-pool of x [segs * n, h, w, c] (statistics per group of n images, from
+// `sums` [segs][2c] = sum and sum of squares over a group's pixels) -> y [segs * n, ho, wo, c], ho = (h + 1) / 2; idx
+// (optional, same shape as y) receives the winning taps for the backward.  The other arguments as in tsp_bn_apply.
+static int pool_geom(int n, int h, int w, int c, int segs, PoolGeom* g) {
+  if (n <= 0 || h < 1 || w < 1 || c % 8 != 0 || c > 4096 || segs < 1) return -3;
+  *g = {n, h, w, c, (h + 1) / 2, (w + 1) / 2};
+  return (int64_t)n * g->ho * g->wo < 0x7fffffff ? 0 : -3;
+}
+
+int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums, const float* w, const float* b,
+                         float* save_mean_rstd, float* acc_sum, float* acc_sumsq, float* acc_count, int64_t acc_seg_stride,
+                         int n, int h, int wd, int c, float eps, int dtype, int segs, cudaStream_t stream) {
+  PoolGeom g;
+  const int rc = pool_geom(n, h, wd, c, segs, &g);
+  if (rc != 0) return rc;
+  const int64_t work = (int64_t)n * ((g.ho + kPoolRows - 1) / kPoolRows) * g.wo * (c / 4);
+  const dim3 grid(tsp::row_stride_blocks(work, c / 4, kBlock, 1, 1, 148 * 32 / segs), segs);
+  if (dtype == TSP_DTYPE_BF16)
+    bn_relu_pool_kernel<__nv_bfloat16><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, idx, sums, w,
+                                                                    b, save_mean_rstd, acc_sum, acc_sumsq, acc_count,
+                                                                    acc_seg_stride, g, eps);
+  else
+    bn_relu_pool_kernel<float><<<grid, kBlock, 0, stream>>>((const float*)x, (float*)y, idx, sums, w, b, save_mean_rstd,
+                                                            acc_sum, acc_sumsq, acc_count, acc_seg_stride, g, eps);
+  return TSP_LAUNCH_CHECK();
+}
+
+// Its backward: dy [segs * n, ho, wo, c], idx and x as above -> dx; sums [segs][2c] is zeroed and receives db and dw.
+int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* x, const float* mean_rstd, const float* w,
+                         const float* b, float* sums, void* dx, int n, int h, int wd, int c, int dtype, int segs,
+                         cudaStream_t stream) {
+  PoolGeom g;
+  const int rc = pool_geom(n, h, wd, c, segs, &g);
+  if (rc != 0) return rc;
+  cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(float) * 2 * (size_t)c * segs, stream);
+  if (e != cudaSuccess) return (int)e;
+  const int64_t work = (int64_t)n * g.ho * g.wo * (c / 4);
+  const dim3 grid_r(tsp::row_stride_blocks(work, c / 4, kBlock, 8, 148 * 2 / segs, 148 * 3 / segs), segs);
+  const dim3 grid_a(tsp::row_stride_blocks(work, c / 4, kBlock, 1, 1, 148 * 32 / segs), segs);
+  if (dtype == TSP_DTYPE_BF16) {
+    using B = __nv_bfloat16;
+    bn_relu_pool_bwd_kernel<B, false><<<grid_r, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, b, sums,
+                                                                     nullptr, g);
+    bn_relu_pool_bwd_kernel<B, true><<<grid_a, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, b, sums,
+                                                                    (B*)dx, g);
+  } else {
+    bn_relu_pool_bwd_kernel<float, false><<<grid_r, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd,
+                                                                         w, b, sums, nullptr, g);
+    bn_relu_pool_bwd_kernel<float, true><<<grid_a, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd, w,
+                                                                        b, sums, (float*)dx, g);
+  }
   return TSP_LAUNCH_CHECK();
 }
 

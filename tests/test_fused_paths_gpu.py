@@ -102,6 +102,50 @@ def test_batchnorm_passes_at_odd_widths(m, c, res, dtype):
         assert _rel(a, b) < 4 * EPS[dtype] + 2e-5
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape,views", [((2, 64, 8, 8), 2), ((3, 8, 5, 7), 1), ((4, 24, 9, 2), 2), ((2, 64, 30, 16), 1),
+                                         ((1, 512, 2, 3), 1)])
+def test_batchnorm_relu_maxpool_equals_the_separate_passes(shape, views, dtype):
+    """Odd extents (last window of two rows or columns), strips that end early, channel counts off the block size."""
+    from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
+    from tspipe_b200.ops import bn as fbn
+    from tspipe_b200.ops.pool import MaxPool3x3s2
+    torch.manual_seed(8)
+    x = _cl(*shape, dtype=dtype).requires_grad_()
+    outs = []
+    for fused in (True, False):
+        mod = DeferredBatchNorm(shape[1]).to(DEV)
+        with torch.no_grad():
+            mod.weight.copy_(torch.linspace(-1, 2, shape[1]))
+            mod.bias.copy_(torch.linspace(0.5, -0.5, shape[1]))
+        group = BatchNormGroup(mod, chunks=10)
+        with fbn.segments(views):
+            y = fbn.bn_relu_pool(mod, x) if fused else MaxPool3x3s2()(fbn.bn_act(mod, x, None, True))
+        assert y is not None
+        torch.manual_seed(9)
+        g = _cl(*y.shape, dtype=dtype)
+        outs.append([y.detach(), *torch.autograd.grad(y, [x, mod.weight, mod.bias], g), group._acc])
+    for a, b in zip(outs[0], outs[1]):                 # same roundings, sums in another order
+        assert _rel(a, b) < EPS[dtype] + 1e-5
+
+
+# ---- tensor-core products -----------------------------------------------------------------------------------------
+@pytest.mark.parametrize("m,n,k", [(128, 64, 64), (300, 192, 128), (12608, 768, 64), (257, 4096, 192), (5000, 1024, 64)])
+def test_linear_products_at_every_tile_width(m, n, k):
+    """The widths that ``pick_bn`` chooses between: full and ragged last tiles in every direction, k tails in the weight
+    gradient (rows that are no multiple of 64)."""
+    from tspipe_b200.ops import gemm
+    torch.manual_seed(10)
+    x, w, dy = torch.randn(m, k, device=DEV).bfloat16(), torch.randn(n, k, device=DEV).bfloat16(), \
+        torch.randn(m, n, device=DEV).bfloat16()
+    assert _rel(gemm.matmul_nt(x, w), x.double() @ w.double().t()) < EPS[torch.bfloat16]
+    assert _rel(gemm.matmul_nn([dy], w), dy.double() @ w.double()) < EPS[torch.bfloat16]
+    dw = torch.ones(n, k, device=DEV)
+    gemm._add_weight_grad(dw, [dy], x)
+    gemm.check_status()
+    assert _rel(dw - 1, dy.double().t() @ x.double()) < 1e-5
+
+
 def test_loss_gradient_scaling_in_place_and_not():
     """A retained graph gives the same gradient again, with any factor; a freed one takes the buffer over."""
     from tspipe_b200.ops import fused

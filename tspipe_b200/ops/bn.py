@@ -86,7 +86,8 @@ def applicable(bn, x: torch.Tensor) -> bool:
 def _lib():
     L = _f.lib()
     if not hasattr(L, "_bn_ready"):
-        for n in ("tsp_bn_stats", "tsp_bn_apply", "tsp_bn_bwd_reduce", "tsp_bn_bwd_apply"):
+        for n in ("tsp_bn_stats", "tsp_bn_apply", "tsp_bn_bwd_reduce", "tsp_bn_bwd_apply", "tsp_bn_relu_pool_fwd",
+                  "tsp_bn_relu_pool_bwd"):
             getattr(L, n).restype = _c.c_int
         L._bn_ready = True
     return L
@@ -236,3 +237,71 @@ def bn_act(bn, x: torch.Tensor, residual: Optional[torch.Tensor] = None, relu: b
             bn.running_mean.mul_(1 - mom).add_(mean.to(bn.running_mean.dtype), alpha=mom)
             bn.running_var.mul_(1 - mom).add_(var.to(bn.running_var.dtype), alpha=mom)
     return y
+
+
+class _BnReluPool(torch.autograd.Function):
+    """``max_pool2d(relu(bn(x)), 3, stride 2, padding 1)`` in training mode; see ``bn_relu_pool_kernel``."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, eps, acc_sum, acc_sumsq, acc_count, sums, segs, acc_stride):
+        n, c, h, w = x.shape
+        L = _lib()
+        dt = _f._dt(x)
+        y = torch.empty((n, c, (h + 1) // 2, (w + 1) // 2), dtype=x.dtype, device=x.device,
+                        memory_format=torch.channels_last)
+        idx = torch.empty(y.numel(), dtype=torch.uint8, device=x.device) if any(ctx.needs_input_grad[:3]) else None
+        save = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
+        wf = weight.detach() if weight.dtype == torch.float32 else weight.detach().float()
+        bf = bias.detach() if bias.dtype == torch.float32 else bias.detach().float()
+        with _f.on_device(x.device):
+            st = _f._stream()
+            if sums is None:
+                sums = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
+                _f._check(L.tsp_bn_stats(_f._ptr(x), _c.c_int64(n * h * w), _c.c_int(c), _c.c_int(dt), _f._ptr(sums),
+                                         _c.c_int(segs), st), "tsp_bn_stats")
+                _f._count(2)
+            _f._check(L.tsp_bn_relu_pool_fwd(_f._ptr(x), _f._ptr(y), _f._ptr(idx), _f._ptr(sums), _f._ptr(wf), _f._ptr(bf),
+                                             _f._ptr(save), _f._ptr(acc_sum), _f._ptr(acc_sumsq), _f._ptr(acc_count),
+                                             _c.c_int64(acc_stride), _c.c_int(n // segs), _c.c_int(h), _c.c_int(w),
+                                             _c.c_int(c), _c.c_float(eps), _c.c_int(dt), _c.c_int(segs), st),
+                      "tsp_bn_relu_pool_fwd")
+            _f._count()
+        ctx.save_for_backward(x, idx, save, wf, bf)
+        ctx.segs, ctx.wdtype, ctx.bdtype = segs, weight.dtype, bias.dtype
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, idx, save, wf, bf = ctx.saved_tensors
+        n, c, h, w = x.shape
+        segs = ctx.segs
+        ho, wo = (h + 1) // 2, (w + 1) // 2
+        if dy.dtype != x.dtype or dy.stride() != (ho * wo * c, 1, wo * c, c) or dy.data_ptr() % 16:
+            dy = dy.to(x.dtype).clone(memory_format=torch.channels_last)
+        dx = torch.empty_like(x)
+        sums = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
+        with _f.on_device(x.device):
+            _f._check(_lib().tsp_bn_relu_pool_bwd(_f._ptr(dy), _f._ptr(idx), _f._ptr(x), _f._ptr(save), _f._ptr(wf),
+                                                  _f._ptr(bf), _f._ptr(sums), _f._ptr(dx), _c.c_int(n // segs),
+                                                  _c.c_int(h), _c.c_int(w), _c.c_int(c), _c.c_int(_f._dt(x)),
+                                                  _c.c_int(segs), _f._stream()), "tsp_bn_relu_pool_bwd")
+        _f._count(3)
+        if segs > 1:
+            sums = sums.view(segs, 2 * c).sum(0)
+        return dx, sums[c:].to(ctx.wdtype), sums[:c].to(ctx.bdtype), None, None, None, None, None, None, None
+
+
+def bn_relu_pool(bn, x: torch.Tensor, sums: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """``max_pool2d(relu(bn(x)), 3, 2, 1)`` with the statistics semantics of ``bn``, without the normalised activation in
+    memory; None where the fused passes do not apply (anything but a training-mode layer of a
+    :class:`~tspipe_b200.batchnorm.BatchNormGroup` on a channels-last activation)."""
+    from ..batchnorm import DeferredBatchNorm
+    if not (isinstance(bn, DeferredBatchNorm) and bn.group is not None and bn.training and applicable(bn, x)
+            and x.dim() == 4 and x.shape[2] > 1 and x.data_ptr() % 16 == 0 and x.shape[2] * x.shape[3] > 1):
+        return None
+    n, c, h, w = x.shape
+    segs = _SEGMENTS
+    if x.stride() != (h * w * c, 1, w * c, c) or n % segs or segs > bn.group.max_segments \
+            or n * (h + 1) * (w + 1) >= 1 << 31 or (segs > 1 and not applicable(bn, x[: n // segs])):
+        return None
+    return _BnReluPool.apply(x, bn.weight, bn.bias, bn.eps, bn.sum, bn.sum_squares, bn.count, sums, segs, bn.group.total)

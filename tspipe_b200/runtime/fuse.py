@@ -8,6 +8,8 @@ children in order but lets neighbouring ones share a kernel:
 * ``BatchNorm -> ReLU``                      one fused normalise + activation pass (``ops.bn.bn_act``);
 * ``Conv2d(3, 64, 7, stride 2) -> BatchNorm`` the tcgen05 stem convolution, whose epilogue already produces the
   BatchNorm statistics (``ops.conv.stem_conv``), so the statistics pass over the activation disappears;
+* that stem convolution's ``BatchNorm -> ReLU -> MaxPool 3x3/2``  one pass forward, two backward
+  (``ops.bn.bn_relu_pool``): the normalised activation is never written;
 * ``Linear`` children (the MLP heads)        the tcgen05 GEMM path of ``ops.linear.linear``, forward and backward.
 
 The reference runs these layers one library call at a time
@@ -22,6 +24,10 @@ from torch import nn
 from torch.nn.modules.batchnorm import _BatchNorm
 
 
+def _has_hooks(m: nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
 class FusedSequential(nn.Sequential):
     """Same children, same parameters and state-dict keys as the ``nn.Sequential`` it replaces."""
 
@@ -29,6 +35,7 @@ class FusedSequential(nn.Sequential):
         from ..ops import bn as _bn
         from ..ops import conv as _conv
         from ..ops import linear as _linear
+        from ..ops.pool import MaxPool3x3s2
         mods: List[nn.Module] = list(self._modules.values())
         i, n = 0, len(mods)
         while i < n:
@@ -41,6 +48,11 @@ class FusedSequential(nn.Sequential):
                 y, sums = _conv.stem_conv(x, m.weight, want_sums=bn_next, segments=segs)
                 if bn_next and _bn.applicable(nxt, y):
                     relu = i + 2 < n and isinstance(mods[i + 2], nn.ReLU)
+                    if relu and i + 3 < n and type(mods[i + 3]) is MaxPool3x3s2 and not _has_hooks(mods[i + 3]):
+                        z = _bn.bn_relu_pool(nxt, y, sums=sums)
+                        if z is not None:
+                            x, i = z, i + 4
+                            continue
                     x = _bn.bn_act(nxt, y, relu=relu, sums=sums)
                     i += 3 if relu else 2
                 else:
