@@ -103,6 +103,43 @@ def test_batchnorm_passes_at_odd_widths(m, c, res, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gelu_special_values_and_wide_bias(dtype):
+    from tspipe_b200.ops import fused
+    x = torch.tensor([math.inf, -1e30, 0.0, -0.0, 40.0, -40.0, math.nan, 1.0], device=DEV).to(dtype)
+    y = fused.gelu(x).float()
+    assert y[0] == math.inf and y[1] == 0 and y[2] == 0 and y[4] == 40 and y[5] == 0 and y[6].isnan()
+    torch.manual_seed(6)
+    for rows, d in ((3, 8), (5, 24), (300, 5120)):
+        v = (torch.randn(rows, d, device=DEV) * 3).to(dtype).requires_grad_()
+        b = torch.randn(d, device=DEV, requires_grad=True)
+        out = fused.gelu(v, b)
+        g = torch.randn_like(out)
+        gv, gb = torch.autograd.grad(out, [v, b], g)
+        v6, b6 = v.detach().double().requires_grad_(), b.detach().double().requires_grad_()
+        ref = F.gelu(v6 + b6)
+        rv, rb = torch.autograd.grad(ref, [v6, b6], g.double())
+        for a, w in ((out, ref), (gv, rv), (gb, rb)):
+            assert _rel(a, w) < 2 * EPS[dtype] + 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d", [(1, 8), (17, 256), (16, 264), (4800, 520), (33, 776), (5000, 1024)])
+def test_layer_norm_widths(rows, d, dtype):
+    from tspipe_b200.ops import fused
+    torch.manual_seed(7)
+    x = (torch.randn(rows, d, device=DEV) + 1).to(dtype).requires_grad_()
+    w, b = torch.randn(d, device=DEV, requires_grad=True), torch.randn(d, device=DEV, requires_grad=True)
+    y = fused.layer_norm(x, w, b, 1e-6)
+    g = torch.randn_like(y)
+    got = torch.autograd.grad(y, [x, w, b], g)
+    leaves = [t.detach().double().requires_grad_() for t in (x, w, b)]
+    ref = F.layer_norm(leaves[0], (d,), leaves[1], leaves[2], 1e-6)
+    assert _rel(y, ref) < EPS[dtype] + 1e-6
+    for a, r in zip(got, torch.autograd.grad(ref, leaves, g.double())):
+        assert _rel(a, r) < 2 * EPS[dtype] + 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape,views", [((2, 64, 8, 8), 2), ((3, 8, 5, 7), 1), ((4, 24, 9, 2), 2), ((2, 64, 30, 16), 1),
                                          ((1, 512, 2, 3), 1)])
 def test_batchnorm_relu_maxpool_equals_the_separate_passes(shape, views, dtype):
