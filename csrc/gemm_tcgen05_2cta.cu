@@ -1,6 +1,7 @@
-// bf16 GEMM with two SMs per output tile: C[M,N] = A[M,K] * B[N,K]^T, fp32 accumulation, 256 x 256 tiles.
+// bf16 GEMM with two SMs per output tile: C[M,N] = A[M,K] * B[N,K]^T, fp32 accumulation, 256 x BN tiles (BN = 256, 128
+// or 64, see pick_bn).
 //
-// A cluster of two CTAs owns one 256 x 256 tile.  CTA r of the pair loads rows [128 r, 128 r + 128) of the A tile and
+// A cluster of two CTAs owns one 256 x BN tile (figures for BN = 256).  CTA r of the pair loads rows [128 r, 128 r + 128) of the A tile and
 // rows [128 r, 128 r + 128) of the B tile (half of N) with its own TMA loads; the leader CTA (rank 0) issues
 // tcgen05.mma.cta_group::2, which reads A from both CTAs' shared memory and the two halves of B, and writes each
 // CTA's 128 x 256 accumulator slice into that CTA's tensor memory.  Compared with the one-CTA kernel
@@ -28,21 +29,23 @@ extern int g_tsp_sm_reserve;          // defined in peer.cu
 namespace {
 
 constexpr int BM = 128;          // rows per CTA (pair tile: 256)
-constexpr int BN = 256;          // tile columns; each CTA stages BN / 2 rows of B
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int kStages = 6;
 constexpr int kThreads = 192;
 constexpr uint64_t kWaitNs = 2000000000ull;   // every mbarrier wait gives up after two seconds
 constexpr int kGroup = 2;                       // stages released per tcgen05.commit
-constexpr int kGroups = kStages / kGroup;
 constexpr int kABytes = BM * BK * 2;
-constexpr int kBBytes = (BN / 2) * BK * 2;
-constexpr int kStageBytes = kABytes + kBBytes;                  // per CTA
-constexpr int kTmemCols = 2 * BN;                               // two accumulator buffers
 constexpr int kStoreBufBytes = 32 * 128;                        // 32 rows x 128 bytes of C, one TMA store
 constexpr int kStoreBytes = 4 * 2 * kStoreBufBytes;             // two buffers per epilogue warp
-constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256;
+// BN = tile columns (256, 128 or 64); each CTA stages BN / 2 rows of B
+template <int BN> struct Cfg {
+  static constexpr int kStages = BN == 256 ? 6 : 8;
+  static constexpr int kGroups = kStages / kGroup;
+  static constexpr int kBBytes = (BN / 2) * BK * 2;
+  static constexpr int kStageBytes = kABytes + kBBytes;         // per CTA
+  static constexpr int kTmemCols = 2 * BN;                      // two accumulator buffers
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256;
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -79,9 +82,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       : "memory");
 }
 
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
 // one commit that arrives on the barrier at the same shared-memory offset in BOTH CTAs of the pair (a commit costs
 // the issuing thread about as much as eight MMA issues, so the pair is signalled with one instruction, not two)
 __device__ __forceinline__ void umma_commit_pair_both(uint32_t local_bar_addr) {
@@ -122,6 +122,13 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void*
                : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+// The same block added element by element to what is in memory (fp32), in L2.
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const void* smem_src, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&t);
@@ -129,12 +136,33 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 
 __device__ __forceinline__ float gelu_erf(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
 
-template <typename OutT, bool STATS>
+// The three products of a linear layer.  An operand whose contraction index is the slow one in memory is staged as boxes
+// of 64 contraction rows x 64 columns and read by the tensor core as an MN-major tile: no transposed copy exists anywhere.
+enum Kind {
+  kTN = 0,      // C = A[m, k] B[n, k]^T      forward
+  kNN = 1,      // C = A[m, k] B[k, n]        gradient of the input; A may be up to three matrices side by side along k
+  kRed = 2      // C += A[k, m]^T B[k, n]     gradient of the weight: fp32, split along k, added in L2 by the TMA unit; A may
+                //                            be up to three matrices side by side along m
+};
+constexpr int kMaxASrc = 3;
+struct AMaps {
+  CUtensorMap m[kMaxASrc];
+};
+// Where the columns of C go: with kTN up to three matrices of n_per columns side by side (a fused projection whose
+// blocks are wanted apart), n_per a multiple of 64.
+constexpr int kMaxCDst = 3;
+struct CMaps {
+  CUtensorMap m[kMaxCDst];
+};
+
+template <typename OutT, bool STATS, int BN, int KIND>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                         const __grid_constant__ CUtensorMap tmap_c, int tma_store, OutT* __restrict__ c,
-                         const float* __restrict__ bias, int m, int n, int k, int ldc, int epi,
+gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const __grid_constant__ CUtensorMap tmap_b,
+                         const __grid_constant__ CMaps tmap_c, int n_per, int tma_store, OutT* __restrict__ c,
+                         const float* __restrict__ bias, int m, int n, int k, int ldc, int epi, int splits,
                          float* __restrict__ col_sums, int seg_rows, int* __restrict__ status) {
+  using C = Cfg<BN>;
+  constexpr int kStages = C::kStages, kGroups = C::kGroups, kStageBytes = C::kStageBytes, kTmemCols = C::kTmemCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* store_bufs = tiles + kStages * kStageBytes; // 1024-aligned: the swizzle pattern follows address bits
@@ -152,6 +180,18 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   const int tiles_m = (m + 2 * BM - 1) / (2 * BM), tiles_n = (n + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
   const int num_kb = (k + BK - 1) / BK;
+  // work items: tiles, and with kRed each tile in `splits` pieces of the contraction (item = piece * num_tiles + tile)
+  const int num_items = num_tiles * (KIND == kRed ? splits : 1);
+  auto item_range = [&](int t, int& tile, int& kb_lo, int& kb_hi) {
+    if constexpr (KIND == kRed) {
+      const int sp = t / num_tiles;
+      tile = t - sp * num_tiles;
+      kb_lo = (int)((int64_t)num_kb * sp / splits);
+      kb_hi = (int)((int64_t)num_kb * (sp + 1) / splits);
+    } else {
+      tile = t; kb_lo = 0; kb_hi = num_kb;
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -163,7 +203,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       mbar_init(tmem_empty_bar + a, 8);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a.m[0]) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
   }
   if (warp == 1) {        // warp 1 of BOTH CTAs: paired allocation of both accumulator buffers
@@ -183,12 +223,14 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (int t = pair; t < num_tiles && ok; t += num_pairs) {
+      for (int t = pair; t < num_items && ok; t += num_pairs) {
         // N tiles fastest: the pairs that run together share rows of A (read from DRAM once, then from L2) and sweep
         // the weights, which stay in L2; walking all of M per N tile would stream A from DRAM once per N tile
-        const int m0 = (t / tiles_n) * 2 * BM + (int)rank * BM;
-        const int n0 = (t % tiles_n) * BN + (int)rank * (BN / 2);
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        int tile, kb_lo, kb_hi;
+        item_range(t, tile, kb_lo, kb_hi);
+        const int m0 = (tile / tiles_n) * 2 * BM + (int)rank * BM;
+        const int n0 = (tile % tiles_n) * BN + (int)rank * (BN / 2);
+        for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
           const int s = it % kStages;
           if (it % kGroup == 0) {                 // first stage of a group: the whole group must have been released
             const uint32_t grp = (it / kGroup) % kGroups, round = (it / kGroup) / kGroups;
@@ -198,19 +240,39 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           uint8_t* b_dst = a_dst + kABytes;
           if (leader) mbar_expect_tx(full_bar + s, 2u * (uint32_t)kStageBytes);
           const uint32_t lbar = map_to_cta(smem_u32(full_bar + s), 0);
-          tma_load_2d_pair(a_dst, &tmap_a, lbar, kb * BK, m0);
-          tma_load_2d_pair(b_dst, &tmap_b, lbar, kb * BK, n0);
+          if constexpr (KIND == kRed) {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j) {        // a_per: columns per source; past the last one reads as zeros
+              const int col = m0 + j * 64, src = min(col / a_per, (m - 1) / a_per);
+              tma_load_2d_pair(a_dst + j * 8192, &tmap_a.m[src], lbar, col - src * a_per, kb * BK);
+            }
+          } else if constexpr (KIND == kNN) {
+            const int src = kb / a_per;                // k blocks per source
+            tma_load_2d_pair(a_dst, &tmap_a.m[src], lbar, (kb - src * a_per) * BK, m0);
+          } else {
+            tma_load_2d_pair(a_dst, &tmap_a.m[0], lbar, kb * BK, m0);
+          }
+          if constexpr (KIND == kTN) {
+            tma_load_2d_pair(b_dst, &tmap_b, lbar, kb * BK, n0);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(b_dst + j * 8192, &tmap_b, lbar, n0 + j * 64, kb * BK);
+          }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
     if (lane == 0 && leader) {
-      constexpr uint32_t idesc = make_idesc(2 * BM, BN);
+      static_assert(KIND == kTN || BN % 128 == 0, "an MN-major half tile of B is whole 64-column boxes");
+      constexpr bool kAmn = KIND == kRed, kBmn = KIND != kTN;
+      constexpr uint32_t idesc = tc5::make_idesc(2 * BM, BN, kAmn, kBmn);
       const uint32_t tiles_addr = smem_u32(tiles);
       uint32_t it = 0, lt = 0;
       bool ok = true;
-      for (int t = pair; t < num_tiles && ok; t += num_pairs, ++lt) {
+      for (int t = pair; t < num_items && ok; t += num_pairs, ++lt) {
+        int tile, kb_lo, kb_hi;
+        item_range(t, tile, kb_lo, kb_hi);
         const uint32_t acc = lt & 1, use = lt >> 1;
         if (use > 0) {
           ok = tc5::mbar_wait(tmem_empty_bar + acc, (use - 1) & 1, status, 4, kWaitNs);
@@ -219,17 +281,18 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         }
         const uint32_t d_tmem = tmem_base + acc * BN;
         uint32_t accum = 0u;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t round = it / kStages;
           ok = tc5::mbar_wait(full_bar + s, round & 1, status, 2, kWaitNs);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_addr = tiles_addr + s * kStageBytes;
-          const uint32_t a_lo = tc5::desc_lo_k_major(a_addr), b_lo = tc5::desc_lo_k_major(a_addr + kABytes);
+          const uint32_t a_lo = kAmn ? tc5::desc_lo_mn_major(a_addr, 8192) : tc5::desc_lo_k_major(a_addr);
+          const uint32_t b_lo = kBmn ? tc5::desc_lo_mn_major(a_addr + kABytes, 8192) : tc5::desc_lo_k_major(a_addr + kABytes);
 #pragma unroll
-          for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            umma_bf16_pair_lo(d_tmem, a_lo + 2 * kk, b_lo + 2 * kk, idesc, accum);
+          for (int kk = 0; kk < BK / UMMA_K; ++kk) {  // 16 along K: +32 bytes in a K-major row, +2048 bytes (16 rows) MN-major
+            umma_bf16_pair_lo(d_tmem, a_lo + (kAmn ? 128 : 2) * kk, b_lo + (kBmn ? 128 : 2) * kk, idesc, accum);
             accum = 1u;
           }
           // the group's slots are free again in both CTAs once these MMAs have read them
@@ -268,8 +331,10 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         }
       }
     };
-    for (int t = pair; t < num_tiles && ok; t += num_pairs, ++lt) {
-      const int m0 = (t / tiles_n) * 2 * BM + (int)rank * BM, n0 = (t % tiles_n) * BN;
+    for (int t = pair; t < num_items && ok; t += num_pairs, ++lt) {
+      int tile, kb_lo, kb_hi;
+      item_range(t, tile, kb_lo, kb_hi);
+      const int m0 = (tile / tiles_n) * 2 * BM + (int)rank * BM, n0 = (tile % tiles_n) * BN;
       const uint32_t acc = lt & 1, use = lt >> 1;
       if (STATS) {
         const int seg = m0 / seg_rows;
@@ -338,8 +403,11 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) {
-            if (row0 < m && col < n) tma_store_2d(&tmap_c, buf, col, row0);
-            else asm volatile("cp.async.bulk.commit_group;" ::: "memory");     // keep the group count in step
+            if (row0 < m && col < n) {
+              const int dst = KIND == kTN ? col / n_per : 0;
+              if constexpr (KIND == kRed) tma_reduce_add_2d(&tmap_c.m[0], buf, col, row0);
+              else tma_store_2d(&tmap_c.m[dst], buf, col - dst * n_per, row0);
+            } else asm volatile("cp.async.bulk.commit_group;" ::: "memory");     // keep the group count in step
           }
           ++nstore;
           if (STATS && st != nullptr) {
@@ -362,7 +430,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         return true;
       };
       if constexpr (STATS) {
-        static_assert(!STATS || kCols == 64, "column statistics are kept for bf16 outputs");
+        static_assert(!STATS || (kCols == 64 && BN == 256), "column statistics are kept for bf16 outputs and the widest tile");
         if (chunk(0, cs[0]) && chunk(64, cs[1]) && chunk(128, cs[2])) chunk(192, cs[3]);
       } else {
 #pragma unroll 1
@@ -432,32 +500,81 @@ bool make_store_map(CUtensorMap* map, void* ptr, int rows, int cols, int ld, boo
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename OutT, bool STATS>
-int launch(const void* a, const void* b, void* c, const float* bias, int m, int n, int k, int lda, int ldb, int ldc,
-           int epi, float* col_sums, int seg_rows, int* status, cudaStream_t stream) {
-  CUtensorMap ta, tb;
-  if (!make_map(&ta, a, m, k, lda, BM) || !make_map(&tb, b, n, k, ldb, BN / 2)) return -6;
-  CUtensorMap tc = ta;          // placeholder when C cannot be described (the kernel then stores directly)
-  const bool aligned_c = (((uintptr_t)c & 15) == 0) && ((ldc * (int)sizeof(OutT)) % 16 == 0);
-  const int tma_store = aligned_c && make_store_map(&tc, c, m, n, ldc, sizeof(OutT) == 2) ? 1 : 0;
-  if (STATS && !tma_store) return -3;           // the statistics are taken from the staged blocks
-  auto kern = gemm_tcgen05_2cta_kernel<OutT, STATS>;
+// About the clocks that a pair needs for 64 rows of the contraction, and what an item of a weight gradient costs besides:
+// its accumulator goes out as fp32 additions.
+constexpr int kBlockClocks = 740, kRedClocks = 3000;
+
+// Tile width: 256 columns, halved while all tiles of the narrower width still run at once.  A step is bound by the
+// operands' way from L2, so a narrower tile does not pay for a fuller last wave (12608 x 3072 x 768: 53.4 us at 256
+// columns, 61.3 at 192, 87.6 at 128), but shorter tiles on more SMs do where the wide ones leave the chip idle
+// (788 x 768 x 768: 10.5 us at 256, 9.4 at 64; 2048 x 384 x 384: 8.3 and 7.3).
+int pick_bn(int m, int n, int pairs, int least) {
+  const int64_t tiles_m = (m + 2 * BM - 1) / (2 * BM);
+  int bn = 256;
+  while (bn > least && tiles_m * ((n + bn / 2 - 1) / (bn / 2)) <= pairs) bn /= 2;
+  return bn;
+}
+
+// Pieces of the contraction of a weight gradient: the number that finishes soonest by these clocks.
+int pick_splits(int m, int n, int k, int bn, int pairs) {
+  const int64_t tiles = (int64_t)((m + 2 * BM - 1) / (2 * BM)) * ((n + bn - 1) / bn), kb = (k + BK - 1) / BK;
+  int best = 1;
+  int64_t best_cost = 0;
+  for (int sp = 1; sp <= kb && (sp == 1 || tiles * sp <= 2 * pairs); ++sp) {
+    const int64_t cost = (tiles * sp + pairs - 1) / pairs * ((kb + sp - 1) / sp * kBlockClocks + kRedClocks);
+    if (sp == 1 || cost < best_cost) { best = sp; best_cost = cost; }
+  }
+  return best;
+}
+
+struct Args {
+  const void* a[kMaxASrc];
+  int n_src;                    // matrices side by side, each k / n_src (kNN) or m / n_src (kRed) wide
+  const void* b;
+  void* c[kMaxCDst];
+  int n_dst;                    // matrices side by side along n, each n / n_dst wide (kTN, through the TMA unit only)
+  const float* bias;
+  int m, n, k, lda, ldb, ldc, epi;
+  float* col_sums;
+  int seg_rows;
+  int* status;
+};
+
+template <typename OutT, bool STATS, int BN, int KIND>
+int launch_bn(const Args& p, int dev, int max_pairs, cudaStream_t stream) {
+  constexpr int kSmemBytes = Cfg<BN>::kSmemBytes;
+  AMaps ta;
+  CUtensorMap tb;
+  const int a_src = (KIND == kRed ? p.m : p.k) / p.n_src;
+  for (int i = 0; i < kMaxASrc; ++i) {
+    if (i >= p.n_src) { ta.m[i] = ta.m[0]; continue; }
+    const void* a = p.a[i];
+    if (!(KIND == kRed ? make_map(&ta.m[i], a, p.k, a_src, p.lda, 64) : make_map(&ta.m[i], a, p.m, a_src, p.lda, BM))) return -6;
+  }
+  if (!(KIND == kTN ? make_map(&tb, p.b, p.n, p.k, p.ldb, BN / 2) : make_map(&tb, p.b, p.k, p.n, p.ldb, 64))) return -6;
+  CMaps tc;
+  const int n_per = p.n / p.n_dst;
+  int tma_store = 1;
+  for (int i = 0; i < kMaxCDst; ++i) {
+    if (i >= p.n_dst) { tc.m[i] = tc.m[0]; continue; }
+    void* c = p.c[i];
+    tc.m[i] = tb;               // placeholder when C cannot be described (the kernel then stores directly)
+    if ((((uintptr_t)c & 15) != 0) || ((p.ldc * (int)sizeof(OutT)) % 16 != 0) ||
+        !make_store_map(&tc.m[i], c, p.m, n_per, p.ldc, sizeof(OutT) == 2))
+      tma_store = 0;
+  }
+  // statistics come from the staged blocks, sums and several destinations need the TMA unit
+  if ((STATS || KIND == kRed || p.n_dst > 1) && !tma_store) return -3;
+  auto kern = gemm_tcgen05_2cta_kernel<OutT, STATS, BN, KIND>;
   static bool attr_set[64] = {};
-  static int n_sm[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 63;
   if (!attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return (int)e;
-    cudaDeviceGetAttribute(&n_sm[dev], cudaDevAttrMultiProcessorCount, dev);
-    if (n_sm[dev] <= 0) n_sm[dev] = 148;
     attr_set[dev] = true;
   }
-  const int num_tiles = ((n + BN - 1) / BN) * ((m + 2 * BM - 1) / (2 * BM));
-  int pairs = (n_sm[dev] - g_tsp_sm_reserve) / 2;      // SMs left to communication kernels stay free
-  if (pairs < 4) pairs = 4;
-  if (pairs > num_tiles) pairs = num_tiles;
+  const int splits = KIND == kRed ? pick_splits(p.m, p.n, p.k, BN, max_pairs) : 1;
+  const int num_items = ((p.n + BN - 1) / BN) * ((p.m + 2 * BM - 1) / (2 * BM)) * splits;
+  const int pairs = max_pairs > num_items ? num_items : max_pairs;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
@@ -470,8 +587,39 @@ int launch(const void* a, const void* b, void* c, const float* bias, int m, int 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tma_store, (OutT*)c, bias, m, n, k, ldc, epi, col_sums, seg_rows, status);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, p.n_src > 1 ? (KIND == kRed ? a_src : a_src / BK) : 0x7fffffff, tb, tc, p.n_dst > 1 ? n_per : 0x7fffffff, tma_store,
+                                     (OutT*)p.c[0], p.bias,
+                                     p.m, p.n, p.k, p.ldc, p.epi, splits, p.col_sums, p.seg_rows, p.status);
   return (int)e;
+}
+
+template <typename OutT, bool STATS, int KIND = kTN>
+int launch(const Args& p, cudaStream_t stream) {
+  static int n_sm[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  dev &= 63;
+  if (n_sm[dev] == 0) {
+    int v = 0;
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    n_sm[dev] = v > 0 ? v : 148;
+  }
+  int pairs = (n_sm[dev] - g_tsp_sm_reserve) / 2;      // SMs left to communication kernels stay free
+  if (pairs < 4) pairs = 4;
+  if constexpr (KIND == kRed) {
+    // the contraction is split until the chip is full, so the width only matters where the output is narrower
+    return p.n > 128 ? launch_bn<OutT, STATS, 256, KIND>(p, dev, pairs, stream)
+                     : launch_bn<OutT, STATS, 128, KIND>(p, dev, pairs, stream);
+  } else if constexpr (!STATS) {
+    const int bn = pick_bn(p.m, p.n, pairs, KIND == kTN ? 64 : 128);   // MN-major B: halves of whole 64-column boxes
+    if constexpr (KIND == kTN) {
+      if (bn == 64) return launch_bn<OutT, STATS, 64, KIND>(p, dev, pairs, stream);
+    }
+    if (bn == 128) return launch_bn<OutT, STATS, 128, KIND>(p, dev, pairs, stream);
+    return launch_bn<OutT, STATS, 256, KIND>(p, dev, pairs, stream);
+  } else {
+    return launch_bn<OutT, STATS, 256, KIND>(p, dev, pairs, stream);
+  }
 }
 
 }  // namespace
@@ -488,8 +636,53 @@ int tsp_gemm_bf16_tn_2cta(const void* a, const void* b, void* c, const float* bi
   if (epi != 0 && bias == nullptr) return -3;
   if ((lda % 8) || (ldb % 8) || (k % 8)) return -3;
   if (((uintptr_t)a | (uintptr_t)b) & 15) return -2;
-  if (out_dtype == TSP_DTYPE_BF16) return launch<__nv_bfloat16, false>(a, b, c, bias, m, n, k, lda, ldb, ldc, epi, nullptr, 1, status, stream);
-  return launch<float, false>(a, b, c, bias, m, n, k, lda, ldb, ldc, epi, nullptr, 1, status, stream);
+  const Args p = {{a, nullptr, nullptr}, 1, b, {c, nullptr, nullptr}, 1, bias, m, n, k, lda, ldb, ldc, epi, nullptr, 1, status};
+  return out_dtype == TSP_DTYPE_BF16 ? launch<__nv_bfloat16, false>(p, stream) : launch<float, false>(p, stream);
+}
+
+// [C0 | C1 | C2] = A[m,k] * B[n,k]^T (+ bias[n]), bf16: one product whose n columns go to n_dst matrices of n / n_dst
+// columns each (a multiple of 64), all with row pitch ldc.  3 x 768 columns of 12608 rows: 49 us, B200,
+// against 64 for three products.
+int tsp_gemm_bf16_tn_2cta_split(const void* a, const void* b, void* const* c, int n_dst, const float* bias, int m, int n,
+                                int k, int lda, int ldb, int ldc, int* status, cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0) return 0;
+  if (n_dst < 1 || n_dst > kMaxCDst || n % n_dst != 0 || (n / n_dst) % 64 != 0) return -3;
+  if ((lda % 8) || (ldb % 8) || (k % 8)) return -3;
+  if (((uintptr_t)a | (uintptr_t)b) & 15) return -2;
+  Args p = {{a, nullptr, nullptr}, 1, b, {c[0], nullptr, nullptr}, n_dst, bias, m, n, k, lda, ldb, ldc,
+            bias != nullptr ? 1 : 0, nullptr, 1, status};
+  for (int i = 0; i < n_dst; ++i) p.c[i] = c[i];
+  return launch<__nv_bfloat16, false>(p, stream);
+}
+
+// C[m,n] (bf16) = [A0 | A1 | A2] B with B [k, n] row-major: the gradient of a linear layer's input (A = dY, B = W), or of
+// n_src layers that share it (A_i = dY_i, B = their weights stacked).  A_i [m, k / n_src] with row pitch lda; k / n_src a
+// multiple of 64 when n_src > 1.
+int tsp_gemm_bf16_nn_2cta(const void* const* a, int n_src, const void* b, void* c, int m, int n, int k, int lda, int ldb,
+                          int ldc, int* status, cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0) return 0;
+  if (n_src < 1 || n_src > kMaxASrc || k % n_src != 0 || (n_src > 1 && (k / n_src) % BK != 0)) return -3;
+  if ((lda % 8) || (ldb % 8)) return -3;
+  Args p = {{a[0], nullptr, nullptr}, n_src, b, {c, nullptr, nullptr}, 1, nullptr, m, n, k, lda, ldb, ldc, 0, nullptr, 1, status};
+  uintptr_t bits = (uintptr_t)b;
+  for (int i = 0; i < n_src; ++i) { p.a[i] = a[i]; bits |= (uintptr_t)a[i]; }
+  if (bits & 15) return -2;
+  return launch<__nv_bfloat16, false, kNN>(p, stream);
+}
+
+// C[m,n] (fp32) += [A0 | A1 | A2]^T B with A_i [k, m / n_src], B [k, n]: the gradient of a linear layer's weight (A = dY,
+// B = X), or of the stacked weights of n_src layers that share their input.  m / n_src a multiple of 64 when n_src > 1; C
+// 16-byte aligned with a row pitch that is a multiple of 4.
+int tsp_gemm_bf16_wgrad_2cta(const void* const* a, int n_src, const void* b, float* c, int m, int n, int k, int lda, int ldb,
+                             int ldc, int* status, cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0) return 0;
+  if (n_src < 1 || n_src > kMaxASrc || m % n_src != 0 || (n_src > 1 && (m / n_src) % 64 != 0)) return -3;
+  if ((lda % 8) || (ldb % 8)) return -3;
+  Args p = {{a[0], nullptr, nullptr}, n_src, b, {c, nullptr, nullptr}, 1, nullptr, m, n, k, lda, ldb, ldc, 0, nullptr, 1, status};
+  uintptr_t bits = (uintptr_t)b;
+  for (int i = 0; i < n_src; ++i) { p.a[i] = a[i]; bits |= (uintptr_t)a[i]; }
+  if (bits & 15) return -2;
+  return launch<float, false, kRed>(p, stream);
 }
 
 // C (bf16) = A B^T as above, plus per-column statistics of the rounded result for a BatchNorm that follows:
@@ -501,7 +694,9 @@ int tsp_gemm_bf16_tn_2cta_stats(const void* a, const void* b, void* c, int m, in
   if (m <= 0 || n <= 0 || k <= 0) return 0;
   if ((lda % 8) || (ldb % 8) || (k % 8) || segs < 1 || m % segs != 0 || (m / segs) % 128 != 0) return -3;
   if (((uintptr_t)a | (uintptr_t)b) & 15) return -2;
-  return launch<__nv_bfloat16, true>(a, b, c, nullptr, m, n, k, lda, ldb, ldc, 0, col_sums, m / segs, status, stream);
+  const Args p = {{a, nullptr, nullptr}, 1, b, {c, nullptr, nullptr}, 1, nullptr, m, n, k, lda, ldb, ldc, 0, col_sums, m / segs,
+                  status};
+  return launch<__nv_bfloat16, true>(p, stream);
 }
 
 }  // extern "C"

@@ -183,6 +183,29 @@ def test_linear_products_at_every_tile_width(m, n, k):
     assert _rel(dw - 1, dy.double().t() @ x.double()) < 1e-5
 
 
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("rows,c,heads", [((2, 65), 192, 3), ((3, 197), 768, 12)])
+def test_fused_qkv_projection_matches_three_linears(rows, c, heads, bias):
+    from tspipe_b200.ops import gemm
+    from tspipe_b200.ops.attention import project_qkv
+    torch.manual_seed(11)
+    x = torch.randn(*rows, c, device=DEV).bfloat16().requires_grad_()
+    w = (torch.randn(3 * c, c, device=DEV) / math.sqrt(c)).requires_grad_()
+    b = torch.randn(3 * c, device=DEV, requires_grad=True) if bias else None
+    qkv = project_qkv(x, w, b, heads)
+    g = [torch.randn_like(t) for t in qkv]
+    leaves = [x, w] + ([b] if bias else [])
+    got = torch.autograd.grad(qkv, leaves, g)
+    gemm.check_status()
+    ref_leaves = [x.detach().double().requires_grad_(), w.detach().bfloat16().double().requires_grad_()] + \
+        ([b.detach().double().requires_grad_()] if bias else [])
+    ref = F.linear(*ref_leaves).view(*rows, 3, heads, c // heads).permute(2, 0, 3, 1, 4).unbind(0)
+    for a, r in zip(qkv, ref):
+        assert _rel(a, r) < EPS[torch.bfloat16]
+    for a, r in zip(got, torch.autograd.grad(ref, ref_leaves, [t.double() for t in g])):
+        assert _rel(a, r) < EPS[torch.bfloat16]
+
+
 def test_loss_gradient_scaling_in_place_and_not():
     """A retained graph gives the same gradient again, with any factor; a freed one takes the buffer over."""
     from tspipe_b200.ops import fused

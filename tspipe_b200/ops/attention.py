@@ -51,9 +51,12 @@ def project_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     """``q, k, v`` as ``[B, H, N, D]`` views from the fused projection parameters ``weight [3C, C]``, ``bias [3C]``.
     On CUDA in "split" mode this is three GEMMs on slices of the parameters, so that no packed qkv tensor exists
     whose gradient autograd would have to assemble from dq, dk and dv; otherwise one GEMM and an unbind."""
-    from .linear import linear
+    from .linear import linear, linear_qkv
     b, n, c = x.shape
     if x.is_cuda and _QKV_MODE == "split":
+        qkv = linear_qkv(x, weight, bias)
+        if qkv is not None:
+            return tuple(t.view(b, n, heads, c // heads).transpose(1, 2) for t in qkv)
         return tuple(linear(x, weight[i * c:(i + 1) * c], None if bias is None else bias[i * c:(i + 1) * c])
                      .view(b, n, heads, c // heads).transpose(1, 2) for i in range(3))
     qkv = linear(x, weight, bias).reshape(b, n, 3, heads, c // heads)

@@ -2,10 +2,9 @@
 
 ``matmul_nt(a, b)`` computes ``a @ b.T`` for row-major bf16 ``a [M, K]`` and ``b [N, K]`` with fp32
 accumulation in tensor memory, optional fused ``+ bias`` and GELU epilogue.  ``linear`` is the autograd
-wrapper used by the transformer blocks and heads: forward on the CTA-pair tcgen05 GEMM, ``dX = dY W`` and
-``dW = dY^T X`` on the implicit-GEMM kernels of ``csrc/conv_igemm_tcgen05.cu`` (a linear layer is a 1x1
-convolution over its rows: the weight is read in place as MN-major tiles, the weight gradient is added into
-the fp32 gradient buffer), the bias gradient on the streaming column-sum kernel.  ``info_nce`` is the MoCo-v3 contrastive loss
+wrapper used by the transformer blocks and heads: forward, ``dX = dY W`` and ``dW = dY^T X`` on the CTA-pair
+tcgen05 GEMM (operands whose contraction index is the slow one are read in place as MN-major tiles, the weight
+gradient is added into the fp32 gradient buffer), the bias gradient on the column-sum kernel.  ``info_nce`` is the MoCo-v3 contrastive loss
 (`benchmarks/moco-v3/main.py:147-162`): row-normalised ``q @ k.T / T`` on the tcgen05 kernel followed
 by the fused cross-entropy kernel (value + gradient in one launch).
 
@@ -94,7 +93,6 @@ _W16 = {}        # id(parameter) -> (parameter, version, bf16 copy); dropped at 
 
 def clear_weight_cache() -> None:
     _W16.clear()
-    _W16T.clear()
 
 
 def _w16(weight: torch.Tensor) -> torch.Tensor:
@@ -118,23 +116,6 @@ def _w16(weight: torch.Tensor) -> torch.Tensor:
     return b16.as_strided(weight.shape, weight.stride(), weight.storage_offset() - base.storage_offset())
 
 
-_W16T = {}       # id(parameter slice base) -> (weight, version, bf16 transposed copy [K, N])
-
-
-def _w16_t(weight: torch.Tensor) -> torch.Tensor:
-    """bf16 ``weight.T`` as a contiguous ``[K, N]`` matrix (the B operand of ``dX = dY @ W`` on the ``A @ B^T`` GEMM),
-    made once per weight and optimizer step."""
-    if _f.IN_CAPTURE:
-        return weight.detach().to(torch.bfloat16).t().contiguous()
-    base = weight._base if weight._base is not None else weight
-    key = (id(base), weight.storage_offset(), tuple(weight.shape))
-    hit = _W16T.get(key)
-    if hit is None or hit[0] is not base or hit[1] != base._version:
-        hit = (base, base._version, _w16(weight).t().contiguous())
-        _W16T[key] = hit
-    return hit[2]
-
-
 def _column_sums(dy2: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """fp32 column sums of a matrix (the bias gradient) on the column-sum kernel."""
     m, n = dy2.shape
@@ -149,9 +130,51 @@ def _column_sums(dy2: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch
     return sums
 
 
-# dX = dY @ W: on the CTA-pair GEMM against a cached transposed bf16 copy of W (True), or on the implicit-GEMM
-# data-gradient kernel that reads W in place as MN-major tiles (False; no transposed copy, about half the speed)
-_DX_ON_PAIR_GEMM = True
+def matmul_nn(a, b: torch.Tensor) -> torch.Tensor:
+    """``[a_0 | a_1 | ..] @ b`` (bf16, fp32 accumulation): ``a`` = up to three ``[M, K_i]`` matrices of one width, ``b
+    [K, N]`` read in place as MN-major tiles.  ``dX = dY @ W`` of a linear layer, or of layers that share their input."""
+    m, n = a[0].shape[0], b.shape[1]
+    c = torch.empty((m, n), dtype=torch.bfloat16, device=b.device)
+    ptrs = (_c.c_void_p * len(a))(*(t.data_ptr() for t in a))
+    L = _f.lib()
+    with _f.on_device(b.device):
+        code = L.tsp_gemm_bf16_nn_2cta(ptrs, _c.c_int(len(a)), _f._ptr(b), _f._ptr(c), _c.c_int(m), _c.c_int(n),
+                                       _c.c_int(b.shape[0]), _c.c_int(a[0].shape[1]), _c.c_int(n), _c.c_int(n),
+                                       _f._ptr(_status_word(b.device)), _f._stream())
+    _f._check(code, "tsp_gemm_bf16_nn_2cta")
+    _f._count()
+    return c
+
+
+def _add_weight_grad(target: torch.Tensor, dys, x2: torch.Tensor) -> None:
+    """``target += [dy_0 | dy_1 | ..]^T @ x2`` (fp32 ``[N, K]``, contiguous) for up to three gradients of one width."""
+    n, k = target.shape
+    ptrs = (_c.c_void_p * len(dys))(*(t.data_ptr() for t in dys))
+    L = _f.lib()
+    with _f.on_device(x2.device):
+        code = L.tsp_gemm_bf16_wgrad_2cta(ptrs, _c.c_int(len(dys)), _f._ptr(x2), _f._ptr(target), _c.c_int(n), _c.c_int(k),
+                                          _c.c_int(x2.shape[0]), _c.c_int(n // len(dys)), _c.c_int(k), _c.c_int(k),
+                                          _f._ptr(_status_word(x2.device)), _f._stream())
+    _f._check(code, "tsp_gemm_bf16_wgrad_2cta")
+    _f._count()
+
+
+def _bf16_rows(t: torch.Tensor, width: int) -> torch.Tensor:
+    """``t`` as a contiguous, 16-byte aligned bf16 ``[rows, width]`` matrix."""
+    t2 = t.reshape(-1, width)
+    if t2.dtype != torch.bfloat16 or not t2.is_contiguous():
+        t2 = t2.to(torch.bfloat16).contiguous()
+    return t2 if t2.data_ptr() % 16 == 0 else t2.clone()
+
+
+def _grad_target(weight: torch.Tensor):
+    """The fp32 buffer that a weight gradient may be added to in place, or None."""
+    from . import conv as _conv
+    g = weight.grad if weight.is_leaf else None
+    if (_conv._ACCUMULATE_IN_PLACE and g is not None and g.dtype == torch.float32 and g.is_contiguous()
+            and g.shape == weight.shape and g.data_ptr() % 16 == 0):
+        return g
+    return None
 
 
 class _Linear(torch.autograd.Function):
@@ -169,46 +192,81 @@ class _Linear(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        from . import conv as _conv
         x2, weight = ctx.saved_tensors
-        m, k = x2.shape
-        n = weight.shape[0]
-        dy2 = dy.reshape(-1, n)
-        if dy2.dtype != torch.bfloat16 or not dy2.is_contiguous():
-            dy2 = dy2.to(torch.bfloat16).contiguous()
-        L = _conv._lib()
-        status = _f._ptr(_status_word(x2.device))
-        dims = (_c.c_int(m), _c.c_int(1), _c.c_int(1), _c.c_int(k), _c.c_int(n), _c.c_int(1), _c.c_int(1))
+        n, k = weight.shape
+        dy2 = _bf16_rows(dy, n)
         dx = dw = db = None
-        with _f.on_device(x2.device):
-            st = _f._stream()
-            if ctx.needs_input_grad[0]:
-                if _DX_ON_PAIR_GEMM:
-                    dx2 = matmul_nt(dy2, _w16_t(weight))          # dX = dY @ W on the CTA-pair GEMM
-                else:
-                    dx2 = torch.empty((m, k), dtype=torch.bfloat16, device=x2.device)
-                    _f._check(L.tsp_conv_dgrad(_f._ptr(dy2), _f._ptr(_w16(weight)), _f._ptr(dx2), *dims, status, st),
-                              "tsp_conv_dgrad")
-                    _f._count()
-                dx = dx2.view(ctx.in_shape)
-                if ctx.dtypes[0] != torch.bfloat16:
-                    dx = dx.to(ctx.dtypes[0])
-            if ctx.needs_input_grad[1]:
-                g = weight.grad if weight.is_leaf else None
-                if (_conv._ACCUMULATE_IN_PLACE and g is not None and g.dtype == torch.float32 and g.is_contiguous()
-                        and g.shape == weight.shape):
-                    target = g                     # the kernel adds into the existing gradient buffer
-                else:
-                    target = torch.zeros((n, k), dtype=torch.float32, device=x2.device)
-                    dw = target if weight.dtype == torch.float32 else target.to(weight.dtype)
-                _f._check(L.tsp_conv_wgrad(_f._ptr(x2), _f._ptr(dy2), _f._ptr(target), *dims, status, st),
-                          "tsp_conv_wgrad")
-                _f._count()
-                if dw is not None and dw is not target:
-                    dw = target.to(weight.dtype)
+        if ctx.needs_input_grad[0]:
+            dx = matmul_nn([dy2], _w16(weight)).view(ctx.in_shape)
+            if ctx.dtypes[0] != torch.bfloat16:
+                dx = dx.to(ctx.dtypes[0])
+        if ctx.needs_input_grad[1]:
+            target = _grad_target(weight)          # the kernel adds into the existing gradient buffer
+            if target is None:
+                target = torch.zeros((n, k), dtype=torch.float32, device=x2.device)
+                dw = target
+            _add_weight_grad(target, [dy2], x2)
+            if dw is not None and weight.dtype != torch.float32:
+                dw = target.to(weight.dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = _column_sums(dy2).to(ctx.dtypes[2])
         return dx, dw, db
+
+
+class _LinearQKV(torch.autograd.Function):
+    """``q, k, v = (x W_i^T + b_i)`` with ``W_i``, ``b_i`` the row blocks of a fused projection: one GEMM with three
+    destinations; in the backward one GEMM for dX over the three gradients side by side (fp32 accumulation across them, no sums of bf16
+    partial results) and one for the fused weight's gradient."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias):
+        x2 = _bf16_rows(x, x.shape[-1])
+        w16 = _w16(weight)
+        c = weight.shape[0] // 3
+        ctx.save_for_backward(x2, weight)
+        ctx.in_shape, ctx.dtypes = x.shape, (x.dtype, weight.dtype, None if bias is None else bias.dtype)
+        m, k = x2.shape
+        out = [torch.empty((m, c), dtype=torch.bfloat16, device=x2.device) for _ in range(3)]
+        bf = None if bias is None else bias.detach().float().contiguous()
+        ptrs = (_c.c_void_p * 3)(*(t.data_ptr() for t in out))
+        with _f.on_device(x2.device):
+            code = _f.lib().tsp_gemm_bf16_tn_2cta_split(_f._ptr(x2), _f._ptr(w16), ptrs, _c.c_int(3), _f._ptr(bf), _c.c_int(m),
+                                                        _c.c_int(3 * c), _c.c_int(k), _c.c_int(k), _c.c_int(k), _c.c_int(c),
+                                                        _f._ptr(_status_word(x2.device)), _f._stream())
+        _f._check(code, "tsp_gemm_bf16_tn_2cta_split")
+        _f._count()
+        return tuple(t.view(*x.shape[:-1], c) for t in out)
+
+    @staticmethod
+    def backward(ctx, *dys):
+        x2, weight = ctx.saved_tensors
+        n, k = weight.shape
+        c = n // 3
+        dy2 = [_bf16_rows(dy, c) for dy in dys]
+        dx = dw = db = None
+        if ctx.needs_input_grad[0]:
+            dx = matmul_nn(dy2, _w16(weight)).view(ctx.in_shape)
+            if ctx.dtypes[0] != torch.bfloat16:
+                dx = dx.to(ctx.dtypes[0])
+        if ctx.needs_input_grad[1]:
+            target = _grad_target(weight)
+            if target is None:
+                target = torch.zeros((n, k), dtype=torch.float32, device=x2.device)
+                dw = target
+            _add_weight_grad(target, dy2, x2)
+            if dw is not None and weight.dtype != torch.float32:
+                dw = target.to(weight.dtype)
+        if ctx.dtypes[2] is not None and ctx.needs_input_grad[2]:
+            db = torch.empty(n, dtype=torch.float32, device=x2.device)
+            for i in range(3):
+                _column_sums(dy2[i], db[i * c:(i + 1) * c])
+            db = db.to(ctx.dtypes[2])
+        return dx, dw, db
+
+
+def linear_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None):
+    """``(q, k, v)`` of a fused projection ``weight [3C, K]``; see :class:`_LinearQKV`."""
+    return _LinearQKV.apply(x, weight, bias)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:

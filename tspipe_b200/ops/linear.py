@@ -2,7 +2,7 @@
 
 On CUDA under bf16 compute, layers whose shapes fit the tile constraints (feature counts multiples of 64, at least
 128 rows) run on the hand-written tcgen05 / TMEM / TMA kernels - forward on the CTA-pair GEMM with the bias in its
-epilogue, both backward products on the implicit-GEMM kernels (:mod:`tspipe_b200.ops.gemm`).  Everything else
+epilogue, both backward products on the same GEMM (:mod:`tspipe_b200.ops.gemm`).  Everything else
 (CPU, fp32 compute, odd shapes) goes to the library GEMM.  Reference call sites: every ``nn.Linear`` of
 `benchmarks/moco-v3/vits.py`, `benchmarks/distilbert/bert.py:104-266`, `benchmarks/byol/models/mlp_head.py:4-26`.
 """
@@ -30,3 +30,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         if gemm.eligible(x, weight):
             return gemm.linear(x, weight, bias)
     return F.linear(x, weight, bias)
+
+
+def linear_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None):
+    """``(q, k, v)`` = ``x @ W_i^T + b_i`` for the three row blocks of ``weight [3C, K]``, or None where the blocks are not
+    what the tcgen05 kernels take."""
+    if _USE_TCGEN05 and x.is_cuda and weight.shape[0] % 3 == 0:
+        from . import gemm
+        if gemm.eligible(x, weight[:weight.shape[0] // 3]):
+            return gemm.linear_qkv(x, weight, bias)
+    return None
