@@ -170,8 +170,8 @@ template <int D, int DV, int BN, bool SAME, typename OutT>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ KMaps kmaps, int rows_per_src,
                 const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
-                float* __restrict__ lse, int nq, int nk, int heads, float scale, float fixed_max, int use_fixed_max,
-                int* __restrict__ status) {
+                float* __restrict__ lse, int nq, int nk_head, int nk_total, int share_q, int heads, float scale,
+                float fixed_max, int use_fixed_max, int* __restrict__ status) {
   using C = Cfg<D, DV, BN, SAME>;
   static_assert(!SAME || D == DV, "one tile can only serve both products when the widths agree");
   extern __shared__ uint8_t smem_raw[];
@@ -193,6 +193,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q0 = blockIdx.x * BM, bh = blockIdx.y, head = bh % heads, bat = bh / heads;
+  // keys split over the heads (contrastive loss): the last head may hold fewer than nk_head
+  const int nk = share_q ? min(nk_head, nk_total - head * nk_head) : nk_head;
   const int n_tiles = (nk + BN - 1) / BN;
 
   if (threadIdx.x == 0) {
@@ -226,7 +228,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       mbar_expect_tx(q_full, (uint32_t)C::kQBytes);
-      for (int kb = 0; kb < D / 64; ++kb) tma_load_4d(q_s + kb * (BM * 128), &tmap_q, q_full, kb * 64, q0, head, bat);
+      for (int kb = 0; kb < D / 64; ++kb) tma_load_4d(q_s + kb * (BM * 128), &tmap_q, q_full, kb * 64, q0, share_q ? 0 : head, bat);
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j % kStages;
         const uint32_t round = j / kStages;
@@ -461,7 +463,8 @@ struct Strides { int64_t ld, hs, bs; };
 template <int D, int DV, int BN, bool SAME, typename OutT>
 int launch(const void* q, void* const* k_srcs, int n_src, const void* v, void* o, float* lse, int batch, int heads, int nq,
            int nk, Strides sq, Strides sk, Strides sv, Strides so, float scale, float fixed_max, int use_fixed_max,
-           int* status, cudaStream_t stream) {
+           int* status, cudaStream_t stream, int split_keys = 0) {
+  // split_keys > 0: that many keys per batch entry, split over the heads in pieces of nk; every head has the same queries
   using C = Cfg<D, DV, BN, SAME>;
   CUtensorMap tq, tv, to;
   KMaps tk;
@@ -470,7 +473,7 @@ int launch(const void* q, void* const* k_srcs, int n_src, const void* v, void* o
   for (int i = 0; i < kMaxKSources; ++i)
     if (!make_map4(&tk.m[i], k_srcs[i < n_src ? i : 0], batch, heads, rows_per_src, D, sk.ld, sk.hs, sk.bs, 64, BN, false))
       return -6;
-  if (!make_map4(&tq, q, batch, heads, nq, D, sq.ld, sq.hs, sq.bs, 64, BM, false) ||
+  if (!make_map4(&tq, q, batch, split_keys > 0 ? 1 : heads, nq, D, sq.ld, sq.hs, sq.bs, 64, BM, false) ||
       !make_map4(&tv, v, batch, heads, SAME ? rows_per_src : nk, DV, sv.ld, sv.hs, sv.bs, 64, BN, false) ||
       !make_map4(&to, o, batch, heads, nq, DV, so.ld, so.hs, so.bs, f32 ? 32 : 64, 32, f32))
     return -6;
@@ -485,8 +488,128 @@ int launch(const void* q, void* const* k_srcs, int n_src, const void* v, void* o
     attr_set[dev] = true;
   }
   dim3 grid((nq + BM - 1) / BM, batch * heads);
-  kern<<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, n_src == 1 ? nk + BN : rows_per_src, tv, to, lse, nq, nk, heads,
+  kern<<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, n_src == 1 ? nk + BN : rows_per_src, tv, to, lse, nq, nk,
+                                                  split_keys, split_keys > 0 ? 1 : 0, heads,
                                                   scale, fixed_max, use_fixed_max, status);
+  return TSP_LAUNCH_CHECK();
+}
+
+// ---------------------------------------------------------------------------------------------
+// The passes around the fused contrastive loss of two (queries, keys) pairs.  One warp per row of 256 elements, 8 per
+// lane; blockIdx.y = pair.
+// ---------------------------------------------------------------------------------------------
+constexpr int kNceDim = 256;
+template <typename T>
+struct NcePairs {
+  const T* q[2];
+  const T* k[2];
+};
+
+__device__ __forceinline__ float row_norm(const float (&v)[8]) {
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) s += v[e] * v[e];
+  return fmaxf(sqrtf(tsp::warp_sum(s)), 1e-12f);
+}
+
+// Unit-norm bf16 rows of the queries and keys; the key rows from n up to n_pad are zeros.
+template <typename T>
+__global__ void __launch_bounds__(256) nce_prepare_kernel(const NcePairs<T> in, int n, int n_pad,
+                                                          __nv_bfloat16* __restrict__ q16,
+                                                          __nv_bfloat16* __restrict__ k16) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = blockIdx.x * 8 + warp;                   // rows 0 .. n - 1: queries, then n_pad key rows
+  if (row >= n + n_pad) return;
+  const bool query = row < n;
+  const int r = query ? row : row - n;
+  const T* src = query ? (blockIdx.y ? in.q[1] : in.q[0]) : (blockIdx.y ? in.k[1] : in.k[0]);
+  __nv_bfloat16* dst = query ? q16 + ((int64_t)blockIdx.y * n + r) * kNceDim
+                             : k16 + ((int64_t)blockIdx.y * n_pad + r) * kNceDim;
+  float v[8] = {};
+  if (r < n) {
+    tsp::ld8(src, (int64_t)r * kNceDim + lane * 8, v);
+    const float norm = row_norm(v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] /= norm;
+  }
+  tsp::st8(dst, lane * 8, v);
+}
+
+// Merges the key chunks' softmax-weighted key sums o [2][chunks][n][256] with their weights (lse [2][chunks][n]), adds
+// 2T/n * (lse - q.k/T) to the loss and writes the gradient with respect to the queries as they came in, i.e. through
+// the normalisation: g = 2/n * (o - k), dq = (g - q^ (q^.g)) / |q|.
+template <typename T>
+__global__ void __launch_bounds__(256) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
+                                                         const __nv_bfloat16* __restrict__ q16,
+                                                         const __nv_bfloat16* __restrict__ k16,
+                                                         const float* __restrict__ o, const float* __restrict__ lse,
+                                                         float* __restrict__ loss, T* __restrict__ gq) {
+  __shared__ float part[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = lane * 8;
+  const int row = blockIdx.x * 8 + warp, pair = blockIdx.y;
+  float contrib = 0.f;
+  if (row < n) {
+    float q[8], qb[8], kb[8], acc[8] = {};
+    tsp::ld8(pair ? in.q[1] : in.q[0], (int64_t)row * kNceDim + col, q);
+    tsp::ld8(q16, ((int64_t)pair * n + row) * kNceDim + col, qb);
+    tsp::ld8(k16, ((int64_t)pair * n_pad + row) * kNceDim + col, kb);
+    const float* l = lse + (int64_t)pair * chunks * n + row;
+    float m = -INFINITY;
+    for (int c = 0; c < chunks; ++c) m = fmaxf(m, l[(int64_t)c * n]);
+    float z = 0.f;
+    for (int c = 0; c < chunks; ++c) {
+      const float wgt = expf(l[(int64_t)c * n] - m);
+      z += wgt;
+      float ov[8];
+      tsp::ld8(o, (((int64_t)pair * chunks + c) * n + row) * kNceDim + col, ov);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += wgt * ov[e];
+    }
+    float pos = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) pos += qb[e] * kb[e];
+    pos = tsp::warp_sum(pos) / temp;
+    contrib = (m + logf(z) - pos) * (2.f * temp / n);
+    const float norm = row_norm(q), gs = 2.f / n;
+    float dot = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      q[e] /= norm;
+      acc[e] = gs * (acc[e] / z - kb[e]);
+      dot += q[e] * acc[e];
+    }
+    dot = norm > 1e-12f ? tsp::warp_sum(dot) : 0.f;       // a clamped norm is a constant
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = (acc[e] - q[e] * dot) / norm;
+    tsp::st8(gq, ((int64_t)pair * n + row) * kNceDim + col, acc);
+  }
+  if (lane == 0) part[warp] = contrib;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += part[i];
+    atomicAdd(loss, s);
+  }
+}
+
+template <typename T>
+int launch_nce_pair(const NcePairs<T>& in, int n, int chunk, int chunks, float temp, void* q16, void* k16, float* o,
+                    float* lse, float* loss, void* gq, int* status, cudaStream_t stream) {
+  const int n_pad = chunk * chunks;
+  cudaError_t e = cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  if (e != cudaSuccess) return (int)e;
+  nce_prepare_kernel<T><<<dim3((n + n_pad + 7) / 8, 2), 256, 0, stream>>>(in, n, n_pad, (__nv_bfloat16*)q16,
+                                                                          (__nv_bfloat16*)k16);
+  const Strides sq = {kNceDim, (int64_t)n * kNceDim, (int64_t)n * kNceDim};
+  const Strides sk = {kNceDim, (int64_t)chunk * kNceDim, (int64_t)n_pad * kNceDim};
+  const Strides so = {kNceDim, (int64_t)n * kNceDim, (int64_t)chunks * n * kNceDim};
+  void* const srcs[1] = {k16};
+  const int rc = launch<256, 256, 64, true, float>(q16, srcs, 1, k16, o, lse, 2, chunks, n, chunk, sq, sk, sk, so,
+                                                   1.f / temp, 1.f / temp, 1, status, stream, n);
+  if (rc != 0) return rc;
+  nce_finish_kernel<T><<<dim3((n + 7) / 8, 2), 256, 0, stream>>>(in, n, n_pad, chunks, temp, (const __nv_bfloat16*)q16,
+                                                                 (const __nv_bfloat16*)k16, o, lse, loss, (T*)gq);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -523,6 +646,29 @@ int tsp_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ls
     return bf16 ? launch<256, 256, 64, true, __nv_bfloat16>(TSP_ATTN_ARGS) : launch<256, 256, 64, true, float>(TSP_ATTN_ARGS);
 #undef TSP_ATTN_ARGS
   return -3;
+}
+
+// Symmetric contrastive loss of two pairs (q0, k0) and (q1, k1) of [n][256] matrices (dtype), keys without gradient:
+// loss = sum over the pairs of 2T/n * sum_i (logsumexp_j(q^_i.k^_j / T) - q^_i.k^_i / T), q^ and k^ the unit-norm rows;
+// gq [2][n][256] = its gradient with respect to q0 and q1.  The keys are split into `chunks` pieces of `chunk` rows (a
+// multiple of 64; (chunks - 1) * chunk < n <= chunks * chunk), one per head of the attention grid, so that the grid fills
+// the chip.  Scores are bounded by 1/T, which is used as the fixed maximum: exp(-2/T) must not underflow.
+// Scratch: q16 [2][n][256] bf16, k16 [2][chunk * chunks][256] bf16, o [2][chunks][n][256] fp32, lse [2][chunks][n] fp32.
+int tsp_nce_pair(const void* q0, const void* k0, const void* q1, const void* k1, int n, int dtype, int chunk, int chunks,
+                 float temp, void* q16, void* k16, float* o, float* lse, float* loss, void* gq, int* status,
+                 cudaStream_t stream) {
+  if (n <= 0 || chunk <= 0 || chunk % 64 != 0 || chunks <= 0 || chunks > 32767) return -3;
+  if ((int64_t)(chunks - 1) * chunk >= n || (int64_t)chunks * chunk < n) return -3;
+  if ((((uintptr_t)q0 | (uintptr_t)k0 | (uintptr_t)q1 | (uintptr_t)k1 | (uintptr_t)q16 | (uintptr_t)k16 | (uintptr_t)o |
+        (uintptr_t)gq) & 15) != 0)
+    return -2;
+  if (dtype == TSP_DTYPE_BF16) {
+    using B = __nv_bfloat16;
+    return launch_nce_pair<B>({{(const B*)q0, (const B*)q1}, {(const B*)k0, (const B*)k1}}, n, chunk, chunks, temp, q16,
+                              k16, o, lse, loss, gq, status, stream);
+  }
+  return launch_nce_pair<float>({{(const float*)q0, (const float*)q1}, {(const float*)k0, (const float*)k1}}, n, chunk,
+                                chunks, temp, q16, k16, o, lse, loss, gq, status, stream);
 }
 
 // Contrastive-loss form with the keys of `n_src` replicas read in place: Q [nq][256] bf16 (pitch 256), K = V = the

@@ -102,6 +102,9 @@ int tsp_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ls
                  const int64_t* o_strides, float scale, float fixed_max, int use_fixed_max, int out_dtype, int* status,
                  cudaStream_t stream);
 
+int tsp_nce_pair(const void* q0, const void* k0, const void* q1, const void* k1, int n, int dtype, int chunk, int chunks,
+                 float temp, void* q16, void* k16, float* o, float* lse, float* loss, void* gq, int* status,
+                 cudaStream_t stream);
 int tsp_attn_nce_gathered(const void* q, void* const* k_srcs, int n_src, int rows_per_src, void* o, float* lse, int nq,
                           float scale, float fixed_max, int* status, cudaStream_t stream);
 

@@ -75,6 +75,72 @@ def test_byol_pair_equals_two_single_losses(n, d, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [128, 129, 200, 1000, 2048])
+def test_nce_pair_matches_cross_entropy(n, dtype):
+    """Ragged query tiles, key chunks whose last one is short."""
+    from tspipe_b200.losses import moco_loss
+    from tspipe_b200.ops import gemm
+    torch.manual_seed(2)
+    q1, q2, k1, k2 = ((torch.randn(n, 256, device=DEV) * 2).to(dtype) for _ in range(4))
+    q1, q2 = (q1 + k2).requires_grad_(), (q2 + k1).requires_grad_()
+    chunk, c = gemm.nce_pair_chunks(n)
+    assert chunk % 64 == 0 and (c - 1) * chunk < n <= c * chunk
+    assert gemm.info_nce_pair(q1, k2, q2, k1, 0.2) is not None
+    loss = moco_loss(q1, q2, k1, k2)
+    g = torch.autograd.grad(loss, [q1, q2])
+    gemm.check_status()
+    r = [t.detach().double().requires_grad_() for t in (q1, q2)]
+    lab = torch.arange(n, device=DEV)
+    ref = sum(0.4 * F.cross_entropy(F.normalize(a, dim=1) @ F.normalize(b.double(), dim=1).t() / 0.2, lab)
+              for a, b in zip(r, (k2, k1)))
+    assert abs(float(loss.detach()) - float(ref.detach())) < 2e-3 * abs(float(ref.detach()))       # unit rows and probabilities in bf16
+    for a, b in zip(g, torch.autograd.grad(ref, r)):
+        assert _rel(a, b) < 8e-3
+
+
+# ---- optimizers ---------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("name", ["adamw", "sgd"])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_vectorised_optimizer_on_an_unaligned_teacher(name, shift):
+    """A teacher buffer off the 16-byte grid, and one whose end cuts a vector, take the scalar loop."""
+    from tspipe_b200.optim import SGD, AdamW
+    from tspipe_b200.runtime.state import FlatParams
+    torch.manual_seed(3)
+    ps = [nn.Parameter(torch.randn(37, 53, device=DEV)), nn.Parameter(torch.randn(130, device=DEV))]
+    ref = [nn.Parameter(p.detach().clone()) for p in ps]
+    mk = (lambda q: AdamW(q, lr=1e-2, weight_decay=0.1)) if name == "adamw" else \
+        (lambda q: SGD(q, lr=0.05, momentum=0.9, weight_decay=1e-3))
+    flat = FlatParams(ps, DEV, with_grad=True)
+    opt, ropt = mk(ps), mk(ref)
+    opt.bind_flat(flat, use_kernel=True)
+    n = flat.total - 64 + shift * 2                 # shift 1: an end inside the last parameter's vectors
+    teacher = torch.zeros(flat.total + 8, device=DEV)[shift: shift + n]
+    opt.teacher_flat, opt.ema_momentum = teacher, 0.5
+    for p, q in zip(ps, ref):
+        q.grad = torch.randn_like(q)
+        p.grad.copy_(q.grad)
+    opt.step()
+    ropt.step()
+    for p, q in zip(ps, ref):
+        torch.testing.assert_close(p.detach(), q.detach(), rtol=1e-5, atol=1e-6)
+    torch.testing.assert_close(teacher, 0.5 * flat.data[:n], rtol=1e-6, atol=1e-7)
+
+
+# ---- elementwise and row passes -----------------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,n", [(2, 8), (77, 24), (1000, 768), (300, 4096), (130, 5120)])
+def test_column_sums(m, n, dtype):
+    from tspipe_b200.ops import gemm
+    torch.manual_seed(4)
+    x = torch.randn(m, n, device=DEV).to(dtype)
+    want = x.double().sum(0)
+    torch.testing.assert_close(gemm._column_sums(x).double(), want, rtol=0, atol=1e-5 * math.sqrt(m) * 4)
+    base = torch.full((n,), 2.0, device=DEV)
+    assert gemm._column_sums(x, add_to=base) is None
+    torch.testing.assert_close(base.double() - 2, want, rtol=0, atol=1e-5 * math.sqrt(m) * 4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("m,c,res", [(16, 4096, False), (64, 4096, True), (37, 24, True), (515, 1000, False),
                                      (4099, 64, True), (9, 2056, False)])
 def test_batchnorm_passes_at_odd_widths(m, c, res, dtype):

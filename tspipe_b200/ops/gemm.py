@@ -427,6 +427,64 @@ class _FusedNCE(torch.autograd.Function):
         return ((o - kn16[: ctx.n].float()) * (g * 2.0 / ctx.n)).to(ctx.qdtype), None, None
 
 
+def nce_pair_chunks(n: int, target_ctas: int = 148):
+    """``(rows per chunk, chunks)`` of the keys for the two-pair loss: 64-row key tiles dealt to as many chunks as bring
+    (2 pairs) x (128-query tiles) x (chunks) closest below ``target_ctas`` CTAs, two tiles per chunk at least."""
+    tiles_q, tiles_k = -(-n // 128), -(-n // 64)
+    c = max(1, min(target_ctas // (2 * tiles_q), tiles_k // 2)) if _NCE_KEY_SPLIT else 1
+    per = -(-tiles_k // c)
+    return per * 64, -(-tiles_k // per)
+
+
+class _NCEPair(torch.autograd.Function):
+    """Both directions of the symmetric contrastive loss: unit-norm bf16 rows, the fused attention kernel with V = K over
+    (pair, key chunk, query tile), and one pass that merges the chunks into the loss and the gradient with respect to the
+    queries."""
+
+    @staticmethod
+    def forward(ctx, q1, q2, k1, k2, temp):
+        n, d = q1.shape
+        chunk, c = nce_pair_chunks(n)
+        dev = q1.device
+        q16 = torch.empty((2, n, d), dtype=torch.bfloat16, device=dev)
+        k16 = torch.empty((2, c * chunk, d), dtype=torch.bfloat16, device=dev)
+        o = torch.empty((2, c, n, d), dtype=torch.float32, device=dev)
+        lse = torch.empty((2, c, n), dtype=torch.float32, device=dev)
+        loss = torch.empty((), dtype=torch.float32, device=dev)
+        gq = torch.empty((2, n, d), dtype=q1.dtype, device=dev)
+        L = _f.lib()
+        with _f.on_device(dev):
+            code = L.tsp_nce_pair(_f._ptr(q1), _f._ptr(k1), _f._ptr(q2), _f._ptr(k2), _c.c_int(n), _c.c_int(_f._dt(q1)),
+                                  _c.c_int(chunk), _c.c_int(c), _c.c_float(temp), _f._ptr(q16), _f._ptr(k16), _f._ptr(o),
+                                  _f._ptr(lse), _f._ptr(loss), _f._ptr(gq), _f._ptr(_status_word(dev)), _f._stream())
+        _f._check(code, "tsp_nce_pair")
+        _f._count(3)
+        ctx.save_for_backward(gq)
+        return loss
+
+    @staticmethod
+    def backward(ctx, gout):
+        (gq,) = ctx.saved_tensors
+        g1, g2 = _f._scaled(gq, gout).unbind(0)
+        need = ctx.needs_input_grad
+        return g1 if need[0] else None, g2 if need[1] else None, None, None, None
+
+
+def info_nce_pair(q1: torch.Tensor, k1: torch.Tensor, q2: torch.Tensor, k2: torch.Tensor, temp: float
+                  ) -> Optional[torch.Tensor]:
+    """``info_nce(q1, k1, temp) + info_nce(q2, k2, temp)`` of one replica from three launches, or None where they do not
+    apply: 256 columns and at least one query tile of plain contiguous tensors, a temperature whose ``exp(-2 / T)`` is
+    far from underflow."""
+    if not (_fused_nce and q1.is_cuda and q1.dim() == 2 and q1.shape[1] == 256 and q1.shape[0] >= 128 and temp >= 0.05
+            and q1.dtype in (torch.float32, torch.bfloat16)):
+        return None
+    for t in (q1, k1, q2, k2):
+        if not (t.shape == q1.shape and t.dtype == q1.dtype and t.device == q1.device and t.is_contiguous()
+                and t.data_ptr() % 16 == 0):
+            return None
+    return _NCEPair.apply(q1, q2, k1.detach(), k2.detach(), float(temp))
+
+
 class _FusedNCEGathered(torch.autograd.Function):
     """:class:`_FusedNCE` against the keys of ALL replicas, read in place from the GPUs that own them (positives
     are the local keys: row i of this replica pairs with key ``i + n * replica`` of the concatenation)."""
