@@ -300,7 +300,7 @@ def _conv_one(cin, cout, k, stride, side, n, flush):
     dw = torch.zeros(cout, k, k, cin, device=dev)
     w16k = conv._w16(wgt)
     args = (C.c_int(n), C.c_int(side), C.c_int(side), C.c_int(cin), C.c_int(cout), C.c_int(k), C.c_int(stride))
-    t_d = _time(lambda: L.tsp_conv_dgrad(f._ptr(g), f._ptr(w16k), f._ptr(dx), *args, st, f._stream()), flush=flush)
+    t_d = _time(lambda: L.tsp_conv_dgrad(f._ptr(g), f._ptr(w16k), f._ptr(None), f._ptr(dx), *args, st, f._stream()), flush=flush)
     t_w = _time(lambda: L.tsp_conv_wgrad(f._ptr(x), f._ptr(g), f._ptr(dw), *args, st, f._stream()), flush=flush)
     gemm.check_status()
     t_lf = _time(lambda: F.conv2d(x, w16, stride=stride, padding=pad), flush=flush)

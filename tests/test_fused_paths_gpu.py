@@ -272,6 +272,37 @@ def test_fused_qkv_projection_matches_three_linears(rows, c, heads, bias):
         assert _rel(a, r) < EPS[torch.bfloat16]
 
 
+@pytest.mark.parametrize("block,cin,planes,stride,side", [("bottleneck", 256, 64, 1, 14), ("bottleneck", 128, 64, 2, 10),
+                                                          ("basic", 64, 64, 1, 9), ("basic", 64, 128, 2, 8)])
+def test_residual_gradient_rides_in_the_data_gradient(block, cin, planes, stride, side):
+    """The gradient of a block's input with the skip branch added by the first convolution's data gradient (1x1, 3x3 and
+    3x3 / 2 kernels, ragged pixel tiles) against the sum that autograd forms: the same roundings."""
+    from tspipe_b200.models.resnet import BasicBlock, Bottleneck
+    from tspipe_b200.ops import conv, gemm
+    cls = Bottleneck if block == "bottleneck" else BasicBlock
+    out = planes * cls.expansion
+    down = nn.Sequential(nn.Conv2d(cin, out, 1, stride=stride, bias=False), nn.BatchNorm2d(out)) \
+        if stride != 1 or cin != out else None
+    torch.manual_seed(13)
+    blk = cls(cin, planes, stride, down).to(DEV).to(memory_format=torch.channels_last)
+    x = _cl(3, cin, side, side)
+    x1, x2 = x.clone(memory_format=torch.preserve_format).requires_grad_(), x.clone(memory_format=torch.preserve_format).requires_grad_()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y, skip = conv.conv_bn_act_fork(blk.conv1, blk.bn1, x1, relu=True)
+        z = conv.conv_bn_act(blk.conv1, blk.bn1, x2, relu=True)
+    g, gs = _cl(*y.shape), _cl(*x.shape)
+    assert skip.grad_fn is not None
+    (a,) = torch.autograd.grad([y, skip], x1, [g, gs])
+    (b,) = torch.autograd.grad(z, x2, g)
+    assert _rel(a, b + gs) < 1e-3                      # bit-equal but for the order of the BatchNorm sums
+    (c,) = torch.autograd.grad(conv.conv2d(x1, blk.conv1.weight, blk.conv1.stride[0])[0], x1, _cl(*y.shape), retain_graph=True)
+    assert c.shape == x.shape
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        blk(x1).float().square().mean().backward()
+    gemm.check_status()
+    assert torch.isfinite(x1.grad).all()
+
+
 def test_loss_gradient_scaling_in_place_and_not():
     """A retained graph gives the same gradient again, with any factor; a freed one takes the buffer over."""
     from tspipe_b200.ops import fused

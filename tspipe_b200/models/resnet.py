@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 from torch import nn
 
-from ..ops.conv import conv_bn_act
+from ..ops.conv import conv_bn_act, conv_bn_act_fork
 from ..ops.pool import GlobalAvgPool, MaxPool3x3s2
 
 
@@ -40,8 +40,9 @@ class Bottleneck(nn.Module):
         self.downsample = downsample
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        identity = x if self.downsample is None else _downsample(self.downsample, x)
-        out = conv_bn_act(self.conv1, self.bn1, x, relu=True)
+        out, identity = conv_bn_act_fork(self.conv1, self.bn1, x, relu=True)
+        if self.downsample is not None:
+            identity = _downsample(self.downsample, identity)
         out = conv_bn_act(self.conv2, self.bn2, out, relu=True)
         return conv_bn_act(self.conv3, self.bn3, out, residual=identity, relu=True)
 
@@ -59,8 +60,9 @@ class BasicBlock(nn.Module):
         self.downsample = downsample
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        identity = x if self.downsample is None else _downsample(self.downsample, x)
-        out = conv_bn_act(self.conv1, self.bn1, x, relu=True)
+        out, identity = conv_bn_act_fork(self.conv1, self.bn1, x, relu=True)
+        if self.downsample is not None:
+            identity = _downsample(self.downsample, identity)
         return conv_bn_act(self.conv2, self.bn2, out, residual=identity, relu=True)
 
 

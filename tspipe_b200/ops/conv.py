@@ -209,6 +209,10 @@ class _Conv2d(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy, _dsums):
+        return _Conv2d._backward(ctx, dy, None)
+
+    @staticmethod
+    def _backward(ctx, dy, addend):
         x, weight = ctx.saved_tensors
         stride = ctx.stride
         n, h, w, cin, cout, k, ho, wo = _geom(x, weight, stride)
@@ -221,9 +225,9 @@ class _Conv2d(torch.autograd.Function):
             st = _f._stream()
             if ctx.needs_input_grad[0]:
                 dx = torch.empty_like(x)
-                code = L.tsp_conv_dgrad(_f._ptr(dy), _f._ptr(_w16(weight)), _f._ptr(dx), _c.c_int(n), _c.c_int(h),
-                                        _c.c_int(w), _c.c_int(cin), _c.c_int(cout), _c.c_int(k), _c.c_int(stride),
-                                        status, st)
+                code = L.tsp_conv_dgrad(_f._ptr(dy), _f._ptr(_w16(weight)), _f._ptr(addend), _f._ptr(dx), _c.c_int(n),
+                                        _c.c_int(h), _c.c_int(w), _c.c_int(cin), _c.c_int(cout), _c.c_int(k),
+                                        _c.c_int(stride), status, st)
                 _f._check(code, "tsp_conv_dgrad")
                 _f._count(4 if stride == 2 and k == 3 else 1)
             if ctx.needs_input_grad[1]:
@@ -244,6 +248,29 @@ class _Conv2d(torch.autograd.Function):
                 if dw is not None and weight.dtype != torch.float32:
                     dw = dw.to(weight.dtype)
         return dx, dw, None, None, None
+
+
+class _Conv2dFork(torch.autograd.Function):
+    """:class:`_Conv2d` of an input that is also handed on unchanged (the other branch of a residual block): the
+    gradient that comes back on that branch is added by the data-gradient kernel as it stores its result."""
+
+    @staticmethod
+    def forward(ctx, x, weight, stride, want_sums, segs):
+        ctx.set_materialize_grads(False)
+        y, sums = _Conv2d.forward(ctx, x, weight, stride, want_sums, segs)
+        return y, sums, x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, _dsums, dskip):
+        x, _ = ctx.saved_tensors
+        if dy is None:
+            return dskip, None, None, None, None
+        fits = (dskip is not None and dskip.dtype == x.dtype and _nhwc(dskip) and dskip.data_ptr() % 16 == 0
+                and ctx.needs_input_grad[0])
+        grads = _Conv2d._backward(ctx, dy, dskip if fits else None)
+        if dskip is not None and not fits and grads[0] is not None:
+            return (grads[0] + dskip,) + grads[1:]
+        return grads
 
 
 _ACCUMULATE_IN_PLACE = True
@@ -279,6 +306,23 @@ def conv_bn_act(conv: nn.Module, bn: nn.Module, x: torch.Tensor, residual: Optio
         y, sums = conv2d(x, conv.weight, conv.stride[0], want_sums=want, segments=segs)
         return _bn.bn_act(bn, y, residual, relu, sums=sums if (sums is not None and _bn.applicable(bn, y)) else None)
     return _bn.bn_act(bn, conv(x), residual, relu)
+
+
+def conv_bn_act_fork(conv: nn.Module, bn: nn.Module, x: torch.Tensor, relu: bool = False
+                     ) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``(relu(bn(conv(x))), x)`` for the first convolution of a residual block: the second output is ``x`` for the
+    block's other branch, whose gradient the convolution's data gradient takes along (see :class:`_Conv2dFork`)."""
+    from . import bn as _bn
+    if not (_IGEMM and torch.is_grad_enabled() and x.requires_grad and torch.is_autocast_enabled()
+            and igemm_eligible(conv, x) and (conv.kernel_size[0], conv.stride[0]) != (1, 2)):
+        return conv_bn_act(conv, bn, x, relu=relu), x
+    want = bool(bn.training)
+    segs = _bn.current_segments() if want else 1
+    n, h, w, _, _, k, ho, wo = _geom(x, conv.weight, conv.stride[0])
+    want = want and _stats_ok(n, ho, wo, k, conv.stride[0], segs)
+    y, sums, skip = _Conv2dFork.apply(x, conv.weight, conv.stride[0], want, segs)
+    y = _bn.bn_act(bn, y, None, relu, sums=sums if (want and _bn.applicable(bn, y)) else None)
+    return y, skip
 
 
 def conv(m: nn.Module, x: torch.Tensor) -> torch.Tensor:
