@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(kBlock, 3) bn_bwd_apply_kernel(const T* __rest
                                                               const float* __restrict__ w,
                                                               const float* __restrict__ bias,
                                                               const float* __restrict__ sums, T* __restrict__ dx,
+                                                              float* __restrict__ gw, float* __restrict__ gb,
                                                               int64_t m, int c) {
   {   // blockIdx.y = segment
     const int64_t so = (int64_t)blockIdx.y * m * c;
@@ -525,6 +526,14 @@ __global__ void __launch_bounds__(kBlock, 3) bn_bwd_apply_kernel(const T* __rest
       }
   };
   load(i);
+  if (gw != nullptr && blockIdx.y == 0 && first < cpv) {      // the parameters' gradients: the sums over the segments
+    for (int e = 0; e < 8; ++e) {
+      float db = 0.f, dw = 0.f;
+      for (int g = 0; g < (int)gridDim.y; ++g) { db += sums[(int64_t)g * 2 * c + ch + e]; dw += sums[(int64_t)(g * 2 + 1) * c + ch + e]; }
+      gb[ch + e] += db;
+      gw[ch + e] += dw;
+    }
+  }
   float A[8], B[8], D[8], sh[8];
   {
     const float inv_m = 1.f / (float)m;
@@ -708,6 +717,7 @@ __global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_bwd_kernel(const T* __
                                                                   const float* __restrict__ wgt,
                                                                   const float* __restrict__ bias,
                                                                   float* __restrict__ sums, T* __restrict__ dx,
+                                                                  float* __restrict__ gw, float* __restrict__ gb,
                                                                   const PoolGeom g) {
   constexpr int pitch = kBlock + 8;
   __shared__ float sm[APPLY ? 1 : 8 * pitch];
@@ -725,6 +735,14 @@ __global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_bwd_kernel(const T* __
   const int64_t stride = (int64_t)gridDim.x * kBlock;
   const int first = blockIdx.x * kBlock + threadIdx.x;
   const int ch = (first % cpv) * 4;
+  if (APPLY && gw != nullptr && blockIdx.y == 0 && first < cpv) {
+    for (int e = 0; e < 4; ++e) {
+      float db = 0.f, dw = 0.f;
+      for (int k = 0; k < (int)gridDim.y; ++k) { db += sums[(int64_t)k * 2 * c + ch + e]; dw += sums[(int64_t)(k * 2 + 1) * c + ch + e]; }
+      gb[ch + e] += db;
+      gw[ch + e] += dw;
+    }
+  }
   float A[4], B[4], D[4], sh[4];                // APPLY: dx = A g + B x + D; else xhat = (x - D) * B; mask: x * A + sh > 0
   {
     const float inv_m = 1.f / (float)((int64_t)g.n * g.h * g.w);
@@ -919,11 +937,11 @@ int tsp_bn_stats(const void* x, int64_t m, int c, int dtype, float* sums, int se
   return TSP_LAUNCH_CHECK();
 }
 
-// sums [c] fp32 = column sums of x [m, c] (the gradient of a bias).
-int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, cudaStream_t stream) {
+// sums [c] fp32 = (or, with `add`, +=) column sums of x [m, c] (the gradient of a bias).
+int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, int add, cudaStream_t stream) {
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 8192) return -3;
-  cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(float) * (size_t)c, stream);
+  cudaError_t e = add ? cudaSuccess : cudaMemsetAsync(sums, 0, sizeof(float) * (size_t)c, stream);
   if (e != cudaSuccess) return (int)e;
   const Tile tl = make_tile(c / 8);
   const int slabs = (c / 8 + tl.tx_n - 1) / tl.tx_n;
@@ -957,15 +975,13 @@ int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, con
   return TSP_LAUNCH_CHECK();
 }
 
-// sums [segs][2*c] is zeroed, then receives per group sum(dy') and sum(dy' * xhat) (db and dw are their sums over
+// sums [segs][2*c], zeroed by the caller, receives per group sum(dy') and sum(dy' * xhat) (db and dw are their sums over
 // the groups).  `y` non-null applies the ReLU mask; `dres` non-null receives dy'.
 int tsp_bn_bwd_reduce(const void* dy, const void* x, const void* y, void* dres, const float* mean_rstd, const float* w,
                       const float* bias, int relu, int64_t m, int c, int dtype, float* sums, int segs,
                       cudaStream_t stream) {
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 8192 || segs < 1 || m % segs != 0) return -3;
-  cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(float) * 2 * (size_t)c * segs, stream);
-  if (e != cudaSuccess) return (int)e;
   m /= segs;
   if (stream_ok(m, c, dtype))
     return launch_stream<1>(x, dy, y, dres, mean_rstd, w, bias, relu, m, c, segs, sums, stream);
@@ -983,9 +999,10 @@ int tsp_bn_bwd_reduce(const void* dy, const void* x, const void* y, void* dres, 
   return TSP_LAUNCH_CHECK();
 }
 
+// gw / gb (optional, together): the gradients of the weight and the bias are added to them.
 int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* mean_rstd, const float* w,
-                     const float* bias, int relu, const float* sums, void* dx, int64_t m, int c, int dtype, int segs,
-                     cudaStream_t stream) {
+                     const float* bias, int relu, const float* sums, void* dx, float* gw, float* gb, int64_t m, int c,
+                     int dtype, int segs, cudaStream_t stream) {
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 4096 || segs < 1 || m % segs != 0) return -3;
   m /= segs;
@@ -993,7 +1010,7 @@ int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* 
 #define TSP_BN_BWD(T, MASK)                                                                                             \
   bn_bwd_apply_kernel<T, MASK>                                                                                          \
       <<<dim3(apply_blocks(m * (c / 8), c / 8, ApplyVecs<T>::bwd, segs), segs), kBlock, 0, stream>>>(                   \
-          (const T*)dy, (const T*)x, (const T*)y, mean_rstd, w, bias, sums, (T*)dx, m, c)
+          (const T*)dy, (const T*)x, (const T*)y, mean_rstd, w, bias, sums, (T*)dx, gw, gb, m, c)
 #define TSP_BN_BWD_MASK(T)                                                                                              \
   do { if (mask == 2) TSP_BN_BWD(T, 2); else if (mask == 1) TSP_BN_BWD(T, 1); else TSP_BN_BWD(T, 0); } while (0)
   if (dtype == TSP_DTYPE_BF16) TSP_BN_BWD_MASK(__nv_bfloat16);
@@ -1030,29 +1047,28 @@ int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums
   return TSP_LAUNCH_CHECK();
 }
 
-// Its backward: dy [segs * n, ho, wo, c], idx and x as above -> dx; sums [segs][2c] is zeroed and receives db and dw.
+// Its backward: dy [segs * n, ho, wo, c], idx and x as above -> dx; sums [segs][2c], zeroed by the
+// caller, receives db and dw; gw / gb as in tsp_bn_bwd_apply.
 int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* x, const float* mean_rstd, const float* w,
-                         const float* b, float* sums, void* dx, int n, int h, int wd, int c, int dtype, int segs,
-                         cudaStream_t stream) {
+                         const float* b, float* sums, void* dx, float* gw, float* gb, int n, int h, int wd, int c,
+                         int dtype, int segs, cudaStream_t stream) {
   PoolGeom g;
   const int rc = pool_geom(n, h, wd, c, segs, &g);
   if (rc != 0) return rc;
-  cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(float) * 2 * (size_t)c * segs, stream);
-  if (e != cudaSuccess) return (int)e;
   const int64_t work = (int64_t)n * g.ho * g.wo * (c / 4);
   const dim3 grid_r(tsp::row_stride_blocks(work, c / 4, kBlock, 8, 148 * 2 / segs, 148 * 3 / segs), segs);
   const dim3 grid_a(tsp::row_stride_blocks(work, c / 4, kBlock, 1, 1, 148 * 32 / segs), segs);
   if (dtype == TSP_DTYPE_BF16) {
     using B = __nv_bfloat16;
     bn_relu_pool_bwd_kernel<B, false><<<grid_r, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, b, sums,
-                                                                     nullptr, g);
+                                                                     nullptr, nullptr, nullptr, g);
     bn_relu_pool_bwd_kernel<B, true><<<grid_a, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, b, sums,
-                                                                    (B*)dx, g);
+                                                                    (B*)dx, gw, gb, g);
   } else {
     bn_relu_pool_bwd_kernel<float, false><<<grid_r, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd,
-                                                                         w, b, sums, nullptr, g);
+                                                                         w, b, sums, nullptr, nullptr, nullptr, g);
     bn_relu_pool_bwd_kernel<float, true><<<grid_a, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd, w,
-                                                                        b, sums, (float*)dx, g);
+                                                                        b, sums, (float*)dx, gw, gb, g);
   }
   return TSP_LAUNCH_CHECK();
 }

@@ -157,7 +157,7 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __
 // part 2: dw[j] = sum_blocks partial[b][0][j], db likewise.  Block = 32 columns x kLnReduce slices of the blocks.
 constexpr int kLnReduce = 32;
 __global__ void __launch_bounds__(32 * kLnReduce) ln_bwd_reduce_kernel(const float* __restrict__ partial, int nblocks, int d,
-                                                            float* __restrict__ dw, float* __restrict__ db) {
+                                                            float* __restrict__ dw, float* __restrict__ db, int add) {
   __shared__ float sm[kLnReduce][33];
   const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
@@ -174,7 +174,8 @@ __global__ void __launch_bounds__(32 * kLnReduce) ln_bwd_reduce_kernel(const flo
   __syncthreads();
   if (slice == 0 && j < 2 * d) {
     acc = sm[0][lane];
-    if (j < d) dw[j] = acc; else db[j - d] = acc;
+    float* out = j < d ? dw + j : db + (j - d);
+    *out = add ? *out + acc : acc;
   }
 }
 
@@ -292,7 +293,7 @@ int launch_ln_fwd(const void* x, const float* w, const float* b, void* y, float*
 
 template <typename T>
 int launch_ln_bwd(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
-                  float* dw, float* db, float* partial, int rows, int d, int nb, cudaStream_t stream) {
+                  float* dw, float* db, float* partial, int rows, int d, int nb, int add, cudaStream_t stream) {
 #define TSP_LN(NV)                                                                                                   \
   ln_bwd_kernel<T, NV><<<nb, kLnBwdWarps * 32, 0, stream>>>((const T*)dy, (const T*)x, w, mean, rstd, (T*)dx, partial, \
                                                             rows, d)
@@ -301,7 +302,7 @@ int launch_ln_bwd(const void* dy, const void* x, const float* w, const float* me
   else if (d <= 768) TSP_LN(3);
   else TSP_LN(4);
 #undef TSP_LN
-  ln_bwd_reduce_kernel<<<(2 * d + 31) / 32, 32 * kLnReduce, 0, stream>>>(partial, nb, d, dw, db);
+  ln_bwd_reduce_kernel<<<(2 * d + 31) / 32, 32 * kLnReduce, 0, stream>>>(partial, nb, d, dw, db, add);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -324,15 +325,21 @@ int tsp_layernorm_bwd_blocks(int rows) {
   return nb > cap ? cap : (nb < 1 ? 1 : nb);
 }
 
-// `partial` is scratch of tsp_layernorm_bwd_blocks(rows) * 2 * d floats.
-int tsp_layernorm_bwd(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
-                      float* dw, float* db, float* partial, int rows, int d, int dtype, cudaStream_t stream) {
+// `partial` is scratch of tsp_layernorm_bwd_blocks(rows) * 2 * d floats; `add`: dw and db are added to instead of set.
+int tsp_layernorm_bwd_add(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
+                          float* dw, float* db, float* partial, int rows, int d, int dtype, int add,
+                          cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8 * 32 * kLnMaxVec) return -3;
   const int nb = tsp_layernorm_bwd_blocks(rows);
   return dtype == TSP_DTYPE_BF16
-             ? launch_ln_bwd<__nv_bfloat16>(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, nb, stream)
-             : launch_ln_bwd<float>(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, nb, stream);
+             ? launch_ln_bwd<__nv_bfloat16>(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, nb, add, stream)
+             : launch_ln_bwd<float>(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, nb, add, stream);
+}
+
+int tsp_layernorm_bwd(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
+                      float* dw, float* db, float* partial, int rows, int d, int dtype, cudaStream_t stream) {
+  return tsp_layernorm_bwd_add(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, dtype, 0, stream);
 }
 
 // Blocks of the GELU passes: `per_thread` vectors per thread on large tensors, at most eight blocks per SM, rounded so
@@ -399,8 +406,8 @@ int tsp_layernorm_bwd_noalloc(const void* dy, const void* x, const float* w, con
   // Nothing in the scratch has to start at zero: each of the nb blocks overwrites its whole 2*d slice and the
   // reduction reads exactly those nb slices, so what an earlier call left behind is never read.
   return dtype == TSP_DTYPE_BF16
-             ? launch_ln_bwd<__nv_bfloat16>(dy, x, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, stream)
-             : launch_ln_bwd<float>(dy, x, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, stream);
+             ? launch_ln_bwd<__nv_bfloat16>(dy, x, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, 0, stream)
+             : launch_ln_bwd<float>(dy, x, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, 0, stream);
 }
 
 }  // extern "C"

@@ -44,6 +44,9 @@ int tsp_layernorm_fwd(const void* x, const float* w, const float* b, void* y, fl
 int tsp_layernorm_bwd_blocks(int rows);
 int tsp_layernorm_bwd(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
                       float* dw, float* db, float* partial, int rows, int d, int dtype, cudaStream_t stream);
+int tsp_layernorm_bwd_add(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
+                          float* dw, float* db, float* partial, int rows, int d, int dtype, int add,
+                          cudaStream_t stream);
 int tsp_gelu_fwd(const void* x, const float* bias, void* y, int64_t n, int d, int dtype, cudaStream_t stream);
 int tsp_gelu_bwd(const void* dy, const void* x, const float* bias, void* dx, int64_t n, int d, int dtype,
                  cudaStream_t stream);
@@ -51,7 +54,7 @@ int tsp_gelu_bwd(const void* dy, const void* x, const float* bias, void* dx, int
 // ---- batchnorm.cu -----------------------------------------------------------------------------------------------
 int tsp_bn_stats(const void* x, int64_t m, int c, int dtype, float* sums, int segs, cudaStream_t stream);
 int tsp_bn_stream_status(int reset);
-int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, cudaStream_t stream);
+int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, int add, cudaStream_t stream);
 int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, const float* fixed_mean_var,
                  const float* w, const float* b, float* save_mean_rstd, float* acc_sum, float* acc_sumsq,
                  float* acc_count, int64_t acc_seg_stride, int64_t m, int c, float eps, int relu, int dtype, int segs,
@@ -60,14 +63,14 @@ int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums
                          float* save_mean_rstd, float* acc_sum, float* acc_sumsq, float* acc_count, int64_t acc_seg_stride,
                          int n, int h, int wd, int c, float eps, int dtype, int segs, cudaStream_t stream);
 int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* x, const float* mean_rstd, const float* w,
-                         const float* b, float* sums, void* dx, int n, int h, int wd, int c, int dtype, int segs,
-                         cudaStream_t stream);
+                         const float* b, float* sums, void* dx, float* gw, float* gb, int n, int h, int wd, int c,
+                         int dtype, int segs, cudaStream_t stream);
 int tsp_bn_bwd_reduce(const void* dy, const void* x, const void* y, void* dres, const float* mean_rstd, const float* w,
                       const float* bias, int relu, int64_t m, int c, int dtype, float* sums, int segs,
                       cudaStream_t stream);
 int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* mean_rstd, const float* w,
-                     const float* bias, int relu, const float* sums, void* dx, int64_t m, int c, int dtype, int segs,
-                     cudaStream_t stream);
+                     const float* bias, int relu, const float* sums, void* dx, float* gw, float* gb, int64_t m, int c,
+                     int dtype, int segs, cudaStream_t stream);
 
 // ---- peer.cu ------------------------------------------------------------------------------------------------------
 int tsp_enable_peer_access(int peer_device);

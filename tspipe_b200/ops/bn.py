@@ -133,6 +133,7 @@ class _BnAct(torch.autograd.Function):
         ctx.save_for_backward(x, y if (relu and residual is not None) else None, save, wf, bf)
         ctx.relu, ctx.has_res, ctx.mc, ctx.segs = relu, residual is not None, (m, c), segs
         ctx.wdtype, ctx.bdtype = weight.dtype, bias.dtype
+        ctx.owners = (weight, bias) if _f.IN_CAPTURE else (None, None)
         ctx.fixed = fixed is not None
         ctx.mark_non_differentiable(sums)
         return y, sums
@@ -149,7 +150,7 @@ class _BnAct(torch.autograd.Function):
         dx = torch.empty_like(x)
         dres = torch.empty_like(x) if (ctx.has_res and ctx.relu) else None
         segs = ctx.segs
-        sums = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
+        sums = _f.zeroed(segs * 2 * c, x.device)
         with _f.on_device(x.device):
             st = _f._stream()
             relu = _c.c_int(1 if ctx.relu else 0)
@@ -163,17 +164,20 @@ class _BnAct(torch.autograd.Function):
             else:
                 sums_for_dx = sums
             src, mask, relu2 = (dres, None, _c.c_int(0)) if dres is not None else (dy, y, relu)
+            gw, gb = (_f.recorded_grad(p) for p in ctx.owners)
+            if gw is None or gb is None or ctx.fixed:
+                gw = gb = None
             _f._check(L.tsp_bn_bwd_apply(_f._ptr(src), _f._ptr(x), _f._ptr(mask), _f._ptr(save), _f._ptr(wf),
-                                         _f._ptr(bf), relu2, _f._ptr(sums_for_dx), _f._ptr(dx), _c.c_int64(m), _c.c_int(c), _c.c_int(dt),
-                                         _c.c_int(segs), st), "tsp_bn_bwd_apply")
+                                         _f._ptr(bf), relu2, _f._ptr(sums_for_dx), _f._ptr(dx), _f._ptr(gw), _f._ptr(gb),
+                                         _c.c_int64(m), _c.c_int(c), _c.c_int(dt), _c.c_int(segs), st),
+                      "tsp_bn_bwd_apply")
             _f._count(3)
+        gres = (dres if dres is not None else dy) if ctx.has_res else None
+        if gw is not None:
+            return dx, None, None, gres, None, None, None, None, None, None, None, None, None
         if segs > 1:
             sums = sums.view(segs, 2 * c).sum(0)
         db, dw = sums[:c], sums[c:]
-        if ctx.has_res:
-            gres = dres if dres is not None else dy
-        else:
-            gres = None
         return dx, dw.to(ctx.wdtype), db.to(ctx.bdtype), gres, None, None, None, None, None, None, None, None, None
 
 
@@ -268,6 +272,7 @@ class _BnReluPool(torch.autograd.Function):
             _f._count()
         ctx.save_for_backward(x, idx, save, wf, bf)
         ctx.segs, ctx.wdtype, ctx.bdtype = segs, weight.dtype, bias.dtype
+        ctx.owners = (weight, bias) if _f.IN_CAPTURE else (None, None)
         return y
 
     @staticmethod
@@ -279,13 +284,19 @@ class _BnReluPool(torch.autograd.Function):
         if dy.dtype != x.dtype or dy.stride() != (ho * wo * c, 1, wo * c, c) or dy.data_ptr() % 16:
             dy = dy.to(x.dtype).clone(memory_format=torch.channels_last)
         dx = torch.empty_like(x)
-        sums = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
+        sums = _f.zeroed(segs * 2 * c, x.device)
+        gw, gb = (_f.recorded_grad(p) for p in ctx.owners)
+        if gw is None or gb is None:
+            gw = gb = None
         with _f.on_device(x.device):
             _f._check(_lib().tsp_bn_relu_pool_bwd(_f._ptr(dy), _f._ptr(idx), _f._ptr(x), _f._ptr(save), _f._ptr(wf),
-                                                  _f._ptr(bf), _f._ptr(sums), _f._ptr(dx), _c.c_int(n // segs),
-                                                  _c.c_int(h), _c.c_int(w), _c.c_int(c), _c.c_int(_f._dt(x)),
-                                                  _c.c_int(segs), _f._stream()), "tsp_bn_relu_pool_bwd")
+                                                  _f._ptr(bf), _f._ptr(sums), _f._ptr(dx), _f._ptr(gw), _f._ptr(gb),
+                                                  _c.c_int(n // segs), _c.c_int(h), _c.c_int(w), _c.c_int(c),
+                                                  _c.c_int(_f._dt(x)), _c.c_int(segs), _f._stream()),
+                      "tsp_bn_relu_pool_bwd")
         _f._count(3)
+        if gw is not None:
+            return dx, None, None, None, None, None, None, None, None, None
         if segs > 1:
             sums = sums.view(segs, 2 * c).sum(0)
         return dx, sums[c:].to(ctx.wdtype), sums[:c].to(ctx.bdtype), None, None, None, None, None, None, None

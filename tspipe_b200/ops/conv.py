@@ -56,7 +56,7 @@ class _StemConv(torch.autograd.Function):
         n, _, h, w = x.shape
         y = torch.empty((n, 64, h // 2, w // 2), dtype=torch.bfloat16, device=x.device,
                         memory_format=torch.channels_last)
-        sums = torch.zeros(segs * 128, dtype=torch.float32, device=x.device) if want_sums else None
+        sums = _f.zeroed(segs * 128, x.device) if want_sums else None
         wm = weight_matrix(weight)
         L = _f.lib()
         L.tsp_conv_stem_fwd.restype = _c.c_int
@@ -119,8 +119,8 @@ def _w16(weight: torch.Tensor) -> torch.Tensor:
     """bf16 copy of a convolution weight laid out ``[Cout][kh][kw][Cin]`` (no copy beyond the cast when the
     parameter is stored channels-last, which is how the runtime keeps 4-D parameters)."""
     if _f.IN_CAPTURE:                   # inside a CUDA graph the cast is part of the graph
-        w = weight.detach().to(torch.bfloat16).permute(0, 2, 3, 1)
-        return w if w.is_contiguous() else w.contiguous()
+        w = _f.recorded_bf16(weight).permute(0, 2, 3, 1)
+        return w if w.is_contiguous() and w.data_ptr() % 16 == 0 else w.clone(memory_format=torch.contiguous_format)
     hit = _W16.get(id(weight))
     if hit is not None and hit[0] is weight and hit[1] == weight._version and hit[2].device == weight.device:
         return hit[2]
@@ -193,7 +193,7 @@ class _Conv2d(torch.autograd.Function):
         n, h, w, cin, cout, k, ho, wo = _geom(x, weight, stride)
         w16 = _w16(weight)
         y = torch.empty((n, cout, ho, wo), dtype=torch.bfloat16, device=x.device, memory_format=torch.channels_last)
-        sums = torch.zeros(segs * 2 * cout, dtype=torch.float32, device=x.device) if want_sums else None
+        sums = _f.zeroed(segs * 2 * cout, x.device) if want_sums else None
         with _f.on_device(x.device):
             code = _lib().tsp_conv_fprop(_f._ptr(x), _f._ptr(w16), _f._ptr(y), _f._ptr(sums), _c.c_int(segs), _c.c_int(n),
                                          _c.c_int(h), _c.c_int(w), _c.c_int(cin), _c.c_int(cout), _c.c_int(k),

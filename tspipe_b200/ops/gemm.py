@@ -105,7 +105,8 @@ def _w16(weight: torch.Tensor) -> torch.Tensor:
     if not base.is_contiguous() or base.dtype == torch.bfloat16:
         return weight.detach().to(torch.bfloat16).contiguous()
     if _f.IN_CAPTURE:                   # inside a CUDA graph the cast is part of the graph
-        return weight.detach().to(torch.bfloat16).contiguous()
+        w = _f.recorded_bf16(weight)
+        return w if w.is_contiguous() and w.data_ptr() % 16 == 0 else w.clone(memory_format=torch.contiguous_format)
     hit = _W16.get(id(base))
     if hit is None or hit[0] is not base or hit[1] != base._version:
         hit = (base, base._version, base.detach().to(torch.bfloat16))
@@ -116,18 +117,25 @@ def _w16(weight: torch.Tensor) -> torch.Tensor:
     return b16.as_strided(weight.shape, weight.stride(), weight.storage_offset() - base.storage_offset())
 
 
-def _column_sums(dy2: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """fp32 column sums of a matrix (the bias gradient) on the column-sum kernel."""
+def _column_sums(dy2: torch.Tensor, out: Optional[torch.Tensor] = None, add_to: Optional[torch.Tensor] = None
+                 ) -> Optional[torch.Tensor]:
+    """fp32 column sums of a matrix (the bias gradient) on the column-sum kernel, in ``out`` when given; with ``add_to``
+    they are added to it and None is returned."""
     m, n = dy2.shape
-    sums = torch.empty(n, dtype=torch.float32, device=dy2.device) if out is None else out
     if n % 8 or n > 8192 or m < 2:
-        return torch.sum(dy2, 0, dtype=torch.float32, out=sums)
+        sums = torch.sum(dy2, 0, dtype=torch.float32)
+        if add_to is not None:
+            add_to.add_(sums)
+            return None
+        return sums if out is None else out.copy_(sums)
+    sums = add_to if add_to is not None else out if out is not None else \
+        torch.empty(n, dtype=torch.float32, device=dy2.device)
     L = _f.lib()
     with _f.on_device(dy2.device):
         _f._check(L.tsp_col_sums(_f._ptr(dy2), _c.c_int64(m), _c.c_int(n), _c.c_int(_f._dt(dy2)), _f._ptr(sums),
-                                 _f._stream()), "tsp_col_sums")
+                                 _c.c_int(0 if add_to is None else 1), _f._stream()), "tsp_col_sums")
     _f._count()
-    return sums
+    return None if add_to is not None else sums
 
 
 def matmul_nn(a, b: torch.Tensor) -> torch.Tensor:
@@ -186,6 +194,7 @@ class _Linear(torch.autograd.Function):
         y = matmul_nt(x2, _w16(weight), bias)
         ctx.save_for_backward(x2, weight)
         ctx.has_bias = bias is not None
+        ctx.bias = bias if _f.IN_CAPTURE else None
         ctx.in_shape = x.shape
         ctx.dtypes = (x.dtype, weight.dtype, None if bias is None else bias.dtype)
         return y.view(*x.shape[:-1], weight.shape[0])
@@ -209,7 +218,8 @@ class _Linear(torch.autograd.Function):
             if dw is not None and weight.dtype != torch.float32:
                 dw = target.to(weight.dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = _column_sums(dy2).to(ctx.dtypes[2])
+            db = _column_sums(dy2, add_to=_f.recorded_grad(ctx.bias))
+            db = None if db is None else db.to(ctx.dtypes[2])
         return dx, dw, db
 
 
@@ -225,6 +235,7 @@ class _LinearQKV(torch.autograd.Function):
         c = weight.shape[0] // 3
         ctx.save_for_backward(x2, weight)
         ctx.in_shape, ctx.dtypes = x.shape, (x.dtype, weight.dtype, None if bias is None else bias.dtype)
+        ctx.bias = bias if _f.IN_CAPTURE else None
         m, k = x2.shape
         out = [torch.empty((m, c), dtype=torch.bfloat16, device=x2.device) for _ in range(3)]
         bf = None if bias is None else bias.detach().float().contiguous()
@@ -257,10 +268,13 @@ class _LinearQKV(torch.autograd.Function):
             if dw is not None and weight.dtype != torch.float32:
                 dw = target.to(weight.dtype)
         if ctx.dtypes[2] is not None and ctx.needs_input_grad[2]:
-            db = torch.empty(n, dtype=torch.float32, device=x2.device)
+            gb = _f.recorded_grad(ctx.bias)
+            if gb is None:
+                db = torch.empty(n, dtype=torch.float32, device=x2.device)
             for i in range(3):
-                _column_sums(dy2[i], db[i * c:(i + 1) * c])
-            db = db.to(ctx.dtypes[2])
+                rows = slice(i * c, (i + 1) * c)
+                _column_sums(dy2[i], *((None, gb[rows]) if db is None else (db[rows],)))
+            db = None if db is None else db.to(ctx.dtypes[2])
         return dx, dw, db
 
 
