@@ -112,6 +112,7 @@ int tsp_attn_nce_gathered(const void* q, void* const* k_srcs, int n_src, int row
                           float scale, float fixed_max, int* status, cudaStream_t stream);
 
 // ---- conv_stem_tcgen05.cu -----------------------------------------------------------------------------------------
+int tsp_conv_stem_wgrad(const void* x, const void* dy, float* dw, int n, int h, int w, int* status, cudaStream_t stream);
 int tsp_conv_stem_fwd(const void* x, const void* wmat, void* y, float* sums, int n, int h, int w, int segs,
                       int* status, cudaStream_t stream);
 

@@ -272,6 +272,24 @@ def test_fused_qkv_projection_matches_three_linears(rows, c, heads, bias):
         assert _rel(a, r) < EPS[torch.bfloat16]
 
 
+@pytest.mark.parametrize("n,h,w", [(1, 8, 8), (3, 10, 24), (2, 32, 224), (5, 64, 96)])
+def test_stem_weight_gradient(n, h, w):
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(12)
+    x = _cl(n, 3, h, w)
+    weight = (torch.randn(64, 3, 7, 7, device=DEV) * 0.1).requires_grad_()
+    y, _ = conv.stem_conv(x, weight, want_sums=False)
+    g = _cl(*y.shape)
+    want = torch.autograd.grad(F.conv2d(x.double(), (w6 := weight.detach().double().requires_grad_()), stride=2, padding=3),
+                               w6, g.double())[0]
+    (dw,) = torch.autograd.grad(y, weight, g, retain_graph=True)
+    assert _rel(dw, want) < 1e-5
+    weight.grad = torch.ones_like(weight).to(memory_format=torch.channels_last)
+    y.backward(g)                                      # added in place to an existing gradient
+    gemm.check_status()
+    assert _rel(weight.grad - 1, want) < 1e-5
+
+
 @pytest.mark.parametrize("block,cin,planes,stride,side", [("bottleneck", 256, 64, 1, 14), ("bottleneck", 128, 64, 2, 10),
                                                           ("basic", 64, 64, 1, 9), ("basic", 64, 128, 2, 8)])
 def test_residual_gradient_rides_in_the_data_gradient(block, cin, planes, stride, side):

@@ -5,7 +5,7 @@
   TMA-fetched pixel boxes (``csrc/conv_igemm_tcgen05.cu``); the forward can hand the following BatchNorm its
   per-channel statistics from the epilogue, one set per stacked view.
 * :func:`stem_conv` - the ResNet stem (7 x 7, stride 2, 3 -> 64 channels; ``csrc/conv_stem_tcgen05.cu``), also with
-  BatchNorm statistics in the epilogue.
+  BatchNorm statistics in the epilogue, and its weight gradient.
 * :func:`conv_bn_act` - ``relu(bn(conv(x)) + residual)`` built from the two and :func:`tspipe_b200.ops.bn.bn_act`.
 
 Reference call sites: the convolutions of the torchvision ResNet that
@@ -76,14 +76,38 @@ class _StemConv(torch.autograd.Function):
         x, weight = ctx.saved_tensors
         dx = dw = None
         need_dx = ctx.needs_input_grad[0]
-        gi, gw, _ = torch.ops.aten.convolution_backward(
-            dy.contiguous(memory_format=torch.channels_last), x, weight.to(torch.bfloat16), None, [2, 2], [3, 3],
-            [1, 1], False, [0, 0], 1, [need_dx, ctx.needs_input_grad[1], False])
-        if need_dx:
-            dx = gi
+        dy = dy.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+        if need_dx:                        # images that want a gradient themselves: the library's data gradient
+            dx = torch.ops.aten.convolution_backward(dy, x, weight.to(torch.bfloat16), None, [2, 2], [3, 3], [1, 1], False,
+                                                     [0, 0], 1, [True, False, False])[0]
         if ctx.needs_input_grad[1]:
-            dw = gw.to(weight.dtype)
+            target = _grad_target(weight)
+            if target is None:
+                target = torch.zeros((64, 7, 7, 3), dtype=torch.float32, device=x.device)
+                dw = target.permute(0, 3, 1, 2)
+            if dy.data_ptr() % 16:
+                dy = dy.clone(memory_format=torch.channels_last)
+            n, _, h, w = x.shape
+            L = _f.lib()
+            L.tsp_conv_stem_wgrad.restype = _c.c_int
+            with _f.on_device(x.device):
+                code = L.tsp_conv_stem_wgrad(_f._ptr(x), _f._ptr(dy), _f._ptr(target), _c.c_int(n), _c.c_int(h),
+                                             _c.c_int(w), _f._ptr(_gemm._status_word(x.device)), _f._stream())
+            _f._check(code, "tsp_conv_stem_wgrad")
+            _f._count()
+            if dw is not None and weight.dtype != torch.float32:
+                dw = dw.to(weight.dtype)
         return dx, dw, None, None
+
+
+def _grad_target(weight: torch.Tensor) -> Optional[torch.Tensor]:
+    """The weight's fp32 gradient when a kernel can add to it in place: it lives in the layout [Cout][k][k][Cin], i.e.
+    channels-last, as in the runtime's flat gradient buffer (autograd then gets nothing more to accumulate)."""
+    g = weight.grad if weight.is_leaf else None
+    if (_ACCUMULATE_IN_PLACE and g is not None and g.dtype == torch.float32 and g.shape == weight.shape
+            and g.permute(0, 2, 3, 1).is_contiguous()):
+        return g
+    return None
 
 
 def stem_conv(x: torch.Tensor, weight: torch.Tensor, want_sums: bool = True, segments: int = 1
@@ -231,14 +255,8 @@ class _Conv2d(torch.autograd.Function):
                 _f._check(code, "tsp_conv_dgrad")
                 _f._count(4 if stride == 2 and k == 3 else 1)
             if ctx.needs_input_grad[1]:
-                # The kernel ADDS into its output.  When the parameter's gradient already lives in an fp32 buffer of
-                # the kernel's layout ([Cout][k][k][Cin], i.e. channels-last, as in the runtime's flat gradient
-                # buffer) the sum goes straight there and autograd gets nothing more to accumulate.
-                g = weight.grad if weight.is_leaf else None
-                if (_ACCUMULATE_IN_PLACE and g is not None and g.dtype == torch.float32 and g.shape == weight.shape
-                        and g.permute(0, 2, 3, 1).is_contiguous()):
-                    target = g
-                else:
+                target = _grad_target(weight)      # the kernel ADDS into its output
+                if target is None:
                     target = torch.zeros((cout, k, k, cin), dtype=torch.float32, device=x.device)
                     dw = target.permute(0, 3, 1, 2)
                 code = L.tsp_conv_wgrad(_f._ptr(x), _f._ptr(dy), _f._ptr(target), _c.c_int(n), _c.c_int(h), _c.c_int(w),
