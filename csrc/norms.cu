@@ -13,10 +13,12 @@ constexpr int kLnMaxVec = 4;   // per-lane register tile: 4 x 8 elements -> rows
 
 // ---------------------------------------------------------------------------------------------
 // LayerNorm forward: one warp per row, NV 16-byte vectors per lane (rows of up to 256 * NV elements), single pass from
-// registers.  Each warp loads two rows before it reduces the first.
+// registers.  Each warp loads two rows before it reduces the first.  ADD: the rows are x + a, rounded to T and written to
+// `sum` as the separate addition would (residual connections: one read and one launch less).
 // ---------------------------------------------------------------------------------------------
-template <typename T, int NV>
-__global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
+template <typename T, int NV, bool ADD>
+__global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ a, T* __restrict__ sum,
+                                                     const float* __restrict__ w,
                                                      const float* __restrict__ b, T* __restrict__ y,
                                                      float* __restrict__ mean, float* __restrict__ rstd, int rows,
                                                      int d, float eps) {
@@ -24,12 +26,16 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ x, co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = (blockIdx.x * 4 + warp) * R;
   const int nvec = d >> 3;
-  tsp::Raw8<T> raw[R][NV];
+  tsp::Raw8<T> raw[R][NV], add[ADD ? R : 1][ADD ? NV : 1];
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int k = 0; k < NV; ++k)
-      if (row0 + r < rows && lane + 32 * k < nvec) tsp::ldraw(x + (int64_t)(row0 + r) * d, (int64_t)(lane + 32 * k) * 8, raw[r][k]);
+      if (row0 + r < rows && lane + 32 * k < nvec) {
+        const int64_t at = (int64_t)(row0 + r) * d + (lane + 32 * k) * 8;
+        tsp::ldraw(x, at, raw[r][k]);
+        if constexpr (ADD) tsp::ldraw(a, at, add[r][k]);
+      }
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int row = row0 + r;
@@ -40,6 +46,14 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ x, co
     for (int k = 0; k < NV; ++k)
       if (lane + 32 * k < nvec) {
         tsp::cvt8(raw[r][k], v[k]);
+        if constexpr (ADD) {
+          float av[8];
+          tsp::cvt8(add[r][k], av);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[k][e] += av[e];
+          tsp::round_as<T>(v[k]);
+          if (sum != nullptr) tsp::st8(sum, (int64_t)row * d + (lane + 32 * k) * 8, v[k]);
+        }
 #pragma unroll
         for (int e = 0; e < 8; ++e) s += v[k][e];
       }
@@ -75,9 +89,10 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ x, co
 // B200: 40 us as separate kernels, 31 this way.  (Requesting the next row ahead of the current one: 36, fewer warps fit.)
 // partial layout: [gridDim.x][2][d] fp32 (scratch memory owned by the caller), summed by ln_bwd_reduce_kernel.
 constexpr int kLnBwdWarps = 8;
-template <typename T, int NV>
+// ADD: `skip` (the gradient that reaches the row on a residual connection) is added to the rounded dx.
+template <typename T, int NV, bool ADD>
 __global__ void __launch_bounds__(kLnBwdWarps * 32, sizeof(T) == 2 ? 2 : 1)
-ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ w,
+ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ skip, const float* __restrict__ w,
               const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
               float* __restrict__ partial, int rows, int d) {
   __shared__ float sm[2 * 256 * NV];       // [2][256 * NV] the block's sums
@@ -128,6 +143,13 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __
         tsp::ld8(w, (int64_t)vi * 8, wv);
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] = rs * (gv[e] * wv[e] - s1 - (xv[e] - mu) * rs * s2);
+        if constexpr (ADD) {
+          float sv[8];
+          tsp::ld8(skip + (int64_t)row * d, (int64_t)vi * 8, sv);
+          tsp::round_as<T>(o);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] += sv[e];
+        }
         tsp::st8(dx + (int64_t)row * d, (int64_t)vi * 8, o);
       }
     }
@@ -278,11 +300,13 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const T* __restrict__ dy,
   }
 }
 
-template <typename T>
-int launch_ln_fwd(const void* x, const float* w, const float* b, void* y, float* mean, float* rstd, int rows, int d,
-                  float eps, cudaStream_t stream) {
+template <typename T, bool ADD>
+int launch_ln_fwd(const void* x, const void* a, void* sum, const float* w, const float* b, void* y, float* mean, float* rstd,
+                  int rows, int d, float eps, cudaStream_t stream) {
   const int grid = (rows + 7) / 8;
-#define TSP_LN(NV) ln_fwd_kernel<T, NV><<<grid, 128, 0, stream>>>((const T*)x, w, b, (T*)y, mean, rstd, rows, d, eps)
+#define TSP_LN(NV)                                                                                                       \
+  ln_fwd_kernel<T, NV, ADD><<<grid, 128, 0, stream>>>((const T*)x, (const T*)a, (T*)sum, w, b, (T*)y, mean, rstd, rows, d, \
+                                                      eps)
   if (d <= 256) TSP_LN(1);
   else if (d <= 512) TSP_LN(2);
   else if (d <= 768) TSP_LN(3);
@@ -291,12 +315,12 @@ int launch_ln_fwd(const void* x, const float* w, const float* b, void* y, float*
   return TSP_LAUNCH_CHECK();
 }
 
-template <typename T>
-int launch_ln_bwd(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
-                  float* dw, float* db, float* partial, int rows, int d, int nb, int add, cudaStream_t stream) {
-#define TSP_LN(NV)                                                                                                   \
-  ln_bwd_kernel<T, NV><<<nb, kLnBwdWarps * 32, 0, stream>>>((const T*)dy, (const T*)x, w, mean, rstd, (T*)dx, partial, \
-                                                            rows, d)
+template <typename T, bool ADD>
+int launch_ln_bwd(const void* dy, const void* x, const void* skip, const float* w, const float* mean, const float* rstd,
+                  void* dx, float* dw, float* db, float* partial, int rows, int d, int nb, int add, cudaStream_t stream) {
+#define TSP_LN(NV)                                                                                                    \
+  ln_bwd_kernel<T, NV, ADD><<<nb, kLnBwdWarps * 32, 0, stream>>>((const T*)dy, (const T*)x, (const T*)skip, w, mean, rstd, \
+                                                                 (T*)dx, partial, rows, d)
   if (d <= 256) TSP_LN(1);
   else if (d <= 512) TSP_LN(2);
   else if (d <= 768) TSP_LN(3);
@@ -314,8 +338,18 @@ int tsp_layernorm_fwd(const void* x, const float* w, const float* b, void* y, fl
                       float eps, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8 * 32 * kLnMaxVec) return -3;
-  return dtype == TSP_DTYPE_BF16 ? launch_ln_fwd<__nv_bfloat16>(x, w, b, y, mean, rstd, rows, d, eps, stream)
-                                 : launch_ln_fwd<float>(x, w, b, y, mean, rstd, rows, d, eps, stream);
+  return dtype == TSP_DTYPE_BF16
+             ? launch_ln_fwd<__nv_bfloat16, false>(x, nullptr, nullptr, w, b, y, mean, rstd, rows, d, eps, stream)
+             : launch_ln_fwd<float, false>(x, nullptr, nullptr, w, b, y, mean, rstd, rows, d, eps, stream);
+}
+
+// sum = x + a (rounded; optional), y = LayerNorm(sum).
+int tsp_add_layernorm_fwd(const void* x, const void* a, void* sum, const float* w, const float* b, void* y, float* mean,
+                          float* rstd, int rows, int d, float eps, int dtype, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (d % 8 != 0 || d > 8 * 32 * kLnMaxVec) return -3;
+  return dtype == TSP_DTYPE_BF16 ? launch_ln_fwd<__nv_bfloat16, true>(x, a, sum, w, b, y, mean, rstd, rows, d, eps, stream)
+                                 : launch_ln_fwd<float, true>(x, a, sum, w, b, y, mean, rstd, rows, d, eps, stream);
 }
 
 // Two blocks per SM, at least two rows per warp.
@@ -325,21 +359,23 @@ int tsp_layernorm_bwd_blocks(int rows) {
   return nb > cap ? cap : (nb < 1 ? 1 : nb);
 }
 
-// `partial` is scratch of tsp_layernorm_bwd_blocks(rows) * 2 * d floats; `add`: dw and db are added to instead of set.
-int tsp_layernorm_bwd_add(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
+// `partial` is scratch of tsp_layernorm_bwd_blocks(rows) * 2 * d floats; `skip` (optional, dx's shape) is added to dx;
+// `add`: dw and db are added to instead of set.
+int tsp_layernorm_bwd_add(const void* dy, const void* x, const void* skip, const float* w, const float* mean, const float* rstd, void* dx,
                           float* dw, float* db, float* partial, int rows, int d, int dtype, int add,
                           cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8 * 32 * kLnMaxVec) return -3;
   const int nb = tsp_layernorm_bwd_blocks(rows);
-  return dtype == TSP_DTYPE_BF16
-             ? launch_ln_bwd<__nv_bfloat16>(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, nb, add, stream)
-             : launch_ln_bwd<float>(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, nb, add, stream);
+#define TSP_LN(T, ADD) launch_ln_bwd<T, ADD>(dy, x, skip, w, mean, rstd, dx, dw, db, partial, rows, d, nb, add, stream)
+  if (dtype == TSP_DTYPE_BF16) return skip != nullptr ? TSP_LN(__nv_bfloat16, true) : TSP_LN(__nv_bfloat16, false);
+  return skip != nullptr ? TSP_LN(float, true) : TSP_LN(float, false);
+#undef TSP_LN
 }
 
 int tsp_layernorm_bwd(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
                       float* dw, float* db, float* partial, int rows, int d, int dtype, cudaStream_t stream) {
-  return tsp_layernorm_bwd_add(dy, x, w, mean, rstd, dx, dw, db, partial, rows, d, dtype, 0, stream);
+  return tsp_layernorm_bwd_add(dy, x, nullptr, w, mean, rstd, dx, dw, db, partial, rows, d, dtype, 0, stream);
 }
 
 // Blocks of the GELU passes: `per_thread` vectors per thread on large tensors, at most eight blocks per SM, rounded so
@@ -406,8 +442,8 @@ int tsp_layernorm_bwd_noalloc(const void* dy, const void* x, const float* w, con
   // Nothing in the scratch has to start at zero: each of the nb blocks overwrites its whole 2*d slice and the
   // reduction reads exactly those nb slices, so what an earlier call left behind is never read.
   return dtype == TSP_DTYPE_BF16
-             ? launch_ln_bwd<__nv_bfloat16>(dy, x, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, 0, stream)
-             : launch_ln_bwd<float>(dy, x, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, 0, stream);
+             ? launch_ln_bwd<__nv_bfloat16, false>(dy, x, nullptr, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, 0, stream)
+             : launch_ln_bwd<float, false>(dy, x, nullptr, w, mean, rstd, dx, dw, db, scratch, rows, d, nb, 0, stream);
 }
 
 }  // extern "C"

@@ -44,7 +44,9 @@ int tsp_layernorm_fwd(const void* x, const float* w, const float* b, void* y, fl
 int tsp_layernorm_bwd_blocks(int rows);
 int tsp_layernorm_bwd(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
                       float* dw, float* db, float* partial, int rows, int d, int dtype, cudaStream_t stream);
-int tsp_layernorm_bwd_add(const void* dy, const void* x, const float* w, const float* mean, const float* rstd, void* dx,
+int tsp_add_layernorm_fwd(const void* x, const void* a, void* sum, const float* w, const float* b, void* y, float* mean,
+                          float* rstd, int rows, int d, float eps, int dtype, cudaStream_t stream);
+int tsp_layernorm_bwd_add(const void* dy, const void* x, const void* skip, const float* w, const float* mean, const float* rstd, void* dx,
                           float* dw, float* db, float* partial, int rows, int d, int dtype, int add,
                           cudaStream_t stream);
 int tsp_gelu_fwd(const void* x, const float* bias, void* y, int64_t n, int d, int dtype, cudaStream_t stream);

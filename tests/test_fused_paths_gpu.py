@@ -206,6 +206,28 @@ def test_layer_norm_widths(rows, d, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d,with_a", [(1, 8, True), (33, 264, True), (700, 768, True), (700, 768, False), (19, 1024, False)])
+def test_add_layer_norm_equals_the_separate_passes(rows, d, with_a, dtype):
+    from tspipe_b200.ops import fused
+    torch.manual_seed(14)
+    x, a = ((torch.randn(rows, d, device=DEV)).to(dtype).requires_grad_() for _ in range(2))
+    w, b = torch.randn(d, device=DEV, requires_grad=True), torch.randn(d, device=DEV, requires_grad=True)
+    gs, gy = torch.randn(rows, d, device=DEV).to(dtype), torch.randn(rows, d, device=DEV).to(dtype)
+    leaves = [x, w, b] + ([a] if with_a else [])
+    s, y = fused.add_layer_norm(x, a if with_a else None, w, b, 1e-6)
+    got = torch.autograd.grad([s, y], leaves, [gs, gy])
+    s2 = x + a if with_a else x
+    y2 = fused.layer_norm(s2, w, b, 1e-6)
+    want = torch.autograd.grad([s2, y2] if with_a else [y2], leaves, [gs, gy] if with_a else [gy])
+    if not with_a:
+        want = (want[0] + gs,) + want[1:]
+    for p, q in zip((s, y) + tuple(got), (s2, y2) + tuple(want)):
+        assert _rel(p, q) < 1e-6                       # bit-equal in bf16; fp32 products may be contracted differently
+    (only,) = torch.autograd.grad(fused.add_layer_norm(x, a if with_a else None, w, b, 1e-6)[1], x, gy)     # no gradient for s
+    assert _rel(only, torch.autograd.grad(fused.layer_norm(s2, w, b, 1e-6), x, gy)[0]) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape,views", [((2, 64, 8, 8), 2), ((3, 8, 5, 7), 1), ((4, 24, 9, 2), 2), ((2, 64, 30, 16), 1),
                                          ((1, 512, 2, 3), 1)])
 def test_batchnorm_relu_maxpool_equals_the_separate_passes(shape, views, dtype):

@@ -27,7 +27,7 @@ from ..model_wrapper import TSPipeModelWrapper
 from ..ops import fused
 from ..ops.attention import attention, project_qkv
 from ..ops.linear import linear
-from .vit import LayerNorm
+from .vit import LayerNorm, norm_of_sum
 
 
 @dataclass
@@ -90,9 +90,9 @@ class EncoderLayer(nn.Module):
         q, k, v = project_qkv(x, self.qkv.weight, self.qkv.bias, self.heads)
         key_mask = mask.to(torch.bool)[:, None, None, :]
         a = attention(q, k, v, key_mask).transpose(1, 2).reshape(b, l, c)
-        x = self.norm1(x + self.drop(linear(a, self.out.weight, self.out.bias)))
+        _, x = norm_of_sum(self.norm1, x, self.drop(linear(a, self.out.weight, self.out.bias)), need_sum=False)
         h = fused.gelu(linear(x, self.fc1.weight, None), self.fc1.bias)
-        x = self.norm2(x + self.drop(linear(h, self.fc2.weight, self.fc2.bias)))
+        _, x = norm_of_sum(self.norm2, x, self.drop(linear(h, self.fc2.weight, self.fc2.bias)), need_sum=False)
         return {"hidden": x, "mask": mask}
 
 

@@ -61,6 +61,17 @@ class LayerNorm(nn.LayerNorm):
         return fused.layer_norm(x, self.weight, self.bias, self.eps)
 
 
+def norm_of_sum(norm: nn.Module, x: torch.Tensor, a: Optional[torch.Tensor] = None, need_sum: bool = True
+                ) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
+    """``(s, norm(s))`` for ``s = x + a``, or for ``s = x`` that goes on as a residual connection; in one pass when ``norm``
+    is this file's LayerNorm and nothing hooks into it.  ``s`` may be None without ``need_sum``."""
+    if type(norm) is LayerNorm and not (norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks
+                                        or norm._backward_pre_hooks):
+        return fused.add_layer_norm(x, a, norm.weight, norm.bias, norm.eps, need_sum)
+    s = x if a is None else x + a
+    return s, norm(s)
+
+
 class PatchEmbed(nn.Module):
     def __init__(self, cfg: ViTConfig, in_chans: int = 3):
         super().__init__()
@@ -163,8 +174,9 @@ class Block(nn.Module):
         self.mlp = Mlp(cfg.embed_dim, int(cfg.embed_dim * cfg.mlp_ratio))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        x = x + self.attn(self.norm1(x))
-        return x + self.mlp(self.norm2(x))
+        x, h = norm_of_sum(self.norm1, x)
+        x, h = norm_of_sum(self.norm2, x, self.attn(h))
+        return x + self.mlp(h)
 
 
 class PreLogits(nn.Module):

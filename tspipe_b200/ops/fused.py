@@ -455,6 +455,10 @@ class _LayerNorm(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
+        return _LayerNorm._backward(ctx, dy, None)
+
+    @staticmethod
+    def _backward(ctx, dy, skip):
         x2, wf, mean, rstd = ctx.saved_tensors
         rows, d = x2.shape
         dy2 = dy.reshape(rows, d).to(x2.dtype).contiguous()
@@ -466,13 +470,67 @@ class _LayerNorm(torch.autograd.Function):
         nb = lib().tsp_layernorm_bwd_blocks(_c.c_int(rows))
         partial = torch.empty(nb * 2 * d, dtype=torch.float32, device=x2.device)
         with on_device(x2.device):
-            _check(lib().tsp_layernorm_bwd_add(_ptr(dy2), _ptr(x2), _ptr(wf), _ptr(mean), _ptr(rstd), _ptr(dx), _ptr(dw),
-                                               _ptr(db), _ptr(partial), _c.c_int(rows), _c.c_int(d), _c.c_int(_dt(x2)),
-                                               _c.c_int(1 if add else 0), _stream()), "tsp_layernorm_bwd")
+            _check(lib().tsp_layernorm_bwd_add(_ptr(dy2), _ptr(x2), _ptr(skip), _ptr(wf), _ptr(mean), _ptr(rstd), _ptr(dx),
+                                               _ptr(dw), _ptr(db), _ptr(partial), _c.c_int(rows), _c.c_int(d),
+                                               _c.c_int(_dt(x2)), _c.c_int(1 if add else 0), _stream()),
+                   "tsp_layernorm_bwd")
         _count(2)
         if add:
             return dx.view(ctx.shape), None, None, None
         return dx.view(ctx.shape), dw.to(ctx.wdtype), db.to(ctx.wdtype), None
+
+
+class _AddLayerNorm(torch.autograd.Function):
+    """``(s, layer_norm(s))`` with ``s = x + a``, or ``s = x`` where ``a`` is None (a residual connection that starts here):
+    the gradient that comes back for ``s`` is added as the LayerNorm's own is stored."""
+
+    @staticmethod
+    def forward(ctx, x, a, w, b, eps, need_sum):
+        ctx.set_materialize_grads(False)
+        if a is None:
+            return x.view_as(x), _LayerNorm.forward(ctx, x, w, b, eps)
+        d = x.shape[-1]
+        rows = x.numel() // d
+        s = torch.empty_like(x) if need_sum or any(ctx.needs_input_grad) else None
+        y = torch.empty_like(x)
+        mean = torch.empty(rows, dtype=torch.float32, device=x.device)
+        rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
+        wf, bf = w.detach().float().contiguous(), b.detach().float().contiguous()
+        with on_device(x.device):
+            _check(lib().tsp_add_layernorm_fwd(_ptr(x), _ptr(a), _ptr(s), _ptr(wf), _ptr(bf), _ptr(y), _ptr(mean), _ptr(rstd),
+                                               _c.c_int(rows), _c.c_int(d), _c.c_float(eps), _c.c_int(_dt(x)), _stream()),
+                   "tsp_add_layernorm_fwd")
+        _count()
+        if s is not None:
+            ctx.save_for_backward(s.view(rows, d), wf, mean, rstd)
+        ctx.shape, ctx.wdtype = x.shape, w.dtype
+        ctx.owners = (w, b) if IN_CAPTURE else (None, None)
+        return s, y
+
+    @staticmethod
+    def backward(ctx, ds, dy):
+        if dy is None:
+            return ds, (ds if ctx.needs_input_grad[1] else None), None, None, None, None
+        x2 = ctx.saved_tensors[0]
+        fits = ds is not None and ds.dtype == x2.dtype and ds.is_contiguous() and ds.data_ptr() % 16 == 0
+        dx, dw, db, _ = _LayerNorm._backward(ctx, dy, ds if fits else None)
+        if ds is not None and not fits:
+            dx = dx + ds
+        return dx, (dx if ctx.needs_input_grad[1] else None), dw, db, None, None
+
+
+def add_layer_norm(x: torch.Tensor, a: Optional[torch.Tensor], weight: torch.Tensor, bias: torch.Tensor, eps: float = 1e-5,
+                   need_sum: bool = True):
+    """``(s, layer_norm(s))`` for ``s = x + a`` (``s = x`` without ``a``), in one pass each way where the kernels apply.
+    Without ``need_sum`` the first may be None (it is not written then)."""
+    d = x.shape[-1]
+    if (x.is_cuda and d % 8 == 0 and d <= 1024 and x.dtype in (torch.float32, torch.bfloat16) and x.is_contiguous()
+            and x.data_ptr() % 16 == 0 and x.numel() > 0
+            and (a is None or (a.dtype == x.dtype and a.shape == x.shape and a.device == x.device and a.is_contiguous()
+                               and a.data_ptr() % 16 == 0))):
+        return _AddLayerNorm.apply(x, a, weight, bias, eps, need_sum)
+    s = x if a is None else x + a
+    return s, layer_norm(s, weight, bias, eps)
 
 
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
