@@ -1239,6 +1239,14 @@ int tsp_conv_wgrad(const void* x, const void* dy, float* dw, int n, int h, int w
                    int* status, cudaStream_t stream) {
   if (!shape_ok(n, h, w, cin, cout, k, s)) return -3;
   if (((uintptr_t)x | (uintptr_t)dy) & 15) return -2;
+  // A 1x1 stride-1 convolution is a linear layer over its pixels.  The CTA-pair product's tile is 256 output channels high:
+  // where it is full it is faster at every size tried (B200, 256 images: 64 -> 256 at 56 x 56 79 us against 84, 512 -> 256
+  // at 28 x 28 54 / 67, 1024 -> 256 at 14 x 14 29 / 39, 512 -> 2048 at 7 x 7 28 / 39; 37 images: 11 - 16 / 20 - 23); with
+  // 64 or 128 output channels it is not (256 -> 64 at 56 x 56 86 / 79).
+  if (k == 1 && s == 1 && cout % 256 == 0 && ((uintptr_t)dw & 15) == 0) {
+    const void* const dys[1] = {dy};
+    return tsp_gemm_bf16_wgrad_2cta(dys, 1, x, dw, cout, cin, n * h * w, cout, cin, cin, status, stream);
+  }
   const int bn = cout % 256 == 0 ? 256 : (cout % 128 == 0 ? 128 : 64);
   Plan p = plan_input(x, n, h, w, cin, k, s, bn == 256 ? 64 : 128);
   if (!p.ok) return -6;

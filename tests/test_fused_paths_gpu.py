@@ -312,6 +312,23 @@ def test_stem_weight_gradient(n, h, w):
     assert _rel(weight.grad - 1, want) < 1e-5
 
 
+@pytest.mark.parametrize("n,h,w,cin,cout,k", [(1, 8, 16, 64, 256, 1), (3, 10, 10, 128, 256, 1), (2, 7, 7, 512, 512, 1)])
+def test_convolution_weight_gradient_paths(n, h, w, cin, cout, k):
+    """1x1 as a linear layer on the CTA-pair GEMM: the fp32 sums of exact bf16 products, against float64."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(14)
+    x = _cl(n, cin, h, w)
+    weight = (torch.randn(cout, cin, k, k, device=DEV) * 0.1).to(memory_format=torch.channels_last).requires_grad_()
+    y, _ = conv.conv2d(x, weight)
+    g = _cl(*y.shape)
+    want = torch.autograd.grad(F.conv2d(x.double(), (w6 := weight.detach().double().requires_grad_()), padding=k // 2),
+                               w6, g.double())[0]
+    for twice in (1, 2):                               # the second one is added to the gradient that is there
+        y.backward(g, retain_graph=True)
+        gemm.check_status()
+        assert _rel(weight.grad, twice * want) < 1e-5
+
+
 @pytest.mark.parametrize("block,cin,planes,stride,side", [("bottleneck", 256, 64, 1, 14), ("bottleneck", 128, 64, 2, 10),
                                                           ("basic", 64, 64, 1, 9), ("basic", 64, 128, 2, 8)])
 def test_residual_gradient_rides_in_the_data_gradient(block, cin, planes, stride, side):
