@@ -312,9 +312,12 @@ def test_stem_weight_gradient(n, h, w):
     assert _rel(weight.grad - 1, want) < 1e-5
 
 
-@pytest.mark.parametrize("n,h,w,cin,cout,k", [(1, 8, 16, 64, 256, 1), (3, 10, 10, 128, 256, 1), (2, 7, 7, 512, 512, 1)])
+@pytest.mark.parametrize("n,h,w,cin,cout,k", [(1, 8, 16, 64, 256, 1), (3, 10, 10, 128, 256, 1), (2, 7, 7, 512, 512, 1),
+                                              (1, 8, 8, 64, 64, 3), (3, 13, 9, 64, 64, 3), (2, 5, 61, 64, 64, 3),
+                                              (2, 56, 56, 64, 64, 3), (1, 64, 2, 64, 64, 3), (200, 8, 8, 64, 64, 3)])
 def test_convolution_weight_gradient_paths(n, h, w, cin, cout, k):
-    """1x1 as a linear layer on the CTA-pair GEMM: the fp32 sums of exact bf16 products, against float64."""
+    """1x1 as a linear layer on the CTA-pair GEMM and 64 to 64 channels 3x3 with the bordered box resident: the fp32 sums of
+    exact bf16 products, against float64."""
     from tspipe_b200.ops import conv, gemm
     torch.manual_seed(14)
     x = _cl(n, cin, h, w)
