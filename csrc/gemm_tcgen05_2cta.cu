@@ -14,13 +14,14 @@
 //                  ONE tcgen05.commit that arrives on the barrier of both CTAs (a commit costs the issuing thread as
 //                  much as eight MMA issues; two per k-block made the issuing thread, not the tensor core, the limit);
 //   tmem_full[a]   in each CTA: committed by the leader (to both CTAs at once) after the last MMA of a tile;
-//   tmem_empty[a]  in the leader: 8 arrivals, one per epilogue warp of the pair (the peer's arrive remotely).
+//   tmem_empty[a]  in the leader: one arrival per epilogue warp of the pair (the peer's arrive remotely).
 // Epilogue: TMEM -> registers -> swizzled shared memory -> TMA store (32 rows x 128 bytes per store, two buffers
 // per warp); direct per-thread stores when C has no 16-byte-aligned base and row pitch.
 // The cluster is synchronised once after barrier initialisation and once before exit, so no CTA leaves while its
 // partner can still touch its shared memory.
 #include <cuda.h>
 
+#include "gelu.cuh"
 #include "tcgen05.cuh"
 #include "tspipe_kernels.h"
 
@@ -31,12 +32,11 @@ namespace {
 constexpr int BM = 128;          // rows per CTA (pair tile: 256)
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int kThreads = 192;
 constexpr uint64_t kWaitNs = 2000000000ull;   // every mbarrier wait gives up after two seconds
 constexpr int kGroup = 2;                       // stages released per tcgen05.commit
 constexpr int kABytes = BM * BK * 2;
 constexpr int kStoreBufBytes = 32 * 128;                        // 32 rows x 128 bytes of C, one TMA store
-constexpr int kStoreBytes = 4 * 2 * kStoreBufBytes;             // two buffers per epilogue warp
+constexpr int kStoreBytes = 8 * kStoreBufBytes;                 // two buffers per epilogue warp, or one for each of eight
 // BN = tile columns (256, 128 or 64); each CTA stages BN / 2 rows of B
 template <int BN> struct Cfg {
   static constexpr int kStages = BN == 256 ? 6 : 8;
@@ -141,9 +141,13 @@ __device__ __forceinline__ float gelu_erf(float x) { return 0.5f * x * (1.f + er
 enum Kind {
   kTN = 0,      // C = A[m, k] B[n, k]^T      forward
   kNN = 1,      // C = A[m, k] B[k, n]        gradient of the input; A may be up to three matrices side by side along k
+  kGelu = 3,    // C0 = A[m, k] B[n, k]^T rounded, C1 = gelu(C0 + bias): the first half of an MLP; C0 only where a backward needs it
   kRed = 2      // C += A[k, m]^T B[k, n]     gradient of the weight: fp32, split along k, added in L2 by the TMA unit; A may
                 //                            be up to three matrices side by side along m
 };
+// Epilogue warps: two per TMEM lane quarter where the epilogue computes (256 GELUs per row and tile would take one longer
+// than the tile's products), with one staging buffer each instead of two.
+__host__ __device__ constexpr int epi_warps(int kind) { return kind == kGelu ? 8 : 4; }
 constexpr int kMaxASrc = 3;
 struct AMaps {
   CUtensorMap m[kMaxASrc];
@@ -156,7 +160,7 @@ struct CMaps {
 };
 
 template <typename OutT, bool STATS, int BN, int KIND>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const __grid_constant__ CUtensorMap tmap_b,
                          const __grid_constant__ CMaps tmap_c, int n_per, int tma_store, OutT* __restrict__ c,
                          const float* __restrict__ bias, int m, int n, int k, int ldc, int epi, int splits,
@@ -200,7 +204,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tmem_full_bar + a, 1);
-      mbar_init(tmem_empty_bar + a, 8);
+      mbar_init(tmem_empty_bar + a, 2 * epi_warps(KIND));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a.m[0]) : "memory");
@@ -252,7 +256,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
           } else {
             tma_load_2d_pair(a_dst, &tmap_a.m[0], lbar, kb * BK, m0);
           }
-          if constexpr (KIND == kTN) {
+          if constexpr (KIND == kTN || KIND == kGelu) {
             tma_load_2d_pair(b_dst, &tmap_b, lbar, kb * BK, n0);
           } else {
 #pragma unroll
@@ -264,8 +268,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
     if (lane == 0 && leader) {
-      static_assert(KIND == kTN || BN % 128 == 0, "an MN-major half tile of B is whole 64-column boxes");
-      constexpr bool kAmn = KIND == kRed, kBmn = KIND != kTN;
+      constexpr bool kAmn = KIND == kRed, kBmn = KIND == kNN || KIND == kRed;
+      static_assert(!kBmn || BN % 128 == 0, "an MN-major half tile of B is whole 64-column boxes");
       constexpr uint32_t idesc = tc5::make_idesc(2 * BM, BN, kAmn, kBmn);
       const uint32_t tiles_addr = smem_u32(tiles);
       uint32_t it = 0, lt = 0;
@@ -308,8 +312,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
     // buffers per warp, so the store of block i overlaps the conversion of block i + 1.  Without a usable
     // tensor map for C (unaligned base or row pitch) every thread stores its own row directly.
     constexpr int kCols = 128 / (int)sizeof(OutT);
-    const int quarter = warp & 3;
-    uint8_t* my_bufs = store_bufs + quarter * 2 * kStoreBufBytes;
+    constexpr int kBufs = 8 / epi_warps(KIND);         // staging buffers per warp
+    const int quarter = warp & 3, group = (warp - 2) >> 2;
+    uint8_t* my_bufs = store_bufs + (warp - 2) * kBufs * kStoreBufBytes;
     uint32_t lt = 0, nstore = 0;
     bool ok = true;
     // STATS: per-column sum and sum of squares of the rounded outputs (the statistics of a BatchNorm that
@@ -344,6 +349,43 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row0 = m0 + quarter * 32, row = row0 + lane;
+      // the block's values -> swizzled staging buffer -> TMA store at column x of `map`; returns the buffer
+      auto stage = [&](const float (&v)[kCols], const CUtensorMap* map, int x, bool inside) -> uint8_t* {
+        uint8_t* buf = my_bufs + (nstore % kBufs) * kStoreBufBytes;
+        if (nstore >= kBufs) {       // the store issued kBufs blocks ago has finished reading this buffer
+          if (lane == 0) {
+            if constexpr (kBufs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          }
+          __syncwarp();
+        }
+        uint8_t* my_row = buf + lane * 128;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {   // 16-byte piece j of this row sits at piece (j ^ (row & 7))
+          uint4 q;
+          if constexpr (kCols == 64) {
+            q.x = pack_bf16x2(v[8 * j + 0], v[8 * j + 1]);
+            q.y = pack_bf16x2(v[8 * j + 2], v[8 * j + 3]);
+            q.z = pack_bf16x2(v[8 * j + 4], v[8 * j + 5]);
+            q.w = pack_bf16x2(v[8 * j + 6], v[8 * j + 7]);
+          } else {
+            q.x = __float_as_uint(v[4 * j + 0]);
+            q.y = __float_as_uint(v[4 * j + 1]);
+            q.z = __float_as_uint(v[4 * j + 2]);
+            q.w = __float_as_uint(v[4 * j + 3]);
+          }
+          *reinterpret_cast<uint4*>(my_row + ((j ^ (lane & 7)) << 4)) = q;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          if (!inside) asm volatile("cp.async.bulk.commit_group;" ::: "memory");     // keep the group count in step
+          else if constexpr (KIND == kRed) tma_reduce_add_2d(map, buf, x, row0);
+          else tma_store_2d(map, buf, x, row0);
+        }
+        ++nstore;
+        return buf;
+      };
       // one block of kCols columns; returns false past the matrix edge
       auto chunk = [&](int c0, float* st) -> bool {
         if (n0 + c0 >= n) return false;            // columns past the matrix edge: nothing to convert or store
@@ -358,6 +400,22 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
           for (int j = 0; j < kCols; ++j) v[j] = __uint_as_float(r[j]);
         }
         const int col = n0 + c0;
+        if constexpr (KIND == kGelu) {             // n is a multiple of 64, C is written by the TMA unit
+          const bool inside = row0 < m;
+          tsp::round_as<OutT>(v);
+          if (epi != 0) stage(v, &tmap_c.m[0], col, inside);
+          const float4* bp = reinterpret_cast<const float4*>(bias + col);
+#pragma unroll
+          for (int j = 0; j < kCols / 4; ++j) {
+            const float4 b4 = __ldg(bp + j);
+            v[4 * j + 0] = tsp::gelu_f<OutT>(v[4 * j + 0] + b4.x);
+            v[4 * j + 1] = tsp::gelu_f<OutT>(v[4 * j + 1] + b4.y);
+            v[4 * j + 2] = tsp::gelu_f<OutT>(v[4 * j + 2] + b4.z);
+            v[4 * j + 3] = tsp::gelu_f<OutT>(v[4 * j + 3] + b4.w);
+          }
+          stage(v, &tmap_c.m[1], col, inside);
+          return true;
+        }
         if (epi != 0 && col < n) {
           if (col + kCols <= n && (((uintptr_t)(bias + col)) & 15) == 0) {
             // whole block inside the matrix: the block's bias values as 16-byte loads (every lane reads the same
@@ -378,38 +436,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
           }
         }
         if (tma_store) {
-          uint8_t* buf = my_bufs + (nstore & 1) * kStoreBufBytes;
-          if (nstore >= 2) {         // the store issued two blocks ago has finished reading this buffer
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-            __syncwarp();
-          }
-          uint8_t* my_row = buf + lane * 128;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {   // 16-byte piece j of this row sits at piece (j ^ (row & 7))
-            uint4 q;
-            if constexpr (kCols == 64) {
-              q.x = pack_bf16x2(v[8 * j + 0], v[8 * j + 1]);
-              q.y = pack_bf16x2(v[8 * j + 2], v[8 * j + 3]);
-              q.z = pack_bf16x2(v[8 * j + 4], v[8 * j + 5]);
-              q.w = pack_bf16x2(v[8 * j + 6], v[8 * j + 7]);
-            } else {
-              q.x = __float_as_uint(v[4 * j + 0]);
-              q.y = __float_as_uint(v[4 * j + 1]);
-              q.z = __float_as_uint(v[4 * j + 2]);
-              q.w = __float_as_uint(v[4 * j + 3]);
-            }
-            *reinterpret_cast<uint4*>(my_row + ((j ^ (lane & 7)) << 4)) = q;
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) {
-            if (row0 < m && col < n) {
-              const int dst = KIND == kTN ? col / n_per : 0;
-              if constexpr (KIND == kRed) tma_reduce_add_2d(&tmap_c.m[0], buf, col, row0);
-              else tma_store_2d(&tmap_c.m[dst], buf, col - dst * n_per, row0);
-            } else asm volatile("cp.async.bulk.commit_group;" ::: "memory");     // keep the group count in step
-          }
-          ++nstore;
+          const int dst = KIND == kTN ? col / n_per : 0;
+          const uint8_t* buf = stage(v, &tmap_c.m[dst], col - dst * n_per, row0 < m && col < n);
           if (STATS && st != nullptr) {
             // column sums of the staged (rounded) block: lane owns columns 2*lane, 2*lane+1; rows past the
             // matrix edge hold exact zeros (their A rows were zero-filled)
@@ -434,7 +462,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
         if (chunk(0, cs[0]) && chunk(64, cs[1]) && chunk(128, cs[2])) chunk(192, cs[3]);
       } else {
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += kCols)
+        for (int c0 = KIND == kGelu ? group * kCols : 0; c0 < BN; c0 += kCols * (epi_warps(KIND) / 4))
           if (!chunk(c0, nullptr)) break;
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -551,13 +579,15 @@ int launch_bn(const Args& p, int dev, int max_pairs, cudaStream_t stream) {
     const void* a = p.a[i];
     if (!(KIND == kRed ? make_map(&ta.m[i], a, p.k, a_src, p.lda, 64) : make_map(&ta.m[i], a, p.m, a_src, p.lda, BM))) return -6;
   }
-  if (!(KIND == kTN ? make_map(&tb, p.b, p.n, p.k, p.ldb, BN / 2) : make_map(&tb, p.b, p.k, p.n, p.ldb, 64))) return -6;
+  constexpr bool kBmn = KIND == kNN || KIND == kRed;
+  if (!(kBmn ? make_map(&tb, p.b, p.k, p.n, p.ldb, 64) : make_map(&tb, p.b, p.n, p.k, p.ldb, BN / 2))) return -6;
   CMaps tc;
-  const int n_per = p.n / p.n_dst;
+  const int n_per = KIND == kGelu ? p.n : p.n / p.n_dst;
   int tma_store = 1;
   for (int i = 0; i < kMaxCDst; ++i) {
     if (i >= p.n_dst) { tc.m[i] = tc.m[0]; continue; }
     void* c = p.c[i];
+    if (c == nullptr) c = p.c[1];                       // (kGelu without C0)
     tc.m[i] = tb;               // placeholder when C cannot be described (the kernel then stores directly)
     if ((((uintptr_t)c & 15) != 0) || ((p.ldc * (int)sizeof(OutT)) % 16 != 0) ||
         !make_store_map(&tc.m[i], c, p.m, n_per, p.ldc, sizeof(OutT) == 2))
@@ -577,7 +607,7 @@ int launch_bn(const Args& p, int dev, int max_pairs, cudaStream_t stream) {
   const int pairs = max_pairs > num_items ? num_items : max_pairs;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.blockDim = dim3(64 + 32 * epi_warps(KIND), 1, 1);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -587,7 +617,7 @@ int launch_bn(const Args& p, int dev, int max_pairs, cudaStream_t stream) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, p.n_src > 1 ? (KIND == kRed ? a_src : a_src / BK) : 0x7fffffff, tb, tc, p.n_dst > 1 ? n_per : 0x7fffffff, tma_store,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, p.n_src > 1 ? (KIND == kRed ? a_src : a_src / BK) : 0x7fffffff, tb, tc, KIND == kTN && p.n_dst > 1 ? n_per : 0x7fffffff, tma_store,
                                      (OutT*)p.c[0], p.bias,
                                      p.m, p.n, p.k, p.ldc, p.epi, splits, p.col_sums, p.seg_rows, p.status);
   return (int)e;
@@ -611,8 +641,8 @@ int launch(const Args& p, cudaStream_t stream) {
     return p.n > 128 ? launch_bn<OutT, STATS, 256, KIND>(p, dev, pairs, stream)
                      : launch_bn<OutT, STATS, 128, KIND>(p, dev, pairs, stream);
   } else if constexpr (!STATS) {
-    const int bn = pick_bn(p.m, p.n, pairs, KIND == kTN ? 64 : 128);   // MN-major B: halves of whole 64-column boxes
-    if constexpr (KIND == kTN) {
+    const int bn = pick_bn(p.m, p.n, pairs, KIND == kNN ? 128 : 64);   // MN-major B: halves of whole 64-column boxes
+    if constexpr (KIND != kNN) {
       if (bn == 64) return launch_bn<OutT, STATS, 64, KIND>(p, dev, pairs, stream);
     }
     if (bn == 128) return launch_bn<OutT, STATS, 128, KIND>(p, dev, pairs, stream);
@@ -638,6 +668,19 @@ int tsp_gemm_bf16_tn_2cta(const void* a, const void* b, void* c, const float* bi
   if (((uintptr_t)a | (uintptr_t)b) & 15) return -2;
   const Args p = {{a, nullptr, nullptr}, 1, b, {c, nullptr, nullptr}, 1, bias, m, n, k, lda, ldb, ldc, epi, nullptr, 1, status};
   return out_dtype == TSP_DTYPE_BF16 ? launch<__nv_bfloat16, false>(p, stream) : launch<float, false>(p, stream);
+}
+
+// h[m,n] (bf16, optional) = A[m,k] * B[n,k]^T, act[m,n] (bf16) = gelu(h + bias[n]) of the rounded h: a linear layer and its
+// activation in one pass.  n a multiple of 64, bias 16-byte aligned.  B200: 12608 x 3072 x 768 with
+// both outputs 77 us against 54 + 34 for product and activation, 16384 rows without h 88 against 65 + 43.
+int tsp_gemm_bf16_tn_gelu_2cta(const void* a, const void* b, void* h, void* act, const float* bias, int m, int n, int k,
+                               int lda, int ldb, int ldc, int* status, cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (k % 8) || n % 64 != 0 || bias == nullptr || act == nullptr) return -3;
+  if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)h | (uintptr_t)act | (uintptr_t)bias) & 15) return -2;
+  const Args p = {{a, nullptr, nullptr}, 1, b, {h, act, nullptr}, 2, bias, m, n, k, lda, ldb, ldc, h != nullptr ? 1 : 0,
+                  nullptr, 1, status};
+  return launch<__nv_bfloat16, false, kGelu>(p, stream);
 }
 
 // [C0 | C1 | C2] = A[m,k] * B[n,k]^T (+ bias[n]), bf16: one product whose n columns go to n_dst matrices of n / n_dst

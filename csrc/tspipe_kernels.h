@@ -122,6 +122,8 @@ int tsp_gemm_bf16_tn_stats(const void* a, const void* b, void* c, int m, int n, 
                            float* col_sums, int segs, int* status, cudaStream_t stream);
 
 // ---- gemm_tcgen05_2cta.cu -----------------------------------------------------------------------------------------
+int tsp_gemm_bf16_tn_gelu_2cta(const void* a, const void* b, void* h, void* act, const float* bias, int m, int n, int k,
+                               int lda, int ldb, int ldc, int* status, cudaStream_t stream);
 int tsp_gemm_bf16_tn_2cta_split(const void* a, const void* b, void* const* c, int n_dst, const float* bias, int m, int n,
                                 int k, int lda, int ldb, int ldc, int* status, cudaStream_t stream);
 int tsp_gemm_bf16_nn_2cta(const void* const* a, int n_src, const void* b, void* c, int m, int n, int k, int lda, int ldb,

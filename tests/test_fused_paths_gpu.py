@@ -294,6 +294,24 @@ def test_fused_qkv_projection_matches_three_linears(rows, c, heads, bias):
         assert _rel(a, r) < EPS[torch.bfloat16]
 
 
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("m,n,k", [(128, 64, 64), (300, 192, 128), (1000, 3072, 768)])
+def test_linear_gelu_epilogue_equals_the_separate_kernel(m, n, k, grad):
+    from tspipe_b200.ops import fused, gemm
+    torch.manual_seed(16)
+    x = torch.randn(m, k, device=DEV).bfloat16().requires_grad_(grad)
+    w = (torch.randn(n, k, device=DEV) * 2 / math.sqrt(k)).requires_grad_(grad)
+    b = torch.randn(n, device=DEV, requires_grad=grad)
+    y, ref = gemm.linear_gelu(x, w, b), fused.gelu(gemm.linear(x, w, None), b)
+    gemm.check_status()
+    assert _rel(y, ref) < 1e-4                         # the same roundings
+    if grad:
+        g = torch.randn_like(y)
+        for p, q in zip(torch.autograd.grad(y, [x, w, b], g), torch.autograd.grad(ref, [x, w, b], g)):
+            assert _rel(p, q) < 1e-4
+        gemm.check_status()
+
+
 @pytest.mark.parametrize("n,h,w", [(1, 8, 8), (3, 10, 24), (2, 32, 224), (5, 64, 96)])
 def test_stem_weight_gradient(n, h, w):
     from tspipe_b200.ops import conv, gemm

@@ -24,9 +24,8 @@ import torch.nn.functional as F
 from torch import nn
 
 from ..model_wrapper import TSPipeModelWrapper
-from ..ops import fused
 from ..ops.attention import attention, project_qkv
-from ..ops.linear import linear
+from ..ops.linear import linear, linear_gelu
 from .vit import LayerNorm, norm_of_sum
 
 
@@ -91,7 +90,7 @@ class EncoderLayer(nn.Module):
         key_mask = mask.to(torch.bool)[:, None, None, :]
         a = attention(q, k, v, key_mask).transpose(1, 2).reshape(b, l, c)
         _, x = norm_of_sum(self.norm1, x, self.drop(linear(a, self.out.weight, self.out.bias)), need_sum=False)
-        h = fused.gelu(linear(x, self.fc1.weight, None), self.fc1.bias)
+        h = linear_gelu(x, self.fc1.weight, self.fc1.bias)
         _, x = norm_of_sum(self.norm2, x, self.drop(linear(h, self.fc2.weight, self.fc2.bias)), need_sum=False)
         return {"hidden": x, "mask": mask}
 
@@ -108,7 +107,7 @@ class MlmHead(nn.Module):
 
     def forward(self, s: Dict[str, torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor]:
         x = s["hidden"]
-        h = self.norm(fused.gelu(linear(x, self.dense.weight, None), self.dense.bias))
+        h = self.norm(linear_gelu(x, self.dense.weight, self.dense.bias))
         w, b = self.decoder.weight, self.decoder.bias
         pad = (-w.shape[0]) % 8
         if h.is_cuda and pad:

@@ -27,7 +27,7 @@ from torch import nn
 
 from ..ops import fused
 from ..ops.attention import attention, packed_attention, project_qkv, qkv_mode
-from ..ops.linear import linear
+from ..ops.linear import linear, linear_gelu
 
 
 @dataclass
@@ -160,8 +160,7 @@ class Mlp(nn.Module):
         self.fc2 = nn.Linear(hidden, dim)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        h = linear(x, self.fc1.weight, None)
-        h = fused.gelu(h, self.fc1.bias)            # bias add fused into the activation kernel
+        h = linear_gelu(x, self.fc1.weight, self.fc1.bias)
         return linear(h, self.fc2.weight, self.fc2.bias)
 
 

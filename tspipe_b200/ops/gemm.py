@@ -278,6 +278,66 @@ class _LinearQKV(torch.autograd.Function):
         return dx, dw, db
 
 
+class _LinearGelu(torch.autograd.Function):
+    """``gelu(x W^T + b)``: the GEMM's epilogue forms the activation from the rounded product, which is kept for the backward
+    only.  Backward: the activation's derivative as one elementwise pass, then the linear layer's products."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, grads):
+        x2 = _bf16_rows(x, x.shape[-1])
+        (m, k), n = x2.shape, weight.shape[0]
+        bf = bias.detach().float().contiguous()
+        if bf.data_ptr() % 16:
+            bf = bf.clone()
+        act = torch.empty((m, n), dtype=torch.bfloat16, device=x2.device)
+        h = torch.empty_like(act) if grads and any(ctx.needs_input_grad) else None
+        with _f.on_device(x2.device):
+            code = _f.lib().tsp_gemm_bf16_tn_gelu_2cta(_f._ptr(x2), _f._ptr(_w16(weight)), _f._ptr(h), _f._ptr(act),
+                                                       _f._ptr(bf), _c.c_int(m), _c.c_int(n), _c.c_int(k), _c.c_int(k),
+                                                       _c.c_int(k), _c.c_int(n), _f._ptr(_status_word(x2.device)),
+                                                       _f._stream())
+        _f._check(code, "tsp_gemm_bf16_tn_gelu_2cta")
+        _f._count()
+        if h is not None:
+            ctx.save_for_backward(x2, weight, h, bf)
+        ctx.in_shape, ctx.dtypes = x.shape, (x.dtype, weight.dtype, bias.dtype)
+        ctx.bias = bias if _f.IN_CAPTURE else None
+        return act.view(*x.shape[:-1], n)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x2, weight, h, bf = ctx.saved_tensors
+        n, k = weight.shape
+        dy2 = _bf16_rows(dy, n)
+        dh = torch.empty_like(h)
+        with _f.on_device(h.device):
+            _f._check(_f.lib().tsp_gelu_bwd(_f._ptr(dy2), _f._ptr(h), _f._ptr(bf), _f._ptr(dh), _c.c_int64(h.numel()),
+                                            _c.c_int(n), _c.c_int(_f._dt(h)), _f._stream()), "tsp_gelu_bwd")
+        _f._count()
+        dx = dw = db = None
+        if ctx.needs_input_grad[0]:
+            dx = matmul_nn([dh], _w16(weight)).view(ctx.in_shape)
+            if ctx.dtypes[0] != torch.bfloat16:
+                dx = dx.to(ctx.dtypes[0])
+        if ctx.needs_input_grad[1]:
+            target = _grad_target(weight)
+            if target is None:
+                target = torch.zeros((n, k), dtype=torch.float32, device=x2.device)
+                dw = target
+            _add_weight_grad(target, [dh], x2)
+            if dw is not None and weight.dtype != torch.float32:
+                dw = target.to(weight.dtype)
+        if ctx.needs_input_grad[2]:
+            db = _column_sums(dh, add_to=_f.recorded_grad(ctx.bias))
+            db = None if db is None else db.to(ctx.dtypes[2])
+        return dx, dw, db, None
+
+
+def linear_gelu(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
+    """``gelu(x @ weight^T + bias)``; see :class:`_LinearGelu`."""
+    return _LinearGelu.apply(x, weight, bias, torch.is_grad_enabled())
+
+
 def linear_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None):
     """``(q, k, v)`` of a fused projection ``weight [3C, K]``; see :class:`_LinearQKV`."""
     return _LinearQKV.apply(x, weight, bias)

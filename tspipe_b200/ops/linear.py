@@ -40,3 +40,14 @@ def linear_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
         if gemm.eligible(x, weight[:weight.shape[0] // 3]):
             return gemm.linear_qkv(x, weight, bias)
     return None
+
+
+def linear_gelu(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
+    """``gelu(x @ weight^T + bias)`` (erf form): the activation in the GEMM's epilogue on the tcgen05 path, the linear layer
+    followed by the fused bias + GELU kernel otherwise."""
+    if _USE_TCGEN05 and x.is_cuda and bias is not None:
+        from . import gemm
+        if gemm._two_cta and gemm.eligible(x, weight):
+            return gemm.linear_gelu(x, weight, bias)
+    from . import fused
+    return fused.gelu(linear(x, weight, None), bias)
