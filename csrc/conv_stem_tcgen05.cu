@@ -29,6 +29,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 #include "tspipe_kernels.h"
 
 extern int g_tsp_sm_reserve;          // defined in peer.cu
@@ -643,17 +644,12 @@ int tsp_conv_stem_wgrad(const void* x, const void* dy, float* dw, int n, int h, 
   if ((h & 1) || (w & 7) || w > 224 || h < 8 || w < 8) return -3;
   if ((((uintptr_t)x | (uintptr_t)dy) & 15) != 0) return -2;
   const int oh = h / 2, ow = w / 2;
-  EncodeTiledFn enc = get_encode();
-  if (enc == nullptr) return -6;
   CUtensorMap td;
   {
     cuuint64_t dims[3] = {(cuuint64_t)kCout, (cuuint64_t)ow, (cuuint64_t)n * oh};
     cuuint64_t strides[2] = {(cuuint64_t)kCout * 2, (cuuint64_t)ow * kCout * 2};
     cuuint32_t box[3] = {(cuuint32_t)kCout, 128, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    if (enc(&td, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(dy), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    if (!tc5::encode_tiled(&td, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, dy, 3, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_L2_256B))
       return -6;
   }
   static bool attr_set[64] = {};

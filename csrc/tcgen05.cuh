@@ -225,26 +225,33 @@ inline EncodeTiledFn get_encode() {
   return fn;
 }
 
-// bf16 tensor of up to 4 dimensions, innermost first: dims[i] elements, strides[i] BYTES for i >= 1 (the innermost
-// dimension is contiguous), box[i] elements.  128-byte swizzle: box[0] must be 64.  Out-of-range elements read as 0.
-inline bool make_bf16_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
-                          const uint32_t* box) {
+// Tensor map with a 128-byte swizzle and zeros out of range.
+inline bool encode_tiled(CUtensorMap* map, CUtensorMapDataType type, const void* base, int rank, const cuuint64_t* dims,
+                         const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapL2promotion promotion) {
   EncodeTiledFn enc = get_encode();
   if (enc == nullptr) return false;
-  cuuint64_t d[4], s[3];
-  cuuint32_t b[4], e[4];
-  for (int i = 0; i < rank; ++i) { d[i] = dims[i]; b[i] = box[i]; e[i] = 1; }
-  for (int i = 1; i < rank; ++i) s[i - 1] = strides[i];
+  const cuuint32_t e[4] = {1, 1, 1, 1};
   CUresult r = CUDA_ERROR_UNKNOWN;
-  for (int attempt = 0; attempt < 2 && r != CUDA_SUCCESS; ++attempt) {
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    r = enc(map, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     // The encoder is a driver call and wants a current context.  A thread that has not made a runtime call yet (an
     // autograd worker calling straight into this library) has none: bind the device's primary context and retry.
-    if (attempt == 1) (void)cudaFree(nullptr);
-    r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r == CUDA_SUCCESS) break;
+    if (attempt == 0) (void)cudaFree(nullptr);
   }
   return r == CUDA_SUCCESS;
+}
+
+// bf16 tensor of up to 4 dimensions, innermost first: dims[i] elements, strides[i] BYTES for i >= 1 (the innermost
+// dimension is contiguous), box[i] elements; box[0] must be 64.
+inline bool make_bf16_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
+                          const uint32_t* box) {
+  cuuint64_t d[4], s[3];
+  cuuint32_t b[4];
+  for (int i = 0; i < rank; ++i) { d[i] = dims[i]; b[i] = box[i]; }
+  for (int i = 1; i < rank; ++i) s[i - 1] = strides[i];
+  return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, rank, d, s, b, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
 }  // namespace tc5

@@ -312,6 +312,31 @@ def test_linear_gelu_epilogue_equals_the_separate_kernel(m, n, k, grad):
         gemm.check_status()
 
 
+def test_products_on_a_thread_that_has_made_no_runtime_call():
+    """Autograd's worker may enter the library with no device context bound: tensor maps have to be made all the same."""
+    import threading
+    from tspipe_b200.ops import gemm
+    a = torch.randn(256, 128, device=DEV).bfloat16()
+    b = torch.randn(128, 192, device=DEV).bfloat16()
+    target = torch.zeros(128, 128, device=DEV)
+    want = gemm.matmul_nn([a], b)
+    out, errors = [], []
+
+    def work():
+        try:
+            gemm._add_weight_grad(target, [a], a)
+            out.append(gemm.matmul_nn([a], b))
+        except Exception as e:                         # noqa: BLE001
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert not errors, errors
+    assert torch.equal(out[0], want) and _rel(target, a.double().t() @ a.double()) < 1e-5
+
+
 @pytest.mark.parametrize("n,h,w", [(1, 8, 8), (3, 10, 24), (2, 32, 224), (5, 64, 96)])
 def test_stem_weight_gradient(n, h, w):
     from tspipe_b200.ops import conv, gemm
