@@ -581,25 +581,110 @@ __global__ void __launch_bounds__(kBlock, 3) bn_bwd_apply_kernel(const T* __rest
 // ---------------------------------------------------------------------------------------------
 // BatchNorm + ReLU + 3x3 / stride 2 / pad 1 max-pool (the ResNet stem) without the normalised activation in memory.
 //
-// Forward: one pass reads x and writes the pooled rows and the winning tap (0..8) of every output, a byte; values are
-// rounded to T before they are compared and the first maximum in (row, column) order wins, so the result is that of
-// the two separate passes.  A thread walks kPoolRows output rows of one column and 4 channels and forms each input
-// row's maximum over the three columns once (an odd row is the last of one window and the first of the next); the next
-// row is on its way meanwhile.
+// The passes are bound by the arithmetic on every element of x as much as by memory, so it is kept short.
+// Forward: a value and its tap travel as one integer key, the value's bits (not negative behind the ReLU, so they order
+// as integers) above a code that is larger for an earlier tap: the maximum of the keys is the first maximum in (row,
+// column) order, one instruction for three values.  Values are rounded to T before they are compared, so the result is
+// that of the separate passes.  A thread walks kPoolRows output rows of one column and 8 channels and forms each input
+// row's maximum over the three columns once (an odd row is the last of one window and the first of the next).  idx gets
+// the code of the winner, kNoTap where the maximum is zero: there the ReLU passes no gradient.
 // Backward: dy' of an input pixel is gathered from the <= 4 windows it belongs to where it is needed, in the reduction
 // and again in the pass for dx, instead of being scattered to an activation-sized tensor that both would read.  A
-// thread takes a 2 x 2 block of input pixels, which meets exactly the four windows (a, b) .. (a + 1, b + 1).
-// Four channels per thread: the arithmetic (nine taps per block) needs more warps than eight would leave registers for.
-// 256 images of 112 x 112 x 64 bf16 (205 MB), B200: forward 178 us as two passes, 139 as one; backward 410 as three, 320 as two.
+// thread takes a 2 x 2 block of input pixels, which meets exactly the four windows (a, b) .. (a + 1, b + 1), two channels
+// at a time.
+// A block is kBlock / (c / 8) pixels by all channels (by 2048 of them, blockIdx.z, where there are more).
+// 256 images of 112 x 112 x 64 bf16 (205 MB), B200: forward 178 us as two passes, 139 with a comparison per value, 91 this
+// way; backward 410 us as three passes, 320 with the ReLU mask recomputed from x and one 64-bit division per item, 190.
 // ---------------------------------------------------------------------------------------------
 constexpr int kPoolRows = 4;
+constexpr uint32_t kNoTap = 0xff;
+__host__ __device__ constexpr uint32_t tap_code(int ky, int kx) { return (uint32_t)((2 - ky) * 4 + 2 - kx); }
+
+// Unsigned division of numbers below 2^31 by a constant of the launch: multiply-high and shift (Granlund and Montgomery).
+struct FastDiv {
+  uint32_t d, mul, shift;
+  explicit FastDiv(uint32_t div = 1) : d(div), mul(0), shift(0) {
+    while ((1ull << shift) < d) ++shift;
+    mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(mul, n) + n) >> shift; }
+};
 
 struct PoolGeom {
   int n, h, w, c, ho, wo;      // images of one segment, extents
+  FastDiv by_wo, by_rows;      // by_rows: strips of kPoolRows output rows (forward), output rows (backward)
+  uint32_t items;              // pixels or strips of pixels of one segment
+};
+
+// Elements 2j and 2j + 1 of a raw vector.
+__device__ __forceinline__ float2 get2(const tsp::Raw8<__nv_bfloat16>& r, int j) {
+  const uint32_t u = reinterpret_cast<const uint32_t*>(&r.a)[j];
+  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+__device__ __forceinline__ float2 get2(const tsp::Raw8<float>& r, int j) { return reinterpret_cast<const float2*>(&r)[j]; }
+__device__ __forceinline__ void set2(tsp::Raw8<__nv_bfloat16>& r, int j, float2 v) {
+  reinterpret_cast<__nv_bfloat162*>(&r.a)[j] = __floats2bfloat162_rn(v.x, v.y);
+}
+__device__ __forceinline__ void set2(tsp::Raw8<float>& r, int j, float2 v) { reinterpret_cast<float2*>(&r)[j] = v; }
+template <typename T>
+__device__ __forceinline__ float2 round2(float2 v) {
+  if constexpr (sizeof(T) == 2) v = __bfloat1622float2(__floats2bfloat162_rn(v.x, v.y));
+  return v;
+}
+
+// Keys of max(v, 0) for two values: bf16 bits << 16 | code, fp32 bits << 32 | code.
+template <typename T> struct PoolKey;
+template <> struct PoolKey<__nv_bfloat16> {
+  using K = uint32_t;
+  static __device__ __forceinline__ void make(float2 v, uint32_t code, K& k0, K& k1) {
+    const __nv_bfloat162 p = __hmax2(__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(0.f, 0.f));
+    const uint32_t u = *reinterpret_cast<const uint32_t*>(&p);
+    k0 = __byte_perm(u, code, 0x1054);
+    k1 = __byte_perm(u, code, 0x3254);
+  }
+  static __device__ __forceinline__ K max3(K a, K b, K c) { return __vimax3_u32(a, b, c); }
+  static __device__ __forceinline__ bool zero(K k) { return k < 0x10000u; }
+  static __device__ __forceinline__ void set2(tsp::Raw8<__nv_bfloat16>& r, int j, K k0, K k1) {
+    reinterpret_cast<uint32_t*>(&r.a)[j] = __byte_perm(k0, k1, 0x7632);
+  }
+};
+template <> struct PoolKey<float> {
+  using K = unsigned long long;
+  static __device__ __forceinline__ void make(float2 v, uint32_t code, K& k0, K& k1) {
+    k0 = (K)__float_as_uint(fmaxf(v.x, 0.f) + 0.f) << 32 | code;
+    k1 = (K)__float_as_uint(fmaxf(v.y, 0.f) + 0.f) << 32 | code;
+  }
+  static __device__ __forceinline__ K max3(K a, K b, K c) { return max(max(a, b), c); }
+  static __device__ __forceinline__ bool zero(K k) { return (k >> 32) == 0; }
+  static __device__ __forceinline__ void set2(tsp::Raw8<float>& r, int j, K k0, K k1) {
+    reinterpret_cast<float2*>(&r)[j] = make_float2(__uint_as_float((uint32_t)(k0 >> 32)), __uint_as_float((uint32_t)(k1 >> 32)));
+  }
+};
+template <typename T>
+__device__ __forceinline__ void st_raw(T* p, int64_t i, const tsp::Raw8<T>& r) {
+  if constexpr (sizeof(T) == 2) {
+    *reinterpret_cast<uint4*>(p + i) = r.a;
+  } else {
+    *reinterpret_cast<float4*>(p + i) = r.a;
+    *reinterpret_cast<float4*>(p + i + 4) = r.b;
+  }
+}
+
+// The channel vector and the first pixel of a thread, the pixels of a block.
+struct PoolThread {
+  int per_block, slot, vec;
+  bool active;
+  __device__ __forceinline__ explicit PoolThread(int cpv) {
+    const int width = min(cpv, kBlock);
+    per_block = kBlock / width;
+    slot = threadIdx.x / width;
+    vec = blockIdx.z * kBlock + threadIdx.x % width;
+    active = slot < per_block && vec < cpv;
+  }
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_kernel(const T* __restrict__ x, T* __restrict__ y,
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 2 ? 3 : 2) bn_relu_pool_kernel(const T* __restrict__ x, T* __restrict__ y,
                                                               uint8_t* __restrict__ idx, const float* __restrict__ sums,
                                                               const float* __restrict__ wgt,
                                                               const float* __restrict__ bias,
@@ -607,6 +692,8 @@ __global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_kernel(const T* __rest
                                                               float* __restrict__ acc_sum, float* __restrict__ acc_sumsq,
                                                               float* __restrict__ acc_count, int64_t acc_seg_stride,
                                                               const PoolGeom g, float eps) {
+  using P = PoolKey<T>;
+  using K = typename P::K;
   {   // blockIdx.y = segment
     const int64_t seg = blockIdx.y;
     x += seg * g.n * g.h * g.w * g.c;
@@ -617,111 +704,112 @@ __global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_kernel(const T* __rest
     if (acc_sum != nullptr) { acc_sum += seg * acc_seg_stride; acc_sumsq += seg * acc_seg_stride; }
     if (acc_count != nullptr) acc_count += seg * acc_seg_stride;
   }
-  const int c = g.c, cpv = c >> 2, strips = (g.ho + kPoolRows - 1) / kPoolRows;
-  const int64_t total = (int64_t)g.n * strips * g.wo * cpv;
-  const int64_t stride = (int64_t)gridDim.x * kBlock;
-  const int first = blockIdx.x * kBlock + threadIdx.x;
-  if (first >= total) return;
-  const int ch = (first % cpv) * 4;             // the grid stride is a multiple of c/4
-  float sc[4], sh[4];
+  const int c = g.c;
+  const PoolThread th(c >> 3);
+  if (!th.active) return;
+  const int ch = th.vec * 8;
+  float sc[8], sh[8];
   {
     const float rows = (float)((int64_t)g.n * g.h * g.w), inv_m = 1.f / rows;
+    float s[8], q[8], wv[8], bv[8];
+    tsp::ld8(sums, ch, s);
+    tsp::ld8(sums + c, ch, q);
+    tsp::ld8(wgt, ch, wv);
+    tsp::ld8(bias, ch, bv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float s = sums[ch + e], q = sums[c + ch + e];
-      const float mean = s * inv_m, rstd = rsqrtf(fmaxf(q * inv_m - mean * mean, 0.f) + eps);
-      if (first < cpv) {
-        if (acc_sum != nullptr) { acc_sum[ch + e] += s; acc_sumsq[ch + e] += q; }
+    for (int e = 0; e < 8; ++e) {
+      const float mean = s[e] * inv_m, rstd = rsqrtf(fmaxf(q[e] * inv_m - mean * mean, 0.f) + eps);
+      if (blockIdx.x == 0 && th.slot == 0) {
+        if (acc_sum != nullptr) { acc_sum[ch + e] += s[e]; acc_sumsq[ch + e] += q[e]; }
         if (acc_count != nullptr) acc_count[ch + e] += rows;
         save_mean_rstd[ch + e] = mean;
         save_mean_rstd[c + ch + e] = rstd;
       }
-      sc[e] = wgt[ch + e] * rstd;
-      sh[e] = bias[ch + e] - mean * sc[e];
+      sc[e] = wv[e] * rstd;
+      sh[e] = bv[e] - mean * sc[e];
     }
   }
-  for (int64_t i = first; i < total; i += stride) {
-    uint32_t p = (uint32_t)(i / cpv);
-    const int ox = (int)(p % (uint32_t)g.wo);
-    p /= (uint32_t)g.wo;
-    const int oy0 = (int)(p % (uint32_t)strips) * kPoolRows;
-    const int img = (int)(p / (uint32_t)strips);
-    const int ix0 = 2 * ox - 1, iy0 = 2 * oy0 - 1;
-    const bool left = ix0 >= 0, right = ix0 + 2 < g.w;
-    const T* xi = x + (int64_t)img * g.h * g.w * c + ch;
-    const int64_t o0 = (((int64_t)img * g.ho + oy0) * g.wo + ox) * c + ch;
-    // input rows iy0 .. iy0 + 2 kPoolRows that exist and that a window of this strip needs
-    const int rows = min(g.h - iy0, 2 * min(kPoolRows, g.ho - oy0) + 1);
-    auto load = [&](int r, tsp::Raw4<T> (&raw)[3]) {
-      const T* row = xi + ((int64_t)(iy0 + r) * g.w + ix0) * c;
-      if (left) tsp::ldraw(row, 0, raw[0]);
-      tsp::ldraw(row, c, raw[1]);
-      if (right) tsp::ldraw(row, 2 * (int64_t)c, raw[2]);
+  const int pitch = g.w * c;                     // (below 2^31: n * h * w is)
+  for (uint32_t i = blockIdx.x * th.per_block + th.slot; i < g.items; i += gridDim.x * th.per_block) {
+    const uint32_t strip = g.by_wo.div(i), img = g.by_rows.div(strip);
+    const int ox = (int)(i - strip * g.by_wo.d), oy0 = (int)(strip - img * g.by_rows.d) * kPoolRows;
+    const bool left = ox > 0, right = 2 * ox + 1 < g.w;
+    const T* xi = x + ((int64_t)img * g.h + 2 * oy0) * pitch + (2 * ox) * c + ch;      // the centre of the first window
+    int64_t o = (((int64_t)img * g.ho + oy0) * g.wo + ox) * c + ch;
+    auto load = [&](const T* row, tsp::Raw8<T> (&raw)[3]) {
+      if (left) tsp::ldraw(row, -c, raw[0]);
+      tsp::ldraw(row, 0, raw[1]);
+      if (right) tsp::ldraw(row, c, raw[2]);
     };
-    tsp::Raw4<T> cur[3], nxt[3];
-    float best[4], m[4];                         // maximum of the current window and of the current row
-    uint32_t arg = 0, col = 0;                   // their taps and columns, a byte per channel
+    // largest key of a row over the window's columns; a column that does not exist has the smallest key
+    auto row_keys = [&](const tsp::Raw8<T> (&raw)[3], K (&m)[8]) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) best[e] = -INFINITY;
-    if (iy0 >= 0) load(0, cur);
-    load(1, nxt);                                // (row 2 * oy0 always exists)
+      for (int j = 0; j < 4; ++j) {
+        K k[3][2];
 #pragma unroll
-    for (int r = 0; r <= 2 * kPoolRows; ++r) {
-      if (r > 0) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) cur[k] = nxt[k];
-        if (r + 1 < rows) load(r + 1, nxt);
+        for (int kx = 0; kx < 3; ++kx) {
+          const float2 v = get2(raw[kx], j);
+          P::make(make_float2(v.x * sc[2 * j] + sh[2 * j], v.y * sc[2 * j + 1] + sh[2 * j + 1]), (uint32_t)(2 - kx), k[kx][0],
+                  k[kx][1]);
+        }
+        if (!left) k[0][0] = k[0][1] = 0;
+        if (!right) k[2][0] = k[2][1] = 0;
+        m[2 * j] = P::max3(k[0][0], k[1][0], k[2][0]);
+        m[2 * j + 1] = P::max3(k[0][1], k[1][1], k[2][1]);
       }
-      const bool have = r < rows && (r > 0 || iy0 >= 0);
-      if (have) {
+    };
+    tsp::Raw8<T> raw0[3] = {}, raw1[3] = {};
+    K top[8];                                    // the row above the window's centre
 #pragma unroll
-        for (int e = 0; e < 4; ++e) m[e] = -INFINITY;
-        col = 0;
+    for (int e = 0; e < 8; ++e) top[e] = 0;
+    if (oy0 > 0) {
+      load(xi - pitch, raw0);
+      row_keys(raw0, top);
+    }
+#pragma unroll 1
+    for (int oy = oy0; oy < oy0 + kPoolRows && oy < g.ho; ++oy) {
+      const bool below = 2 * oy + 1 < g.h;       // an odd height ends in a window of two rows
+      load(xi, raw0);
+      if (below) load(xi + pitch, raw1);
+      K mid[8], low[8];
+      row_keys(raw0, mid);
 #pragma unroll
-        for (int kx = 0; kx < 3; ++kx)
-          if (kx == 1 || (kx == 0 ? left : right)) {
-            float v[4];
-            tsp::cvt4(cur[kx], v);
+      for (int e = 0; e < 8; ++e) low[e] = 0;
+      if (below) row_keys(raw1, low);
+      tsp::Raw8<T> out;
+      uint32_t code[2] = {0, 0};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = fmaxf(v[e] * sc[e] + sh[e], 0.f);
-            tsp::round_as<T>(v);
+      for (int j = 0; j < 4; ++j) {
+        K k[2];
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (v[e] > m[e]) { m[e] = v[e]; col = (col & ~(0xffu << (8 * e))) | ((uint32_t)kx << (8 * e)); }
-          }
-        const uint32_t tap = r == 0 ? 0u : (r & 1) ? 3u : 6u;              // first tap of this row in the current window
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (m[e] > best[e]) {
-            best[e] = m[e];
-            arg = (arg & ~(0xffu << (8 * e))) | ((col & (0xffu << (8 * e))) + (tap << (8 * e)));
-          }
+        for (int s = 0; s < 2; ++s) {
+          const int e = 2 * j + s;
+          k[s] = P::max3(top[e] | 8u, mid[e] | 4u, low[e]);
+          top[e] = low[e];
+          code[e >> 2] |= (P::zero(k[s]) ? kNoTap : (uint32_t)k[s] & 15u) << (8 * (e & 3));
+        }
+        P::set2(out, j, k[0], k[1]);
       }
-      if (r > 0 && (r & 1) == 0 && r - 1 < rows) {                         // the window's last row (which may not exist)
-        const int64_t o = o0 + (int64_t)(r / 2 - 1) * g.wo * c;
-        tsp::st4(y, o, best);
-        if (idx != nullptr) *reinterpret_cast<uint32_t*>(idx + o) = arg;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) best[e] = m[e];                        // the odd row opens the next window
-        arg = col;
-      }
+      st_raw(y, o, out);
+      if (idx != nullptr) *reinterpret_cast<uint2*>(idx + o) = make_uint2(code[0], code[1]);
+      xi += 2 * (int64_t)pitch;
+      o += (int64_t)g.wo * c;
     }
   }
 }
 
 // APPLY false: sums[seg] += (sum dy', sum dy' * xhat).  APPLY true: dx from those sums.
 template <typename T, bool APPLY>
-__global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_bwd_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ idx,
+__global__ void __launch_bounds__(kBlock, 2) bn_relu_pool_bwd_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ idx,
                                                                   const T* __restrict__ x,
                                                                   const float* __restrict__ mean_rstd,
                                                                   const float* __restrict__ wgt,
-                                                                  const float* __restrict__ bias,
                                                                   float* __restrict__ sums, T* __restrict__ dx,
                                                                   float* __restrict__ gw, float* __restrict__ gb,
                                                                   const PoolGeom g) {
-  constexpr int pitch = kBlock + 8;
-  __shared__ float sm[APPLY ? 1 : 8 * pitch];
-  const int c = g.c, cpv = c >> 2;
+  constexpr int sm_pitch = kBlock + 8;
+  __shared__ float sm[APPLY ? 1 : 16 * sm_pitch];
+  const int c = g.c;
   {   // blockIdx.y = segment
     const int64_t seg = blockIdx.y, in = seg * g.n * g.h * g.w * c, outs = seg * g.n * g.ho * g.wo * c;
     x += in;
@@ -731,113 +819,118 @@ __global__ void __launch_bounds__(kBlock, 3) bn_relu_pool_bwd_kernel(const T* __
     mean_rstd += seg * 2 * c;
     sums += seg * 2 * c;
   }
-  const int64_t total = (int64_t)g.n * g.ho * g.wo * cpv;
-  const int64_t stride = (int64_t)gridDim.x * kBlock;
-  const int first = blockIdx.x * kBlock + threadIdx.x;
-  const int ch = (first % cpv) * 4;
-  if (APPLY && gw != nullptr && blockIdx.y == 0 && first < cpv) {
-    for (int e = 0; e < 4; ++e) {
+  const PoolThread th(c >> 3);
+  const int ch = th.vec * 8;
+  if (APPLY && !th.active) return;
+  if (APPLY && gw != nullptr && blockIdx.y == 0 && blockIdx.x == 0 && th.slot == 0) {
+    for (int e = 0; e < 8; ++e) {
       float db = 0.f, dw = 0.f;
       for (int k = 0; k < (int)gridDim.y; ++k) { db += sums[(int64_t)k * 2 * c + ch + e]; dw += sums[(int64_t)(k * 2 + 1) * c + ch + e]; }
       gb[ch + e] += db;
       gw[ch + e] += dw;
     }
   }
-  float A[4], B[4], D[4], sh[4];                // APPLY: dx = A g + B x + D; else xhat = (x - D) * B; mask: x * A + sh > 0
-  {
-    const float inv_m = 1.f / (float)((int64_t)g.n * g.h * g.w);
+  float A[8], B[8], D[8];                       // APPLY: dx = A dy' + B x + D; else D = mean, A and B the two sums
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float mean = mean_rstd[ch + e], rs = mean_rstd[c + ch + e];
-      A[e] = wgt[ch + e] * rs;
-      sh[e] = bias[ch + e] - mean * A[e];
-      if constexpr (APPLY) {
-        B[e] = -A[e] * rs * (sums[c + ch + e] * inv_m);
-        D[e] = -A[e] * (sums[ch + e] * inv_m) - B[e] * mean;
-      } else {
-        B[e] = rs;
-        D[e] = mean;
+  for (int e = 0; e < 8; ++e) { A[e] = 0.f; B[e] = 0.f; D[e] = 0.f; }
+  if (th.active) {
+    float mean[8];
+    tsp::ld8(mean_rstd, ch, mean);
+    if constexpr (APPLY) {
+      float rs[8], wv[8], k1[8], k2[8];
+      tsp::ld8(mean_rstd + c, ch, rs);
+      tsp::ld8(wgt, ch, wv);
+      tsp::ld8(sums, ch, k1);
+      tsp::ld8(sums + c, ch, k2);
+      const float inv_m = 1.f / (float)((int64_t)g.n * g.h * g.w);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        A[e] = wv[e] * rs[e];
+        B[e] = -A[e] * rs[e] * (k2[e] * inv_m);
+        D[e] = -A[e] * (k1[e] * inv_m) - B[e] * mean[e];
       }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) D[e] = mean[e];
     }
   }
-  float a[4], b[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) { a[e] = 0.f; b[e] = 0.f; }
-  for (int64_t i = first; i < total; i += stride) {
-    uint32_t p = (uint32_t)(i / cpv);
-    const int wb = (int)(p % (uint32_t)g.wo);
-    p /= (uint32_t)g.wo;
-    const int wa = (int)(p % (uint32_t)g.ho);
-    const int img = (int)(p / (uint32_t)g.ho);
+  const uint32_t items = th.active ? g.items : 0;
+  for (uint32_t i = blockIdx.x * th.per_block + th.slot; i < items; i += gridDim.x * th.per_block) {
+    const uint32_t row = g.by_wo.div(i), img = g.by_rows.div(row);
+    const int wb = (int)(i - row * g.by_wo.d), wa = (int)(row - img * g.by_rows.d);
     const bool down = wa + 1 < g.ho, right = wb + 1 < g.wo;             // windows below and to the right
     const bool row1 = 2 * wa + 1 < g.h, col1 = 2 * wb + 1 < g.w;        // second input row and column
-    const T* dyi = dy + (((int64_t)img * g.ho + wa) * g.wo + wb) * c + ch;
-    const uint8_t* ti = idx + (((int64_t)img * g.ho + wa) * g.wo + wb) * c + ch;
+    const int64_t o = (int64_t)i * c + ch;
     const int64_t q = (((int64_t)img * g.h + 2 * wa) * g.w + 2 * wb) * c + ch;
-    tsp::Raw4<T> gr[4], xr[4];
-    uint32_t tap[4];
+    tsp::Raw8<T> gr[4] = {}, xr[4] = {};
+    uint32_t tap[4][2];
     const bool have[4] = {true, right, down, down && right};
     const bool pix[4] = {true, col1, row1, row1 && col1};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int oo = ((k >> 1) * g.wo + (k & 1)) * c;
-      tap[k] = 0xffffffffu;                                             // no tap: a window that does not exist wins nothing
+      const int64_t oo = o + ((k >> 1) * g.wo + (k & 1)) * (int64_t)c;
+      tap[k][0] = tap[k][1] = 0xffffffffu;                              // a window that does not exist has no winner
       if (have[k]) {
-        tsp::ldraw(dyi, oo, gr[k]);
-        tap[k] = *reinterpret_cast<const uint32_t*>(ti + oo);
+        tsp::ldraw(dy, oo, gr[k]);
+        const uint2 t = *reinterpret_cast<const uint2*>(idx + oo);
+        tap[k][0] = t.x;
+        tap[k][1] = t.y;
       }
-      if (pix[k]) tsp::ldraw(x + q, ((k >> 1) * g.w + (k & 1)) * c, xr[k]);
+      if (pix[k]) tsp::ldraw(x, q + ((k >> 1) * g.w + (k & 1)) * (int64_t)c, xr[k]);
     }
-    float gv[4][4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (have[k]) tsp::cvt4(gr[k], gv[k]);
+    for (int j = 0; j < 4; ++j) {                                       // channels 2j and 2j + 1
+      float2 gv[4];
+      uint32_t code[4][2];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (!pix[k]) continue;
-      const int dr = k >> 1, dc = k & 1;                                // pixel (2 wa + dr, 2 wb + dc)
-      float d[4], xv[4];
-      tsp::cvt4(xr[k], xv);
+      for (int k = 0; k < 4; ++k) {
+        gv[k] = get2(gr[k], j);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) d[e] = 0.f;
-#pragma unroll
-      for (int kw = 0; kw < 4; ++kw) {                                  // window (wa + kw / 2, wb + kw % 2)
-        const int ky = dr + 1 - 2 * (kw >> 1), kx = dc + 1 - 2 * (kw & 1);
-        if (ky < 0 || kx < 0) continue;
-        const uint32_t want = (uint32_t)(ky * 3 + kx);
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (((tap[kw] >> (8 * e)) & 0xffu) == want) d[e] += gv[kw][e];
+        for (int s = 0; s < 2; ++s) code[k][s] = (tap[k][j >> 1] >> (8 * ((2 * j + s) & 3))) & 0xffu;
       }
-      tsp::round_as<T>(d);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) d[e] = (xv[e] * A[e] + sh[e]) > 0.f ? d[e] : 0.f;
-      if constexpr (APPLY) {
+      for (int k = 0; k < 4; ++k) {                                     // pixel (2 wa + k / 2, 2 wb + k % 2)
+        if (!APPLY && !pix[k]) continue;
+        float2 d = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) d[e] = A[e] * d[e] + B[e] * xv[e] + D[e];
-        tsp::st4(dx + q, (dr * g.w + dc) * c, d);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { a[e] += d[e]; b[e] += d[e] * (xv[e] - D[e]) * B[e]; }
+        for (int kw = 0; kw < 4; ++kw) {                                // window (wa + kw / 2, wb + kw % 2)
+          const int ky = (k >> 1) + 1 - 2 * (kw >> 1), kx = (k & 1) + 1 - 2 * (kw & 1);
+          if (ky < 0 || kx < 0) continue;
+          if (code[kw][0] == tap_code(ky, kx)) d.x += gv[kw].x;
+          if (code[kw][1] == tap_code(ky, kx)) d.y += gv[kw].y;
+        }
+        if (k > 0) d = round2<T>(d);                                    // (pixel 0 is in one window only)
+        const float2 xv = get2(xr[k], j);
+        if constexpr (APPLY) {
+          set2(xr[k], j, make_float2(A[2 * j] * d.x + B[2 * j] * xv.x + D[2 * j],
+                                     A[2 * j + 1] * d.y + B[2 * j + 1] * xv.y + D[2 * j + 1]));
+        } else {
+          A[2 * j] += d.x;
+          A[2 * j + 1] += d.y;
+          B[2 * j] += d.x * (xv.x - D[2 * j]);
+          B[2 * j + 1] += d.y * (xv.y - D[2 * j + 1]);
+        }
       }
+    }
+    if constexpr (APPLY) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (pix[k]) st_raw(dx, q + ((k >> 1) * g.w + (k & 1)) * (int64_t)c, xr[k]);
     }
   }
   if constexpr (!APPLY) {
-    // threads that are cpv apart hold the same channels when cpv divides the block (one addition per channel and block,
-    // lane = channel, as in bn_colsum_kernel), else every thread adds its own
-    if (kBlock % cpv == 0) {
+    // one addition per channel and block, lane = channel, as in bn_colsum_kernel
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { sm[e * pitch + threadIdx.x] = a[e]; sm[(4 + e) * pitch + threadIdx.x] = b[e]; }
-      __syncthreads();
-      for (int p = threadIdx.x; p < 2 * c; p += kBlock) {
-        const int half = p >= c ? 1 : 0, cc = p - half * c;
-        float acc = 0.f;
-        for (int k = cc >> 2; k < kBlock; k += cpv) acc += sm[(half * 4 + (cc & 3)) * pitch + k];
-        atomicAdd(sums + p, acc);
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { atomicAdd(sums + ch + e, a[e]); atomicAdd(sums + c + ch + e, b[e]); }
+    for (int e = 0; e < 8; ++e) { sm[e * sm_pitch + threadIdx.x] = A[e]; sm[(8 + e) * sm_pitch + threadIdx.x] = B[e]; }
+    __syncthreads();
+    const int width = min(c >> 3, kBlock), base = blockIdx.z * kBlock * 8;
+    for (int p = threadIdx.x; p < 16 * width; p += kBlock) {
+      const int half = p >= 8 * width ? 1 : 0, cc = p - half * 8 * width;
+      if (base + cc >= c) continue;
+      float acc = 0.f;
+      for (int k = 0; k < th.per_block; ++k) acc += sm[(half * 8 + (cc & 7)) * sm_pitch + k * width + (cc >> 3)];
+      if (half) acc *= mean_rstd[c + base + cc];
+      atomicAdd(sums + half * c + base + cc, acc);
     }
   }
 }
@@ -1023,20 +1116,30 @@ int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* 
 // Training-mode BatchNorm + ReLU + 3x3 / 2 / 1 max-pool of x [segs * n, h, w, c] (statistics per group of n images, from
 // `sums` [segs][2c] = sum and sum of squares over a group's pixels) -> y [segs * n, ho, wo, c], ho = (h + 1) / 2; idx
 // (optional, same shape as y) receives the winning taps for the backward.  The other arguments as in tsp_bn_apply.
-static int pool_geom(int n, int h, int w, int c, int segs, PoolGeom* g) {
+static int pool_geom(int n, int h, int w, int c, int segs, int rows_per_item, PoolGeom* g) {
   if (n <= 0 || h < 1 || w < 1 || c % 8 != 0 || c > 4096 || segs < 1) return -3;
-  *g = {n, h, w, c, (h + 1) / 2, (w + 1) / 2};
-  return (int64_t)n * g->ho * g->wo < 0x7fffffff ? 0 : -3;
+  const int ho = (h + 1) / 2, wo = (w + 1) / 2, rows = (ho + rows_per_item - 1) / rows_per_item;
+  if ((int64_t)n * (h + 1) * (w + 1) >= 0x7fffffff || (int64_t)w * c >= 0x7fffffff) return -3;
+  *g = {n, h, w, c, ho, wo, FastDiv(wo), FastDiv(rows), (uint32_t)((int64_t)n * rows * wo)};
+  return 0;
+}
+
+// Blocks for all items of a segment, at most `waves` per SM over all segments, and its segments and channel slabs.
+static dim3 pool_grid(const PoolGeom& g, int segs, int waves) {
+  const int cpv = g.c / 8, per_block = kBlock / (cpv < kBlock ? cpv : kBlock), slabs = (cpv + kBlock - 1) / kBlock;
+  int64_t blocks = ((int64_t)g.items + per_block - 1) / per_block;
+  const int64_t most = 148 * waves / ((int64_t)segs * slabs);
+  if (blocks > most) blocks = most;
+  return dim3((unsigned)(blocks < 1 ? 1 : blocks), (unsigned)segs, (unsigned)slabs);
 }
 
 int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums, const float* w, const float* b,
                          float* save_mean_rstd, float* acc_sum, float* acc_sumsq, float* acc_count, int64_t acc_seg_stride,
                          int n, int h, int wd, int c, float eps, int dtype, int segs, cudaStream_t stream) {
   PoolGeom g;
-  const int rc = pool_geom(n, h, wd, c, segs, &g);
+  const int rc = pool_geom(n, h, wd, c, segs, kPoolRows, &g);
   if (rc != 0) return rc;
-  const int64_t work = (int64_t)n * ((g.ho + kPoolRows - 1) / kPoolRows) * g.wo * (c / 4);
-  const dim3 grid(tsp::row_stride_blocks(work, c / 4, kBlock, 1, 1, 148 * 32 / segs), segs);
+  const dim3 grid = pool_grid(g, segs, 32);
   if (dtype == TSP_DTYPE_BF16)
     bn_relu_pool_kernel<__nv_bfloat16><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, idx, sums, w,
                                                                     b, save_mean_rstd, acc_sum, acc_sumsq, acc_count,
@@ -1050,25 +1153,23 @@ int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums
 // Its backward: dy [segs * n, ho, wo, c], idx and x as above -> dx; sums [segs][2c], zeroed by the
 // caller, receives db and dw; gw / gb as in tsp_bn_bwd_apply.
 int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* x, const float* mean_rstd, const float* w,
-                         const float* b, float* sums, void* dx, float* gw, float* gb, int n, int h, int wd, int c,
+                         float* sums, void* dx, float* gw, float* gb, int n, int h, int wd, int c,
                          int dtype, int segs, cudaStream_t stream) {
   PoolGeom g;
-  const int rc = pool_geom(n, h, wd, c, segs, &g);
+  const int rc = pool_geom(n, h, wd, c, segs, 1, &g);
   if (rc != 0) return rc;
-  const int64_t work = (int64_t)n * g.ho * g.wo * (c / 4);
-  const dim3 grid_r(tsp::row_stride_blocks(work, c / 4, kBlock, 8, 148 * 2 / segs, 148 * 3 / segs), segs);
-  const dim3 grid_a(tsp::row_stride_blocks(work, c / 4, kBlock, 1, 1, 148 * 32 / segs), segs);
+  const dim3 grid_r = pool_grid(g, segs, 2), grid_a = pool_grid(g, segs, 32);
   if (dtype == TSP_DTYPE_BF16) {
     using B = __nv_bfloat16;
-    bn_relu_pool_bwd_kernel<B, false><<<grid_r, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, b, sums,
+    bn_relu_pool_bwd_kernel<B, false><<<grid_r, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, sums,
                                                                      nullptr, nullptr, nullptr, g);
-    bn_relu_pool_bwd_kernel<B, true><<<grid_a, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, b, sums,
+    bn_relu_pool_bwd_kernel<B, true><<<grid_a, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, sums,
                                                                     (B*)dx, gw, gb, g);
   } else {
     bn_relu_pool_bwd_kernel<float, false><<<grid_r, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd,
-                                                                         w, b, sums, nullptr, nullptr, nullptr, g);
+                                                                         w, sums, nullptr, nullptr, nullptr, g);
     bn_relu_pool_bwd_kernel<float, true><<<grid_a, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd, w,
-                                                                        b, sums, (float*)dx, gw, gb, g);
+                                                                        sums, (float*)dx, gw, gb, g);
   }
   return TSP_LAUNCH_CHECK();
 }

@@ -118,31 +118,6 @@ __device__ __forceinline__ void round_as(float (&v)[N]) {
   }
 }
 
-// 4 consecutive elements (8 bytes of bf16, 16 of fp32), for passes that need more threads than bytes per thread.
-template <typename T> struct Raw4;
-template <> struct Raw4<float> { float4 a; };
-template <> struct Raw4<__nv_bfloat16> { uint2 a; };
-template <typename T>
-__device__ __forceinline__ void ldraw(const T* p, int64_t i, Raw4<T>& r) {
-  r.a = *reinterpret_cast<const decltype(r.a)*>(p + i);
-}
-__device__ __forceinline__ void cvt4(const Raw4<float>& r, float (&v)[4]) { v[0] = r.a.x; v[1] = r.a.y; v[2] = r.a.z; v[3] = r.a.w; }
-__device__ __forceinline__ void cvt4(const Raw4<__nv_bfloat16>& r, float (&v)[4]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r.a);
-#pragma unroll
-  for (int k = 0; k < 2; ++k) { const float2 f = __bfloat1622float2(h[k]); v[2 * k] = f.x; v[2 * k + 1] = f.y; }
-}
-__device__ __forceinline__ void st4(float* p, int64_t i, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p + i) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void st4(__nv_bfloat16* p, int64_t i, const float (&v)[4]) {
-  uint2 raw;
-  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int k = 0; k < 2; ++k) h[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-  *reinterpret_cast<uint2*>(p + i) = raw;
-}
-
 // Blocks of `threads` threads for an elementwise pass over nvec vectors, cpv of them per row: `per_thread` vectors per
 // thread where that leaves at least `least` blocks, fewer per thread (down to one) on smaller tensors, at most `most`
 // blocks; rounded up so that the grid stride is a multiple of a row, i.e. a thread meets one column of vectors only.

@@ -270,14 +270,14 @@ class _BnReluPool(torch.autograd.Function):
                                              _c.c_int(c), _c.c_float(eps), _c.c_int(dt), _c.c_int(segs), st),
                       "tsp_bn_relu_pool_fwd")
             _f._count()
-        ctx.save_for_backward(x, idx, save, wf, bf)
+        ctx.save_for_backward(x, idx, save, wf)
         ctx.segs, ctx.wdtype, ctx.bdtype = segs, weight.dtype, bias.dtype
         ctx.owners = (weight, bias) if _f.IN_CAPTURE else (None, None)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, idx, save, wf, bf = ctx.saved_tensors
+        x, idx, save, wf = ctx.saved_tensors
         n, c, h, w = x.shape
         segs = ctx.segs
         ho, wo = (h + 1) // 2, (w + 1) // 2
@@ -290,7 +290,7 @@ class _BnReluPool(torch.autograd.Function):
             gw = gb = None
         with _f.on_device(x.device):
             _f._check(_lib().tsp_bn_relu_pool_bwd(_f._ptr(dy), _f._ptr(idx), _f._ptr(x), _f._ptr(save), _f._ptr(wf),
-                                                  _f._ptr(bf), _f._ptr(sums), _f._ptr(dx), _f._ptr(gw), _f._ptr(gb),
+                                                  _f._ptr(sums), _f._ptr(dx), _f._ptr(gw), _f._ptr(gb),
                                                   _c.c_int(n // segs), _c.c_int(h), _c.c_int(w), _c.c_int(c),
                                                   _c.c_int(_f._dt(x)), _c.c_int(segs), _f._stream()),
                       "tsp_bn_relu_pool_bwd")
