@@ -133,13 +133,16 @@ class _BnAct(torch.autograd.Function):
         ctx.save_for_backward(x, y if (relu and residual is not None) else None, save, wf, bf)
         ctx.relu, ctx.has_res, ctx.mc, ctx.segs = relu, residual is not None, (m, c), segs
         ctx.wdtype, ctx.bdtype = weight.dtype, bias.dtype
-        ctx.owners = (weight, bias) if _f.IN_CAPTURE else (None, None)
+        ctx.owners = (weight, bias) if _f.IN_CAPTURE else None
         ctx.fixed = fixed is not None
         ctx.mark_non_differentiable(sums)
+        ctx.set_materialize_grads(False)   # (sums' gradient would be a tensor of zeros, allocated and filled on every call)
         return y, sums
 
     @staticmethod
     def backward(ctx, dy, _dsums):
+        if dy is None:
+            return (None,) * 13
         x, y, save, wf, bf = ctx.saved_tensors
         m, c = ctx.mc
         L = _lib()
@@ -164,9 +167,11 @@ class _BnAct(torch.autograd.Function):
             else:
                 sums_for_dx = sums
             src, mask, relu2 = (dres, None, _c.c_int(0)) if dres is not None else (dy, y, relu)
-            gw, gb = (_f.recorded_grad(p) for p in ctx.owners)
-            if gw is None or gb is None or ctx.fixed:
-                gw = gb = None
+            gw = gb = None
+            if ctx.owners is not None and not ctx.fixed:
+                gw, gb = (_f.recorded_grad(p) for p in ctx.owners)
+                if gw is None or gb is None:
+                    gw = gb = None
             _f._check(L.tsp_bn_bwd_apply(_f._ptr(src), _f._ptr(x), _f._ptr(mask), _f._ptr(save), _f._ptr(wf),
                                          _f._ptr(bf), relu2, _f._ptr(sums_for_dx), _f._ptr(dx), _f._ptr(gw), _f._ptr(gb),
                                          _c.c_int64(m), _c.c_int(c), _c.c_int(dt), _c.c_int(segs), st),

@@ -69,10 +69,13 @@ class _StemConv(torch.autograd.Function):
         if sums is None:
             sums = torch.empty(0, device=x.device)
         ctx.mark_non_differentiable(sums)
+        ctx.set_materialize_grads(False)   # (sums' gradient would be a tensor of zeros, allocated and filled on every call)
         return y, sums
 
     @staticmethod
     def backward(ctx, dy, _dsums):
+        if dy is None:
+            return None, None, None, None
         x, weight = ctx.saved_tensors
         dx = dw = None
         need_dx = ctx.needs_input_grad[0]
@@ -229,11 +232,12 @@ class _Conv2d(torch.autograd.Function):
         if sums is None:
             sums = torch.empty(0, device=x.device)
         ctx.mark_non_differentiable(sums)
+        ctx.set_materialize_grads(False)   # (sums' gradient would be a tensor of zeros, allocated and filled on every call)
         return y, sums
 
     @staticmethod
     def backward(ctx, dy, _dsums):
-        return _Conv2d._backward(ctx, dy, None)
+        return _Conv2d._backward(ctx, dy, None) if dy is not None else (None,) * 5
 
     @staticmethod
     def _backward(ctx, dy, addend):
@@ -274,7 +278,6 @@ class _Conv2dFork(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, weight, stride, want_sums, segs):
-        ctx.set_materialize_grads(False)
         y, sums = _Conv2d.forward(ctx, x, weight, stride, want_sums, segs)
         return y, sums, x.view_as(x)
 
