@@ -480,7 +480,10 @@ struct HaloCfg {
 // base-offset field stays 0; setting it to the start's phase gives wrong products - measured).
 // One tile = a bordered box of up to 256 accumulator rows (two 128-row accumulators that share every weight tile).
 // g.b_resident: all weight tiles of the problem (9 taps, one channel block, one N tile) fit the weight ring; they are
-// loaded once and stay.
+// loaded once and stay.  With 64 output channels a product takes the tensor pipe 63 clocks (its shared-memory reads), so
+// the issuing thread is the bound: the taps are unrolled without the ring's waits, and one commit per tile tells the
+// epilogue and, in place of a_empty, the producer.  256 images of 56 x 56, B200: forward with statistics
+// 119 us with the ring's loop, 96 this way; data gradient 110 and 94.
 template <int BN, bool B_MN, bool STATS, bool ADD>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap,
@@ -506,6 +509,9 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
   const int kcb = g.kc >> 6;
   const int n_sub = (g.pix + 127) >> 7;
   const bool resident = g.b_resident != 0;
+  // (resident: one channel block, so unit = tile, and stage u % 2 of the boxes goes with accumulator buffer u % 2)
+  constexpr bool kMayReside = C::kBStages >= 9 && C::kAccBufs == C::kAStages;
+  uint64_t* box_free = kMayReside && resident ? tmem_full_bar : a_empty;
 
   // Rows of an A stage past the bordered box are never written by TMA but are read for accumulator rows that are
   // thrown away; they are zeroed once so that those rows stay finite.
@@ -548,7 +554,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         tile_origin(g, tm, w0, h0, n0);
         const int s = u % C::kAStages;
         const uint32_t round = (uint32_t)u / C::kAStages;
-        if (round > 0 && !mbar_wait_parked(a_empty + s, (round - 1) & 1, status, 1, g.wait_ns)) return false;
+        if (round > 0 && !mbar_wait_parked(box_free + s, (round - 1) & 1, status, 1, g.wait_ns)) return false;
         mbar_expect_tx(a_full + s, (uint32_t)g.halo_rows * 128u);
         tma_load_4d(a_tiles + s * C::kABytes, &amap, a_full + s, cb * 64, w0 - 1, h0 - 1, n0);
         return true;
@@ -600,12 +606,30 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
           ok = mbar_wait(a_full + sa, (ia / C::kAStages) & 1, status, 2, g.wait_ns);
           if (!ok) break;
           const uint32_t a_lo0 = desc_lo_k_major(a_addr0 + sa * C::kABytes);
-          for (int tap = 0; tap < 9; ++tap, ++ib) {
-            const int sb = resident ? tap : (int)(ib % C::kBStages);
-            if (!resident || ia == 0) {
-              ok = mbar_wait(b_full + sb, resident ? 0u : ((ib / C::kBStages) & 1), status, 2, g.wait_ns);
+          if constexpr (kMayReside) {
+            if (resident) {
+              if (ia == 0)
+                for (int tap = 0; tap < 9 && ok; ++tap) ok = mbar_wait(b_full + tap, 0u, status, 2, g.wait_ns);
               if (!ok) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t b_lo0 = B_MN ? desc_lo_mn_major(b_addr0, 8192) : desc_lo_k_major(b_addr0);
+              auto products = [&](uint32_t d, uint32_t a_first) {
+#pragma unroll
+                for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+                  for (int kk = 0; kk < 4; ++kk)
+                    umma_bf16_lo(d, a_first + 8 * g.tap_off[tap] + 2 * kk,
+                                 b_lo0 + tap * (C::kBBytes >> 4) + (B_MN ? 128 * kk : 2 * kk), idesc, tap + kk > 0 ? 1u : 0u);
+              };
+              products(d_tmem, a_lo0);
+              if (n_sub > 1) products(d_tmem + BN, a_lo0 + 1024);   // second accumulator: 128 rows further on
+              continue;
             }
+          }
+          for (int tap = 0; tap < 9; ++tap, ++ib) {
+            const int sb = (int)(ib % C::kBStages);
+            ok = mbar_wait(b_full + sb, (ib / C::kBStages) & 1, status, 2, g.wait_ns);
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t b_addr = b_addr0 + sb * C::kBBytes;
             const uint32_t b_lo = B_MN ? desc_lo_mn_major(b_addr, 8192) : desc_lo_k_major(b_addr);
@@ -620,7 +644,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                              kk == 0 ? accum : 1u);
             }
             accum = 1u;
-            if (!resident && ib % C::kBGroup == C::kBGroup - 1) umma_commit(b_empty + (ib / C::kBGroup) % C::kBGroups);
+            if (ib % C::kBGroup == C::kBGroup - 1) umma_commit(b_empty + (ib / C::kBGroup) % C::kBGroups);
           }
           if (ok) umma_commit(a_empty + sa);
         }
