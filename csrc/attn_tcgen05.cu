@@ -498,7 +498,7 @@ int launch(const void* q, void* const* k_srcs, int n_src, const void* v, void* o
 // The passes around the fused contrastive loss of two (queries, keys) pairs.  One warp per row of 256 elements, 8 per
 // lane; blockIdx.y = pair.
 // ---------------------------------------------------------------------------------------------
-constexpr int kNceDim = 256;
+constexpr int kNceDim = 256, kNceRows = 16;       // rows (warps) of a block of the last pass
 template <typename T>
 struct NcePairs {
   const T* q[2];
@@ -539,14 +539,15 @@ __global__ void __launch_bounds__(256) nce_prepare_kernel(const NcePairs<T> in, 
 // 2T/n * (lse - q.k/T) to the loss and writes the gradient with respect to the queries as they came in, i.e. through
 // the normalisation: g = 2/n * (o - k), dq = (g - q^ (q^.g)) / |q|.
 template <typename T>
-__global__ void __launch_bounds__(256) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
+__global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
                                                          const __nv_bfloat16* __restrict__ q16,
                                                          const __nv_bfloat16* __restrict__ k16,
                                                          const float* __restrict__ o, const float* __restrict__ lse,
-                                                         float* __restrict__ loss, T* __restrict__ gq) {
-  __shared__ float part[8];
+                                                         double* __restrict__ sum, float* __restrict__ loss,
+                                                         T* __restrict__ gq) {
+  __shared__ float part[kNceRows];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = lane * 8;
-  const int row = blockIdx.x * 8 + warp, pair = blockIdx.y;
+  const int row = blockIdx.x * kNceRows + warp, pair = blockIdx.y;
   float contrib = 0.f;
   if (row < n) {
     float q[8], qb[8], kb[8], acc[8] = {};
@@ -586,10 +587,13 @@ __global__ void __launch_bounds__(256) nce_finish_kernel(const NcePairs<T> in, i
   if (lane == 0) part[warp] = contrib;
   __syncthreads();
   if (threadIdx.x == 0) {
-    float s = 0.f;
+    double s = 0.;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s += part[i];
-    atomicAdd(loss, s);
+    for (int i = 0; i < kNceRows; ++i) s += part[i];
+    atomicAdd(sum, s);
+    __threadfence();
+    unsigned* done = reinterpret_cast<unsigned*>(sum + 1);
+    if (atomicAdd(done, 1u) == gridDim.x * gridDim.y - 1) *loss = (float)atomicAdd(sum, 0.);      // the last block
   }
 }
 
@@ -597,7 +601,8 @@ template <typename T>
 int launch_nce_pair(const NcePairs<T>& in, int n, int chunk, int chunks, float temp, void* q16, void* k16, float* o,
                     float* lse, float* loss, void* gq, int* status, cudaStream_t stream) {
   const int n_pad = chunk * chunks;
-  cudaError_t e = cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  double* sum = reinterpret_cast<double*>(lse + (int64_t)2 * chunks * n);       // and behind it the blocks that are done
+  cudaError_t e = cudaMemsetAsync(sum, 0, 2 * sizeof(double), stream);
   if (e != cudaSuccess) return (int)e;
   nce_prepare_kernel<T><<<dim3((n + n_pad + 7) / 8, 2), 256, 0, stream>>>(in, n, n_pad, (__nv_bfloat16*)q16,
                                                                           (__nv_bfloat16*)k16);
@@ -608,8 +613,8 @@ int launch_nce_pair(const NcePairs<T>& in, int n, int chunk, int chunks, float t
   const int rc = launch<256, 256, 64, true, float>(q16, srcs, 1, k16, o, lse, 2, chunks, n, chunk, sq, sk, sk, so,
                                                    1.f / temp, 1.f / temp, 1, status, stream, n);
   if (rc != 0) return rc;
-  nce_finish_kernel<T><<<dim3((n + 7) / 8, 2), 256, 0, stream>>>(in, n, n_pad, chunks, temp, (const __nv_bfloat16*)q16,
-                                                                 (const __nv_bfloat16*)k16, o, lse, loss, (T*)gq);
+  nce_finish_kernel<T><<<dim3((n + kNceRows - 1) / kNceRows, 2), 32 * kNceRows, 0, stream>>>(
+      in, n, n_pad, chunks, temp, (const __nv_bfloat16*)q16, (const __nv_bfloat16*)k16, o, lse, sum, loss, (T*)gq);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -653,7 +658,8 @@ int tsp_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ls
 // gq [2][n][256] = its gradient with respect to q0 and q1.  The keys are split into `chunks` pieces of `chunk` rows (a
 // multiple of 64; (chunks - 1) * chunk < n <= chunks * chunk), one per head of the attention grid, so that the grid fills
 // the chip.  Scores are bounded by 1/T, which is used as the fixed maximum: exp(-2/T) must not underflow.
-// Scratch: q16 [2][n][256] bf16, k16 [2][chunk * chunks][256] bf16, o [2][chunks][n][256] fp32, lse [2][chunks][n] fp32.
+// Scratch: q16 [2][n][256] bf16, k16 [2][chunk * chunks][256] bf16, o [2][chunks][n][256] fp32, lse [2][chunks][n] fp32 and
+// 16 bytes behind it (the loss is summed in 64 bits, as 512 fp32 additions in turn would be 1e-6 off).
 int tsp_nce_pair(const void* q0, const void* k0, const void* q1, const void* k1, int n, int dtype, int chunk, int chunks,
                  float temp, void* q16, void* k16, float* o, float* lse, float* loss, void* gq, int* status,
                  cudaStream_t stream) {

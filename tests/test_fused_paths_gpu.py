@@ -57,6 +57,19 @@ def test_kd_ce_rows_vectorised_and_not(n, c, dtype):
     assert _rel(g, gr) < max(2 * EPS[dtype], 1e-5)
 
 
+def test_losses_of_many_rows_lose_nothing_in_their_sum():
+    """20000 terms added one by one in fp32 would be some 1e-6 to 1e-5 off; the terms' own roundings cancel to below 2^-24."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(17)
+    s, t = torch.randn(20000, 16, device=DEV) * 2, torch.randn(20000, 16, device=DEV) * 2
+    y = torch.randint(0, 16, (20000,), device=DEV)
+    s6, t6 = s.double(), t.double()
+    kd = F.kl_div(F.log_softmax(s6 / 2, 1), F.log_softmax(t6 / 2, 1), reduction="sum", log_target=True)
+    for got, want in ((fused.kd_ce_loss(s, t, y, 2.0, 0.5, 0.25), 0.25 * 4 * kd + 0.5 * F.cross_entropy(s6, y, reduction="sum")),
+                      (fused.cosine_embedding_loss(s, t, 0.5), 0.5 * (1 - F.cosine_similarity(s6, t6)).sum())):
+        assert got.dtype == torch.float32 and abs(float(got) - float(want)) <= 4e-7 * abs(float(want))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,d", [(1, 8), (7, 256), (130, 100)])
 def test_byol_pair_equals_two_single_losses(n, d, dtype):

@@ -359,7 +359,7 @@ class _KdCe(torch.autograd.Function):
         else:
             t2 = t.detach().reshape(-1, t.shape[-1]).contiguous()
         n, c = s2.shape
-        loss = torch.zeros((), dtype=torch.float32, device=s.device)
+        loss = torch.zeros((), dtype=torch.float64, device=s.device)      # thousands of rows add to it in turn
         gs = torch.empty_like(s2)
         lab = None if labels is None else labels.reshape(-1).to(torch.int64).contiguous()
         msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
@@ -371,7 +371,7 @@ class _KdCe(torch.autograd.Function):
         _count()
         ctx.save_for_backward(gs)
         ctx.shape = s.shape
-        return loss
+        return loss.float()
 
     @staticmethod
     def backward(ctx, gout):
@@ -402,7 +402,7 @@ class _Cosine(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
         y2 = y.detach().reshape(-1, y.shape[-1]).to(x2.dtype).contiguous()
         n, d = x2.shape
-        loss = torch.zeros((), dtype=torch.float32, device=x.device)
+        loss = torch.zeros((), dtype=torch.float64, device=x.device)
         gx = torch.empty_like(x2)
         msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
         with on_device(x.device):
@@ -411,7 +411,7 @@ class _Cosine(torch.autograd.Function):
         _count()
         ctx.save_for_backward(gx)
         ctx.shape = x.shape
-        return loss
+        return loss.float()
 
     @staticmethod
     def backward(ctx, gout):

@@ -523,7 +523,7 @@ class _NCEPair(torch.autograd.Function):
         q16 = torch.empty((2, n, d), dtype=torch.bfloat16, device=dev)
         k16 = torch.empty((2, c * chunk, d), dtype=torch.bfloat16, device=dev)
         o = torch.empty((2, c, n, d), dtype=torch.float32, device=dev)
-        lse = torch.empty((2, c, n), dtype=torch.float32, device=dev)
+        lse = torch.empty(2 * c * n + 4, dtype=torch.float32, device=dev)      # and the loss's 64-bit sum
         loss = torch.empty((), dtype=torch.float32, device=dev)
         gq = torch.empty((2, n, d), dtype=q1.dtype, device=dev)
         L = _f.lib()
