@@ -8,7 +8,7 @@ children in order but lets neighbouring ones share a kernel:
 * ``BatchNorm -> ReLU``                      one fused normalise + activation pass (``ops.bn.bn_act``);
 * ``Conv2d(3, 64, 7, stride 2) -> BatchNorm`` the tcgen05 stem convolution, whose epilogue already produces the
   BatchNorm statistics (``ops.conv.stem_conv``), so the statistics pass over the activation disappears;
-* that stem convolution's ``BatchNorm -> ReLU -> MaxPool 3x3/2``  one pass forward, two backward
+* that stem convolution's ``BatchNorm -> ReLU -> MaxPool 3x3/2`` one pass forward and two backward
   (``ops.bn.bn_relu_pool``): the normalised activation is never written;
 * ``Linear`` children (the MLP heads)        the tcgen05 GEMM path of ``ops.linear.linear``, forward and backward.
 
