@@ -322,6 +322,9 @@ __global__ void __launch_bounds__(128) cosine_kernel(const T* __restrict__ x, co
   if (threadIdx.x == 0) atomicAdd(loss, (double)(scale * (part[0] + part[1] + part[2] + part[3])));
 }
 
+// The rows of a loss add to a 64-bit sum (`sum`, scratch): thousands of fp32 additions in turn are some 1e-6 off.
+__global__ void round_sum_kernel(const double* __restrict__ sum, float* __restrict__ loss) { *loss = (float)*sum; }
+
 // Rows of `d` elements on these bases can be accessed 8 elements (16 or 32 bytes) at a time.
 bool rows_of_8(int d, const void* a, const void* b, const void* c) {
   return d % 8 == 0 && ((((uintptr_t)a) | ((uintptr_t)b) | ((uintptr_t)c)) & 15) == 0;
@@ -361,22 +364,25 @@ int tsp_byol_loss_pair(const void* x0, const void* y0, const void* x1, const voi
 }
 
 int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,
-                    double* loss, void* gx, cudaStream_t stream) {
-  if (n <= 0) return 0;
+                    double* sum, float* loss, void* gx, cudaStream_t stream) {
+  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  if (cudaError_t e = cudaMemsetAsync(sum, 0, sizeof(double), stream); e != cudaSuccess) return (int)e;
   const int grid = (n + 3) / 4;
   const bool vec = rows_of_8(d, x, y, gx);
 #define TSP_COS(T, VEC) \
-  cosine_kernel<T, VEC><<<grid, 128, 0, stream>>>((const T*)x, (const T*)y, row_mask, n, d, scale, loss, (T*)gx)
+  cosine_kernel<T, VEC><<<grid, 128, 0, stream>>>((const T*)x, (const T*)y, row_mask, n, d, scale, sum, (T*)gx)
   if (dtype == TSP_DTYPE_BF16) { if (vec) TSP_COS(__nv_bfloat16, true); else TSP_COS(__nv_bfloat16, false); }
   else { if (vec) TSP_COS(float, true); else TSP_COS(float, false); }
 #undef TSP_COS
+  round_sum_kernel<<<1, 1, 0, stream>>>(sum, loss);
   return TSP_LAUNCH_CHECK();
 }
 
 int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
-                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* loss, void* gs,
+                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* sum, float* loss, void* gs,
                    cudaStream_t stream) {
-  if (n <= 0) return 0;
+  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  if (cudaError_t e = cudaMemsetAsync(sum, 0, sizeof(double), stream); e != cudaSuccess) return (int)e;
   const bool vec = rows_of_8(c, s, t, gs);
   // at least four accesses per thread and sweep on long rows, one warp of latency on short ones
   const int parts = vec ? c / 8 : c;
@@ -385,16 +391,17 @@ int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const ui
   do {                                                                                                               \
     if (vec)                                                                                                         \
       kd_ce_kernel<TS, TT, true><<<n, threads, 0, stream>>>((const TS*)s, (const TT*)t, labels, row_mask, n, c, temp, \
-                                                            w_ce, w_kd, loss, (TS*)gs);                              \
+                                                            w_ce, w_kd, sum, (TS*)gs);                               \
     else                                                                                                             \
       kd_ce_kernel<TS, TT, false><<<n, threads, 0, stream>>>((const TS*)s, (const TT*)t, labels, row_mask, n, c,     \
-                                                             temp, w_ce, w_kd, loss, (TS*)gs);                       \
+                                                             temp, w_ce, w_kd, sum, (TS*)gs);                        \
   } while (0)
   if (s_dtype == TSP_DTYPE_BF16 && t_dtype == TSP_DTYPE_BF16) TSP_KD(__nv_bfloat16, __nv_bfloat16);
   else if (s_dtype == TSP_DTYPE_BF16) TSP_KD(__nv_bfloat16, float);
   else if (t_dtype == TSP_DTYPE_BF16) TSP_KD(float, __nv_bfloat16);
   else TSP_KD(float, float);
 #undef TSP_KD
+  round_sum_kernel<<<1, 1, 0, stream>>>(sum, loss);
   return TSP_LAUNCH_CHECK();
 }
 

@@ -32,9 +32,9 @@ int tsp_byol_loss(const void* x, const void* y, int n, int d, int dtype, float s
 int tsp_byol_loss_pair(const void* x0, const void* y0, const void* x1, const void* y1, int n, int d, int dtype,
                        float scale, float* loss, void* gx, cudaStream_t stream);
 int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,
-                    double* loss, void* gx, cudaStream_t stream);
+                    double* sum, float* loss, void* gx, cudaStream_t stream);
 int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
-                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* loss, void* gs,
+                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* sum, float* loss, void* gs,
                    cudaStream_t stream);
 int tsp_scale(const void* in, const float* gout, void* out, int64_t n, int dtype, cudaStream_t stream);
 

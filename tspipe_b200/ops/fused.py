@@ -359,19 +359,20 @@ class _KdCe(torch.autograd.Function):
         else:
             t2 = t.detach().reshape(-1, t.shape[-1]).contiguous()
         n, c = s2.shape
-        loss = torch.zeros((), dtype=torch.float64, device=s.device)      # thousands of rows add to it in turn
+        loss = torch.empty((), dtype=torch.float32, device=s.device)
+        total = torch.empty((), dtype=torch.float64, device=s.device)
         gs = torch.empty_like(s2)
         lab = None if labels is None else labels.reshape(-1).to(torch.int64).contiguous()
         msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
         with on_device(s.device):
             _check(lib().tsp_kd_ce_loss(_ptr(s2), _ptr(t2), _ptr(lab), _ptr(msk), _c.c_int(n), _c.c_int(c),
                                         _c.c_int(_dt(s2)), _c.c_int(0 if t2 is None else _dt(t2)), _c.c_float(temp),
-                                        _c.c_float(w_ce), _c.c_float(w_kd), _ptr(loss), _ptr(gs), _stream()),
+                                        _c.c_float(w_ce), _c.c_float(w_kd), _ptr(total), _ptr(loss), _ptr(gs), _stream()),
                    "tsp_kd_ce_loss")
-        _count()
+        _count(2)
         ctx.save_for_backward(gs)
         ctx.shape = s.shape
-        return loss.float()
+        return loss
 
     @staticmethod
     def backward(ctx, gout):
@@ -402,16 +403,18 @@ class _Cosine(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
         y2 = y.detach().reshape(-1, y.shape[-1]).to(x2.dtype).contiguous()
         n, d = x2.shape
-        loss = torch.zeros((), dtype=torch.float64, device=x.device)
+        loss = torch.empty((), dtype=torch.float32, device=x.device)
+        total = torch.empty((), dtype=torch.float64, device=x.device)
         gx = torch.empty_like(x2)
         msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
         with on_device(x.device):
             _check(lib().tsp_cosine_loss(_ptr(x2), _ptr(y2), _ptr(msk), _c.c_int(n), _c.c_int(d), _c.c_int(_dt(x2)),
-                                         _c.c_float(scale), _ptr(loss), _ptr(gx), _stream()), "tsp_cosine_loss")
-        _count()
+                                         _c.c_float(scale), _ptr(total), _ptr(loss), _ptr(gx), _stream()),
+                   "tsp_cosine_loss")
+        _count(2)
         ctx.save_for_backward(gx)
         ctx.shape = x.shape
-        return loss.float()
+        return loss
 
     @staticmethod
     def backward(ctx, gout):
