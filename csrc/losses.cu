@@ -198,8 +198,11 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
   float z[3] = {z1 * ex2((ps.ref() - ms) * kLog2e), zs * ex2((ps.ref() - ms) * k2), kd ? zt * ex2((pt.ref() - mt) * k2) : 0.f};
   block_all<3, false>(z, scratch + 64);
   const float l1 = has_ce ? log2f(z[0]) : 0.f, ls = kd ? log2f(z[1]) : 0.f, lt = kd ? log2f(z[2]) : 0.f;
+  // The divergence is formed from differences of logits in their own scale, not from the scaled logarithms: a class that the
+  // type's lowest value switches off stays finite there at every temperature above one (times log2(e) / T it is -inf below
+  // T = 1.44), and a class that the teacher gives no probability adds nothing, whatever the other factor is.
   float kl = 0.f;
-  const float wt = w_kd * temp;
+  const float wt = w_kd * temp, inv_t = 1.f / temp, dl = (lt - ls) * kLn2;
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
     float a[V], b[V], g[V];
     load_part<TS, V>(sr, i, a);
@@ -207,10 +210,10 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
     if (kd) {
 #pragma unroll
       for (int e = 0; e < V; ++e) {
-        const float lps = (a[e] - ms) * k2 - ls, lpt = (b[e] - mt) * k2 - lt;
-        const float p = ex2(lpt);
-        kl += p * (lpt - lps);
-        g[e] = wt * (ex2(lps) - p);
+        const float da = a[e] - ms, db = b[e] - mt;
+        const float p = ex2(db * k2 - lt), t = p * ((db - da) * inv_t - dl);
+        kl += p != 0.f ? t : 0.f;                // (a NaN is kept)
+        g[e] = wt * (ex2(da * k2 - ls) - p);
       }
     } else {
 #pragma unroll
@@ -227,7 +230,7 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
   if (threadIdx.x == 0) {
     float v = 0.f;
     if (has_ce) v += w_ce * (l1 * kLn2 - (tsp::ld(sr, label) - ms));
-    if (kd) v += w_kd * temp * temp * (total[0] * kLn2);
+    if (kd) v += w_kd * temp * temp * total[0];
     atomicAdd(loss, (double)v);
   }
 }

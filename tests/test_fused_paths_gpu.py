@@ -57,6 +57,32 @@ def test_kd_ce_rows_vectorised_and_not(n, c, dtype):
     assert _rel(g, gr) < max(2 * EPS[dtype], 1e-5)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("temp", [0.5, 1.0, 1.4, 2.0])
+def test_kd_with_classes_switched_off_at_every_temperature(temp, dtype):
+    """Classes that the type's lowest value, or -inf, switches off in the teacher, or in the teacher and the student, add
+    nothing to the divergence on either side of T = log2(e) = 1.44; a NaN still shows."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(18)
+    low = torch.finfo(dtype).min
+    for off, in_student in ((low, False), (low, True), (-math.inf, False), (-math.inf, True)):
+        s, t = ((torch.randn(4, 264, device=DEV) * 2).to(dtype) for _ in range(2))
+        t[:, :100] = off
+        if in_student:
+            s[:, :100] = off
+        s.requires_grad_()
+        loss = fused.kd_ce_loss(s, t, None, temp, 0.0, 1.0)
+        (g,) = torch.autograd.grad(loss, s)
+        r, t6 = s.detach().double().requires_grad_(), t.double()
+        ls, lt = F.log_softmax(r / temp, 1), F.log_softmax(t6 / temp, 1)
+        ref = temp ** 2 * (lt.exp() * (lt - ls))[:, 100:].sum()
+        (gr,) = torch.autograd.grad(ref, r)
+        assert abs(float(loss.detach()) - float(ref.detach())) <= 1e-5 * abs(float(ref.detach()))
+        assert _rel(g, torch.nan_to_num(gr, nan=0.0)) < max(2 * EPS[dtype], 1e-5)
+    t[1, 200] = math.nan
+    assert fused.kd_ce_loss(s, t, None, temp, 0.0, 1.0).isnan()
+
+
 def test_losses_of_many_rows_lose_nothing_in_their_sum():
     """20000 terms added one by one in fp32 would be some 1e-6 to 1e-5 off; the terms' own roundings cancel to below 2^-24."""
     from tspipe_b200.ops import fused
