@@ -7,6 +7,7 @@ library cannot be loaded on a CUDA machine.
 from __future__ import annotations
 
 import ctypes
+import weakref
 from typing import Optional, Sequence
 
 import torch
@@ -81,8 +82,8 @@ class capturing:
 
 
 class _Recording:
-    """What the launches of one recording share: bf16 copies of whole flat parameter buffers (by the buffer's address) and
-    what is left of its block of zeroed floats."""
+    """What the launches of one recording share: bf16 copies of whole flat parameter buffers and what is left of its block of
+    zeroed floats."""
 
     def __init__(self):
         self.copies, self.zeros = {}, None
@@ -114,25 +115,38 @@ def zeroed(n: int, device) -> torch.Tensor:
 
 
 _FLAT_COPY_MAX = 32 << 20
+_FLAT_PARAMS = weakref.WeakValueDictionary()      # every living FlatParams of fp32, by its id
+
+
+def register_flat(flat) -> None:
+    """``flat`` (:class:`~tspipe_b200.runtime.state.FlatParams`) holds parameters that may be cast together."""
+    _FLAT_PARAMS[id(flat)] = flat
 
 
 def recorded_bf16(weight: torch.Tensor) -> torch.Tensor:
-    """bf16 copy of a parameter for a graph under recording, with the parameter's strides.  Parameters that are views of
-    one flat fp32 buffer are cast together, once per recording: a cast per parameter is a launch per parameter, 2.4 us each
-    for the 52 convolution weights of a ResNet-50 against 21 us
-    for the whole buffer.  Larger buffers, whose casts are bound by memory one by one, and parameters of their own are cast
-    singly."""
+    """bf16 copy of a parameter for a graph under recording, with the parameter's strides.  The parameters of a
+    ``FlatParams`` are cast together, once per recording: a cast per parameter is a launch per parameter, 2.4 us each for the
+    52 convolution weights of a ResNet-50 against 21 us for the whole buffer.  The copy (two bytes a parameter, 64 MB at
+    most) lives as long as the recording, where single casts are freed layer by layer.  Cast singly: larger buffers, whose
+    casts are bound by memory one by one; tensors that are no parameter of such a buffer (a computed weight may be freed within
+    the recording and its address used again); and a parameter written in place since the buffer was cast (by its version, as in
+    the caches of eager calls)."""
     w = weight.detach()
-    store = w.untyped_storage()
-    total = store.nbytes() // 4
     rec = _recording()
-    if rec is None or w.dtype != torch.float32 or not w.numel() < total <= _FLAT_COPY_MAX:
+    owner = weight._base if weight._base is not None else weight
+    if rec is None or w.dtype != torch.float32:
         return w.to(torch.bfloat16)
-    key = store.data_ptr()
-    if key not in rec.copies:
-        flat = torch.empty(0, dtype=torch.float32, device=w.device).set_(store, 0, (total,), (1,))
-        rec.copies[key] = flat.to(torch.bfloat16)
-    return rec.copies[key].as_strided(w.shape, w.stride(), w.storage_offset())
+    store = w.untyped_storage().data_ptr()
+    for ref in _FLAT_PARAMS.valuerefs():
+        flat = ref()
+        if flat is not None and flat.data.untyped_storage().data_ptr() == store \
+                and flat.total <= _FLAT_COPY_MAX:
+            if flat not in rec.copies:
+                rec.copies[flat] = (flat.data.to(torch.bfloat16), {id(p): p._version for p in flat.params})
+            copy, versions = rec.copies[flat]
+            if versions.get(id(owner)) == owner._version:
+                return copy.as_strided(w.shape, w.stride(), w.storage_offset() - flat.data.storage_offset())
+    return w.to(torch.bfloat16)
 
 
 def recorded_grad(p: Optional[torch.Tensor]) -> Optional[torch.Tensor]:

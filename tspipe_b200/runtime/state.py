@@ -18,6 +18,8 @@ from typing import List, Sequence, Tuple
 import torch
 from torch import nn
 
+from ..ops.fused import register_flat
+
 ALIGN = 64          # elements; 256 B for fp32 so every tensor starts on a vector-load boundary
 
 
@@ -46,6 +48,8 @@ class FlatParams:
         self.data = torch.zeros(self.total, dtype=dtype, device=device)
         self.grad = torch.zeros(self.total, dtype=dtype, device=device) if with_grad else None
         self._bind()
+        if dtype == torch.float32:
+            register_flat(self)
 
     def _view(self, flat: torch.Tensor, i: int, like: torch.Tensor) -> torch.Tensor:
         seg = flat[self.offsets[i]: self.offsets[i] + self.numels[i]]
