@@ -1,4 +1,6 @@
 """What the launches of a stage under recording share, and where they take other ways than eager ones."""
+import threading
+
 import torch
 from torch import nn
 
@@ -40,3 +42,19 @@ def test_recorded_copy_follows_a_parameter_written_in_place():
         ps[1].mul_(3.0)                                 # a layer that renormalises its weight before it uses it
         assert torch.equal(fused.recorded_bf16(ps[1]), ps[1].bfloat16())
         assert torch.equal(fused.recorded_bf16(ps[0]), ps[0].bfloat16())
+
+
+def test_gradients_are_added_in_place_only_where_they_are_recorded(monkeypatch):
+    """Not on another thread's stream while one is recorded, and not past a parameter's hooks."""
+    ps, flat = _flat((7,), (9,), (11,))
+    ps[1].register_hook(lambda g: 2 * g)
+    ps[2].register_post_accumulate_grad_hook(lambda p: None)
+    monkeypatch.setattr(fused, "_stream_key", threading.get_ident)       # a stream of its own per thread
+    seen = []
+    with fused.capturing():
+        assert fused.recorded_grad(ps[0]) is ps[0].grad
+        assert fused.recorded_grad(ps[1]) is None and fused.recorded_grad(ps[2]) is None
+        t = threading.Thread(target=lambda: seen.append(fused.recorded_grad(ps[0])))
+        t.start()
+        t.join()
+    assert seen == [None] and fused.recorded_grad(ps[0]) is None

@@ -149,12 +149,17 @@ def recorded_bf16(weight: torch.Tensor) -> torch.Tensor:
     return w.to(torch.bfloat16)
 
 
+def adds_in_place(p: Optional[torch.Tensor]) -> bool:
+    """Whether a backward adds a parameter's gradient where it lies instead of handing it to autograd: on a stream whose
+    launches are being recorded (elsewhere, also on other threads meanwhile, the gradient may have been asked for by name),
+    for a leaf without hooks that want to see it."""
+    return (_recording() is not None and p is not None and p.is_leaf and p.requires_grad
+            and not p._backward_hooks and not p._post_accumulate_grad_hooks)
+
+
 def recorded_grad(p: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """The fp32 gradient buffer of a leaf parameter that a backward under recording adds to in place, or None.  (Outside
-    a recording the gradient is handed to autograd, which may have been asked for it by name.)"""
-    if IN_CAPTURE == 0 or p is None or not (p.is_leaf and p.requires_grad):
-        return None
-    g = p.grad
+    """The fp32 gradient buffer of a parameter that a backward adds to in place, or None."""
+    g = p.grad if adds_in_place(p) else None
     return g if g is not None and g.dtype == torch.float32 and g.is_contiguous() and g.shape == p.shape else None
 
 
