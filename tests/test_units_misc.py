@@ -147,3 +147,23 @@ def test_bench_cuts_and_grids_are_consistent():
         for pp, dp, ub in bench.pipeline_grids(world, "byol"):
             assert pp * dp == world and pp in bench.BYOL_SPLITS and (128 * world // dp) % ub == 0
     assert bench.pipeline_grids(8, "moco") == []
+
+
+def test_hooks_on_all_modules_see_the_norms_of_a_block_and_the_pooling_of_a_stem():
+    """A hook registered for every module (a profiler's, a module tracker's) is called for the modules whose work a fused pass
+    would otherwise take over."""
+    import torch
+    from torch.nn.modules.module import register_module_forward_hook
+    from tspipe_b200.models.vit import Block, LayerNorm, ViTConfig
+    from tspipe_b200.ops.pool import MaxPool3x3s2
+    from tspipe_b200.runtime.fuse import has_hooks
+    blk, x, seen = Block(ViTConfig(embed_dim=64, num_heads=2)), torch.randn(2, 5, 64), []
+    ref = blk(x)
+    handle = register_module_forward_hook(lambda m, args, out: seen.append(m))
+    try:
+        assert torch.equal(blk(x), ref)
+        assert has_hooks(MaxPool3x3s2())
+    finally:
+        handle.remove()
+    assert [m for m in seen if isinstance(m, LayerNorm)] == [blk.norm1, blk.norm2]
+    assert not has_hooks(MaxPool3x3s2())

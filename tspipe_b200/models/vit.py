@@ -28,6 +28,7 @@ from torch import nn
 from ..ops import fused
 from ..ops.attention import attention, packed_attention, project_qkv, qkv_mode
 from ..ops.linear import linear, linear_gelu
+from ..runtime.fuse import has_hooks
 
 
 @dataclass
@@ -65,8 +66,7 @@ def norm_of_sum(norm: nn.Module, x: torch.Tensor, a: Optional[torch.Tensor] = No
                 ) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
     """``(s, norm(s))`` for ``s = x + a``, or for ``s = x`` that goes on as a residual connection; in one pass when ``norm``
     is this file's LayerNorm and nothing hooks into it.  ``s`` may be None without ``need_sum``."""
-    if type(norm) is LayerNorm and not (norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks
-                                        or norm._backward_pre_hooks):
+    if type(norm) is LayerNorm and not has_hooks(norm):
         return fused.add_layer_norm(x, a, norm.weight, norm.bias, norm.eps, need_sum)
     s = x if a is None else x + a
     return s, norm(s)

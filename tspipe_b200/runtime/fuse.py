@@ -22,10 +22,13 @@ from typing import Any, List
 import torch
 from torch import nn
 from torch.nn.modules.batchnorm import _BatchNorm
+from torch.nn.modules.module import _has_any_global_hook
 
 
-def _has_hooks(m: nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+def has_hooks(m: nn.Module) -> bool:
+    """Whether something watches calls of ``m``: hooks of its own, or ones on all modules (profilers, module trackers)."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or _has_any_global_hook())
 
 
 class FusedSequential(nn.Sequential):
@@ -48,7 +51,7 @@ class FusedSequential(nn.Sequential):
                 y, sums = _conv.stem_conv(x, m.weight, want_sums=bn_next, segments=segs)
                 if bn_next and _bn.applicable(nxt, y):
                     relu = i + 2 < n and isinstance(mods[i + 2], nn.ReLU)
-                    if relu and i + 3 < n and type(mods[i + 3]) is MaxPool3x3s2 and not _has_hooks(mods[i + 3]):
+                    if relu and i + 3 < n and type(mods[i + 3]) is MaxPool3x3s2 and not has_hooks(mods[i + 3]):
                         z = _bn.bn_relu_pool(nxt, y, sums=sums)
                         if z is not None:
                             x, i = z, i + 4
