@@ -207,6 +207,34 @@ def test_batchnorm_passes_at_odd_widths(m, c, res, dtype):
         assert _rel(a, b) < 4 * EPS[dtype] + 2e-5
 
 
+@pytest.mark.parametrize("train,relu,res", [(True, True, False), (True, False, False), (True, True, True), (False, False, False),
+                                            (False, True, False)])
+def test_batchnorm_with_parameters_anywhere_in_a_vector(train, relu, res):
+    """Weight and bias as slices of one vector, off the 16-byte grid, give what aligned ones give."""
+    from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
+    from tspipe_b200.ops import bn as fbn
+    c = 64
+    torch.manual_seed(19)
+    x, r, g = (_cl(4, c, 6, 10) for _ in range(3))
+    vec = torch.cat([torch.zeros(1, device=DEV), torch.randn(2 * c, device=DEV)])
+    outs = []
+    for off in (0, 1):
+        mod = DeferredBatchNorm(c).to(DEV).train(train)
+        BatchNormGroup(mod, chunks=10)
+        flat = vec[1:].clone() if off == 0 else vec
+        torch.nn.utils.vector_to_parameters(flat[off:], mod.parameters())
+        assert (mod.weight.data_ptr() % 16 != 0) == (off != 0)
+        xi = x.clone(memory_format=torch.preserve_format).requires_grad_()
+        y = fbn.bn_act(mod, xi, r if res else None, relu)
+        out = [y, *torch.autograd.grad(y, [xi, mod.weight, mod.bias], g)]
+        if train and relu and not res:
+            z = fbn.bn_relu_pool(mod, xi)
+            out += [z, *torch.autograd.grad(z, [xi, mod.weight, mod.bias], _cl(*z.shape).fill_(1.0))]
+        outs.append(out)
+    for a, b in zip(*outs):
+        assert _rel(a, b) < 1e-3                       # the sums' additions come in any order: a rounding here and there
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gelu_special_values_and_wide_bias(dtype):
     from tspipe_b200.ops import fused

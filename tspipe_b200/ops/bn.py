@@ -116,8 +116,7 @@ class _BnAct(torch.autograd.Function):
         # statistics handed over by the producer of x (a convolution epilogue) replace the statistics pass
         sums = pre_sums if pre_sums is not None else torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
         save = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
-        wf = weight.detach() if weight.dtype == torch.float32 else weight.detach().float()
-        bf = bias.detach() if bias.dtype == torch.float32 else bias.detach().float()
+        wf, bf = _f.param_f32(weight), _f.param_f32(bias)
         with _f.on_device(x.device):
             st = _f._stream()
             if fixed is None and pre_sums is None:
@@ -260,8 +259,7 @@ class _BnReluPool(torch.autograd.Function):
                         memory_format=torch.channels_last)
         idx = torch.empty(y.numel(), dtype=torch.uint8, device=x.device) if any(ctx.needs_input_grad[:3]) else None
         save = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
-        wf = weight.detach() if weight.dtype == torch.float32 else weight.detach().float()
-        bf = bias.detach() if bias.dtype == torch.float32 else bias.detach().float()
+        wf, bf = _f.param_f32(weight), _f.param_f32(bias)
         with _f.on_device(x.device):
             st = _f._stream()
             if sums is None:

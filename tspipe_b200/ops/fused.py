@@ -189,6 +189,15 @@ def _check(code: int, what: str) -> None:
         raise RuntimeError(f"{what} failed with code {code}")
 
 
+def param_f32(p: torch.Tensor) -> torch.Tensor:
+    """A weight or bias vector as the kernels read it: fp32, contiguous, on a 16-byte boundary (a parameter may be a slice of
+    any vector)."""
+    t = p.detach()
+    if t.dtype != torch.float32 or not t.is_contiguous():
+        t = t.float().contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _dt(t: torch.Tensor) -> int:
     if t.dtype == torch.float32:
         return 0
