@@ -235,6 +235,23 @@ def test_batchnorm_with_parameters_anywhere_in_a_vector(train, relu, res):
         assert _rel(a, b) < 1e-3                       # the sums' additions come in any order: a rounding here and there
 
 
+def test_layer_norm_and_gelu_with_parameters_anywhere_in_a_vector():
+    """Weights and biases as slices of a vector, off the 16-byte grid, give what aligned ones give."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(20)
+    d = 72
+    x, a, g = (torch.randn(9, d, device=DEV) for _ in range(3))
+    x.requires_grad_()
+    vec = torch.randn(3 * d + 1, device=DEV)
+    outs = []
+    for w, b, c in (vec[1:].view(3, d).unbind(0), vec[1:].clone().view(3, d).unbind(0)):
+        w, b, c = (t.detach().requires_grad_() for t in (w, b, c))
+        ys = [fused.layer_norm(x, w, b), *fused.add_layer_norm(x, a, w, b), fused.gelu(x, c)]
+        outs.append([t for y in ys for t in (y, *torch.autograd.grad(y, [x], g, retain_graph=True))])
+    for p, q in zip(*outs):
+        assert torch.equal(p, q)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gelu_special_values_and_wide_bias(dtype):
     from tspipe_b200.ops import fused

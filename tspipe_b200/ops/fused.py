@@ -472,7 +472,7 @@ class _LayerNorm(torch.autograd.Function):
         y = torch.empty_like(x2)
         mean = torch.empty(rows, dtype=torch.float32, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        wf, bf = w.detach().float().contiguous(), b.detach().float().contiguous()
+        wf, bf = param_f32(w), param_f32(b)
         with on_device(x.device):
             _check(lib().tsp_layernorm_fwd(_ptr(x2), _ptr(wf), _ptr(bf), _ptr(y), _ptr(mean), _ptr(rstd),
                                            _c.c_int(rows), _c.c_int(d), _c.c_float(eps), _c.c_int(_dt(x2)), _stream()),
@@ -526,7 +526,7 @@ class _AddLayerNorm(torch.autograd.Function):
         y = torch.empty_like(x)
         mean = torch.empty(rows, dtype=torch.float32, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        wf, bf = w.detach().float().contiguous(), b.detach().float().contiguous()
+        wf, bf = param_f32(w), param_f32(b)
         with on_device(x.device):
             _check(lib().tsp_add_layernorm_fwd(_ptr(x), _ptr(a), _ptr(s), _ptr(wf), _ptr(bf), _ptr(y), _ptr(mean), _ptr(rstd),
                                                _c.c_int(rows), _c.c_int(d), _c.c_float(eps), _c.c_int(_dt(x)), _stream()),
@@ -577,7 +577,7 @@ class _Gelu(torch.autograd.Function):
         x = x.contiguous()
         d = x.shape[-1]
         y = torch.empty_like(x)
-        bf = None if bias is None else bias.detach().float().contiguous()
+        bf = None if bias is None else param_f32(bias)
         with on_device(x.device):
             _check(lib().tsp_gelu_fwd(_ptr(x), _ptr(bf), _ptr(y), _c.c_int64(x.numel()), _c.c_int(d), _c.c_int(_dt(x)),
                                       _stream()), "tsp_gelu_fwd")

@@ -286,9 +286,7 @@ class _LinearGelu(torch.autograd.Function):
     def forward(ctx, x, weight, bias, grads):
         x2 = _bf16_rows(x, x.shape[-1])
         (m, k), n = x2.shape, weight.shape[0]
-        bf = bias.detach().float().contiguous()
-        if bf.data_ptr() % 16:
-            bf = bf.clone()
+        bf = _f.param_f32(bias)
         act = torch.empty((m, n), dtype=torch.bfloat16, device=x2.device)
         h = torch.empty_like(act) if grads and any(ctx.needs_input_grad) else None
         with _f.on_device(x2.device):
