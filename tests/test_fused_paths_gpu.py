@@ -440,6 +440,22 @@ def test_stem_weight_gradient(n, h, w):
     assert _rel(weight.grad - 1, want) < 1e-5
 
 
+def test_stem_weight_gradient_by_name_and_past_hooks():
+    """Eagerly the gradient goes to autograd, also where a channels-last one is there already: whoever asks for it by name
+    gets it, and hooks see it."""
+    from tspipe_b200.ops import conv
+    torch.manual_seed(21)
+    x, g = _cl(2, 3, 16, 16), _cl(2, 64, 8, 8)
+    weight = (torch.randn(64, 3, 7, 7, device=DEV) * 0.1).to(memory_format=torch.channels_last).requires_grad_()
+    want = torch.autograd.grad(conv.stem_conv(x, weight)[0], weight, g)[0]
+    weight.grad = torch.ones_like(weight)
+    (got,) = torch.autograd.grad(conv.stem_conv(x, weight)[0], weight, g)
+    assert _rel(got, want) < 1e-6 and torch.equal(weight.grad, torch.ones_like(weight))
+    weight.register_hook(lambda t: 2 * t)
+    conv.stem_conv(x, weight)[0].backward(g)
+    assert _rel(weight.grad - 1, 2 * want) < 1e-5
+
+
 @pytest.mark.parametrize("n,h,w,cin,cout,k", [(1, 8, 16, 64, 256, 1), (3, 10, 10, 128, 256, 1), (2, 7, 7, 512, 512, 1),
                                               (1, 8, 8, 64, 64, 3), (3, 13, 9, 64, 64, 3), (2, 5, 61, 64, 64, 3),
                                               (2, 56, 56, 64, 64, 3), (1, 64, 2, 64, 64, 3), (200, 8, 8, 64, 64, 3)])

@@ -84,7 +84,8 @@ class _StemConv(torch.autograd.Function):
             dx = torch.ops.aten.convolution_backward(dy, x, weight.to(torch.bfloat16), None, [2, 2], [3, 3], [1, 1], False,
                                                      [0, 0], 1, [True, False, False])[0]
         if ctx.needs_input_grad[1]:
-            target = _grad_target(weight)
+            # (added in place in a recording only: an eager call may have asked for this gradient by name)
+            target = _grad_target(weight) if _f.adds_in_place(weight) else None
             if target is None:
                 target = torch.zeros((64, 7, 7, 3), dtype=torch.float32, device=x.device)
                 dw = target.permute(0, 3, 1, 2)
