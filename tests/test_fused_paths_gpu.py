@@ -520,3 +520,22 @@ def test_loss_gradient_scaling_in_place_and_not():
     assert torch.equal(one, again) and torch.equal(half.float(), one.float() * 0.5)
     (last,) = torch.autograd.grad(loss, s, torch.tensor(2.0, device=DEV))
     assert torch.equal(last.float(), one.float() * 2)
+
+
+def test_loss_gradient_scaling_leaves_what_saved_tensor_hooks_keep():
+    from tspipe_b200 import losses
+    from tspipe_b200.ops import fused
+    torch.manual_seed(22)
+    o1, o2, t1, t2 = (torch.randn(128, 256, device=DEV) for _ in range(4))
+    o1.requires_grad_()
+    y = torch.randint(0, 256, (128,), device=DEV)
+    for loss in (lambda: losses.byol_loss(o1, o2, t1, t2), lambda: losses.moco_loss(o1, o2, t1, t2),
+                 lambda: fused.cross_entropy(o1, y), lambda: fused.cosine_embedding_loss(o1, t1, 1.0),
+                 lambda: fused.byol_pair_loss(o1, t1, 1.0)):
+        kept = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(t) or t, lambda t: t):
+            value = loss()
+        before = [t.clone() for t in kept]
+        (g,) = torch.autograd.grad(value, o1, torch.tensor(3.0, device=DEV))
+        assert kept and all(torch.equal(a, b) for a, b in zip(kept, before))
+        assert _rel(g, 3 * torch.autograd.grad(loss(), o1)[0]) < 1e-6

@@ -302,15 +302,23 @@ def _plain(t: torch.Tensor) -> bool:
                                             or torch._C._functorch.is_functorch_wrapped_tensor(t))
 
 
-def _scaled(g: torch.Tensor, gout: torch.Tensor) -> torch.Tensor:
+def save_gradient(ctx, g: torch.Tensor) -> None:
+    """Saves a gradient that a forward has computed for :func:`_scaled`, and whether it stays this function's own: hooks on
+    saved tensors may keep what they are given, or hand out the same tensor elsewhere."""
+    ctx.save_for_backward(g)
+    ctx.own = torch._C._autograd._top_saved_tensors_default_hooks(False) is None
+
+
+def _scaled(g: torch.Tensor, gout: torch.Tensor, own: bool) -> torch.Tensor:
     """``g * gout`` for a gradient ``g`` that the forward has computed and saved and the loss's gradient ``gout`` (a scalar).
     As plain ops where the product is recorded itself (``create_graph``) or ``gout`` is no plain fp32 scalar.  In place where
-    the graph is freed behind this backward, so that nobody else will read ``g`` (a CUDA graph may be replayed: not
-    there); then ``gout = 1``, a loss that is differentiated as it is, costs no pass over the gradient."""
+    ``g`` is the function's ``own`` and the graph is freed behind this backward, so that nobody else will read it (a CUDA graph
+    may be replayed: not there); then ``gout = 1``, a loss that is differentiated as it is, costs no pass over the gradient."""
     if (torch.is_grad_enabled() or not (_plain(g) and _plain(gout)) or gout.dtype != torch.float32 or gout.dim() != 0
             or gout.device != g.device or not g.is_contiguous() or g.data_ptr() % 16):
         return g * gout.to(g.dtype)
-    own = not torch._C._autograd._get_current_graph_task_keep_graph() and not torch.cuda.is_current_stream_capturing()
+    own = (own and not torch._C._autograd._get_current_graph_task_keep_graph()
+           and not torch.cuda.is_current_stream_capturing())
     out = g if own else torch.empty_like(g)
     with on_device(g.device):
         _check(lib().tsp_scale(_ptr(g), _ptr(gout), _ptr(out), _c.c_int64(g.numel()), _c.c_int(_dt(g)), _stream()),
@@ -331,13 +339,13 @@ class _ByolPair(torch.autograd.Function):
             _check(lib().tsp_byol_loss(_ptr(x), _ptr(y), _c.c_int(n), _c.c_int(d), _c.c_int(_dt(x)),
                                        _c.c_float(scale), _ptr(loss), _ptr(gx), _stream()), "tsp_byol_loss")
         _count()
-        ctx.save_for_backward(gx)
+        save_gradient(ctx, gx)
         return loss
 
     @staticmethod
     def backward(ctx, gout):
         (gx,) = ctx.saved_tensors
-        return _scaled(gx, gout), None, None
+        return _scaled(gx, gout, ctx.own), None, None
 
 
 def byol_pair_loss(x: torch.Tensor, y: torch.Tensor, scale: float) -> torch.Tensor:
@@ -359,13 +367,13 @@ class _ByolBoth(torch.autograd.Function):
                                             _c.c_int(_dt(x1)), _c.c_float(scale), _ptr(loss), _ptr(gx), _stream()),
                    "tsp_byol_loss_pair")
         _count()
-        ctx.save_for_backward(gx)
+        save_gradient(ctx, gx)
         return loss
 
     @staticmethod
     def backward(ctx, gout):
         (gx,) = ctx.saved_tensors
-        g1, g2 = _scaled(gx, gout).unbind(0)
+        g1, g2 = _scaled(gx, gout, ctx.own).unbind(0)
         need = ctx.needs_input_grad
         return g1 if need[0] else None, g2 if need[1] else None, None, None, None
 
@@ -398,14 +406,14 @@ class _KdCe(torch.autograd.Function):
                                         _c.c_float(w_ce), _c.c_float(w_kd), _ptr(total), _ptr(loss), _ptr(gs), _stream()),
                    "tsp_kd_ce_loss")
         _count(2)
-        ctx.save_for_backward(gs)
+        save_gradient(ctx, gs)
         ctx.shape = s.shape
         return loss
 
     @staticmethod
     def backward(ctx, gout):
         (gs,) = ctx.saved_tensors
-        return _scaled(gs, gout).view(ctx.shape), None, None, None, None, None, None
+        return _scaled(gs, gout, ctx.own).view(ctx.shape), None, None, None, None, None, None
 
 
 def kd_ce_loss(s, t, labels, temp: float, w_ce: float, w_kd: float, row_mask=None) -> torch.Tensor:
@@ -440,14 +448,14 @@ class _Cosine(torch.autograd.Function):
                                          _c.c_float(scale), _ptr(total), _ptr(loss), _ptr(gx), _stream()),
                    "tsp_cosine_loss")
         _count(2)
-        ctx.save_for_backward(gx)
+        save_gradient(ctx, gx)
         ctx.shape = x.shape
         return loss
 
     @staticmethod
     def backward(ctx, gout):
         (gx,) = ctx.saved_tensors
-        return _scaled(gx, gout).view(ctx.shape), None, None, None
+        return _scaled(gx, gout, ctx.own).view(ctx.shape), None, None, None
 
 
 def cosine_embedding_loss(x, y, scale: float, row_mask=None) -> torch.Tensor:

@@ -531,13 +531,13 @@ class _NCEPair(torch.autograd.Function):
                                   _f._ptr(lse), _f._ptr(loss), _f._ptr(gq), _f._ptr(_status_word(dev)), _f._stream())
         _f._check(code, "tsp_nce_pair")
         _f._count(3)
-        ctx.save_for_backward(gq)
+        _f.save_gradient(ctx, gq)
         return loss
 
     @staticmethod
     def backward(ctx, gout):
         (gq,) = ctx.saved_tensors
-        g1, g2 = _f._scaled(gq, gout).unbind(0)
+        g1, g2 = _f._scaled(gq, gout, ctx.own).unbind(0)
         need = ctx.needs_input_grad
         return g1 if need[0] else None, g2 if need[1] else None, None, None, None
 
