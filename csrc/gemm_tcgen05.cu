@@ -49,9 +49,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
     // The error word lives in global memory, so this check costs a round trip to L2 per failed poll.  That is
     // deliberate: it is the back-off of the spin loop.  Polling the barrier flat out was measured slower (the
     // waiting warps take issue slots from the one thread that feeds the pipeline).
-    if (*((volatile int*)status) != 0) return false;
+    if (*((volatile int*)status) != 0) break;
   }
   atomicCAS(status, 0, code);
+  // what this CTA has in flight (copies, products) lands before the block's end lets its memory go to another one
+#pragma unroll 1
+  for (int i = 0; i < 64; ++i) __nanosleep(1000);
   return false;
 }
 

@@ -38,6 +38,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t addr, uint32_t parity) {
   return done != 0;
 }
 
+// A role whose wait ran out pauses before it leaves: what its CTA has in flight (copies into shared memory, products, all of
+// which take microseconds) lands before the barrier in front of the kernel's end lets the memory go to another block.
+__device__ __forceinline__ void drain_in_flight() {
+#pragma unroll 1
+  for (int i = 0; i < 64; ++i) __nanosleep(1000);
+}
+
 // Bounded wait.  Returns false (and leaves `code` in *status unless another role got there first) when the phase
 // did not complete within `limit_ns` nanoseconds.  mbarrier.try_wait suspends the thread for a short,
 // hardware-chosen time per attempt, so the loop does not fight the issuing threads for slots; every 32 failed
@@ -51,12 +58,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
 #pragma unroll 1
     for (int i = 0; i < 32; ++i)
       if (mbar_try_wait(addr, parity)) return true;
-    if (*((volatile int*)status) != 0) return false;
+    if (*((volatile int*)status) != 0) break;
     const uint64_t now = global_timer_ns();
     if (t0 == 0) t0 = now;
     else if (now - t0 > limit_ns) break;
   }
   atomicCAS(status, 0, code);
+  drain_in_flight();
   return false;
 }
 
@@ -80,12 +88,13 @@ __device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity,
           : "memory");
       if (done) return true;
     }
-    if (*((volatile int*)status) != 0) return false;
+    if (*((volatile int*)status) != 0) break;
     const uint64_t now = global_timer_ns();
     if (t0 == 0) t0 = now;
     else if (now - t0 > limit_ns) break;
   }
   atomicCAS(status, 0, code);
+  drain_in_flight();
   return false;
 }
 // The same for a whole warp: lane 0 waits, the others park at the warp barrier; every lane gets the result.
