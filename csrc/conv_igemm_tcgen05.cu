@@ -817,7 +817,8 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int m = mt * 128 + quarter * 32 + lane;             // index into the (tap, ci) axis
-      const bool row_ok = m < m_blocks * 64 && b_hi > b_lo;     // (an empty pixel range leaves the accumulator unset)
+      // an empty pixel range leaves the accumulator unset, a wait that ran out may leave part of a sum in it
+      const bool row_ok = m < m_blocks * 64 && b_hi > b_lo && *((volatile int*)status) == 0;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         const int co0 = nt * BN + c0;

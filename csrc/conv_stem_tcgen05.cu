@@ -498,7 +498,9 @@ conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_b
   if (warp < kProducers / 32) {
     produce_tiles(a_tiles, ring, full_bar, empty_bar, x, h, w, oh_n, ow_n, t_begin, t_end, status, tid, lane);
     // ---------------- epilogue: warps 0..3, TMEM lanes 32 * warp .. + 31 ----------------
-    if (warp < 4 && t_begin < t_end && __all_sync(0xffffffffu, mbar_wait(done_bar, 0, status, 3))) {
+    // (after a wait that ran out the accumulators hold part of their sums, or nothing: none of it is added)
+    if (warp < 4 && t_begin < t_end &&
+        __all_sync(0xffffffffu, mbar_wait(done_bar, 0, status, 3) && *((volatile int*)status) == 0)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int part = 0; part < 2; ++part) {

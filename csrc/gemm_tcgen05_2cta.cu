@@ -348,6 +348,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
       ok = tc5::mbar_wait_warp(tmem_full_bar + acc, use & 1, status, 3, kWaitNs, lane);   // one way out per warp
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      bool live = true;                            // after a wait that ran out the accumulator may hold part of its sum
+      if constexpr (KIND == kRed) live = *((volatile int*)status) == 0;
       const int row0 = m0 + quarter * 32, row = row0 + lane;
       // the block's values -> swizzled staging buffer -> TMA store at column x of `map`; returns the buffer
       auto stage = [&](const float (&v)[kCols], const CUtensorMap* map, int x, bool inside) -> uint8_t* {
@@ -437,7 +439,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
         }
         if (tma_store) {
           const int dst = KIND == kTN ? col / n_per : 0;
-          const uint8_t* buf = stage(v, &tmap_c.m[dst], col - dst * n_per, row0 < m && col < n);
+          const uint8_t* buf = stage(v, &tmap_c.m[dst], col - dst * n_per, live && row0 < m && col < n);
           if (STATS && st != nullptr) {
             // column sums of the staged (rounded) block: lane owns columns 2*lane, 2*lane+1; rows past the
             // matrix edge hold exact zeros (their A rows were zero-filled)

@@ -539,3 +539,34 @@ def test_loss_gradient_scaling_leaves_what_saved_tensor_hooks_keep():
         (g,) = torch.autograd.grad(value, o1, torch.tensor(3.0, device=DEV))
         assert kept and all(torch.equal(a, b) for a, b in zip(kept, before))
         assert _rel(g, 3 * torch.autograd.grad(loss(), o1)[0]) < 1e-6
+
+
+def test_weight_gradients_add_nothing_after_a_wait_that_ran_out():
+    """The status word as a wait that gave up leaves it: every role leaves, gradients that are there stay as they are, and the
+    next check reports it."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(23)
+    word = gemm._status_word(DEV)
+    a = torch.randn(300, 128, device=DEV).bfloat16()
+    target = torch.ones(128, 128, device=DEV)
+    layers = [(_cl(2, cin, 12, 12), (torch.randn(cout, cin, 3, 3, device=DEV) * 0.1).to(memory_format=torch.channels_last))
+              for cin, cout in ((64, 64), (64, 128))]
+    ys = []
+    for x, w in layers:
+        w.requires_grad_().grad = torch.ones_like(w)
+        ys.append(conv.conv2d(x, w)[0])
+    gs = [_cl(*y.shape) for y in ys]
+    gemm.check_status()
+    word.fill_(7)
+    gemm._add_weight_grad(target, [a], a)
+    torch.autograd.backward(ys, gs)
+    x, dw, dy = _cl(2, 3, 16, 16), torch.ones(64, 147, device=DEV), _cl(2, 64, 8, 8)
+    assert conv._f.lib().tsp_conv_stem_wgrad(conv._f._ptr(x), conv._f._ptr(dy), conv._f._ptr(dw), 2, 16, 16, conv._f._ptr(word),
+                                             conv._f._stream()) == 0
+    with pytest.raises(RuntimeError, match="role 7"):
+        gemm.check_status()
+    for t in [target, dw] + [w.grad for _, w in layers]:
+        assert torch.equal(t, torch.ones_like(t))
+    gemm._add_weight_grad(target, [a], a)              # the context stays usable
+    gemm.check_status()
+    assert _rel(target - 1, a.double().t() @ a.double()) < 1e-5
