@@ -133,6 +133,18 @@ inline int row_stride_blocks(int64_t nvec, int cpv, int threads, int per_thread,
   return (int)((g + unit - 1) / unit * unit);
 }
 
+// Hyperparameters of an optimizer's parameter groups for one launch.  They change from step to step (learning rates, bias
+// corrections), so they travel with the launch: a table in device memory would have to be copied before each step.  Few
+// groups go by value; a table serves more of them.  What does not change is a code per segment: group << 1 | adapt.
+constexpr int kHyperVals = 8, kHyperGroups = 32;
+struct Hyper {                                // (filled in by the caller: optim/flat.py has the same layout)
+  const int* seg_code;                        // device memory
+  const float* table;                         // [groups][kHyperVals] in device memory, or null
+  float by_value[kHyperGroups][kHyperVals];
+  __device__ __forceinline__ const float* of(int code) const {
+    return table != nullptr ? table + kHyperVals * (int64_t)(code >> 1) : by_value[code >> 1];
+  }
+};
 }  // namespace tsp
 
 // Every launcher returns the cudaError_t of its launch as int (0 = ok).

@@ -11,6 +11,8 @@
 
 namespace {
 
+using tsp::Hyper;
+
 constexpr int kThreads = 256;
 
 // ---------------------------------------------------------------------------------------------
@@ -66,16 +68,16 @@ __device__ __forceinline__ int vec4_body(const ChunkView& c, uintptr_t bits, boo
   return ((c.begin & 3) == 0 && (bits & 15) == 0 && !(has_t && (teacher_n & 3) != 0)) ? c.len >> 2 : 0;
 }
 
-// norms[2*seg] += sum p^2 ; norms[2*seg+1] += sum (grad_scale*g + wd*p)^2   (only segments with adapt != 0)
+// norms[2*seg] += sum p^2 ; norms[2*seg+1] += sum (grad_scale*g + wd*p)^2   (only segments with the adapt bit)
 __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __restrict__ p, const float* __restrict__ g,
                                                               const int64_t* __restrict__ chunks,
-                                                              const float* __restrict__ seg_hp, float grad_scale,
+                                                              const __grid_constant__ Hyper hyper, float grad_scale,
                                                               float* __restrict__ norms) {
   __shared__ float scratch[33];
   const ChunkView c = load_chunk(chunks, blockIdx.x);
-  const float* hp = seg_hp + 5 * (int64_t)c.seg;      // lr, wd, momentum, trust, adapt
-  if (hp[4] == 0.f) return;
-  const float wd = hp[1];
+  const int code = hyper.seg_code[c.seg];
+  if ((code & 1) == 0) return;
+  const float wd = hyper.of(code)[1];                 // lr, wd, momentum, trust
   float sp = 0.f, su = 0.f;
   const bool vec = ((c.begin & 3) == 0);
   if (vec) {
@@ -118,14 +120,15 @@ __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __res
 __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict__ p, const float* __restrict__ g,
                                                               float* __restrict__ mu,
                                                               const int64_t* __restrict__ chunks,
-                                                              const float* __restrict__ seg_hp, float grad_scale,
+                                                              const __grid_constant__ Hyper hyper, float grad_scale,
                                                               const float* __restrict__ norms,
                                                               float* __restrict__ teacher, int64_t teacher_n,
                                                               float ema_m, int last_first) {
   const ChunkView c = load_chunk(chunks, last_first ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
-  const float* hp = seg_hp + 5 * (int64_t)c.seg;
+  const int code = hyper.seg_code[c.seg];
+  const float* hp = hyper.of(code);
   const float lr = hp[0], wd = hp[1], mom = hp[2], trust = hp[3];
-  const bool adapt = hp[4] != 0.f;
+  const bool adapt = (code & 1) != 0;
   float q = 1.f;
   if (adapt) {
     const float pn = sqrtf(norms[2 * c.seg]), un = sqrtf(norms[2 * c.seg + 1]);
@@ -171,14 +174,14 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
   }
 }
 
-// AdamW (decoupled weight decay), per-segment hyper-parameters: lr, beta1, beta2, eps, wd, bias1, bias2
+// AdamW (decoupled weight decay), hyper-parameters of a group: lr, beta1, beta2, eps, wd, bias1, bias2
 __global__ void __launch_bounds__(kThreads) adamw_kernel(float* __restrict__ p, const float* __restrict__ g,
                                                          float* __restrict__ m, float* __restrict__ v,
                                                          const int64_t* __restrict__ chunks,
-                                                         const float* __restrict__ seg_hp, float grad_scale,
+                                                         const __grid_constant__ Hyper hyper, float grad_scale,
                                                          float* __restrict__ teacher, int64_t teacher_n, float ema_m) {
   const ChunkView c = load_chunk(chunks, blockIdx.x);
-  const float* hp = seg_hp + 7 * (int64_t)c.seg;
+  const float* hp = hyper.of(hyper.seg_code[c.seg]);
   const float lr = hp[0], b1 = hp[1], b2 = hp[2], eps = hp[3], wd = hp[4], bc1 = hp[5], bc2 = hp[6];
   const float om = 1.f - ema_m;
   const float step = lr / bc1;
@@ -225,13 +228,13 @@ __global__ void __launch_bounds__(kThreads) adamw_kernel(float* __restrict__ p, 
   }
 }
 
-// SGD with momentum / nesterov / L2 weight decay; per-segment: lr, momentum, dampening, wd, nesterov, first_step
+// SGD with momentum / nesterov / L2 weight decay; of a group: lr, momentum, dampening, wd, nesterov, first_step
 __global__ void __launch_bounds__(kThreads) sgd_kernel(float* __restrict__ p, const float* __restrict__ g,
                                                        float* __restrict__ buf, const int64_t* __restrict__ chunks,
-                                                       const float* __restrict__ seg_hp, float grad_scale,
+                                                       const __grid_constant__ Hyper hyper, float grad_scale,
                                                        float* __restrict__ teacher, int64_t teacher_n, float ema_m) {
   const ChunkView c = load_chunk(chunks, blockIdx.x);
-  const float* hp = seg_hp + 6 * (int64_t)c.seg;
+  const float* hp = hyper.of(hyper.seg_code[c.seg]);
   const float lr = hp[0], mom = hp[1], damp = hp[2], wd = hp[3];
   const bool nesterov = hp[4] != 0.f, first = hp[5] != 0.f;
   const float om = 1.f - ema_m;
@@ -297,48 +300,48 @@ int tsp_ema_update(float* teacher, const float* student, int64_t n, float moment
   return TSP_LAUNCH_CHECK();
 }
 
-int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const void* hyper,
                   float grad_scale, float* norms, int n_seg, float* teacher, int64_t teacher_n, float ema_m,
                   cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
   cudaError_t e = cudaMemsetAsync(norms, 0, sizeof(float) * 2 * (size_t)n_seg, stream);
   if (e != cudaSuccess) return (int)e;
-  lars_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, chunks, seg_hp, grad_scale, norms);
-  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, seg_hp, grad_scale, norms, teacher,
+  lars_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, chunks, *(const Hyper*)hyper, grad_scale, norms);
+  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms, teacher,
                                                        teacher_n, ema_m, 1);
   return TSP_LAUNCH_CHECK();
 }
 
-int tsp_lars_norms(const float* p, const float* g, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_lars_norms(const float* p, const float* g, const int64_t* chunks, int n_chunks, const void* hyper,
                    float grad_scale, float* norms, int n_seg, cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
   cudaError_t e = cudaMemsetAsync(norms, 0, sizeof(float) * 2 * (size_t)n_seg, stream);
   if (e != cudaSuccess) return (int)e;
-  lars_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, chunks, seg_hp, grad_scale, norms);
+  lars_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, chunks, *(const Hyper*)hyper, grad_scale, norms);
   return TSP_LAUNCH_CHECK();
 }
 
-int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const void* hyper,
                    float grad_scale, const float* norms, float* teacher, int64_t teacher_n, float ema_m,
                    cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
-  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, seg_hp, grad_scale, norms, teacher,
+  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms, teacher,
                                                        teacher_n, ema_m, 0);
   return TSP_LAUNCH_CHECK();
 }
 
 int tsp_adamw_step(float* p, const float* g, float* m, float* v, const int64_t* chunks, int n_chunks,
-                   const float* seg_hp, float grad_scale, float* teacher, int64_t teacher_n, float ema_m,
+                   const void* hyper, float grad_scale, float* teacher, int64_t teacher_n, float ema_m,
                    cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
-  adamw_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, m, v, chunks, seg_hp, grad_scale, teacher, teacher_n, ema_m);
+  adamw_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, m, v, chunks, *(const Hyper*)hyper, grad_scale, teacher, teacher_n, ema_m);
   return TSP_LAUNCH_CHECK();
 }
 
-int tsp_sgd_step(float* p, const float* g, float* buf, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_sgd_step(float* p, const float* g, float* buf, const int64_t* chunks, int n_chunks, const void* hyper,
                  float grad_scale, float* teacher, int64_t teacher_n, float ema_m, cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
-  sgd_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, buf, chunks, seg_hp, grad_scale, teacher, teacher_n, ema_m);
+  sgd_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, buf, chunks, *(const Hyper*)hyper, grad_scale, teacher, teacher_n, ema_m);
   return TSP_LAUNCH_CHECK();
 }
 

@@ -19,6 +19,8 @@
 
 namespace {
 
+using tsp::Hyper;
+
 constexpr int kThreads = 256;
 constexpr int kMaxPeers = 8;
 
@@ -45,13 +47,13 @@ __global__ void __launch_bounds__(kThreads) dp_reduce_norms_kernel(PeerPtrs grad
                                                                    float* __restrict__ g_out,
                                                                    const float* __restrict__ p,
                                                                    const int64_t* __restrict__ chunks,
-                                                                   const float* __restrict__ seg_hp,
+                                                                   const __grid_constant__ Hyper hyper,
                                                                    float* __restrict__ norms) {
   __shared__ float scratch[33];
   const ChunkView c = load_chunk(chunks, blockIdx.x);
-  const float* hp = seg_hp + 5 * (int64_t)c.seg;
-  const bool adapt = norms != nullptr && hp[4] != 0.f;
-  const float wd = hp[1];
+  const int code = hyper.seg_code[c.seg];
+  const bool adapt = norms != nullptr && (code & 1) != 0;
+  const float wd = hyper.of(code)[1];
   float sp = 0.f, su = 0.f;
   // 16-byte peer loads where the chunk starts on a 4-element boundary (flat segments and replica shards do): a
   // quarter of the round trips over NVLink; the last len % 4 elements (and unaligned chunks) go one by one.
@@ -102,12 +104,13 @@ __global__ void __launch_bounds__(kThreads) dp_reduce_norms_kernel(PeerPtrs grad
 __global__ void __launch_bounds__(kThreads) dp_lars_apply_kernel(PeerPtrs params, int n_peers, int self,
                                                                  const float* __restrict__ g, float* __restrict__ mu,
                                                                  const int64_t* __restrict__ chunks,
-                                                                 const float* __restrict__ seg_hp,
+                                                                 const __grid_constant__ Hyper hyper,
                                                                  const float* __restrict__ norms) {
   const ChunkView c = load_chunk(chunks, blockIdx.x);
-  const float* hp = seg_hp + 5 * (int64_t)c.seg;
+  const int code = hyper.seg_code[c.seg];
+  const float* hp = hyper.of(code);
   const float lr = hp[0], wd = hp[1], mom = hp[2], trust = hp[3];
-  const bool adapt = hp[4] != 0.f;
+  const bool adapt = (code & 1) != 0;
   float q = 1.f;
   if (adapt) {
     const float pn = sqrtf(norms[2 * c.seg]), un = sqrtf(norms[2 * c.seg + 1]);
@@ -148,9 +151,9 @@ __global__ void __launch_bounds__(kThreads) dp_lars_apply_kernel(PeerPtrs params
 __global__ void __launch_bounds__(kThreads) dp_adamw_kernel(PeerPtrs grads, PeerPtrs params, int n_peers, int self,
                                                             float scale, float* __restrict__ m, float* __restrict__ v,
                                                             const int64_t* __restrict__ chunks,
-                                                            const float* __restrict__ seg_hp) {
+                                                            const __grid_constant__ Hyper hyper) {
   const ChunkView c = load_chunk(chunks, blockIdx.x);
-  const float* hp = seg_hp + 7 * (int64_t)c.seg;
+  const float* hp = hyper.of(hyper.seg_code[c.seg]);
   const float lr = hp[0], b1 = hp[1], b2 = hp[2], eps = hp[3], wd = hp[4], bc1 = hp[5], bc2 = hp[6];
   const float step = lr / bc1, inv_sqrt_bc2 = rsqrtf(bc2);
   const float* p_self = params.p[self];
@@ -407,7 +410,7 @@ int tsp_sum_norms(const float* table, int n_peers, int n, float* norms, cudaStre
 }
 
 int tsp_dp_reduce_norms(void* const* grads, int n_peers, float scale, float* g_out, const float* p,
-                        const int64_t* chunks, int n_chunks, const float* seg_hp, float* norms, int n_seg,
+                        const int64_t* chunks, int n_chunks, const void* hyper, float* norms, int n_seg,
                         cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
   PeerPtrs gp;
@@ -416,25 +419,25 @@ int tsp_dp_reduce_norms(void* const* grads, int n_peers, float scale, float* g_o
     cudaError_t e = cudaMemsetAsync(norms, 0, sizeof(float) * 2 * (size_t)n_seg, stream);
     if (e != cudaSuccess) return (int)e;
   }
-  dp_reduce_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(gp, n_peers, scale, g_out, p, chunks, seg_hp, norms);
+  dp_reduce_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(gp, n_peers, scale, g_out, p, chunks, *(const Hyper*)hyper, norms);
   return TSP_LAUNCH_CHECK();
 }
 
 int tsp_dp_lars_apply(void* const* params, int n_peers, int self, const float* g, float* mu, const int64_t* chunks,
-                      int n_chunks, const float* seg_hp, const float* norms, cudaStream_t stream) {
+                      int n_chunks, const void* hyper, const float* norms, cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
   PeerPtrs pp;
   if (!fill(pp, params, n_peers) || self < 0 || self >= n_peers) return -3;
-  dp_lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(pp, n_peers, self, g, mu, chunks, seg_hp, norms);
+  dp_lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(pp, n_peers, self, g, mu, chunks, *(const Hyper*)hyper, norms);
   return TSP_LAUNCH_CHECK();
 }
 
 int tsp_dp_adamw_step(void* const* grads, void* const* params, int n_peers, int self, float scale, float* m, float* v,
-                      const int64_t* chunks, int n_chunks, const float* seg_hp, cudaStream_t stream) {
+                      const int64_t* chunks, int n_chunks, const void* hyper, cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
   PeerPtrs gp, pp;
   if (!fill(gp, grads, n_peers) || !fill(pp, params, n_peers) || self < 0 || self >= n_peers) return -3;
-  dp_adamw_kernel<<<n_chunks, kThreads, 0, stream>>>(gp, pp, n_peers, self, scale, m, v, chunks, seg_hp);
+  dp_adamw_kernel<<<n_chunks, kThreads, 0, stream>>>(gp, pp, n_peers, self, scale, m, v, chunks, *(const Hyper*)hyper);
   return TSP_LAUNCH_CHECK();
 }
 

@@ -12,18 +12,18 @@ extern "C" {
 // ---- flat_optim.cu ---------------------------------------------------------------------------------------------
 int tsp_ema_update(float* teacher, const float* student, int64_t n, float momentum, void* bf16_shadow,
                    cudaStream_t stream);
-int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const void* hyper,
                   float grad_scale, float* norms, int n_seg, float* teacher, int64_t teacher_n, float ema_m,
                   cudaStream_t stream);
-int tsp_lars_norms(const float* p, const float* g, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_lars_norms(const float* p, const float* g, const int64_t* chunks, int n_chunks, const void* hyper,
                    float grad_scale, float* norms, int n_seg, cudaStream_t stream);
-int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const void* hyper,
                    float grad_scale, const float* norms, float* teacher, int64_t teacher_n, float ema_m,
                    cudaStream_t stream);
 int tsp_adamw_step(float* p, const float* g, float* m, float* v, const int64_t* chunks, int n_chunks,
-                   const float* seg_hp, float grad_scale, float* teacher, int64_t teacher_n, float ema_m,
+                   const void* hyper, float grad_scale, float* teacher, int64_t teacher_n, float ema_m,
                    cudaStream_t stream);
-int tsp_sgd_step(float* p, const float* g, float* buf, const int64_t* chunks, int n_chunks, const float* seg_hp,
+int tsp_sgd_step(float* p, const float* g, float* buf, const int64_t* chunks, int n_chunks, const void* hyper,
                  float grad_scale, float* teacher, int64_t teacher_n, float ema_m, cudaStream_t stream);
 
 // ---- losses.cu ---------------------------------------------------------------------------------------------------
@@ -80,12 +80,12 @@ int tsp_ipc_import(const unsigned char* handle64, void** base);
 int tsp_ipc_close(void* base);
 int tsp_gather_blocks(void* const* srcs, int n_peers, int64_t bytes_each, void* dst, cudaStream_t stream);
 int tsp_dp_reduce_norms(void* const* grads, int n_peers, float scale, float* g_out, const float* p,
-                        const int64_t* chunks, int n_chunks, const float* seg_hp, float* norms, int n_seg,
+                        const int64_t* chunks, int n_chunks, const void* hyper, float* norms, int n_seg,
                         cudaStream_t stream);
 int tsp_dp_lars_apply(void* const* params, int n_peers, int self, const float* g, float* mu, const int64_t* chunks,
-                      int n_chunks, const float* seg_hp, const float* norms, cudaStream_t stream);
+                      int n_chunks, const void* hyper, const float* norms, cudaStream_t stream);
 int tsp_dp_adamw_step(void* const* grads, void* const* params, int n_peers, int self, float scale, float* m, float* v,
-                      const int64_t* chunks, int n_chunks, const float* seg_hp, cudaStream_t stream);
+                      const int64_t* chunks, int n_chunks, const void* hyper, cudaStream_t stream);
 
 // ---- pool.cu ------------------------------------------------------------------------------------------------------
 int tsp_maxpool3x3s2_fwd(const void* x, void* y, uint8_t* idx, int n, int h, int w, int c, int dtype,

@@ -1,0 +1,108 @@
+"""Flat optimizer steps with hyperparameters that change from step to step, by value and as a table."""
+import pytest
+import torch
+from torch import nn
+
+from tspipe_b200.optim import LARS, SGD, AdamW
+from tspipe_b200.runtime.state import FlatParams
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda", 0)
+MAKE = {"lars": lambda gs: LARS(gs, lr=0.1, weight_decay=1e-3), "adamw": lambda gs: AdamW(gs, lr=1e-2, weight_decay=0.1),
+        "sgd": lambda gs: SGD(gs, lr=0.05, momentum=0.9, weight_decay=1e-3)}
+
+
+def _params(n):
+    torch.manual_seed(0)
+    return [nn.Parameter(torch.randn(*((33, 17 + i % 5) if i % 3 else (41,)), device=DEV)) for i in range(n)]
+
+
+def _groups(ps, k):
+    return [dict(params=ps[i::k], lr=0.01 * (1 + i % 5), weight_decay=1e-3 * (i % 3)) for i in range(k)]
+
+
+def _same(ps, ref, steps):
+    """A step rounds values no larger than the largest parameter (or update) some four times, on either side."""
+    for p, q in zip(ps, ref):
+        atol = 2 * 4 * steps * 2 ** -24 * max(1.0, float(q.detach().abs().max()))
+        torch.testing.assert_close(p.detach(), q.detach(), rtol=0, atol=atol)
+
+
+@pytest.mark.parametrize("name", sorted(MAKE))
+@pytest.mark.parametrize("groups", [1, 3, 32, 33, 40])
+def test_groups_with_a_schedule_match_the_step_per_tensor(name, groups):
+    """One group to more than travel by value, every group with its own and a new learning rate in every step."""
+    ps, ref = _params(80), _params(80)
+    opt, ropt = MAKE[name](_groups(ps, groups)), MAKE[name](_groups(ref, groups))
+    flat = FlatParams(ps, DEV, with_grad=True)
+    opt.bind_flat(flat, use_kernel=True)
+    for step in range(3):
+        torch.manual_seed(step)
+        for p, q in zip(ps, ref):
+            q.grad = torch.randn_like(q)
+            p.grad.copy_(q.grad)
+        for o in (opt, ropt):
+            for i, g in enumerate(o.param_groups):
+                g["lr"] *= 0.9 + 0.002 * i
+            o.step()
+    _same(ps, ref, 3)
+
+
+def test_a_recorded_step_repeats_its_values_and_refuses_new_ones():
+    ps, qs = _params(5), _params(5)
+    lars, adam = MAKE["lars"](ps), MAKE["adamw"](qs)
+    for o, x in ((lars, ps), (adam, qs)):
+        o.bind_flat(FlatParams(x, DEV, with_grad=True), use_kernel=True)
+        o.step()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        lars.step()                                   # nothing has changed since the last step
+    with pytest.raises(RuntimeError, match="cannot be recorded"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            adam.step()                               # the bias corrections have
+    for p in ps:
+        p.grad.fill_(0.5)
+    before = [p.detach().clone() for p in ps]
+    g.replay()
+    assert all(not torch.equal(p, b) for p, b in zip(ps, before))
+
+
+@pytest.mark.parametrize("name", ["lars", "adamw"])
+@pytest.mark.parametrize("groups", [2, 40])
+def test_data_parallel_kernels_on_the_same_values(name, groups):
+    """The replicas' kernels, which do not wait for one another, with two replicas' buffers on one GPU: each updates its half
+    of the range in both, from the mean of both gradients."""
+    from tspipe_b200.comm.peer import pointer_table
+    from tspipe_b200.ops import fused
+    ps, ref = _params(80), _params(80)
+    opt, ropt = MAKE[name](_groups(ps, groups)), MAKE[name](_groups(ref, groups))
+    flat = FlatParams(ps, DEV, with_grad=True, pad_to=2)
+    opt.bind_flat(flat, use_kernel=True)
+    torch.manual_seed(1)
+    for p, q in zip(ps, ref):
+        p.grad.normal_()
+        q.grad = p.grad.clone()
+    data2, grad2 = flat.data.clone(), flat.grad.clone()
+    flat.grad.mul_(0.5)
+    grad2.mul_(1.5)                                   # the mean is the reference's gradient
+    grads, params = pointer_table([flat.grad, grad2]), pointer_table([flat.data, data2])
+    ropt.step()
+    half = flat.total // 2
+    chunks = [fused.build_chunks(flat.offsets, flat.numels, DEV, r * half, (r + 1) * half) for r in (0, 1)]
+    if name == "lars":
+        hp = opt._hyper_of([[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"]] for g in opt._groups])
+        g_out, mu, norms = torch.zeros_like(flat.grad), torch.zeros_like(flat.grad), []
+        for r in (0, 1):
+            norms.append(torch.zeros_like(opt._norms))
+            fused.dp_reduce_norms_(grads, 2, 0.5, g_out, flat.data, chunks[r], hp, norms[r])
+        for r in (0, 1):
+            fused.dp_lars_apply_(params, 2, r, g_out, mu, chunks[r], hp, norms[0] + norms[1])
+    else:
+        hp = opt._hyper_of([[g["lr"], *g["betas"], g["eps"], g["weight_decay"], 1 - g["betas"][0], 1 - g["betas"][1]]
+                            for g in opt._groups])
+        m, v = torch.zeros_like(flat.grad), torch.zeros_like(flat.grad)
+        for r in (0, 1):
+            fused.dp_adamw_step_(grads, params, 2, r, 0.5, m, v, chunks[r], hp)
+    assert torch.equal(flat.data, data2)
+    _same(ps, ref, 1)

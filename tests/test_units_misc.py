@@ -167,3 +167,29 @@ def test_hooks_on_all_modules_see_the_norms_of_a_block_and_the_pooling_of_a_stem
         handle.remove()
     assert [m for m in seen if isinstance(m, LayerNorm)] == [blk.norm1, blk.norm2]
     assert not has_hooks(MaxPool3x3s2())
+
+
+def test_hyperparameters_of_a_launch():
+    """A code per segment (group and whether the trust ratio applies), the groups' values by value; only a change rewrites
+    them; more groups than travel by value go through a table."""
+    import torch
+    from torch import nn
+    from tspipe_b200.ops import fused
+    from tspipe_b200.optim import LARS
+    from tspipe_b200.runtime.state import FlatParams
+    for n in (2, 33):
+        ps = [nn.Parameter(torch.randn(4, 3) if i % 2 else torch.randn(5)) for i in range(2 * n)]
+        opt = LARS([dict(params=ps[i::n], lr=0.5 + i) for i in range(n)], weight_decay=0.25)
+        flat = FlatParams(ps, torch.device("cpu"), with_grad=True)
+        opt.bind_flat(flat, use_kernel=True)
+        assert opt._codes.tolist() == [(i % n) << 1 | i % 2 for i in range(2 * n)]
+        rows = [[g["lr"], g["weight_decay"]] for g in opt._groups]
+        if n <= fused.Hyper.GROUPS:
+            h = opt._hyper_of(rows)
+            assert not h.table and h.by_value[8:10] == [1.5, 0.25]
+            h.by_value[8] = 7.0
+            assert opt._hyper_of([list(r) for r in rows]).by_value[8] == 7.0         # unchanged: not written again
+            assert opt._hyper_of([[2.5, 0.0], [3.5, 1.0]]).by_value[8] == 3.5
+        else:
+            assert opt._hyper_of(rows).table == opt._hyper_table.data_ptr()
+            assert opt._hyper_table[32, :2].tolist() == [32.5, 0.25]

@@ -243,30 +243,36 @@ def build_chunks(offsets: Sequence[int], numels: Sequence[int], device, lo: int 
     return torch.tensor(rows, dtype=torch.int64, device=device)
 
 
+class Hyper(ctypes.Structure):
+    """Hyperparameters of a launch (``tsp::Hyper``): a code per segment, ``group << 1 | adapt``, in device memory, and the
+    groups' values, by value or as a table in device memory."""
+    VALS, GROUPS = 8, 32
+    _fields_ = [("seg_code", ctypes.c_void_p), ("table", ctypes.c_void_p), ("by_value", ctypes.c_float * (8 * 32))]
+
+
 @torch.no_grad()
-def lars_step_(p, g, mu, chunks, seg_hp, norms, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
-    n_seg = seg_hp.shape[0]
+def lars_step_(p, g, mu, chunks, hyper, norms, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_lars_step(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _ptr(seg_hp),
-                                   _c.c_float(grad_scale), _ptr(norms), _c.c_int(n_seg), _ptr(teacher),
+        _check(lib().tsp_lars_step(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
+                                   _c.c_float(grad_scale), _ptr(norms), _c.c_int(norms.numel() // 2), _ptr(teacher),
                                    _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m),
                                    _stream()), "tsp_lars_step")
     _count(3)
 
 
 @torch.no_grad()
-def lars_norms_(p, g, chunks, seg_hp, norms, grad_scale=1.0) -> None:
+def lars_norms_(p, g, chunks, hyper, norms, grad_scale=1.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_lars_norms(_ptr(p), _ptr(g), _ptr(chunks), _c.c_int(chunks.shape[0]), _ptr(seg_hp),
-                                    _c.c_float(grad_scale), _ptr(norms), _c.c_int(seg_hp.shape[0]), _stream()),
+        _check(lib().tsp_lars_norms(_ptr(p), _ptr(g), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
+                                    _c.c_float(grad_scale), _ptr(norms), _c.c_int(norms.numel() // 2), _stream()),
                "tsp_lars_norms")
     _count(2)
 
 
 @torch.no_grad()
-def lars_apply_(p, g, mu, chunks, seg_hp, norms, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
+def lars_apply_(p, g, mu, chunks, hyper, norms, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_lars_apply(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _ptr(seg_hp),
+        _check(lib().tsp_lars_apply(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
                                     _c.c_float(grad_scale), _ptr(norms), _ptr(teacher),
                                     _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m),
                                     _stream()), "tsp_lars_apply")
@@ -274,19 +280,19 @@ def lars_apply_(p, g, mu, chunks, seg_hp, norms, grad_scale=1.0, teacher=None, e
 
 
 @torch.no_grad()
-def adamw_step_(p, g, m, v, chunks, seg_hp, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
+def adamw_step_(p, g, m, v, chunks, hyper, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
         _check(lib().tsp_adamw_step(_ptr(p), _ptr(g), _ptr(m), _ptr(v), _ptr(chunks), _c.c_int(chunks.shape[0]),
-                                    _ptr(seg_hp), _c.c_float(grad_scale), _ptr(teacher),
+                                    _c.byref(hyper), _c.c_float(grad_scale), _ptr(teacher),
                                     _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m),
                                     _stream()), "tsp_adamw_step")
     _count()
 
 
 @torch.no_grad()
-def sgd_step_(p, g, buf, chunks, seg_hp, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
+def sgd_step_(p, g, buf, chunks, hyper, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_sgd_step(_ptr(p), _ptr(g), _ptr(buf), _ptr(chunks), _c.c_int(chunks.shape[0]), _ptr(seg_hp),
+        _check(lib().tsp_sgd_step(_ptr(p), _ptr(g), _ptr(buf), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
                                   _c.c_float(grad_scale), _ptr(teacher),
                                   _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m), _stream()),
                "tsp_sgd_step")
@@ -626,13 +632,13 @@ def gelu(x: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
 # data-parallel reduce-scatter + sharded step + all-gather over peer-mapped buffers (csrc/peer.cu)
 # ---------------------------------------------------------------------------------------------
 @torch.no_grad()
-def dp_reduce_norms_(grad_ptrs, n_peers, scale, g_out, p, chunks, seg_hp, norms) -> None:
+def dp_reduce_norms_(grad_ptrs, n_peers, scale, g_out, p, chunks, hyper, norms) -> None:
     L = lib()
     L.tsp_dp_reduce_norms.restype = _c.c_int
     with on_device(p.device):
         _check(L.tsp_dp_reduce_norms(grad_ptrs, _c.c_int(n_peers), _c.c_float(scale), _ptr(g_out), _ptr(p),
-                                     _ptr(chunks), _c.c_int(chunks.shape[0]), _ptr(seg_hp), _ptr(norms),
-                                     _c.c_int(seg_hp.shape[0]), _stream()), "tsp_dp_reduce_norms")
+                                     _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper), _ptr(norms),
+                                     _c.c_int(norms.numel() // 2), _stream()), "tsp_dp_reduce_norms")
     _count(2)
 
 
@@ -659,22 +665,22 @@ def sum_norms_(table, n_peers, norms) -> None:
 
 
 @torch.no_grad()
-def dp_lars_apply_(param_ptrs, n_peers, self_idx, g, mu, chunks, seg_hp, norms) -> None:
+def dp_lars_apply_(param_ptrs, n_peers, self_idx, g, mu, chunks, hyper, norms) -> None:
     L = lib()
     L.tsp_dp_lars_apply.restype = _c.c_int
     with on_device(g.device):
         _check(L.tsp_dp_lars_apply(param_ptrs, _c.c_int(n_peers), _c.c_int(self_idx), _ptr(g), _ptr(mu), _ptr(chunks),
-                                   _c.c_int(chunks.shape[0]), _ptr(seg_hp), _ptr(norms), _stream()),
+                                   _c.c_int(chunks.shape[0]), _c.byref(hyper), _ptr(norms), _stream()),
                "tsp_dp_lars_apply")
     _count()
 
 
 @torch.no_grad()
-def dp_adamw_step_(grad_ptrs, param_ptrs, n_peers, self_idx, scale, m, v, chunks, seg_hp) -> None:
+def dp_adamw_step_(grad_ptrs, param_ptrs, n_peers, self_idx, scale, m, v, chunks, hyper) -> None:
     L = lib()
     L.tsp_dp_adamw_step.restype = _c.c_int
     with on_device(m.device):
         _check(L.tsp_dp_adamw_step(grad_ptrs, param_ptrs, _c.c_int(n_peers), _c.c_int(self_idx), _c.c_float(scale),
-                                   _ptr(m), _ptr(v), _ptr(chunks), _c.c_int(chunks.shape[0]), _ptr(seg_hp),
+                                   _ptr(m), _ptr(v), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
                                    _stream()), "tsp_dp_adamw_step")
     _count()

@@ -6,7 +6,7 @@ parameters with ``ndim <= 1``), ``AdamW`` and ``SGD`` follow ``torch.optim`` (wh
 They are ordinary ``torch.optim.Optimizer`` subclasses - usable on their own, per tensor - and
 gain the fused path when the engine calls :meth:`bind_flat` with the partition's
 :class:`~tspipe_b200.runtime.state.FlatParams`: state lives in flat buffers too, per-tensor
-hyper-parameters go into a small table, and on CUDA the sm_100a kernels of
+hyper-parameters travel with the launch, and on CUDA the sm_100a kernels of
 ``csrc/flat_optim.cu`` do the work.  With ``fuse_ema`` the momentum-teacher update of the
 corresponding local teacher buffer rides in the same launch.
 """
@@ -43,7 +43,12 @@ class _FlatMixin:
             from ..ops import fused
             self._chunks = fused.build_chunks(flat.offsets, flat.numels, flat.device)
             self._norms = torch.zeros(2 * max(len(flat.params), 1), dtype=torch.float32, device=flat.device)
-        self._hp_cache = None
+            self._groups = list({id(g): g for g in self._seg_group}.values())
+            index = {id(g): i for i, g in enumerate(self._groups)}
+            self._codes = torch.tensor([index[id(g)] << 1 | (p.ndim > 1) for p, g in zip(flat.params, self._seg_group)],
+                                       dtype=torch.int32, device=flat.device)
+            self._hyper = fused.Hyper(seg_code=self._codes.data_ptr())
+            self._hyper_rows, self._hyper_table = None, None
 
     def enable_dp(self, group, peer_grads, peer_params, self_index: int) -> None:
         """Data-parallel mode over peer-mapped buffers: this rank owns ``1/R`` of the flat range; the step
@@ -101,18 +106,27 @@ class _FlatMixin:
     def _views(self, flat_tensor: torch.Tensor, i: int) -> torch.Tensor:
         return self.flat._view(flat_tensor, i, self.flat.params[i].data)
 
-    def _hp_table(self, rows: List[List[float]]) -> torch.Tensor:
-        key = tuple(tuple(r) for r in rows)
-        if self._hp_cache is None or self._hp_cache[0] != key:
-            dev = self.flat.device
-            if dev.type == "cuda" and not torch.cuda.is_current_stream_capturing():
-                # a copy from pinned memory (kept by the host allocator until the copy is done) is ordered on the stream;
-                # one from pageable memory would first wait on the host for everything enqueued before it
-                table = torch.tensor(rows, dtype=torch.float32).pin_memory().to(dev, non_blocking=True)
+    def _hyper_of(self, rows: List[List[float]]):
+        """The launch argument for these values of the parameter groups (``self._groups``, in order).  They go by value: no
+        table to copy before a step, on whatever stream.  More groups than that has room for go through a table, copied
+        from pageable memory when they change, i.e. complete for every stream when the copy returns."""
+        from ..ops import fused
+        if rows != self._hyper_rows:
+            if self.flat.data.is_cuda and torch.cuda.is_current_stream_capturing():
+                raise RuntimeError("an optimizer step whose hyperparameters have changed cannot be recorded into a CUDA graph: "
+                                   "each replay would repeat the values of the recording")
+            h, n = self._hyper, fused.Hyper.VALS
+            if len(rows) <= fused.Hyper.GROUPS:
+                for i, r in enumerate(rows):
+                    h.by_value[n * i: n * i + len(r)] = r
             else:
-                table = torch.tensor(rows, dtype=torch.float32, device=dev)
-            self._hp_cache = (key, table)
-        return self._hp_cache[1]
+                self._hyper_table = torch.tensor([r + [0.0] * (n - len(r)) for r in rows], dtype=torch.float32,
+                                                 device=self.flat.device)
+                h.table = self._hyper_table.data_ptr()
+            self._hyper_rows = rows
+        if self._hyper_table is not None and self._hyper_table.is_cuda:
+            self._hyper_table.record_stream(torch.cuda.current_stream(self.flat.device))
+        return self._hyper
 
     def flat_state_dict(self) -> Dict[str, Any]:
         return {"flat": {k: v.detach().cpu() for k, v in self._flat_state.items()}, "steps": self._steps}
@@ -178,11 +192,10 @@ class LARS(_FlatMixin, Optimizer):
         mu = self._buf("mu")
         if self.use_kernel:
             from ..ops import fused
-            rows = [[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"], 1.0 if p.ndim > 1 else 0.0]
-                    for p, g in zip(flat.params, self._seg_group)]
+            rows = [[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"]] for g in self._groups]
             if self.handles_dp:
                 d = self._dp
-                hp = self._hp_table(rows)
+                hp = self._hyper_of(rows)
                 if not d["reduced"]:
                     self.dp_reduce(grad_scale)
                 d["reduced"] = False
@@ -192,7 +205,7 @@ class LARS(_FlatMixin, Optimizer):
                 fused.dp_lars_apply_(d["params"], d["r"], d["idx"], flat.grad, mu, d["chunks"], hp, self._norms)
                 self._dp_barrier()                      # every replica's parameters are complete
                 return
-            fused.lars_step_(flat.data, flat.grad, mu, self._chunks, self._hp_table(rows), self._norms, grad_scale,
+            fused.lars_step_(flat.data, flat.grad, mu, self._chunks, self._hyper_of(rows), self._norms, grad_scale,
                              self.teacher_flat, self.ema_momentum)
             return
         for i, (p, g) in enumerate(zip(flat.params, self._seg_group)):
@@ -206,9 +219,7 @@ class LARS(_FlatMixin, Optimizer):
         import torch.distributed as dist
         from ..ops import fused
         flat, d = self.flat, self._dp
-        rows = [[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"], 1.0 if p.ndim > 1 else 0.0]
-                for p, g in zip(flat.params, self._seg_group)]
-        hp = self._hp_table(rows)
+        hp = self._hyper_of([[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"]] for g in self._groups])
         self._dp_barrier()                              # every replica's backward is complete
         fused.dp_reduce_norms_(d["grads"], d["r"], grad_scale / d["r"], flat.grad, flat.data, d["chunks"], hp,
                                self._norms)
@@ -258,7 +269,7 @@ class AdamW(_FlatMixin, Optimizer):
         if self.use_kernel:
             from ..ops import fused
             rows = [[g["lr"], g["betas"][0], g["betas"][1], g["eps"], g["weight_decay"],
-                     1.0 - g["betas"][0] ** t, 1.0 - g["betas"][1] ** t] for g in self._seg_group]
+                     1.0 - g["betas"][0] ** t, 1.0 - g["betas"][1] ** t] for g in self._groups]
             if self.handles_dp:
                 d = self._dp
                 if not d["reduced"]:
@@ -267,10 +278,10 @@ class AdamW(_FlatMixin, Optimizer):
                 if d["signals"] is not None:
                     d["signals"].wait(d["phase"])       # every replica's backward is complete
                 fused.dp_adamw_step_(d["grads"], d["params"], d["r"], d["idx"], grad_scale / d["r"], m, v, d["chunks"],
-                                     self._hp_table(rows))
+                                     self._hyper_of(rows))
                 self._dp_barrier()
                 return
-            fused.adamw_step_(flat.data, flat.grad, m, v, self._chunks, self._hp_table(rows), grad_scale,
+            fused.adamw_step_(flat.data, flat.grad, m, v, self._chunks, self._hyper_of(rows), grad_scale,
                               self.teacher_flat, self.ema_momentum)
             return
         for i, (p, g) in enumerate(zip(flat.params, self._seg_group)):
@@ -329,8 +340,8 @@ class SGD(_FlatMixin, Optimizer):
         if self.use_kernel:
             from ..ops import fused
             rows = [[g["lr"], g["momentum"], g["dampening"], g["weight_decay"], 1.0 if g["nesterov"] else 0.0,
-                     1.0 if first else 0.0] for g in self._seg_group]
-            fused.sgd_step_(flat.data, flat.grad, buf, self._chunks, self._hp_table(rows), grad_scale,
+                     1.0 if first else 0.0] for g in self._groups]
+            fused.sgd_step_(flat.data, flat.grad, buf, self._chunks, self._hyper_of(rows), grad_scale,
                             self.teacher_flat, self.ema_momentum)
             return
         for i, (p, g) in enumerate(zip(flat.params, self._seg_group)):
