@@ -69,10 +69,10 @@ def test_a_recorded_step_repeats_its_values_and_refuses_new_ones():
 
 
 @pytest.mark.parametrize("name", ["lars", "adamw"])
-@pytest.mark.parametrize("groups", [2, 40])
-def test_data_parallel_kernels_on_the_same_values(name, groups):
+@pytest.mark.parametrize("groups,rows", [(2, False), (40, False), (2, True)])
+def test_data_parallel_kernels_on_the_same_values(name, groups, rows):
     """The replicas' kernels, which do not wait for one another, with two replicas' buffers on one GPU: each updates its half
-    of the range in both, from the mean of both gradients."""
+    of the range in both, from the mean of both gradients; with the optimizer's values or a row of them per segment."""
     from tspipe_b200.comm.peer import pointer_table
     from tspipe_b200.ops import fused
     ps, ref = _params(80), _params(80)
@@ -91,7 +91,9 @@ def test_data_parallel_kernels_on_the_same_values(name, groups):
     half = flat.total // 2
     chunks = [fused.build_chunks(flat.offsets, flat.numels, DEV, r * half, (r + 1) * half) for r in (0, 1)]
     if name == "lars":
-        hp = opt._hyper_of([[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"]] for g in opt._groups])
+        vals = [[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"]] for g in opt._groups]
+        hp = torch.tensor([vals[i % groups] + [float(p.ndim > 1)] for i, p in enumerate(ps)], device=DEV) if rows \
+            else opt._hyper_of(vals)
         g_out, mu, norms = torch.zeros_like(flat.grad), torch.zeros_like(flat.grad), []
         for r in (0, 1):
             norms.append(torch.zeros_like(opt._norms))
@@ -99,8 +101,8 @@ def test_data_parallel_kernels_on_the_same_values(name, groups):
         for r in (0, 1):
             fused.dp_lars_apply_(params, 2, r, g_out, mu, chunks[r], hp, norms[0] + norms[1])
     else:
-        hp = opt._hyper_of([[g["lr"], *g["betas"], g["eps"], g["weight_decay"], 1 - g["betas"][0], 1 - g["betas"][1]]
-                            for g in opt._groups])
+        vals = [[g["lr"], *g["betas"], g["eps"], g["weight_decay"], 1 - g["betas"][0], 1 - g["betas"][1]] for g in opt._groups]
+        hp = torch.tensor([vals[i % groups] for i in range(len(ps))], device=DEV) if rows else opt._hyper_of(vals)
         m, v = torch.zeros_like(flat.grad), torch.zeros_like(flat.grad)
         for r in (0, 1):
             fused.dp_adamw_step_(grads, params, 2, r, 0.5, m, v, chunks[r], hp)

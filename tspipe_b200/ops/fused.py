@@ -249,11 +249,26 @@ class Hyper(ctypes.Structure):
     VALS, GROUPS = 8, 32
     _fields_ = [("seg_code", ctypes.c_void_p), ("table", ctypes.c_void_p), ("by_value", ctypes.c_float * (8 * 32))]
 
+    @staticmethod
+    def of(hp) -> "Hyper":
+        """``hp`` itself, or what stands for a matrix in device memory with one row of values per segment (a fifth and last
+        value: adapt), to be used on the current stream."""
+        if isinstance(hp, Hyper):
+            return hp
+        n, k = hp.shape
+        codes = torch.arange(n, dtype=torch.int32, device=hp.device) << 1
+        if k == 5:
+            codes |= (hp[:, 4] != 0).to(torch.int32)
+        table = torch.nn.functional.pad(hp.float(), (0, Hyper.VALS - k)).contiguous()
+        h = Hyper(seg_code=codes.data_ptr(), table=table.data_ptr())
+        h.keep = (codes, table)
+        return h
+
 
 @torch.no_grad()
 def lars_step_(p, g, mu, chunks, hyper, norms, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_lars_step(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
+        _check(lib().tsp_lars_step(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(Hyper.of(hyper)),
                                    _c.c_float(grad_scale), _ptr(norms), _c.c_int(norms.numel() // 2), _ptr(teacher),
                                    _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m),
                                    _stream()), "tsp_lars_step")
@@ -263,7 +278,7 @@ def lars_step_(p, g, mu, chunks, hyper, norms, grad_scale=1.0, teacher=None, ema
 @torch.no_grad()
 def lars_norms_(p, g, chunks, hyper, norms, grad_scale=1.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_lars_norms(_ptr(p), _ptr(g), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
+        _check(lib().tsp_lars_norms(_ptr(p), _ptr(g), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(Hyper.of(hyper)),
                                     _c.c_float(grad_scale), _ptr(norms), _c.c_int(norms.numel() // 2), _stream()),
                "tsp_lars_norms")
     _count(2)
@@ -272,7 +287,7 @@ def lars_norms_(p, g, chunks, hyper, norms, grad_scale=1.0) -> None:
 @torch.no_grad()
 def lars_apply_(p, g, mu, chunks, hyper, norms, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_lars_apply(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
+        _check(lib().tsp_lars_apply(_ptr(p), _ptr(g), _ptr(mu), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(Hyper.of(hyper)),
                                     _c.c_float(grad_scale), _ptr(norms), _ptr(teacher),
                                     _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m),
                                     _stream()), "tsp_lars_apply")
@@ -283,7 +298,7 @@ def lars_apply_(p, g, mu, chunks, hyper, norms, grad_scale=1.0, teacher=None, em
 def adamw_step_(p, g, m, v, chunks, hyper, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
         _check(lib().tsp_adamw_step(_ptr(p), _ptr(g), _ptr(m), _ptr(v), _ptr(chunks), _c.c_int(chunks.shape[0]),
-                                    _c.byref(hyper), _c.c_float(grad_scale), _ptr(teacher),
+                                    _c.byref(Hyper.of(hyper)), _c.c_float(grad_scale), _ptr(teacher),
                                     _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m),
                                     _stream()), "tsp_adamw_step")
     _count()
@@ -292,7 +307,7 @@ def adamw_step_(p, g, m, v, chunks, hyper, grad_scale=1.0, teacher=None, ema_m=0
 @torch.no_grad()
 def sgd_step_(p, g, buf, chunks, hyper, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
     with on_device(p.device):
-        _check(lib().tsp_sgd_step(_ptr(p), _ptr(g), _ptr(buf), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
+        _check(lib().tsp_sgd_step(_ptr(p), _ptr(g), _ptr(buf), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(Hyper.of(hyper)),
                                   _c.c_float(grad_scale), _ptr(teacher),
                                   _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m), _stream()),
                "tsp_sgd_step")
@@ -637,7 +652,7 @@ def dp_reduce_norms_(grad_ptrs, n_peers, scale, g_out, p, chunks, hyper, norms) 
     L.tsp_dp_reduce_norms.restype = _c.c_int
     with on_device(p.device):
         _check(L.tsp_dp_reduce_norms(grad_ptrs, _c.c_int(n_peers), _c.c_float(scale), _ptr(g_out), _ptr(p),
-                                     _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper), _ptr(norms),
+                                     _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(Hyper.of(hyper)), _ptr(norms),
                                      _c.c_int(norms.numel() // 2), _stream()), "tsp_dp_reduce_norms")
     _count(2)
 
@@ -670,7 +685,7 @@ def dp_lars_apply_(param_ptrs, n_peers, self_idx, g, mu, chunks, hyper, norms) -
     L.tsp_dp_lars_apply.restype = _c.c_int
     with on_device(g.device):
         _check(L.tsp_dp_lars_apply(param_ptrs, _c.c_int(n_peers), _c.c_int(self_idx), _ptr(g), _ptr(mu), _ptr(chunks),
-                                   _c.c_int(chunks.shape[0]), _c.byref(hyper), _ptr(norms), _stream()),
+                                   _c.c_int(chunks.shape[0]), _c.byref(Hyper.of(hyper)), _ptr(norms), _stream()),
                "tsp_dp_lars_apply")
     _count()
 
@@ -681,6 +696,6 @@ def dp_adamw_step_(grad_ptrs, param_ptrs, n_peers, self_idx, scale, m, v, chunks
     L.tsp_dp_adamw_step.restype = _c.c_int
     with on_device(m.device):
         _check(L.tsp_dp_adamw_step(grad_ptrs, param_ptrs, _c.c_int(n_peers), _c.c_int(self_idx), _c.c_float(scale),
-                                   _ptr(m), _ptr(v), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(hyper),
+                                   _ptr(m), _ptr(v), _ptr(chunks), _c.c_int(chunks.shape[0]), _c.byref(Hyper.of(hyper)),
                                    _stream()), "tsp_dp_adamw_step")
     _count()
