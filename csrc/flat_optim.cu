@@ -14,6 +14,8 @@ namespace {
 using tsp::Hyper;
 
 constexpr int kThreads = 256;
+// From this many chunks of up to 64 KB on, over all buffers of a step (80 MB), lars_apply_kernel<true> is used.
+constexpr int64_t kLarsBig = 1280;
 
 // ---------------------------------------------------------------------------------------------
 // EMA: t = m*t + (1-m)*s ; `s` may point into a peer GPU's memory (plain loads over NVLink).
@@ -112,11 +114,26 @@ __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __res
   }
 }
 
+template <bool BIG>
+__device__ __forceinline__ float4 ld_once(const float4* at) {
+  if constexpr (BIG) return __ldcs(at);
+  else return *at;
+}
+template <bool BIG>
+__device__ __forceinline__ void st_once(float4* at, float4 v) {
+  if constexpr (BIG) __stcs(at, v);
+  else *at = v;
+}
+
 // LARS apply (+ optional fused momentum-teacher update for segments that have a local teacher copy):
 //   dp = adapt ? q*(gs*g + wd*p) : gs*g ; mu = mom*mu + dp ; p -= lr*mu ; [t = m*t + (1-m)*p]
-// `last_first`: the chunks are walked from the last one back, right behind lars_norms_kernel, which has left the end of
-// p and g in L2 (up to 126 MB of them); the buffers that only this kernel touches pass L2 with evict-first hints.  Both passes
-// over 25.6 M parameters: 163.6 us walked in the same order, 161.3 this way.
+// BIG: buffers that do not fit L2 together (kLarsBig).  The chunks are then walked from the last one back, right behind
+// lars_norms_kernel, which has left the end of p and g in L2 (up to 126 MB of them); what only this kernel touches passes
+// L2 with evict-first hints.  Both passes over 25.6 M parameters with the teacher (409 MB): 164 us walked in the same order
+// without hints, 156 this way; 6 M (96 MB): 44 and 35.  Smaller buffers stay in L2 from step to step, where the hints
+// would push them out: 4 M without the teacher (48 MB), step and wait: 43.6 us with hints, 40.8 without.  (The order is an
+// argument of the launch: as a constant of the instantiation it costs 4 us at 25.6 M, by the schedule it gets.)
+template <bool BIG>
 __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict__ p, const float* __restrict__ g,
                                                               float* __restrict__ mu,
                                                               const int64_t* __restrict__ chunks,
@@ -145,10 +162,10 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
   float4* t4 = has_t ? reinterpret_cast<float4*>(teacher + c.begin) : nullptr;
 #pragma unroll 2
   for (int i = threadIdx.x; i < n4; i += kThreads) {
-    float4 pv = p4[i], mv = __ldcs(m4 + i);
-    const float4 gv = __ldcs(g4 + i);
+    float4 pv = p4[i], mv = ld_once<BIG>(m4 + i);
+    const float4 gv = ld_once<BIG>(g4 + i);
     const bool t_ok = has_t && (c.begin + 4 * (int64_t)i + 3 < teacher_n);
-    float4 tv = t_ok ? __ldcs(t4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 tv = t_ok ? ld_once<BIG>(t4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #define TSP_LARS1(X)                                                   \
     {                                                                  \
       const float dp = q * (grad_scale * gv.X + wd_eff * pv.X);        \
@@ -159,8 +176,8 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
     TSP_LARS1(x) TSP_LARS1(y) TSP_LARS1(z) TSP_LARS1(w)
 #undef TSP_LARS1
     p4[i] = pv;
-    __stcs(m4 + i, mv);
-    if (t_ok) __stcs(t4 + i, tv);
+    st_once<BIG>(m4 + i, mv);
+    if (t_ok) st_once<BIG>(t4 + i, tv);
   }
   for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += kThreads) {
     const int64_t k = c.begin + i;
@@ -307,8 +324,12 @@ int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, in
   cudaError_t e = cudaMemsetAsync(norms, 0, sizeof(float) * 2 * (size_t)n_seg, stream);
   if (e != cudaSuccess) return (int)e;
   lars_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, chunks, *(const Hyper*)hyper, grad_scale, norms);
-  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms, teacher,
-                                                       teacher_n, ema_m, 1);
+  if ((int64_t)n_chunks * (teacher != nullptr ? 4 : 3) >= kLarsBig)
+    lars_apply_kernel<true><<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms,
+                                                               teacher, teacher_n, ema_m, 1);
+  else
+    lars_apply_kernel<false><<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms,
+                                                                teacher, teacher_n, ema_m, 0);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -325,8 +346,8 @@ int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, i
                    float grad_scale, const float* norms, float* teacher, int64_t teacher_n, float ema_m,
                    cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
-  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms, teacher,
-                                                       teacher_n, ema_m, 0);
+  lars_apply_kernel<false><<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms,
+                                                              teacher, teacher_n, ema_m, 0);
   return TSP_LAUNCH_CHECK();
 }
 
