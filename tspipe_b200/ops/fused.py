@@ -31,6 +31,11 @@ def lib():
                      "tsp_sgd_step", "tsp_byol_loss", "tsp_cosine_loss", "tsp_kd_ce_loss", "tsp_layernorm_fwd",
                      "tsp_layernorm_bwd", "tsp_layernorm_bwd_blocks", "tsp_gelu_fwd", "tsp_gelu_bwd"):
             getattr(L, name).restype = _c.c_int
+        # declared argument types: plain numbers at a call, an object per argument less where a whole loss takes 100 us of host
+        v, i, f = _c.c_void_p, _c.c_int, _c.c_float
+        L.tsp_kd_ce_loss.argtypes = [v] * 4 + [i] * 4 + [f] * 3 + [v] * 4
+        L.tsp_cosine_loss.argtypes = [v] * 3 + [i] * 3 + [f] + [v] * 4
+        L.tsp_scale.argtypes = [v] * 3 + [_c.c_int64, i, v]
         _lib = L
     return _lib
 
@@ -51,9 +56,13 @@ def _ptr(t: Optional[torch.Tensor]):
     return _c.c_void_p(0 if t is None else t.data_ptr())
 
 
-def _stream():
+def _raw_stream() -> int:
     """Raw handle of the current stream of the current device (the launchers' last argument)."""
-    return _c.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _stream():
+    return _c.c_void_p(_raw_stream())
 
 
 IN_CAPTURE = 0          # > 0 while a stage is being recorded into a CUDA graph
@@ -317,10 +326,18 @@ def sgd_step_(p, g, buf, chunks, hyper, grad_scale=1.0, teacher=None, ema_m=0.0)
 # ---------------------------------------------------------------------------------------------
 # losses: forward computes value AND gradient; backward only scales
 # ---------------------------------------------------------------------------------------------
-def _plain(t: torch.Tensor) -> bool:
-    """A tensor whose memory a kernel can read: not a batched or otherwise wrapped stand-in (vmap, tracing)."""
-    return type(t) is torch.Tensor and not (torch._C._functorch.is_legacy_batchedtensor(t)
-                                            or torch._C._functorch.is_functorch_wrapped_tensor(t))
+def _wrapped(t: torch.Tensor) -> bool:
+    """A batched or otherwise wrapped stand-in (vmap, tracing), whose memory a kernel cannot read."""
+    return torch._C._functorch.is_legacy_batchedtensor(t) or torch._C._functorch.is_functorch_wrapped_tensor(t)
+
+
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as a contiguous matrix of its rows (its last dimension)."""
+    return t if t.dim() == 2 and t.is_contiguous() else t.reshape(-1, t.shape[-1]).contiguous()
+
+
+def _address(t) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def save_gradient(ctx, g: torch.Tensor) -> None:
@@ -335,15 +352,15 @@ def _scaled(g: torch.Tensor, gout: torch.Tensor, own: bool) -> torch.Tensor:
     As plain ops where the product is recorded itself (``create_graph``) or ``gout`` is no plain fp32 scalar.  In place where
     ``g`` is the function's ``own`` and the graph is freed behind this backward, so that nobody else will read it (a CUDA graph
     may be replayed: not there); then ``gout = 1``, a loss that is differentiated as it is, costs no pass over the gradient."""
-    if (torch.is_grad_enabled() or not (_plain(g) and _plain(gout)) or gout.dtype != torch.float32 or gout.dim() != 0
-            or gout.device != g.device or not g.is_contiguous() or g.data_ptr() % 16):
+    if (torch.is_grad_enabled() or type(g) is not torch.Tensor or type(gout) is not torch.Tensor
+            or gout.dtype != torch.float32 or gout.dim() != 0 or gout.get_device() != g.get_device()
+            or not g.is_contiguous() or g.data_ptr() % 16 or _wrapped(gout) or _wrapped(g)):
         return g * gout.to(g.dtype)
     own = (own and not torch._C._autograd._get_current_graph_task_keep_graph()
-           and not torch.cuda.is_current_stream_capturing())
+           and not torch._C._cuda_isCurrentStreamCapturing())
     out = g if own else torch.empty_like(g)
     with on_device(g.device):
-        _check(lib().tsp_scale(_ptr(g), _ptr(gout), _ptr(out), _c.c_int64(g.numel()), _c.c_int(_dt(g)), _stream()),
-               "tsp_scale")
+        _check(lib().tsp_scale(g.data_ptr(), gout.data_ptr(), out.data_ptr(), g.numel(), _dt(g), _raw_stream()), "tsp_scale")
     _count()
     return out
 
@@ -410,22 +427,20 @@ def byol_loss(o1, o2, t1, t2) -> torch.Tensor:
 class _KdCe(torch.autograd.Function):
     @staticmethod
     def forward(ctx, s, t, labels, row_mask, temp, w_ce, w_kd):
-        s2 = s.reshape(-1, s.shape[-1]).contiguous()
-        if t is None or not isinstance(t, torch.Tensor):
-            t2 = t          # None, or a peer-mapped [rows, classes] matrix read in place over NVLink
-        else:
-            t2 = t.detach().reshape(-1, t.shape[-1]).contiguous()
+        s2 = _rows(s)
+        t2 = _rows(t) if isinstance(t, torch.Tensor) else t      # None, or a peer-mapped matrix read in place over NVLink
         n, c = s2.shape
-        loss = torch.empty((), dtype=torch.float32, device=s.device)
-        total = torch.empty((), dtype=torch.float64, device=s.device)
+        loss = torch.empty((), dtype=torch.float32, device=s2.device)
+        total = torch.empty((), dtype=torch.float64, device=s2.device)
         gs = torch.empty_like(s2)
-        lab = None if labels is None else labels.reshape(-1).to(torch.int64).contiguous()
+        lab = labels
+        if lab is not None and not (lab.dim() == 1 and lab.dtype == torch.int64 and lab.is_contiguous()):
+            lab = lab.reshape(-1).to(torch.int64).contiguous()
         msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
-        with on_device(s.device):
-            _check(lib().tsp_kd_ce_loss(_ptr(s2), _ptr(t2), _ptr(lab), _ptr(msk), _c.c_int(n), _c.c_int(c),
-                                        _c.c_int(_dt(s2)), _c.c_int(0 if t2 is None else _dt(t2)), _c.c_float(temp),
-                                        _c.c_float(w_ce), _c.c_float(w_kd), _ptr(total), _ptr(loss), _ptr(gs), _stream()),
-                   "tsp_kd_ce_loss")
+        with on_device(s2.device):
+            _check(lib().tsp_kd_ce_loss(s2.data_ptr(), _address(t2), _address(lab), _address(msk), n, c, _dt(s2),
+                                        0 if t2 is None else _dt(t2), temp, w_ce, w_kd, total.data_ptr(),
+                                        loss.data_ptr(), gs.data_ptr(), _raw_stream()), "tsp_kd_ce_loss")
         _count(2)
         save_gradient(ctx, gs)
         ctx.shape = s.shape
@@ -434,7 +449,8 @@ class _KdCe(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         (gs,) = ctx.saved_tensors
-        return _scaled(gs, gout, ctx.own).view(ctx.shape), None, None, None, None, None, None
+        g = _scaled(gs, gout, ctx.own)
+        return g if g.shape == ctx.shape else g.view(ctx.shape), None, None, None, None, None, None
 
 
 def kd_ce_loss(s, t, labels, temp: float, w_ce: float, w_kd: float, row_mask=None) -> torch.Tensor:
@@ -457,16 +473,16 @@ def cross_entropy(s, labels) -> torch.Tensor:
 class _Cosine(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, y, row_mask, scale):
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        y2 = y.detach().reshape(-1, y.shape[-1]).to(x2.dtype).contiguous()
+        x2 = _rows(x)
+        y2 = _rows(y).to(x2.dtype)
         n, d = x2.shape
-        loss = torch.empty((), dtype=torch.float32, device=x.device)
-        total = torch.empty((), dtype=torch.float64, device=x.device)
+        loss = torch.empty((), dtype=torch.float32, device=x2.device)
+        total = torch.empty((), dtype=torch.float64, device=x2.device)
         gx = torch.empty_like(x2)
         msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
-        with on_device(x.device):
-            _check(lib().tsp_cosine_loss(_ptr(x2), _ptr(y2), _ptr(msk), _c.c_int(n), _c.c_int(d), _c.c_int(_dt(x2)),
-                                         _c.c_float(scale), _ptr(total), _ptr(loss), _ptr(gx), _stream()),
+        with on_device(x2.device):
+            _check(lib().tsp_cosine_loss(x2.data_ptr(), y2.data_ptr(), _address(msk), n, d, _dt(x2), scale,
+                                         total.data_ptr(), loss.data_ptr(), gx.data_ptr(), _raw_stream()),
                    "tsp_cosine_loss")
         _count(2)
         save_gradient(ctx, gx)
@@ -476,7 +492,8 @@ class _Cosine(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         (gx,) = ctx.saved_tensors
-        return _scaled(gx, gout, ctx.own).view(ctx.shape), None, None, None
+        g = _scaled(gx, gout, ctx.own)
+        return g if g.shape == ctx.shape else g.view(ctx.shape), None, None, None
 
 
 def cosine_embedding_loss(x, y, scale: float, row_mask=None) -> torch.Tensor:
