@@ -24,6 +24,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 #include "tspipe_kernels.h"
 
 namespace {
@@ -428,34 +429,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn get_encode() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
-  }
-  return fn;
-}
-
 // [batch][head][rows][cols] view: `ld` elements between rows, `hs` between heads, `bs` between batches.
 bool make_map4(CUtensorMap* map, const void* ptr, int batch, int heads, int rows, int cols, int64_t ld, int64_t hs,
                int64_t bs, int box_cols, int box_rows, bool fp32) {
-  EncodeTiledFn enc = get_encode();
-  if (enc == nullptr) return false;
   const int esz = fp32 ? 4 : 2;
-  cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)heads, (cuuint64_t)batch};
-  cuuint64_t strides[3] = {(cuuint64_t)ld * esz, (cuuint64_t)hs * esz, (cuuint64_t)bs * esz};
-  cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  return enc(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr),
-             dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  const cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)heads, (cuuint64_t)batch};
+  const cuuint64_t strides[3] = {(cuuint64_t)ld * esz, (cuuint64_t)hs * esz, (cuuint64_t)bs * esz};
+  const cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1, 1};
+  return tc5::encode_tiled(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, 4, dims,
+                           strides, box, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
 struct Strides { int64_t ld, hs, bs; };

@@ -565,22 +565,6 @@ conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_b
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
-  }
-  return fn;
-}
-
 }  // namespace
 
 extern "C" {
@@ -597,27 +581,18 @@ int tsp_conv_stem_fwd(const void* x, const void* wmat, void* y, float* sums, int
   if ((h & 1) || (w & 7) || w > 224 || h < 8 || w < 8) return -3;
   if ((((uintptr_t)x | (uintptr_t)wmat | (uintptr_t)y) & 15) != 0) return -2;
   const int oh = h / 2, ow = w / 2;
-  EncodeTiledFn enc = get_encode();
-  if (enc == nullptr) return -6;
   CUtensorMap tw, ty;
   {
-    cuuint64_t dims[2] = {(cuuint64_t)kKPad, (cuuint64_t)kCout};
-    cuuint64_t strides[1] = {(cuuint64_t)kKPad * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)kCout};
-    cuuint32_t estr[2] = {1, 1};
-    if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(wmat), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    const cuuint64_t dims[2] = {(cuuint64_t)kKPad, (cuuint64_t)kCout}, strides[1] = {(cuuint64_t)kKPad * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)kCout};
+    if (!tc5::encode_tiled(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, wmat, 2, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_L2_256B))
       return -6;
   }
   {
-    cuuint64_t dims[3] = {(cuuint64_t)kCout, (cuuint64_t)ow, (cuuint64_t)n * oh};
-    cuuint64_t strides[2] = {(cuuint64_t)kCout * 2, (cuuint64_t)ow * kCout * 2};
-    cuuint32_t box[3] = {(cuuint32_t)kCout, 32, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    if (enc(&ty, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
-        CUDA_SUCCESS)
+    const cuuint64_t dims[3] = {(cuuint64_t)kCout, (cuuint64_t)ow, (cuuint64_t)n * oh};
+    const cuuint64_t strides[2] = {(cuuint64_t)kCout * 2, (cuuint64_t)ow * kCout * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)kCout, 32, 1};
+    if (!tc5::encode_tiled(&ty, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, y, 3, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_NONE))
       return -6;
   }
   static bool attr_set[64] = {};

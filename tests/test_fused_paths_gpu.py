@@ -422,6 +422,37 @@ def test_products_on_a_thread_that_has_made_no_runtime_call():
     assert torch.equal(out[0], want) and _rel(target, a.double().t() @ a.double()) < 1e-5
 
 
+def test_forward_kernels_on_threads_that_have_made_no_runtime_call():
+    """A forward that autograd's worker computes again (a checkpoint), for the kernels with maps of their own."""
+    import threading
+    from tspipe_b200.ops import attention, conv, gemm
+    f = conv._f
+    torch.manual_seed(24)
+    a = torch.randn(256, 128, device=DEV).bfloat16()
+    q = torch.randn(1, 2, 128, 64, device=DEV).bfloat16()
+    x, wm = _cl(2, 3, 16, 16), conv.weight_matrix(torch.randn(64, 3, 7, 7, device=DEV) * 0.1)
+    y, word = _cl(2, 64, 8, 8), gemm._status_word(DEV)
+    runs = {"gemm": lambda: gemm.matmul_nt(a, a, two_cta=False), "attention": lambda: attention.flash_fwd(q, q, q),
+            "stem": lambda: f.lib().tsp_conv_stem_fwd(f._ptr(x), f._ptr(wm), f._ptr(y), None, 2, 16, 16, 1, f._ptr(word), f._stream())}
+    for run in runs.values():
+        run()                                          # (memory for the outputs is cached from here on)
+    torch.cuda.synchronize()
+    errors = {}
+    for name, run in runs.items():
+        def work():
+            try:
+                code = run()
+                if isinstance(code, int) and code != 0:
+                    errors[name] = code
+            except Exception as e:                     # noqa: BLE001
+                errors[name] = e
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+    gemm.check_status()
+    assert not errors, errors
+
+
 @pytest.mark.parametrize("n,h,w", [(1, 8, 8), (3, 10, 24), (2, 32, 224), (5, 64, 96)])
 def test_stem_weight_gradient(n, h, w):
     from tspipe_b200.ops import conv, gemm
