@@ -853,9 +853,9 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
 // box of x and its box of dY come once, both enumerated in the bordered pitch (dY's border columns are zero-filled by TMA
 // and cancel what x holds there), and the operand of tap (kh, kw) is the resident box read from row kh * pitch + kw on, as
 // in conv_halo_kernel.  M = two taps (their 64-channel blocks LBO apart: the distance of the two shifts), N = co, K = the
-// box's rows; the nine taps' accumulators, five of 128 x 64, stay in tensor memory over all tiles of a CTA.  (An infinite or
-// NaN x in an image's first or last column meets those zeros too: it reaches all three taps of a filter row, not only the
-// two that pair it with a dY.)
+// box's rows; the nine taps' accumulators, five of 128 x 64, stay in tensor memory over all tiles of a CTA.  An infinite or
+// NaN x in an image's first or last column or row meets those zeros too, in taps that do not pair it with a dY: sums that
+// come out infinite or NaN are formed again from the definition (add_wgrad_exact), so that they are so where they should be.
 // 256 images of 56 x 56, B200: 137 us with conv_wgrad_kernel, 79 with this one.
 struct WgHaloCfg {
   static constexpr int kXBytes = 384 * 128;                     // bordered box: up to 256 + 2 pitches + 2 rows
@@ -866,11 +866,41 @@ struct WgHaloCfg {
   static constexpr int kTmemCols = 512;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
 };
+// The share of a CTA's tiles in dW[co0 .. co0 + 31][tap][ci], one (tap, ci) per thread, as the sum over its pixels of dY and
+// the zero-padded x.
+__device__ __noinline__ void add_wgrad_exact(const Geom& g, const __nv_bfloat16* __restrict__ x,
+                                             const __nv_bfloat16* __restrict__ dy, int t_begin, int t_end, int tap, int ci,
+                                             int co0, float* __restrict__ dw) {
+  float acc[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+  for (int t = t_begin; t < t_end; ++t) {
+    int w0, h0, n0;
+    tile_origin(g, t, w0, h0, n0);
+    for (int h = h0; h < min(h0 + g.box_h, g.out_h); ++h)
+      for (int w = 0; w < g.out_w; ++w) {
+        const int xh = h + tap / 3 - 1, xw = w + tap % 3 - 1;
+        const bool inside = xh >= 0 && xh < g.out_h && xw >= 0 && xw < g.out_w;
+        const float xv = inside ? __bfloat162float(x[(((int64_t)n0 * g.out_h + xh) * g.out_w + xw) * 64 + ci]) : 0.f;
+        const __nv_bfloat16* row = dy + (((int64_t)n0 * g.out_h + h) * g.out_w + w) * 64 + co0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float v[8];
+          tsp::ld8(row, q * 8, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[q * 8 + e] = fmaf(xv, v[e], acc[q * 8 + e]);
+        }
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < 32; ++j) atomicAdd(dw + (int64_t)(co0 + j) * 576 + tap * 64 + ci, acc[j]);
+}
 __device__ __forceinline__ int first_tap(int pair) { return pair < 4 ? 2 * pair : 7; }      // the last pair repeats tap 7
 
 __global__ void __launch_bounds__(kWgThreads, 1)
 conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap dymap,
-                       const __grid_constant__ Geom g, float* __restrict__ dw, int* __restrict__ status) {
+                       const __grid_constant__ Geom g, const __nv_bfloat16* __restrict__ x,
+                       const __nv_bfloat16* __restrict__ dy, float* __restrict__ dw, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   using C = WgHaloCfg;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -963,14 +993,23 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
 #pragma unroll 1
       for (int a = 0; a < C::kPairs; ++a) {
         if (a == C::kPairs - 1 && quarter < 2) continue;
-        float* dst = dw + (first_tap(a) + (m >> 6)) * 64 + (m & 63);
+        const int tap = first_tap(a) + (m >> 6), ci = m & 63;
+        float* dst = dw + tap * 64 + ci;
 #pragma unroll 1
         for (int c0 = 0; c0 < 64; c0 += 32) {
           uint32_t r[32];
           tmem_ld_32x32_issue(tmem_base + ((uint32_t)(quarter * 32) << 16) + a * 64 + c0, r);
           tmem_ld_wait();
+          bool finite = true;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) atomicAdd(dst + (int64_t)(c0 + j) * 576, __uint_as_float(r[j]));
+          for (int j = 0; j < 32; ++j) finite = finite && (r[j] & 0x7f800000u) != 0x7f800000u;
+          if (finite) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) atomicAdd(dst + (int64_t)(c0 + j) * 576, __uint_as_float(r[j]));
+          } else {
+            add_wgrad_exact(g, x, dy, t_begin, t_end, tap, ci, c0, dw);
+          }
+          __syncwarp();
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1249,7 +1288,8 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int n, int h, in
   }
   const int num_tiles = g.tiles_w * g.tiles_h * g.tiles_n;
   const int n_sm = sm_count();
-  kern<<<num_tiles < n_sm ? num_tiles : n_sm, kWgThreads, WgHaloCfg::kSmemBytes, stream>>>(xmap, dymap, g, dw, status);
+  kern<<<num_tiles < n_sm ? num_tiles : n_sm, kWgThreads, WgHaloCfg::kSmemBytes, stream>>>(
+      xmap, dymap, g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, dw, status);
   return TSP_LAUNCH_CHECK();
 }
 

@@ -507,6 +507,27 @@ def test_convolution_weight_gradient_paths(n, h, w, cin, cout, k):
         assert _rel(weight.grad, twice * want) < 1e-5
 
 
+@pytest.mark.parametrize("n,h,w", [(1, 13, 9), (2, 5, 61), (3, 56, 56), (1, 66, 2)])
+def test_infinities_stay_in_the_taps_that_they_meet(n, h, w):
+    """3x3 weight gradient with the bordered box resident: infinite and NaN activations in the corners and along the borders
+    of an image, against the taps' sums over the zero-padded activation one by one."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(25)
+    x, g = _cl(n, 64, h, w), _cl(n, 64, h, w)
+    for c, (i, j, v) in enumerate([(0, 0, math.inf), (h - 1, w - 1, math.nan), (h // 2, 0, -math.inf), (h // 2, w - 1, math.inf),
+                                   (0, w // 2, math.nan), (h - 1, w // 2, math.inf), (h - 1, 0, math.inf)]):
+        x[n - 1, 8 * c, i, j] = v
+    weight = (torch.randn(64, 64, 3, 3, device=DEV) * 0.1).to(memory_format=torch.channels_last).requires_grad_()
+    conv.conv2d(x, weight)[0].backward(g)
+    gemm.check_status()
+    xp, g6 = F.pad(x.double(), (1, 1, 1, 1)), g.double()
+    want = torch.stack([torch.stack([torch.einsum("nohw,nihw->oi", g6, xp[:, :, i: i + h, j: j + w]) for j in range(3)], -1)
+                        for i in range(3)], -2)
+    got, fin = weight.grad.double(), torch.isfinite(want)
+    assert not fin.all() and torch.equal(fin, torch.isfinite(got)) and torch.equal(want.isnan(), got.isnan())
+    assert torch.equal(want[want.isinf()], got[want.isinf()]) and _rel(got[fin], want[fin]) < 1e-5
+
+
 @pytest.mark.parametrize("block,cin,planes,stride,side", [("bottleneck", 256, 64, 1, 14), ("bottleneck", 128, 64, 2, 10),
                                                           ("basic", 64, 64, 1, 9), ("basic", 64, 128, 2, 8)])
 def test_residual_gradient_rides_in_the_data_gradient(block, cin, planes, stride, side):
