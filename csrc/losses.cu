@@ -198,11 +198,12 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
   float z[3] = {z1 * ex2((ps.ref() - ms) * kLog2e), zs * ex2((ps.ref() - ms) * k2), kd ? zt * ex2((pt.ref() - mt) * k2) : 0.f};
   block_all<3, false>(z, scratch + 64);
   const float l1 = has_ce ? log2f(z[0]) : 0.f, ls = kd ? log2f(z[1]) : 0.f, lt = kd ? log2f(z[2]) : 0.f;
-  // The divergence is formed from differences of logits in their own scale, not from the scaled logarithms: a class that the
-  // type's lowest value switches off stays finite there at every temperature above one (times log2(e) / T it is -inf below
-  // T = 1.44), and a class that the teacher gives no probability adds nothing, whatever the other factor is.
+  // The divergence is sum p (db - da) / T - (ln Zt - ln Zs) with db, da the logits below their row's maximum, not a sum of
+  // differences of logarithms: a class that the type's lowest value switches off stays finite at every temperature (times
+  // log2(e) / T it is -inf below T = 1.44), and the logarithms' own rounding does not enter.  A class that the teacher gives
+  // no probability adds nothing, whatever the other factor is (a NaN is kept).
   float kl = 0.f;
-  const float wt = w_kd * temp, inv_t = 1.f / temp, dl = (lt - ls) * kLn2;
+  const float wt = w_kd * temp;
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
     float a[V], b[V], g[V];
     load_part<TS, V>(sr, i, a);
@@ -211,8 +212,8 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
 #pragma unroll
       for (int e = 0; e < V; ++e) {
         const float da = a[e] - ms, db = b[e] - mt;
-        const float p = ex2(db * k2 - lt), t = p * ((db - da) * inv_t - dl);
-        kl += p != 0.f ? t : 0.f;                // (a NaN is kept)
+        const float p = ex2(db * k2 - lt);
+        if (p != 0.f) kl = fmaf(p, db - da, kl);
         g[e] = wt * (ex2(da * k2 - ls) - p);
       }
     } else {
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
   if (threadIdx.x == 0) {
     float v = 0.f;
     if (has_ce) v += w_ce * (l1 * kLn2 - (tsp::ld(sr, label) - ms));
-    if (kd) v += w_kd * temp * temp * total[0];
+    if (kd) v += w_kd * temp * (total[0] - temp * (lt - ls) * kLn2);
     atomicAdd(loss, (double)v);
   }
 }
