@@ -1048,6 +1048,12 @@ int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, int ad
   return TSP_LAUNCH_CHECK();
 }
 
+// The per-channel vectors that a kernel reads 16 bytes at a time.
+static bool vectors_ok(const void* a, const void* b, const void* c, const void* d) {
+  return ((((uintptr_t)a) | ((uintptr_t)b) | ((uintptr_t)c) | ((uintptr_t)d)) & 15) == 0;
+}
+
+// w, b, sums and fixed_mean_var: 16-byte aligned.
 // acc_sum / acc_sumsq / acc_count (optional): accumulators of the deferred running statistics; group g adds into
 // acc + g * acc_seg_stride, so that each group's mini-batch can be committed on its own.
 int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, const float* fixed_mean_var,
@@ -1056,6 +1062,7 @@ int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, con
                  cudaStream_t stream) {
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 4096 || segs < 1 || m % segs != 0) return -3;
+  if (!vectors_ok(w, b, sums, fixed_mean_var)) return -2;
   m /= segs;
 #define TSP_BN_APPLY(T, RES)                                                                                            \
   bn_apply_kernel<T, RES><<<dim3(apply_blocks(m * (c / 8), c / 8, RES ? ApplyVecs<T>::fwd_res : ApplyVecs<T>::fwd, segs), \
@@ -1075,6 +1082,7 @@ int tsp_bn_bwd_reduce(const void* dy, const void* x, const void* y, void* dres, 
                       cudaStream_t stream) {
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 8192 || segs < 1 || m % segs != 0) return -3;
+  if (!vectors_ok(w, bias, mean_rstd, nullptr)) return -2;
   m /= segs;
   if (stream_ok(m, c, dtype))
     return launch_stream<1>(x, dy, y, dres, mean_rstd, w, bias, relu, m, c, segs, sums, stream);
@@ -1098,6 +1106,7 @@ int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* 
                      int dtype, int segs, cudaStream_t stream) {
   if (m <= 0) return 0;
   if (c % 8 != 0 || c > 4096 || segs < 1 || m % segs != 0) return -3;
+  if (!vectors_ok(w, bias, mean_rstd, sums)) return -2;
   m /= segs;
   const int mask = y != nullptr ? 2 : (relu ? 1 : 0);
 #define TSP_BN_BWD(T, MASK)                                                                                             \
@@ -1139,6 +1148,7 @@ int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums
   PoolGeom g;
   const int rc = pool_geom(n, h, wd, c, segs, kPoolRows, &g);
   if (rc != 0) return rc;
+  if (!vectors_ok(w, b, sums, nullptr)) return -2;
   const dim3 grid = pool_grid(g, segs, 32);
   if (dtype == TSP_DTYPE_BF16)
     bn_relu_pool_kernel<__nv_bfloat16><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, idx, sums, w,
@@ -1158,6 +1168,7 @@ int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* x, cons
   PoolGeom g;
   const int rc = pool_geom(n, h, wd, c, segs, 1, &g);
   if (rc != 0) return rc;
+  if (!vectors_ok(w, mean_rstd, sums, nullptr)) return -2;
   const dim3 grid_r = pool_grid(g, segs, 2), grid_a = pool_grid(g, segs, 32);
   if (dtype == TSP_DTYPE_BF16) {
     using B = __nv_bfloat16;

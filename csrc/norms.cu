@@ -303,6 +303,7 @@ int tsp_layernorm_fwd(const void* x, const float* w, const float* b, void* y, fl
                       float eps, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8 * 32 * kLnMaxVec) return -3;
+  if ((((uintptr_t)w | (uintptr_t)b) & 15) != 0) return -2;            // (read 16 bytes at a time)
   return dtype == TSP_DTYPE_BF16
              ? launch_ln_fwd<__nv_bfloat16, false>(x, nullptr, nullptr, w, b, y, mean, rstd, rows, d, eps, stream)
              : launch_ln_fwd<float, false>(x, nullptr, nullptr, w, b, y, mean, rstd, rows, d, eps, stream);
@@ -313,6 +314,7 @@ int tsp_add_layernorm_fwd(const void* x, const void* a, void* sum, const float* 
                           float* rstd, int rows, int d, float eps, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8 * 32 * kLnMaxVec) return -3;
+  if ((((uintptr_t)w | (uintptr_t)b) & 15) != 0) return -2;            // (read 16 bytes at a time)
   return dtype == TSP_DTYPE_BF16 ? launch_ln_fwd<__nv_bfloat16, true>(x, a, sum, w, b, y, mean, rstd, rows, d, eps, stream)
                                  : launch_ln_fwd<float, true>(x, a, sum, w, b, y, mean, rstd, rows, d, eps, stream);
 }
@@ -331,6 +333,7 @@ int tsp_layernorm_bwd_add(const void* dy, const void* x, const void* skip, const
                           cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8 * 32 * kLnMaxVec) return -3;
+  if (((uintptr_t)w & 15) != 0) return -2;
   const int nb = tsp_layernorm_bwd_blocks(rows);
 #define TSP_LN(T, ADD) launch_ln_bwd<T, ADD>(dy, x, skip, w, mean, rstd, dx, dw, db, partial, rows, d, nb, add, stream)
   if (dtype == TSP_DTYPE_BF16) return skip != nullptr ? TSP_LN(__nv_bfloat16, true) : TSP_LN(__nv_bfloat16, false);
@@ -352,6 +355,7 @@ static int gelu_blocks(int64_t nv, int cpv, int per_thread) {
 int tsp_gelu_fwd(const void* x, const float* bias, void* y, int64_t n, int d, int dtype, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (n % 8 != 0 || (bias && d % 8 != 0)) return -3;
+  if (((uintptr_t)bias & 15) != 0) return -2;
   const int blocks = gelu_blocks(n / 8, bias ? d / 8 : 1, kGeluFwdVecs);
   if (dtype == TSP_DTYPE_BF16)
     gelu_fwd_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)x, bias, (__nv_bfloat16*)y, n, d);
@@ -364,6 +368,7 @@ int tsp_gelu_bwd(const void* dy, const void* x, const float* bias, void* dx, int
                  cudaStream_t stream) {
   if (n <= 0) return 0;
   if (n % 8 != 0 || (bias && d % 8 != 0)) return -3;
+  if (((uintptr_t)bias & 15) != 0) return -2;
   const int blocks = gelu_blocks(n / 8, bias ? d / 8 : 1, kGeluBwdVecs);
   if (dtype == TSP_DTYPE_BF16)
     gelu_bwd_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, bias,
