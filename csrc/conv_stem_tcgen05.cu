@@ -117,16 +117,6 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
-// MN-major operand tile: rows of 64 elements (128 bytes), 8-row groups 1024 bytes apart, the next 64 elements `lbo` on.
-__device__ __forceinline__ uint64_t mn_desc(uint32_t smem_addr, uint32_t lbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 __host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
@@ -534,9 +524,9 @@ conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_b
         const uint32_t a_addr = smem_u32(a_tiles + s * kAStageBytes), d_addr = smem_u32(dy_tiles + s * kDyBytes);
         for (int ks = 0; ks < ksteps; ++ks) {                  // 16 pixels further on: +2048 bytes
           const uint32_t acc = it > 0 || ks > 0 ? 1u : 0u;
-          const uint64_t db = mn_desc(d_addr + ks * 2048, kABlockBytes);
-          umma_bf16(tmem_base, mn_desc(a_addr + ks * 2048, kABlockBytes), db, idesc, acc);
-          umma_bf16(tmem_base + kCout, mn_desc(a_addr + kABlockBytes + ks * 2048, kABlockBytes), db, idesc, acc);
+          const uint64_t db = tc5::desc_mn_major(d_addr + ks * 2048, kABlockBytes);
+          umma_bf16(tmem_base, tc5::desc_mn_major(a_addr + ks * 2048, kABlockBytes), db, idesc, acc);
+          umma_bf16(tmem_base + kCout, tc5::desc_mn_major(a_addr + kABlockBytes + ks * 2048, kABlockBytes), db, idesc, acc);
         }
         umma_commit(empty_bar + s);
       }
