@@ -50,8 +50,9 @@ def qkv_mode() -> str:
 
 def project_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], heads: int):
     """``q, k, v`` as ``[B, H, N, D]`` views from the fused projection parameters ``weight [3C, C]``, ``bias [3C]``.
-    On CUDA in "split" mode this is three GEMMs on slices of the parameters, so that no packed qkv tensor exists
-    whose gradient autograd would have to assemble from dq, dk and dv; otherwise one GEMM and an unbind."""
+    On CUDA in "split" mode this is one GEMM whose column tiles go to three tensors (three GEMMs on slices of the parameters
+    where the blocks are not what the tcgen05 kernels take), so that no packed qkv tensor exists whose gradient autograd would
+    have to assemble from dq, dk and dv; otherwise one GEMM and an unbind."""
     from .linear import linear, linear_qkv
     b, n, c = x.shape
     if x.is_cuda and _QKV_MODE == "split":
