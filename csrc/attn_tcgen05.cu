@@ -518,8 +518,12 @@ __global__ void __launch_bounds__(256) nce_prepare_kernel(const NcePairs<T> in, 
 }
 
 // Merges the key chunks' softmax-weighted key sums o [2][chunks][n][256] with their weights (lse [2][chunks][n]), adds
-// 2T/n * (lse - q.k/T) to the loss and writes the gradient with respect to the queries as they came in, i.e. through
-// the normalisation: g = 2/n * (o - k), dq = (g - q^ (q^.g)) / |q|.
+// 2T/n * (lse - q^.k^ / T) to the loss and writes the gradient with respect to the queries as they came in, i.e. through
+// the normalisation: g = 2/n * (o - k^), dq = (g - q^ (q^.g)) / |q|.
+// lse and o come from rows q~, k~ rounded to bf16.  What the rounding of the row's own query and key does to lse is added to
+// first order, ((q^ - q~).o + p (k^ - k~).q~) / T with p the probability of the row's own key; q^.k^ and the gradient's k^ are
+// taken as they are.  Error of the loss and of the gradient against 64 bits, 256 rows: 6e-6 and 2.8e-3 with rounded rows
+// throughout (and as much with the logits in memory), 3e-7 and 1.7e-3 this way, in the same time.
 template <typename T>
 __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
                                                          const __nv_bfloat16* __restrict__ q16,
@@ -532,8 +536,9 @@ __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePair
   const int row = blockIdx.x * kNceRows + warp, pair = blockIdx.y;
   float contrib = 0.f;
   if (row < n) {
-    float q[8], qb[8], kb[8], acc[8] = {};
+    float q[8], k[8], qb[8], kb[8], acc[8] = {};
     tsp::ld8(pair ? in.q[1] : in.q[0], (int64_t)row * kNceDim + col, q);
+    tsp::ld8(pair ? in.k[1] : in.k[0], (int64_t)row * kNceDim + col, k);
     tsp::ld8(q16, ((int64_t)pair * n + row) * kNceDim + col, qb);
     tsp::ld8(k16, ((int64_t)pair * n_pad + row) * kNceDim + col, kb);
     const float* l = lse + (int64_t)pair * chunks * n + row;
@@ -548,19 +553,22 @@ __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePair
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] += wgt * ov[e];
     }
-    float pos = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) pos += qb[e] * kb[e];
-    pos = tsp::warp_sum(pos) / temp;
-    contrib = (m + logf(z) - pos) * (2.f * temp / n);
-    const float norm = row_norm(q), gs = 2.f / n;
-    float dot = 0.f;
+    const float norm = row_norm(q), knorm = row_norm(k), gs = 2.f / n;
+    float own = 0.f, dk = 0.f, rest = 0.f, dot = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       q[e] /= norm;
-      acc[e] = gs * (acc[e] / z - kb[e]);
+      k[e] /= knorm;
+      acc[e] /= z;
+      own += qb[e] * kb[e];
+      dk += (k[e] - kb[e]) * qb[e];
+      rest += (q[e] - qb[e]) * acc[e] - q[e] * k[e];
+      acc[e] = gs * (acc[e] - k[e]);
       dot += q[e] * acc[e];
     }
+    own = tsp::warp_sum(own); dk = tsp::warp_sum(dk); rest = tsp::warp_sum(rest);
+    const float lse_row = m + logf(z);
+    contrib = (lse_row + (rest + expf(own / temp - lse_row) * dk) / temp) * (2.f * temp / n);
     dot = norm > 1e-12f ? tsp::warp_sum(dot) : 0.f;       // a clamped norm is a constant
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = (acc[e] - q[e] * dot) / norm;

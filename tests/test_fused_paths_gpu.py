@@ -137,6 +137,22 @@ def test_nce_pair_matches_cross_entropy(n, dtype):
         assert _rel(a, b) < 8e-3
 
 
+@pytest.mark.parametrize("noise", [0.05, 0.7])
+@pytest.mark.parametrize("n,dtype", [(128, torch.float32), (512, torch.float32), (512, torch.bfloat16)])
+def test_nce_pair_does_not_round_its_value_to_16_bits(n, dtype, noise):
+    """Rounding rows to bf16 moves a score by some 2^-9 / sqrt(256) / T, 6e-4; the mean over n rows of either direction by 6e-4 /
+    sqrt(2 n) = 4e-5 at 128.  Corrected to first order what is left is second order and fp32 sums: a tenth of that at most."""
+    from tspipe_b200.ops import gemm
+    torch.manual_seed(26)
+    base = [torch.randn(n, 256, device=DEV) for _ in range(2)]
+    q1, q2, k1, k2 = ((base[i % 2] + noise * torch.randn(n, 256, device=DEV)).to(dtype) for i in range(4))
+    loss = gemm.info_nce_pair(q1, k1, q2, k2, 0.2)
+    lab = torch.arange(n, device=DEV)
+    ref = sum(0.4 * F.cross_entropy(F.normalize(a.double(), dim=1) @ F.normalize(b.double(), dim=1).t() / 0.2, lab)
+              for a, b in ((q1, k1), (q2, k2)))
+    assert abs(float(loss) - float(ref)) < 4e-6 * max(1.0, float(ref))
+
+
 # ---- optimizers ---------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("name", ["adamw", "sgd"])
 @pytest.mark.parametrize("shift", [0, 1])
