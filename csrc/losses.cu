@@ -49,7 +49,7 @@ struct PairPtrs {
   const T* y[2];
 };
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(128) byol_kernel(const PairPtrs<T> in, int n, int d, float scale,
+__global__ void __launch_bounds__(128) byol_kernel(const PairPtrs<T> in, int n, int d, float scale, double* __restrict__ sum,
                                                    float* __restrict__ loss, T* __restrict__ gx) {
   constexpr int V = VEC ? 8 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -87,7 +87,16 @@ __global__ void __launch_bounds__(128) byol_kernel(const PairPtrs<T> in, int n, 
   __shared__ float part[4];
   if (lane == 0) part[warp] = contrib;
   __syncthreads();
-  if (threadIdx.x == 0) atomicAdd(loss, scale * (part[0] + part[1] + part[2] + part[3]));
+  if (threadIdx.x == 0) {
+    const float v = part[0] + part[1] + part[2] + part[3];
+    if (sum == nullptr) {
+      atomicAdd(loss, scale * v);
+    } else {                                 // summed in 64 bits; behind the sum, how many blocks are done
+      atomicAdd(sum, (double)scale * v);
+      __threadfence();
+      if (atomicAdd(reinterpret_cast<unsigned*>(sum + 1), 1u) == gridDim.x * gridDim.y - 1) *loss = (float)atomicAdd(sum, 0.);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -335,13 +344,13 @@ bool rows_of_8(int d, const void* a, const void* b, const void* c) {
 }
 
 template <typename T>
-int launch_byol(const void* x0, const void* y0, const void* x1, const void* y1, int n, int d, float scale, float* loss,
-                void* gx, cudaStream_t stream) {
+int launch_byol(const void* x0, const void* y0, const void* x1, const void* y1, int n, int d, float scale, double* sum,
+                float* loss, void* gx, cudaStream_t stream) {
   const PairPtrs<T> in = {{(const T*)x0, (const T*)x1}, {(const T*)y0, (const T*)y1}};
   const dim3 grid((n + 3) / 4, x1 != nullptr ? 2 : 1);
   const bool vec = rows_of_8(d, x0, y0, gx) && rows_of_8(d, x1, y1, nullptr);
-  if (vec) byol_kernel<T, true><<<grid, 128, 0, stream>>>(in, n, d, scale, loss, (T*)gx);
-  else byol_kernel<T, false><<<grid, 128, 0, stream>>>(in, n, d, scale, loss, (T*)gx);
+  if (vec) byol_kernel<T, true><<<grid, 128, 0, stream>>>(in, n, d, scale, sum, loss, (T*)gx);
+  else byol_kernel<T, false><<<grid, 128, 0, stream>>>(in, n, d, scale, sum, loss, (T*)gx);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -352,19 +361,19 @@ extern "C" {
 int tsp_byol_loss(const void* x, const void* y, int n, int d, int dtype, float scale, float* loss, void* gx,
                   cudaStream_t stream) {
   if (n <= 0) return 0;
-  return dtype == TSP_DTYPE_BF16 ? launch_byol<__nv_bfloat16>(x, y, nullptr, nullptr, n, d, scale, loss, gx, stream)
-                                 : launch_byol<float>(x, y, nullptr, nullptr, n, d, scale, loss, gx, stream);
+  return dtype == TSP_DTYPE_BF16 ? launch_byol<__nv_bfloat16>(x, y, nullptr, nullptr, n, d, scale, nullptr, loss, gx, stream)
+                                 : launch_byol<float>(x, y, nullptr, nullptr, n, d, scale, nullptr, loss, gx, stream);
 }
 
 // Both directions of the symmetric loss: loss = scale * sum of the pairs (x0, y0) and (x1, y1), set and not added to;
-// gx [2][n][d].
+// gx [2][n][d]; `sum`: two doubles of scratch.
 int tsp_byol_loss_pair(const void* x0, const void* y0, const void* x1, const void* y1, int n, int d, int dtype,
-                       float scale, float* loss, void* gx, cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(loss, 0, sizeof(float), stream);
+                       float scale, double* sum, float* loss, void* gx, cudaStream_t stream) {
+  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  cudaError_t e = cudaMemsetAsync(sum, 0, 2 * sizeof(double), stream);
   if (e != cudaSuccess) return (int)e;
-  if (n <= 0) return 0;
-  return dtype == TSP_DTYPE_BF16 ? launch_byol<__nv_bfloat16>(x0, y0, x1, y1, n, d, scale, loss, gx, stream)
-                                 : launch_byol<float>(x0, y0, x1, y1, n, d, scale, loss, gx, stream);
+  return dtype == TSP_DTYPE_BF16 ? launch_byol<__nv_bfloat16>(x0, y0, x1, y1, n, d, scale, sum, loss, gx, stream)
+                                 : launch_byol<float>(x0, y0, x1, y1, n, d, scale, sum, loss, gx, stream);
 }
 
 int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,

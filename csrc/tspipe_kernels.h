@@ -30,7 +30,7 @@ int tsp_sgd_step(float* p, const float* g, float* buf, const int64_t* chunks, in
 int tsp_byol_loss(const void* x, const void* y, int n, int d, int dtype, float scale, float* loss, void* gx,
                   cudaStream_t stream);
 int tsp_byol_loss_pair(const void* x0, const void* y0, const void* x1, const void* y1, int n, int d, int dtype,
-                       float scale, float* loss, void* gx, cudaStream_t stream);
+                       float scale, double* sum, float* loss, void* gx, cudaStream_t stream);
 int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,
                     double* sum, float* loss, void* gx, cudaStream_t stream);
 int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,

@@ -96,6 +96,18 @@ def test_losses_of_many_rows_lose_nothing_in_their_sum():
         assert got.dtype == torch.float32 and abs(float(got) - float(want)) <= 4e-7 * abs(float(want))
 
 
+@pytest.mark.parametrize("n,d", [(1, 8), (2048, 256), (20000, 16)])
+def test_byol_loss_of_many_rows_loses_nothing_in_its_sum(n, d):
+    """Both directions' terms go into one 64-bit sum; every term is right to some 2^-22 and the roundings cancel."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(27)
+    o1, o2, t1, t2 = (torch.randn(n, d, device=DEV) for _ in range(4))
+    want = sum((2 - 2 * F.cosine_similarity(a.double(), b.double())).mean() for a, b in ((o1, t2), (o2, t1)))
+    for _ in range(2):                                 # (scratch of an earlier call)
+        got = fused.byol_loss(o1, o2, t1, t2)
+        assert got.dtype == torch.float32 and abs(float(got) - float(want)) <= (4e-7 if n == 1 else 2e-7) * abs(float(want))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,d", [(1, 8), (7, 256), (130, 100)])
 def test_byol_pair_equals_two_single_losses(n, d, dtype):

@@ -34,6 +34,7 @@ def lib():
         # declared argument types: plain numbers at a call, an object per argument less where a whole loss takes 100 us of host
         v, i, f = _c.c_void_p, _c.c_int, _c.c_float
         L.tsp_kd_ce_loss.argtypes = [v] * 4 + [i] * 4 + [f] * 3 + [v] * 4
+        L.tsp_byol_loss_pair.argtypes = [v] * 4 + [i] * 3 + [f] + [v] * 4
         L.tsp_cosine_loss.argtypes = [v] * 3 + [i] * 3 + [f] + [v] * 4
         L.tsp_scale.argtypes = [v] * 3 + [_c.c_int64, i, v]
         _lib = L
@@ -399,10 +400,11 @@ class _ByolBoth(torch.autograd.Function):
     def forward(ctx, x1, x2, y1, y2, scale):
         n, d = x1.shape
         loss = torch.empty((), dtype=torch.float32, device=x1.device)
+        total = torch.empty(2, dtype=torch.float64, device=x1.device)
         gx = torch.empty((2, n, d), dtype=x1.dtype, device=x1.device)
         with on_device(x1.device):
-            _check(lib().tsp_byol_loss_pair(_ptr(x1), _ptr(y1), _ptr(x2), _ptr(y2), _c.c_int(n), _c.c_int(d),
-                                            _c.c_int(_dt(x1)), _c.c_float(scale), _ptr(loss), _ptr(gx), _stream()),
+            _check(lib().tsp_byol_loss_pair(x1.data_ptr(), y1.data_ptr(), x2.data_ptr(), y2.data_ptr(), n, d, _dt(x1), scale,
+                                            total.data_ptr(), loss.data_ptr(), gx.data_ptr(), _raw_stream()),
                    "tsp_byol_loss_pair")
         _count()
         save_gradient(ctx, gx)
