@@ -193,3 +193,21 @@ def test_hyperparameters_of_a_launch():
         else:
             assert opt._hyper_of(rows).table == opt._hyper_table.data_ptr()
             assert opt._hyper_table[32, :2].tolist() == [32.5, 0.25]
+
+
+def test_learning_rate_set_after_loading_a_state_is_used():
+    """Loading replaces the optimizer's group dicts; a step on the flat buffers reads the new ones."""
+    import torch
+    from torch import nn
+    from tspipe_b200.optim import SGD
+    from tspipe_b200.runtime.state import FlatParams
+    ps = [nn.Parameter(torch.ones(5)), nn.Parameter(torch.ones(3))]
+    opt = SGD([dict(params=ps[:1]), dict(params=ps[1:], lr=0.5)], lr=0.25)
+    opt.bind_flat(FlatParams(ps, torch.device("cpu"), with_grad=True), use_kernel=False)
+    opt.load_state_dict(opt.state_dict())
+    opt.param_groups[0]["lr"] = 0.125
+    for p in ps:
+        p.grad.fill_(1.0)
+    opt.step()
+    assert torch.equal(ps[0].detach(), torch.full((5,), 0.875)) and torch.equal(ps[1].detach(), torch.full((3,), 0.5))
+    assert [g is h for g, h in zip(opt._groups, opt.param_groups)] == [True, True]

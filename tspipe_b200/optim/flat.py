@@ -26,15 +26,7 @@ class _FlatMixin:
 
     def bind_flat(self, flat, use_kernel: bool) -> None:
         self.flat, self.use_kernel = flat, bool(use_kernel)
-        self._seg_group: List[Dict[str, Any]] = []
-        by_id = {}
-        for g in self.param_groups:
-            for p in g["params"]:
-                by_id[id(p)] = g
-        for p in flat.params:
-            if id(p) not in by_id:
-                raise ValueError("a partition parameter is missing from the optimizer's param groups")
-            self._seg_group.append(by_id[id(p)])
+        self._bind_groups()
         self._flat_state: Dict[str, torch.Tensor] = {}
         self._steps = 0
         self.teacher_flat: Optional[torch.Tensor] = None     # set by the engine to fuse the EMA
@@ -43,12 +35,19 @@ class _FlatMixin:
             from ..ops import fused
             self._chunks = fused.build_chunks(flat.offsets, flat.numels, flat.device)
             self._norms = torch.zeros(2 * max(len(flat.params), 1), dtype=torch.float32, device=flat.device)
-            self._groups = list({id(g): g for g in self._seg_group}.values())
             index = {id(g): i for i, g in enumerate(self._groups)}
             self._codes = torch.tensor([index[id(g)] << 1 | (p.ndim > 1) for p, g in zip(flat.params, self._seg_group)],
                                        dtype=torch.int32, device=flat.device)
             self._hyper = fused.Hyper(seg_code=self._codes.data_ptr())
             self._hyper_rows, self._hyper_table = None, None
+
+    def _bind_groups(self) -> None:
+        """The parameter group of every segment, and the groups in the order of their first segment."""
+        by_id = {id(p): g for g in self.param_groups for p in g["params"]}
+        if any(id(p) not in by_id for p in self.flat.params):
+            raise ValueError("a partition parameter is missing from the optimizer's param groups")
+        self._seg_group: List[Dict[str, Any]] = [by_id[id(p)] for p in self.flat.params]
+        self._groups = list({id(g): g for g in self._seg_group}.values())
 
     def enable_dp(self, group, peer_grads, peer_params, self_index: int) -> None:
         """Data-parallel mode over peer-mapped buffers: this rank owns ``1/R`` of the flat range; the step
@@ -172,6 +171,8 @@ class _FlatMixin:
             sd = dict(sd)                      # the caller's dict stays as it was
             extra = sd.pop("tspipe_flat")
         super().load_state_dict(sd)
+        if self.flat is not None:
+            self._bind_groups()                # loading puts new dicts in the place of the groups
         if extra is not None and self.flat is not None:
             for k, v in extra["flat"].items():
                 self._buf(k).copy_(v)
