@@ -422,7 +422,8 @@ def byol_loss(o1, o2, t1, t2) -> torch.Tensor:
     n = o1.shape[0]
     if all(t.dim() == 2 and t.shape == o1.shape and t.dtype == o1.dtype and t.device == o1.device
            and t.is_contiguous() for t in (o1, o2, t1, t2)) and o1.dtype in (torch.float32, torch.bfloat16) and n > 0:
-        return _ByolBoth.apply(o1, o2, t2.detach(), t1.detach(), 1.0 / n)
+        t1, t2 = (t.detach() if t.requires_grad else t for t in (t1, t2))
+        return _ByolBoth.apply(o1, o2, t2, t1, 1.0 / n)
     return byol_pair_loss(o1, t2, 1.0 / n) + byol_pair_loss(o2, t1, 1.0 / n)
 
 

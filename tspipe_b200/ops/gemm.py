@@ -554,7 +554,8 @@ def info_nce_pair(q1: torch.Tensor, k1: torch.Tensor, q2: torch.Tensor, k2: torc
         if not (t.shape == q1.shape and t.dtype == q1.dtype and t.device == q1.device and t.is_contiguous()
                 and t.data_ptr() % 16 == 0):
             return None
-    return _NCEPair.apply(q1, q2, k1.detach(), k2.detach(), float(temp))
+    k1, k2 = (t.detach() if t.requires_grad else t for t in (k1, k2))
+    return _NCEPair.apply(q1, q2, k1, k2, float(temp))
 
 
 class _FusedNCEGathered(torch.autograd.Function):
