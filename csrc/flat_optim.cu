@@ -5,7 +5,7 @@
 // `benchmarks/soft_target/train_kd.py:209-213`, momentum update `benchmarks/byol/trainer.py:198-212`.
 // The reference runs 6-10 elementwise launches and two norm reductions PER TENSOR; here a whole
 // partition is one flat fp32 buffer cut into fixed-size chunks that never straddle a tensor, so a step
-// is two launches (LARS: norms, apply) or one (AdamW, SGD, EMA), bound by HBM (or NVLink for a peer source).
+// is one launch (LARS on buffers that fit L2: two), bound by HBM (or NVLink for a peer source).
 #include "common.cuh"
 #include "tspipe_kernels.h"
 
@@ -14,8 +14,8 @@ namespace {
 using tsp::Hyper;
 
 constexpr int kThreads = 256;
-// From this many chunks of up to 64 KB on, over all buffers of a step (80 MB), lars_apply_kernel<true> is used.
-constexpr int64_t kLarsBig = 1280;
+constexpr int kStepThreads = 256, kStepBlocks = 4;      // of lars_step_kernel, blocks per SM
+constexpr uint64_t kWaitNs = 2000000000ull;   // its waits give up after two seconds
 
 // ---------------------------------------------------------------------------------------------
 // EMA: t = m*t + (1-m)*s ; `s` may point into a peer GPU's memory (plain loads over NVLink).
@@ -70,6 +70,29 @@ __device__ __forceinline__ int vec4_body(const ChunkView& c, uintptr_t bits, boo
   return ((c.begin & 3) == 0 && (bits & 15) == 0 && !(has_t && (teacher_n & 3) != 0)) ? c.len >> 2 : 0;
 }
 
+// sum p^2 and sum (grad_scale*g + wd*p)^2 of this thread's share of a chunk
+__device__ __forceinline__ void lars_sums(const float* p, const float* __restrict__ g, const ChunkView& c, float grad_scale,
+                                          float wd, float& sp, float& su) {
+  sp = 0.f; su = 0.f;
+  const int n4 = ((c.begin & 3) == 0) ? (c.len >> 2) : 0;
+  const float4* p4 = reinterpret_cast<const float4*>(p + c.begin);
+  const float4* g4 = reinterpret_cast<const float4*>(g + c.begin);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n4; i += blockDim.x) {
+    const float4 a = p4[i], b = g4[i];
+    float u;
+    sp += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+    u = grad_scale * b.x + wd * a.x; su += u * u;
+    u = grad_scale * b.y + wd * a.y; su += u * u;
+    u = grad_scale * b.z + wd * a.z; su += u * u;
+    u = grad_scale * b.w + wd * a.w; su += u * u;
+  }
+  for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += blockDim.x) {
+    const float a = p[c.begin + i], u = grad_scale * g[c.begin + i] + wd * a;
+    sp += a * a; su += u * u;
+  }
+}
+
 // norms[2*seg] += sum p^2 ; norms[2*seg+1] += sum (grad_scale*g + wd*p)^2   (only segments with the adapt bit)
 __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __restrict__ p, const float* __restrict__ g,
                                                               const int64_t* __restrict__ chunks,
@@ -79,33 +102,8 @@ __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __res
   const ChunkView c = load_chunk(chunks, blockIdx.x);
   const int code = hyper.seg_code[c.seg];
   if ((code & 1) == 0) return;
-  const float wd = hyper.of(code)[1];                 // lr, wd, momentum, trust
-  float sp = 0.f, su = 0.f;
-  const bool vec = ((c.begin & 3) == 0);
-  if (vec) {
-    const float4* p4 = reinterpret_cast<const float4*>(p + c.begin);
-    const float4* g4 = reinterpret_cast<const float4*>(g + c.begin);
-    const int n4 = c.len >> 2;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < n4; i += kThreads) {
-      const float4 a = p4[i], b = g4[i];
-      float u;
-      sp += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
-      u = grad_scale * b.x + wd * a.x; su += u * u;
-      u = grad_scale * b.y + wd * a.y; su += u * u;
-      u = grad_scale * b.z + wd * a.z; su += u * u;
-      u = grad_scale * b.w + wd * a.w; su += u * u;
-    }
-    for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += kThreads) {
-      const float a = p[c.begin + i], u = grad_scale * g[c.begin + i] + wd * a;
-      sp += a * a; su += u * u;
-    }
-  } else {
-    for (int i = threadIdx.x; i < c.len; i += kThreads) {
-      const float a = p[c.begin + i], u = grad_scale * g[c.begin + i] + wd * a;
-      sp += a * a; su += u * u;
-    }
-  }
+  float sp, su;
+  lars_sums(p, g, c, grad_scale, hyper.of(code)[1], sp, su);         // lr, wd, momentum, trust
   sp = tsp::block_sum(sp, scratch);
   su = tsp::block_sum(su, scratch);
   if (threadIdx.x == 0) {
@@ -114,44 +112,25 @@ __global__ void __launch_bounds__(kThreads) lars_norms_kernel(const float* __res
   }
 }
 
-template <bool BIG>
+template <bool ONCE>
 __device__ __forceinline__ float4 ld_once(const float4* at) {
-  if constexpr (BIG) return __ldcs(at);
+  if constexpr (ONCE) return __ldcs(at);
   else return *at;
 }
-template <bool BIG>
+template <bool ONCE>
 __device__ __forceinline__ void st_once(float4* at, float4 v) {
-  if constexpr (BIG) __stcs(at, v);
+  if constexpr (ONCE) __stcs(at, v);
   else *at = v;
 }
 
-// LARS apply (+ optional fused momentum-teacher update for segments that have a local teacher copy):
+// LARS update of a chunk (+ optional fused momentum-teacher update for segments that have a local teacher copy):
 //   dp = adapt ? q*(gs*g + wd*p) : gs*g ; mu = mom*mu + dp ; p -= lr*mu ; [t = m*t + (1-m)*p]
-// BIG: buffers that do not fit L2 together (kLarsBig).  The chunks are then walked from the last one back, right behind
-// lars_norms_kernel, which has left the end of p and g in L2 (up to 126 MB of them); what only this kernel touches passes
-// L2 with evict-first hints.  Both passes over 25.6 M parameters with the teacher (409 MB): 164 us walked in the same order
-// without hints, 156 this way; 6 M (96 MB): 44 and 35.  Smaller buffers stay in L2 from step to step, where the hints
-// would push them out: 4 M without the teacher (48 MB), step and wait: 43.6 us with hints, 40.8 without.  (The order is an
-// argument of the launch: as a constant of the instantiation it costs 4 us at 25.6 M, by the schedule it gets.)
-template <bool BIG>
-__global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict__ p, const float* __restrict__ g,
-                                                              float* __restrict__ mu,
-                                                              const int64_t* __restrict__ chunks,
-                                                              const __grid_constant__ Hyper hyper, float grad_scale,
-                                                              const float* __restrict__ norms,
-                                                              float* __restrict__ teacher, int64_t teacher_n,
-                                                              float ema_m, int last_first) {
-  const ChunkView c = load_chunk(chunks, last_first ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
-  const int code = hyper.seg_code[c.seg];
-  const float* hp = hyper.of(code);
-  const float lr = hp[0], wd = hp[1], mom = hp[2], trust = hp[3];
-  const bool adapt = (code & 1) != 0;
-  float q = 1.f;
-  if (adapt) {
-    const float pn = sqrtf(norms[2 * c.seg]), un = sqrtf(norms[2 * c.seg + 1]);
-    q = (pn > 0.f && un > 0.f) ? trust * pn / un : 1.f;
-  }
-  const float wd_eff = adapt ? wd : 0.f;
+// ONCE: nothing of it is read again soon, so loads and stores carry evict-first hints.
+template <bool ONCE>
+__device__ __forceinline__ void lars_update(float* p, const float* __restrict__ g, float* __restrict__ mu,
+                                            const ChunkView& c, const float* hp, float q, float wd_eff, float grad_scale,
+                                            float* __restrict__ teacher, int64_t teacher_n, float ema_m) {
+  const float lr = hp[0], mom = hp[2];
   const float om = 1.f - ema_m;
   const bool has_t = teacher != nullptr;
   // 16-byte vectors over the aligned body (segments start on 256-byte boundaries), scalars for the tail
@@ -161,11 +140,11 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
   float4* m4 = reinterpret_cast<float4*>(mu + c.begin);
   float4* t4 = has_t ? reinterpret_cast<float4*>(teacher + c.begin) : nullptr;
 #pragma unroll 2
-  for (int i = threadIdx.x; i < n4; i += kThreads) {
-    float4 pv = p4[i], mv = ld_once<BIG>(m4 + i);
-    const float4 gv = ld_once<BIG>(g4 + i);
+  for (int i = threadIdx.x; i < n4; i += blockDim.x) {
+    float4 pv = ld_once<ONCE>(p4 + i), mv = ld_once<ONCE>(m4 + i);
+    const float4 gv = ld_once<ONCE>(g4 + i);
     const bool t_ok = has_t && (c.begin + 4 * (int64_t)i + 3 < teacher_n);
-    float4 tv = t_ok ? ld_once<BIG>(t4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 tv = t_ok ? ld_once<ONCE>(t4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #define TSP_LARS1(X)                                                   \
     {                                                                  \
       const float dp = q * (grad_scale * gv.X + wd_eff * pv.X);        \
@@ -175,11 +154,11 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
     }
     TSP_LARS1(x) TSP_LARS1(y) TSP_LARS1(z) TSP_LARS1(w)
 #undef TSP_LARS1
-    p4[i] = pv;
-    st_once<BIG>(m4 + i, mv);
-    if (t_ok) st_once<BIG>(t4 + i, tv);
+    st_once<ONCE>(p4 + i, pv);
+    st_once<ONCE>(m4 + i, mv);
+    if (t_ok) st_once<ONCE>(t4 + i, tv);
   }
-  for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += kThreads) {
+  for (int i = (n4 << 2) + threadIdx.x; i < c.len; i += blockDim.x) {
     const int64_t k = c.begin + i;
     const float pv = p[k];
     const float dp = q * (grad_scale * g[k] + wd_eff * pv);
@@ -188,6 +167,105 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
     const float np = pv - lr * m2;
     p[k] = np;
     if (has_t && k < teacher_n) teacher[k] = ema_m * teacher[k] + om * np;
+  }
+}
+
+// Trust ratio of a segment from the sums of its squares.
+__device__ __forceinline__ float lars_ratio(float trust, float pp, float uu) {
+  const float pn = sqrtf(pp), un = sqrtf(uu);
+  return (pn > 0.f && un > 0.f) ? trust * pn / un : 1.f;
+}
+
+// The second of two launches, behind lars_norms_kernel (or the exchange of norms between replicas).
+__global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict__ p, const float* __restrict__ g,
+                                                              float* __restrict__ mu,
+                                                              const int64_t* __restrict__ chunks,
+                                                              const __grid_constant__ Hyper hyper, float grad_scale,
+                                                              const float* __restrict__ norms,
+                                                              float* __restrict__ teacher, int64_t teacher_n,
+                                                              float ema_m) {
+  const ChunkView c = load_chunk(chunks, blockIdx.x);
+  const int code = hyper.seg_code[c.seg];
+  const float* hp = hyper.of(code);
+  const bool adapt = (code & 1) != 0;
+  const float q = adapt ? lars_ratio(hp[3], norms[2 * c.seg], norms[2 * c.seg + 1]) : 1.f;
+  lars_update<false>(p, g, mu, c, hp, q, adapt ? hp[1] : 0.f, grad_scale, teacher, teacher_n, ema_m);
+}
+
+// Norms and updates in one launch, for buffers that do not fit L2: a chunk's update follows its norms at a distance that
+// L2 holds, so p and g leave DRAM once.  `order` lists the work: every chunk twice (row = {segment << 1 | update, length,
+// begin}), its norms and, some chunks after the last norms of its segment, its update.  Blocks draw rows by ticket, so a
+// wait for a segment's norms is a wait for rows that blocks drew before and are working on: whatever the number of
+// resident blocks, the earliest unfinished row never waits.  sync[0] = ticket, sync[1 + seg] = pieces of the segment whose
+// norms are in; `need` = pieces per segment.  Bound by DRAM (p, g, mu, t once in, p, mu, t once out: 5.0 TB/s of it).  A step
+// over 25.6 M parameters with the teacher, microseconds: two launches 160, this one 144; without the teacher 127 and 109; 86 M
+// 494 and 463; 6 M (96 MB) 42 and 40.  Pieces of 32 KB and four blocks of 256 threads per SM: with pieces of 64 KB 147, of 16
+// KB 152; two blocks of 512 threads 149; three blocks of 256 159.
+__global__ void __launch_bounds__(kStepThreads, kStepBlocks)
+lars_step_kernel(float* p, const float* __restrict__ g, float* __restrict__ mu, const int4* __restrict__ order,
+                 int n_items, const int* __restrict__ need, const __grid_constant__ Hyper hyper, float grad_scale, float* norms,
+                 int* sync, float* __restrict__ teacher, int64_t teacher_n, float ema_m, int* __restrict__ status) {
+  __shared__ float scratch[33];
+  __shared__ int4 row;
+  __shared__ float ratio;
+  __shared__ int state;                             // of this block's row: 0 work, 1 no row left, 2 a wait ran out
+  int next = 0;
+  if (threadIdx.x == 0) next = atomicAdd(sync, 1);
+  for (;;) {
+    if (threadIdx.x == 0) {
+      state = 1;
+      if (next < n_items) {
+        state = 0;
+        row = __ldg(order + next);
+        next = atomicAdd(sync, 1);                  // the ticket after this one, under way while this row is worked on
+      }
+    }
+    __syncthreads();
+    if (state != 0) return;
+    ChunkView c;
+    c.seg = row.x >> 1;
+    c.len = row.y;
+    c.begin = (int64_t)(uint32_t)row.z | ((int64_t)row.w << 32);
+    const bool update = (row.x & 1) != 0;
+    const int code = __ldg(hyper.seg_code + c.seg);
+    const float* hp = hyper.of(code);
+    const bool adapt = (code & 1) != 0;
+    if (!update) {
+      if (adapt) {
+        float sp, su;
+        lars_sums(p, g, c, grad_scale, hp[1], sp, su);
+        sp = tsp::block_sum(sp, scratch);
+        su = tsp::block_sum(su, scratch);
+        if (threadIdx.x == 0) {
+          atomicAdd(norms + 2 * c.seg, sp);
+          atomicAdd(norms + 2 * c.seg + 1, su);
+          __threadfence();
+          atomicAdd(sync + 1 + c.seg, 1);
+        }
+      }
+    } else {
+      if (adapt && threadIdx.x == 0) {
+        const int want = __ldg(need + c.seg);
+        uint64_t t0 = 0;
+        for (int spin = 0; *((volatile int*)(sync + 1 + c.seg)) < want; ++spin) {
+          if ((spin & 31) != 31) continue;
+          uint64_t now;
+          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+          if (t0 == 0) t0 = now;
+          if (now - t0 > kWaitNs) {
+            atomicCAS(status, 0, 7);
+            state = 2;
+            break;
+          }
+        }
+        __threadfence();
+        ratio = lars_ratio(hp[3], __ldcg(norms + 2 * c.seg), __ldcg(norms + 2 * c.seg + 1));
+      }
+      __syncthreads();
+      if (state != 0) return;
+      lars_update<true>(p, g, mu, c, hp, adapt ? ratio : 1.f, adapt ? hp[1] : 0.f, grad_scale, teacher, teacher_n, ema_m);
+    }
+    __syncthreads();                                // the row and the ratio are read before the next ones are written
   }
 }
 
@@ -324,12 +402,25 @@ int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, in
   cudaError_t e = cudaMemsetAsync(norms, 0, sizeof(float) * 2 * (size_t)n_seg, stream);
   if (e != cudaSuccess) return (int)e;
   lars_norms_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, chunks, *(const Hyper*)hyper, grad_scale, norms);
-  if ((int64_t)n_chunks * (teacher != nullptr ? 4 : 3) >= kLarsBig)
-    lars_apply_kernel<true><<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms,
-                                                               teacher, teacher_n, ema_m, 1);
-  else
-    lars_apply_kernel<false><<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms,
-                                                                teacher, teacher_n, ema_m, 0);
+  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms, teacher,
+                                                       teacher_n, ema_m);
+  return TSP_LAUNCH_CHECK();
+}
+
+int tsp_lars_step_ordered(float* p, const float* g, float* mu, const void* order, int n_items, const int* need,
+                          const void* hyper, float grad_scale, float* work, int n_seg, float* teacher, int64_t teacher_n,
+                          float ema_m, int* status, cudaStream_t stream) {
+  if (n_items <= 0) return 0;
+  if ((reinterpret_cast<uintptr_t>(order) & 15) != 0) return -2;
+  cudaError_t e = cudaMemsetAsync(work, 0, sizeof(float) * (3 * (size_t)n_seg + 1), stream);
+  int dev = 0, sms = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return (int)e;
+  const int grid = n_items < kStepBlocks * sms ? n_items : kStepBlocks * sms;
+  lars_step_kernel<<<grid, kStepThreads, 0, stream>>>(p, g, mu, (const int4*)order, n_items, need, *(const Hyper*)hyper,
+                                                      grad_scale, work, (int*)(work + 2 * (size_t)n_seg), teacher, teacher_n,
+                                                      ema_m, status);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -346,8 +437,8 @@ int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, i
                    float grad_scale, const float* norms, float* teacher, int64_t teacher_n, float ema_m,
                    cudaStream_t stream) {
   if (n_chunks <= 0) return 0;
-  lars_apply_kernel<false><<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms,
-                                                              teacher, teacher_n, ema_m, 0);
+  lars_apply_kernel<<<n_chunks, kThreads, 0, stream>>>(p, g, mu, chunks, *(const Hyper*)hyper, grad_scale, norms, teacher,
+                                                       teacher_n, ema_m);
   return TSP_LAUNCH_CHECK();
 }
 

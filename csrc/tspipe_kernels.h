@@ -15,6 +15,9 @@ int tsp_ema_update(float* teacher, const float* student, int64_t n, float moment
 int tsp_lars_step(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const void* hyper,
                   float grad_scale, float* norms, int n_seg, float* teacher, int64_t teacher_n, float ema_m,
                   cudaStream_t stream);
+int tsp_lars_step_ordered(float* p, const float* g, float* mu, const void* order, int n_items, const int* need,
+                          const void* hyper, float grad_scale, float* work, int n_seg, float* teacher, int64_t teacher_n,
+                          float ema_m, int* status, cudaStream_t stream);
 int tsp_lars_norms(const float* p, const float* g, const int64_t* chunks, int n_chunks, const void* hyper,
                    float grad_scale, float* norms, int n_seg, cudaStream_t stream);
 int tsp_lars_apply(float* p, const float* g, float* mu, const int64_t* chunks, int n_chunks, const void* hyper,

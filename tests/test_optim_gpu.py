@@ -48,6 +48,37 @@ def test_groups_with_a_schedule_match_the_step_per_tensor(name, groups):
     _same(ps, ref, 3)
 
 
+@pytest.mark.parametrize("lag", [0, 1, 7, 1000])
+@pytest.mark.parametrize("ema", [False, True])
+def test_lars_norms_and_updates_in_one_launch(lag, ema):
+    """Tensors of less than a chunk to many, one with an odd length, at distances between norms and update from none to all
+    of the work; two steps, the second on the counters that the first has left."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(0)
+    shapes = [(33, 17), (41,), (700, 257), (3, 16384), (5,), (16384,), (900, 1024), (16385, 1)]
+    ps = [nn.Parameter(torch.randn(*s, device=DEV)) for s in shapes]
+    ref = [nn.Parameter(p.detach().clone()) for p in ps]
+    flat = FlatParams(ps, DEV, with_grad=True)
+    opt, ropt = MAKE["lars"](ps), MAKE["lars"](ref)
+    opt.bind_flat(flat, use_kernel=True)
+    order = fused.LarsOrder(opt._chunks, len(ps), DEV, lag=lag)
+    teacher = flat.data.clone() if ema else None
+    mu = torch.zeros_like(flat.data)
+    want = [p.detach().clone() for p in ref]
+    for step in range(2):
+        for p, q in zip(ps, ref):
+            q.grad = torch.randn_like(q)
+            p.grad.copy_(q.grad)
+        rows = [[g["lr"], g["weight_decay"], g["momentum"], g["trust_coefficient"]] for g in opt._groups]
+        fused.lars_step_ordered_(flat.data, flat.grad, mu, order, opt._hyper_of(rows), 1.0, teacher, 0.9)
+        ropt.step()
+        want = [0.9 * w + 0.1 * q.detach() for w, q in zip(want, ref)]
+    assert int(order.status) == 0
+    _same(ps, ref, 2)
+    if ema:
+        _same([flat._view(teacher, i, p.data) for i, p in enumerate(ps)], want, 2)
+
+
 def test_a_recorded_step_repeats_its_values_and_refuses_new_ones():
     ps, qs = _params(5), _params(5)
     lars, adam = MAKE["lars"](ps), MAKE["adamw"](qs)

@@ -211,3 +211,27 @@ def test_learning_rate_set_after_loading_a_state_is_used():
     opt.step()
     assert torch.equal(ps[0].detach(), torch.full((5,), 0.875)) and torch.equal(ps[1].detach(), torch.full((3,), 0.5))
     assert [g is h for g, h in zip(opt._groups, opt.param_groups)] == [True, True]
+
+
+@pytest.mark.parametrize("lag", [0, 3, 50, 10_000])
+def test_lars_order_updates_after_the_norms_of_the_whole_tensor(lag):
+    """Every chunk's norms and update once each, an update after all norms of its tensor (the wait in the kernel ends by this
+    order alone) and no earlier than ``lag`` chunks after its own."""
+    from tspipe_b200.ops import fused
+    numels = [5, 3 * fused.CHUNK, 100 * fused.CHUNK + 1, 64, 7 * fused.CHUNK - 1]
+    offsets = [sum((n + 63) // 64 * 64 for n in numels[:i]) for i in range(len(numels))]
+    chunks = fused.build_chunks(offsets, numels, "cpu").tolist()
+    rows, need = fused.LarsOrder.plan(chunks, len(numels), lag)
+    assert need == [-(-n // fused.CHUNK) for n in numels] and len(rows) == 2 * len(chunks)
+    at = [{}, {}]
+    for pos, (word, begin) in enumerate(rows):
+        seg, update, length = (word & 0xFFFFFFFF) >> 1, word & 1, word >> 32
+        assert begin not in at[update]
+        at[update][begin] = (pos, seg, length)
+    norms = [p for p, _, _ in sorted(at[0].values())]
+    for seg, begin, length in chunks:
+        assert at[0][begin][1:] == at[1][begin][1:] == (seg, length)
+        pos = at[1][begin][0]
+        assert pos > max(p for p, s, _ in at[0].values() if s == seg)
+        mine = norms.index(at[0][begin][0])
+        assert pos > norms[min(mine + lag, len(norms) - 1)]

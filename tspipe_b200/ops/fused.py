@@ -27,7 +27,7 @@ def lib():
     global _lib
     if _lib is None:
         L = _build.load()
-        for name in ("tsp_ema_update", "tsp_lars_step", "tsp_lars_norms", "tsp_lars_apply", "tsp_adamw_step",
+        for name in ("tsp_ema_update", "tsp_lars_step", "tsp_lars_step_ordered", "tsp_lars_norms", "tsp_lars_apply", "tsp_adamw_step",
                      "tsp_sgd_step", "tsp_byol_loss", "tsp_cosine_loss", "tsp_kd_ce_loss", "tsp_layernorm_fwd",
                      "tsp_layernorm_bwd", "tsp_layernorm_bwd_blocks", "tsp_gelu_fwd", "tsp_gelu_bwd"):
             getattr(L, name).restype = _c.c_int
@@ -253,6 +253,49 @@ def build_chunks(offsets: Sequence[int], numels: Sequence[int], device, lo: int 
     return torch.tensor(rows, dtype=torch.int64, device=device)
 
 
+# LARS with norms and updates in one launch (:class:`LarsOrder`): from this many chunks on over all buffers of a step
+# (80 MB), i.e. where they do not stay in L2 from one step to the next.
+LARS_ORDERED = 1280
+# Pieces of p and g (64 KB) between the norms and the update of a piece: 50 MB of L2.  Blocks hold 592 pieces and as many
+# tickets; with less between, updates wait for norms (592: 165 us where 769 takes 144), with more the time creeps up (1776: 147).
+LARS_LAG, LARS_PIECE = 768, 8192
+
+
+class LarsOrder:
+    """The order in which one launch forms the norms and makes the updates of a LARS step, and its workspace."""
+
+    def __init__(self, chunks: torch.Tensor, n_seg: int, device, lag: int = LARS_LAG):
+        rows, need = self.plan([(s, pos, min(LARS_PIECE, begin + ln - pos)) for s, begin, ln in chunks.tolist()
+                                for pos in range(begin, begin + ln, LARS_PIECE)], n_seg, lag)
+        self.order = torch.tensor(rows, dtype=torch.int64, device=device).view(-1, 2)
+        self.need = torch.tensor(need, dtype=torch.int32, device=device)
+        self.n_seg = n_seg
+        from .gemm import _status_word
+        self.status = _status_word(torch.device(device))
+        # sums of squares [2 n_seg], the ticket, finished pieces per segment
+        self.work = torch.zeros(3 * n_seg + 1, dtype=torch.float32, device=device)
+
+    @staticmethod
+    def plan(chunks, n_seg: int, lag: int):
+        """Rows ``(segment << 1 | update | length << 32, begin)`` from pieces ``(segment, begin, length)``: a piece's update
+        comes after the norms of all pieces of its segment (what makes the kernel's waits end), at the earliest ``lag`` pieces
+        after its own norms."""
+        need = [0] * n_seg
+        for s, _, _ in chunks:
+            need[s] += 1
+        last = {s: i for i, (s, _, _) in enumerate(chunks)}
+        rows, out = [], 0
+        for i in range(len(chunks) + lag):
+            if i < len(chunks):
+                s, begin, ln = chunks[i]
+                rows.append((s << 1 | ln << 32, begin))
+            while out < len(chunks) and out + lag <= i and last[chunks[out][0]] <= i:
+                s, begin, ln = chunks[out]
+                rows.append((s << 1 | 1 | ln << 32, begin))
+                out += 1
+        return rows, need
+
+
 class Hyper(ctypes.Structure):
     """Hyperparameters of a launch (``tsp::Hyper``): a code per segment, ``group << 1 | adapt``, in device memory, and the
     groups' values, by value or as a table in device memory."""
@@ -283,6 +326,16 @@ def lars_step_(p, g, mu, chunks, hyper, norms, grad_scale=1.0, teacher=None, ema
                                    _c.c_int64(0 if teacher is None else teacher.numel()), _c.c_float(ema_m),
                                    _stream()), "tsp_lars_step")
     _count(3)
+
+
+@torch.no_grad()
+def lars_step_ordered_(p, g, mu, order: LarsOrder, hyper, grad_scale=1.0, teacher=None, ema_m=0.0) -> None:
+    with on_device(p.device):
+        _check(lib().tsp_lars_step_ordered(_ptr(p), _ptr(g), _ptr(mu), _ptr(order.order), _c.c_int(order.order.shape[0]),
+                                           _ptr(order.need), _c.byref(Hyper.of(hyper)), _c.c_float(grad_scale), _ptr(order.work),
+                                           _c.c_int(order.n_seg), _ptr(teacher), _c.c_int64(0 if teacher is None else teacher.numel()),
+                                           _c.c_float(ema_m), _ptr(order.status), _stream()), "tsp_lars_step_ordered")
+    _count(2)
 
 
 @torch.no_grad()

@@ -184,6 +184,14 @@ class LARS(_FlatMixin, Optimizer):
         super().__init__(params, dict(lr=lr, weight_decay=weight_decay, momentum=momentum,
                                       trust_coefficient=trust_coefficient))
 
+    def bind_flat(self, flat, use_kernel: bool) -> None:
+        super().bind_flat(flat, use_kernel)
+        self._order = None
+        if self.use_kernel:
+            from ..ops import fused
+            if 4 * self._chunks.shape[0] >= fused.LARS_ORDERED:
+                self._order = fused.LarsOrder(self._chunks, len(flat.params), flat.device)
+
     @torch.no_grad()
     def step(self, closure=None, grad_scale: float = 1.0):
         if self.flat is None:
@@ -205,6 +213,10 @@ class LARS(_FlatMixin, Optimizer):
                     fused.sum_norms_(d["norm_table"], d["r"], self._norms)
                 fused.dp_lars_apply_(d["params"], d["r"], d["idx"], flat.grad, mu, d["chunks"], hp, self._norms)
                 self._dp_barrier()                      # every replica's parameters are complete
+                return
+            if self._order is not None and self._chunks.shape[0] * (3 if self.teacher_flat is None else 4) >= fused.LARS_ORDERED:
+                fused.lars_step_ordered_(flat.data, flat.grad, mu, self._order, self._hyper_of(rows), grad_scale,
+                                         self.teacher_flat, self.ema_momentum)
                 return
             fused.lars_step_(flat.data, flat.grad, mu, self._chunks, self._hyper_of(rows), self._norms, grad_scale,
                              self.teacher_flat, self.ema_momentum)
