@@ -109,6 +109,41 @@ __device__ __forceinline__ void cvt8(const Raw8<__nv_bfloat16>& r, float (&v)[8]
   for (int k = 0; k < 4; ++k) { const float2 f = __bfloat1622float2(h[k]); v[2 * k] = f.x; v[2 * k + 1] = f.y; }
 }
 
+// Two fp32 values that one instruction works on; each half is rounded as the scalar operation rounds.
+struct Pair {
+  uint64_t v;
+  __device__ __forceinline__ Pair() {}
+  __device__ __forceinline__ Pair(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+  __device__ __forceinline__ void split(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+};
+__device__ __forceinline__ Pair operator+(Pair a, Pair b) {
+  Pair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair operator-(Pair a, Pair b) {
+  Pair r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair operator*(Pair a, Pair b) {
+  Pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ float total(Pair x) {
+  float a, b;
+  x.split(a, b);
+  return a + b;
+}
+// two bf16 values as they lie in memory
+__device__ __forceinline__ Pair unpack2(uint32_t x) { return Pair(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u)); }
+
 // The values as T holds them.
 template <typename T, int N>
 __device__ __forceinline__ void round_as(float (&v)[N]) {

@@ -1,6 +1,7 @@
 """tcgen05 convolutions (stem 7 x 7 / 2, implicit-GEMM 1x1 / 3x3) and fused partition execution against plain PyTorch
 in fp32."""
 import copy
+import math
 
 import pytest
 import torch
@@ -31,6 +32,32 @@ def test_stem_conv_matches_fp32_reference(n, h, w):
     y.backward(g)
     ref.backward(g.float())
     torch.testing.assert_close(weight.grad, wr.grad, rtol=5e-2, atol=5e-2 * wr.grad.abs().max().item())
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 8, 8), (2, 10, 16), (3, 50, 200), (37, 18, 224), (1, 600, 24)])
+def test_stem_conv_rows_and_runs(n, h, w):
+    """Widths whose rows end inside a product, odd numbers of output rows, CTAs that begin and end inside an image; infinite and
+    NaN pixels reach the outputs whose window holds them and no other."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(5)
+    dev = torch.device("cuda", 0)
+    x = torch.randn(n, 3, h, w, device=dev).to(dtype=torch.bfloat16, memory_format=torch.channels_last)
+    weight = (torch.randn(64, 3, 7, 7, device=dev) * 0.1)
+    weight[3, 1, 2, 3] = 0.0
+    for bad in (False, True):
+        if bad:
+            x[0, 1, h // 2, w // 2], x[-1, 0, 0, 0], x[-1, 2, h - 1, w - 1] = math.inf, -math.inf, math.nan
+        y, sums = conv.stem_conv(x, weight, segments=n if n < 4 else 1)
+        gemm.check_status()
+        ref = F.conv2d(x.double(), weight.bfloat16().double(), stride=2, padding=3)
+        assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isinf(), ref.isinf())
+        ok = ref.isfinite()
+        # 147 products in fp32 and one rounding to bf16
+        assert float((y.double() - ref)[ok].norm() / ref[ok].norm()) < 2 ** -8
+        if not bad:
+            part = y.float().view(n if n < 4 else 1, -1, 64, h // 2, w // 2)
+            want = torch.stack([part.sum((1, 3, 4)), part.square().sum((1, 3, 4))], 1).view(sums.shape)
+            torch.testing.assert_close(sums, want, rtol=1e-4, atol=1e-4 * float(want.abs().max()))
 
 
 def test_fused_partition_matches_plain_sequential():
