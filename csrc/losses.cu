@@ -7,7 +7,7 @@
 // second sweep in autograd; the loss GPU holds the whole mini-batch, so these are latency- and
 // bandwidth-bound row kernels: one read of the rows (teacher rows may sit behind a peer pointer), one write of
 // the student gradient.
-#include "common.cuh"
+#include "tcgen05.cuh"
 #include "tspipe_kernels.h"
 
 namespace {
@@ -245,6 +245,283 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same on long bf16 rows (a vocabulary), one persistent block per SM, one exponential per logit instead of two (three on
+// labelled rows): the first sweep keeps e = 2^((x - m) k), m the warp's running maximum at that vector, of the teacher in
+// registers and of the student in shared memory (122 KB each for 30528 classes), and the second only scales them by one factor
+// per vector.  The divergence is summed in the first sweep as well, sum e_t ((b - mt) - (a - ms)), and follows the maxima
+// as the other sums do.  Meanwhile a producer warp streams the next rows into a ring with bulk copies.
+// Only for what it was made for, rows that fill the five vectors and several of them per SM: 8192 rows of 30528, a quarter masked
+// and one in seven labelled, 381 us with the kernel above and 342 with this one, 1000 rows 64.7 and 60.5; but 8192 of 24576 (four
+// vectors) 307 and 296, 8192 of 16384 226 and 234, 300 of 30528 27.5 and 30.6.  What bounds it is instruction issue beside the
+// exponentials (per vector: waits, maxima, references; per row: the sums over 24 warps); fewer warps with more of a row each are
+// slower for want of warps (12: 460 us where 24 take 410, unmasked).
+// Rows are drawn by ticket: masked ones cost next to nothing (the producer warp writes their zeros), so a fixed share of
+// rows per block would leave blocks idle at the end.  Per row one barrier among the computing warps, behind the first
+// sweep; its partial sums alternate between two buffers.
+// ---------------------------------------------------------------------------------------------
+constexpr int kRowWarps = 24, kRowThreads = kRowWarps * 32;     // computing threads; one more warp copies
+constexpr int kRowVecs = 5;                                     // 16-byte vectors of a row per thread
+constexpr int kPieceElems = kRowThreads * 8;                    // of one tensor: one vector per thread
+constexpr int kPieceBytes = kPieceElems * 2;
+constexpr int kRing = 4;                                        // pieces of s and t, 24 KB each
+constexpr int kRowSmem = kRing * 2 * kPieceBytes + kRowVecs * kPieceElems * 4 + 2 * kRing * 8 + 128;
+constexpr int kRowQueue = 4;                                    // rows that the ring and the sweeps may hold
+static_assert(kRing < kRowQueue * 2 && kRowSmem <= 227 * 1024, "a row in the ring is two pieces at least");
+constexpr uint64_t kRowWaitNs = 2000000000ull;                  // a wait gives up after two seconds
+constexpr int kStreamMin = (kRowVecs - 1) * kPieceElems + 8;    // elements of a row
+constexpr int kStreamRows = 1024;                               // rows: seven per SM
+
+using tsp::Pair;
+using tsp::fma2;
+using tsp::total;
+using tsp::unpack2;
+__device__ __forceinline__ Pair ex2(Pair x) {
+  float a, b;
+  x.split(a, b);
+  return Pair(ex2(a), ex2(b));
+}
+// The largest of eight values as they lie in memory (NaN only where all are, as fmaxf).
+__device__ __forceinline__ float top_of(const uint4& q) {
+  auto h = [](uint32_t x) { return *reinterpret_cast<const __nv_bfloat162*>(&x); };
+  const __nv_bfloat162 m = __hmax2(__hmax2(h(q.x), h(q.y)), __hmax2(h(q.z), h(q.w)));
+  return fmaxf(__low2float(m), __high2float(m));
+}
+// sum e (d + shift) f from sum e d and z = sum e, where references move by `shift` and sums shrink by `f`; nothing is left
+// of sums whose factor is zero, whatever they were
+__device__ __forceinline__ float moved(float sum, float z, float f, float shift) {
+  return f == 0.f ? 0.f : fmaf(z * f, shift, sum * f);
+}
+__device__ __forceinline__ float warp_top(float v) {            // as tsp::warp_max
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ void row_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kRowThreads) : "memory"); }
+
+__global__ void __launch_bounds__(kRowThreads + 32, 1)
+kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __restrict__ t,
+                    const int64_t* __restrict__ labels, const uint8_t* __restrict__ row_mask, int n, int c, float temp,
+                    float w_ce, float w_kd, double* __restrict__ sum, float* __restrict__ loss,
+                    __nv_bfloat16* __restrict__ gs) {
+  extern __shared__ __align__(128) uint8_t ring[];
+  float4* kept = (float4*)(ring + kRing * 2 * kPieceBytes);       // the student's exponentials, [vector][half][thread]
+  uint64_t* full = (uint64_t*)(ring + kRing * 2 * kPieceBytes + kRowVecs * kPieceElems * 4);
+  uint64_t* empty = full + kRing;
+  __shared__ int2 rows[kRowQueue];                    // the rows in the ring: index (-1: no more) and label (-1: none)
+  __shared__ float part[2][6][32];
+  __shared__ int failed[2];                           // by row, as `part`: a wait of a computing warp ran out
+  __shared__ double block_part[kRowWarps];
+  __shared__ float2 refs[kRowWarps][kRowVecs];        // the maxima that a warp's exponentials refer to, of s and t
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nv = c / 8, pieces = (nv + kRowThreads - 1) / kRowThreads;
+  unsigned* counters = reinterpret_cast<unsigned*>(sum + 1);      // [0] ticket, [1] blocks that are done
+  int* status = reinterpret_cast<int*>(sum + 2);      // not 0 once a wait has run out: the loss is NaN then
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kRing; ++i) {
+      tc5::mbar_init(full + i, 1);
+      tc5::mbar_init(empty + i, kRowWarps);
+    }
+    failed[0] = failed[1] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (warp == kRowWarps) {
+    // ---------------- producer ----------------
+    uint32_t it = 0;
+    bool ok = true;
+    for (int r = 0; ok;) {
+      int row = 0;
+      if (lane == 0) row = (int)atomicAdd(counters, 1u);
+      row = __shfl_sync(0xffffffffu, row, 0);
+      if (row < n && row_mask != nullptr && row_mask[row] == 0) {
+        if (gs != nullptr) {
+          uint4* gr = reinterpret_cast<uint4*>(gs + (int64_t)row * c);
+          for (int i = lane; i < nv; i += 32) __stcs(gr + i, make_uint4(0, 0, 0, 0));
+        }
+        continue;
+      }
+      if (lane == 0) {
+        int label = -1;
+        if (row < n && labels != nullptr) {
+          const int64_t l = labels[row];
+          if (w_ce != 0.f && l >= 0 && l < c) label = (int)l;
+        }
+        for (int k = 0; k < pieces && ok; ++k, ++it) {
+          const int slot = it % kRing;
+          const uint32_t round = it / kRing;
+          if (round > 0) ok = tc5::mbar_wait_parked(empty + slot, (round - 1) & 1, status, 8, kRowWaitNs);
+          if (!ok) break;
+          // an entry is written again four rows on, behind a piece that every computing warp has released since it read it
+          if (k == 0) rows[r % kRowQueue] = make_int2(row < n ? row : -1, label);
+          if (row >= n) {
+            tc5::mbar_arrive(full + slot);
+            break;
+          }
+          const int first = k * kPieceElems;
+          const int64_t at = (int64_t)row * c + first;
+          const uint32_t bytes = 2u * (uint32_t)min(kPieceElems, c - first);
+          uint8_t* dst = ring + slot * 2 * kPieceBytes;
+          tc5::mbar_expect_tx(full + slot, 2 * bytes);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             tc5::smem_u32(dst + j * kPieceBytes)),
+                         "l"((j == 0 ? s : t) + at), "r"(bytes), "r"(tc5::smem_u32(full + slot))
+                         : "memory");
+        }
+        if (row >= n) ok = false;
+      }
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      ++r;
+    }
+  } else {
+    // ---------------- sweeps ----------------
+    const float k2 = kLog2e / temp, wt = w_kd * temp;
+    const Pair k2p(k2, k2);
+    double acc = 0.;
+    uint32_t slot = 0, phase = 0;                       // of the next piece
+    for (int r = 0;; ++r) {
+      int2 id = make_int2(0, -1);
+      bool ok = true;                                   // (the same for a whole warp)
+      Pair et[kRowVecs][4];                             // the teacher's exponentials
+      RowPart ps = {-INFINITY}, pt = {-INFINITY};
+      float z1 = 0.f, zs = 0.f, zt = 0.f, kl = 0.f;
+#pragma unroll
+      for (int k = 0; k < kRowVecs; ++k) {
+        if (k < pieces && ok && id.x >= 0) {
+          ok = __all_sync(0xffffffffu, tc5::mbar_wait(full + slot, phase, status, 9, kRowWaitNs)) != 0;
+          if (k == 0) id = ok ? rows[r % kRowQueue] : make_int2(-1, -1);
+          if (id.x >= 0 && ok) {
+            const uint4* piece = reinterpret_cast<const uint4*>(ring + slot * 2 * kPieceBytes) + threadIdx.x;
+            const bool mine = k * kRowThreads + threadIdx.x < nv;
+            uint4 qa = make_uint4(0, 0, 0, 0), qb = qa;
+            if (mine) { qa = piece[0]; qb = piece[kPieceBytes / 16]; }
+            __syncwarp();
+            if (lane == 0) tc5::mbar_arrive(empty + slot);             // every lane has its vectors
+            if (++slot == kRing) { slot = 0; phase ^= 1; }
+            const float tops = warp_top(mine ? top_of(qa) : -INFINITY), topt = warp_top(mine ? top_of(qb) : -INFINITY);
+            if (tops > ps.m || topt > pt.m) {
+              const RowPart ns = {fmaxf(ps.m, tops)}, nt = {fmaxf(pt.m, topt)};
+              const float ft = ex2((pt.ref() - nt.ref()) * k2);
+              if (id.y >= 0) z1 *= ex2((ps.ref() - ns.ref()) * kLog2e);
+              zs *= ex2((ps.ref() - ns.ref()) * k2);
+              kl = moved(kl, zt, ft, (pt.ref() - ps.ref()) - (nt.ref() - ns.ref()));
+              zt *= ft;
+              ps = ns;
+              pt = nt;
+            }
+            if (lane == 0) refs[warp][k] = make_float2(ps.ref(), pt.ref());
+            if (mine) {
+              const uint32_t a[4] = {qa.x, qa.y, qa.z, qa.w}, b[4] = {qb.x, qb.y, qb.z, qb.w};
+              const Pair ms2(ps.ref(), ps.ref()), mt2(pt.ref(), pt.ref());
+              Pair ss(0.f, 0.f), st(0.f, 0.f), sk(0.f, 0.f);
+              float es[8];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const Pair da = unpack2(a[j]) - ms2, db = unpack2(b[j]) - mt2, ea = ex2(da * k2p);
+                et[k][j] = ex2(db * k2p);
+                ss = ss + ea;
+                st = st + et[k][j];
+                ea.split(es[2 * j], es[2 * j + 1]);
+                float p0, p1, d0, d1;
+                et[k][j].split(p0, p1);
+                (db - da).split(d0, d1);
+                // a class that the teacher gives no probability adds nothing, whatever the other factor is
+                sk = fma2(et[k][j], Pair(p0 != 0.f ? d0 : 0.f, p1 != 0.f ? d1 : 0.f), sk);
+                if (id.y >= 0) {
+                  float da0, da1;
+                  da.split(da0, da1);
+                  z1 += ex2(da0 * kLog2e) + ex2(da1 * kLog2e);
+                }
+              }
+              zs += total(ss);
+              zt += total(st);
+              kl += total(sk);
+              float4* keep = kept + 2 * k * kRowThreads + threadIdx.x;
+              keep[0] = make_float4(es[0], es[1], es[2], es[3]);
+              keep[kRowThreads] = make_float4(es[4], es[5], es[6], es[7]);
+            }
+          }
+        }
+      }
+      const bool has_ce = id.y >= 0;
+      // the warp's sums, then the block's; a warp whose part is empty refers to a finite maximum
+      float (*pp)[32] = part[r & 1];
+      {
+        kl = tsp::warp_sum(kl);
+        z1 = has_ce ? tsp::warp_sum(z1) : 0.f;
+        zs = tsp::warp_sum(zs);
+        zt = tsp::warp_sum(zt);
+        if (lane == 0) {
+          pp[0][warp] = ps.m; pp[1][warp] = pt.m; pp[2][warp] = z1; pp[3][warp] = zs; pp[4][warp] = zt; pp[5][warp] = kl;
+          if (!ok) *((volatile int*)(failed + (r & 1))) = 1;
+        }
+      }
+      row_barrier();
+      if (*((volatile int*)(failed + (r & 1))) != 0 || id.x < 0) break;      // the same for all computing warps
+      const bool in = lane < kRowWarps;
+      const RowPart ws = {in ? pp[0][lane] : -INFINITY}, wtop = {in ? pp[1][lane] : -INFINITY};
+      const float ms = warp_top(ws.m), mt = warp_top(wtop.m);
+      if (warp == 0) {                                  // the divergence, by one warp
+        const float f = in ? ex2((wtop.ref() - mt) * k2) : 0.f;
+        kl = tsp::warp_sum(in ? moved(pp[5][lane], pp[4][lane], f, (wtop.ref() - ws.ref()) - (mt - ms)) : 0.f);
+      }
+      z1 = has_ce ? tsp::warp_sum(in ? pp[2][lane] * ex2((ws.ref() - ms) * kLog2e) : 0.f) : 0.f;
+      zs = tsp::warp_sum(in ? pp[3][lane] * ex2((ws.ref() - ms) * k2) : 0.f);
+      zt = tsp::warp_sum(in ? pp[4][lane] * ex2((wtop.ref() - mt) * k2) : 0.f);
+      const float l1 = has_ce ? log2f(z1) : 0.f, ls = log2f(zs), lt = log2f(zt);
+      if (threadIdx.x == 0) acc += (double)(wt * (kl / zt)) - (double)(w_kd * temp * (temp * (lt - ls) * kLn2));
+      // second sweep: the gradient
+      uint4* gr = gs ? reinterpret_cast<uint4*>(gs + (int64_t)id.x * c) : nullptr;
+      const uint4* sr = reinterpret_cast<const uint4*>(s + (int64_t)id.x * c);
+#pragma unroll
+      for (int k = 0; k < kRowVecs; ++k) {
+        const int i = k * kRowThreads + threadIdx.x;
+        if (i < nv) {
+          const float2 ref = refs[warp][k];
+          const float fs = wt * ex2((ref.x - ms) * k2 - ls), ft = -wt * ex2((ref.y - mt) * k2 - lt);
+          const Pair fs2(fs, fs), ft2(ft, ft);
+          const float4* keep = kept + 2 * k * kRowThreads + threadIdx.x;
+          const float4 e0 = keep[0], e1 = keep[kRowThreads];
+          Pair g[4] = {fma2(fs2, Pair(e0.x, e0.y), ft2 * et[k][0]), fma2(fs2, Pair(e0.z, e0.w), ft2 * et[k][1]),
+                       fma2(fs2, Pair(e1.x, e1.y), ft2 * et[k][2]), fma2(fs2, Pair(e1.z, e1.w), ft2 * et[k][3])};
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) g[j].split(v[2 * j], v[2 * j + 1]);
+          if (has_ce) {                                 // (the row once more, from L2)
+            float x[8];
+            const uint4 q = __ldg(sr + i);
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) unpack2(w[j]).split(x[2 * j], x[2 * j + 1]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float d = x[e] - ms;
+              v[e] += w_ce * (ex2(d * kLog2e - l1) - (i * 8 + e == id.y ? 1.f : 0.f));
+              if (i * 8 + e == id.y) acc += (double)(w_ce * (l1 * kLn2 - d));
+            }
+          }
+          if (gr) __stcs(gr + i, make_uint4(tc5::pack_bf16x2(v[0], v[1]), tc5::pack_bf16x2(v[2], v[3]),
+                                            tc5::pack_bf16x2(v[4], v[5]), tc5::pack_bf16x2(v[6], v[7])));
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) block_part[warp] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double v = 0.;
+    for (int w = 0; w < kRowWarps; ++w) v += block_part[w];
+    atomicAdd(sum, v);
+    __threadfence();
+    if (atomicAdd(counters + 1, 1u) == gridDim.x - 1)
+      *loss = *((volatile int*)status) == 0 ? (float)atomicAdd(sum, 0.) : __int_as_float(0x7fffffff);
+  }
+}
+
 // out = in * gout, the scaling of a precomputed loss gradient by the gradient of the loss (a scalar in device memory),
 // rounded to the tensor's type first as the product of two tensors of that type would be.  16-byte loads and stores, four in
 // flight per thread.  In place (out == in) a factor of one leaves nothing to do: 500 MB of gradient, forward and backward of
@@ -391,12 +668,25 @@ int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n
   return TSP_LAUNCH_CHECK();
 }
 
+// `sum`: three doubles of scratch.
 int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
                    int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* sum, float* loss, void* gs,
                    cudaStream_t stream) {
   if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
-  if (cudaError_t e = cudaMemsetAsync(sum, 0, sizeof(double), stream); e != cudaSuccess) return (int)e;
+  if (cudaError_t e = cudaMemsetAsync(sum, 0, 3 * sizeof(double), stream); e != cudaSuccess) return (int)e;
   const bool vec = rows_of_8(c, s, t, gs);
+  if (vec && t != nullptr && w_kd != 0.f && s_dtype == TSP_DTYPE_BF16 && t_dtype == TSP_DTYPE_BF16 &&
+      n >= kStreamRows && c >= kStreamMin && c <= kRowVecs * kPieceElems) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kd_ce_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmem);
+    if (e != cudaSuccess) return (int)e;
+    kd_ce_stream_kernel<<<n < sms ? n : sms, kRowThreads + 32, kRowSmem, stream>>>(
+        (const __nv_bfloat16*)s, (const __nv_bfloat16*)t, labels, row_mask, n, c, temp, w_ce, w_kd, sum, loss,
+        (__nv_bfloat16*)gs);
+    return TSP_LAUNCH_CHECK();
+  }
   // at least four accesses per thread and sweep on long rows, one warp of latency on short ones
   const int parts = vec ? c / 8 : c;
   const int threads = parts >= 2048 ? 512 : parts >= 512 ? 256 : parts >= 96 ? 128 : 64;

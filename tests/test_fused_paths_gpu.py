@@ -57,6 +57,39 @@ def test_kd_ce_rows_vectorised_and_not(n, c, dtype):
     assert _rel(g, gr) < max(2 * EPS[dtype], 1e-5)
 
 
+@pytest.mark.parametrize("n,c", [(1, 30528), (1023, 24584), (1024, 24576), (1024, 24584), (1025, 30528), (1100, 30720),
+                                 (1024, 30728)])
+def test_kd_ce_long_rows(n, c):
+    """Either side of the limits of the kernel that keeps a row on the chip (1024 rows, 24584 to 30720 elements), with masked
+    rows, a row without a label, one with classes switched off."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(0)
+    s, t = ((torch.randn(n, c, device=DEV) * 3).bfloat16() for _ in range(2))
+    s[0, : c // 2] = t[0, : c // 2] = torch.finfo(torch.bfloat16).min
+    y = torch.randint(c // 2 + 1, c, (n,), device=DEV)
+    on = torch.arange(n, device=DEV) % 5 != 3
+    y[n // 2] = -100 if n > 1 else c - 1
+    s.requires_grad_()
+    for row_mask, keep in ((on, on), (None, torch.ones_like(on))):
+        loss = fused.kd_ce_loss(s, t, y, 2.0, 0.5, 0.25, row_mask=row_mask)
+        (g,) = torch.autograd.grad(loss, s)
+        want, err, norm = 0.0, 0.0, 0.0
+        for rows in torch.arange(n, device=DEV).split(64):
+            r = s.detach()[rows].double().requires_grad_()
+            ls, lt = F.log_softmax(r / 2, 1), F.log_softmax(t[rows].double() / 2, 1)
+            term = torch.where(lt.exp() > 0, lt.exp() * (lt - ls), torch.zeros_like(ls))[keep[rows]]
+            ref = term.sum() + 0.5 * F.cross_entropy(r[keep[rows]], y[rows][keep[rows]], ignore_index=-100, reduction="sum")
+            (gr,) = torch.autograd.grad(ref, r)
+            want += float(ref.detach())
+            err += float((g[rows].double() - gr).square().sum())
+            norm += float(gr.square().sum())
+        assert abs(float(loss.detach()) - want) <= 1e-5 * abs(want)
+        assert math.sqrt(err / norm) < 2 * EPS[torch.bfloat16]
+        assert not g[~keep].any()
+    t[n - 1 if keep[n - 1] else 0, 9] = math.nan
+    assert fused.kd_ce_loss(s, t, y, 2.0, 0.5, 0.25).isnan()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("temp", [0.5, 1.0, 1.4, 2.0])
 def test_kd_with_classes_switched_off_at_every_temperature(temp, dtype):

@@ -487,7 +487,7 @@ class _KdCe(torch.autograd.Function):
         t2 = _rows(t) if isinstance(t, torch.Tensor) else t      # None, or a peer-mapped matrix read in place over NVLink
         n, c = s2.shape
         loss = torch.empty((), dtype=torch.float32, device=s2.device)
-        total = torch.empty((), dtype=torch.float64, device=s2.device)
+        total = torch.empty(3, dtype=torch.float64, device=s2.device)
         gs = torch.empty_like(s2)
         lab = labels
         if lab is not None and not (lab.dim() == 1 and lab.dtype == torch.int64 and lab.is_contiguous()):
