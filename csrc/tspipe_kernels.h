@@ -105,6 +105,9 @@ int tsp_gemm_bf16_tn_gathered_b(const void* a, void* const* b_srcs, int n_src, i
                                 int lda, int ldb, int ldc, int out_dtype, int* status, cudaStream_t stream);
 
 // ---- attn_tcgen05.cu ----------------------------------------------------------------------------------------------
+int tsp_attn_heads_fwd(const void* q, const void* k, const void* v, const uint8_t* mask, int64_t mask_stride, void* out,
+                       int batch, int heads, int nq, int nk, const int64_t* q_strides, const int64_t* k_strides,
+                       const int64_t* v_strides, float scale, int* status, cudaStream_t stream);
 int tsp_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int batch, int heads, int nq, int nk,
                  int d, int dv, const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                  const int64_t* o_strides, float scale, float fixed_max, int use_fixed_max, int out_dtype, int* status,

@@ -33,6 +33,60 @@ def test_flash_forward_head_dim_64(b, h, nq, nk):
     torch.testing.assert_close(lse, rl, rtol=1e-3, atol=1e-2)
 
 
+@pytest.mark.parametrize("b,h,nq,nk", [(2, 3, 197, 197), (1, 1, 1, 1), (1, 2, 128, 127), (2, 2, 257, 129), (3, 12, 50, 500),
+                                       (40, 12, 300, 512), (1, 1, 64, 4096)])
+@pytest.mark.parametrize("masked", ["none", "padding", "holes", "one for all"])
+def test_heads_forward(b, h, nq, nk, masked):
+    """Edges of the tiles of queries and keys, one item to several per SM, tiles of keys that are switched off at the end and in
+    between; maxima that grow from tile to tile.  Rounding: P and the output in bf16, sums in fp32."""
+    from tspipe_b200.ops import attention, gemm
+    torch.manual_seed(0)
+    dev = torch.device("cuda", 0)
+    n = max(nq, nk)
+    qkv = (torch.randn(b, n, 3, h, 64, device=dev) * 1.5).bfloat16()
+    qkv[:, :, 1] *= torch.linspace(0.2, 2, n, device=dev).bfloat16()[None, :, None, None]
+    q, k, v = qkv.permute(2, 0, 3, 1, 4)
+    q, k, v = q[:, :, :nq], k[:, :, :nk], v[:, :, :nk]
+    at = torch.arange(nk, device=dev)
+    mask = {"none": None, "padding": at[None] < torch.randint(1, nk + 1, (b, 1), device=dev),
+            "holes": ((at[None] // 128 % 2 == 1) & (torch.rand(b, nk, device=dev) < 0.5)) | (at[None] == nk - 1),
+            "one for all": (at % 3 != 1)[None] | (at == 0)[None]}[masked]
+    mask = None if mask is None else mask[:, None, None, :]
+    o = attention.heads_fwd(q, k, v, mask)
+    gemm.check_status()
+    assert o.shape == (b, h, nq, 64) and o.transpose(1, 2).is_contiguous()
+    s = (q.double() @ k.double().transpose(-1, -2)) / 8
+    want = torch.softmax(s if mask is None else s.masked_fill(~mask, -math.inf), -1) @ v.double()
+    assert float((o.double() - want).norm() / want.norm()) < 2 * 2 ** -8
+    if mask is not None and attention._TCGEN05 is None:
+        with torch.no_grad():
+            assert torch.equal(attention.attention(q, k, v, mask), o)
+
+
+def test_heads_forward_without_any_key():
+    from tspipe_b200.ops import attention
+    dev = torch.device("cuda", 0)
+    q, k, v = (torch.randn(3, 2, 300, 64, device=dev).bfloat16() for _ in range(3))
+    mask = torch.rand(3, 1, 1, 300, device=dev) < 0.5
+    mask[1] = False
+    assert torch.equal(attention.heads_fwd(q, k, v, mask)[1], attention.heads_fwd(q, k, v)[1])
+
+
+def test_heads_forward_leaves_the_rest_to_the_library():
+    from tspipe_b200.ops import attention
+    dev = torch.device("cuda", 0)
+    q = torch.randn(2, 3, 40, 64, device=dev).bfloat16()
+    full = torch.ones(2, 3, 40, 40, dtype=torch.bool, device=dev)
+    assert attention.heads_fwd(q, q, q, full) is None                             # per query
+    assert attention.heads_fwd(q, q, q, torch.zeros(2, 1, 1, 40, device=dev)) is None      # additive
+    assert attention.heads_fwd(q.float(), q.float(), q.float()) is None
+    assert attention.heads_fwd(q[..., :32], q[..., :32], q[..., :32]) is None
+    assert attention.heads_fwd(q, q[:1].expand(2, -1, -1, -1), q) is None         # a stride of zero
+    assert attention.heads_fwd(q, q[:, :, :30], q) is None
+    assert attention.heads_fwd(q[:, :, 1:], q, q) is not None
+    assert torch.vmap(lambda t: attention.attention(t, t, t))(q[None]).shape == (1, 2, 3, 40, 64)
+
+
 def test_attention_dispatch_and_vit_block_without_grad():
     """A ViT block gives the same result through the three attention paths: tcgen05 kernel (no gradient needed,
     opt-in), the library's fused attention on unbound q / k / v, and the packed-qkv library entry point."""

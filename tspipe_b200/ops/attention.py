@@ -5,9 +5,9 @@ The reference models run it unfused - two batched GEMMs, a softmax and a dropout
 `benchmarks/distilbert/bert.py`).  Here it is one fused call; ``mask`` is an additive or boolean
 key-padding mask broadcastable to [B, 1, 1, N] / [B, H, N, N].
 
-Forward passes that need no gradient (the teacher / momentum encoder) with head dimension 64 and no mask run on
-the tcgen05 kernel of ``csrc/attn_tcgen05.cu`` (:func:`flash_fwd`); everything else goes to the library's fused
-attention, which also provides the backward.
+Forward passes that need no gradient (the frozen teacher) with head dimension 64 and a boolean key-padding mask run on the
+tcgen05 kernel of ``csrc/attn_heads_tcgen05.cu`` (:func:`heads_fwd`); everything else goes to the library's fused attention,
+which also provides the backward.
 """
 from __future__ import annotations
 
@@ -18,15 +18,15 @@ from typing import Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-# The tcgen05 kernel launches one CTA per (128-query tile, head): at ViT sizes (197 tokens) that is two key tiles per
-# CTA and the per-CTA start-up dominates (343 us against the library's 105 us on [256, 12, 197, 64]), so it is opt-in
-# for attention; the contrastive loss (long key loops) uses it by default.
-_TCGEN05 = False
+# Forwards without a gradient on :func:`heads_fwd`: None = those with a mask, True = all, False = none.  The library turns a
+# mask into an additive matrix, which costs it more than the attention: [32, 12, 512, 64] 110 us with a padding mask and 45
+# without one, the kernel 58 and 57; [64, 12, 197, 64] without a mask 32 and 40.
+_TCGEN05: Optional[bool] = None
 
 
-def set_tcgen05(flag: bool) -> None:
+def set_tcgen05(flag: Optional[bool]) -> None:
     global _TCGEN05
-    _TCGEN05 = bool(flag)
+    _TCGEN05 = None if flag is None else bool(flag)
 
 
 _PACKED = {"state": None}     # None = not probed yet, True / False = usable or not
@@ -144,10 +144,56 @@ def flash_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional
     return o, (lse.view(b, h, nq) if want_lse else None)
 
 
+def _key_mask(mask: torch.Tensor, b: int, nk: int) -> Optional[torch.Tensor]:
+    """``mask`` as ``[b or 1, nk]`` when it is boolean and depends on the key (and the batch) alone, else None."""
+    if mask.dtype != torch.bool or mask.dim() != 4 or mask.shape[1] != 1 or mask.shape[2] != 1:
+        return None
+    if mask.shape[0] not in (1, b) or mask.shape[3] != nk or (nk > 1 and mask.stride(3) != 1):
+        return None
+    return mask[:, 0, 0]
+
+
+def heads_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: Optional[torch.Tensor] = None
+              ) -> Optional[torch.Tensor]:
+    """``softmax(q k^T / 8 + mask) v`` for bf16 ``[B, H, N, 64]`` tensors (any strides with a contiguous last dimension)
+    without a gradient, as a ``[B, H, Nq, 64]`` view of a ``[B, Nq, H, 64]`` buffer; None where the kernel does not take
+    them.  ``mask``: boolean, True = the key takes part, ``[B or 1, 1, 1, Nk]``."""
+    from . import fused as _f
+    from . import gemm as _gemm
+    ts = (q, k, v) if mask is None else (q, k, v, mask)
+    if any(_f._wrapped(t) for t in ts) or torch.autograd.forward_ad._current_level >= 0:
+        return None
+    if q.dim() != 4 or q.shape[-1] != 64 or not flash_eligible(q, k, v) or any(t.device != q.device for t in ts):
+        return None
+    b, h, nq, d = q.shape
+    nk = k.shape[2]
+    if k.shape != (b, h, nk, d) or v.shape != k.shape or nk > 4096 or b * h * nq == 0:
+        return None
+    if any(s <= 0 for t in (q, k, v) for s in t.stride()):
+        return None
+    m = None
+    if mask is not None:
+        m = _key_mask(mask, b, nk)
+        if m is None:
+            return None
+    o = torch.empty((b, nq, h, d), dtype=torch.bfloat16, device=q.device)
+    L = _f.lib()
+    L.tsp_attn_heads_fwd.restype = _c.c_int
+    with _f.on_device(q.device):
+        code = L.tsp_attn_heads_fwd(_f._ptr(q), _f._ptr(k), _f._ptr(v), _f._ptr(m),
+                                    _c.c_int64(0 if m is None or m.shape[0] == 1 else m.stride(0)), _f._ptr(o), _c.c_int(b),
+                                    _c.c_int(h), _c.c_int(nq), _c.c_int(nk), _strides3(q), _strides3(k), _strides3(v),
+                                    _c.c_float(1.0 / math.sqrt(d)), _f._ptr(_gemm._status_word(q.device)), _f._stream())
+    _f._check(code, "tsp_attn_heads_fwd")
+    _f._count()
+    return o.transpose(1, 2)
+
+
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: Optional[torch.Tensor] = None,
               dropout_p: float = 0.0) -> torch.Tensor:
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
-    if _TCGEN05 and mask is None and dropout_p == 0.0 and not needs_grad and q.shape[-1] == 64 \
-            and flash_eligible(q, k, v):
-        return flash_fwd(q, k, v)[0]
+    if (_TCGEN05 or (_TCGEN05 is None and mask is not None)) and dropout_p == 0.0 and not needs_grad and q.is_cuda:
+        o = heads_fwd(q, k, v, mask)
+        if o is not None:
+            return o
     return F.scaled_dot_product_attention(q, k, v, attn_mask=mask, dropout_p=dropout_p)
