@@ -96,16 +96,16 @@ __device__ __forceinline__ uint64_t desc_plain(uint32_t smem_addr, uint32_t lbo,
   return (uint64_t)((smem_addr >> 4) & 0x3FFF) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 | (uint64_t)1 << 46;
 }
 
-// Barrier over the first four warps that also ANDs a flag.
-__device__ __forceinline__ bool four_warps_and(bool ok) {
+// Barrier over the loading warps that also ANDs a flag.
+__device__ __forceinline__ bool loaders_and(bool ok) {
   uint32_t out;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 q, %1, 0;\n\t"
-      "bar.red.and.pred p, 1, 128, q;\n\t"
+      "bar.red.and.pred p, 1, %2, q;\n\t"
       "selp.b32 %0, 1, 0, p;\n\t}"
       : "=r"(out)
-      : "r"((uint32_t)ok)
+      : "r"((uint32_t)ok), "n"(kLoaders * 32)
       : "memory");
   return out != 0;
 }
@@ -395,13 +395,34 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
   }
 }
 
+// The share of tiles [t_begin, t_end) in dW[co][kh][kw][ch], i = co * 147 + kh * 21 + kw * 3 + ch, by a warp, lane = pixel.
+__device__ __noinline__ float exact_sum(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, int h, int w,
+                                        int oh_n, int ow_n, int per_image, int t_begin, int t_end, int i, int lane) {
+  const int co = i / kK, kh = i % kK / 21, kw = i % 21 / 3, ch = i % 3;
+  float v = 0.f;
+  for (int t = t_begin; t < t_end; ++t) {
+    const int n = t / per_image, oh0 = (t - n * per_image) * kTileRows;
+    for (int oh = oh0; oh < oh0 + kTileRows && oh < oh_n; ++oh) {
+      const int ih = 2 * oh - 3 + kh;
+      if (ih < 0 || ih >= h) continue;
+      for (int ox = lane; ox < ow_n; ox += 32) {
+        const int iw = 2 * ox - 3 + kw;
+        if (iw < 0 || iw >= w) continue;
+        v = fmaf(__bfloat162float(dy[(((int64_t)n * oh_n + oh) * ow_n + ox) * kCout + co]),
+                 __bfloat162float(x[(((int64_t)n * h + ih) * w + iw) * 3 + ch]), v);
+      }
+    }
+  }
+  return tsp::warp_sum(v);
+}
+
 // The pitch of a row is an odd multiple of 16 bytes: what a product reads of one pixel, 16 bytes of each of 16 rows, then lies in
 // all banks (with a pitch of 29 x 64 bytes in two 16-byte columns of them: 103 us, 97 this way, 82 issued by an elected lane).
 // dw[co][147] (fp32) += sum over this CTA's output rows of dY^T patch.  Accumulator c (columns 128 c ..): lane 8 r + 4 dx + ch,
 // column 64 j + co holds tap row r - 2 j, tap 2 c + dx.
 __global__ void __launch_bounds__(kWgThreads, 1)
-conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_bfloat16* __restrict__ x, int n_img, int h,
-                       int w, int oh_n, int ow_n, float* __restrict__ dw, int* __restrict__ status) {
+conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_bfloat16* __restrict__ x,
+                       const __nv_bfloat16* __restrict__ dy, int n_img, int h, int w, int oh_n, int ow_n, float* __restrict__ dw, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* dy_tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* ring = dy_tiles + kDyStages * kDyBytes;
@@ -444,34 +465,49 @@ conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_b
     load_rows<false>(ring, nullptr, full_bar, empty_bar, x, h, w, per_image, t_begin, t_end, status, warp, lane);
     // ---------------- epilogue: warps 0..3, TMEM lanes 32 * warp .. + 31 ----------------
     // (after a wait that ran out the accumulators hold part of their sums, or nothing: none of it is added)
-    if (warp < 4 && t_begin < t_end) {
-      const bool good = tc5::mbar_wait_warp(done_bar, 0, status, 3, kWaitNs, lane) && *((volatile int*)status) == 0;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (t_begin < t_end) {
+      bool good = true;
       float* sum = reinterpret_cast<float*>(dy_tiles);         // [co][147]; every tile of dY has been used
-      const int m = warp * 32 + lane, dx = (m >> 2) & 1, ch = m & 3;
+      if (warp < 4) {
+        good = tc5::mbar_wait_warp(done_bar, 0, status, 3, kWaitNs, lane) && *((volatile int*)status) == 0;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int m = warp * 32 + lane, dx = (m >> 2) & 1, ch = m & 3;
 #pragma unroll 1
-      for (int j = 0; j < 2; ++j) {
-        const int kh = (m >> 3) - 2 * j;
+        for (int j = 0; j < 2; ++j) {
+          const int kh = (m >> 3) - 2 * j;
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[64];
-          const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + c * 128 + j * kCout;
-          tc5::tmem_ld_32x32_issue(taddr, r);
-          tc5::tmem_ld_32x32_issue(taddr + 32, r + 32);
-          tc5::tmem_ld_wait();
-          const int kw = 2 * c + dx;
-          if (kh >= 0 && kh < 7 && kw < 7 && ch < 3) {
-            float* dst = sum + kh * 21 + kw * 3 + ch;
+          for (int c = 0; c < 4; ++c) {
+            uint32_t r[64];
+            const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + c * 128 + j * kCout;
+            tc5::tmem_ld_32x32_issue(taddr, r);
+            tc5::tmem_ld_32x32_issue(taddr + 32, r + 32);
+            tc5::tmem_ld_wait();
+            const int kw = 2 * c + dx;
+            if (kh >= 0 && kh < 7 && kw < 7 && ch < 3) {
+              float* dst = sum + kh * 21 + kw * 3 + ch;
 #pragma unroll
-            for (int co = 0; co < kCout; ++co)
-              dst[co * kK] = j == 0 ? __uint_as_float(r[co]) : dst[co * kK] + __uint_as_float(r[co]);
+              for (int co = 0; co < kCout; ++co)
+                dst[co * kK] = j == 0 ? __uint_as_float(r[co]) : dst[co * kK] + __uint_as_float(r[co]);
+            }
+          }
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      }
+      if (loaders_and(good)) {
+        // An infinite or NaN pixel also meets the zeros of dY past a row's end and of missing rows (0 x inf = NaN), in taps that
+        // do not pair it with a dY: sums that are not finite are formed again from the definition.
+        for (int i0 = warp * 32; i0 < kCout * kK; i0 += kLoaders * 32) {
+          const int i = i0 + lane;
+          uint32_t todo = __ballot_sync(0xffffffffu, i < kCout * kK && (__float_as_uint(sum[i]) & 0x7f800000u) == 0x7f800000u);
+          for (; todo != 0; todo &= todo - 1) {
+            const int k = i0 + __ffs(todo) - 1;
+            const float v = exact_sum(x, dy, h, w, oh_n, ow_n, per_image, t_begin, t_end, k, lane);
+            if (lane == 0) sum[k] = v;
           }
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      if (four_warps_and(good)) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        loaders_and(true);
         if ((reinterpret_cast<uintptr_t>(dw) & 15) == 0) {
           if (tid == 0) {
             asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dw),
@@ -481,7 +517,7 @@ conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_b
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
           }
         } else {
-          for (int i = tid; i < kCout * kK; i += 128) atomicAdd(dw + i, sum[i]);
+          for (int i = tid; i < kCout * kK; i += kLoaders * 32) atomicAdd(dw + i, sum[i]);
         }
       }
     }
@@ -625,7 +661,7 @@ int tsp_conv_stem_wgrad(const void* x, const void* dy, float* dw, int n, int h, 
   const int tiles = n * ((oh + kTileRows - 1) / kTileRows);
   const int usable = n_sm[dev] - g_tsp_sm_reserve > 8 ? n_sm[dev] - g_tsp_sm_reserve : 8;
   const int grid = tiles < usable ? tiles : usable;
-  conv_stem_wgrad_kernel<<<grid, kWgThreads, kWgSmemBytes, stream>>>(td, (const __nv_bfloat16*)x, n, h, w, oh, ow, dw, status);
+  conv_stem_wgrad_kernel<<<grid, kWgThreads, kWgSmemBytes, stream>>>(td, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, n, h, w, oh, ow, dw, status);
   return TSP_LAUNCH_CHECK();
 }
 
