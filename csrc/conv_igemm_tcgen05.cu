@@ -81,17 +81,20 @@ struct ActMaps {
   CUtensorMap m[4];
 };
 
-template <int BN>
+// ADD: 0 no addend, 1 read by the epilogue's threads, 2 fetched by TMA (flat pixel grid): see add_epilogue
+constexpr int kAddBufs = 4;
+template <int BN, int ADD>
 struct FwdCfg {
   static constexpr int kABytes = kBoxBytes;
   static constexpr int kBBytes = BN * 128;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = BN == 256 ? 4 : 6;
+  static constexpr int kStages = ADD == 2 ? (BN == 64 ? 4 : 2) : BN == 256 ? 4 : 6;
   static constexpr int kGroup = 2;                          // stages released per tcgen05.commit (a commit costs the
   static constexpr int kGroups = kStages / kGroup;          // issuing thread about as much as eight MMAs)
   static constexpr int kTmemCols = 2 * BN;
-  static constexpr int kStoreBytes = 8 * 32 * 128;          // one 32-row x 128-byte staging block per epilogue warp
-  static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256;
+  // 32-row x 128-byte staging blocks per epilogue warp
+  static constexpr int kStoreBytes = 8 * (ADD == 2 ? kAddBufs : 1) * 32 * 128;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256 + (ADD == 2 ? 8 * 8 * kAddBufs : 0);
 };
 
 // Tiles are dealt to the CTAs in contiguous ranges (tile index = n_tile * tiles_m + m_tile): a CTA then stays on one
@@ -137,22 +140,24 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
   uint32_t lt = 0;
   bool ok = true;
   constexpr int kStatBlocks = BN / 64;
-  float cs[kStatBlocks][4];
+  ColSums cs[(kStatBlocks + 1) / 2];                      // of this warp's 64-channel blocks
 #pragma unroll
-  for (int i = 0; i < kStatBlocks; ++i) { cs[i][0] = cs[i][1] = cs[i][2] = cs[i][3] = 0.f; }
+  for (int j = 0; j < (kStatBlocks + 1) / 2; ++j) cs[j].clear();
   int cur_c0 = -1, cur_seg = 0;
   auto flush_stats = [&]() {
     if (cur_c0 >= 0) {
       float* dst = col_sums + (int64_t)cur_seg * 2 * g.nc;
 #pragma unroll
-      for (int i = 0; i < kStatBlocks; ++i) {
-        const int col = cur_c0 + 64 * i + 2 * lane;
-        // (the blocks of the other warp of this lane quarter hold zeros here; nc is even: col and col + 1 exist together)
-        if (col < g.nc && (cs[i][1] != 0.f || cs[i][3] != 0.f)) {
-          atomicAdd(dst + col, cs[i][0]); atomicAdd(dst + g.nc + col, cs[i][1]);
-          atomicAdd(dst + col + 1, cs[i][2]); atomicAdd(dst + g.nc + col + 1, cs[i][3]);
+      for (int j = 0; j < (kStatBlocks + 1) / 2; ++j) {
+        float s[2], q[2];
+        cs[j].reduce(lane, s, q);
+        const int col = cur_c0 + 64 * (kStatBlocks == 1 ? 0 : 2 * j + group) + ColSums::channel(lane);
+        // (nc is a multiple of 64: col and col + 1 exist together)
+        if (col < g.nc && (q[0] != 0.f || q[1] != 0.f)) {
+          atomicAdd(dst + col, s[0]); atomicAdd(dst + g.nc + col, q[0]);
+          atomicAdd(dst + col + 1, s[1]); atomicAdd(dst + g.nc + col + 1, q[1]);
         }
-        cs[i][0] = cs[i][1] = cs[i][2] = cs[i][3] = 0.f;
+        cs[j].clear();
       }
     }
   };
@@ -257,17 +262,7 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
               __syncwarp();
             }
             // (the block's stores are on their way: the sums overlap them)
-            if (STATS) {
-              // column sums of the rounded block (rows that are not stored hold zeros): this lane owns columns
-              // 2 * lane and 2 * lane + 1
-#pragma unroll 8
-              for (int rr = 0; rr < 32; ++rr) {
-                const uint32_t wv = *reinterpret_cast<const uint32_t*>(buf + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) +
-                                                                       (lane & 3) * 4);
-                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wv));
-                cs[i][0] += f.x; cs[i][1] = fmaf(f.x, f.x, cs[i][1]); cs[i][2] += f.y; cs[i][3] = fmaf(f.y, f.y, cs[i][3]);
-              }
-            }
+            if (STATS) cs[i / 2].add(buf, lane);         // of the rounded block (rows that are not stored hold zeros)
           }
         }
       }
@@ -285,13 +280,10 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
     float* st = reinterpret_cast<float*>(buf);
 #pragma unroll
     for (int j = 0; j < (kStatBlocks + 1) / 2; ++j) {
-      const int i = kStatBlocks == 1 ? 0 : 2 * j + group;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int b = 0; b < kStatBlocks; ++b)
-        if (b == i) { v[0] = cs[b][0]; v[1] = cs[b][1]; v[2] = cs[b][2]; v[3] = cs[b][3]; }
-      *reinterpret_cast<float2*>(st + j * 128 + 2 * lane) = make_float2(v[0], v[2]);
-      *reinterpret_cast<float2*>(st + j * 128 + 64 + 2 * lane) = make_float2(v[1], v[3]);
+      float s[2], q[2];
+      cs[j].reduce(lane, s, q);
+      *reinterpret_cast<float2*>(st + j * 128 + ColSums::channel(lane)) = make_float2(s[0], s[1]);
+      *reinterpret_cast<float2*>(st + j * 128 + 64 + ColSums::channel(lane)) = make_float2(q[0], q[1]);
     }
     if (lane == 0) { st[512] = __int_as_float(ok ? cur_c0 : -1); st[513] = __int_as_float(cur_seg); }
   }
@@ -324,16 +316,99 @@ __device__ __forceinline__ void flush_cta_stats(const Geom& g, const uint8_t* st
   }
 }
 
+// Epilogue of a data gradient with an addend on a flat pixel grid.  Per warp a ring of staging blocks: the addend's block of
+// the third unit from here is on its way by TMA while this unit's sum is formed in its block and leaves it by TMA, so that
+// 96 KB per SM are in flight whatever the tile is waiting for.  Read by the threads instead, one tile ahead in registers, the
+// gradient of [256, 56, 56, 256] took 223 us, 157 this way (141 at the rate of a copy).
+template <int BN>
+__device__ __forceinline__ void add_epilogue(const Geom& g, int num_tiles, int tiles_m, uint32_t tmem_base,
+                                             uint64_t* tmem_full_bar, uint64_t* tmem_empty_bar, uint8_t* store_bufs,
+                                             uint64_t* add_bars, const CUtensorMap* __restrict__ omap,
+                                             const CUtensorMap* __restrict__ amap, int* __restrict__ status, int warp, int lane) {
+  const int quarter = warp & 3, group = (warp - 2) >> 2;
+  constexpr int kBlocks = BN / 64, kMine = (kBlocks + 1) / 2;         // 64-channel blocks of a tile, and of them this warp's
+  uint8_t* bufs = store_bufs + (warp - 2) * kAddBufs * (32 * 128);
+  uint64_t* bars = add_bars + (warp - 2) * kAddBufs;
+  const int t_begin = tile_begin(num_tiles, blockIdx.x), t_end = tile_begin(num_tiles, blockIdx.x + 1);
+  const bool idle = kBlocks == 1 && group == 1;
+  const int units = idle ? 0 : (t_end - t_begin) * kMine;
+  auto place = [&](int u, int& col, int& row) {
+    int w0, h0, n0, tm, tn;
+    split_tile(g, t_begin + u / kMine, tiles_m, (g.nc + BN - 1) / BN, tm, tn);
+    tile_origin(g, tm, w0, h0, n0);
+    col = tn * BN + 64 * (kBlocks == 1 ? 0 : 2 * (u % kMine) + group);
+    row = w0 + quarter * 32;
+  };
+  auto fetch = [&](int u) {                     // (a block past the last channel or pixel reads as zeros)
+    int col, row;
+    place(u, col, row);
+    uint64_t* bar = bars + u % kAddBufs;
+    mbar_expect_tx(bar, 32 * 128);
+    tma_load_2d(bufs + u % kAddBufs * (32 * 128), amap, bar, col, row);
+  };
+  if (lane == 0)
+    for (int u = 0; u < kAddBufs - 1 && u < units; ++u) fetch(u);
+  bool ok = true;
+  for (int t = t_begin, lt = 0; t < t_end && ok; ++t, ++lt) {
+    const uint32_t acc = lt & 1, use = lt >> 1;
+    ok = mbar_wait_warp(tmem_full_bar + acc, use & 1, status, 3, g.wait_ns, lane);
+    if (!ok) break;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < kMine; ++j) {
+      if (idle) continue;
+      const int u = lt * kMine + j;
+      uint8_t* buf = bufs + u % kAddBufs * (32 * 128);
+      uint32_t r[64];
+      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + (uint32_t)(64 * (kBlocks == 1 ? 0 : 2 * j + group));
+      tmem_ld_32x32_issue(taddr, r);
+      tmem_ld_32x32_issue(taddr + 32, r + 32);
+      ok = mbar_wait_warp(bars + u % kAddBufs, (u / kAddBufs) & 1, status, 3, g.wait_ns, lane);
+      tmem_ld_wait();
+      if (!ok) break;
+      uint8_t* my_row = buf + lane * 128;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        uint4* at = reinterpret_cast<uint4*>(my_row + ((q ^ (lane & 7)) << 4));
+        uint4 v = *at;
+        __nv_bfloat162* a = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          a[e] = __hadd2(__floats2bfloat162_rn(__uint_as_float(r[8 * q + 2 * e]), __uint_as_float(r[8 * q + 2 * e + 1])), a[e]);
+        *at = v;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        int col, row;
+        place(u, col, row);
+        if (col < g.nc && row < g.out_w) tma_store_2d(omap, buf, col, row);             // rows past the end are clipped
+        else asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        // the block of unit u - 1 is free once its store has read it: the next to be fetched takes it
+        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        if (u + kAddBufs - 1 < units) fetch(u + kAddBufs - 1);
+      }
+      __syncwarp();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(tmem_empty_bar + acc);
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  __syncwarp();
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // forward / data gradient
 // ---------------------------------------------------------------------------------------------------------------
-template <int BN, bool B_MN, bool STATS, bool ADD>
+template <int BN, bool B_MN, bool STATS, int ADD>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ CUtensorMap wmap,
-                const __grid_constant__ CUtensorMap omap, const __grid_constant__ Geom g, __nv_bfloat16* __restrict__ out,
+                const __grid_constant__ CUtensorMap omap, const __grid_constant__ CUtensorMap addmap,
+                const __grid_constant__ Geom g, __nv_bfloat16* __restrict__ out,
                 const __nv_bfloat16* __restrict__ addend, float* __restrict__ col_sums, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
-  using C = FwdCfg<BN>;
+  using C = FwdCfg<BN, ADD>;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* store_bufs = tiles + C::kStages * C::kStageBytes;
   uint64_t* bars = (uint64_t*)(store_bufs + C::kStoreBytes);
@@ -342,6 +417,7 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
   uint64_t* tmem_full_bar = bars + 2 * C::kStages;
   uint64_t* tmem_empty_bar = bars + 2 * C::kStages + 2;
   uint32_t* tmem_slot = (uint32_t*)(bars + 2 * C::kStages + 4);
+  uint64_t* add_bars = bars + 2 * C::kStages + 5;             // [8 warps][kAddBufs]  addend -> epilogue (ADD == 2)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = g.tiles_w * g.tiles_h * g.tiles_n, tiles_nn = (g.nc + BN - 1) / BN;
@@ -358,6 +434,8 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       mbar_init(tmem_full_bar + a, 1);
       mbar_init(tmem_empty_bar + a, 8);
     }
+    if (ADD == 2)
+      for (int i = 0; i < 8 * kAddBufs; ++i) mbar_init(add_bars + i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&amaps.m[0]) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
@@ -444,8 +522,12 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       }
     }
   } else {
-    fwd_epilogue<BN, 1, 2, STATS, ADD>(g, num_tiles, tiles_m, 1, tmem_base, tmem_full_bar, tmem_empty_bar, store_bufs,
-                                       out, addend, col_sums, status, warp, lane, &omap);
+    if constexpr (ADD == 2)
+      add_epilogue<BN>(g, num_tiles, tiles_m, tmem_base, tmem_full_bar, tmem_empty_bar, store_bufs, add_bars, &omap, &addmap,
+                       status, warp, lane);
+    else
+      fwd_epilogue<BN, 1, 2, STATS, ADD == 1>(g, num_tiles, tiles_m, 1, tmem_base, tmem_full_bar, tmem_empty_bar, store_bufs,
+                                              out, addend, col_sums, status, warp, lane, &omap);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1146,25 +1228,33 @@ Plan plan_input(const void* x, int n, int h, int w, int cin, int k, int s, int m
   return p;
 }
 
-template <int BN, bool B_MN, bool STATS, bool ADD>
-int launch_fwd(const Plan& p, const CUtensorMap& wmap, void* out, const void* addend, float* col_sums, int* status,
-               cudaStream_t stream) {
+template <int BN, bool B_MN, bool STATS, int ADD>
+int launch_fwd_kernel(const Plan& p, const CUtensorMap& wmap, const CUtensorMap& omap, const CUtensorMap& addmap, const Geom& g,
+                      void* out, const void* addend, float* col_sums, int* status, cudaStream_t stream) {
   auto kern = conv_fwd_kernel<BN, B_MN, STATS, ADD>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   dev &= 63;
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<BN>::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<BN, ADD>::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  Geom g = p.g;
   const int num_tiles = g.tiles_w * g.tiles_h * g.tiles_n * ((g.nc + BN - 1) / BN);
   const int n_sm = sm_count();
   const int grid = num_tiles < n_sm ? num_tiles : n_sm;
+  kern<<<grid, kThreads, FwdCfg<BN, ADD>::kSmemBytes, stream>>>(p.maps, wmap, omap, addmap, g, (__nv_bfloat16*)out,
+                                                                (const __nv_bfloat16*)addend, col_sums, status);
+  return TSP_LAUNCH_CHECK();
+}
+
+template <int BN, bool B_MN, bool STATS, bool ADD>
+int launch_fwd(const Plan& p, const CUtensorMap& wmap, void* out, const void* addend, float* col_sums, int* status,
+               cudaStream_t stream) {
+  Geom g = p.g;
   // flat pixel grid (1x1 stride 1, dense output rows): [pixels, nc] matrix written in 32-row x 64-channel TMA stores
-  CUtensorMap omap = wmap;
+  CUtensorMap omap = wmap, addmap = wmap;
   g.tma_store = 0;
   g.n_fastest = STATS ? 0 : 1;
   if (g.out_h == 1 && g.out_n == 1 && g.out_sw * 8 == g.nc && g.box_w == 128) {
@@ -1172,10 +1262,12 @@ int launch_fwd(const Plan& p, const CUtensorMap& wmap, void* out, const void* ad
     const uint64_t strides[2] = {2, (uint64_t)g.nc * 2};
     const uint32_t box[2] = {64, 32};
     if (make_bf16_map(&omap, out, 2, dims, strides, box)) g.tma_store = 1;
+    if constexpr (ADD) {
+      if (g.tma_store != 0 && make_bf16_map(&addmap, addend, 2, dims, strides, box))
+        return launch_fwd_kernel<BN, B_MN, STATS, 2>(p, wmap, omap, addmap, g, out, addend, col_sums, status, stream);
+    }
   }
-  kern<<<grid, kThreads, FwdCfg<BN>::kSmemBytes, stream>>>(p.maps, wmap, omap, g, (__nv_bfloat16*)out, (const __nv_bfloat16*)addend,
-                                                       col_sums, status);
-  return TSP_LAUNCH_CHECK();
+  return launch_fwd_kernel<BN, B_MN, STATS, ADD ? 1 : 0>(p, wmap, omap, addmap, g, out, addend, col_sums, status, stream);
 }
 
 template <bool B_MN, bool STATS, bool ADD = false>
@@ -1377,7 +1469,7 @@ int tsp_conv_fprop(const void* x, const void* wgt, void* y, float* col_sums, int
 // wgt[cout][k][k][cin] (read in place through MN-major operand tiles).  Every element of dx is written.  `addend`
 // (optional, dx's shape and layout; not for a 1x1 kernel of stride 2): added to the rounded result, the gradient that
 // reaches the input on another way (a residual connection).  The gradient of
-// [256, 56, 56, 256], B200: 220 us with it, 91 and 172 for the product and a separate addition.
+// [256, 56, 56, 256], B200: 157 us with it, 91 and 172 for the product and a separate addition.
 int tsp_conv_dgrad(const void* dy, const void* wgt, const void* addend, void* dx, int n, int h, int w, int cin, int cout,
                    int k, int s, int* status, cudaStream_t stream) {
   if (!shape_ok(n, h, w, cin, cout, k, s)) return -3;
