@@ -488,7 +488,11 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const bool issuer = tc5::elect_one();
+      auto arrived = [&](uint64_t* bar, uint32_t parity, int code) -> bool {      // the same for the warp
+        return __all_sync(0xffffffffu, tc5::mbar_wait(bar, parity, status, code, g.wait_ns)) != 0;
+      };
       constexpr uint32_t idesc = make_idesc(128, BN, false, B_MN);
       const uint32_t tiles_addr = smem_u32(tiles);
       uint32_t it = 0, lt = 0;
@@ -496,7 +500,7 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       for (int t = tile_begin(num_tiles, blockIdx.x); t < tile_begin(num_tiles, blockIdx.x + 1) && ok; ++t, ++lt) {
         const uint32_t acc = lt & 1, use = lt >> 1;
         if (use > 0) {
-          ok = mbar_wait(tmem_empty_bar + acc, (use - 1) & 1, status, 4, g.wait_ns);
+          ok = arrived(tmem_empty_bar + acc, (use - 1) & 1, 4);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
@@ -505,7 +509,7 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % C::kStages;
           const uint32_t round = it / C::kStages;
-          ok = mbar_wait(full_bar + s, round & 1, status, 2, g.wait_ns);
+          ok = arrived(full_bar + s, round & 1, 2);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_addr = tiles_addr + s * C::kStageBytes;
@@ -513,12 +517,12 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
           const uint32_t b_lo = B_MN ? desc_lo_mn_major(a_addr + C::kABytes, 8192) : desc_lo_k_major(a_addr + C::kABytes);
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {          // 16 along K: +32 bytes in a K-major row, +2048 bytes (16 rows) MN-major
-            umma_bf16_lo(d_tmem, a_lo + 2 * kk, b_lo + (B_MN ? 128 * kk : 2 * kk), idesc, accum);
+            if (issuer) umma_bf16_lo(d_tmem, a_lo + 2 * kk, b_lo + (B_MN ? 128 * kk : 2 * kk), idesc, accum);
             accum = 1u;
           }
-          if (it % C::kGroup == C::kGroup - 1) umma_commit(empty_bar + (it / C::kGroup) % C::kGroups);
+          if (issuer && it % C::kGroup == C::kGroup - 1) umma_commit(empty_bar + (it / C::kGroup) % C::kGroups);
         }
-        umma_commit(tmem_full_bar + acc);
+        if (issuer) umma_commit(tmem_full_bar + acc);
       }
     }
   } else {
@@ -565,7 +569,7 @@ struct HaloCfg {
 // loaded once and stay.  With 64 output channels a product takes the tensor pipe 63 clocks (its shared-memory reads), so
 // the issuing thread is the bound: the taps are unrolled without the ring's waits, and one commit per tile tells the
 // epilogue and, in place of a_empty, the producer.  256 images of 56 x 56, B200: forward with statistics
-// 119 us with the ring's loop, 96 this way; data gradient 110 and 94.
+// 119 us with the ring's loop, 96 this way, 77 with the products issued by a converged warp; data gradient 110, 94 and 72.
 template <int BN, bool B_MN, bool STATS, bool ADD>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap,
@@ -669,7 +673,11 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const bool issuer = tc5::elect_one();
+      auto arrived = [&](uint64_t* bar, uint32_t parity, int code) -> bool {      // the same for the warp
+        return __all_sync(0xffffffffu, tc5::mbar_wait(bar, parity, status, code, g.wait_ns)) != 0;
+      };
       constexpr uint32_t idesc = make_idesc(128, BN, false, B_MN);
       const uint32_t a_addr0 = smem_u32(a_tiles), b_addr0 = smem_u32(b_tiles);
       uint32_t ia = 0, ib = 0;
@@ -677,7 +685,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
       for (int lt = 0; lt < my_tiles && ok; ++lt) {
         const uint32_t acc = (uint32_t)lt % C::kAccBufs, use = (uint32_t)lt / C::kAccBufs;
         if (use > 0) {
-          ok = mbar_wait(tmem_empty_bar + acc, (use - 1) & 1, status, 4, g.wait_ns);
+          ok = arrived(tmem_empty_bar + acc, (use - 1) & 1, 4);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
@@ -685,13 +693,13 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         uint32_t accum = 0u;
         for (int cb = 0; cb < kcb && ok; ++cb, ++ia) {
           const int sa = ia % C::kAStages;
-          ok = mbar_wait(a_full + sa, (ia / C::kAStages) & 1, status, 2, g.wait_ns);
+          ok = arrived(a_full + sa, (ia / C::kAStages) & 1, 2);
           if (!ok) break;
           const uint32_t a_lo0 = desc_lo_k_major(a_addr0 + sa * C::kABytes);
           if constexpr (kMayReside) {
             if (resident) {
               if (ia == 0)
-                for (int tap = 0; tap < 9 && ok; ++tap) ok = mbar_wait(b_full + tap, 0u, status, 2, g.wait_ns);
+                for (int tap = 0; tap < 9 && ok; ++tap) ok = arrived(b_full + tap, 0u, 2);
               if (!ok) break;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
               const uint32_t b_lo0 = B_MN ? desc_lo_mn_major(b_addr0, 8192) : desc_lo_k_major(b_addr0);
@@ -700,7 +708,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                 for (int tap = 0; tap < 9; ++tap)
 #pragma unroll
                   for (int kk = 0; kk < 4; ++kk)
-                    umma_bf16_lo(d, a_first + 8 * g.tap_off[tap] + 2 * kk,
+                    if (issuer) umma_bf16_lo(d, a_first + 8 * g.tap_off[tap] + 2 * kk,
                                  b_lo0 + tap * (C::kBBytes >> 4) + (B_MN ? 128 * kk : 2 * kk), idesc, tap + kk > 0 ? 1u : 0u);
               };
               products(d_tmem, a_lo0);
@@ -710,7 +718,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
           }
           for (int tap = 0; tap < 9; ++tap, ++ib) {
             const int sb = (int)(ib % C::kBStages);
-            ok = mbar_wait(b_full + sb, (ib / C::kBStages) & 1, status, 2, g.wait_ns);
+            ok = arrived(b_full + sb, (ib / C::kBStages) & 1, 2);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t b_addr = b_addr0 + sb * C::kBBytes;
@@ -718,19 +726,19 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             const uint32_t a_lo = a_lo0 + 8 * g.tap_off[tap];        // one row = 128 bytes = 8 address units
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              umma_bf16_lo(d_tmem, a_lo + 2 * kk, b_lo + (B_MN ? 128 * kk : 2 * kk), idesc, kk == 0 ? accum : 1u);
+              if (issuer) umma_bf16_lo(d_tmem, a_lo + 2 * kk, b_lo + (B_MN ? 128 * kk : 2 * kk), idesc, kk == 0 ? accum : 1u);
             if (n_sub > 1) {
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)                         // second accumulator: 128 rows further on
-                umma_bf16_lo(d_tmem + BN, a_lo + 1024 + 2 * kk, b_lo + (B_MN ? 128 * kk : 2 * kk), idesc,
+                if (issuer) umma_bf16_lo(d_tmem + BN, a_lo + 1024 + 2 * kk, b_lo + (B_MN ? 128 * kk : 2 * kk), idesc,
                              kk == 0 ? accum : 1u);
             }
             accum = 1u;
-            if (ib % C::kBGroup == C::kBGroup - 1) umma_commit(b_empty + (ib / C::kBGroup) % C::kBGroups);
+            if (issuer && ib % C::kBGroup == C::kBGroup - 1) umma_commit(b_empty + (ib / C::kBGroup) % C::kBGroups);
           }
-          if (ok) umma_commit(a_empty + sa);
+          if (issuer && ok) umma_commit(a_empty + sa);
         }
-        umma_commit(tmem_full_bar + acc);
+        if (issuer) umma_commit(tmem_full_bar + acc);
       }
     }
   } else {
@@ -853,7 +861,11 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const bool issuer = tc5::elect_one();
+      auto arrived = [&](uint64_t* bar, uint32_t parity, int code) -> bool {      // the same for the warp
+        return __all_sync(0xffffffffu, tc5::mbar_wait(bar, parity, status, code, g.wait_ns)) != 0;
+      };
       constexpr uint32_t idesc = make_idesc(128, BN, true, true);
       const uint32_t tiles_addr = smem_u32(tiles);
       uint32_t it = 0, lt = 0;
@@ -863,7 +875,7 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
         const int b_lo = (int)((int64_t)boxes * sp / g.splits), b_hi = (int)((int64_t)boxes * (sp + 1) / g.splits);
         const uint32_t acc = lt & 1, use = lt >> 1;
         if (use > 0) {
-          ok = mbar_wait(tmem_empty_bar + acc, (use - 1) & 1, status, 4, g.wait_ns);
+          ok = arrived(tmem_empty_bar + acc, (use - 1) & 1, 4);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
@@ -872,18 +884,18 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
         for (int bx = b_lo; bx < b_hi; ++bx, ++it) {
           const int s = it % C::kStages;
           const uint32_t round = it / C::kStages;
-          ok = mbar_wait(full_bar + s, round & 1, status, 2, g.wait_ns);
+          ok = arrived(full_bar + s, round & 1, 2);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_addr = tiles_addr + s * C::kStageBytes;
           const uint32_t a_dlo = desc_lo_mn_major(a_addr, C::kBox), b_dlo = desc_lo_mn_major(a_addr + C::kABytes, C::kBox);
           for (int ks = 0; ks < ksteps; ++ks) {                     // 16 pixels further on: +2048 bytes
-            umma_bf16_lo(d_tmem, a_dlo + 128 * ks, b_dlo + 128 * ks, idesc, accum);
+            if (issuer) umma_bf16_lo(d_tmem, a_dlo + 128 * ks, b_dlo + 128 * ks, idesc, accum);
             accum = 1u;
           }
-          if (it % C::kGroup == C::kGroup - 1) umma_commit(empty_bar + (it / C::kGroup) % C::kGroups);
+          if (issuer && it % C::kGroup == C::kGroup - 1) umma_commit(empty_bar + (it / C::kGroup) % C::kGroups);
         }
-        umma_commit(tmem_full_bar + acc);
+        if (issuer) umma_commit(tmem_full_bar + acc);
       }
     }
   } else {
@@ -938,7 +950,7 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
 // box's rows; the nine taps' accumulators, five of 128 x 64, stay in tensor memory over all tiles of a CTA.  An infinite or
 // NaN x in an image's first or last column or row meets those zeros too, in taps that do not pair it with a dY: sums that
 // come out infinite or NaN are formed again from the definition (add_wgrad_exact), so that they are so where they should be.
-// 256 images of 56 x 56, B200: 137 us with conv_wgrad_kernel, 79 with this one.
+// 256 images of 56 x 56, B200: 137 us with conv_wgrad_kernel, 79 with this one (67 once the products were issued by a converged warp).
 struct WgHaloCfg {
   static constexpr int kXBytes = 384 * 128;                     // bordered box: up to 256 + 2 pitches + 2 rows
   static constexpr int kDyBytes = 256 * 128;
@@ -1040,13 +1052,17 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const bool issuer = tc5::elect_one();
+      auto arrived = [&](uint64_t* bar, uint32_t parity, int code) -> bool {      // the same for the warp
+        return __all_sync(0xffffffffu, tc5::mbar_wait(bar, parity, status, code, g.wait_ns)) != 0;
+      };
       constexpr uint32_t idesc = make_idesc(128, 64, true, true);
       const uint32_t tiles_addr = smem_u32(tiles);
       uint32_t accum = 0u;
       for (int t = t_begin; t < t_end; ++t) {
         const int it = t - t_begin, s = it % C::kStages;
-        if (!mbar_wait(full_bar + s, ((uint32_t)it / C::kStages) & 1, status, 2, g.wait_ns)) break;
+        if (!arrived(full_bar + s, ((uint32_t)it / C::kStages) & 1, 2)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t x_addr = tiles_addr + s * C::kStageBytes;
         const uint32_t b_lo = desc_lo_mn_major(x_addr + C::kXBytes, 8192);
@@ -1059,12 +1075,12 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
         for (int ks = 0; ks < ksteps; ++ks) {                     // 16 rows further on: +2048 bytes
 #pragma unroll
           for (int a = 0; a < C::kPairs; ++a)
-            umma_bf16_lo(tmem_base + a * 64, a_lo[a] + 128 * ks, b_lo + 128 * ks, idesc, accum);
+            if (issuer) umma_bf16_lo(tmem_base + a * 64, a_lo[a] + 128 * ks, b_lo + 128 * ks, idesc, accum);
           accum = 1u;
         }
-        umma_commit(empty_bar + s);
+        if (issuer) umma_commit(empty_bar + s);
       }
-      umma_commit(done_bar);
+      if (issuer) umma_commit(done_bar);
     }
   } else if (t_begin < t_end) {
     // ---------------- epilogue: add the accumulators into dW[co][(tap, ci)] ----------------

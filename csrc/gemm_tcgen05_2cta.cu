@@ -267,7 +267,11 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool issuer = tc5::elect_one();
+      auto arrived = [&](uint64_t* bar, uint32_t parity, int code) -> bool {      // the same for the warp
+        return __all_sync(0xffffffffu, tc5::mbar_wait(bar, parity, status, code, kWaitNs)) != 0;
+      };
       constexpr bool kAmn = KIND == kRed, kBmn = KIND == kNN || KIND == kRed;
       static_assert(!kBmn || BN % 128 == 0, "an MN-major half tile of B is whole 64-column boxes");
       constexpr uint32_t idesc = tc5::make_idesc(2 * BM, BN, kAmn, kBmn);
@@ -279,7 +283,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
         item_range(t, tile, kb_lo, kb_hi);
         const uint32_t acc = lt & 1, use = lt >> 1;
         if (use > 0) {
-          ok = tc5::mbar_wait(tmem_empty_bar + acc, (use - 1) & 1, status, 4, kWaitNs);
+          ok = arrived(tmem_empty_bar + acc, (use - 1) & 1, 4);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
@@ -288,7 +292,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
         for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t round = it / kStages;
-          ok = tc5::mbar_wait(full_bar + s, round & 1, status, 2, kWaitNs);
+          ok = arrived(full_bar + s, round & 1, 2);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_addr = tiles_addr + s * kStageBytes;
@@ -296,13 +300,13 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
           const uint32_t b_lo = kBmn ? tc5::desc_lo_mn_major(a_addr + kABytes, 8192) : tc5::desc_lo_k_major(a_addr + kABytes);
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {  // 16 along K: +32 bytes in a K-major row, +2048 bytes (16 rows) MN-major
-            umma_bf16_pair_lo(d_tmem, a_lo + (kAmn ? 128 : 2) * kk, b_lo + (kBmn ? 128 : 2) * kk, idesc, accum);
+            if (issuer) umma_bf16_pair_lo(d_tmem, a_lo + (kAmn ? 128 : 2) * kk, b_lo + (kBmn ? 128 : 2) * kk, idesc, accum);
             accum = 1u;
           }
           // the group's slots are free again in both CTAs once these MMAs have read them
-          if (it % kGroup == kGroup - 1) umma_commit_pair_both(smem_u32(empty_bar + (it / kGroup) % kGroups));
+          if (issuer && it % kGroup == kGroup - 1) umma_commit_pair_both(smem_u32(empty_bar + (it / kGroup) % kGroups));
         }
-        umma_commit_pair_both(smem_u32(tmem_full_bar + acc));
+        if (issuer) umma_commit_pair_both(smem_u32(tmem_full_bar + acc));
       }
     }
   } else {
