@@ -265,6 +265,54 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const T* __restrict__ dy,
   }
 }
 
+// The same with the column sums of dx (the gradient of the bias), of the values as they are stored: 32 lanes = 256 columns of a
+// row, eight warps = eight rows, blocks stacked over the rows, so that a thread keeps its columns' sums in registers and a
+// block adds one number per column.  [12608, 3072] bf16: 41 us and a pass of 16 for the sums, 48 this way.
+constexpr int kGeluSumRows = 8, kGeluSumVecs = 2;
+
+template <typename T>
+__global__ void __launch_bounds__(256) gelu_bwd_sums_kernel(const T* __restrict__ dy, const T* __restrict__ x,
+                                                            const float* __restrict__ bias, T* __restrict__ dx,
+                                                            float* __restrict__ sums, int64_t rows, int d) {
+  constexpr int U = kGeluSumVecs;
+  __shared__ float part[kGeluSumRows][256 + 8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int col = (blockIdx.x * 32 + lane) * 8;
+  const bool in = col < d;
+  float b[8] = {}, acc[8] = {};
+  if (in) tsp::ld8(bias, (int64_t)col, b);
+  const int64_t step = (int64_t)gridDim.y * kGeluSumRows;
+  for (int64_t r = (int64_t)blockIdx.y * kGeluSumRows + warp; in && r < rows; r += U * step) {
+    tsp::Raw8<T> xr[U], gr[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (r + u * step < rows) { tsp::ldraw(x, (r + u * step) * d + col, xr[u]); tsp::ldraw(dy, (r + u * step) * d + col, gr[u]); }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (r + u * step < rows) {
+        float v[8], g[8];
+        tsp::cvt8(xr[u], v);
+        tsp::cvt8(gr[u], g);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) g[e] *= tsp::gelu_grad_f<T>(v[e] + b[e]);
+        tsp::round_as<T>(g);
+        tsp::st8(dx, (r + u * step) * d + col, g);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += g[e];
+      }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) part[warp][lane * 8 + e] = acc[e];
+  __syncthreads();
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c < d) {
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < kGeluSumRows; ++k) v += part[k][threadIdx.x];
+    atomicAdd(sums + c, v);
+  }
+}
+
 template <typename T, bool ADD>
 int launch_ln_fwd(const void* x, const void* a, void* sum, const float* w, const float* b, void* y, float* mean, float* rstd,
                   int rows, int d, float eps, cudaStream_t stream) {
@@ -375,6 +423,25 @@ int tsp_gelu_bwd(const void* dy, const void* x, const float* bias, void* dx, int
                                                                (__nv_bfloat16*)dx, n, d);
   else
     gelu_bwd_kernel<float><<<blocks, 256, 0, stream>>>((const float*)dy, (const float*)x, bias, (float*)dx, n, d);
+  return TSP_LAUNCH_CHECK();
+}
+
+// Also adds the column sums of dx [rows, d] to sums [d] (fp32).  d % 8 == 0, bias 16-byte aligned.
+int tsp_gelu_bwd_sums(const void* dy, const void* x, const float* bias, void* dx, float* sums, int64_t rows, int d, int dtype,
+                      cudaStream_t stream) {
+  if (rows <= 0 || d <= 0) return 0;
+  if (d % 8 != 0) return -3;
+  if (bias == nullptr || ((uintptr_t)bias & 15) != 0) return -2;
+  const int slabs = (d + 255) / 256;
+  int64_t blocks = (rows + kGeluSumRows * kGeluSumVecs - 1) / (kGeluSumRows * kGeluSumVecs);
+  const int64_t most = (148 * 6 + slabs - 1) / slabs;                  // six blocks per SM
+  if (blocks > most) blocks = most;
+  const dim3 grid((unsigned)slabs, (unsigned)blocks);
+  if (dtype == TSP_DTYPE_BF16)
+    gelu_bwd_sums_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, bias,
+                                                                  (__nv_bfloat16*)dx, sums, rows, d);
+  else
+    gelu_bwd_sums_kernel<float><<<grid, 256, 0, stream>>>((const float*)dy, (const float*)x, bias, (float*)dx, sums, rows, d);
   return TSP_LAUNCH_CHECK();
 }
 

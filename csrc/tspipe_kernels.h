@@ -55,6 +55,8 @@ int tsp_layernorm_bwd_add(const void* dy, const void* x, const void* skip, const
 int tsp_gelu_fwd(const void* x, const float* bias, void* y, int64_t n, int d, int dtype, cudaStream_t stream);
 int tsp_gelu_bwd(const void* dy, const void* x, const float* bias, void* dx, int64_t n, int d, int dtype,
                  cudaStream_t stream);
+int tsp_gelu_bwd_sums(const void* dy, const void* x, const float* bias, void* dx, float* sums, int64_t rows, int d, int dtype,
+                      cudaStream_t stream);
 
 // ---- batchnorm.cu -----------------------------------------------------------------------------------------------
 int tsp_bn_stats(const void* x, int64_t m, int c, int dtype, float* sums, int segs, cudaStream_t stream);

@@ -333,6 +333,150 @@ def test_gelu_special_values_and_wide_bias(dtype):
             assert _rel(a, w) < 2 * EPS[dtype] + 1e-6
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d", [(1, 8), (17, 256), (16, 264), (4800, 520), (33, 776), (5000, 1024)])
+def test_layer_norm_widths(rows, d, dtype):
+    from tspipe_b200.ops import fused
+    torch.manual_seed(7)
+    x = (torch.randn(rows, d, device=DEV) + 1).to(dtype).requires_grad_()
+    w, b = torch.randn(d, device=DEV, requires_grad=True), torch.randn(d, device=DEV, requires_grad=True)
+    y = fused.layer_norm(x, w, b, 1e-6)
+    g = torch.randn_like(y)
+    got = torch.autograd.grad(y, [x, w, b], g)
+    leaves = [t.detach().double().requires_grad_() for t in (x, w, b)]
+    ref = F.layer_norm(leaves[0], (d,), leaves[1], leaves[2], 1e-6)
+    assert _rel(y, ref) < EPS[dtype] + 1e-6
+    for a, r in zip(got, torch.autograd.grad(ref, leaves, g.double())):
+        assert _rel(a, r) < 2 * EPS[dtype] + 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d,with_a", [(1, 8, True), (33, 264, True), (700, 768, True), (700, 768, False), (19, 1024, False)])
+def test_add_layer_norm_equals_the_separate_passes(rows, d, with_a, dtype):
+    from tspipe_b200.ops import fused
+    torch.manual_seed(14)
+    x, a = ((torch.randn(rows, d, device=DEV)).to(dtype).requires_grad_() for _ in range(2))
+    w, b = torch.randn(d, device=DEV, requires_grad=True), torch.randn(d, device=DEV, requires_grad=True)
+    gs, gy = torch.randn(rows, d, device=DEV).to(dtype), torch.randn(rows, d, device=DEV).to(dtype)
+    leaves = [x, w, b] + ([a] if with_a else [])
+    s, y = fused.add_layer_norm(x, a if with_a else None, w, b, 1e-6)
+    got = torch.autograd.grad([s, y], leaves, [gs, gy])
+    s2 = x + a if with_a else x
+    y2 = fused.layer_norm(s2, w, b, 1e-6)
+    want = torch.autograd.grad([s2, y2] if with_a else [y2], leaves, [gs, gy] if with_a else [gy])
+    if not with_a:
+        want = (want[0] + gs,) + want[1:]
+    for p, q in zip((s, y) + tuple(got), (s2, y2) + tuple(want)):
+        assert _rel(p, q) < 1e-6                       # bit-equal in bf16; fp32 products may be contracted differently
+    (only,) = torch.autograd.grad(fused.add_layer_norm(x, a if with_a else None, w, b, 1e-6)[1], x, gy)     # no gradient for s
+    assert _rel(only, torch.autograd.grad(fused.layer_norm(s2, w, b, 1e-6), x, gy)[0]) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape,views", [((2, 64, 8, 8), 2), ((3, 8, 5, 7), 1), ((4, 24, 9, 2), 2), ((2, 64, 30, 16), 1),
+                                         ((1, 512, 2, 3), 1), ((2, 64, 18, 33), 2), ((1, 2056, 3, 5), 1)])
+def test_batchnorm_relu_maxpool_equals_the_separate_passes(shape, views, dtype):
+    """Odd extents (last window of two rows or columns), strips that end early, channel counts off the block size, more
+    channels than a block takes."""
+    from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
+    from tspipe_b200.ops import bn as fbn
+    from tspipe_b200.ops.pool import MaxPool3x3s2
+    torch.manual_seed(8)
+    x = _cl(*shape, dtype=dtype).requires_grad_()
+    outs = []
+    for fused in (True, False):
+        mod = DeferredBatchNorm(shape[1]).to(DEV)
+        with torch.no_grad():
+            mod.weight.copy_(torch.linspace(-1, 2, shape[1]))
+            mod.bias.copy_(torch.linspace(0.5, -0.5, shape[1]))
+        group = BatchNormGroup(mod, chunks=10)
+        with fbn.segments(views):
+            y = fbn.bn_relu_pool(mod, x) if fused else MaxPool3x3s2()(fbn.bn_act(mod, x, None, True))
+        assert y is not None
+        torch.manual_seed(9)
+        g = _cl(*y.shape, dtype=dtype)
+        outs.append([y.detach(), *torch.autograd.grad(y, [x, mod.weight, mod.bias], g), group._acc])
+    for a, b in zip(outs[0], outs[1]):                 # same roundings, sums in another order
+        assert _rel(a, b) < EPS[dtype] + 1e-5
+
+
+# ---- tensor-core products -----------------------------------------------------------------------------------------
+@pytest.mark.parametrize("m,n,k", [(128, 64, 64), (300, 192, 128), (12608, 768, 64), (257, 4096, 192), (5000, 1024, 64)])
+def test_linear_products_at_every_tile_width(m, n, k):
+    """The widths that ``pick_bn`` chooses between: full and ragged last tiles in every direction, k tails in the weight
+    gradient (rows that are no multiple of 64)."""
+    from tspipe_b200.ops import gemm
+    torch.manual_seed(10)
+    x, w, dy = torch.randn(m, k, device=DEV).bfloat16(), torch.randn(n, k, device=DEV).bfloat16(), \
+        torch.randn(m, n, device=DEV).bfloat16()
+    assert _rel(gemm.matmul_nt(x, w), x.double() @ w.double().t()) < EPS[torch.bfloat16]
+    assert _rel(gemm.matmul_nn([dy], w), dy.double() @ w.double()) < EPS[torch.bfloat16]
+    dw = torch.ones(n, k, device=DEV)
+    gemm._add_weight_grad(dw, [dy], x)
+    gemm.check_status()
+    assert _rel(dw - 1, dy.double().t() @ x.double()) < 1e-5
+
+
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("rows,c,heads", [((2, 65), 192, 3), ((3, 197), 768, 12)])
+def test_fused_qkv_projection_matches_three_linears(rows, c, heads, bias):
+    from tspipe_b200.ops import gemm
+    from tspipe_b200.ops.attention import project_qkv
+    torch.manual_seed(11)
+    x = torch.randn(*rows, c, device=DEV).bfloat16().requires_grad_()
+    w = (torch.randn(3 * c, c, device=DEV) / math.sqrt(c)).requires_grad_()
+    b = torch.randn(3 * c, device=DEV, requires_grad=True) if bias else None
+    qkv = project_qkv(x, w, b, heads)
+    g = [torch.randn_like(t) for t in qkv]
+    leaves = [x, w] + ([b] if bias else [])
+    got = torch.autograd.grad(qkv, leaves, g)
+    gemm.check_status()
+    ref_leaves = [x.detach().double().requires_grad_(), w.detach().bfloat16().double().requires_grad_()] + \
+        ([b.detach().double().requires_grad_()] if bias else [])
+    ref = F.linear(*ref_leaves).view(*rows, 3, heads, c // heads).permute(2, 0, 3, 1, 4).unbind(0)
+    for a, r in zip(qkv, ref):
+        assert _rel(a, r) < EPS[torch.bfloat16]
+    for a, r in zip(got, torch.autograd.grad(ref, ref_leaves, [t.double() for t in g])):
+        assert _rel(a, r) < EPS[torch.bfloat16]
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("m,n,k", [(128, 64, 64), (300, 192, 128), (1000, 3072, 768)])
+def test_linear_gelu_epilogue_equals_the_separate_kernel(m, n, k, grad):
+    from tspipe_b200.ops import fused, gemm
+    torch.manual_seed(16)
+    x = torch.randn(m, k, device=DEV).bfloat16().requires_grad_(grad)
+    w = (torch.randn(n, k, device=DEV) * 2 / math.sqrt(k)).requires_grad_(grad)
+    b = torch.randn(n, device=DEV, requires_grad=grad)
+    y, ref = gemm.linear_gelu(x, w, b), fused.gelu(gemm.linear(x, w, None), b)
+    gemm.check_status()
+    assert _rel(y, ref) < 1e-4                         # the same roundings
+    if grad:
+        g = torch.randn_like(y)
+        for p, q in zip(torch.autograd.grad(y, [x, w, b], g), torch.autograd.grad(ref, [x, w, b], g)):
+            assert _rel(p, q) < 1e-4
+        gemm.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,d", [(1, 8), (17, 264), (16, 256), (128, 3072), (5000, 1000), (20000, 8200)])
+def test_gelu_backward_with_the_bias_gradient(rows, d, dtype):
+    """dx as the separate pass writes it, and its column sums added to what is there."""
+    from tspipe_b200.ops import fused as f
+    torch.manual_seed(25)
+    dy, x = ((torch.randn(rows, d, device=DEV) * 2).to(dtype) for _ in range(2))
+    b = torch.randn(d, device=DEV)
+    dx, want, sums = torch.empty_like(x), torch.empty_like(x), torch.ones(d, device=DEV)
+    c = f._c
+    assert f.lib().tsp_gelu_bwd(f._ptr(dy), f._ptr(x), f._ptr(b), f._ptr(want), c.c_int64(x.numel()), c.c_int(d), c.c_int(f._dt(x)),
+                                f._stream()) == 0
+    assert f.lib().tsp_gelu_bwd_sums(f._ptr(dy), f._ptr(x), f._ptr(b), f._ptr(dx), f._ptr(sums), c.c_int64(rows), c.c_int(d),
+                                     c.c_int(f._dt(x)), f._stream()) == 0
+    assert torch.equal(dx, want)
+    # fp32 sums of up to 20000 terms, in groups of some twenty
+    torch.testing.assert_close((sums - 1).double(), dx.double().sum(0), rtol=0, atol=2e-6 * float(dx.double().abs().sum(0).max()))
+
+
 def test_products_on_a_thread_that_has_made_no_runtime_call():
     """Autograd's worker may enter the library with no device context bound: tensor maps have to be made all the same."""
     import threading

@@ -308,11 +308,21 @@ class _LinearGelu(torch.autograd.Function):
         n, k = weight.shape
         dy2 = _bf16_rows(dy, n)
         dh = torch.empty_like(h)
+        sums = db = None
+        if ctx.needs_input_grad[2]:                # the bias gradient: column sums of dh, formed as it is written
+            sums = _f.recorded_grad(ctx.bias)
+            if sums is None:
+                sums = db = torch.zeros(n, dtype=torch.float32, device=h.device)
         with _f.on_device(h.device):
-            _f._check(_f.lib().tsp_gelu_bwd(_f._ptr(dy2), _f._ptr(h), _f._ptr(bf), _f._ptr(dh), _c.c_int64(h.numel()),
-                                            _c.c_int(n), _c.c_int(_f._dt(h)), _f._stream()), "tsp_gelu_bwd")
+            if sums is None:
+                _f._check(_f.lib().tsp_gelu_bwd(_f._ptr(dy2), _f._ptr(h), _f._ptr(bf), _f._ptr(dh), _c.c_int64(h.numel()),
+                                                _c.c_int(n), _c.c_int(_f._dt(h)), _f._stream()), "tsp_gelu_bwd")
+            else:
+                _f._check(_f.lib().tsp_gelu_bwd_sums(_f._ptr(dy2), _f._ptr(h), _f._ptr(bf), _f._ptr(dh), _f._ptr(sums),
+                                                     _c.c_int64(h.shape[0]), _c.c_int(n), _c.c_int(_f._dt(h)), _f._stream()),
+                          "tsp_gelu_bwd_sums")
         _f._count()
-        dx = dw = db = None
+        dx = dw = None
         if ctx.needs_input_grad[0]:
             dx = matmul_nn([dh], _w16(weight)).view(ctx.in_shape)
             if ctx.dtypes[0] != torch.bfloat16:
@@ -325,10 +335,7 @@ class _LinearGelu(torch.autograd.Function):
             _add_weight_grad(target, [dh], x2)
             if dw is not None and weight.dtype != torch.float32:
                 dw = target.to(weight.dtype)
-        if ctx.needs_input_grad[2]:
-            db = _column_sums(dh, add_to=_f.recorded_grad(ctx.bias))
-            db = None if db is None else db.to(ctx.dtypes[2])
-        return dx, dw, db, None
+        return dx, dw, None if db is None else db.to(ctx.dtypes[2]), None
 
 
 def linear_gelu(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
