@@ -31,8 +31,11 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int kThreads = 192;
-constexpr int kStages = 2;
-constexpr uint32_t kSpinLimit = 1u << 22;
+// Tiles of keys in shared memory.  Two are not enough: the load of tile j + 2 starts when the products of tile j are done, which is
+// when its scores are due (contrastive loss of 2 x 4096 rows
+// in two chunks, all launches: 93 us with two, 78 with three).
+constexpr int kStages = 3;
+constexpr uint64_t kWaitNs = 2000000000ull;
 constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -46,25 +49,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-    // The error word lives in global memory, so this check costs a round trip to L2 per failed poll.  That is
-    // deliberate: it is the back-off of the spin loop.  Polling the barrier flat out, or backing off with a short
-    // nanosleep instead, were both measured slower (fused contrastive loss: 481 us with this loop, 607 us polling
-    // flat out, 740 us with __nanosleep(32)).
-    if (*((volatile int*)status) != 0) return false;
-  }
-  atomicCAS(status, 0, code);
-  return false;
+  return tc5::mbar_wait(bar, parity, status, code, kWaitNs);
 }
 // coordinates: (column, row, head, batch)
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z,
@@ -248,23 +233,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const bool issuer = tc5::elect_one();
+      auto arrived = [&](uint64_t* bar, uint32_t parity, int code) -> bool {      // the same for the warp
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code)) != 0;
+      };
       constexpr uint32_t idesc_s = make_idesc(BM, BN, false);
       constexpr uint32_t idesc_o = make_idesc(BM, DV, true);
-      bool ok = mbar_wait(q_full, 0, status, 2);
+      bool ok = arrived(q_full, 0, 2);
       auto issue_s = [&](int j) -> bool {              // S[j & 1] = Q K_j^T
         const int s = j % kStages;
-        if (!mbar_wait(kv_full + s, (j / kStages) & 1, status, 2)) return false;
-        if (j >= 2 && !mbar_wait(s_empty + (j & 1), ((j >> 1) - 1) & 1, status, 4)) return false;
+        if (!arrived(kv_full + s, (j / kStages) & 1, 2)) return false;
+        if (j >= 2 && !arrived(s_empty + (j & 1), ((j >> 1) - 1) & 1, 4)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t q_addr = smem_u32(q_s), k_addr = smem_u32(kv_s + s * (C::kKBytes + C::kVBytes));
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const int kb = kk >> 2, in = kk & 3;
-          umma_bf16(tmem_base + (uint32_t)((j & 1) * BN), desc_k_major(q_addr + kb * (BM * 128)) + (uint64_t)(2 * in),
+          if (issuer) umma_bf16(tmem_base + (uint32_t)((j & 1) * BN), desc_k_major(q_addr + kb * (BM * 128)) + (uint64_t)(2 * in),
                     desc_k_major(k_addr + kb * (BN * 128)) + (uint64_t)(2 * in), idesc_s, kk > 0 ? 1u : 0u);
         }
-        umma_commit(s_full + (j & 1));
+        if (issuer) umma_commit(s_full + (j & 1));
         return true;
       };
       if (ok && n_tiles > 0) ok = issue_s(0);
@@ -273,7 +262,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           ok = issue_s(j + 1);
           if (!ok) break;
         }
-        ok = mbar_wait(p_full + (j & 1), (j >> 1) & 1, status, 5);
+        ok = arrived(p_full + (j & 1), (j >> 1) & 1, 5);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int s = j % kStages;
@@ -282,14 +271,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
         for (int ks = 0; ks < BN / 16; ++ks) {           // 16 keys per MMA
           const int kb = ks >> 2, in = ks & 3;
-          umma_bf16(tmem_base + (uint32_t)C::kOCol, desc_k_major(p_addr + kb * (BM * 128)) + (uint64_t)(2 * in),
+          if (issuer) umma_bf16(tmem_base + (uint32_t)C::kOCol, desc_k_major(p_addr + kb * (BM * 128)) + (uint64_t)(2 * in),
                     desc_mn_major(v_addr + ks * (16 * 128), BN * 128), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         }
-        umma_commit(kv_empty + s);
-        umma_commit(p_empty + (j & 1));
-        umma_commit(o_done);
+        if (issuer) umma_commit(kv_empty + s);
+        if (issuer) umma_commit(p_empty + (j & 1));
+        if (issuer) umma_commit(o_done);
       }
-      if (ok) umma_commit(o_final);
+      if (ok && issuer) umma_commit(o_final);
     }
   } else {
     // ---------------- softmax + epilogue: thread = query row ----------------
@@ -480,7 +469,7 @@ int launch(const void* q, void* const* k_srcs, int n_src, const void* v, void* o
 // The passes around the fused contrastive loss of two (queries, keys) pairs.  One warp per row of 256 elements, 8 per
 // lane; blockIdx.y = pair.
 // ---------------------------------------------------------------------------------------------
-constexpr int kNceDim = 256, kNceRows = 16;       // rows (warps) of a block of the last pass
+constexpr int kNceDim = 256, kNceRows = 32;       // rows (warps) of a block of the last pass
 template <typename T>
 struct NcePairs {
   const T* q[2];
@@ -498,7 +487,8 @@ __device__ __forceinline__ float row_norm(const float (&v)[8]) {
 template <typename T>
 __global__ void __launch_bounds__(256) nce_prepare_kernel(const NcePairs<T> in, int n, int n_pad,
                                                           __nv_bfloat16* __restrict__ q16,
-                                                          __nv_bfloat16* __restrict__ k16) {
+                                                          __nv_bfloat16* __restrict__ k16, double* __restrict__ sum) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sum[0] = sum[1] = 0.;      // for nce_finish_kernel
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 8 + warp;                   // rows 0 .. n - 1: queries, then n_pad key rows
   if (row >= n + n_pad) return;
@@ -523,7 +513,9 @@ __global__ void __launch_bounds__(256) nce_prepare_kernel(const NcePairs<T> in, 
 // lse and o come from rows q~, k~ rounded to bf16.  What the rounding of the row's own query and key does to lse is added to
 // first order, ((q^ - q~).o + p (k^ - k~).q~) / T with p the probability of the row's own key; q^.k^ and the gradient's k^ are
 // taken as they are.  Error of the loss and of the gradient against 64 bits, 256 rows: 6e-6 and 2.8e-3 with rounded rows
-// throughout (and as much with the logits in memory), 3e-7 and 1.7e-3 this way, in the same time.
+// throughout (and as much with the logits in memory), 3e-7 and 1.7e-3 this way, in the same time.  At most a block per SM and pair:
+// every block ends in two additions to the same memory, one after the other at some 15 ns (2 x 4096 rows in two
+// chunks: 20.8 us with 512 blocks, 14.9 this way).
 template <typename T>
 __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
                                                          const __nv_bfloat16* __restrict__ q16,
@@ -531,11 +523,10 @@ __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePair
                                                          const float* __restrict__ o, const float* __restrict__ lse,
                                                          double* __restrict__ sum, float* __restrict__ loss,
                                                          T* __restrict__ gq) {
-  __shared__ float part[kNceRows];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = lane * 8;
-  const int row = blockIdx.x * kNceRows + warp, pair = blockIdx.y;
-  float contrib = 0.f;
-  if (row < n) {
+  __shared__ double part[kNceRows];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = lane * 8, pair = blockIdx.y;
+  double mine = 0.;
+  for (int row = blockIdx.x * kNceRows + warp; row < n; row += gridDim.x * kNceRows) {
     float q[8], k[8], qb[8], kb[8], acc[8] = {};
     tsp::ld8(pair ? in.q[1] : in.q[0], (int64_t)row * kNceDim + col, q);
     tsp::ld8(pair ? in.k[1] : in.k[0], (int64_t)row * kNceDim + col, k);
@@ -568,13 +559,13 @@ __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePair
     }
     own = tsp::warp_sum(own); dk = tsp::warp_sum(dk); rest = tsp::warp_sum(rest);
     const float lse_row = m + logf(z);
-    contrib = (lse_row + (rest + expf(own / temp - lse_row) * dk) / temp) * (2.f * temp / n);
+    mine += (lse_row + (rest + expf(own / temp - lse_row) * dk) / temp) * (2.f * temp / n);
     dot = norm > 1e-12f ? tsp::warp_sum(dot) : 0.f;       // a clamped norm is a constant
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = (acc[e] - q[e] * dot) / norm;
     tsp::st8(gq, ((int64_t)pair * n + row) * kNceDim + col, acc);
   }
-  if (lane == 0) part[warp] = contrib;
+  if (lane == 0) part[warp] = mine;
   __syncthreads();
   if (threadIdx.x == 0) {
     double s = 0.;
@@ -592,10 +583,8 @@ int launch_nce_pair(const NcePairs<T>& in, int n, int chunk, int chunks, float t
                     float* lse, float* loss, void* gq, int* status, cudaStream_t stream) {
   const int n_pad = chunk * chunks;
   double* sum = reinterpret_cast<double*>(lse + (int64_t)2 * chunks * n);       // and behind it the blocks that are done
-  cudaError_t e = cudaMemsetAsync(sum, 0, 2 * sizeof(double), stream);
-  if (e != cudaSuccess) return (int)e;
   nce_prepare_kernel<T><<<dim3((n + n_pad + 7) / 8, 2), 256, 0, stream>>>(in, n, n_pad, (__nv_bfloat16*)q16,
-                                                                          (__nv_bfloat16*)k16);
+                                                                          (__nv_bfloat16*)k16, sum);
   const Strides sq = {kNceDim, (int64_t)n * kNceDim, (int64_t)n * kNceDim};
   const Strides sk = {kNceDim, (int64_t)chunk * kNceDim, (int64_t)n_pad * kNceDim};
   const Strides so = {kNceDim, (int64_t)n * kNceDim, (int64_t)chunks * n * kNceDim};
@@ -603,7 +592,8 @@ int launch_nce_pair(const NcePairs<T>& in, int n, int chunk, int chunks, float t
   const int rc = launch<256, 256, 64, true, float>(q16, srcs, 1, k16, o, lse, 2, chunks, n, chunk, sq, sk, sk, so,
                                                    1.f / temp, 1.f / temp, 1, status, stream, n);
   if (rc != 0) return rc;
-  nce_finish_kernel<T><<<dim3((n + kNceRows - 1) / kNceRows, 2), 32 * kNceRows, 0, stream>>>(
+  const int blocks = (n + kNceRows - 1) / kNceRows;
+  nce_finish_kernel<T><<<dim3(blocks < 74 ? blocks : 74, 2), 32 * kNceRows, 0, stream>>>(
       in, n, n_pad, chunks, temp, (const __nv_bfloat16*)q16, (const __nv_bfloat16*)k16, o, lse, sum, loss, (T*)gq);
   return TSP_LAUNCH_CHECK();
 }
