@@ -167,6 +167,46 @@ def test_igemm_convolution_forward_backward_and_statistics(shape, cout, k, strid
     torch.testing.assert_close(m.weight.grad, 2 * wr.grad, rtol=5e-2, atol=1e-1 * wr.grad.abs().max().item())
 
 
+# (images, height, width, cin, cout, kernel): the pixel tiles around the numbers where the channel tile changes its width (74
+# tiles of 256 channels run at once in halves on 148 SMs, 37 in quarters), and grids of several tiles per block
+TILE_CASES = [(37, 16, 16, 256, 256, 1), (75, 16, 8, 256, 256, 1), (37, 16, 8, 256, 256, 1), (19, 16, 16, 256, 256, 3),
+              (37, 16, 16, 256, 256, 3), (38, 16, 16, 256, 256, 3), (74, 7, 7, 128, 256, 3), (148, 7, 7, 128, 256, 3),
+              (150, 7, 7, 128, 256, 3), (16, 56, 56, 64, 256, 1), (16, 56, 56, 64, 128, 1), (16, 56, 56, 128, 64, 1),
+              (16, 56, 56, 512, 128, 1), (8, 56, 56, 128, 128, 3), (64, 14, 14, 448, 512, 1)]
+
+
+@pytest.mark.parametrize("n,h,w,cin,cout,k", TILE_CASES)
+def test_convolution_channel_tiles_and_epilogue_warps(n, h, w, cin, cout, k):
+    """Output, statistics of one and of several image groups, and the data gradient: fp32 sums, rounded once to bf16."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(31)
+    dev = torch.device("cuda", 0)
+    x = torch.randn(n, cin, h, w, device=dev).to(dtype=torch.bfloat16, memory_format=torch.channels_last).requires_grad_()
+    weight = (torch.randn(cout, cin, k, k, device=dev) / (k * cin ** 0.5)).to(memory_format=torch.channels_last).requires_grad_()
+    conv.clear_weight_cache()
+    wr = weight.detach().bfloat16().double()
+    want = F.conv2d(x.detach().double(), wr, padding=(k - 1) // 2)
+    size = F.conv2d(x.detach().double().abs(), wr.abs(), padding=(k - 1) // 2)
+    for segs in (1, 2 if n % 4 == 0 else 1):
+        y, sums = conv.conv2d(x, weight, 1, want_sums=True, segments=segs)
+        gemm.check_status()
+        # a product rounds once to 8 bits; its fp32 sum over k * k * cin terms errs by 2^-22 of the terms' sizes at most
+        assert ((y.double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -20).all()
+        if sums is None:
+            assert k == 1 and (n // segs * h * w) % 128
+            continue
+        for s, part in zip(sums.view(segs, 2, cout).double(), y.detach().double().chunk(segs)):
+            for got, terms in zip(s, (part, part * part)):
+                bound = 2.0 ** -16 * terms.abs().sum((0, 2, 3))       # fp32 sums of some hundred terms each, added up
+                assert ((got - terms.sum((0, 2, 3))).abs() <= bound).all()
+    g = torch.randn(y.shape, device=dev).to(dtype=torch.bfloat16, memory_format=torch.channels_last)
+    (dx,) = torch.autograd.grad(y, x, g)
+    gemm.check_status()
+    want = torch.nn.grad.conv2d_input(x.shape, wr, g.double(), padding=(k - 1) // 2)
+    size = torch.nn.grad.conv2d_input(x.shape, wr.abs(), g.double().abs(), padding=(k - 1) // 2)
+    assert ((dx.double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -20).all()
+
+
 def test_bottleneck_on_igemm_convolutions_matches_library_path():
     from tspipe_b200.batchnorm import DeferredBatchNorm
     from tspipe_b200.models.resnet import Bottleneck
