@@ -51,7 +51,7 @@ namespace {
 
 using namespace tc5;
 
-constexpr int kThreads = 320;           // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two per TMEM lane quarter)
+constexpr int kThreads = 320;           // halo kernel: warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two per TMEM lane quarter)
 constexpr int kWgThreads = 192;         // weight gradient: warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
 constexpr int kBoxBytes = 128 * 128;        // shared memory reserved per pixel box: 128 rows x 64 bf16
 constexpr int kMaxTaps = 9;
@@ -83,17 +83,20 @@ struct ActMaps {
 
 // ADD: 0 no addend, 1 read by the epilogue's threads, 2 fetched by TMA (flat pixel grid): see add_epilogue
 constexpr int kAddBufs = 4;
-template <int BN, int ADD>
+// GROUPS: epilogue warps per TMEM lane quarter
+template <int BN, int ADD, int GROUPS>
 struct FwdCfg {
   static constexpr int kABytes = kBoxBytes;
   static constexpr int kBBytes = BN * 128;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = ADD == 2 ? (BN == 64 ? 4 : 2) : BN == 256 ? 4 : 6;
-  static constexpr int kGroup = 2;                          // stages released per tcgen05.commit (a commit costs the
-  static constexpr int kGroups = kStages / kGroup;          // issuing thread about as much as eight MMAs)
-  static constexpr int kTmemCols = 2 * BN;
+  static constexpr int kThreads = 64 + 128 * GROUPS;
+  static constexpr int kStages = ADD == 2 ? (BN == 64 ? 4 : 2) : BN == 256 ? (GROUPS == 2 ? 4 : 3) : (BN == 128 && GROUPS == 4 ? 5 : 6);
+  static constexpr int kGroup = GROUPS == 2 ? 2 : 1;        // stages released per tcgen05.commit (1024 -> 256 channels at 14 x 14,
+  static constexpr int kGroups = kStages / kGroup;          // 64 images, B200: 13.4 us in twos, 14.5 one by one)
+  static constexpr int kAccBufs = GROUPS == 2 || BN == 256 ? 2 : 4;
+  static constexpr int kTmemCols = kAccBufs * BN;
   // 32-row x 128-byte staging blocks per epilogue warp
-  static constexpr int kStoreBytes = 8 * (ADD == 2 ? kAddBufs : 1) * 32 * 128;
+  static constexpr int kStoreBytes = 4 * GROUPS * (ADD == 2 ? kAddBufs : 1) * 32 * 128;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256 + (ADD == 2 ? 8 * 8 * kAddBufs : 0);
 };
 
@@ -119,15 +122,16 @@ __device__ __forceinline__ void tile_origin(const Geom& g, int tm, int& w0, int&
   n0 = (r / g.tiles_h) * g.box_n;
 }
 
-// Epilogue warps (2..9) of the forward / data-gradient kernels.  A tile has `n_sub` accumulators of 128 rows (SUBS
+// Epilogue warps (from 2 on) of the forward / data-gradient kernels.  A tile has `n_sub` accumulators of 128 rows (SUBS
 // reserved per TMEM buffer); accumulator row p of the tile (p = 128 * sub + TMEM lane) is pixel
 // (p % row_pitch, (p / row_pitch) % box_h, p / (row_pitch * box_h)) of the tile's box; rows in border columns, past
-// the box or outside the image are not stored.  Warp w owns TMEM lanes 32 * (w % 4) .. + 31; the two warps that share
-// a lane quarter split the (accumulator, 64-channel block) units between them.  Per unit: TMEM -> registers -> bf16
+// the box or outside the image are not stored.  Warp w owns TMEM lanes 32 * (w % 4) .. + 31; the GROUPS warps that
+// share a lane quarter split the tile's 64-channel blocks between them, and where there are fewer blocks than warps, a
+// block's accumulators in turn.  Per unit: TMEM -> registers -> bf16
 // -> swizzled shared memory (rows that are not stored are written as zeros) -> per-channel sums from shared memory
 // (STATS) and coalesced 16-byte stores, 8 lanes per pixel.
 // ADD: `addend` has the output's layout and is added to the rounded result, as the sum of two bf16 gradients would be.
-template <int BN, int SUBS, int ACC_BUFS, bool STATS, bool ADD>
+template <int BN, int SUBS, int ACC_BUFS, int GROUPS, bool STATS, bool ADD>
 __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int tiles_m, int n_sub, uint32_t tmem_base,
                                              uint64_t* tmem_full_bar, uint64_t* tmem_empty_bar, uint8_t* store_bufs,
                                              __nv_bfloat16* __restrict__ out,
@@ -139,19 +143,22 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
   uint8_t* buf = store_bufs + (warp - 2) * (32 * 128);
   uint32_t lt = 0;
   bool ok = true;
-  constexpr int kStatBlocks = BN / 64;
-  ColSums cs[(kStatBlocks + 1) / 2];                      // of this warp's 64-channel blocks
+  constexpr int kBlocks = BN / 64;
+  constexpr int kMine = kBlocks > GROUPS ? kBlocks / GROUPS : 1;        // this warp's 64-channel blocks of a tile
+  constexpr int kShare = kBlocks < GROUPS ? GROUPS / kBlocks : 1;       // warps of a lane quarter that share a block
+  auto block = [&](int j) -> int { return kShare > 1 ? group % kBlocks : j * GROUPS + group; };
+  ColSums cs[kMine];
 #pragma unroll
-  for (int j = 0; j < (kStatBlocks + 1) / 2; ++j) cs[j].clear();
+  for (int j = 0; j < kMine; ++j) cs[j].clear();
   int cur_c0 = -1, cur_seg = 0;
   auto flush_stats = [&]() {
     if (cur_c0 >= 0) {
       float* dst = col_sums + (int64_t)cur_seg * 2 * g.nc;
 #pragma unroll
-      for (int j = 0; j < (kStatBlocks + 1) / 2; ++j) {
+      for (int j = 0; j < kMine; ++j) {
         float s[2], q[2];
         cs[j].reduce(lane, s, q);
-        const int col = cur_c0 + 64 * (kStatBlocks == 1 ? 0 : 2 * j + group) + ColSums::channel(lane);
+        const int col = cur_c0 + 64 * block(j) + ColSums::channel(lane);
         // (nc is a multiple of 64: col and col + 1 exist together)
         if (col < g.nc && (q[0] != 0.f || q[1] != 0.f)) {
           atomicAdd(dst + col, s[0]); atomicAdd(dst + g.nc + col, q[0]);
@@ -181,11 +188,11 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
                  ? n * g.out_sn + h * g.out_sh + w * g.out_sw : -1;
     };
     const int pc = lane & 7;
-    constexpr int kUnits = SUBS * kStatBlocks;            // (accumulator, 64-channel block) units, dealt to the two groups
+    auto takes = [&](int sub) -> bool { return kShare == 1 || (int)((lt * n_sub + sub) % kShare) == group / kBlocks; };
     constexpr bool kEarly = ADD && SUBS == 1;
     // ADD: the addend in the layout of the stores below.  One accumulator: the whole tile's is requested before the
     // accumulator is waited for, so that its way from memory overlaps the products.
-    uint4 add[ADD ? (kEarly ? (kUnits + 1) / 2 : 1) : 1][ADD ? 8 : 1];
+    uint4 add[ADD && kEarly ? kMine : 1][ADD ? 8 : 1];
     auto load_add = [&](uint4 (&dst)[ADD ? 8 : 1], int row_off, int col) {
       if constexpr (ADD) {
 #pragma unroll
@@ -199,45 +206,47 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
     if constexpr (kEarly) {
       const int row_off = pixel_off(0);
 #pragma unroll
-      for (int j = 0; j < (kUnits + 1) / 2; ++j) {
-        const int i = kUnits == 1 ? 0 : 2 * j + group;
-        if ((kUnits > 1 || group == 0) && c0 + 64 * i < g.nc) load_add(add[j], row_off, c0 + 64 * i);
-      }
+      for (int j = 0; j < kMine; ++j)
+        if (takes(0) && c0 + 64 * block(j) < g.nc) load_add(add[j], row_off, c0 + 64 * block(j));
     }
     ok = mbar_wait_warp(tmem_full_bar + acc, use & 1, status, 3, g.wait_ns, lane);
     if (!ok) break;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
     for (int sub = 0; sub < SUBS; ++sub) {
-      if (sub < n_sub) {
+      if (sub < n_sub && takes(sub)) {
         const int row_off = pixel_off(sub);
 #pragma unroll
-        for (int i = 0; i < kStatBlocks; ++i) {
-          const int col = c0 + 64 * i;
-          const bool mine = kUnits == 1 ? group == 0 : ((sub * kStatBlocks + i) & 1) == group;
-          if (mine && col < g.nc) {
+        for (int b = 0; b < kMine; ++b) {
+          const int col = c0 + 64 * block(b);
+          if (col < g.nc) {
             if constexpr (ADD && !kEarly) load_add(add[0], row_off, col);
-            uint32_t r[64];
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (acc * SUBS + sub) * BN + (uint32_t)(64 * i);
-            tmem_ld_32x32_issue(taddr, r);
-            tmem_ld_32x32_issue(taddr + 32, r + 32);
-            tmem_ld_wait();
+            // (four warps per quarter have half the registers each, and each other to fill the waits)
+            constexpr int kPart = GROUPS > 2 ? 32 : 64;
+            uint32_t r[kPart];
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (acc * SUBS + sub) * BN + (uint32_t)(64 * block(b));
             uint8_t* my_row = buf + lane * 128;
             const bool keep = row_off >= 0;
-            if (tma_out) {             // the previous block's store has finished reading the staging buffer
-              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-              __syncwarp();
-            }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {         // 16-byte piece j of this row sits at piece (j ^ (row & 7))
-              uint4 q = make_uint4(0u, 0u, 0u, 0u);
-              if (keep) {
-                q.x = pack_bf16x2(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1]));
-                q.y = pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
-                q.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
-                q.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
+            for (int at = 0; at < 64; at += kPart) {
+              tmem_ld_32x32_issue(taddr + at, r);
+              if constexpr (kPart == 64) tmem_ld_32x32_issue(taddr + 32, r + 32);
+              tmem_ld_wait();
+              if (tma_out && at == 0) {             // the previous block's store has finished reading the staging buffer
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                __syncwarp();
               }
-              *reinterpret_cast<uint4*>(my_row + ((j ^ (lane & 7)) << 4)) = q;
+#pragma unroll
+              for (int j = 0; j < kPart / 8; ++j) {         // 16-byte piece j of this row sits at piece (j ^ (row & 7))
+                uint4 q = make_uint4(0u, 0u, 0u, 0u);
+                if (keep) {
+                  q.x = pack_bf16x2(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1]));
+                  q.y = pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
+                  q.z = pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
+                  q.w = pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
+                }
+                *reinterpret_cast<uint4*>(my_row + (((at / 8 + j) ^ (lane & 7)) << 4)) = q;
+              }
             }
             __syncwarp();
             if (tma_out) {
@@ -253,7 +262,7 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
                 uint4 q = *reinterpret_cast<const uint4*>(buf + rr * 128 + ((pc ^ (rr & 7)) << 4));
                 if constexpr (ADD) {
                   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
-                  const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&add[kEarly ? i / 2 : 0][k]);
+                  const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&add[kEarly ? b : 0][k]);
 #pragma unroll
                   for (int e = 0; e < 4; ++e) h[e] = __hadd2(h[e], a[e]);
                 }
@@ -262,7 +271,7 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
               __syncwarp();
             }
             // (the block's stores are on their way: the sums overlap them)
-            if (STATS) cs[i / 2].add(buf, lane);         // of the rounded block (rows that are not stored hold zeros)
+            if (STATS) cs[b].add(buf, lane);         // of the rounded block (rows that are not stored hold zeros)
           }
         }
       }
@@ -279,7 +288,7 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
     // the last sums go through the staging buffer: the CTA adds its warps' up before they leave (flush_cta_stats)
     float* st = reinterpret_cast<float*>(buf);
 #pragma unroll
-    for (int j = 0; j < (kStatBlocks + 1) / 2; ++j) {
+    for (int j = 0; j < kMine; ++j) {
       float s[2], q[2];
       cs[j].reduce(lane, s, q);
       *reinterpret_cast<float2*>(st + j * 128 + ColSums::channel(lane)) = make_float2(s[0], s[1]);
@@ -294,24 +303,24 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
 // its own, two instructions a sector, the 148 CTAs of a convolution with 64 to 256 output channels queued for up to
 // 30 us at their end.  The convolutions of a ResNet-50
 // forward over 64 images, B200: 1354 us then, 1210 now.
-template <int BN>
+template <int BN, int GROUPS>
 __device__ __forceinline__ void flush_cta_stats(const Geom& g, const uint8_t* store_bufs, float* __restrict__ col_sums) {
-  constexpr int kStatBlocks = BN / 64;
+  constexpr int kBlocks = BN / 64, kShare = kBlocks < GROUPS ? GROUPS / kBlocks : 1;        // as in fwd_epilogue
   auto part = [&](int w) { return reinterpret_cast<const float*>(store_bufs + w * (32 * 128)); };
   const int c0 = __float_as_int(part(0)[512]), seg = __float_as_int(part(0)[513]);
-  for (int w = 1; w < 8; ++w)                     // all warps walk the same tiles; after a wait that ran out nothing is added
+  for (int w = 1; w < 4 * GROUPS; ++w)            // all warps walk the same tiles; after a wait that ran out nothing is added
     if (__float_as_int(part(w)[512]) != c0) return;
   if (c0 < 0) return;
   float* dst = col_sums + (int64_t)seg * 2 * g.nc;
-  for (int p = threadIdx.x; p < 2 * BN; p += kThreads) {
-    const int half = p / BN, col = p % BN, i = col >> 6, at = (i >> 1) * 128 + half * 64 + (col & 63);
+  for (int p = threadIdx.x; p < 2 * BN; p += 64 + 128 * GROUPS) {
+    const int half = p / BN, col = p % BN, i = col >> 6;
+    const int group = kShare > 1 ? i : i % GROUPS, at = (kShare > 1 ? 0 : i / GROUPS) * 128 + half * 64 + (col & 63);
     if (c0 + col >= g.nc) continue;
     float v = 0.f;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (kStatBlocks == 1) v += part(q)[at] + part(4 + q)[at];      // both groups have seen this block
-      else v += part((i & 1) * 4 + q)[at];
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int k = 0; k < kShare; ++k) v += part((group + k * kBlocks) * 4 + q)[at];
     atomicAdd(dst + half * g.nc + c0 + col, v);
   }
 }
@@ -401,23 +410,23 @@ __device__ __forceinline__ void add_epilogue(const Geom& g, int num_tiles, int t
 // ---------------------------------------------------------------------------------------------------------------
 // forward / data gradient
 // ---------------------------------------------------------------------------------------------------------------
-template <int BN, bool B_MN, bool STATS, int ADD>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int BN, bool B_MN, bool STATS, int ADD, int GROUPS>
+__global__ void __launch_bounds__(FwdCfg<BN, ADD, GROUPS>::kThreads, 1)
 conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ CUtensorMap wmap,
                 const __grid_constant__ CUtensorMap omap, const __grid_constant__ CUtensorMap addmap,
                 const __grid_constant__ Geom g, __nv_bfloat16* __restrict__ out,
                 const __nv_bfloat16* __restrict__ addend, float* __restrict__ col_sums, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
-  using C = FwdCfg<BN, ADD>;
+  using C = FwdCfg<BN, ADD, GROUPS>;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* store_bufs = tiles + C::kStages * C::kStageBytes;
   uint64_t* bars = (uint64_t*)(store_bufs + C::kStoreBytes);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + C::kStages;
   uint64_t* tmem_full_bar = bars + 2 * C::kStages;
-  uint64_t* tmem_empty_bar = bars + 2 * C::kStages + 2;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * C::kStages + 4);
-  uint64_t* add_bars = bars + 2 * C::kStages + 5;             // [8 warps][kAddBufs]  addend -> epilogue (ADD == 2)
+  uint64_t* tmem_empty_bar = tmem_full_bar + C::kAccBufs;
+  uint32_t* tmem_slot = (uint32_t*)(tmem_empty_bar + C::kAccBufs);
+  uint64_t* add_bars = tmem_empty_bar + C::kAccBufs + 1;             // [8 warps][kAddBufs]  addend -> epilogue (ADD == 2)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = g.tiles_w * g.tiles_h * g.tiles_n, tiles_nn = (g.nc + BN - 1) / BN;
@@ -430,9 +439,9 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       mbar_init(full_bar + s, 1);
       mbar_init(empty_bar + s, 1);
     }
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < C::kAccBufs; ++a) {
       mbar_init(tmem_full_bar + a, 1);
-      mbar_init(tmem_empty_bar + a, 8);
+      mbar_init(tmem_empty_bar + a, 4 * GROUPS);
     }
     if (ADD == 2)
       for (int i = 0; i < 8 * kAddBufs; ++i) mbar_init(add_bars + i, 1);
@@ -498,7 +507,7 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       uint32_t it = 0, lt = 0;
       bool ok = true;
       for (int t = tile_begin(num_tiles, blockIdx.x); t < tile_begin(num_tiles, blockIdx.x + 1) && ok; ++t, ++lt) {
-        const uint32_t acc = lt & 1, use = lt >> 1;
+        const uint32_t acc = lt % C::kAccBufs, use = lt / C::kAccBufs;
         if (use > 0) {
           ok = arrived(tmem_empty_bar + acc, (use - 1) & 1, 4);
           if (!ok) break;
@@ -530,12 +539,13 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       add_epilogue<BN>(g, num_tiles, tiles_m, tmem_base, tmem_full_bar, tmem_empty_bar, store_bufs, add_bars, &omap, &addmap,
                        status, warp, lane);
     else
-      fwd_epilogue<BN, 1, 2, STATS, ADD == 1>(g, num_tiles, tiles_m, 1, tmem_base, tmem_full_bar, tmem_empty_bar, store_bufs,
-                                              out, addend, col_sums, status, warp, lane, &omap);
+      fwd_epilogue<BN, 1, C::kAccBufs, GROUPS, STATS, ADD == 1>(g, num_tiles, tiles_m, 1, tmem_base, tmem_full_bar,
+                                                                       tmem_empty_bar, store_bufs, out, addend, col_sums, status, warp,
+                                                                       lane, &omap);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (STATS) flush_cta_stats<BN>(g, store_bufs, col_sums);
+  if (STATS) flush_cta_stats<BN, GROUPS>(g, store_bufs, col_sums);
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)C::kTmemCols)
                  : "memory");
@@ -742,12 +752,12 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
       }
     }
   } else {
-    fwd_epilogue<BN, 2, C::kAccBufs, STATS, ADD>(g, num_tiles, tiles_m, n_sub, tmem_base, tmem_full_bar, tmem_empty_bar,
+    fwd_epilogue<BN, 2, C::kAccBufs, 2, STATS, ADD>(g, num_tiles, tiles_m, n_sub, tmem_base, tmem_full_bar, tmem_empty_bar,
                                                  store_bufs, out, addend, col_sums, status, warp, lane);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (STATS) flush_cta_stats<BN>(g, store_bufs, col_sums);
+  if (STATS) flush_cta_stats<BN, 2>(g, store_bufs, col_sums);
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)C::kTmemCols)
                  : "memory");
@@ -1244,23 +1254,24 @@ Plan plan_input(const void* x, int n, int h, int w, int cin, int k, int s, int m
   return p;
 }
 
-template <int BN, bool B_MN, bool STATS, int ADD>
+template <int BN, bool B_MN, bool STATS, int ADD, int GROUPS = 2>
 int launch_fwd_kernel(const Plan& p, const CUtensorMap& wmap, const CUtensorMap& omap, const CUtensorMap& addmap, const Geom& g,
                       void* out, const void* addend, float* col_sums, int* status, cudaStream_t stream) {
-  auto kern = conv_fwd_kernel<BN, B_MN, STATS, ADD>;
+  auto kern = conv_fwd_kernel<BN, B_MN, STATS, ADD, GROUPS>;
+  using C = FwdCfg<BN, ADD, GROUPS>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   dev &= 63;
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<BN, ADD>::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
   const int num_tiles = g.tiles_w * g.tiles_h * g.tiles_n * ((g.nc + BN - 1) / BN);
   const int n_sm = sm_count();
   const int grid = num_tiles < n_sm ? num_tiles : n_sm;
-  kern<<<grid, kThreads, FwdCfg<BN, ADD>::kSmemBytes, stream>>>(p.maps, wmap, omap, addmap, g, (__nv_bfloat16*)out,
+  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(p.maps, wmap, omap, addmap, g, (__nv_bfloat16*)out,
                                                                 (const __nv_bfloat16*)addend, col_sums, status);
   return TSP_LAUNCH_CHECK();
 }
@@ -1282,6 +1293,13 @@ int launch_fwd(const Plan& p, const CUtensorMap& wmap, void* out, const void* ad
       if (g.tma_store != 0 && make_bf16_map(&addmap, addend, 2, dims, strides, box))
         return launch_fwd_kernel<BN, B_MN, STATS, 2>(p, wmap, omap, addmap, g, out, addend, col_sums, status, stream);
     }
+  }
+  // Statistics after a short contraction: the epilogue is what a tile waits for, and it has too few warps to fill their waits.
+  // B200, 8 warps against 16 (and one operand stage less): 256 images of 56 x 56, 64 -> 256 110 us and 101, 64 images of
+  // 28 x 28, 128 -> 512 21.2 and 20.0, of 14 x 14, 256 -> 1024 16.4 and 15.3; 512 -> 128 at 28 x 28 16.0 and 17.1.
+  if constexpr (STATS) {
+    if (g.n_taps * g.kc < 512)
+      return launch_fwd_kernel<BN, B_MN, STATS, ADD ? 1 : 0, 4>(p, wmap, omap, addmap, g, out, addend, col_sums, status, stream);
   }
   return launch_fwd_kernel<BN, B_MN, STATS, ADD ? 1 : 0>(p, wmap, omap, addmap, g, out, addend, col_sums, status, stream);
 }
