@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(kBlock, 2) bn_colsum_kernel(const T* __restric
                                                            const float* __restrict__ mean_rstd,
                                                            const float* __restrict__ w, const float* __restrict__ bias,
                                                            int relu, int64_t m, int c, float* __restrict__ out) {
+  tsp::let_next_start();
   __shared__ float sm[(kBlock + 4) * 16];
   {   // blockIdx.z = segment: an independent group of m rows with its own statistics
     const int64_t so = (int64_t)blockIdx.z * m * c;
@@ -217,6 +218,7 @@ bn_colsum_stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
                         const float* __restrict__ bias, int relu, int64_t m, int c, int chunk,
                         float* __restrict__ out) {
   extern __shared__ __align__(128) uint8_t stream_smem[];
+  tsp::let_next_start();
   {   // blockIdx.y = segment: an independent group of m rows with its own statistics
     const int64_t so = (int64_t)blockIdx.y * m * c;
     x += so;
@@ -394,6 +396,7 @@ __global__ void __launch_bounds__(kBlock, 3) bn_apply_kernel(const T* __restrict
                                                           float* __restrict__ acc_sum, float* __restrict__ acc_sumsq,
                                                           float* __restrict__ acc_count, int64_t acc_seg_stride,
                                                           int64_t m, int c, float eps, int relu) {
+  tsp::let_next_start();
   {   // blockIdx.y = segment: m rows with their own statistics (and their own set of accumulators)
     const int64_t so = (int64_t)blockIdx.y * m * c;
     x += so;
@@ -498,6 +501,7 @@ __global__ void __launch_bounds__(kBlock, 3) bn_bwd_apply_kernel(const T* __rest
                                                               const float* __restrict__ sums, T* __restrict__ dx,
                                                               float* __restrict__ gw, float* __restrict__ gb,
                                                               int64_t m, int c) {
+  tsp::let_next_start();
   {   // blockIdx.y = segment
     const int64_t so = (int64_t)blockIdx.y * m * c;
     dy += so;
@@ -692,6 +696,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 2 ? 3 : 2) bn_relu_pool_k
                                                               float* __restrict__ acc_sum, float* __restrict__ acc_sumsq,
                                                               float* __restrict__ acc_count, int64_t acc_seg_stride,
                                                               const PoolGeom g, float eps) {
+  tsp::let_next_start();
   using P = PoolKey<T>;
   using K = typename P::K;
   {   // blockIdx.y = segment
@@ -807,6 +812,7 @@ __global__ void __launch_bounds__(kBlock, 2) bn_relu_pool_bwd_kernel(const T* __
                                                                   float* __restrict__ sums, T* __restrict__ dx,
                                                                   float* __restrict__ gw, float* __restrict__ gb,
                                                                   const PoolGeom g) {
+  tsp::let_next_start();
   constexpr int sm_pitch = kBlock + 8;
   __shared__ float sm[APPLY ? 1 : 16 * sm_pitch];
   const int c = g.c;

@@ -459,6 +459,8 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  tsp::wait_for_previous();
+  addend = tsp::written(addend);
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -494,6 +496,7 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
           }
         }
       }
+      tsp::let_next_start();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -634,6 +637,8 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  tsp::wait_for_previous();
+  addend = tsp::written(addend);
   const int t_first = tile_begin(num_tiles, blockIdx.x), my_tiles = tile_begin(num_tiles, blockIdx.x + 1) - t_first;
 
   if (warp == 0) {
@@ -680,6 +685,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
           }
         }
       }
+      tsp::let_next_start();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -834,6 +840,7 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  tsp::wait_for_previous();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -868,6 +875,7 @@ conv_wgrad_kernel(const __grid_constant__ ActMaps xmaps, const __grid_constant__
             tma_load_4d(b_dst + j * C::kBox, &dymap, full_bar + s, nt * BN + j * 64, w0, h0, n0);
         }
       }
+      tsp::let_next_start();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -1043,6 +1051,8 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  tsp::wait_for_previous();
+  x = tsp::written(x); dy = tsp::written(dy);
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -1059,6 +1069,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
         tma_load_4d(dst, &xmap, full_bar + s, 0, w0 - 1, h0 - 1, n0);
         tma_load_4d(dst + C::kXBytes, &dymap, full_bar + s, 0, w0, h0, n0);
       }
+      tsp::let_next_start();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -1271,8 +1282,8 @@ int launch_fwd_kernel(const Plan& p, const CUtensorMap& wmap, const CUtensorMap&
   const int num_tiles = g.tiles_w * g.tiles_h * g.tiles_n * ((g.nc + BN - 1) / BN);
   const int n_sm = sm_count();
   const int grid = num_tiles < n_sm ? num_tiles : n_sm;
-  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(p.maps, wmap, omap, addmap, g, (__nv_bfloat16*)out,
-                                                                (const __nv_bfloat16*)addend, col_sums, status);
+  tsp::launch_early(kern, grid, C::kThreads, C::kSmemBytes, stream, p.maps, wmap, omap, addmap, g, (__nv_bfloat16*)out,
+                    (const __nv_bfloat16*)addend, col_sums, status);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -1358,8 +1369,8 @@ int launch_halo(Geom& g, const CUtensorMap& amap, const CUtensorMap& wmap, void*
   const int num_tiles = g.tiles_w * g.tiles_h * g.tiles_n * ((g.nc + BN - 1) / BN);
   const int n_sm = sm_count();
   const int grid = num_tiles < n_sm ? num_tiles : n_sm;
-  kern<<<grid, kThreads, HaloCfg<BN>::kSmemBytes, stream>>>(amap, wmap, g, (__nv_bfloat16*)out, (const __nv_bfloat16*)addend,
-                                                       col_sums, status);
+  tsp::launch_early(kern, grid, kThreads, HaloCfg<BN>::kSmemBytes, stream, amap, wmap, g, (__nv_bfloat16*)out,
+                    (const __nv_bfloat16*)addend, col_sums, status);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -1400,7 +1411,7 @@ int launch_wgrad(const Plan& p, const CUtensorMap& dymap, float* dw, int* status
   const int items = m_tiles * n_tiles * g.splits;
   const int n_sm = sm_count();
   const int grid = items < n_sm ? items : n_sm;
-  kern<<<grid, kWgThreads, WgCfg<BN>::kSmemBytes, stream>>>(p.maps, dymap, g, dw, status);
+  tsp::launch_early(kern, grid, kWgThreads, WgCfg<BN>::kSmemBytes, stream, p.maps, dymap, g, dw, status);
   return TSP_LAUNCH_CHECK();
 }
 
@@ -1423,8 +1434,8 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int n, int h, in
   }
   const int num_tiles = g.tiles_w * g.tiles_h * g.tiles_n;
   const int n_sm = sm_count();
-  kern<<<num_tiles < n_sm ? num_tiles : n_sm, kWgThreads, WgHaloCfg::kSmemBytes, stream>>>(
-      xmap, dymap, g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, dw, status);
+  tsp::launch_early(kern, num_tiles < n_sm ? num_tiles : n_sm, kWgThreads, WgHaloCfg::kSmemBytes, stream, xmap, dymap, g,
+                    (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, dw, status);
   return TSP_LAUNCH_CHECK();
 }
 

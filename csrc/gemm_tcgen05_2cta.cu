@@ -221,6 +221,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
   cluster_sync_all();                                   // both CTAs' barriers exist before anyone signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  tsp::wait_for_previous();
+  bias = tsp::written(bias);
 
   if (warp == 0) {
     // ---------------- TMA producer (one thread per CTA) ----------------
@@ -264,6 +266,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
           }
         }
       }
+      tsp::let_next_start();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
@@ -590,13 +593,14 @@ int launch_bn(const Args& p, int dev, int max_pairs, cudaStream_t stream) {
   cfg.blockDim = dim3(64 + 32 * epi_warps(KIND), 1, 1);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1] = tsp::early_start();
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, p.n_src > 1 ? (KIND == kRed ? a_src : a_src / BK) : 0x7fffffff, tb, tc, KIND == kTN && p.n_dst > 1 ? n_per : 0x7fffffff, tma_store,
                                      (OutT*)p.c[0], p.bias,
                                      p.m, p.n, p.k, p.ldc, p.epi, splits, p.col_sums, p.seg_rows, p.status);

@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ x, co
                                                      const float* __restrict__ b, T* __restrict__ y,
                                                      float* __restrict__ mean, float* __restrict__ rstd, int rows,
                                                      int d, float eps) {
+  tsp::let_next_start();
   constexpr int R = 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = (blockIdx.x * 4 + warp) * R;
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(kLnBwdWarps * 32, sizeof(T) == 2 ? 2 : 1)
 ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ skip, const float* __restrict__ w,
               const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
               float* __restrict__ partial, int rows, int d) {
+  tsp::let_next_start();
   __shared__ float sm[2 * 256 * NV];       // [2][256 * NV] the block's sums
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = d >> 3;
@@ -181,6 +183,7 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
 constexpr int kLnReduce = 32;
 __global__ void __launch_bounds__(32 * kLnReduce) ln_bwd_reduce_kernel(const float* __restrict__ partial, int nblocks, int d,
                                                             float* __restrict__ dw, float* __restrict__ db, int add) {
+  tsp::let_next_start();
   __shared__ float sm[kLnReduce][33];
   const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
@@ -214,6 +217,7 @@ constexpr int kGeluFwdVecs = 4, kGeluBwdVecs = 2;
 template <typename T>
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ bias,
                                                        T* __restrict__ y, int64_t n, int d) {
+  tsp::let_next_start();
   constexpr int U = kGeluFwdVecs;
   const int64_t nv = n >> 3;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -241,6 +245,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gelu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                        const float* __restrict__ bias, T* __restrict__ dx, int64_t n,
                                                        int d) {
+  tsp::let_next_start();
   constexpr int U = kGeluBwdVecs;
   const int64_t nv = n >> 3;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -274,6 +279,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gelu_bwd_sums_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                             const float* __restrict__ bias, T* __restrict__ dx,
                                                             float* __restrict__ sums, int64_t rows, int d) {
+  tsp::let_next_start();
   constexpr int U = kGeluSumVecs;
   __shared__ float part[kGeluSumRows][256 + 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

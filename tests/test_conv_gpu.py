@@ -235,3 +235,61 @@ def test_bottleneck_on_igemm_convolutions_matches_library_path():
     torch.testing.assert_close(outs[1], outs[0], rtol=3e-2, atol=3e-2)
     for a, b in zip(grads[1], grads[0]):
         torch.testing.assert_close(a, b, rtol=5e-2, atol=5e-2 * max(b.abs().max().item(), 1e-3))
+
+
+@pytest.mark.parametrize("mode", ["stream", "side stream", "graph", "forked graph"])
+def test_kernels_that_start_early_wait_for_what_they_read(mode):
+    """Convolutions and products in a chain whose every launch overwrites what the next one reads, beside library kernels, a
+    memset and a second stream: the same bits as with a synchronisation after each launch."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(41)
+    dev = torch.device("cuda", 0)
+    x0 = torch.randn(8, 64, 28, 28, device=dev).to(dtype=torch.bfloat16, memory_format=torch.channels_last)
+    w1 = (torch.randn(256, 64, 1, 1, device=dev) * 0.2).to(memory_format=torch.channels_last)
+    w2 = (torch.randn(64, 256, 1, 1, device=dev) * 0.1).to(memory_format=torch.channels_last)
+    w3 = (torch.randn(64, 64, 3, 3, device=dev) * 0.08).to(memory_format=torch.channels_last)
+    lin = (torch.randn(64, 64, device=dev) * 0.2).bfloat16()
+    buf, side_out = torch.empty_like(x0), torch.empty_like(x0)
+    side = torch.cuda.Stream()
+
+    def chain(wait, fork):
+        buf.copy_(x0)
+        for i in range(6):
+            y = conv.conv2d(buf, w1, 1)[0]
+            wait()
+            z = conv.conv2d(y, w2, 1)[0]
+            wait()
+            if fork:
+                side.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(side):
+                    side_out.copy_(conv.conv2d(z, w3, 1)[0])
+                torch.cuda.current_stream().wait_stream(side)
+            buf.zero_()
+            t = conv.conv2d(z, w3, 1)[0]
+            wait()
+            buf.add_(t)
+            rows = buf.permute(0, 2, 3, 1).reshape(-1, 64)
+            p = gemm.matmul_nt(rows, lin)
+            wait()
+            rows.copy_(p.to(rows.dtype) / (p.float().abs().max() + 1))
+        return buf
+
+    with torch.no_grad():
+        want = chain(torch.cuda.synchronize, False).clone()
+        for _ in range(3):
+            if mode == "stream":
+                got = chain(lambda: None, False)
+            elif mode == "side stream":
+                with torch.cuda.stream(side):
+                    side.wait_stream(torch.cuda.default_stream())
+                    got = chain(lambda: None, False)
+            else:
+                graph = torch.cuda.CUDAGraph()
+                torch.cuda.synchronize()
+                with torch.cuda.graph(graph):
+                    got = chain(lambda: None, mode == "forked graph")
+                graph.replay()
+                graph.replay()
+            torch.cuda.synchronize()
+            assert torch.isfinite(want).all() and torch.equal(got, want)
+    gemm.check_status()
