@@ -185,7 +185,11 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
   const int num_tiles = tiles_m * tiles_n;
   const int num_kb = (k + BK - 1) / BK;
   // work items: tiles, and with kRed each tile in `splits` pieces of the contraction (item = piece * num_tiles + tile)
-  const int num_items = num_tiles * (KIND == kRed ? splits : 1);
+  // otherwise the tiles of the last, partial round in `splits` pieces of their columns each, side by side on the idle pairs
+  const int whole = KIND == kRed ? 0 : num_tiles / num_pairs * num_pairs;
+  const int num_items = whole + (num_tiles - whole) * splits;
+  int width = BN;                                      // columns of the item at hand, and its first one within the tile
+  int first_col = 0;
   auto item_range = [&](int t, int& tile, int& kb_lo, int& kb_hi) {
     if constexpr (KIND == kRed) {
       const int sp = t / num_tiles;
@@ -194,6 +198,12 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
       kb_hi = (int)((int64_t)num_kb * (sp + 1) / splits);
     } else {
       tile = t; kb_lo = 0; kb_hi = num_kb;
+      if (t >= whole) {
+        const int j = t - whole;
+        tile = whole + j / splits;
+        width = BN / splits;
+        first_col = j % splits * width;
+      }
     }
   };
 
@@ -235,7 +245,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
         int tile, kb_lo, kb_hi;
         item_range(t, tile, kb_lo, kb_hi);
         const int m0 = (tile / tiles_n) * 2 * BM + (int)rank * BM;
-        const int n0 = (tile % tiles_n) * BN + (int)rank * (BN / 2);
+        const int n0 = (tile % tiles_n) * BN + first_col + (int)rank * (width / 2);    // (a narrow item's box holds more than it uses)
         for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
           const int s = it % kStages;
           if (it % kGroup == 0) {                 // first stage of a group: the whole group must have been released
@@ -277,7 +287,6 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
       };
       constexpr bool kAmn = KIND == kRed, kBmn = KIND == kNN || KIND == kRed;
       static_assert(!kBmn || BN % 128 == 0, "an MN-major half tile of B is whole 64-column boxes");
-      constexpr uint32_t idesc = tc5::make_idesc(2 * BM, BN, kAmn, kBmn);
       const uint32_t tiles_addr = smem_u32(tiles);
       uint32_t it = 0, lt = 0;
       bool ok = true;
@@ -290,7 +299,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * BN, idesc = tc5::make_idesc(2 * BM, width, kAmn, kBmn);
         uint32_t accum = 0u;
         for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
           const int s = it % kStages;
@@ -346,7 +355,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
     for (int t = pair; t < num_items && ok; t += num_pairs, ++lt) {
       int tile, kb_lo, kb_hi;
       item_range(t, tile, kb_lo, kb_hi);
-      const int m0 = (tile / tiles_n) * 2 * BM + (int)rank * BM, n0 = (tile % tiles_n) * BN;
+      const int m0 = (tile / tiles_n) * 2 * BM + (int)rank * BM, n0 = (tile % tiles_n) * BN + first_col;
       const uint32_t acc = lt & 1, use = lt >> 1;
       if (STATS) {
         const int seg = m0 / seg_rows;
@@ -471,7 +480,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
         if (chunk(0, cs[0]) && chunk(64, cs[1]) && chunk(128, cs[2])) chunk(192, cs[3]);
       } else {
 #pragma unroll 1
-        for (int c0 = KIND == kGelu ? group * kCols : 0; c0 < BN; c0 += kCols * (epi_warps(KIND) / 4))
+        for (int c0 = KIND == kGelu ? group * kCols : 0; c0 < width; c0 += kCols * (epi_warps(KIND) / 4))
           if (!chunk(c0, nullptr)) break;
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -538,6 +547,18 @@ int pick_splits(int m, int n, int k, int bn, int pairs) {
   return best;
 }
 
+// Pieces of a tile's columns in the last round of tiles, where it leaves at least half of the pairs idle: as many as `most` and
+// as run at once.  A step of a narrow piece takes less time, and the sums are formed in the same order.  12608 x 768 (150 tiles on 74
+// pairs), B200: K = 3072 56.5 us with whole tiles in the third round, 47.8 in quarters; in halves (MN-major B) 53.8.  Within a
+// ViT-B block, whose products run at the power limit, 880 us and 877.
+int last_round_pieces(int tiles, int pairs, int most) {
+  const int left = tiles % pairs;
+  int pieces = 1;
+  if (tiles > pairs && left != 0)
+    while (2 * pieces <= most && 2 * pieces * left <= pairs) pieces *= 2;
+  return pieces;
+}
+
 struct Args {
   const void* a[kMaxASrc];
   int n_src;                    // matrices side by side, each k / n_src (kNN) or m / n_src (kRed) wide
@@ -585,8 +606,10 @@ int launch_bn(const Args& p, int dev, int max_pairs, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const int splits = KIND == kRed ? pick_splits(p.m, p.n, p.k, BN, max_pairs) : 1;
-  const int num_items = ((p.n + BN - 1) / BN) * ((p.m + 2 * BM - 1) / (2 * BM)) * splits;
+  const int num_tiles = ((p.n + BN - 1) / BN) * ((p.m + 2 * BM - 1) / (2 * BM));
+  const int splits = KIND == kRed ? pick_splits(p.m, p.n, p.k, BN, max_pairs)
+                                  : (STATS ? 1 : last_round_pieces(num_tiles, max_pairs, BN / (kBmn ? 128 : 64)));
+  const int num_items = KIND == kRed ? num_tiles * splits : num_tiles;
   const int pairs = max_pairs > num_items ? num_items : max_pairs;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);

@@ -417,6 +417,31 @@ def test_linear_products_at_every_tile_width(m, n, k):
     assert _rel(dw - 1, dy.double().t() @ x.double()) < 1e-5
 
 
+@pytest.mark.parametrize("m,n,k", [(6400, 768, 320), (6376, 760, 64), (4864, 1000, 200), (9344, 768, 128), (12608, 768, 768),
+                                   (18950, 256, 72)])
+def test_products_with_a_nearly_empty_last_round(m, n, k):
+    """One, two or more tiles past whole rounds of 74 pairs: their columns are dealt to the idle pairs."""
+    from tspipe_b200.ops import gemm
+    torch.manual_seed(29)
+    a, b = torch.randn(m, k, device=DEV).bfloat16(), torch.randn(n, k, device=DEV).bfloat16()
+    bias = torch.randn(n, device=DEV)
+    exact, size = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+
+    def close(got, want, ulp, slack=0.0):      # fp32 sums of k terms err by less than 2^-20 of the terms' sizes
+        assert ((got.double() - want).abs() <= want.abs() * ulp + (size + bias.abs()) * 2.0 ** -20 + slack).all()
+
+    close(gemm.matmul_nt(a, b, bias, out_dtype=torch.float32), exact + bias.double(), 2.0 ** -22)
+    close(gemm.matmul_nt(a, b), exact, 2.0 ** -8)
+    if k % 64 == 0:
+        close(gemm.matmul_nn([a], b.t().contiguous()), exact, 2.0 ** -8)
+    if n % 64 == 0:                            # the activation of the rounded product, rounded once more
+        with torch.no_grad():
+            got = gemm.linear_gelu(a, b, bias)
+        h = exact.bfloat16().double() + bias.double()
+        close(got, F.gelu(h), 2.0 ** -7, exact.abs().max().item() * 2.0 ** -7)
+    gemm.check_status()
+
+
 @pytest.mark.parametrize("bias", [True, False])
 @pytest.mark.parametrize("rows,c,heads", [((2, 65), 192, 3), ((3, 197), 768, 12)])
 def test_fused_qkv_projection_matches_three_linears(rows, c, heads, bias):
