@@ -395,25 +395,49 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
   }
 }
 
-// The share of tiles [t_begin, t_end) in dW[co][kh][kw][ch], i = co * 147 + kh * 21 + kw * 3 + ch, by a warp, lane = pixel.
-__device__ __noinline__ float exact_sum(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, int h, int w,
-                                        int oh_n, int ow_n, int per_image, int t_begin, int t_end, int i, int lane) {
-  const int co = i / kK, kh = i % kK / 21, kw = i % 21 / 3, ch = i % 3;
-  float v = 0.f;
+// The share of tiles [t_begin, t_end) in the sums of tap row kh from the definition (a tap's pixels outside the image are zeros),
+// by a warp, for those of `sum` [co][147] that are not finite: lane = two output channels, all 21 taps and input channels of the row
+// in registers, so that dY is read once per tap row, 128 bytes at a time.
+__device__ __noinline__ void exact_tap_row(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, int h, int w,
+                                           int oh_n, int ow_n, int per_image, int t_begin, int t_end, int kh, int lane, float* sum) {
+  constexpr int kTaps = 21;
+  float acc[kTaps][2];
+#pragma unroll
+  for (int k = 0; k < kTaps; ++k) acc[k][0] = acc[k][1] = 0.f;
   for (int t = t_begin; t < t_end; ++t) {
     const int n = t / per_image, oh0 = (t - n * per_image) * kTileRows;
     for (int oh = oh0; oh < oh0 + kTileRows && oh < oh_n; ++oh) {
       const int ih = 2 * oh - 3 + kh;
-      if (ih < 0 || ih >= h) continue;
-      for (int ox = lane; ox < ow_n; ox += 32) {
-        const int iw = 2 * ox - 3 + kw;
-        if (iw < 0 || iw >= w) continue;
-        v = fmaf(__bfloat162float(dy[(((int64_t)n * oh_n + oh) * ow_n + ox) * kCout + co]),
-                 __bfloat162float(x[(((int64_t)n * h + ih) * w + iw) * 3 + ch]), v);
+      const bool inside = ih >= 0 && ih < h;
+      const __nv_bfloat16* xr = x + ((int64_t)n * h + (inside ? ih : 0)) * w * 3;
+      const uint32_t* dr = reinterpret_cast<const uint32_t*>(dy + ((int64_t)n * oh_n + oh) * ow_n * kCout) + lane;
+      float part[kTaps][2];                    // of an output row
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) part[k][0] = part[k][1] = 0.f;
+#pragma unroll 2
+      for (int ox = 0; ox < ow_n; ++ox) {
+        const int at = (2 * ox - 3) * 3 + lane;              // lane = (tap, channel) of the row
+        const float mine = inside && lane < kTaps && at >= 0 && at < 3 * w ? __bfloat162float(xr[at]) : 0.f;
+        const uint32_t d = __ldg(dr + ox * (kCout / 2));
+        const float d0 = __uint_as_float(d << 16), d1 = __uint_as_float(d & 0xffff0000u);
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) {
+          const float v = __shfl_sync(0xffffffffu, mine, k);
+          part[k][0] = fmaf(d0, v, part[k][0]);
+          part[k][1] = fmaf(d1, v, part[k][1]);
+        }
       }
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) { acc[k][0] += part[k][0]; acc[k][1] += part[k][1]; }
     }
   }
-  return tsp::warp_sum(v);
+#pragma unroll
+  for (int k = 0; k < kTaps; ++k)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float* at = sum + (2 * lane + e) * kK + kh * kTaps + k;
+      if ((__float_as_uint(*at) & 0x7f800000u) == 0x7f800000u) *at = acc[k][e];
+    }
 }
 
 // The pitch of a row is an odd multiple of 16 bytes: what a product reads of one pixel, 16 bytes of each of 16 rows, then lies in
@@ -495,16 +519,13 @@ conv_stem_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy, const __nv_b
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       }
       if (loaders_and(good)) {
-        // An infinite or NaN pixel also meets the zeros of dY past a row's end and of missing rows (0 x inf = NaN), in taps that
-        // do not pair it with a dY: sums that are not finite are formed again from the definition.
-        for (int i0 = warp * 32; i0 < kCout * kK; i0 += kLoaders * 32) {
-          const int i = i0 + lane;
-          uint32_t todo = __ballot_sync(0xffffffffu, i < kCout * kK && (__float_as_uint(sum[i]) & 0x7f800000u) == 0x7f800000u);
-          for (; todo != 0; todo &= todo - 1) {
-            const int k = i0 + __ffs(todo) - 1;
-            const float v = exact_sum(x, dy, h, w, oh_n, ow_n, per_image, t_begin, t_end, k, lane);
-            if (lane == 0) sum[k] = v;
-          }
+        // Zeros of dY past a row's end and of a missing row meet pixels too: an infinite or NaN one makes a NaN (0 x inf) of taps
+        // that do not pair it with a dY.  Where there are such zeros, sums that are not finite are formed again.
+        if ((ow_n & 15) != 0 || (oh_n & 1) != 0) {
+          bool finite = true;
+          for (int i = tid; i < kCout * kK; i += kLoaders * 32) finite = finite && (__float_as_uint(sum[i]) & 0x7f800000u) != 0x7f800000u;
+          if (!loaders_and(finite) && warp < 7)
+            exact_tap_row(x, dy, h, w, oh_n, ow_n, per_image, t_begin, t_end, warp, lane, sum);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         loaders_and(true);

@@ -598,6 +598,51 @@ def test_stem_weight_gradient_of_infinite_pixels(n, h, w):
         assert _rel(dw[ok], want[ok]) < 1e-5
 
 
+@pytest.mark.parametrize("n,h,w", [(1, 8, 8), (3, 10, 24), (2, 22, 200), (2, 16, 224)])
+def test_stem_weight_gradient_of_infinite_gradients(n, h, w):
+    """An infinite or NaN gradient reaches all taps of its channel, those outside the image as a product with zero padding, and
+    no other channel; beside an infinite pixel too."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(14)
+    for at, value in (((0, 5, 0, 0), math.inf), ((n - 1, 63, h // 2 - 1, w // 2 - 1), -math.inf), ((n - 1, 0, h // 4, w // 4), math.nan)):
+        for bad_pixel in (False, True):
+            x = _cl(n, 3, h, w)
+            if bad_pixel:
+                x[0, 2, h - 1, w - 1] = math.inf
+            weight = (torch.randn(64, 3, 7, 7, device=DEV) * 0.1).requires_grad_()
+            y, _ = conv.stem_conv(x, weight, want_sums=False)
+            g = _cl(*y.shape)
+            g[at] = value
+            (dw,) = torch.autograd.grad(y, weight, g)
+            gemm.check_status()
+            patches, g6 = F.unfold(x.double(), 7, padding=3, stride=2), g.double().flatten(2)
+            want = torch.stack([(g6[i, :, None] * patches[i][None]).sum(-1) for i in range(n)]).sum(0).view(64, 3, 7, 7)
+            ok = want.isfinite()
+            assert ok.any() and not ok[at[1]].any() and torch.equal(dw.isfinite(), ok) and torch.equal(dw.isnan(), want.isnan())
+            assert _rel(dw[ok], want[ok]) < 1e-5
+
+
+@pytest.mark.parametrize("h,w", [(224, 224), (218, 216)])
+def test_stem_weight_gradient_of_nan_takes_no_longer(h, w):
+    """A gradient of NaN alone, over images of which some hundred rows fall to a CTA.  Where zeros of dY meet pixels the sums are
+    formed twice, the second time by threads: a millisecond or two."""
+    from tspipe_b200.ops import conv
+    x = _cl(128, 3, h, w)
+    weight = (torch.randn(64, 3, 7, 7, device=DEV) * 0.1).requires_grad_()
+    y, _ = conv.stem_conv(x, weight, want_sums=False)
+    times = {}
+    for name, g in (("finite", _cl(*y.shape)), ("nan", torch.full_like(y, math.nan))):
+        for _ in range(3):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            (dw,) = torch.autograd.grad(y, weight, g, retain_graph=True)
+            b.record()
+            b.synchronize()
+            times[name] = min(times.get(name, math.inf), a.elapsed_time(b))
+        assert dw.isnan().all() if name == "nan" else dw.isfinite().all()
+    assert times["nan"] < (3 * times["finite"] + 0.2 if w % 32 == 0 else 10), times
+
+
 def test_stem_weight_gradient_by_name_and_past_hooks():
     """Eagerly the gradient goes to autograd, also where a channels-last one is there already: whoever asks for it by name
     gets it, and hooks see it."""
