@@ -463,15 +463,17 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
       const bool in = lane < kRowWarps;
       const RowPart ws = {in ? pp[0][lane] : -INFINITY}, wtop = {in ? pp[1][lane] : -INFINITY};
       const float ms = warp_top(ws.m), mt = warp_top(wtop.m);
-      if (warp == 0) {                                  // the divergence, by one warp
-        const float f = in ? ex2((wtop.ref() - mt) * k2) : 0.f;
-        kl = tsp::warp_sum(in ? moved(pp[5][lane], pp[4][lane], f, (wtop.ref() - ws.ref()) - (mt - ms)) : 0.f);
-      }
+      // The divergence.  Before a part refers to the row's maximum, a class that the student has switched off (the type's lowest
+      // value, -inf) can take it past the largest float, or to infinity where the teacher's probability will be no float: a row
+      // with such a part has its divergence formed from the probabilities, behind the second sweep.
+      const float part_kl = in ? moved(pp[5][lane], pp[4][lane], ex2((wtop.ref() - mt) * k2), (wtop.ref() - ws.ref()) - (mt - ms)) : 0.f;
+      const bool redo = __any_sync(0xffffffffu, !(fabsf(part_kl) < 1e30f)) != 0;       // the same for all computing warps
+      if (warp == 0) kl = tsp::warp_sum(part_kl);
       z1 = has_ce ? tsp::warp_sum(in ? pp[2][lane] * ex2((ws.ref() - ms) * kLog2e) : 0.f) : 0.f;
       zs = tsp::warp_sum(in ? pp[3][lane] * ex2((ws.ref() - ms) * k2) : 0.f);
       zt = tsp::warp_sum(in ? pp[4][lane] * ex2((wtop.ref() - mt) * k2) : 0.f);
       const float l1 = has_ce ? log2f(z1) : 0.f, ls = log2f(zs), lt = log2f(zt);
-      if (threadIdx.x == 0) acc += (double)(wt * (kl / zt)) - (double)(w_kd * temp * (temp * (lt - ls) * kLn2));
+      if (threadIdx.x == 0) acc += (redo ? 0. : (double)(wt * (kl / zt))) - (double)(w_kd * temp * (temp * (lt - ls) * kLn2));
       // second sweep: the gradient
       uint4* gr = gs ? reinterpret_cast<uint4*>(gs + (int64_t)id.x * c) : nullptr;
       const uint4* sr = reinterpret_cast<const uint4*>(s + (int64_t)id.x * c);
@@ -505,6 +507,27 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
           if (gr) __stcs(gr + i, make_uint4(tc5::pack_bf16x2(v[0], v[1]), tc5::pack_bf16x2(v[2], v[3]),
                                             tc5::pack_bf16x2(v[4], v[5]), tc5::pack_bf16x2(v[6], v[7])));
         }
+      }
+      if (redo) {                                       // as kd_ce_kernel forms it; the rows once more, from L2
+        const uint4* tr = reinterpret_cast<const uint4*>(t + (int64_t)id.x * c);
+        float part = 0.f;
+#pragma unroll 1
+        for (int i = threadIdx.x; i < nv; i += kRowThreads) {
+          const uint4 qa = __ldg(sr + i), qb = __ldg(tr + i);
+          const uint32_t a[4] = {qa.x, qa.y, qa.z, qa.w}, b[4] = {qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float av[2], bv[2];
+            unpack2(a[j]).split(av[0], av[1]);
+            unpack2(b[j]).split(bv[0], bv[1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float db = bv[e] - mt, p = ex2(db * k2 - lt);
+              if (p != 0.f) part = fmaf(p, db - (av[e] - ms), part);
+            }
+          }
+        }
+        acc += (double)wt * (double)part;
       }
     }
 #pragma unroll
