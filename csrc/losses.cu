@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(128) byol_kernel(const PairPtrs<T> in, int n, 
 // 36 MB) and writes the gradient past L2's reuse order.  The sum that only cross-entropy needs is formed on labelled
 // rows alone.  Bound by DRAM and, next to it, by the exponentials (four per element and two more on labelled rows).
 // VEC: rows whose length is a multiple of 8 on 16-byte aligned bases are read and written 8 elements at a time.
-// 8192 rows of 30528 bf16, one in seven labelled: 476 us (3.2 TB/s); three sweeps of single elements took 1810 us.
+// 8192 rows of 30528 bf16, one in seven labelled, none masked: 480 us (3.1 TB/s); three sweeps of single elements took 1810 us.
 // ---------------------------------------------------------------------------------------------
 struct RowPart {          // running maximum (-inf while empty)
   float m;
@@ -251,9 +251,11 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
 // registers and of the student in shared memory (122 KB each for 30528 classes), and the second only scales them by one factor
 // per vector.  The divergence is summed in the first sweep as well, sum e_t ((b - mt) - (a - ms)), and follows the maxima
 // as the other sums do.  Meanwhile a producer warp streams the next rows into a ring with bulk copies.
-// Only for what it was made for, rows that fill the five vectors and several of them per SM: 8192 rows of 30528, a quarter masked
-// and one in seven labelled, 381 us with the kernel above and 342 with this one, 1000 rows 64.7 and 60.5; but 8192 of 24576 (four
-// vectors) 307 and 296, 8192 of 16384 226 and 234, 300 of 30528 27.5 and 30.6.  What bounds it is instruction issue beside the
+// For rows that nearly fill five vectors per thread, several of them per SM.  Microseconds with the kernel above and with this
+// one, one in seven rows labelled and a quarter masked: 8192 rows of 30528 383 and 340, 2048 113 and 102, 1024 68 and 61, 592 47 and
+// 45, 300 31 and 35.  A vector that few threads have part in costs what a full one does: without masked rows, 2048 of 28672 1.02
+// times as fast, of 26624 1.00, of 24584 0.97, 1024 of them 0.94 (whole vectors fewer, 24576 or 18432: 1.00 at 2048
+// rows, 1.03 at 8192).  What bounds it is instruction issue beside the
 // exponentials (per vector: waits, maxima, references; per row: the sums over 24 warps); fewer warps with more of a row each are
 // slower for want of warps (12: 460 us where 24 take 410, unmasked).
 // Rows are drawn by ticket: masked ones cost next to nothing (the producer warp writes their zeros), so a fixed share of
@@ -269,7 +271,7 @@ constexpr int kRowSmem = kRing * 2 * kPieceBytes + kRowVecs * kPieceElems * 4 + 
 constexpr int kRowQueue = 4;                                    // rows that the ring and the sweeps may hold
 static_assert(kRing < kRowQueue * 2 && kRowSmem <= 227 * 1024, "a row in the ring is two pieces at least");
 constexpr uint64_t kRowWaitNs = 2000000000ull;                  // a wait gives up after two seconds
-constexpr int kStreamMin = (kRowVecs - 1) * kPieceElems + 8;    // elements of a row
+constexpr int kStreamMin = (3 * kRowVecs - 1) * kPieceElems / 3;    // elements of a row: the last vector two thirds full
 constexpr int kStreamRows = 1024;                               // rows: seven per SM
 
 using tsp::Pair;
