@@ -23,8 +23,6 @@
 #include "tcgen05.cuh"
 #include "tspipe_kernels.h"
 
-extern int g_tsp_sm_reserve;          // defined in peer.cu
-
 namespace {
 
 constexpr int kTile = 128, kDim = 64;
@@ -398,12 +396,10 @@ int tsp_attn_heads_fwd(const void* q, const void* k, const void* v, const uint8_
   if (!head_map(&tq, q, nq, heads, batch, q_strides) || !head_map(&tk, k, nk, heads, batch, k_strides) ||
       !head_map(&tv, v, nk, heads, batch, v_strides) || !head_map(&to, out, nq, heads, batch, o_strides, 32))
     return -6;
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int usable = 0;
+  cudaError_t e = tsp::usable_sms(usable);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e != cudaSuccess) return (int)e;
-  const int usable = sms - g_tsp_sm_reserve > 8 ? sms - g_tsp_sm_reserve : 8;
   attn_heads_kernel<<<items < usable ? (int)items : usable, kThreads, kSmemBytes, stream>>>(
       tq, tk, tv, to, mask, mask_stride, nq, nk, heads, (int)items, scale, status);
   return TSP_LAUNCH_CHECK();

@@ -182,7 +182,6 @@ struct Hyper {                                // (filled in by the caller: optim
 };
 }  // namespace tsp
 
-// Every launcher returns the cudaError_t of its launch as int (0 = ok).
 // ---------------------------------------------------------------------------------------------------------------------
 // Launches that overlap the end of the kernel before them (programmatic dependent launch): the grid may be placed when every
 // block of that kernel has called let_next_start or left, and wait_for_previous returns when it is complete and its writes
@@ -223,4 +222,17 @@ inline cudaError_t launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_
 }
 }  // namespace tsp
 
+extern int g_tsp_sm_reserve;          // defined in peer.cu
+namespace tsp {
+// SMs that a persistent kernel may fill: all but those reserved for communication kernels (tsp_set_sm_reserve).
+inline cudaError_t usable_sms(int& n) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  n = n - g_tsp_sm_reserve > 8 ? n - g_tsp_sm_reserve : 8;
+  return e;
+}
+}  // namespace tsp
+
+// Every launcher returns the cudaError_t of its launch as int (0 = ok).
 #define TSP_LAUNCH_CHECK() ((int)cudaGetLastError())

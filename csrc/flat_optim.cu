@@ -413,10 +413,10 @@ int tsp_lars_step_ordered(float* p, const float* g, float* mu, const void* order
   if (n_items <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(order) & 15) != 0) return -2;
   cudaError_t e = cudaMemsetAsync(work, 0, sizeof(float) * (3 * (size_t)n_seg + 1), stream);
-  int dev = 0, sms = 0;
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int sms = 0;
+  if (e == cudaSuccess) e = tsp::usable_sms(sms);
   if (e != cudaSuccess) return (int)e;
+  // (blocks for a whole number of SMs fewer: as many SMs are empty, or four times as many have room for a quarter of theirs)
   const int grid = n_items < kStepBlocks * sms ? n_items : kStepBlocks * sms;
   lars_step_kernel<<<grid, kStepThreads, 0, stream>>>(p, g, mu, (const int4*)order, n_items, need, *(const Hyper*)hyper,
                                                       grad_scale, work, (int*)(work + 2 * (size_t)n_seg), teacher, teacher_n,

@@ -702,9 +702,8 @@ int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const ui
   const bool vec = rows_of_8(c, s, t, gs);
   if (vec && t != nullptr && w_kd != 0.f && s_dtype == TSP_DTYPE_BF16 && t_dtype == TSP_DTYPE_BF16 &&
       n >= kStreamRows && c >= kStreamMin && c <= kRowVecs * kPieceElems) {
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    cudaError_t e = tsp::usable_sms(sms);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kd_ce_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmem);
     if (e != cudaSuccess) return (int)e;
     kd_ce_stream_kernel<<<n < sms ? n : sms, kRowThreads + 32, kRowSmem, stream>>>(

@@ -279,12 +279,12 @@ inline bool fill(PeerPtrs& dst, void* const* src, int n) {
 
 }  // namespace
 
-// SMs that the persistent tensor-core kernels leave free (see tsp_set_sm_reserve)
+// SMs that the persistent kernels leave free (see tsp_set_sm_reserve)
 int g_tsp_sm_reserve = 0;
 
 extern "C" {
 
-// The persistent tcgen05 kernels (convolutions, GEMMs) launch one CTA per SM with almost all of its shared memory; a
+// The persistent kernels (convolutions, GEMMs, attention, the vocabulary loss, the LARS step) fill the SMs that they run on; a
 // communication kernel that becomes ready while one of them runs (an NCCL send / receive of a stage link, a peer
 // reduction on a side stream) finds no SM until a CTA retires, i.e. until the whole persistent kernel ends.  With a
 // reserve of n, those kernels launch on (SM count - n) SMs and the rest stay available.  Set by the runtime when a

@@ -79,6 +79,24 @@ def test_lars_norms_and_updates_in_one_launch(lag, ema):
         _same([flat._view(teacher, i, p.data) for i, p in enumerate(ps)], want, 2)
 
 
+@pytest.mark.parametrize("reserve", [0, 8])
+def test_lars_in_one_launch_leaves_reserved_sms(reserve):
+    """Every block draws a ticket more than it has rows of work."""
+    from tspipe_b200.ops import fused
+    ps = [nn.Parameter(torch.randn(3000, 2048, device=DEV)), nn.Parameter(torch.randn(77, device=DEV))]
+    flat = FlatParams(ps, DEV, with_grad=True)
+    opt = MAKE["lars"](ps)
+    opt.bind_flat(flat, use_kernel=True)
+    order = fused.LarsOrder(opt._chunks, 2, DEV)
+    fused.set_sm_reserve(reserve)
+    try:
+        fused.lars_step_ordered_(flat.data, flat.grad, torch.zeros_like(flat.data), order, opt._hyper_of([[0.1, 0.0, 0.9, 1e-3]]))
+    finally:
+        fused.set_sm_reserve(0)
+    tickets, sms = int(order.work.view(torch.int32)[4]), torch.cuda.get_device_properties(0).multi_processor_count
+    assert order.order.shape[0] > 4 * sms and tickets - order.order.shape[0] == 4 * (sms - reserve)
+
+
 def test_a_recorded_step_repeats_its_values_and_refuses_new_ones():
     ps, qs = _params(5), _params(5)
     lars, adam = MAKE["lars"](ps), MAKE["adamw"](qs)

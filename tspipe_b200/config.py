@@ -35,7 +35,7 @@ New optional keys (all defaulted so reference YAML files load unchanged):
                              (bounded waits) instead of tiny NCCL collectives (default True)
 ``runtime.dp_early_reduce``  start the data-parallel gradient reduction on a side stream right after the backward
                              wave, behind the look-ahead teacher forward (default True)
-``runtime.sm_reserve``       SMs the persistent tensor-core kernels leave free for communication kernels
+``runtime.sm_reserve``       SMs the persistent kernels leave free for communication kernels
                              (default: 8 with stage links, 0 for single-stage jobs)
 ``runtime.heartbeat_s`` / ``runtime.timeout_s``  failure-detection heartbeat period / deadline
 """

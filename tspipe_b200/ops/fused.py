@@ -42,7 +42,8 @@ def lib():
 
 
 def set_sm_reserve(n: int) -> None:
-    """Leave ``n`` SMs free of the persistent tcgen05 kernels (convolutions, GEMMs) so that communication kernels
+    """Leave ``n`` SMs free of the persistent kernels (convolutions, GEMMs, attention, the vocabulary loss, the LARS step)
+    so that communication kernels
     that become ready while one of them runs - NCCL sends / receives of the stage links, peer reductions on a side
     stream - find an SM at once instead of when the persistent kernel ends."""
     lib().tsp_set_sm_reserve(_c.c_int(int(n)))
