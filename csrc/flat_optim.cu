@@ -15,7 +15,7 @@ using tsp::Hyper;
 
 constexpr int kThreads = 256;
 constexpr int kStepThreads = 256, kStepBlocks = 4;      // of lars_step_kernel, blocks per SM
-constexpr uint64_t kWaitNs = 2000000000ull;   // its waits give up after two seconds
+constexpr uint64_t kWaitNs = 2000000000ull;             // its waits give up after two seconds
 
 // ---------------------------------------------------------------------------------------------
 // EMA: t = m*t + (1-m)*s ; `s` may point into a peer GPU's memory (plain loads over NVLink).
@@ -197,31 +197,33 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
 // begin}), its norms and, some chunks after the last norms of its segment, its update.  Blocks draw rows by ticket, so a
 // wait for a segment's norms is a wait for rows that blocks drew before and are working on: whatever the number of
 // resident blocks, the earliest unfinished row never waits.  sync[0] = ticket, sync[1 + seg] = pieces of the segment whose
-// norms are in; `need` = pieces per segment.  Bound by DRAM (p, g, mu, t once in, p, mu, t once out: 5.0 TB/s of it).  A step
+// norms are in, sync[1 + n_seg] = a wait ran out; `need` = pieces per segment.  After a wait that ran out the step still ends: the
+// segment's ratio is NaN then, and with it what is left to update of the segment, and *status (host memory) is set, which the
+// optimizer raises on.  Bound by DRAM (p, g, mu, t once in, p, mu, t once out: 5.0 TB/s of it).  A step
 // over 25.6 M parameters with the teacher, microseconds: two launches 160, this one 144; without the teacher 127 and 109; 86 M
 // 494 and 463; 6 M (96 MB) 42 and 40.  Pieces of 32 KB and four blocks of 256 threads per SM: with pieces of 64 KB 147, of 16
 // KB 152; two blocks of 512 threads 149; three blocks of 256 159.
 __global__ void __launch_bounds__(kStepThreads, kStepBlocks)
 lars_step_kernel(float* p, const float* __restrict__ g, float* __restrict__ mu, const int4* __restrict__ order,
                  int n_items, const int* __restrict__ need, const __grid_constant__ Hyper hyper, float grad_scale, float* norms,
-                 int* sync, float* __restrict__ teacher, int64_t teacher_n, float ema_m, int* __restrict__ status) {
+                 int* sync, int n_seg, float* __restrict__ teacher, int64_t teacher_n, float ema_m, int* __restrict__ status) {
   __shared__ float scratch[33];
   __shared__ int4 row;
   __shared__ float ratio;
-  __shared__ int state;                             // of this block's row: 0 work, 1 no row left, 2 a wait ran out
+  __shared__ int done;                              // no row left
+  int* gave_up = sync + 1 + n_seg;
   int next = 0;
   if (threadIdx.x == 0) next = atomicAdd(sync, 1);
   for (;;) {
     if (threadIdx.x == 0) {
-      state = 1;
+      done = next < n_items ? 0 : 1;
       if (next < n_items) {
-        state = 0;
         row = __ldg(order + next);
         next = atomicAdd(sync, 1);                  // the ticket after this one, under way while this row is worked on
       }
     }
     __syncthreads();
-    if (state != 0) return;
+    if (done != 0) return;
     ChunkView c;
     c.seg = row.x >> 1;
     c.len = row.y;
@@ -246,23 +248,28 @@ lars_step_kernel(float* p, const float* __restrict__ g, float* __restrict__ mu, 
     } else {
       if (adapt && threadIdx.x == 0) {
         const int want = __ldg(need + c.seg);
+        bool in = true;
         uint64_t t0 = 0;
         for (int spin = 0; *((volatile int*)(sync + 1 + c.seg)) < want; ++spin) {
           if ((spin & 31) != 31) continue;
           uint64_t now;
           asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
           if (t0 == 0) t0 = now;
-          if (now - t0 > kWaitNs) {
-            atomicCAS(status, 0, 7);
-            state = 2;
+          const bool late = now - t0 > kWaitNs;
+          if (late || *((volatile int*)gave_up) != 0) {
+            if (late) {
+              atomicExch(gave_up, 1);
+              *((volatile int*)status) = 1;
+              __threadfence_system();
+            }
+            in = false;
             break;
           }
         }
         __threadfence();
-        ratio = lars_ratio(hp[3], __ldcg(norms + 2 * c.seg), __ldcg(norms + 2 * c.seg + 1));
+        ratio = in ? lars_ratio(hp[3], __ldcg(norms + 2 * c.seg), __ldcg(norms + 2 * c.seg + 1)) : __int_as_float(0x7fffffff);
       }
       __syncthreads();
-      if (state != 0) return;
       lars_update<true>(p, g, mu, c, hp, adapt ? ratio : 1.f, adapt ? hp[1] : 0.f, grad_scale, teacher, teacher_n, ema_m);
     }
     __syncthreads();                                // the row and the ratio are read before the next ones are written
@@ -412,14 +419,14 @@ int tsp_lars_step_ordered(float* p, const float* g, float* mu, const void* order
                           float ema_m, int* status, cudaStream_t stream) {
   if (n_items <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(order) & 15) != 0) return -2;
-  cudaError_t e = cudaMemsetAsync(work, 0, sizeof(float) * (3 * (size_t)n_seg + 1), stream);
+  cudaError_t e = cudaMemsetAsync(work, 0, sizeof(float) * (3 * (size_t)n_seg + 2), stream);
   int sms = 0;
   if (e == cudaSuccess) e = tsp::usable_sms(sms);
   if (e != cudaSuccess) return (int)e;
   // (blocks for a whole number of SMs fewer: as many SMs are empty, or four times as many have room for a quarter of theirs)
   const int grid = n_items < kStepBlocks * sms ? n_items : kStepBlocks * sms;
   lars_step_kernel<<<grid, kStepThreads, 0, stream>>>(p, g, mu, (const int4*)order, n_items, need, *(const Hyper*)hyper,
-                                                      grad_scale, work, (int*)(work + 2 * (size_t)n_seg), teacher, teacher_n,
+                                                      grad_scale, work, (int*)(work + 2 * (size_t)n_seg), n_seg, teacher, teacher_n,
                                                       ema_m, status);
   return TSP_LAUNCH_CHECK();
 }

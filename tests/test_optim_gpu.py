@@ -79,6 +79,40 @@ def test_lars_norms_and_updates_in_one_launch(lag, ema):
         _same([flat._view(teacher, i, p.data) for i, p in enumerate(ps)], want, 2)
 
 
+def test_lars_wait_that_runs_out_is_raised():
+    """A tensor whose norms are never all in (an order that asks for a piece too many): the step ends, that tensor is NaN, the
+    others are stepped, and neither a step nor a checkpoint follows until a state is loaded."""
+    shapes = [(600, 4096), (513, 4096), (41,), (700, 4096)]
+    torch.manual_seed(0)
+    ps = [nn.Parameter(torch.randn(*s, device=DEV)) for s in shapes]
+    ref = [nn.Parameter(p.detach().clone()) for p in ps]
+    flat = FlatParams(ps, DEV, with_grad=True)
+    opt, ropt = MAKE["lars"](ps), MAKE["lars"](ref)
+    opt.bind_flat(flat, use_kernel=True)
+    assert opt._order is not None
+    for p, q in zip(ps, ref):
+        q.grad = torch.randn_like(q)
+        p.grad.copy_(q.grad)
+    opt._buf("mu")
+    state = opt.state_dict()
+    before = flat.data.clone()
+    opt._order.need[3] += 1
+    opt.step()
+    ropt.step()
+    torch.cuda.synchronize()
+    _same(ps[:3], ref[:3], 1)
+    assert ps[3].isnan().all()
+    for use in (opt.step, opt.state_dict):
+        with pytest.raises(RuntimeError, match="ran out"):
+            use()
+    flat.data.copy_(before)
+    opt._order.need[3] -= 1
+    opt.load_state_dict(state)
+    opt.step()
+    _same(ps, ref, 1)
+    opt.state_dict()
+
+
 @pytest.mark.parametrize("reserve", [0, 8])
 def test_lars_in_one_launch_leaves_reserved_sms(reserve):
     """Every block draws a ticket more than it has rows of work."""

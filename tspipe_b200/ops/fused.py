@@ -271,10 +271,10 @@ class LarsOrder:
         self.order = torch.tensor(rows, dtype=torch.int64, device=device).view(-1, 2)
         self.need = torch.tensor(need, dtype=torch.int32, device=device)
         self.n_seg = n_seg
-        from .gemm import _status_word
-        self.status = _status_word(torch.device(device))
-        # sums of squares [2 n_seg], the ticket, finished pieces per segment
-        self.work = torch.zeros(3 * n_seg + 1, dtype=torch.float32, device=device)
+        # not zero once a wait in the kernel has run out; in host memory, where it is read without a synchronisation
+        self.status = torch.zeros(1, dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
+        # sums of squares [2 n_seg], the ticket, finished pieces per segment, whether a wait ran out
+        self.work = torch.zeros(3 * n_seg + 2, dtype=torch.float32, device=device)
 
     @staticmethod
     def plan(chunks, n_seg: int, lag: int):

@@ -180,6 +180,8 @@ class _FlatMixin:
 
 
 class LARS(_FlatMixin, Optimizer):
+    _order = None                                    # norms and updates in one launch: the order of the work
+
     def __init__(self, params, lr=0, weight_decay=0, momentum=0.9, trust_coefficient=0.001):
         super().__init__(params, dict(lr=lr, weight_decay=weight_decay, momentum=momentum,
                                       trust_coefficient=trust_coefficient))
@@ -192,10 +194,27 @@ class LARS(_FlatMixin, Optimizer):
             if 4 * self._chunks.shape[0] >= fused.LARS_ORDERED:
                 self._order = fused.LarsOrder(self._chunks, len(flat.params), flat.device)
 
+    def _check_order(self) -> None:
+        """Raise when a wait in an earlier one-launch step ran out (what it left of a tensor is NaN); neither another step nor a
+        checkpoint is made of it, until a state is loaded."""
+        if self._order is not None and self._order.status.item() != 0:
+            raise RuntimeError("LARS step: the wait for the norms of a tensor ran out, its parameters are not valid (NaN)")
+
+    def flat_state_dict(self) -> Dict[str, Any]:
+        sd = super().flat_state_dict()               # (copied to the host: the steps before have ended)
+        self._check_order()
+        return sd
+
+    def load_state_dict(self, sd):  # type: ignore[override]
+        super().load_state_dict(sd)
+        if self._order is not None:
+            self._order.status.zero_()
+
     @torch.no_grad()
     def step(self, closure=None, grad_scale: float = 1.0):
         if self.flat is None:
             return self._step_per_tensor()
+        self._check_order()
         flat = self.flat
         self._steps += 1
         mu = self._buf("mu")
