@@ -266,9 +266,12 @@ class LarsOrder:
     """The order in which one launch forms the norms and makes the updates of a LARS step, and its workspace."""
 
     def __init__(self, chunks: torch.Tensor, n_seg: int, device, lag: int = LARS_LAG):
-        rows, need = self.plan([(s, pos, min(LARS_PIECE, begin + ln - pos)) for s, begin, ln in chunks.tolist()
-                                for pos in range(begin, begin + ln, LARS_PIECE)], n_seg, lag)
-        self.order = torch.tensor(rows, dtype=torch.int64, device=device).view(-1, 2)
+        seg, begin, ln = chunks.cpu().view(-1, 3).unbind(1)
+        parts = (ln + LARS_PIECE - 1) // LARS_PIECE                    # pieces per chunk
+        at = torch.repeat_interleave(torch.arange(len(parts)), parts)
+        past = (torch.arange(len(at)) - (parts.cumsum(0) - parts)[at]) * LARS_PIECE
+        rows, need = self.plan(torch.stack([seg[at], begin[at] + past, (ln[at] - past).clamp_max(LARS_PIECE)], 1), n_seg, lag)
+        self.order = torch.from_numpy(rows).to(device)
         self.need = torch.tensor(need, dtype=torch.int32, device=device)
         self.n_seg = n_seg
         # not zero once a wait in the kernel has run out; in host memory, where it is read without a synchronisation
@@ -281,20 +284,14 @@ class LarsOrder:
         """Rows ``(segment << 1 | update | length << 32, begin)`` from pieces ``(segment, begin, length)``: a piece's update
         comes after the norms of all pieces of its segment (what makes the kernel's waits end), at the earliest ``lag`` pieces
         after its own norms."""
-        need = [0] * n_seg
-        for s, _, _ in chunks:
-            need[s] += 1
-        last = {s: i for i, (s, _, _) in enumerate(chunks)}
-        rows, out = [], 0
-        for i in range(len(chunks) + lag):
-            if i < len(chunks):
-                s, begin, ln = chunks[i]
-                rows.append((s << 1 | ln << 32, begin))
-            while out < len(chunks) and out + lag <= i and last[chunks[out][0]] <= i:
-                s, begin, ln = chunks[out]
-                rows.append((s << 1 | 1 | ln << 32, begin))
-                out += 1
-        return rows, need
+        seg, begin, ln = torch.as_tensor(chunks, dtype=torch.int64).view(-1, 3).unbind(1)
+        i = torch.arange(len(seg))
+        last = torch.zeros(n_seg, dtype=torch.int64).scatter_reduce_(0, seg, i, "amax")
+        when = torch.maximum(i + lag, last[seg]).cummax(0)[0] if len(seg) else i      # the piece whose norms the update follows
+        norms = torch.stack([seg << 1 | ln << 32, begin], 1)
+        updates = torch.stack([norms[:, 0] | 1, begin], 1)
+        rows = torch.cat([norms, updates])[torch.cat([2 * i, 2 * when + 1]).argsort(stable=True)]
+        return rows.numpy(), torch.bincount(seg, minlength=n_seg).tolist()
 
 
 class Hyper(ctypes.Structure):
