@@ -14,7 +14,8 @@
 //               shared memory; O is rescaled only when a row's maximum has grown by more than 2^8 since the last time (O and
 //               the row sum carry the same factor until the division at the end).  The output leaves by TMA through the memory
 //               of the item's queries (stored by the threads: 70 us where this takes 58).
-// A batch entry whose keys are all switched off attends to all of them.  Tensor memory: S 2 x 128 columns, P 2 x 64, O 2 x 64.
+// A batch entry whose keys are all switched off attends to all of them, as it does in the library.  Keys and values that are off are not
+// read where a whole tile of them is, so that an infinite or NaN one there has no part in anything.  Tensor memory: S 2 x 128 columns, P 2 x 64, O 2 x 64.
 // Every mbarrier wait is bounded; a wait that runs out sets *status and all roles leave their loops.
 #include <cuda.h>
 #include <math.h>
@@ -158,7 +159,7 @@ attn_heads_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       uint32_t active = 0;
       for (int j = 0; j < n_tiles; ++j)
         if (mrow == nullptr || __any_sync(0xffffffffu, nibble(j) != 0)) active |= 1u << j;
-      if (active == 0) {                       // no key at all: as without a mask, which is what the library's kernel gives here
+      if (active == 0) {                       // no key at all: as without a mask, which is what the library's kernel gives from two keys on
         mrow = nullptr;
         active = n_tiles == 32 ? 0xffffffffu : (1u << n_tiles) - 1;
       }

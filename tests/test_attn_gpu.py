@@ -72,6 +72,30 @@ def test_heads_forward_without_any_key():
     assert torch.equal(attention.heads_fwd(q, k, v, mask)[1], attention.heads_fwd(q, k, v)[1])
 
 
+@pytest.mark.parametrize("nq,nk", [(300, 300), (64, 64), (40, 2), (1, 384), (128, 127), (40, 1)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_attention_without_any_key_is_what_the_library_gives(nq, nk, packed):
+    """Forwards with a gradient go to the library, those without one to the kernel: a batch entry whose keys are all off gives
+    the same in both."""
+    from tspipe_b200.ops import attention
+    torch.manual_seed(6)
+    dev = torch.device("cuda", 0)
+    n = max(nq, nk)
+    q, k, v = (torch.randn(3, n, 3, 2, 64, device=dev).bfloat16().permute(2, 0, 3, 1, 4) if packed else
+               torch.randn(3, 3, 2, n, 64, device=dev).bfloat16())
+    q, k, v = q[:, :, :nq], k[:, :, :nk], v[:, :, :nk]
+    mask = torch.rand(3, 1, 1, nk, device=dev) < 0.5
+    mask[..., -1] = True
+    mask[1] = False
+    want = F.scaled_dot_product_attention(q, k, v, attn_mask=mask)
+    with torch.no_grad():
+        got = attention.attention(q, k, v, mask)
+    grad = attention.attention(q.detach().requires_grad_(), k, v, mask).detach()
+    assert float((grad.double() - want.double()).norm()) <= 2 * 2 ** -8 * float(want.double().norm())
+    for a, b in zip(got.double(), want.double()):
+        assert float((a - b).norm()) <= 2 * 2 ** -8 * float(b.norm())       # (zeros: equal)
+
+
 def test_heads_forward_leaves_the_rest_to_the_library():
     from tspipe_b200.ops import attention
     dev = torch.device("cuda", 0)
