@@ -96,6 +96,28 @@ def test_attention_without_any_key_is_what_the_library_gives(nq, nk, packed):
         assert float((a - b).norm()) <= 2 * 2 ** -8 * float(b.norm())       # (zeros: equal)
 
 
+def test_attention_is_seen_by_traces_modes_and_autocast():
+    from torch.utils.flop_counter import FlopCounterMode
+    from tspipe_b200.ops import attention
+    dev = torch.device("cuda", 0)
+    q, k, v = (torch.randn(2, 3, 40, 64, device=dev).bfloat16() for _ in range(3))
+    mask = torch.arange(40, device=dev)[None, None, None] < torch.tensor([40, 17], device=dev).view(2, 1, 1, 1)
+    call = lambda q, k, v, mask: attention.attention(q, k, v, mask)      # noqa: E731
+    want = F.scaled_dot_product_attention(v, q, k, attn_mask=mask)
+    with torch.no_grad():
+        traced = torch.jit.trace(call, (q, k, v, mask), check_trace=False)
+        assert torch.equal(traced(v, q, k, mask), want)
+        compiled = torch.compile(call, backend="eager", fullgraph=True)
+        assert torch.equal(compiled(v, q, k, mask), want)
+        with FlopCounterMode(display=False) as flops:
+            call(q, k, v, mask)
+        assert flops.get_total_flops() > 0
+        with torch.autocast("cuda", dtype=torch.float16):
+            assert call(q, k, v, mask).dtype == torch.float16
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            assert torch.equal(call(q, k, v, mask), attention.heads_fwd(q, k, v, mask))
+
+
 def test_heads_forward_leaves_the_rest_to_the_library():
     from tspipe_b200.ops import attention
     dev = torch.device("cuda", 0)

@@ -189,11 +189,18 @@ def heads_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: Optional[
     return o.transpose(1, 2)
 
 
+def _observed() -> bool:
+    """Whether something other than the device is to see the call: a trace, a compilation, a dispatch mode (which a launch
+    through ctypes would pass by), or autocast to another type than the kernel's."""
+    return (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0
+            or (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.bfloat16))
+
+
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: Optional[torch.Tensor] = None,
               dropout_p: float = 0.0) -> torch.Tensor:
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
     if ((_TCGEN05 or (_TCGEN05 is None and mask is not None)) and dropout_p == 0.0 and not needs_grad and q.is_cuda
-            and k.shape[-2] > 1):      # (a single key that is off: the library gives zeros)
+            and not _observed() and k.shape[-2] > 1):      # (a single key that is off: the library gives zeros)
         o = heads_fwd(q, k, v, mask)
         if o is not None:
             return o
