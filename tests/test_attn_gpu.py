@@ -58,7 +58,8 @@ def test_heads_forward(b, h, nq, nk, masked):
     s = (q.double() @ k.double().transpose(-1, -2)) / 8
     want = torch.softmax(s if mask is None else s.masked_fill(~mask, -math.inf), -1) @ v.double()
     assert float((o.double() - want).norm() / want.norm()) < 2 * 2 ** -8
-    if mask is not None and attention._TCGEN05 is None:
+    if mask is not None and nk > 1:
+        attention.set_tcgen05(None)
         with torch.no_grad():
             assert torch.equal(attention.attention(q, k, v, mask), o)
 
@@ -134,8 +135,8 @@ def test_heads_forward_leaves_the_rest_to_the_library():
 
 
 def test_attention_dispatch_and_vit_block_without_grad():
-    """A ViT block gives the same result through the three attention paths: tcgen05 kernel (no gradient needed,
-    opt-in), the library's fused attention on unbound q / k / v, and the packed-qkv library entry point."""
+    """A ViT block gives the same result through the three attention paths: tcgen05 kernel (no gradient needed, without a
+    mask on request), the library's fused attention on unbound q / k / v, and the packed-qkv library entry point."""
     from tspipe_b200.models.vit import CONFIGS, Block
     from tspipe_b200.ops import attention, gemm
     torch.manual_seed(1)
@@ -155,7 +156,7 @@ def test_attention_dispatch_and_vit_block_without_grad():
             attention.set_qkv_mode("split")
             y_split = blk(x)                             # three projection GEMMs + library attention
     finally:
-        attention.set_tcgen05(False)
+        attention.set_tcgen05(None)
         attention.set_packed(None)
         attention.set_qkv_mode("split")
     gemm.check_status()
@@ -175,6 +176,52 @@ def test_attention_dispatch_and_vit_block_without_grad():
             attention.set_qkv_mode("split")
     for a, b in zip(grads["split"], grads["packed"]):
         torch.testing.assert_close(a, b, rtol=5e-2, atol=5e-2 * b.abs().max().item())
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+@pytest.mark.parametrize("b,l", [(3, 50), (2, 300), (9, 128)])
+def test_encoder_layer_of_a_frozen_teacher(b, l, recorded):
+    """A BERT layer with heads of 64 and a padding mask, without a gradient, eagerly and replayed on new inputs: attention runs on
+    the kernel and differs from the library's as one rounding of the attention does from another."""
+    from tspipe_b200.models.bert import BertConfig, EncoderLayer
+    from tspipe_b200.ops import attention, fused, gemm
+    from tspipe_b200.runtime.stage_graph import capture
+    torch.manual_seed(7)
+    dev = torch.device("cuda", 0)
+    m = EncoderLayer(BertConfig(hidden=256, heads=4, ffn=1024)).to(dev).eval()
+
+    def inputs():
+        lens = torch.randint(max(1, l // 3), l + 1, (b, 1), device=dev)
+        return torch.randn(b, l, 256, device=dev).bfloat16(), (torch.arange(l, device=dev)[None] < lens).long()
+
+    def run(x, mask):
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False):
+            return m({"hidden": x, "mask": mask})["hidden"]
+
+    x, mask = inputs()
+    counts = {}
+    try:
+        for flag in (None, False):
+            attention.set_tcgen05(flag)
+            run(x, mask)
+            before = fused.LAUNCHES
+            run(x, mask)
+            counts[flag] = fused.LAUNCHES - before
+        want_in = inputs()
+        want = run(*want_in)                                # the library's attention
+    finally:
+        attention.set_tcgen05(None)
+    assert counts[None] == counts[False] + 1
+    if recorded:
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        got = capture(graph, stream, torch.cuda.graph_pool_handle(), lambda: run(x, mask))
+        x.copy_(want_in[0])
+        mask.copy_(want_in[1])
+        graph.replay()
+    else:
+        got = run(*want_in)
+    gemm.check_status()
+    assert float((got.double() - want.double()).norm() / want.double().norm()) < 2 * 2 ** -8
 
 
 def test_patch_embedding_as_gemm_matches_convolution():
