@@ -293,3 +293,76 @@ def test_kernels_that_start_early_wait_for_what_they_read(mode):
             torch.cuda.synchronize()
             assert torch.isfinite(want).all() and torch.equal(got, want)
     gemm.check_status()
+
+
+def _module_of_early_kernels(kind, dev):
+    """A fused block and its input: what convolutions and products follow directly, and their gradients."""
+    from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
+    from tspipe_b200.models.resnet import Bottleneck, mlp_head_children
+    from tspipe_b200.models.vit import Block, ViTConfig
+    from tspipe_b200.runtime.fuse import fuse_partition
+    torch.manual_seed(43)
+    if kind == "vit block":
+        m, x = Block(ViTConfig(embed_dim=384, num_heads=6)), torch.randn(16, 65, 384, device=dev).bfloat16()
+    elif kind == "head":
+        m, x = nn.Sequential(mlp_head_children(512, 1024, 256)), torch.randn(512, 512, device=dev).bfloat16()
+    else:                                     # the addend of the first data gradient: on a flat pixel grid, on a strided one
+        down = None if kind == "block" else nn.Sequential(nn.Conv2d(256, 512, 1, stride=2, bias=False), nn.BatchNorm2d(512))
+        m = nn.Sequential(Bottleneck(256, 64, 1, None) if down is None else Bottleneck(256, 128, 2, down))
+        x = torch.randn(16, 256, 28, 28, device=dev).to(dtype=torch.bfloat16, memory_format=torch.channels_last)
+    m = fuse_partition(DeferredBatchNorm.convert_deferred_batch_norm(m.to(dev).to(memory_format=torch.channels_last), chunks=1))
+    return m, BatchNormGroup(m, chunks=1), x
+
+
+@pytest.mark.parametrize("mode", ["stream", "graph"])
+@pytest.mark.parametrize("kind", ["block", "strided block", "head", "vit block"])
+def test_kernels_that_start_early_behind_normalisations(kind, mode, monkeypatch):
+    """Forward and backward of blocks in which normalisations and GELU let convolutions, products and weight gradients start
+    as soon as they are placed themselves, on one input buffer that every pass overwrites: what a run with a synchronisation
+    after each call gives.  Sums that atomics add up differ in their last bits, and a value next to a ReLU's corner may take its gradient
+    along; a tile that was read too early is a share of some 10^-2 of a tensor's elements, far off."""
+    from tspipe_b200.ops import bn, conv, fused, gemm
+    from tspipe_b200.runtime.stage_graph import capture
+    dev = torch.device("cuda", 0)
+    m, group, x0 = _module_of_early_kernels(kind, dev)
+    buf, params = torch.empty_like(x0).requires_grad_(), list(m.parameters())
+    g = None
+
+    def chain():
+        nonlocal g
+        out = []
+        for i in range(3):
+            with torch.no_grad():
+                buf.copy_(x0.roll(i, 0) * (i + 1))
+            with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False), bn.segments(2):
+                y = m(buf)
+            if g is None:
+                g = torch.randn(y.shape, device=dev).to(y.dtype)
+                g = g.to(memory_format=torch.channels_last) if g.dim() == 4 else g
+            grads = torch.autograd.grad(y, [buf] + params, g)
+            # (without the gradient of a bias in front of a BatchNorm, which is rounding alone)
+            out += [y.detach()] + [t for j, t in enumerate(grads) if (kind, j) != ("head", 2)]
+        return out
+
+    count = fused._count
+    with monkeypatch.context() as patch:
+        patch.setattr(fused, "_count", lambda *a: (count(*a), torch.cuda.synchronize())[0])
+        chain()
+        want = [t.clone() for t in chain()]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        conv.clear_weight_cache()
+        gemm.clear_weight_cache()
+        if mode == "stream":
+            got = chain()
+        else:
+            graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+            got = capture(graph, stream, torch.cuda.graph_pool_handle(), chain)
+            graph.replay()
+            graph.replay()
+        torch.cuda.synchronize()
+        gemm.check_status()
+        for a, b in zip(got, want):
+            rms = b.float().square().mean().sqrt()
+            off = ((a.float() - b.float()).abs() > 0.5 * rms).float().mean()
+            assert b.isfinite().all() and float(rms) > 0 and float(off) < 2e-3, (kind, tuple(b.shape), float(off))
