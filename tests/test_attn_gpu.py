@@ -97,6 +97,28 @@ def test_attention_without_any_key_is_what_the_library_gives(nq, nk, packed):
         assert float((a - b).norm()) <= 2 * 2 ** -8 * float(b.norm())       # (zeros: equal)
 
 
+@pytest.mark.parametrize("nk", [4096, 4097, 9000])
+def test_attention_on_request_at_any_number_of_keys(nk, monkeypatch):
+    from tspipe_b200.ops import attention, gemm
+    torch.manual_seed(8)
+    dev = torch.device("cuda", 0)
+    q, k, v = (torch.randn(2, 3, n, 64, device=dev).bfloat16() for n in (130, nk, nk))
+    kernel, calls = {}, []
+    for name in ("heads_fwd", "flash_fwd"):
+        kernel[name] = getattr(attention, name)
+        monkeypatch.setattr(attention, name, lambda *a, name=name: [calls.append(name), kernel[name](*a)][1])
+    attention.set_tcgen05(True)
+    try:
+        with torch.no_grad():
+            o = attention.attention(q, k, v)
+    finally:
+        attention.set_tcgen05(None)
+    gemm.check_status()
+    assert calls == (["heads_fwd"] if nk <= 4096 else ["heads_fwd", "flash_fwd"])
+    want = torch.softmax(q.double() @ k.double().transpose(-1, -2) / 8, -1) @ v.double()
+    assert float((o.double() - want).norm() / want.norm()) < 2 * 2 ** -8
+
+
 def test_attention_is_seen_by_traces_modes_and_autocast():
     from torch.utils.flop_counter import FlopCounterMode
     from tspipe_b200.ops import attention

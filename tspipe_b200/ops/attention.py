@@ -18,7 +18,8 @@ from typing import Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-# Forwards without a gradient on :func:`heads_fwd`: None = those with a mask, True = all, False = none.  The library turns a
+# Forwards without a gradient on :func:`heads_fwd`: None = those with a mask, True = all (without a mask from 4097 keys on by
+# :func:`flash_fwd`), False = none.  The library turns a
 # mask into an additive matrix, which costs it more than the attention: [32, 12, 512, 64] 110 us with a padding mask and 45
 # without one, the kernel 58 and 57; [64, 12, 197, 64] without a mask 32 and 40.
 _TCGEN05: Optional[bool] = None
@@ -202,6 +203,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: Optional[
     if ((_TCGEN05 or (_TCGEN05 is None and mask is not None)) and dropout_p == 0.0 and not needs_grad and q.is_cuda
             and not _observed() and k.shape[-2] > 1):      # (a single key that is off: the library gives zeros)
         o = heads_fwd(q, k, v, mask)
+        if o is None and _TCGEN05 and mask is None and k.shape[-2] > 4096 and q.shape[-1] == 64 and flash_eligible(q, k, v):
+            o = flash_fwd(q, k, v)[0]              # (more keys than the other kernel's masks and tiles are made for)
         if o is not None:
             return o
     return F.scaled_dot_product_attention(q, k, v, attn_mask=mask, dropout_p=dropout_p)
