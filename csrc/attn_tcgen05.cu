@@ -513,8 +513,8 @@ __global__ void __launch_bounds__(256) nce_prepare_kernel(const NcePairs<T> in, 
 // lse and o come from rows q~, k~ rounded to bf16.  What the rounding of the row's own query and key does to lse is added to
 // first order, ((q^ - q~).o + p (k^ - k~).q~) / T with p the probability of the row's own key; q^.k^ and the gradient's k^ are
 // taken as they are.  Error of the loss and of the gradient against 64 bits, 256 rows: 6e-6 and 2.8e-3 with rounded rows
-// throughout (and as much with the logits in memory), 3e-7 and 1.7e-3 this way, in the same time.  At most a block per SM and pair:
-// every block ends in two additions to the same memory, one after the other at some 15 ns (2 x 4096 rows in two
+// throughout (and as much with the logits in memory), 3e-7 and 1.7e-3 this way, in the same time.  At most a block per SM, half of
+// them per pair: every block ends in two additions to the same memory, one after the other at some 15 ns (2 x 4096 rows in two
 // chunks: 20.8 us with 512 blocks, 14.9 this way).
 template <typename T>
 __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
@@ -592,8 +592,10 @@ int launch_nce_pair(const NcePairs<T>& in, int n, int chunk, int chunks, float t
   const int rc = launch<256, 256, 64, true, float>(q16, srcs, 1, k16, o, lse, 2, chunks, n, chunk, sq, sk, sk, so,
                                                    1.f / temp, 1.f / temp, 1, status, stream, n);
   if (rc != 0) return rc;
+  int sms = 0;
+  if (cudaError_t e = tsp::usable_sms(sms); e != cudaSuccess) return (int)e;
   const int blocks = (n + kNceRows - 1) / kNceRows;
-  nce_finish_kernel<T><<<dim3(blocks < 74 ? blocks : 74, 2), 32 * kNceRows, 0, stream>>>(
+  nce_finish_kernel<T><<<dim3(blocks < sms / 2 ? blocks : sms / 2, 2), 32 * kNceRows, 0, stream>>>(
       in, n, n_pad, chunks, temp, (const __nv_bfloat16*)q16, (const __nv_bfloat16*)k16, o, lse, sum, loss, (T*)gq);
   return TSP_LAUNCH_CHECK();
 }

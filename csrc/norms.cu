@@ -440,7 +440,9 @@ int tsp_gelu_bwd_sums(const void* dy, const void* x, const float* bias, void* dx
   if (bias == nullptr || ((uintptr_t)bias & 15) != 0) return -2;
   const int slabs = (d + 255) / 256;
   int64_t blocks = (rows + kGeluSumRows * kGeluSumVecs - 1) / (kGeluSumRows * kGeluSumVecs);
-  const int64_t most = (148 * 6 + slabs - 1) / slabs;                  // six blocks per SM
+  int sms = 0;
+  if (cudaError_t e = tsp::usable_sms(sms); e != cudaSuccess) return (int)e;
+  const int64_t most = (sms * 6 + slabs - 1) / slabs;                  // six blocks per SM
   if (blocks > most) blocks = most;
   const dim3 grid((unsigned)slabs, (unsigned)blocks);
   if (dtype == TSP_DTYPE_BF16)
