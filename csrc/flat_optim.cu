@@ -199,7 +199,8 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
 // resident blocks, the earliest unfinished row never waits.  sync[0] = ticket, sync[1 + seg] = pieces of the segment whose
 // norms are in, sync[1 + n_seg] = a wait ran out; `need` = pieces per segment.  After a wait that ran out the step still ends: the
 // segment's ratio is NaN then, and with it what is left to update of the segment, and *status (host memory) is set, which the
-// optimizer raises on.  Bound by DRAM (p, g, mu, t once in, p, mu, t once out: 5.0 TB/s of it).  A step
+// optimizer raises on.  Bound by DRAM (p, g, mu, t once in, p, mu, t once out: 5.0 TB/s of it; by the counters L2 keeps some two
+// fifths of p and g until the update, the rest is read again).  A step
 // over 25.6 M parameters with the teacher, microseconds: two launches 160, this one 144; without the teacher 127 and 109; 86 M
 // 494 and 463; 6 M (96 MB) 42 and 40.  Pieces of 32 KB and four blocks of 256 threads per SM: with pieces of 64 KB 147, of 16
 // KB 152; two blocks of 512 threads 149; three blocks of 256 159.

@@ -105,11 +105,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
-// The MMA-issuing thread is the one serial resource of these kernels (an issue costs it about 50 cycles), so its loop
-// works on 32-bit halves of the matrix descriptors: the high word (stride byte offset 1024, version, 128-byte swizzle)
-// is the same constant for K-major and MN-major tiles, the low word is (address >> 4) plus the leading-byte-offset
-// field, and stepping through a tile only ever adds to the low word (shared-memory addresses stay below 2^18, so the
-// 14-bit address field cannot carry).
+// The MMA-issuing thread is the one serial resource of these kernels (an issue costs it about 50 cycles behind
+// `if (lane == 0)`, a fraction of that from an elected lane, see elect_one), so its loop works on 32-bit halves of the
+// matrix descriptors: the high word (stride byte offset 1024, version, 128-byte swizzle) is the same constant for K-major
+// and MN-major tiles, the low word is (address >> 4) plus the leading-byte-offset field, and stepping through a tile only
+// ever adds to the low word (shared-memory addresses stay below 2^18, so the 14-bit address field cannot carry).
 constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo_k_major(uint32_t smem_addr) { return (smem_addr >> 4) | (1u << 16); }
 __device__ __forceinline__ uint32_t desc_lo_mn_major(uint32_t smem_addr, uint32_t lbo) {
