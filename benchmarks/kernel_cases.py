@@ -122,11 +122,15 @@ def case_stem():
     torch.backends.cudnn.benchmark = True
     t = _time(lambda: conv.stem_conv(x, w), n=10, flush=flush)
     tr = _time(lambda: F.conv2d(x, wb, stride=2, padding=3), n=10, flush=flush)
+    wp = w.clone().requires_grad_()
+    y, _ = conv.stem_conv(x, wp, want_sums=False)
+    g = torch.randn_like(y)
+    tw = _time(lambda: torch.autograd.grad(y, wp, g, retain_graph=True), n=10, flush=flush)
     gemm.check_status()
     out_bytes = 128 * 64 * 112 * 112 * 2
     flops = 2 * 128 * 112 * 112 * 64 * 147
     print(f"stem conv 7x7/2 [128,3,224,224]: {t:8.1f} us  ({(out_bytes + x.numel() * 2) / t / 1e6:5.2f} TB/s, "
-          f"{flops / t / 1e6:6.1f} TFLOP/s)   library: {tr:8.1f} us")
+          f"{flops / t / 1e6:6.1f} TFLOP/s)   library: {tr:8.1f} us   weight gradient {tw:8.1f} us")
 
 
 def case_lars():
@@ -144,7 +148,7 @@ def case_lars():
     t = _time(opt.step, flush=flush)
     n = flat.total
     print(f"lars+ema step over {n / 1e6:.1f} M params: {t:8.1f} us  {n * 4 * 9 / t / 1e6:5.2f} TB/s "
-          "(norms: read p,g; apply: read p,g,mu,t write p,mu,t)")
+          "(read p,g twice, mu,t; write p,mu,t; the second read of p,g from L2 where norms and updates are one launch)")
 
 
 def case_ema():
@@ -160,11 +164,12 @@ def case_ema():
 def case_kd():
     from tspipe_b200.ops import fused
     dev = torch.device("cuda")
-    s = torch.randn(2048, 1000, device=dev).bfloat16().requires_grad_()
-    tt = torch.randn(2048, 1000, device=dev).bfloat16()
-    y = torch.randint(0, 1000, (2048,), device=dev)
+    n, c = (int(v) for v in sys.argv[2:4]) if len(sys.argv) > 3 else (2048, 1000)
+    s = torch.randn(n, c, device=dev).bfloat16().requires_grad_()
+    tt = torch.randn(n, c, device=dev).bfloat16()
+    y = torch.randint(0, c, (n,), device=dev)
     t = _time(lambda: fused.kd_soft_target_loss(s, tt, y, 4.0, 1.0, 1.0))
-    print(f"kd loss [2048,1000] fwd+grad: {t:8.1f} us")
+    print(f"kd loss [{n},{c}] fwd+grad: {t:8.1f} us")
 
 
 def case_ln():
@@ -246,23 +251,45 @@ def case_infonce():
           f"{tr:7.1f} us")
 
 
+def case_moco():
+    """Both directions of the contrastive loss of two views, forward and backward: device time of the replayed graph."""
+    from tspipe_b200 import losses
+    dev = torch.device("cuda")
+    n = int(sys.argv[2]) if len(sys.argv) > 2 else 4096
+    o1, o2, t1, t2 = (torch.randn(n, 256, device=dev).bfloat16() for _ in range(4))
+    o1.requires_grad_()
+    o2.requires_grad_()
+
+    def step():
+        return torch.autograd.grad(losses.moco_loss(o1, o2, t1, t2), [o1, o2])
+    for _ in range(3):
+        step()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        step()
+    print(f"moco loss [{n},256], both views, fwd+bwd on the device: {_time(g.replay, n=10):7.1f} us")
+
+
 def case_attn():
-    """ViT-B attention forward, batch 256 x 12 heads x 197 tokens x 64: tcgen05 kernel against the library."""
+    """Attention forward: tcgen05 kernel against the library, a BERT layer's with a padding mask (a quarter of the keys off) and
+    a ViT-B layer's without one."""
     import torch.nn.functional as F
     from tspipe_b200.ops import attention, gemm
     dev = torch.device("cuda")
-    b, h, n, dh = 256, 12, 197, 64
-    qkv = torch.randn(b, n, 3, h, dh, device=dev).bfloat16()
-    q, k, v = qkv.permute(2, 0, 3, 1, 4)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
-    with torch.no_grad():
-        t = _time(lambda: attention.flash_fwd(q, k, v), n=10, flush=flush)
-        tr = _time(lambda: F.scaled_dot_product_attention(q, k, v), n=10, flush=flush)
-    gemm.check_status()
-    flops = 4 * b * h * n * n * dh
-    byts = 4 * b * h * n * dh * 2
-    print(f"attention fwd [{b},{h},{n},{dh}]: {t:7.1f} us ({flops / t / 1e6:6.1f} TFLOP/s, {byts / t / 1e6:5.2f} TB/s) | "
-          f"library {tr:7.1f} us")
+    for b, h, n, dh, masked in ((32, 12, 512, 64, True), (64, 12, 197, 64, False)):
+        q, k, v = torch.randn(b, n, 3, h, dh, device=dev).bfloat16().permute(2, 0, 3, 1, 4)
+        lens = torch.randint(n // 2, n + 1, (b, 1), device=dev)
+        mask = (torch.arange(n, device=dev)[None] < lens)[:, None, None] if masked else None
+        with torch.no_grad():
+            t = _time(lambda: attention.heads_fwd(q, k, v, mask), n=10, flush=flush)
+            tr = _time(lambda: F.scaled_dot_product_attention(q, k, v, attn_mask=mask), n=10, flush=flush)
+        gemm.check_status()
+        flops = 4 * b * h * n * n * dh
+        byts = 4 * b * h * n * dh * 2
+        print(f"attention fwd [{b},{h},{n},{dh}]{' masked' if masked else ''}: {t:7.1f} us ({flops / t / 1e6:6.1f} TFLOP/s of "
+              f"all keys, {byts / t / 1e6:5.2f} TB/s) | library {tr:7.1f} us")
 
 
 # 1x1 / 3x3 convolutions of ResNet-50 at 224 x 224: (cin, cout, kernel, stride, input side, how many)
@@ -400,4 +427,4 @@ def case_dp():
 
 if __name__ == "__main__":
     {"bn": case_bn, "bn_r50": case_bn_r50, "stem": case_stem, "lars": case_lars, "ema": case_ema, "kd": case_kd, "ln": case_ln, "gemm": case_gemm,
-     "infonce": case_infonce, "attn": case_attn, "conv": case_conv, "conv1": case_conv1, "dp": case_dp}[sys.argv[1]]()
+     "infonce": case_infonce, "moco": case_moco, "attn": case_attn, "conv": case_conv, "conv1": case_conv1, "dp": case_dp}[sys.argv[1]]()
