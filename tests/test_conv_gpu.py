@@ -60,6 +60,27 @@ def test_stem_conv_rows_and_runs(n, h, w):
             torch.testing.assert_close(sums, want, rtol=1e-4, atol=1e-4 * float(want.abs().max()))
 
 
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan, 9.2e-41, 1.2e-38, 3e38])
+def test_stem_conv_weights_that_cannot_be_halved_blindly(value):
+    """The middle tap of a row is in two products with half its weight each: infinite, NaN, subnormal (odd) and large weights."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(6)
+    dev = torch.device("cuda", 0)
+    x = torch.randn(2, 3, 12, 24, device=dev).to(dtype=torch.bfloat16, memory_format=torch.channels_last)
+    weight = torch.zeros(64, 3, 7, 7, device=dev)
+    for c in range(3):
+        weight[5 + c, c, 2, 3] = value
+        weight[20, c, 6, 2 + c] = value
+    scale = 2.0 ** 126 if abs(value) < 1e-30 else 2.0 ** -20 if value == 3e38 else 1.0
+    x = (x.double() * scale).to(torch.bfloat16)
+    y, _ = conv.stem_conv(x, weight, want_sums=False)
+    gemm.check_status()
+    ref = F.conv2d(x.double(), weight.bfloat16().double(), stride=2, padding=3)
+    assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isinf(), ref.isinf())
+    ok = ref.isfinite()
+    assert ((y.double() - ref)[ok].abs() <= 2.0 ** -8 * ref[ok].abs()).all() and (math.isfinite(value) == bool(ok.all()))
+
+
 def test_fused_partition_matches_plain_sequential():
     """conv1 -> bn1 -> relu -> maxpool -> linear head -> bn1d -> relu run through FusedSequential give the same
     outputs, gradients and BatchNorm statistics as the plain modules."""
