@@ -22,6 +22,7 @@
 // Every mbarrier wait is bounded; a wait that runs out sets *status and all roles leave their loops.
 #include <cuda.h>
 #include <math.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -469,7 +470,7 @@ int launch(const void* q, void* const* k_srcs, int n_src, const void* v, void* o
 // The passes around the fused contrastive loss of two (queries, keys) pairs.  One warp per row of 256 elements, 8 per
 // lane; blockIdx.y = pair.
 // ---------------------------------------------------------------------------------------------
-constexpr int kNceDim = 256, kNceRows = 32;       // rows (warps) of a block of the last pass
+constexpr int kNceDim = 256;
 template <typename T>
 struct NcePairs {
   const T* q[2];
@@ -514,19 +515,20 @@ __global__ void __launch_bounds__(256) nce_prepare_kernel(const NcePairs<T> in, 
 // first order, ((q^ - q~).o + p (k^ - k~).q~) / T with p the probability of the row's own key; q^.k^ and the gradient's k^ are
 // taken as they are.  Error of the loss and of the gradient against 64 bits, 256 rows: 6e-6 and 2.8e-3 with rounded rows
 // throughout (and as much with the logits in memory), 3e-7 and 1.7e-3 this way, in the same time.  At most a block per SM, half of
-// them per pair: every block ends in two additions to the same memory, one after the other at some 15 ns (2 x 4096 rows in two
-// chunks: 20.8 us with 512 blocks, 14.9 this way).
-template <typename T>
-__global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
+// them per pair, of ROWS warps with a row each at a time: every block ends in two additions to the same memory, one after the
+// other at some 15 ns (2 x 4096 rows in two chunks: 20.8 us with 512 blocks, 14.9 this way).  ROWS 16 while such blocks
+// are enough for all rows: 2 x 256 rows 6.3 us where 32 take 8.6, 2 x 1024 8.5 and 11.2; 2 x 1536, which are not, 14.0 and 10.9.
+template <typename T, int ROWS>
+__global__ void __launch_bounds__(32 * ROWS) nce_finish_kernel(const NcePairs<T> in, int n, int n_pad, int chunks, float temp,
                                                          const __nv_bfloat16* __restrict__ q16,
                                                          const __nv_bfloat16* __restrict__ k16,
                                                          const float* __restrict__ o, const float* __restrict__ lse,
                                                          double* __restrict__ sum, float* __restrict__ loss,
                                                          T* __restrict__ gq) {
-  __shared__ double part[kNceRows];
+  __shared__ double part[ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = lane * 8, pair = blockIdx.y;
   double mine = 0.;
-  for (int row = blockIdx.x * kNceRows + warp; row < n; row += gridDim.x * kNceRows) {
+  for (int row = blockIdx.x * ROWS + warp; row < n; row += gridDim.x * ROWS) {
     float q[8], k[8], qb[8], kb[8], acc[8] = {};
     tsp::ld8(pair ? in.q[1] : in.q[0], (int64_t)row * kNceDim + col, q);
     tsp::ld8(pair ? in.k[1] : in.k[0], (int64_t)row * kNceDim + col, k);
@@ -570,7 +572,7 @@ __global__ void __launch_bounds__(32 * kNceRows) nce_finish_kernel(const NcePair
   if (threadIdx.x == 0) {
     double s = 0.;
 #pragma unroll
-    for (int i = 0; i < kNceRows; ++i) s += part[i];
+    for (int i = 0; i < ROWS; ++i) s += part[i];
     atomicAdd(sum, s);
     __threadfence();
     unsigned* done = reinterpret_cast<unsigned*>(sum + 1);
@@ -594,9 +596,14 @@ int launch_nce_pair(const NcePairs<T>& in, int n, int chunk, int chunks, float t
   if (rc != 0) return rc;
   int sms = 0;
   if (cudaError_t e = tsp::usable_sms(sms); e != cudaSuccess) return (int)e;
-  const int blocks = (n + kNceRows - 1) / kNceRows;
-  nce_finish_kernel<T><<<dim3(blocks < sms / 2 ? blocks : sms / 2, 2), 32 * kNceRows, 0, stream>>>(
-      in, n, n_pad, chunks, temp, (const __nv_bfloat16*)q16, (const __nv_bfloat16*)k16, o, lse, sum, loss, (T*)gq);
+  auto finish = [&](auto rows) {
+    constexpr int kRows = decltype(rows)::value;
+    const int blocks = (n + kRows - 1) / kRows;
+    nce_finish_kernel<T, kRows><<<dim3(blocks < sms / 2 ? blocks : sms / 2, 2), 32 * kRows, 0, stream>>>(
+        in, n, n_pad, chunks, temp, (const __nv_bfloat16*)q16, (const __nv_bfloat16*)k16, o, lse, sum, loss, (T*)gq);
+  };
+  if (n <= 16 * (sms / 2)) finish(std::integral_constant<int, 16>());
+  else finish(std::integral_constant<int, 32>());
   return TSP_LAUNCH_CHECK();
 }
 

@@ -207,7 +207,7 @@ def test_byol_pair_equals_two_single_losses(n, d, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n", [128, 129, 200, 1000, 2048])
+@pytest.mark.parametrize("n", [128, 129, 200, 1000, 1184, 1185, 2048])
 def test_nce_pair_matches_cross_entropy(n, dtype):
     """Ragged query tiles, key chunks whose last one is short."""
     from tspipe_b200.losses import moco_loss
