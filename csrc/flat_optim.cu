@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) lars_apply_kernel(float* __restrict_
 }
 
 // Norms and updates in one launch, for buffers that do not fit L2: a chunk's update follows its norms at a distance that
-// L2 holds, so p and g leave DRAM once.  `order` lists the work: every chunk twice (row = {segment << 1 | update, length,
+// L2 holds, so that what L2 keeps of p and g leaves DRAM once.  `order` lists the work: every chunk twice (row = {segment << 1 | update, length,
 // begin}), its norms and, some chunks after the last norms of its segment, its update.  Blocks draw rows by ticket, so a
 // wait for a segment's norms is a wait for rows that blocks drew before and are working on: whatever the number of
 // resident blocks, the earliest unfinished row never waits.  sync[0] = ticket, sync[1 + seg] = pieces of the segment whose

@@ -119,6 +119,22 @@ def test_attention_on_request_at_any_number_of_keys(nk, monkeypatch):
     assert float((o.double() - want).norm() / want.norm()) < 2 * 2 ** -8
 
 
+@pytest.mark.parametrize("b,n,kernel", [(2, 32, True), (64, 8, False), (64, 32, False), (64, 33, True), (42, 32, True)])
+def test_attention_of_many_short_sequences_stays_with_the_library(b, n, kernel, monkeypatch):
+    from tspipe_b200.ops import attention
+    torch.manual_seed(9)
+    dev = torch.device("cuda", 0)
+    q, k, v = torch.randn(b, n, 3, 12, 64, device=dev).bfloat16().permute(2, 0, 3, 1, 4)
+    mask = (torch.arange(n, device=dev)[None] < torch.randint(1, n + 1, (b, 1), device=dev))[:, None, None]
+    heads_fwd, calls = attention.heads_fwd, []
+    monkeypatch.setattr(attention, "heads_fwd", lambda *a: [calls.append(1), heads_fwd(*a)][1])
+    with torch.no_grad():
+        o = attention.attention(q, k, v, mask)
+    assert bool(calls) == kernel
+    want = torch.softmax((q.double() @ k.double().transpose(-1, -2) / 8).masked_fill(~mask, -math.inf), -1) @ v.double()
+    assert float((o.double() - want).norm() / want.norm()) < 2 * 2 ** -8
+
+
 def test_attention_is_seen_by_traces_modes_and_autocast():
     from torch.utils.flop_counter import FlopCounterMode
     from tspipe_b200.ops import attention

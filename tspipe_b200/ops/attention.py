@@ -23,6 +23,10 @@ import torch.nn.functional as F
 # mask into an additive matrix, which costs it more than the attention: [32, 12, 512, 64] 110 us with a padding mask and 45
 # without one, the kernel 58 and 57; [64, 12, 197, 64] without a mask 32 and 40.
 _TCGEN05: Optional[bool] = None
+# Heads above which sequences of up to 32 tokens stay with the library: a head is an item of the kernel's there, 128 queries and keys
+# whatever they hold.  Masked, [32, 16, 32, 64] 20.9 us either way, [64, 12, 32, 64] 29.1 and the library 27.0, [8, 12, 32, 64]
+# 9.8 and 12.7; of 100 tokens [64, 12] 31.1 and 41.3.
+_FEW_KEYS = 512
 
 
 def set_tcgen05(flag: Optional[bool]) -> None:
@@ -201,7 +205,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: Optional[
               dropout_p: float = 0.0) -> torch.Tensor:
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
     if ((_TCGEN05 or (_TCGEN05 is None and mask is not None)) and dropout_p == 0.0 and not needs_grad and q.is_cuda
-            and not _observed() and k.shape[-2] > 1):      # (a single key that is off: the library gives zeros)
+            and not _observed() and k.shape[-2] > 1      # (a single key that is off: the library gives zeros)
+            and not (k.shape[-2] <= 32 and q.shape[-2] <= 32 and q.numel() > _FEW_KEYS * q.shape[-2] * q.shape[-1])):
         o = heads_fwd(q, k, v, mask)
         if o is None and _TCGEN05 and mask is None and k.shape[-2] > 4096 and q.shape[-1] == 64 and flash_eligible(q, k, v):
             o = flash_fwd(q, k, v)[0]              # (more keys than the other kernel's masks and tiles are made for)
