@@ -6,8 +6,9 @@ The reference models run it unfused - two batched GEMMs, a softmax and a dropout
 key-padding mask broadcastable to [B, 1, 1, N] / [B, H, N, N].
 
 Forward passes that need no gradient (the frozen teacher) with head dimension 64 and a boolean key-padding mask run on the
-tcgen05 kernel of ``csrc/attn_heads_tcgen05.cu`` (:func:`heads_fwd`); everything else goes to the library's fused attention,
-which also provides the backward.
+tcgen05 kernel of ``csrc/attn_heads_tcgen05.cu`` (:func:`heads_fwd`), but for many short sequences, a single key and calls that a
+trace, a dispatch mode or autocast to another type is to see; everything else goes to the library's fused attention, which also
+provides the backward.
 """
 from __future__ import annotations
 
@@ -162,7 +163,9 @@ def heads_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: Optional[
               ) -> Optional[torch.Tensor]:
     """``softmax(q k^T / 8 + mask) v`` for bf16 ``[B, H, N, 64]`` tensors (any strides with a contiguous last dimension)
     without a gradient, as a ``[B, H, Nq, 64]`` view of a ``[B, Nq, H, 64]`` buffer; None where the kernel does not take
-    them.  ``mask``: boolean, True = the key takes part, ``[B or 1, 1, 1, Nk]``."""
+    them.  ``mask``: boolean, True = the key takes part, ``[B or 1, 1, 1, Nk]``; where no key does, all do.  Of keys and values
+    that are off, tiles of 128 are not read: a NaN there is without effect, one in another tile is not (its probability, zero,
+    times NaN)."""
     from . import fused as _f
     from . import gemm as _gemm
     ts = (q, k, v) if mask is None else (q, k, v, mask)
