@@ -585,24 +585,27 @@ __global__ void __launch_bounds__(kBlock, 3) bn_bwd_apply_kernel(const T* __rest
 // ---------------------------------------------------------------------------------------------
 // BatchNorm + ReLU + 3x3 / stride 2 / pad 1 max-pool (the ResNet stem) without the normalised activation in memory.
 //
-// The passes are bound by the arithmetic on every element of x as much as by memory, so it is kept short.
-// Forward: a value and its tap travel as one integer key, the value's bits (not negative behind the ReLU, so they order
-// as integers) above a code that is larger for an earlier tap: the maximum of the keys is the first maximum in (row,
-// column) order, one instruction for three values.  Values are rounded to T before they are compared, so the result is
-// that of the separate passes.  A thread walks kPoolRows output rows of one column and 8 channels and forms each input
-// row's maximum over the three columns once (an odd row is the last of one window and the first of the next).  idx gets
-// the code of the winner, kNoTap where the maximum is zero: there the ReLU passes no gradient.
-// Backward: dy' of an input pixel is gathered from the <= 4 windows it belongs to where it is needed, in the reduction
-// and again in the pass for dx, instead of being scattered to an activation-sized tensor that both would read.  A
-// thread takes a 2 x 2 block of input pixels, which meets exactly the four windows (a, b) .. (a + 1, b + 1), two channels
-// at a time.
+// The passes are bound by the arithmetic on every element of x as much as by memory, so two channels share an instruction
+// wherever bf16 allows it (Duo).  Values are rounded to T before they are compared, so the result is that of the separate
+// passes.
+// Forward: a row's maximum over the three columns, and a window's over the three rows, with the winner's code and its element
+// of x selected by the mask "the first one is the maximum".  A thread walks a strip of output rows of one column and 8 channels
+// (an odd row is the last of one window and the first of the next) and has the next window's rows on their way meanwhile.  idx
+// gets the winner's code, kNoTap where the maximum is zero: there the ReLU passes no gradient.
+// Backward: the gradient meets the winners only, so the two sums need dy and the winners (an output-sized tensor instead of x),
+// as the reduction of a BatchNorm + ReLU over them.  In the pass for dx, dy' of an input pixel is gathered from the <= 4 windows
+// it belongs to, instead of being scattered to an activation-sized tensor.  A thread takes 2 x 2 blocks of input pixels, which
+// meet exactly the four windows (a, b) .. (a + 1, b + 1), down a strip of rows, two channels at a time.
 // A block is kBlock / (c / 8) pixels by all channels (by 2048 of them, blockIdx.z, where there are more).
-// 256 images of 112 x 112 x 64 bf16 (205 MB), B200: forward 178 us as two passes, 139 with a comparison per value, 91 this
-// way; backward 410 us as three passes, 320 with the ReLU mask recomputed from x and one 64-bit division per item, 190.
+// 128 images of 112 x 112 x 64 bf16 (205 MB), B200: forward for a backward 90 us with keys of value and code for each
+// channel, without the winners' elements; 83 this way with them (51 MB more).  Without a backward (64 images) 46 and 32.  Backward:
+// the sums 79 from x and 25 from the winners, dx 109 with a load of four windows per block and 87 this way (floor 75).
 // ---------------------------------------------------------------------------------------------
-constexpr int kPoolRows = 4;
-constexpr uint32_t kNoTap = 0xff;
-__host__ __device__ constexpr uint32_t tap_code(int ky, int kx) { return (uint32_t)((2 - ky) * 4 + 2 - kx); }
+// Codes of the taps, for two channels: a byte each, in the upper half of a 16-bit lane, where every code reads as a bf16 number
+// that is no denormal but for zero, and no NaN: comparisons of bf16 pairs compare codes.
+__host__ __device__ constexpr uint32_t lanes(uint32_t code) { return code << 8 | code << 24; }
+constexpr uint32_t kNoTap = lanes(0xff);
+__host__ __device__ constexpr uint32_t tap_code(int ky, int kx) { return lanes((uint32_t)((2 - ky) * 4 + 2 - kx)); }
 
 // Unsigned division of numbers below 2^31 by a constant of the launch: multiply-high and shift (Granlund and Montgomery).
 struct FastDiv {
@@ -616,52 +619,55 @@ struct FastDiv {
 
 struct PoolGeom {
   int n, h, w, c, ho, wo;      // images of one segment, extents
-  FastDiv by_wo, by_rows;      // by_rows: strips of kPoolRows output rows (forward), output rows (backward)
-  uint32_t items;              // pixels or strips of pixels of one segment
+  int rows;                    // output rows of a strip, which a thread walks from top to bottom
+  FastDiv by_wo, by_strips;    // by_strips: strips of an image
+  uint32_t items;              // strips of one column each, of one segment
 };
 
-// Elements 2j and 2j + 1 of a raw vector.
-__device__ __forceinline__ float2 get2(const tsp::Raw8<__nv_bfloat16>& r, int j) {
-  const uint32_t u = reinterpret_cast<const uint32_t*>(&r.a)[j];
-  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-}
-__device__ __forceinline__ float2 get2(const tsp::Raw8<float>& r, int j) { return reinterpret_cast<const float2*>(&r)[j]; }
-__device__ __forceinline__ void set2(tsp::Raw8<__nv_bfloat16>& r, int j, float2 v) {
-  reinterpret_cast<__nv_bfloat162*>(&r.a)[j] = __floats2bfloat162_rn(v.x, v.y);
-}
-__device__ __forceinline__ void set2(tsp::Raw8<float>& r, int j, float2 v) { reinterpret_cast<float2*>(&r)[j] = v; }
-template <typename T>
-__device__ __forceinline__ float2 round2(float2 v) {
-  if constexpr (sizeof(T) == 2) v = __bfloat1622float2(__floats2bfloat162_rn(v.x, v.y));
-  return v;
-}
-
-// Keys of max(v, 0) for two values: bf16 bits << 16 | code, fp32 bits << 32 | code.
-template <typename T> struct PoolKey;
-template <> struct PoolKey<__nv_bfloat16> {
-  using K = uint32_t;
-  static __device__ __forceinline__ void make(float2 v, uint32_t code, K& k0, K& k1) {
-    const __nv_bfloat162 p = __hmax2(__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(0.f, 0.f));
-    const uint32_t u = *reinterpret_cast<const uint32_t*>(&p);
-    k0 = __byte_perm(u, code, 0x1054);
-    k1 = __byte_perm(u, code, 0x3254);
+// Two neighbouring channels: values as T holds them, and masks to select by.
+template <typename T> struct Duo;
+template <> struct Duo<__nv_bfloat16> {
+  using V = uint32_t;
+  using M = uint32_t;
+  static __device__ __forceinline__ __nv_bfloat162 h(V v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
+  static __device__ __forceinline__ V u(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
+  static __device__ __forceinline__ V get(const tsp::Raw8<__nv_bfloat16>& r, int j) { return reinterpret_cast<const uint32_t*>(&r.a)[j]; }
+  static __device__ __forceinline__ void set(tsp::Raw8<__nv_bfloat16>& r, int j, V v) { reinterpret_cast<uint32_t*>(&r.a)[j] = v; }
+  static __device__ __forceinline__ tsp::Pair wide(V v) { return tsp::unpack2(v); }
+  static __device__ __forceinline__ V round(tsp::Pair p) {
+    float a, b;
+    p.split(a, b);
+    return u(__floats2bfloat162_rn(a, b));
   }
-  static __device__ __forceinline__ K max3(K a, K b, K c) { return __vimax3_u32(a, b, c); }
-  static __device__ __forceinline__ bool zero(K k) { return k < 0x10000u; }
-  static __device__ __forceinline__ void set2(tsp::Raw8<__nv_bfloat16>& r, int j, K k0, K k1) {
-    reinterpret_cast<uint32_t*>(&r.a)[j] = __byte_perm(k0, k1, 0x7632);
-  }
+  static __device__ __forceinline__ V lowest() { return 0xff80ff80u; }
+  static __device__ __forceinline__ V larger(V a, V b) { return u(__hmax2(h(a), h(b))); }
+  static __device__ __forceinline__ V sum(V a, V b) { return u(__hadd2(h(a), h(b))); }
+  static __device__ __forceinline__ M equal(V a, V b) { return __heq2_mask(h(a), h(b)); }
+  static __device__ __forceinline__ M same_code(uint32_t a, uint32_t b) { return __heq2_mask(h(a), h(b)); }
+  static __device__ __forceinline__ V pick(M m, V a, V b) { return (m & a) | (~m & b); }
+  static __device__ __forceinline__ V keep(M m, V a) { return m & a; }
+  static __device__ __forceinline__ uint32_t pick_code(M m, uint32_t a, uint32_t b) { return (m & a) | (~m & b); }
 };
-template <> struct PoolKey<float> {
-  using K = unsigned long long;
-  static __device__ __forceinline__ void make(float2 v, uint32_t code, K& k0, K& k1) {
-    k0 = (K)__float_as_uint(fmaxf(v.x, 0.f) + 0.f) << 32 | code;
-    k1 = (K)__float_as_uint(fmaxf(v.y, 0.f) + 0.f) << 32 | code;
+template <> struct Duo<float> {
+  using V = float2;
+  struct M { bool a, b; };
+  static __device__ __forceinline__ V get(const tsp::Raw8<float>& r, int j) { return reinterpret_cast<const float2*>(&r)[j]; }
+  static __device__ __forceinline__ void set(tsp::Raw8<float>& r, int j, V v) { reinterpret_cast<float2*>(&r)[j] = v; }
+  static __device__ __forceinline__ tsp::Pair wide(V v) { return tsp::Pair(v.x, v.y); }
+  static __device__ __forceinline__ V round(tsp::Pair p) {
+    float2 v;
+    p.split(v.x, v.y);
+    return v;
   }
-  static __device__ __forceinline__ K max3(K a, K b, K c) { return max(max(a, b), c); }
-  static __device__ __forceinline__ bool zero(K k) { return (k >> 32) == 0; }
-  static __device__ __forceinline__ void set2(tsp::Raw8<float>& r, int j, K k0, K k1) {
-    reinterpret_cast<float2*>(&r)[j] = make_float2(__uint_as_float((uint32_t)(k0 >> 32)), __uint_as_float((uint32_t)(k1 >> 32)));
+  static __device__ __forceinline__ V lowest() { return make_float2(-INFINITY, -INFINITY); }
+  static __device__ __forceinline__ V larger(V a, V b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+  static __device__ __forceinline__ V sum(V a, V b) { return make_float2(a.x + b.x, a.y + b.y); }
+  static __device__ __forceinline__ M equal(V a, V b) { return {a.x == b.x, a.y == b.y}; }
+  static __device__ __forceinline__ M same_code(uint32_t a, uint32_t b) { return {(a & 0xffffu) == (b & 0xffffu), (a >> 16) == (b >> 16)}; }
+  static __device__ __forceinline__ V pick(M m, V a, V b) { return make_float2(m.a ? a.x : b.x, m.b ? a.y : b.y); }
+  static __device__ __forceinline__ V keep(M m, V a) { return make_float2(m.a ? a.x : 0.f, m.b ? a.y : 0.f); }
+  static __device__ __forceinline__ uint32_t pick_code(M m, uint32_t a, uint32_t b) {
+    return __byte_perm(m.a ? a : b, m.b ? a : b, 0x7610);
   }
 };
 template <typename T>
@@ -687,9 +693,11 @@ struct PoolThread {
   }
 };
 
-template <typename T>
+// WIN: with idx and won, for the backward.
+template <typename T, bool WIN>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 2 ? 3 : 2) bn_relu_pool_kernel(const T* __restrict__ x, T* __restrict__ y,
-                                                              uint8_t* __restrict__ idx, const float* __restrict__ sums,
+                                                              uint8_t* __restrict__ idx, T* __restrict__ won,
+                                                              const float* __restrict__ sums,
                                                               const float* __restrict__ wgt,
                                                               const float* __restrict__ bias,
                                                               float* __restrict__ save_mean_rstd,
@@ -697,13 +705,13 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 2 ? 3 : 2) bn_relu_pool_k
                                                               float* __restrict__ acc_count, int64_t acc_seg_stride,
                                                               const PoolGeom g, float eps) {
   tsp::let_next_start();
-  using P = PoolKey<T>;
-  using K = typename P::K;
+  using D = Duo<T>;
+  using V = typename D::V;
   {   // blockIdx.y = segment
     const int64_t seg = blockIdx.y;
     x += seg * g.n * g.h * g.w * g.c;
     y += seg * g.n * g.ho * g.wo * g.c;
-    if (idx != nullptr) idx += seg * g.n * g.ho * g.wo * g.c;
+    if (WIN) { idx += seg * g.n * g.ho * g.wo * g.c; won += seg * g.n * g.ho * g.wo * g.c; }
     sums += seg * 2 * g.c;
     save_mean_rstd += seg * 2 * g.c;
     if (acc_sum != nullptr) { acc_sum += seg * acc_seg_stride; acc_sumsq += seg * acc_seg_stride; }
@@ -713,8 +721,9 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 2 ? 3 : 2) bn_relu_pool_k
   const PoolThread th(c >> 3);
   if (!th.active) return;
   const int ch = th.vec * 8;
-  float sc[8], sh[8];
+  tsp::Pair scale[4], shift[4];
   {
+    float sc[8], sh[8];
     const float rows = (float)((int64_t)g.n * g.h * g.w), inv_m = 1.f / rows;
     float s[8], q[8], wv[8], bv[8];
     tsp::ld8(sums, ch, s);
@@ -733,93 +742,114 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 2 ? 3 : 2) bn_relu_pool_k
       sc[e] = wv[e] * rstd;
       sh[e] = bv[e] - mean * sc[e];
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      scale[j] = tsp::Pair(sc[2 * j], sc[2 * j + 1]);
+      shift[j] = tsp::Pair(sh[2 * j], sh[2 * j + 1]);
+    }
   }
   const int pitch = g.w * c;                     // (below 2^31: n * h * w is)
   for (uint32_t i = blockIdx.x * th.per_block + th.slot; i < g.items; i += gridDim.x * th.per_block) {
-    const uint32_t strip = g.by_wo.div(i), img = g.by_rows.div(strip);
-    const int ox = (int)(i - strip * g.by_wo.d), oy0 = (int)(strip - img * g.by_rows.d) * kPoolRows;
+    const uint32_t strip = g.by_wo.div(i), img = g.by_strips.div(strip);
+    const int ox = (int)(i - strip * g.by_wo.d), oy0 = (int)(strip - img * g.by_strips.d) * g.rows;
+    const int end = min(oy0 + g.rows, g.ho);
     const bool left = ox > 0, right = 2 * ox + 1 < g.w;
     const T* xi = x + ((int64_t)img * g.h + 2 * oy0) * pitch + (2 * ox) * c + ch;      // the centre of the first window
     int64_t o = (((int64_t)img * g.ho + oy0) * g.wo + ox) * c + ch;
-    auto load = [&](const T* row, tsp::Raw8<T> (&raw)[3]) {
-      if (left) tsp::ldraw(row, -c, raw[0]);
+    auto load = [&](const T* row, tsp::Raw8<T> (&raw)[3]) {      // (a column that does not exist: any other)
+      tsp::ldraw(row, left ? -c : 0, raw[0]);
       tsp::ldraw(row, 0, raw[1]);
-      if (right) tsp::ldraw(row, c, raw[2]);
+      tsp::ldraw(row, right ? c : 0, raw[2]);
     };
-    // largest key of a row over the window's columns; a column that does not exist has the smallest key
-    auto row_keys = [&](const tsp::Raw8<T> (&raw)[3], K (&m)[8]) {
+    // The largest value of a row over the window's columns, or of some rows, the first of equal ones: its element of x, its code.
+    struct Best { V v[4], raw[4]; uint32_t code[4]; };
+    auto better = [&](V& v, V& raw, uint32_t& code, V v2, V raw2, uint32_t code2) {      // of this one and a later one
+      const V m = D::larger(v, v2);
+      if (WIN) {
+        const auto first = D::equal(v, m);
+        raw = D::pick(first, raw, raw2);
+        code = D::pick_code(first, code, code2);
+      }
+      v = m;
+    };
+    auto of_row = [&](const tsp::Raw8<T> (&raw)[3], uint32_t row_code, Best& r) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        K k[3][2];
+        V v[3];
 #pragma unroll
-        for (int kx = 0; kx < 3; ++kx) {
-          const float2 v = get2(raw[kx], j);
-          P::make(make_float2(v.x * sc[2 * j] + sh[2 * j], v.y * sc[2 * j + 1] + sh[2 * j + 1]), (uint32_t)(2 - kx), k[kx][0],
-                  k[kx][1]);
-        }
-        if (!left) k[0][0] = k[0][1] = 0;
-        if (!right) k[2][0] = k[2][1] = 0;
-        m[2 * j] = P::max3(k[0][0], k[1][0], k[2][0]);
-        m[2 * j + 1] = P::max3(k[0][1], k[1][1], k[2][1]);
+        for (int kx = 0; kx < 3; ++kx) v[kx] = D::round(tsp::fma2(D::wide(D::get(raw[kx], j)), scale[j], shift[j]));
+        if (!left) v[0] = D::lowest();
+        if (!right) v[2] = D::lowest();
+        r.v[j] = v[0];
+        r.raw[j] = D::get(raw[0], j);
+        r.code[j] = row_code | lanes(2);
+        better(r.v[j], r.raw[j], r.code[j], v[1], D::get(raw[1], j), row_code | lanes(1));
+        better(r.v[j], r.raw[j], r.code[j], v[2], D::get(raw[2], j), row_code);
       }
     };
-    tsp::Raw8<T> raw0[3] = {}, raw1[3] = {};
-    K top[8];                                    // the row above the window's centre
-#pragma unroll
-    for (int e = 0; e < 8; ++e) top[e] = 0;
-    if (oy0 > 0) {
-      load(xi - pitch, raw0);
-      row_keys(raw0, top);
-    }
+    tsp::Raw8<T> raw0[3], raw1[3];
+    Best top;                                    // the row above the window's centre
+    if (oy0 > 0) load(xi - pitch, raw1);
+    load(xi, raw0);
+    if (oy0 > 0) of_row(raw1, 0, top);
+    if (2 * oy0 + 1 < g.h) load(xi + pitch, raw1);
 #pragma unroll 1
-    for (int oy = oy0; oy < oy0 + kPoolRows && oy < g.ho; ++oy) {
-      const bool below = 2 * oy + 1 < g.h;       // an odd height ends in a window of two rows
-      load(xi, raw0);
-      if (below) load(xi + pitch, raw1);
-      K mid[8], low[8];
-      row_keys(raw0, mid);
+    for (int oy = oy0; oy < end; ++oy) {
+      Best mid, win;
+      of_row(raw0, lanes(4), mid);
+      if (oy + 1 < end) load(xi + 2 * (int64_t)pitch, raw0);     // on their way while this window is formed
+      if (oy > 0) {
+        win = top;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) low[e] = 0;
-      if (below) row_keys(raw1, low);
-      tsp::Raw8<T> out;
-      uint32_t code[2] = {0, 0};
+        for (int j = 0; j < 4; ++j) better(win.v[j], win.raw[j], win.code[j] |= lanes(8), mid.v[j], mid.raw[j], mid.code[j]);
+      } else {
+        win = mid;
+      }
+      if (2 * oy + 1 < g.h) {                    // (an odd height ends in a window of two rows)
+        of_row(raw1, 0, top);
+        if (oy + 1 < end && 2 * oy + 3 < g.h) load(xi + 3 * (int64_t)pitch, raw1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) better(win.v[j], win.raw[j], win.code[j], top.v[j], top.raw[j], top.code[j]);
+      }
+      tsp::Raw8<T> out, w;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        K k[2];
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const int e = 2 * j + s;
-          k[s] = P::max3(top[e] | 8u, mid[e] | 4u, low[e]);
-          top[e] = low[e];
-          code[e >> 2] |= (P::zero(k[s]) ? kNoTap : (uint32_t)k[s] & 15u) << (8 * (e & 3));
+        const V zero = {}, v = D::larger(win.v[j], zero);
+        D::set(out, j, v);
+        if (WIN) {
+          D::set(w, j, win.raw[j]);
+          win.code[j] = D::pick_code(D::equal(v, zero), kNoTap, win.code[j]);
         }
-        P::set2(out, j, k[0], k[1]);
       }
       st_raw(y, o, out);
-      if (idx != nullptr) *reinterpret_cast<uint2*>(idx + o) = make_uint2(code[0], code[1]);
+      if (WIN) {
+        st_raw(won, o, w);
+        *reinterpret_cast<uint2*>(idx + o) = make_uint2(__byte_perm(win.code[0], win.code[1], 0x7531),
+                                                        __byte_perm(win.code[2], win.code[3], 0x7531));
+      }
       xi += 2 * (int64_t)pitch;
       o += (int64_t)g.wo * c;
     }
   }
 }
 
-// APPLY false: sums[seg] += (sum dy', sum dy' * xhat).  APPLY true: dx from those sums.
-template <typename T, bool APPLY>
+// dx from the two sums of the gradient behind the ReLU (sums[seg], by the reduction over the winners).
+template <typename T>
 __global__ void __launch_bounds__(kBlock, 2) bn_relu_pool_bwd_kernel(const T* __restrict__ dy, const uint8_t* __restrict__ idx,
                                                                   const T* __restrict__ x,
                                                                   const float* __restrict__ mean_rstd,
                                                                   const float* __restrict__ wgt,
-                                                                  float* __restrict__ sums, T* __restrict__ dx,
+                                                                  const float* __restrict__ sums, T* __restrict__ dx,
                                                                   float* __restrict__ gw, float* __restrict__ gb,
                                                                   const PoolGeom g) {
   tsp::let_next_start();
-  constexpr int sm_pitch = kBlock + 8;
-  __shared__ float sm[APPLY ? 1 : 16 * sm_pitch];
+  using D = Duo<T>;
+  using V = typename D::V;
   const int c = g.c;
   {   // blockIdx.y = segment
     const int64_t seg = blockIdx.y, in = seg * g.n * g.h * g.w * c, outs = seg * g.n * g.ho * g.wo * c;
     x += in;
-    if (APPLY) dx += in;
+    dx += in;
     dy += outs;
     idx += outs;
     mean_rstd += seg * 2 * c;
@@ -827,8 +857,8 @@ __global__ void __launch_bounds__(kBlock, 2) bn_relu_pool_bwd_kernel(const T* __
   }
   const PoolThread th(c >> 3);
   const int ch = th.vec * 8;
-  if (APPLY && !th.active) return;
-  if (APPLY && gw != nullptr && blockIdx.y == 0 && blockIdx.x == 0 && th.slot == 0) {
+  if (!th.active) return;
+  if (gw != nullptr && blockIdx.y == 0 && blockIdx.x == 0 && th.slot == 0) {
     for (int e = 0; e < 8; ++e) {
       float db = 0.f, dw = 0.f;
       for (int k = 0; k < (int)gridDim.y; ++k) { db += sums[(int64_t)k * 2 * c + ch + e]; dw += sums[(int64_t)(k * 2 + 1) * c + ch + e]; }
@@ -836,107 +866,107 @@ __global__ void __launch_bounds__(kBlock, 2) bn_relu_pool_bwd_kernel(const T* __
       gw[ch + e] += dw;
     }
   }
-  float A[8], B[8], D[8];                       // APPLY: dx = A dy' + B x + D; else D = mean, A and B the two sums
-#pragma unroll
-  for (int e = 0; e < 8; ++e) { A[e] = 0.f; B[e] = 0.f; D[e] = 0.f; }
-  if (th.active) {
-    float mean[8];
+  tsp::Pair A[4], B[4], C[4];                   // dx = A dy' + B x + C
+  {
+    float mean[8], rs[8], wv[8], k1[8], k2[8];
     tsp::ld8(mean_rstd, ch, mean);
-    if constexpr (APPLY) {
-      float rs[8], wv[8], k1[8], k2[8];
-      tsp::ld8(mean_rstd + c, ch, rs);
-      tsp::ld8(wgt, ch, wv);
-      tsp::ld8(sums, ch, k1);
-      tsp::ld8(sums + c, ch, k2);
-      const float inv_m = 1.f / (float)((int64_t)g.n * g.h * g.w);
+    tsp::ld8(mean_rstd + c, ch, rs);
+    tsp::ld8(wgt, ch, wv);
+    tsp::ld8(sums, ch, k1);
+    tsp::ld8(sums + c, ch, k2);
+    const float inv_m = 1.f / (float)((int64_t)g.n * g.h * g.w);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        A[e] = wv[e] * rs[e];
-        B[e] = -A[e] * rs[e] * (k2[e] * inv_m);
-        D[e] = -A[e] * (k1[e] * inv_m) - B[e] * mean[e];
+    for (int j = 0; j < 4; ++j) {
+      float a[2], b[2], d[2];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int e = 2 * j + s;
+        a[s] = wv[e] * rs[e];
+        b[s] = -a[s] * rs[e] * (k2[e] * inv_m);
+        d[s] = -a[s] * (k1[e] * inv_m) - b[s] * mean[e];
       }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) D[e] = mean[e];
+      A[j] = tsp::Pair(a[0], a[1]);
+      B[j] = tsp::Pair(b[0], b[1]);
+      C[j] = tsp::Pair(d[0], d[1]);
     }
   }
-  const uint32_t items = th.active ? g.items : 0;
-  for (uint32_t i = blockIdx.x * th.per_block + th.slot; i < items; i += gridDim.x * th.per_block) {
-    const uint32_t row = g.by_wo.div(i), img = g.by_rows.div(row);
-    const int wb = (int)(i - row * g.by_wo.d), wa = (int)(row - img * g.by_rows.d);
-    const bool down = wa + 1 < g.ho, right = wb + 1 < g.wo;             // windows below and to the right
-    const bool row1 = 2 * wa + 1 < g.h, col1 = 2 * wb + 1 < g.w;        // second input row and column
-    const int64_t o = (int64_t)i * c + ch;
-    const int64_t q = (((int64_t)img * g.h + 2 * wa) * g.w + 2 * wb) * c + ch;
-    tsp::Raw8<T> gr[4] = {}, xr[4] = {};
-    uint32_t tap[4][2];
-    const bool have[4] = {true, right, down, down && right};
-    const bool pix[4] = {true, col1, row1, row1 && col1};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int64_t oo = o + ((k >> 1) * g.wo + (k & 1)) * (int64_t)c;
-      tap[k][0] = tap[k][1] = 0xffffffffu;                              // a window that does not exist has no winner
-      if (have[k]) {
-        tsp::ldraw(dy, oo, gr[k]);
-        const uint2 t = *reinterpret_cast<const uint2*>(idx + oo);
-        tap[k][0] = t.x;
-        tap[k][1] = t.y;
+  const int64_t out_pitch = (int64_t)g.wo * c, in_pitch = (int64_t)g.w * c;
+  for (uint32_t i = blockIdx.x * th.per_block + th.slot; i < g.items; i += gridDim.x * th.per_block) {
+    const uint32_t strip = g.by_wo.div(i), img = g.by_strips.div(strip);
+    const int wb = (int)(i - strip * g.by_wo.d), wa0 = (int)(strip - img * g.by_strips.d) * g.rows;
+    const int end = min(wa0 + g.rows, g.ho);
+    const bool right = wb + 1 < g.wo, col1 = 2 * wb + 1 < g.w;          // the window to the right, the second input column
+    int64_t o = (((int64_t)img * g.ho + wa0) * g.wo + wb) * c + ch;
+    int64_t q = (((int64_t)img * g.h + 2 * wa0) * g.w + 2 * wb) * c + ch;
+    // A row of two windows; one that does not exist has no winner.
+    struct Windows { tsp::Raw8<T> dy[2]; uint2 tap[2]; };
+    auto windows = [&](int64_t at, bool have, Windows& r) {
+      r.tap[0] = r.tap[1] = make_uint2(0xffffffffu, 0xffffffffu);
+      if (have) {
+        tsp::ldraw(dy, at, r.dy[0]);
+        r.tap[0] = *reinterpret_cast<const uint2*>(idx + at);
+        if (right) {
+          tsp::ldraw(dy, at + c, r.dy[1]);
+          r.tap[1] = *reinterpret_cast<const uint2*>(idx + at + c);
+        }
       }
-      if (pix[k]) tsp::ldraw(x, q + ((k >> 1) * g.w + (k & 1)) * (int64_t)c, xr[k]);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {                                       // channels 2j and 2j + 1
-      float2 gv[4];
-      uint32_t code[4][2];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        gv[k] = get2(gr[k], j);
-#pragma unroll
-        for (int s = 0; s < 2; ++s) code[k][s] = (tap[k][j >> 1] >> (8 * ((2 * j + s) & 3))) & 0xffu;
+    };
+    auto pixels = [&](int64_t at, bool second, tsp::Raw8<T> (&r)[4]) {
+      tsp::ldraw(x, at, r[0]);
+      if (col1) tsp::ldraw(x, at + c, r[1]);
+      if (second) {
+        tsp::ldraw(x, at + in_pitch, r[2]);
+        if (col1) tsp::ldraw(x, at + in_pitch + c, r[3]);
+      }
+    };
+    Windows up = {}, down = {};
+    tsp::Raw8<T> xr[4] = {};
+    windows(o, true, up);
+    pixels(q, 2 * wa0 + 1 < g.h, xr);
+    windows(o + out_pitch, wa0 + 1 < g.ho, down);
+#pragma unroll 1
+    for (int wa = wa0; wa < end; ++wa) {
+      // the next block of pixels and its lower windows are on their way while this block is computed
+      const bool more = wa + 1 < end;
+      Windows next = {};
+      tsp::Raw8<T> nx[4] = {};
+      if (more) {
+        pixels(q + 2 * in_pitch, 2 * wa + 3 < g.h, nx);
+        windows(o + 2 * out_pitch, wa + 2 < g.ho, next);
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {                                     // pixel (2 wa + k / 2, 2 wb + k % 2)
-        if (!APPLY && !pix[k]) continue;
-        float2 d = make_float2(0.f, 0.f);
+      for (int j = 0; j < 4; ++j) {                                     // channels 2j and 2j + 1
+        V gv[4];
+        uint32_t code[4];
 #pragma unroll
-        for (int kw = 0; kw < 4; ++kw) {                                // window (wa + kw / 2, wb + kw % 2)
+        for (int k = 0; k < 4; ++k) {
+          const Windows& row = k < 2 ? up : down;
+          gv[k] = D::get(row.dy[k & 1], j);
+          code[k] = __byte_perm(j < 2 ? row.tap[k & 1].x : row.tap[k & 1].y, 0, (j & 1) ? 0x3424 : 0x1404);
+        }
+        // what window (wa + kw / 2, wb + kw % 2) gives pixel (2 wa + k / 2, 2 wb + k % 2)
+        auto part = [&](int k, int kw) {
           const int ky = (k >> 1) + 1 - 2 * (kw >> 1), kx = (k & 1) + 1 - 2 * (kw & 1);
-          if (ky < 0 || kx < 0) continue;
-          if (code[kw][0] == tap_code(ky, kx)) d.x += gv[kw].x;
-          if (code[kw][1] == tap_code(ky, kx)) d.y += gv[kw].y;
-        }
-        if (k > 0) d = round2<T>(d);                                    // (pixel 0 is in one window only)
-        const float2 xv = get2(xr[k], j);
-        if constexpr (APPLY) {
-          set2(xr[k], j, make_float2(A[2 * j] * d.x + B[2 * j] * xv.x + D[2 * j],
-                                     A[2 * j + 1] * d.y + B[2 * j + 1] * xv.y + D[2 * j + 1]));
-        } else {
-          A[2 * j] += d.x;
-          A[2 * j + 1] += d.y;
-          B[2 * j] += d.x * (xv.x - D[2 * j]);
-          B[2 * j + 1] += d.y * (xv.y - D[2 * j + 1]);
-        }
+          return D::keep(D::same_code(code[kw], tap_code(ky, kx)), gv[kw]);
+        };
+        V d[4];                                                         // rounded as a tensor of the sums would be
+        d[0] = part(0, 0);
+        d[1] = D::sum(part(1, 0), part(1, 1));
+        d[2] = D::sum(part(2, 0), part(2, 2));
+        d[3] = D::round((D::wide(part(3, 0)) + D::wide(part(3, 1))) + (D::wide(part(3, 2)) + D::wide(part(3, 3))));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          D::set(xr[k], j, D::round(tsp::fma2(A[j], D::wide(d[k]), tsp::fma2(B[j], D::wide(D::get(xr[k], j)), C[j]))));
       }
-    }
-    if constexpr (APPLY) {
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (pix[k]) st_raw(dx, q + ((k >> 1) * g.w + (k & 1)) * (int64_t)c, xr[k]);
-    }
-  }
-  if constexpr (!APPLY) {
-    // one addition per channel and block, lane = channel, as in bn_colsum_kernel
+        if (((k & 1) == 0 || col1) && (k < 2 || 2 * wa + 1 < g.h)) st_raw(dx, q + (k >> 1) * in_pitch + (k & 1) * c, xr[k]);
+      up = down;
+      down = next;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) { sm[e * sm_pitch + threadIdx.x] = A[e]; sm[(8 + e) * sm_pitch + threadIdx.x] = B[e]; }
-    __syncthreads();
-    const int width = min(c >> 3, kBlock), base = blockIdx.z * kBlock * 8;
-    for (int p = threadIdx.x; p < 16 * width; p += kBlock) {
-      const int half = p >= 8 * width ? 1 : 0, cc = p - half * 8 * width;
-      if (base + cc >= c) continue;
-      float acc = 0.f;
-      for (int k = 0; k < th.per_block; ++k) acc += sm[(half * 8 + (cc & 7)) * sm_pitch + k * width + (cc >> 3)];
-      if (half) acc *= mean_rstd[c + base + cc];
-      atomicAdd(sums + half * c + base + cc, acc);
+      for (int k = 0; k < 4; ++k) xr[k] = nx[k];
+      o += out_pitch;
+      q += 2 * in_pitch;
     }
   }
 }
@@ -1129,13 +1159,19 @@ int tsp_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* 
 }
 
 // Training-mode BatchNorm + ReLU + 3x3 / 2 / 1 max-pool of x [segs * n, h, w, c] (statistics per group of n images, from
-// `sums` [segs][2c] = sum and sum of squares over a group's pixels) -> y [segs * n, ho, wo, c], ho = (h + 1) / 2; idx
-// (optional, same shape as y) receives the winning taps for the backward.  The other arguments as in tsp_bn_apply.
-static int pool_geom(int n, int h, int w, int c, int segs, int rows_per_item, PoolGeom* g) {
+// `sums` [segs][2c] = sum and sum of squares over a group's pixels) -> y [segs * n, ho, wo, c], ho = (h + 1) / 2.  For the
+// backward (together, optional, same shape as y): idx receives the winning taps, won the winners' elements of x.  The other
+// arguments as in tsp_bn_apply.
+static int pool_geom(int n, int h, int w, int c, int segs, PoolGeom* g) {
   if (n <= 0 || h < 1 || w < 1 || c % 8 != 0 || c > 4096 || segs < 1) return -3;
-  const int ho = (h + 1) / 2, wo = (w + 1) / 2, rows = (ho + rows_per_item - 1) / rows_per_item;
+  const int ho = (h + 1) / 2, wo = (w + 1) / 2;
   if ((int64_t)n * (h + 1) * (w + 1) >= 0x7fffffff || (int64_t)w * c >= 0x7fffffff) return -3;
-  *g = {n, h, w, c, ho, wo, FastDiv(wo), FastDiv(rows), (uint32_t)((int64_t)n * rows * wo)};
+  // strips of four rows where they give an SM four blocks, of fewer rows on smaller tensors
+  int rows = 4;
+  const int64_t blocks = (int64_t)segs * n * ho * wo * (c / 8) / kBlock;
+  while (rows > 1 && blocks / rows < 148 * 4) rows /= 2;
+  const int strips = (ho + rows - 1) / rows;
+  *g = {n, h, w, c, ho, wo, rows, FastDiv(wo), FastDiv(strips), (uint32_t)((int64_t)n * strips * wo)};
   return 0;
 }
 
@@ -1148,45 +1184,49 @@ static dim3 pool_grid(const PoolGeom& g, int segs, int waves) {
   return dim3((unsigned)(blocks < 1 ? 1 : blocks), (unsigned)segs, (unsigned)slabs);
 }
 
-int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums, const float* w, const float* b,
+int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, void* won, const float* sums, const float* w, const float* b,
                          float* save_mean_rstd, float* acc_sum, float* acc_sumsq, float* acc_count, int64_t acc_seg_stride,
                          int n, int h, int wd, int c, float eps, int dtype, int segs, cudaStream_t stream) {
   PoolGeom g;
-  const int rc = pool_geom(n, h, wd, c, segs, kPoolRows, &g);
+  const int rc = pool_geom(n, h, wd, c, segs, &g);
   if (rc != 0) return rc;
   if (!vectors_ok(w, b, sums, nullptr)) return -2;
+  if ((idx == nullptr) != (won == nullptr)) return -3;
   const dim3 grid = pool_grid(g, segs, 32);
+  auto run = [&](auto kern, auto* px, auto* py, auto* pw) {
+    kern<<<grid, kBlock, 0, stream>>>(px, py, idx, pw, sums, w, b, save_mean_rstd, acc_sum, acc_sumsq, acc_count,
+                                      acc_seg_stride, g, eps);
+  };
+  using B = __nv_bfloat16;
   if (dtype == TSP_DTYPE_BF16)
-    bn_relu_pool_kernel<__nv_bfloat16><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, idx, sums, w,
-                                                                    b, save_mean_rstd, acc_sum, acc_sumsq, acc_count,
-                                                                    acc_seg_stride, g, eps);
+    run(idx != nullptr ? bn_relu_pool_kernel<B, true> : bn_relu_pool_kernel<B, false>, (const B*)x, (B*)y, (B*)won);
   else
-    bn_relu_pool_kernel<float><<<grid, kBlock, 0, stream>>>((const float*)x, (float*)y, idx, sums, w, b, save_mean_rstd,
-                                                            acc_sum, acc_sumsq, acc_count, acc_seg_stride, g, eps);
+    run(idx != nullptr ? bn_relu_pool_kernel<float, true> : bn_relu_pool_kernel<float, false>, (const float*)x, (float*)y,
+        (float*)won);
   return TSP_LAUNCH_CHECK();
 }
 
-// Its backward: dy [segs * n, ho, wo, c], idx and x as above -> dx; sums [segs][2c], zeroed by the
+// Its backward: dy [segs * n, ho, wo, c], idx, won and x as above -> dx; sums [segs][2c], zeroed by the
 // caller, receives db and dw; gw / gb as in tsp_bn_bwd_apply.
-int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* x, const float* mean_rstd, const float* w,
-                         float* sums, void* dx, float* gw, float* gb, int n, int h, int wd, int c,
-                         int dtype, int segs, cudaStream_t stream) {
+int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* won, const void* x, const float* mean_rstd,
+                         const float* w, const float* b, float* sums, void* dx, float* gw, float* gb, int n, int h, int wd,
+                         int c, int dtype, int segs, cudaStream_t stream) {
   PoolGeom g;
-  const int rc = pool_geom(n, h, wd, c, segs, 1, &g);
+  int rc = pool_geom(n, h, wd, c, segs, &g);
   if (rc != 0) return rc;
   if (!vectors_ok(w, mean_rstd, sums, nullptr)) return -2;
-  const dim3 grid_r = pool_grid(g, segs, 2), grid_a = pool_grid(g, segs, 32);
+  // The gradient meets the winners only, one per window: the two sums are those of a BatchNorm + ReLU over them.
+  rc = tsp_bn_bwd_reduce(dy, won, nullptr, nullptr, mean_rstd, w, b, 1, (int64_t)segs * n * g.ho * g.wo, c, dtype, sums, segs,
+                         stream);
+  if (rc != 0) return rc;
+  const dim3 grid = pool_grid(g, segs, 32);
   if (dtype == TSP_DTYPE_BF16) {
     using B = __nv_bfloat16;
-    bn_relu_pool_bwd_kernel<B, false><<<grid_r, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, sums,
-                                                                     nullptr, nullptr, nullptr, g);
-    bn_relu_pool_bwd_kernel<B, true><<<grid_a, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, sums,
-                                                                    (B*)dx, gw, gb, g);
+    bn_relu_pool_bwd_kernel<B><<<grid, kBlock, 0, stream>>>((const B*)dy, idx, (const B*)x, mean_rstd, w, sums, (B*)dx, gw, gb,
+                                                            g);
   } else {
-    bn_relu_pool_bwd_kernel<float, false><<<grid_r, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd,
-                                                                         w, sums, nullptr, nullptr, nullptr, g);
-    bn_relu_pool_bwd_kernel<float, true><<<grid_a, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd, w,
-                                                                        sums, (float*)dx, gw, gb, g);
+    bn_relu_pool_bwd_kernel<float><<<grid, kBlock, 0, stream>>>((const float*)dy, idx, (const float*)x, mean_rstd, w, sums,
+                                                                (float*)dx, gw, gb, g);
   }
   return TSP_LAUNCH_CHECK();
 }

@@ -66,12 +66,12 @@ int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, con
                  const float* w, const float* b, float* save_mean_rstd, float* acc_sum, float* acc_sumsq,
                  float* acc_count, int64_t acc_seg_stride, int64_t m, int c, float eps, int relu, int dtype, int segs,
                  cudaStream_t stream);
-int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, const float* sums, const float* w, const float* b,
+int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, void* won, const float* sums, const float* w, const float* b,
                          float* save_mean_rstd, float* acc_sum, float* acc_sumsq, float* acc_count, int64_t acc_seg_stride,
                          int n, int h, int wd, int c, float eps, int dtype, int segs, cudaStream_t stream);
-int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* x, const float* mean_rstd, const float* w,
-                         float* sums, void* dx, float* gw, float* gb, int n, int h, int wd, int c,
-                         int dtype, int segs, cudaStream_t stream);
+int tsp_bn_relu_pool_bwd(const void* dy, const uint8_t* idx, const void* won, const void* x, const float* mean_rstd,
+                         const float* w, const float* b, float* sums, void* dx, float* gw, float* gb, int n, int h, int wd,
+                         int c, int dtype, int segs, cudaStream_t stream);
 int tsp_bn_bwd_reduce(const void* dy, const void* x, const void* y, void* dres, const float* mean_rstd, const float* w,
                       const float* bias, int relu, int64_t m, int c, int dtype, float* sums, int segs,
                       cudaStream_t stream);

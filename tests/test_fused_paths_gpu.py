@@ -422,10 +422,11 @@ def test_add_layer_norm_equals_the_separate_passes(rows, d, with_a, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape,views", [((2, 64, 8, 8), 2), ((3, 8, 5, 7), 1), ((4, 24, 9, 2), 2), ((2, 64, 30, 16), 1),
-                                         ((1, 512, 2, 3), 1), ((2, 64, 18, 33), 2), ((1, 2056, 3, 5), 1)])
+                                         ((1, 512, 2, 3), 1), ((2, 64, 18, 33), 2), ((1, 2056, 3, 5), 1),
+                                         ((8, 64, 137, 139), 1), ((16, 64, 137, 139), 2)])
 def test_batchnorm_relu_maxpool_equals_the_separate_passes(shape, views, dtype):
-    """Odd extents (last window of two rows or columns), strips that end early, channel counts off the block size, more
-    channels than a block takes."""
+    """Odd extents (last window of two rows or columns), strips of one, two and four rows that end early, channel counts off
+    the block size, more channels than a block takes."""
     from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
     from tspipe_b200.ops import bn as fbn
     from tspipe_b200.ops.pool import MaxPool3x3s2

@@ -257,7 +257,9 @@ class _BnReluPool(torch.autograd.Function):
         dt = _f._dt(x)
         y = torch.empty((n, c, (h + 1) // 2, (w + 1) // 2), dtype=x.dtype, device=x.device,
                         memory_format=torch.channels_last)
-        idx = torch.empty(y.numel(), dtype=torch.uint8, device=x.device) if any(ctx.needs_input_grad[:3]) else None
+        idx = won = None
+        if any(ctx.needs_input_grad[:3]):       # for the backward: the winning taps and what x holds there
+            idx, won = torch.empty(y.numel(), dtype=torch.uint8, device=x.device), torch.empty_like(y)
         save = torch.empty(segs * 2 * c, dtype=torch.float32, device=x.device)
         wf, bf = _f.param_f32(weight), _f.param_f32(bias)
         with _f.on_device(x.device):
@@ -267,20 +269,20 @@ class _BnReluPool(torch.autograd.Function):
                 _f._check(L.tsp_bn_stats(_f._ptr(x), _c.c_int64(n * h * w), _c.c_int(c), _c.c_int(dt), _f._ptr(sums),
                                          _c.c_int(segs), st), "tsp_bn_stats")
                 _f._count(2)
-            _f._check(L.tsp_bn_relu_pool_fwd(_f._ptr(x), _f._ptr(y), _f._ptr(idx), _f._ptr(sums), _f._ptr(wf), _f._ptr(bf),
-                                             _f._ptr(save), _f._ptr(acc_sum), _f._ptr(acc_sumsq), _f._ptr(acc_count),
+            _f._check(L.tsp_bn_relu_pool_fwd(_f._ptr(x), _f._ptr(y), _f._ptr(idx), _f._ptr(won), _f._ptr(sums), _f._ptr(wf),
+                                             _f._ptr(bf), _f._ptr(save), _f._ptr(acc_sum), _f._ptr(acc_sumsq), _f._ptr(acc_count),
                                              _c.c_int64(acc_stride), _c.c_int(n // segs), _c.c_int(h), _c.c_int(w),
                                              _c.c_int(c), _c.c_float(eps), _c.c_int(dt), _c.c_int(segs), st),
                       "tsp_bn_relu_pool_fwd")
             _f._count()
-        ctx.save_for_backward(x, idx, save, wf)
+        ctx.save_for_backward(x, idx, won, save, wf, bf)
         ctx.segs, ctx.wdtype, ctx.bdtype = segs, weight.dtype, bias.dtype
         ctx.owners = (weight, bias) if _f.IN_CAPTURE else (None, None)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, idx, save, wf = ctx.saved_tensors
+        x, idx, won, save, wf, bf = ctx.saved_tensors
         n, c, h, w = x.shape
         segs = ctx.segs
         ho, wo = (h + 1) // 2, (w + 1) // 2
@@ -292,8 +294,8 @@ class _BnReluPool(torch.autograd.Function):
         if gw is None or gb is None:
             gw = gb = None
         with _f.on_device(x.device):
-            _f._check(_lib().tsp_bn_relu_pool_bwd(_f._ptr(dy), _f._ptr(idx), _f._ptr(x), _f._ptr(save), _f._ptr(wf),
-                                                  _f._ptr(sums), _f._ptr(dx), _f._ptr(gw), _f._ptr(gb),
+            _f._check(_lib().tsp_bn_relu_pool_bwd(_f._ptr(dy), _f._ptr(idx), _f._ptr(won), _f._ptr(x), _f._ptr(save),
+                                                  _f._ptr(wf), _f._ptr(bf), _f._ptr(sums), _f._ptr(dx), _f._ptr(gw), _f._ptr(gb),
                                                   _c.c_int(n // segs), _c.c_int(h), _c.c_int(w), _c.c_int(c),
                                                   _c.c_int(_f._dt(x)), _c.c_int(segs), _f._stream()),
                       "tsp_bn_relu_pool_bwd")
