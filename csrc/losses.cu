@@ -247,17 +247,18 @@ __global__ void __launch_bounds__(512, 2) kd_ce_kernel(const TS* __restrict__ s,
 
 // ---------------------------------------------------------------------------------------------
 // The same on long bf16 rows (a vocabulary), one persistent block per SM, one exponential per logit instead of two (three on
-// labelled rows): the first sweep keeps e = 2^((x - m) k), m the warp's running maximum at that vector, of the teacher in
-// registers and of the student in shared memory (122 KB each for 30528 classes), and the second only scales them by one factor
-// per vector.  The divergence is summed in the first sweep as well, sum e_t ((b - mt) - (a - ms)), and follows the maxima
-// as the other sums do.  Meanwhile a producer warp streams the next rows into a ring with bulk copies.
-// For rows that nearly fill five vectors per thread, several of them per SM.  Microseconds with the kernel above and with this
-// one, one in seven rows labelled and a quarter masked: 8192 rows of 30528 383 and 340, 2048 113 and 102, 1024 68 and 61, 592 47 and
-// 45, 300 31 and 35.  A vector that few threads have part in costs what a full one does: without masked rows, 2048 of 28672 1.02
-// times as fast, of 26624 1.00, of 24584 0.97, 1024 of them 0.94 (whole vectors fewer, 24576 or 18432: 1.00 at 2048
-// rows, 1.03 at 8192).  What bounds it is instruction issue beside the
-// exponentials (per vector: waits, maxima, references; per row: the sums over 24 warps); fewer warps with more of a row each are
-// slower for want of warps (12: 460 us where 24 take 410, unmasked).
+// labelled rows): the first sweep keeps e = 2^((x - m) k2), m a reference of the warp's, of the teacher in registers (one vector of
+// five in shared memory) and of the student in shared memory (122 KB for 30528 classes), and the second only scales them by one
+// factor per vector.  A reference is the maximum of the warp's first vectors until a vector is well above it.  The divergence is
+// summed in the first sweep as well, sum e_t ((b - mt) - (a - ms)), and follows the references as the other sums do.  Meanwhile a
+// producer warp streams the next rows into a ring with bulk copies.
+// For rows that reach into the last vector, four of them per SM.  Microseconds with the kernel above and with this one, 15 in a
+// hundred rows labelled, none masked: 8192 rows of 30528 classes 480 and 358, of 24584 398 and 323, 592 rows 53 and 45, 43 and 42;
+// 300 rows, a quarter of them masked, 31 and 29, 26.5 and 27.8.
+// What bounds it is the issue of instructions (270 per warp and vector of 8 pairs, 60 % of the slots) beside their latency: with
+// all of the teacher's exponentials in registers, and the bounded wait unrolled with them, the registers of a block of 25 warps
+// (72 a thread) did not do, and with 221 KB of shared memory in use what spills comes back from L2: 8192 rows as above 439.
+// Fewer warps with more of a row each are slower for want of warps (12: 460 us where 24 took 410).
 // Rows are drawn by ticket: masked ones cost next to nothing (the producer warp writes their zeros), so a fixed share of
 // rows per block would leave blocks idle at the end.  Per row one barrier among the computing warps, behind the first
 // sweep; its partial sums alternate between two buffers.
@@ -266,13 +267,14 @@ constexpr int kRowWarps = 24, kRowThreads = kRowWarps * 32;     // computing thr
 constexpr int kRowVecs = 5;                                     // 16-byte vectors of a row per thread
 constexpr int kPieceElems = kRowThreads * 8;                    // of one tensor: one vector per thread
 constexpr int kPieceBytes = kPieceElems * 2;
-constexpr int kRing = 4;                                        // pieces of s and t, 24 KB each
-constexpr int kRowSmem = kRing * 2 * kPieceBytes + kRowVecs * kPieceElems * 4 + 2 * kRing * 8 + 128;
+constexpr int kRing = 3;                                        // pieces of s and t, 24 KB each
+constexpr int kRowRegs = 4;                                     // vectors of the teacher's exponentials in registers
+constexpr int kRowSmem = kRing * 2 * kPieceBytes + (2 * kRowVecs - kRowRegs) * kPieceElems * 4 + 2 * kRing * 8 + 128;
 constexpr int kRowQueue = 4;                                    // rows that the ring and the sweeps may hold
 static_assert(kRing < kRowQueue * 2 && kRowSmem <= 227 * 1024, "a row in the ring is two pieces at least");
 constexpr uint64_t kRowWaitNs = 2000000000ull;                  // a wait gives up after two seconds
-constexpr int kStreamMin = (3 * kRowVecs - 1) * kPieceElems / 3;    // elements of a row: the last vector two thirds full
-constexpr int kStreamRows = 1024;                               // rows: seven per SM
+constexpr int kStreamMin = (kRowVecs - 1) * kPieceElems + 1;    // elements of a row: only the last vector is partly filled
+constexpr int kStreamRows = 4 * 148;                            // rows: four per SM
 
 using tsp::Pair;
 using tsp::fma2;
@@ -299,6 +301,20 @@ __device__ __forceinline__ float warp_top(float v) {            // as tsp::warp_
   asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
+// Sums of four values over the warp: of a in lanes 0 - 7, b in 8 - 15, c in 16 - 23, d in 24 - 31.
+__device__ __forceinline__ float four_sums(float a, float b, float c, float d, int lane) {
+  const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
+  const float x = (h16 ? c : a) + __shfl_xor_sync(0xffffffffu, h16 ? a : c, 16);
+  const float y = (h16 ? d : b) + __shfl_xor_sync(0xffffffffu, h16 ? b : d, 16);
+  float v = (h8 ? y : x) + __shfl_xor_sync(0xffffffffu, h8 ? x : y, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// (a call: five copies of the bounded loop in the sweep cost registers that its values need)
+__device__ __noinline__ bool wait_for_piece(uint64_t* bar, uint32_t phase, int* status) {
+  return tc5::mbar_wait(bar, phase, status, 9, kRowWaitNs);
+}
 __device__ __forceinline__ void row_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kRowThreads) : "memory"); }
 
 __global__ void __launch_bounds__(kRowThreads + 32, 1)
@@ -308,15 +324,15 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
                     __nv_bfloat16* __restrict__ gs) {
   extern __shared__ __align__(128) uint8_t ring[];
   float4* kept = (float4*)(ring + kRing * 2 * kPieceBytes);       // the student's exponentials, [vector][half][thread]
-  uint64_t* full = (uint64_t*)(ring + kRing * 2 * kPieceBytes + kRowVecs * kPieceElems * 4);
+  uint64_t* full = (uint64_t*)(ring + kRing * 2 * kPieceBytes + (2 * kRowVecs - kRowRegs) * kPieceElems * 4);
   uint64_t* empty = full + kRing;
   __shared__ int2 rows[kRowQueue];                    // the rows in the ring: index (-1: no more) and label (-1: none)
   __shared__ float part[2][6][32];
   __shared__ int failed[2];                           // by row, as `part`: a wait of a computing warp ran out
-  __shared__ double block_part[kRowWarps];
+  __shared__ double block_part;                       // the block's share of the loss
   __shared__ float2 refs[kRowWarps][kRowVecs];        // the maxima that a warp's exponentials refer to, of s and t
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nv = c / 8, pieces = (nv + kRowThreads - 1) / kRowThreads;
+  const int nv = c / 8;
   unsigned* counters = reinterpret_cast<unsigned*>(sum + 1);      // [0] ticket, [1] blocks that are done
   int* status = reinterpret_cast<int*>(sum + 2);      // not 0 once a wait has run out: the loss is NaN then
   if (threadIdx.x == 0) {
@@ -325,6 +341,7 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
       tc5::mbar_init(empty + i, kRowWarps);
     }
     failed[0] = failed[1] = 0;
+    block_part = 0.;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -349,7 +366,7 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
           const int64_t l = labels[row];
           if (w_ce != 0.f && l >= 0 && l < c) label = (int)l;
         }
-        for (int k = 0; k < pieces && ok; ++k, ++it) {
+        for (int k = 0; k < kRowVecs && ok; ++k, ++it) {
           const int slot = it % kRing;
           const uint32_t round = it / kRing;
           if (round > 0) ok = tc5::mbar_wait_parked(empty + slot, (round - 1) & 1, status, 8, kRowWaitNs);
@@ -381,69 +398,87 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
     // ---------------- sweeps ----------------
     const float k2 = kLog2e / temp, wt = w_kd * temp;
     const Pair k2p(k2, k2);
-    double acc = 0.;
+    const float far = fminf(4.f, 4.f / k2);             // exponents stay below 4, and 6 without temperature: as exact as the exponentials
     uint32_t slot = 0, phase = 0;                       // of the next piece
     for (int r = 0;; ++r) {
       int2 id = make_int2(0, -1);
-      bool ok = true;                                   // (the same for a whole warp)
-      Pair et[kRowVecs][4];                             // the teacher's exponentials
+      bool ok = true;
+      Pair et[kRowRegs][4];                             // the teacher's exponentials
       RowPart ps = {-INFINITY}, pt = {-INFINITY};
       float z1 = 0.f, zs = 0.f, zt = 0.f, kl = 0.f;
 #pragma unroll
       for (int k = 0; k < kRowVecs; ++k) {
-        if (k < pieces && ok && id.x >= 0) {
-          ok = __all_sync(0xffffffffu, tc5::mbar_wait(full + slot, phase, status, 9, kRowWaitNs)) != 0;
-          if (k == 0) id = ok ? rows[r % kRowQueue] : make_int2(-1, -1);
-          if (id.x >= 0 && ok) {
-            const uint4* piece = reinterpret_cast<const uint4*>(ring + slot * 2 * kPieceBytes) + threadIdx.x;
-            const bool mine = k * kRowThreads + threadIdx.x < nv;
-            uint4 qa = make_uint4(0, 0, 0, 0), qb = qa;
-            if (mine) { qa = piece[0]; qb = piece[kPieceBytes / 16]; }
-            __syncwarp();
-            if (lane == 0) tc5::mbar_arrive(empty + slot);             // every lane has its vectors
-            if (++slot == kRing) { slot = 0; phase ^= 1; }
-            const float tops = warp_top(mine ? top_of(qa) : -INFINITY), topt = warp_top(mine ? top_of(qb) : -INFINITY);
-            if (tops > ps.m || topt > pt.m) {
-              const RowPart ns = {fmaxf(ps.m, tops)}, nt = {fmaxf(pt.m, topt)};
-              const float ft = ex2((pt.ref() - nt.ref()) * k2);
-              if (id.y >= 0) z1 *= ex2((ps.ref() - ns.ref()) * kLog2e);
-              zs *= ex2((ps.ref() - ns.ref()) * k2);
-              kl = moved(kl, zt, ft, (pt.ref() - ps.ref()) - (nt.ref() - ns.ref()));
-              zt *= ft;
-              ps = ns;
-              pt = nt;
-            }
-            if (lane == 0) refs[warp][k] = make_float2(ps.ref(), pt.ref());
-            if (mine) {
-              const uint32_t a[4] = {qa.x, qa.y, qa.z, qa.w}, b[4] = {qb.x, qb.y, qb.z, qb.w};
-              const Pair ms2(ps.ref(), ps.ref()), mt2(pt.ref(), pt.ref());
-              Pair ss(0.f, 0.f), st(0.f, 0.f), sk(0.f, 0.f);
-              float es[8];
+        // (a wait that ran out: the sums mean nothing then, and are used for nothing behind the barrier)
+        if (!tc5::mbar_try_wait(tc5::smem_u32(full + slot), phase)) ok &= wait_for_piece(full + slot, phase, status);
+        if (k == 0) id = rows[r % kRowQueue];
+        if (k == 0 && id.x < 0) break;
+        const uint4* piece = reinterpret_cast<const uint4*>(ring + slot * 2 * kPieceBytes) + threadIdx.x;
+        const bool mine = k < kRowVecs - 1 || k * kRowThreads + (int)threadIdx.x < nv;
+        uint4 qa = make_uint4(0, 0, 0, 0), qb = qa;
+        if (mine) { qa = piece[0]; qb = piece[kPieceBytes / 16]; }
+        __syncwarp();
+        if (lane == 0) tc5::mbar_arrive(empty + slot);             // every lane has its vectors
+        if (++slot == kRing) { slot = 0; phase ^= 1; }
+        const float tops = warp_top(mine ? top_of(qa) : -INFINITY), topt = warp_top(mine ? top_of(qb) : -INFINITY);
+        if (k == 0 || tops > ps.m + far || topt > pt.m + far) {
+          const RowPart ns = {fmaxf(ps.m, tops)}, nt = {fmaxf(pt.m, topt)};
+          const float ft = ex2((pt.ref() - nt.ref()) * k2);
+          if (id.y >= 0) z1 *= ex2((ps.ref() - ns.ref()) * kLog2e);
+          zs *= ex2((ps.ref() - ns.ref()) * k2);
+          kl = moved(kl, zt, ft, (pt.ref() - ps.ref()) - (nt.ref() - ns.ref()));
+          zt *= ft;
+          ps = ns;
+          pt = nt;
+        }
+        if (lane == 0) refs[warp][k] = make_float2(ps.ref(), pt.ref());
+        if (mine) {
+          const uint32_t a[4] = {qa.x, qa.y, qa.z, qa.w}, b[4] = {qb.x, qb.y, qb.z, qb.w};
+          const Pair ms2(ps.ref(), ps.ref()), mt2(pt.ref(), pt.ref());
+          Pair ss(0.f, 0.f), st(0.f, 0.f), sk(0.f, 0.f);
+          float4* keep = kept + 2 * k * kRowThreads + threadIdx.x;
+          Pair ek[4];                               // the teacher's
+          float es[4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const Pair da = unpack2(a[j]) - ms2, db = unpack2(b[j]) - mt2, ea = ex2(da * k2p);
-                et[k][j] = ex2(db * k2p);
-                ss = ss + ea;
-                st = st + et[k][j];
-                ea.split(es[2 * j], es[2 * j + 1]);
-                float p0, p1, d0, d1;
-                et[k][j].split(p0, p1);
-                (db - da).split(d0, d1);
-                // a class that the teacher gives no probability adds nothing, whatever the other factor is
-                sk = fma2(et[k][j], Pair(p0 != 0.f ? d0 : 0.f, p1 != 0.f ? d1 : 0.f), sk);
-                if (id.y >= 0) {
-                  float da0, da1;
-                  da.split(da0, da1);
-                  z1 += ex2(da0 * kLog2e) + ex2(da1 * kLog2e);
-                }
-              }
-              zs += total(ss);
-              zt += total(st);
-              kl += total(sk);
-              float4* keep = kept + 2 * k * kRowThreads + threadIdx.x;
-              keep[0] = make_float4(es[0], es[1], es[2], es[3]);
-              keep[kRowThreads] = make_float4(es[4], es[5], es[6], es[7]);
+          for (int j = 0; j < 4; ++j) {
+            const Pair da = unpack2(a[j]) - ms2, db = unpack2(b[j]) - mt2, ea = ex2(da * k2p);
+            ek[j] = ex2(db * k2p);
+            ss = ss + ea;
+            st = st + ek[j];
+            ea.split(es[2 * (j & 1)], es[2 * (j & 1) + 1]);
+            if (j & 1) keep[(j >> 1) * kRowThreads] = make_float4(es[0], es[1], es[2], es[3]);
+            sk = fma2(ek[j], db - da, sk);
+          }
+          if (id.y >= 0) {
+            const Pair e2(kLog2e, kLog2e);
+            Pair s1(0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s1 = s1 + ex2((unpack2(a[j]) - ms2) * e2);
+            z1 += total(s1);
+          }
+          zs += total(ss);
+          zt += total(st);
+          float part_kl = total(sk);
+          if (part_kl != part_kl) {                 // a class that the teacher gives no probability adds nothing, whatever
+            part_kl = 0.f;                          // the other factor is
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float p[2], d[2];
+              ek[j].split(p[0], p[1]);
+              ((unpack2(b[j]) - mt2) - (unpack2(a[j]) - ms2)).split(d[0], d[1]);
+              part_kl = fmaf(p[1], p[1] != 0.f ? d[1] : 0.f, fmaf(p[0], p[0] != 0.f ? d[0] : 0.f, part_kl));
             }
+          }
+          kl += part_kl;
+          if (k < kRowRegs) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) et[k < kRowRegs ? k : 0][j] = ek[j];
+          } else {                                  // behind the student's
+            float4* kt = keep + 2 * (kRowVecs - kRowRegs) * kRowThreads;
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) ek[j].split(v[2 * j], v[2 * j + 1]);
+            kt[0] = make_float4(v[0], v[1], v[2], v[3]);
+            kt[kRowThreads] = make_float4(v[4], v[5], v[6], v[7]);
           }
         }
       }
@@ -451,14 +486,10 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
       // the warp's sums, then the block's; a warp whose part is empty refers to a finite maximum
       float (*pp)[32] = part[r & 1];
       {
-        kl = tsp::warp_sum(kl);
-        z1 = has_ce ? tsp::warp_sum(z1) : 0.f;
-        zs = tsp::warp_sum(zs);
-        zt = tsp::warp_sum(zt);
-        if (lane == 0) {
-          pp[0][warp] = ps.m; pp[1][warp] = pt.m; pp[2][warp] = z1; pp[3][warp] = zs; pp[4][warp] = zt; pp[5][warp] = kl;
-          if (!ok) *((volatile int*)(failed + (r & 1))) = 1;
-        }
+        const float v = four_sums(z1, zs, zt, kl, lane);
+        if ((lane & 7) == 0) pp[2 + (lane >> 3)][warp] = v;
+        if (lane == 0) { pp[0][warp] = ps.m; pp[1][warp] = pt.m; }
+        if (!ok) *((volatile int*)(failed + (r & 1))) = 1;
       }
       row_barrier();
       if (*((volatile int*)(failed + (r & 1))) != 0 || id.x < 0) break;      // the same for all computing warps
@@ -470,40 +501,61 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
       // with such a part has its divergence formed from the probabilities, behind the second sweep.
       const float part_kl = in ? moved(pp[5][lane], pp[4][lane], ex2((wtop.ref() - mt) * k2), (wtop.ref() - ws.ref()) - (mt - ms)) : 0.f;
       const bool redo = __any_sync(0xffffffffu, !(fabsf(part_kl) < 1e30f)) != 0;       // the same for all computing warps
-      if (warp == 0) kl = tsp::warp_sum(part_kl);
-      z1 = has_ce ? tsp::warp_sum(in ? pp[2][lane] * ex2((ws.ref() - ms) * kLog2e) : 0.f) : 0.f;
-      zs = tsp::warp_sum(in ? pp[3][lane] * ex2((ws.ref() - ms) * k2) : 0.f);
-      zt = tsp::warp_sum(in ? pp[4][lane] * ex2((wtop.ref() - mt) * k2) : 0.f);
+      {
+        const float v = four_sums(has_ce && in ? pp[2][lane] * ex2((ws.ref() - ms) * kLog2e) : 0.f,
+                                  in ? pp[3][lane] * ex2((ws.ref() - ms) * k2) : 0.f, in ? pp[4][lane] * ex2((wtop.ref() - mt) * k2) : 0.f,
+                                  part_kl, lane);
+        z1 = __shfl_sync(0xffffffffu, v, 0);
+        zs = __shfl_sync(0xffffffffu, v, 8);
+        zt = __shfl_sync(0xffffffffu, v, 16);
+        kl = __shfl_sync(0xffffffffu, v, 24);
+      }
       const float l1 = has_ce ? log2f(z1) : 0.f, ls = log2f(zs), lt = log2f(zt);
-      if (threadIdx.x == 0) acc += (redo ? 0. : (double)(wt * (kl / zt))) - (double)(w_kd * temp * (temp * (lt - ls) * kLn2));
+      if (threadIdx.x == 0) atomicAdd(&block_part, (redo ? 0. : (double)(wt * (kl / zt))) - (double)(w_kd * temp * (temp * (lt - ls) * kLn2)));
       // second sweep: the gradient
       uint4* gr = gs ? reinterpret_cast<uint4*>(gs + (int64_t)id.x * c) : nullptr;
       const uint4* sr = reinterpret_cast<const uint4*>(s + (int64_t)id.x * c);
 #pragma unroll
       for (int k = 0; k < kRowVecs; ++k) {
         const int i = k * kRowThreads + threadIdx.x;
-        if (i < nv) {
+        if (k < kRowVecs - 1 || i < nv) {
           const float2 ref = refs[warp][k];
           const float fs = wt * ex2((ref.x - ms) * k2 - ls), ft = -wt * ex2((ref.y - mt) * k2 - lt);
           const Pair fs2(fs, fs), ft2(ft, ft);
           const float4* keep = kept + 2 * k * kRowThreads + threadIdx.x;
           const float4 e0 = keep[0], e1 = keep[kRowThreads];
-          Pair g[4] = {fma2(fs2, Pair(e0.x, e0.y), ft2 * et[k][0]), fma2(fs2, Pair(e0.z, e0.w), ft2 * et[k][1]),
-                       fma2(fs2, Pair(e1.x, e1.y), ft2 * et[k][2]), fma2(fs2, Pair(e1.z, e1.w), ft2 * et[k][3])};
+          Pair ek[4];
+          if (k < kRowRegs) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) ek[j] = et[k < kRowRegs ? k : 0][j];
+          } else {
+            const float4* kt = keep + 2 * (kRowVecs - kRowRegs) * kRowThreads;
+            const float4 t0 = kt[0], t1 = kt[kRowThreads];
+            ek[0] = Pair(t0.x, t0.y);
+            ek[1] = Pair(t0.z, t0.w);
+            ek[2] = Pair(t1.x, t1.y);
+            ek[3] = Pair(t1.z, t1.w);
+          }
+          Pair g[4] = {fma2(fs2, Pair(e0.x, e0.y), ft2 * ek[0]), fma2(fs2, Pair(e0.z, e0.w), ft2 * ek[1]),
+                       fma2(fs2, Pair(e1.x, e1.y), ft2 * ek[2]), fma2(fs2, Pair(e1.z, e1.w), ft2 * ek[3])};
           float v[8];
 #pragma unroll
           for (int j = 0; j < 4; ++j) g[j].split(v[2 * j], v[2 * j + 1]);
           if (has_ce) {                                 // (the row once more, from L2)
-            float x[8];
             const uint4 q = __ldg(sr + i);
             const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+            const Pair ms2(ms, ms), e2(kLog2e, kLog2e), l2(l1, l1), wc(w_ce, w_ce);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) unpack2(w[j]).split(x[2 * j], x[2 * j + 1]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float d = x[e] - ms;
-              v[e] += w_ce * (ex2(d * kLog2e - l1) - (i * 8 + e == id.y ? 1.f : 0.f));
-              if (i * 8 + e == id.y) acc += (double)(w_ce * (l1 * kLn2 - d));
+            for (int j = 0; j < 4; ++j) {
+              const Pair d = unpack2(w[j]) - ms2;
+              Pair p = ex2(d * e2 - l2);
+              if (i * 4 + j == (id.y >> 1)) {
+                float d0, d1;
+                d.split(d0, d1);
+                atomicAdd(&block_part, (double)(w_ce * (l1 * kLn2 - ((id.y & 1) ? d1 : d0))));
+                p = p - ((id.y & 1) ? Pair(0.f, 1.f) : Pair(1.f, 0.f));
+              }
+              fma2(wc, p, g[j]).split(v[2 * j], v[2 * j + 1]);
             }
           }
           if (gr) __stcs(gr + i, make_uint4(tc5::pack_bf16x2(v[0], v[1]), tc5::pack_bf16x2(v[2], v[3]),
@@ -529,18 +581,14 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
             }
           }
         }
-        acc += (double)wt * (double)part;
+        part = tsp::warp_sum(part);
+        if (lane == 0) atomicAdd(&block_part, (double)wt * (double)part);
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) block_part[warp] = acc;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double v = 0.;
-    for (int w = 0; w < kRowWarps; ++w) v += block_part[w];
-    atomicAdd(sum, v);
+    atomicAdd(sum, block_part);
     __threadfence();
     if (atomicAdd(counters + 1, 1u) == gridDim.x - 1)
       *loss = *((volatile int*)status) == 0 ? (float)atomicAdd(sum, 0.) : __int_as_float(0x7fffffff);
@@ -678,10 +726,8 @@ int tsp_byol_loss_pair(const void* x0, const void* y0, const void* x1, const voi
                                  : launch_byol<float>(x0, y0, x1, y1, n, d, scale, sum, loss, gx, stream);
 }
 
-int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,
-                    double* sum, float* loss, void* gx, cudaStream_t stream) {
-  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
-  if (cudaError_t e = cudaMemsetAsync(sum, 0, sizeof(double), stream); e != cudaSuccess) return (int)e;
+static void launch_cosine(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,
+                          double* sum, void* gx, cudaStream_t stream) {
   const int grid = (n + 3) / 4;
   const bool vec = rows_of_8(d, x, y, gx);
 #define TSP_COS(T, VEC) \
@@ -689,16 +735,21 @@ int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n
   if (dtype == TSP_DTYPE_BF16) { if (vec) TSP_COS(__nv_bfloat16, true); else TSP_COS(__nv_bfloat16, false); }
   else { if (vec) TSP_COS(float, true); else TSP_COS(float, false); }
 #undef TSP_COS
+}
+
+int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n, int d, int dtype, float scale,
+                    double* sum, float* loss, void* gx, cudaStream_t stream) {
+  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  if (cudaError_t e = cudaMemsetAsync(sum, 0, sizeof(double), stream); e != cudaSuccess) return (int)e;
+  launch_cosine(x, y, row_mask, n, d, dtype, scale, sum, gx, stream);
   round_sum_kernel<<<1, 1, 0, stream>>>(sum, loss);
   return TSP_LAUNCH_CHECK();
 }
 
-// `sum`: three doubles of scratch.
-int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
-                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* sum, float* loss, void* gs,
-                   cudaStream_t stream) {
-  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
-  if (cudaError_t e = cudaMemsetAsync(sum, 0, 3 * sizeof(double), stream); e != cudaSuccess) return (int)e;
+// The loss of tsp_kd_ce_loss, on top of what *sum holds.
+static int launch_kd_ce(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
+                        int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* sum, float* loss, void* gs,
+                        cudaStream_t stream) {
   const bool vec = rows_of_8(c, s, t, gs);
   if (vec && t != nullptr && w_kd != 0.f && s_dtype == TSP_DTYPE_BF16 && t_dtype == TSP_DTYPE_BF16 &&
       n >= kStreamRows && c >= kStreamMin && c <= kRowVecs * kPieceElems) {
@@ -730,6 +781,26 @@ int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const ui
 #undef TSP_KD
   round_sum_kernel<<<1, 1, 0, stream>>>(sum, loss);
   return TSP_LAUNCH_CHECK();
+}
+
+// `sum`: three doubles of scratch.
+int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
+                   int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* sum, float* loss, void* gs,
+                   cudaStream_t stream) {
+  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  if (cudaError_t e = cudaMemsetAsync(sum, 0, 3 * sizeof(double), stream); e != cudaSuccess) return (int)e;
+  return launch_kd_ce(s, t, labels, row_mask, n, c, s_dtype, t_dtype, temp, w_ce, w_kd, sum, loss, gs, stream);
+}
+
+// tsp_kd_ce_loss and tsp_cosine_loss over the same n rows and mask as one loss: the terms share the sum.
+int tsp_distil_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
+                    int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, const void* x, const void* y, int d,
+                    int x_dtype, float scale, double* sum, float* loss, void* gs, void* gx, cudaStream_t stream) {
+  if (n <= 0) return (int)cudaMemsetAsync(loss, 0, sizeof(float), stream);
+  if (cudaError_t e = cudaMemsetAsync(sum, 0, 3 * sizeof(double), stream); e != cudaSuccess) return (int)e;
+  launch_cosine(x, y, row_mask, n, d, x_dtype, scale, sum, gx, stream);
+  if (const int rc = TSP_LAUNCH_CHECK(); rc != 0) return rc;
+  return launch_kd_ce(s, t, labels, row_mask, n, c, s_dtype, t_dtype, temp, w_ce, w_kd, sum, loss, gs, stream);
 }
 
 // out = in * *gout (see scale_kernel; out may be in); `in` and `out` 16-byte aligned.

@@ -39,6 +39,9 @@ int tsp_cosine_loss(const void* x, const void* y, const uint8_t* row_mask, int n
 int tsp_kd_ce_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
                    int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, double* sum, float* loss, void* gs,
                    cudaStream_t stream);
+int tsp_distil_loss(const void* s, const void* t, const int64_t* labels, const uint8_t* row_mask, int n, int c,
+                    int s_dtype, int t_dtype, float temp, float w_ce, float w_kd, const void* x, const void* y, int d,
+                    int x_dtype, float scale, double* sum, float* loss, void* gs, void* gx, cudaStream_t stream);
 int tsp_scale(const void* in, const float* gout, void* out, int64_t n, int dtype, cudaStream_t stream);
 
 // ---- norms.cu ----------------------------------------------------------------------------------------------------

@@ -58,9 +58,9 @@ def test_kd_ce_rows_vectorised_and_not(n, c, dtype):
 
 
 @pytest.mark.parametrize("n,c", [(1, 30528), (1023, 24584), (1024, 24576), (1024, 28664), (1024, 28672), (1024, 24584), (1025, 30528), (1100, 30720),
-                                 (1024, 30728)])
+                                 (1024, 30728), (591, 24584), (592, 24584), (592, 24576), (592, 30720)])
 def test_kd_ce_long_rows(n, c):
-    """Either side of the limits of the kernel that keeps a row on the chip (1024 rows, 28672 to 30720 elements), with masked
+    """Either side of the limits of the kernel that keeps a row on the chip (592 rows, 24584 to 30720 elements), with masked
     rows, a row without a label, one with classes switched off."""
     from tspipe_b200.ops import fused
     torch.manual_seed(0)
@@ -88,6 +88,53 @@ def test_kd_ce_long_rows(n, c):
         assert not g[~keep].any()
     t[n - 1 if keep[n - 1] else 0, 9] = math.nan
     assert fused.kd_ce_loss(s, t, y, 2.0, 0.5, 0.25).isnan()
+
+
+def test_kd_ce_long_rows_with_maxima_that_grow_along_a_row():
+    """Logits that rise from vector to vector, in steps that stay with a warp's reference and in steps that move it, for the
+    student, the teacher and both, in labelled rows and others."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(4)
+    n, c = 600, 30528
+    part = torch.arange(c, device=DEV) // 6144
+    s, t = (torch.randn(n, c, device=DEV) for _ in range(2))
+    rise = torch.tensor([0.0, 1.5, 3.0, 10.0, 60.0], device=DEV).repeat_interleave(n // 5)[:, None] * part
+    s[::3] += rise[::3]
+    t[1::3] += rise[1::3]
+    s[2::3] += rise[2::3]
+    t[2::3] += 0.5 * rise[2::3]
+    s, t = s.bfloat16().requires_grad_(), t.bfloat16()
+    y = torch.where(torch.arange(n, device=DEV) % 2 == 0, torch.randint(0, c, (n,), device=DEV), -100)
+    loss = fused.kd_ce_loss(s, t, y, 2.0, 0.5, 0.25)
+    (g,) = torch.autograd.grad(loss, s)
+    r = s.detach().double().requires_grad_()
+    ls, lt = F.log_softmax(r / 2, 1), F.log_softmax(t.double() / 2, 1)
+    ref = (lt.exp() * (lt - ls)).sum() + 0.5 * F.cross_entropy(r, y, ignore_index=-100, reduction="sum")
+    (gr,) = torch.autograd.grad(ref, r)
+    assert abs(float(loss.detach()) - float(ref.detach())) <= 1e-6 * abs(float(ref.detach()))
+    for i in range(n):                                  # every row by itself: bf16's rounding
+        assert _rel(g[i], gr[i]) < 2 * EPS[torch.bfloat16]
+
+
+@pytest.mark.parametrize("n,c,dtype,mask", [(40, 1000, torch.float32, None), (40, 1001, torch.bfloat16, torch.int64),
+                                            (600, 30528, torch.bfloat16, torch.bool)])
+def test_distil_loss_equals_its_terms(n, c, dtype, mask):
+    """One call for both terms, above and below the limits of the kernel for long rows: value, gradients, scaled backward."""
+    from tspipe_b200.ops import fused
+    torch.manual_seed(5)
+    s, t = ((torch.randn(n // 4, 4, c, device=DEV) * 2).to(dtype) for _ in range(2))
+    x, y = (torch.randn(n // 4, 4, 72, device=DEV).to(dtype) for _ in range(2))
+    lab = torch.randint(-1, c, (n // 4, 4), device=DEV)
+    on = None if mask is None else (torch.arange(n, device=DEV).view(-1, 4) % 3 != 1).to(mask)
+    s.requires_grad_()
+    x.requires_grad_()
+    one = fused.distil_loss(s, t, lab, 2.0, 0.5, 0.25, x, y, 0.125, row_mask=on)
+    two = fused.kd_ce_loss(s, t, lab, 2.0, 0.5, 0.25, row_mask=on) + fused.cosine_embedding_loss(x, y, 0.125, row_mask=on)
+    assert abs(float(one.detach()) - float(two.detach())) <= 3e-7 * abs(float(two.detach()))
+    for a, b in zip(torch.autograd.grad(3 * one, [s, x]), torch.autograd.grad(3 * two, [s, x])):
+        assert a.shape == b.shape and _rel(a, b) < 1e-6
+    (only,) = torch.autograd.grad(fused.distil_loss(s.detach(), t, lab, 2.0, 0.5, 0.25, x, y, 0.125, row_mask=on), x)
+    assert _rel(only, torch.autograd.grad(fused.cosine_embedding_loss(x, y, 0.125, row_mask=on), x)[0]) < 1e-6
 
 
 @pytest.mark.parametrize("reserve", [0, 8])

@@ -131,10 +131,10 @@ def distil_loss(student_out, teacher_out, labels, args=None, extra_args=None, ep
     n_sel, n_lab = max(n_sel, 1), max(n_lab, 1)
     if _fused_ok(s_logits, t_logits) and not getattr(extra_args, "no_fused", False):
         from .ops import fused
-        loss = fused.kd_ce_loss(s_logits, t_logits, lm_labels, T, a_mlm / n_lab, a_ce / n_sel, row_mask=sel)
         if a_cos > 0:
-            loss = loss + fused.cosine_embedding_loss(s_hidden, t_hidden, a_cos / n_sel, row_mask=sel)
-        return loss
+            return fused.distil_loss(s_logits, t_logits, lm_labels, T, a_mlm / n_lab, a_ce / n_sel, s_hidden, t_hidden,
+                                     a_cos / n_sel, row_mask=sel)
+        return fused.kd_ce_loss(s_logits, t_logits, lm_labels, T, a_mlm / n_lab, a_ce / n_sel, row_mask=sel)
     v = s_logits.shape[-1]
     s_sel = s_logits.float()[sel]
     t_sel = t_logits.float()[sel]

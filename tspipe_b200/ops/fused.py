@@ -34,6 +34,7 @@ def lib():
         # declared argument types: plain numbers at a call, an object per argument less where a whole loss takes 100 us of host
         v, i, f = _c.c_void_p, _c.c_int, _c.c_float
         L.tsp_kd_ce_loss.argtypes = [v] * 4 + [i] * 4 + [f] * 3 + [v] * 4
+        L.tsp_distil_loss.argtypes = [v] * 4 + [i] * 4 + [f] * 3 + [v] * 2 + [i] * 2 + [f] + [v] * 5
         L.tsp_byol_loss_pair.argtypes = [v] * 4 + [i] * 3 + [f] + [v] * 4
         L.tsp_cosine_loss.argtypes = [v] * 3 + [i] * 3 + [f] + [v] * 4
         L.tsp_scale.argtypes = [v] * 3 + [_c.c_int64, i, v]
@@ -392,11 +393,15 @@ def _address(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+def _owns_saved() -> bool:
+    return torch._C._autograd._top_saved_tensors_default_hooks(False) is None
+
+
 def save_gradient(ctx, g: torch.Tensor) -> None:
     """Saves a gradient that a forward has computed for :func:`_scaled`, and whether it stays this function's own: hooks on
     saved tensors may keep what they are given, or hand out the same tensor elsewhere."""
     ctx.save_for_backward(g)
-    ctx.own = torch._C._autograd._top_saved_tensors_default_hooks(False) is None
+    ctx.own = _owns_saved()
 
 
 def _scaled(g: torch.Tensor, gout: torch.Tensor, own: bool) -> torch.Tensor:
@@ -478,6 +483,20 @@ def byol_loss(o1, o2, t1, t2) -> torch.Tensor:
     return byol_pair_loss(o1, t2, 1.0 / n) + byol_pair_loss(o2, t1, 1.0 / n)
 
 
+def _mask_bytes(row_mask: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """A row mask as the kernels read it: a byte per row, zero where a row is off (a bool is one already)."""
+    if row_mask is None:
+        return None
+    m = row_mask.reshape(-1)
+    return (m.view(torch.uint8) if m.dtype == torch.bool else m.to(torch.uint8)).contiguous()
+
+
+def _labels(labels: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    if labels is not None and not (labels.dim() == 1 and labels.dtype == torch.int64 and labels.is_contiguous()):
+        labels = labels.reshape(-1).to(torch.int64).contiguous()
+    return labels
+
+
 class _KdCe(torch.autograd.Function):
     @staticmethod
     def forward(ctx, s, t, labels, row_mask, temp, w_ce, w_kd):
@@ -487,10 +506,7 @@ class _KdCe(torch.autograd.Function):
         loss = torch.empty((), dtype=torch.float32, device=s2.device)
         total = torch.empty(3, dtype=torch.float64, device=s2.device)
         gs = torch.empty_like(s2)
-        lab = labels
-        if lab is not None and not (lab.dim() == 1 and lab.dtype == torch.int64 and lab.is_contiguous()):
-            lab = lab.reshape(-1).to(torch.int64).contiguous()
-        msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
+        lab, msk = _labels(labels), _mask_bytes(row_mask)
         with on_device(s2.device):
             _check(lib().tsp_kd_ce_loss(s2.data_ptr(), _address(t2), _address(lab), _address(msk), n, c, _dt(s2),
                                         0 if t2 is None else _dt(t2), temp, w_ce, w_kd, total.data_ptr(),
@@ -533,7 +549,7 @@ class _Cosine(torch.autograd.Function):
         loss = torch.empty((), dtype=torch.float32, device=x2.device)
         total = torch.empty((), dtype=torch.float64, device=x2.device)
         gx = torch.empty_like(x2)
-        msk = None if row_mask is None else row_mask.reshape(-1).to(torch.uint8).contiguous()
+        msk = _mask_bytes(row_mask)
         with on_device(x2.device):
             _check(lib().tsp_cosine_loss(x2.data_ptr(), y2.data_ptr(), _address(msk), n, d, _dt(x2), scale,
                                          total.data_ptr(), loss.data_ptr(), gx.data_ptr(), _raw_stream()),
@@ -552,6 +568,47 @@ class _Cosine(torch.autograd.Function):
 
 def cosine_embedding_loss(x, y, scale: float, row_mask=None) -> torch.Tensor:
     return _Cosine.apply(x, y, row_mask, scale)
+
+
+class _Distil(torch.autograd.Function):
+    """:func:`kd_ce_loss` and :func:`cosine_embedding_loss` over the same rows, their terms in one sum."""
+
+    @staticmethod
+    def forward(ctx, s, x, t, y, labels, row_mask, temp, w_ce, w_kd, scale):
+        s2, t2, x2, y2 = _rows(s), _rows(t), _rows(x), _rows(y)
+        (n, c), d = s2.shape, x2.shape[1]
+        loss = torch.empty((), dtype=torch.float32, device=s2.device)
+        total = torch.empty(3, dtype=torch.float64, device=s2.device)
+        gs, gx = torch.empty_like(s2), torch.empty_like(x2)
+        lab, msk = _labels(labels), _mask_bytes(row_mask)
+        with on_device(s2.device):
+            _check(lib().tsp_distil_loss(s2.data_ptr(), t2.data_ptr(), _address(lab), _address(msk), n, c, _dt(s2), _dt(t2),
+                                         temp, w_ce, w_kd, x2.data_ptr(), y2.data_ptr(), d, _dt(x2), scale,
+                                         total.data_ptr(), loss.data_ptr(), gs.data_ptr(), gx.data_ptr(), _raw_stream()),
+                   "tsp_distil_loss")
+        _count(3)
+        ctx.save_for_backward(gs, gx)
+        ctx.own = _owns_saved()
+        ctx.shapes = s.shape, x.shape
+        return loss
+
+    @staticmethod
+    def backward(ctx, gout):
+        out = []
+        for g, shape, need in zip(ctx.saved_tensors, ctx.shapes, ctx.needs_input_grad):
+            g = _scaled(g, gout, ctx.own) if need else None
+            out.append(g if g is None or g.shape == shape else g.view(shape))
+        return (*out, None, None, None, None, None, None, None, None)
+
+
+def distil_loss(s, t, labels, temp: float, w_ce: float, w_kd: float, x, y, scale: float, row_mask=None) -> torch.Tensor:
+    """``kd_ce_loss(s, t, ...) + cosine_embedding_loss(x, y, scale)`` under one row mask."""
+    ts = (s, t, x, y)
+    if all(type(v) is torch.Tensor and v.dim() > 1 and v.numel() > 0 and v.dtype in (torch.float32, torch.bfloat16)
+           and v.device == s.device and not _wrapped(v) for v in ts) and y.dtype == x.dtype \
+            and s.shape == t.shape and x.shape == y.shape and s.shape[:-1] == x.shape[:-1]:
+        return _Distil.apply(s, x, t, y, labels, row_mask, temp, w_ce, w_kd, scale)
+    return kd_ce_loss(s, t, labels, temp, w_ce, w_kd, row_mask) + cosine_embedding_loss(x, y, scale, row_mask)
 
 
 def info_nce_loss(q: torch.Tensor, k: torch.Tensor, temp: float) -> torch.Tensor:
