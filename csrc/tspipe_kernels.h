@@ -69,6 +69,8 @@ int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, con
                  const float* w, const float* b, float* save_mean_rstd, float* acc_sum, float* acc_sumsq,
                  float* acc_count, int64_t acc_seg_stride, int64_t m, int c, float eps, int relu, int dtype, int segs,
                  cudaStream_t stream);
+int tsp_bn_commit(float* acc, int sets, int total, int segs, unsigned commits, const float* momentum, float* running_mean,
+                  float* running_var, long long* batches, int layers, cudaStream_t stream);
 int tsp_bn_relu_pool_fwd(const void* x, void* y, uint8_t* idx, void* won, const float* sums, const float* w, const float* b,
                          float* save_mean_rstd, float* acc_sum, float* acc_sumsq, float* acc_count, int64_t acc_seg_stride,
                          int n, int h, int wd, int c, float eps, int dtype, int segs, cudaStream_t stream);

@@ -496,6 +496,31 @@ def test_batchnorm_relu_maxpool_equals_the_separate_passes(shape, views, dtype):
         assert _rel(a, b) < EPS[dtype] + 1e-5
 
 
+@pytest.mark.parametrize("widths", [(8,), (64, 8, 256, 2048)])
+@pytest.mark.parametrize("chunks", [1, 2, 3])
+def test_statistics_commit_equals_the_library_ops(chunks, widths):
+    """Steps of one and two views, commits behind the first and the second view, a layer that has seen nothing."""
+    from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
+    torch.manual_seed(22)
+    groups = [BatchNormGroup(torch.nn.Sequential(*(DeferredBatchNorm(c, momentum=0.1 + 0.2 * i, chunks=chunks)
+                                                   for i, c in enumerate(widths))).to(dev)) for dev in ("cpu", DEV)]
+    for step, segs in enumerate((1, 2, 2, 1, 2)):
+        acc = torch.rand(3, 2, sum(widths)) * 4
+        acc[1] += acc[0].square()
+        acc[2] = torch.randint(2, 50, acc[2].shape)
+        acc[:, segs:] = 0
+        acc[:, :, : widths[0]] *= (step > 2)
+        for g in groups:
+            g._acc += acc.to(g._acc.device)
+            g.step(segments=segs)
+    groups[1].commit()
+    groups[0].commit()
+    for name in ("running_mean", "running_var", "_acc", "nbt"):
+        a, b = (getattr(g, name).double().cpu() for g in groups)
+        assert _rel(b, a) < 1e-6, name
+    assert groups[0].tracked == groups[1].tracked
+
+
 # ---- tensor-core products -----------------------------------------------------------------------------------------
 @pytest.mark.parametrize("m,n,k", [(128, 64, 64), (300, 192, 128), (12608, 768, 64), (257, 4096, 192), (5000, 1024, 64)])
 def test_linear_products_at_every_tile_width(m, n, k):

@@ -173,6 +173,16 @@ class BatchNormGroup:
         after the other, exactly as separate forwards would have been."""
         if not self.layers or not self.module.training:
             return
+        if self.sum.is_cuda and not self.any_cma and segments <= self.max_segments:
+            commits = 0
+            for g in range(segments):
+                self.tracked += 1
+                if self.tracked >= self.chunks:
+                    commits |= 1 << g
+                    self.tracked = 0
+            if commits or segments > 1:
+                self._commit_views(segments, commits)
+            return
         for g in range(segments):
             if g > 0:
                 self._acc[:, 0] += self._acc[:, g]
@@ -181,8 +191,17 @@ class BatchNormGroup:
             if self.tracked >= self.chunks:
                 self.commit()
 
+    def _commit_views(self, segments: int, commits: int) -> None:
+        """What :meth:`step` does to the statistics, as one launch; bit g of ``commits``: a commit behind view g."""
+        from .ops import bn as _bn
+        _bn.commit_views(self._acc, segments, commits, self.momentum, self.running_mean, self.running_var, self.nbt)
+
     @torch.no_grad()
     def commit(self) -> None:
+        if self.sum.is_cuda and not self.any_cma:
+            self._commit_views(1, 1)
+            self.tracked = 0
+            return
         self.nbt += 1
         cnt = self.count.clamp_min(1.0)
         mean = self.sum / cnt

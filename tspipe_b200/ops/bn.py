@@ -247,6 +247,17 @@ def bn_act(bn, x: torch.Tensor, residual: Optional[torch.Tensor] = None, relu: b
     return y
 
 
+def commit_views(acc: torch.Tensor, segments: int, commits: int, momentum: torch.Tensor, running_mean: torch.Tensor,
+                 running_var: torch.Tensor, batches: torch.Tensor) -> None:
+    """See ``bn_commit_kernel``: ``acc`` is ``[3][sets][channels]``, ``batches`` the layers' batch counters."""
+    with _f.on_device(acc.device):
+        _f._check(_lib().tsp_bn_commit(_f._ptr(acc), acc.shape[1], acc.shape[2], segments, _c.c_uint(commits),
+                                       _f._ptr(momentum), _f._ptr(running_mean), _f._ptr(running_var), _f._ptr(batches),
+                                       batches.numel(), _f._stream()), "tsp_bn_commit")
+    _f._count()
+    torch.autograd.graph.increment_version((acc, running_mean, running_var, batches))
+
+
 class _BnReluPool(torch.autograd.Function):
     """``max_pool2d(relu(bn(x)), 3, stride 2, padding 1)`` in training mode; see ``bn_relu_pool_kernel``."""
 
