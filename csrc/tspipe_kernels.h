@@ -131,6 +131,14 @@ int tsp_conv_stem_wgrad(const void* x, const void* dy, float* dw, int n, int h, 
 int tsp_conv_stem_fwd(const void* x, const void* wmat, void* y, float* sums, int n, int h, int w, int segs,
                       int* status, cudaStream_t stream);
 
+// ---- conv_igemm_tcgen05.cu ----------------------------------------------------------------------------------------
+int tsp_conv_fprop(const void* x, const void* wgt, void* y, float* col_sums, int segs, int n, int h, int w, int cin,
+                   int cout, int k, int s, int* status, cudaStream_t stream);
+int tsp_conv_dgrad(const void* dy, const void* wgt, const void* addend, void* dx, int n, int h, int w, int cin, int cout,
+                   int k, int s, int* status, cudaStream_t stream);
+int tsp_conv_wgrad(const void* x, const void* dy, float* dw, int n, int h, int w, int cin, int cout, int k, int s,
+                   int* status, cudaStream_t stream);
+
 int tsp_gemm_bf16_tn_stats(const void* a, const void* b, void* c, int m, int n, int k, int lda, int ldb, int ldc,
                            float* col_sums, int segs, int* status, cudaStream_t stream);
 

@@ -1,0 +1,261 @@
+"""Eager calls as C++ autograd functions (``csrc/host/eager.cpp``) against the Python functions of the same layers."""
+import contextlib
+
+import pytest
+import torch
+from torch import nn
+
+from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
+from tspipe_b200.ops import fused
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _cl(*shape, dtype=torch.bfloat16):
+    return torch.randn(*shape, device=DEV).to(dtype).contiguous(memory_format=torch.channels_last)
+
+
+def _both(monkeypatch, make, call):
+    """``call(*make())`` with the C++ functions and with the Python ones; the first have run."""
+    outs = []
+    for native in (True, False):
+        torch.manual_seed(0)
+        with monkeypatch.context() as m:
+            if not native:
+                m.setattr(fused, "eager", lambda: None)
+            args = make()
+            before = 0 if fused._host is None else fused._host.launches()
+            outs.append(call(*args))
+            assert ((0 if fused._host is None else fused._host.launches()) > before) == native
+    return outs
+
+
+def _same(a, b, tol=2e-3):
+    assert (a is None) == (b is None)
+    if a is not None:
+        assert a.shape == b.shape and a.dtype == b.dtype
+        a, b = a.double(), b.double()
+        assert float((a - b).norm()) <= tol * float(b.norm()) + 1e-12
+
+
+def _conv_block(k, stride, cin, cout, n, side, views, res, fork, dtype=torch.bfloat16):
+    conv = nn.Conv2d(cin, cout, k, stride=stride, padding=(k - 1) // 2, bias=False).to(DEV, memory_format=torch.channels_last)
+    bn = DeferredBatchNorm(cout).to(DEV)
+    group = BatchNormGroup(bn, chunks=10)
+    with torch.no_grad():
+        bn.weight.uniform_(0.5, 1.5)
+        bn.bias.normal_()
+    so = (side + 2 * ((k - 1) // 2) - k) // stride + 1
+    x = _cl(n, cin, side, side).requires_grad_()
+    r = _cl(n, cout, so, so, dtype=dtype).requires_grad_() if res else None
+    gy, gx = _cl(n, cout, so, so), _cl(n, cin, side, side)
+    return conv, bn, group, x, r, gy, gx, views, fork
+
+
+def _run_conv(conv, bn, group, x, r, gy, gx, views, fork):
+    from tspipe_b200.ops import bn as fbn
+    from tspipe_b200.ops import conv as fconv
+    leaves = [x, conv.weight, bn.weight, bn.bias] + ([r] if r is not None else [])
+    with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False), fbn.segments(views):
+        if fork:
+            y, skip = fconv.conv_bn_act_fork(conv, bn, x, relu=True)
+        else:
+            y, skip = fconv.conv_bn_act(conv, bn, x, residual=r, relu=True), None
+    fconv.clear_weight_cache()
+    out = [y] + ([skip] if fork else [])
+    grads = torch.autograd.grad(out, leaves, [gy] + ([gx] if fork else []), retain_graph=True)
+    again = torch.autograd.grad(out, leaves, [gy] + ([gx] if fork else []))
+    only = None
+    return [y.detach(), group._acc, *grads, *again], only
+
+
+@pytest.mark.parametrize("k,stride,cin,cout,n,side,views,res,fork",
+                         [(1, 1, 64, 64, 4, 8, 1, False, False), (1, 1, 64, 256, 4, 8, 2, True, False),
+                          (3, 1, 64, 64, 3, 14, 1, False, False), (3, 2, 128, 64, 5, 8, 1, False, False),
+                          (1, 2, 64, 128, 2, 10, 2, False, False), (1, 1, 256, 64, 6, 7, 2, False, True),
+                          (3, 1, 64, 64, 2, 9, 1, False, True), (1, 1, 64, 64, 3, 5, 3, False, False)])
+def test_convolution_and_batchnorm(monkeypatch, k, stride, cin, cout, n, side, views, res, fork):
+    """Strides, taps, residuals, forks, views, statistics from the epilogue and from a pass of their own (7 x 7 images of two
+    views); three views are no case for the C++ function, nor for the Python one (they run one after the other)."""
+    if views > 2:
+        make = lambda: _conv_block(k, stride, cin, cout, n, side, views, res, fork)     # noqa: E731
+        a = _run_conv(*make())[0]
+        assert all(torch.isfinite(t).all() for t in a)
+        return
+    a, b = _both(monkeypatch, lambda: _conv_block(k, stride, cin, cout, n, side, views, res, fork), lambda *v: _run_conv(*v)[0])
+    for p, q in zip(a, b):
+        _same(p, q)
+
+
+def test_convolution_gradients_in_place_by_name_and_with_hooks(monkeypatch):
+    """The weight's gradient goes to an existing buffer only when it is asked for; BatchNorm's through its hooks."""
+    def call(conv, bn, group, x, r, gy, gx, views, fork):
+        from tspipe_b200.ops import conv as fconv
+        conv.weight.grad = torch.ones_like(conv.weight)
+        bn.weight.grad, bn.bias.grad = torch.ones_like(bn.weight), torch.ones_like(bn.bias)
+        seen = []
+        bn.weight.register_hook(lambda g: seen.append(1) or 2 * g)
+        with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False):
+            y = fconv.conv_bn_act(conv, bn, x, relu=True)
+        (dw,) = torch.autograd.grad(y, [bn.bias], gy, retain_graph=True)
+        assert torch.equal(conv.weight.grad, torch.ones_like(conv.weight)) and not seen
+        y.backward(gy)
+        assert seen == [1]
+        return [dw, conv.weight.grad, bn.weight.grad, bn.bias.grad, x.grad]
+    a, b = _both(monkeypatch, lambda: _conv_block(3, 1, 64, 128, 2, 8, 1, False, False), call)
+    for p, q in zip(a, b):
+        _same(p, q)
+
+
+@pytest.mark.parametrize("watch", ["nothing", "post", "node", "no_buffer", "by_name"])
+def test_vector_gradients_in_place_only_where_nobody_watches(monkeypatch, watch):
+    """BatchNorm's and a linear layer's bias gradients go to the parameter's own buffer in a plain backward(); a hook behind the
+    accumulation, one on its node, a parameter without a buffer and a backward over named inputs get them as before."""
+    def make():
+        lin = nn.Linear(64, 128).to(DEV)
+        bn = DeferredBatchNorm(128).to(DEV)
+        return lin, bn, BatchNormGroup(bn, chunks=10), torch.randn(256, 64, device=DEV).bfloat16(), torch.randn(256, 128, device=DEV).bfloat16()
+
+    def call(lin, bn, group, x, g):
+        from tspipe_b200.ops import bn as fbn
+        from tspipe_b200.ops import gemm
+        ps = [lin.weight, lin.bias, bn.weight, bn.bias]
+        for p in ps:
+            p.grad = None if watch == "no_buffer" else torch.ones_like(p)
+        seen = []
+        if watch == "post":
+            for p in ps[1:]:
+                p.register_post_accumulate_grad_hook(lambda p: seen.append(p.shape))
+        nodes = [p.expand_as(p).grad_fn.next_functions[0][0] for p in ps[1:]]
+        if watch == "node":
+            for node in nodes:
+                node.register_hook(lambda *a: seen.append(1))
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = fbn.bn_act(bn, gemm.linear(x, lin.weight, lin.bias), None, True)
+        if watch == "by_name":
+            y.backward(g, inputs=ps[2:])
+            assert torch.equal(lin.bias.grad, torch.ones_like(lin.bias))
+        else:
+            y.backward(g, retain_graph=True)
+            y.backward(g)
+        assert len(seen) == (6 if watch in ("post", "node") else 0)
+        return [p.grad for p in (ps[2:] if watch == "by_name" else ps)]
+    a, b = _both(monkeypatch, make, call)
+    # (the bias in front of a BatchNorm has a gradient of zero, of which the rounding is left)
+    for p, q in zip(a, b):
+        if watch in ("by_name",) or p is not a[1]:
+            _same(p, q)
+        else:
+            assert float((p - q).abs().max()) < 0.1
+
+
+@pytest.mark.parametrize("mode", ["no_grad", "inference", "cpu_hooks", "written", "fp32_residual"])
+def test_convolution_under_other_modes(monkeypatch, mode):
+    from tspipe_b200.ops import conv as fconv
+
+    def call(conv, bn, group, x, r, gy, gx, views, fork):
+        ctx = {"no_grad": torch.no_grad, "inference": torch.inference_mode,
+               "cpu_hooks": torch.autograd.graph.save_on_cpu}.get(mode, contextlib.nullcontext)
+        with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False), ctx():
+            y = fconv.conv_bn_act(conv, bn, x, residual=r, relu=True)
+        if mode in ("no_grad", "inference"):
+            assert not y.requires_grad
+            return [y.clone()]
+        if mode == "written":                   # a weight changed in place between forward and backward is refused
+            with torch.no_grad():
+                conv.weight.mul_(2)
+            with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+                y.backward(gy)
+            return [y.detach()]
+        return [y.detach(), *torch.autograd.grad(y, [x, conv.weight, bn.weight, bn.bias, r], gy)]
+    make = lambda: _conv_block(1, 1, 64, 64, 4, 8, 1, True, False,                      # noqa: E731
+                               torch.float32 if mode == "fp32_residual" else torch.bfloat16)
+    if mode == "fp32_residual":                 # not for the C++ function: converted by the Python one
+        assert all(torch.isfinite(t).all() for t in call(*make()))
+        return
+    a, b = _both(monkeypatch, make, call)
+    for p, q in zip(a, b):
+        _same(p, q)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape,views,res,relu", [((128, 64), 1, False, True), ((256, 4096), 2, False, True),
+                                                  ((64, 72), 2, True, True), ((4, 64, 6, 5), 2, True, False)])
+def test_batchnorm(monkeypatch, shape, views, res, relu, dtype):
+    from tspipe_b200.ops import bn as fbn
+
+    def make():
+        bn = DeferredBatchNorm(shape[1]).to(DEV)
+        return (bn, BatchNormGroup(bn, chunks=10), *((_cl if len(shape) == 4 else lambda *s, dtype: torch.randn(*s, device=DEV).to(dtype))
+                                                     (*shape, dtype=dtype) for _ in range(3)))
+
+    def call(bn, group, x, r, g):
+        x.requires_grad_()
+        r.requires_grad_()
+        with fbn.segments(views):
+            y = fbn.bn_act(bn, x, r if res else None, relu)
+        return [y.detach(), group._acc, *torch.autograd.grad(y, [x, bn.weight, bn.bias] + ([r] if res else []), g)]
+    a, b = _both(monkeypatch, make, call)
+    for p, q in zip(a, b):
+        _same(p, q, 2e-3 if dtype == torch.bfloat16 else 1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,k,n,bias,grad", [((128,), 64, 64, True, False), ((4, 50), 128, 192, False, True),
+                                                ((300,), 256, 64, True, True), ((2, 100), 64, 8256, True, False)])
+def test_linear(monkeypatch, rows, k, n, bias, grad, dtype):
+    """With and without a bias and a gradient buffer, a bias wider than the column-sum kernel takes."""
+    from tspipe_b200.ops import gemm
+
+    def make():
+        m = nn.Linear(k, n, bias=bias).to(DEV)
+        if grad:
+            m.weight.grad = torch.ones_like(m.weight)
+        return m, torch.randn(*rows, k, device=DEV).to(dtype).requires_grad_(), torch.randn(*rows, n, device=DEV).bfloat16()
+
+    def call(m, x, g):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = gemm.linear(x, m.weight, m.bias)
+        gemm.clear_weight_cache()
+        y.backward(g)
+        return [y.detach(), x.grad, m.weight.grad, m.bias.grad if bias else None]
+    a, b = _both(monkeypatch, make, call)
+    for p, q in zip(a, b):
+        _same(p, q)
+
+
+@pytest.mark.parametrize("kind", ["byol", "nce"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_pair_losses(monkeypatch, kind, dtype):
+    """Value and gradients, differentiated as it is, scaled, twice, with a recorded product, under hooks, for one input."""
+    from tspipe_b200.ops import gemm
+
+    def make():
+        base = [torch.randn(160, 256, device=DEV) for _ in range(2)]
+        ts = [(base[i % 2] + 0.7 * torch.randn(160, 256, device=DEV)).to(dtype) for i in range(4)]
+        return [t.requires_grad_() for t in ts]
+
+    def call(o1, o2, t1, t2):
+        def loss():
+            return fused.byol_loss(o1, o2, t1, t2) if kind == "byol" else gemm.info_nce_pair(o1, t2, o2, t1, 0.2)
+        l0 = loss()
+        out = [l0.detach(), *torch.autograd.grad(l0, [o1, o2])]
+        l1 = loss()
+        out += torch.autograd.grad(3 * l1, [o1, o2], retain_graph=True)
+        out += torch.autograd.grad(l1, [o1, o2])
+        out += torch.autograd.grad(loss(), [o2])
+        scale = torch.ones((), device=DEV, requires_grad=True)
+        (g,) = torch.autograd.grad(loss() * scale, o1, create_graph=True)
+        out += torch.autograd.grad(g.float().sum(), scale)
+        with torch.autograd.graph.save_on_cpu():
+            l2 = loss()
+        out += torch.autograd.grad(2 * l2, [o1])
+        out.append(torch.autograd.grad(loss(), [o1], torch.full((), 2.0, device=DEV))[0])
+        return out
+    a, b = _both(monkeypatch, make, call)
+    for p, q in zip(a, b):
+        _same(p, q, 1e-5)
+    ts = make()
+    with pytest.raises(Exception):              # (teachers have no gradient)
+        torch.autograd.grad(fused.byol_loss(*ts) if kind == "byol" else gemm.info_nce_pair(ts[0], ts[3], ts[1], ts[2], 0.2), [ts[2]])

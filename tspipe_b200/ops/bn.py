@@ -185,6 +185,29 @@ class _BnAct(torch.autograd.Function):
         return dx, dw.to(ctx.wdtype), db.to(ctx.bdtype), gres, None, None, None, None, None, None, None, None, None
 
 
+def _tracked(bn, x, residual, relu, sums, segs):
+    """A layer in training whose statistics a :class:`~tspipe_b200.batchnorm.BatchNormGroup` keeps."""
+    if sums is None and type(x) is torch.Tensor:
+        host = _f.eager()
+        if host is not None:
+            y = host.bn_act(x, bn.weight, bn.bias, residual, bn.sum, bn.sum_squares, bn.count, bn.group.total, bn.eps, relu, segs)
+            if y is not None:
+                return y
+    return _BnAct.apply(x, bn.weight, bn.bias, residual, relu, bn.eps, None, bn.sum, bn.sum_squares, bn.count, sums, segs,
+                        bn.group.total)[0]
+
+
+def tracked_segments(bn, m: int, n: int, c: int) -> int:
+    """Into how many views a training-mode layer of a group takes ``n`` images with ``m`` pixels of ``c`` bf16 channels
+    (channels-last), or 0 where another path is due."""
+    from ..batchnorm import DeferredBatchNorm
+    if not (_ENABLED and isinstance(bn, DeferredBatchNorm) and bn.training and bn.group is not None and bn.affine
+            and c % 8 == 0 and c <= 4096):
+        return 0
+    segs = _SEGMENTS
+    return segs if segs <= bn.group.max_segments and n % segs == 0 and m // segs >= 2 else 0
+
+
 def bn_act(bn, x: torch.Tensor, residual: Optional[torch.Tensor] = None, relu: bool = False,
            sums: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``relu(bn(x) + residual)`` with the statistics semantics of ``bn`` (plain running-stat
@@ -210,9 +233,7 @@ def bn_act(bn, x: torch.Tensor, residual: Optional[torch.Tensor] = None, relu: b
                 finally:
                     _SEG_INDEX = 0
                 return torch.cat(outs)
-        y, _ = _BnAct.apply(x, bn.weight, bn.bias, residual, relu, bn.eps, None, bn.sum, bn.sum_squares, bn.count,
-                            sums, segs, bn.group.total)
-        return y
+        return _tracked(bn, x, residual, relu, sums, segs)
     if not applicable(bn, x):
         y = bn(x)
         if residual is not None:
@@ -225,9 +246,7 @@ def bn_act(bn, x: torch.Tensor, residual: Optional[torch.Tensor] = None, relu: b
         return y
     if isinstance(bn, DeferredBatchNorm) and bn.group is not None:
         # the partition's statistics live in flat buffers; the group commits them (one launch set per mini-batch)
-        y, _ = _BnAct.apply(x, bn.weight, bn.bias, residual, relu, bn.eps, None, bn.sum, bn.sum_squares, bn.count,
-                            sums)
-        return y
+        return _tracked(bn, x, residual, relu, sums, 1)
     if isinstance(bn, DeferredBatchNorm):
         y, _ = _BnAct.apply(x, bn.weight, bn.bias, residual, relu, bn.eps, None, bn.sum, bn.sum_squares, None, sums)
         bn.counter += m

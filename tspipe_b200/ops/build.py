@@ -24,8 +24,14 @@ HASH_PATH = LIB_PATH + ".srchash"
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-shared", "-Xcompiler", "-fPIC"]
 
+# Eager calls as C++ autograd functions (csrc/host): an extension module against the installed torch, next to the kernels
+HOST_SOURCE = os.path.join(CSRC, "host", "eager.cpp")
+HOST_NAME = "tspipe_eager"
+HOST_PATH = os.path.join(LIB_DIR, HOST_NAME + ".so")
+
 _lock = threading.Lock()
 _lib: Optional[ctypes.CDLL] = None
+_host = None
 
 
 def sources() -> List[str]:
@@ -95,3 +101,77 @@ def load() -> ctypes.CDLL:
         if _lib is None:
             _lib = ctypes.CDLL(LIB_PATH)
     return _lib
+
+
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-DTORCH_EXTENSION_NAME={HOST_NAME}"]
+
+
+def _host_command(out: str) -> List[str]:
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc_path() or "/usr/local/cuda/bin/nvcc"))
+    incl = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    return ["g++", *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[a for p in incl for a in ("-isystem", p)], HOST_SOURCE, "-o", out,
+            "-L", LIB_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
+            "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+            "-L", os.path.join(cuda, "lib64"), "-lcudart"]
+
+
+def _host_hash() -> str:
+    import sys
+
+    import torch
+    h = hashlib.sha256()
+    for f in (HOST_SOURCE, os.path.join(CSRC, "tspipe_kernels.h")):
+        with open(f, "rb") as fh:
+            h.update(fh.read())
+    h.update(f"{torch.__version__} {sys.version_info[:2]} {' '.join(HOST_FLAGS)}".encode())
+    return h.hexdigest()
+
+
+def host_is_fresh() -> bool:
+    if not (os.path.exists(HOST_PATH) and os.path.exists(HOST_PATH + ".srchash")):
+        return False
+    with open(HOST_PATH + ".srchash") as f:
+        return f.read().strip() == _host_hash()
+
+
+def build_host() -> str:
+    """Compile ``csrc/host/eager.cpp`` against the installed torch and the kernels' library."""
+    build()
+    with _lock:
+        if host_is_fresh():
+            return HOST_PATH
+        tmp = HOST_PATH + f".tmp{os.getpid()}"
+        cmd = _host_command(tmp)
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"g++ failed:\n{' '.join(cmd)}\n{res.stdout}\n{res.stderr}")
+        os.replace(tmp, HOST_PATH)
+        with open(HOST_PATH + ".srchash", "w") as f:
+            f.write(_host_hash())
+        return HOST_PATH
+
+
+def load_host():
+    """The extension module of the eager calls, built first when it is missing or stale (as :func:`load`)."""
+    global _host
+    if _host is None:
+        load()
+        if not host_is_fresh():
+            if shutil.which("g++") is not None:
+                build_host()
+            elif not os.path.exists(HOST_PATH):
+                raise RuntimeError(f"{HOST_PATH} is missing and g++ is unavailable; run __graft_entry__.build()")
+        import importlib.util
+        with _lock:
+            if _host is None:
+                spec = importlib.util.spec_from_file_location(HOST_NAME, HOST_PATH)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                _host = module
+    return _host

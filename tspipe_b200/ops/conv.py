@@ -20,6 +20,7 @@ from typing import Optional, Tuple
 import torch
 from torch import nn
 
+from . import bn as _bn
 from . import fused as _f
 from . import gemm as _gemm
 
@@ -303,6 +304,9 @@ def set_accumulate_in_place(flag: bool) -> None:
     instead of handing autograd a fresh tensor to accumulate."""
     global _ACCUMULATE_IN_PLACE
     _ACCUMULATE_IN_PLACE = bool(flag)
+    if torch.cuda.is_available():
+        _f.lib()
+        _f._build.load_host().set_accumulate(_ACCUMULATE_IN_PLACE)
 
 
 def conv2d(x: torch.Tensor, weight: torch.Tensor, stride: int = 1, want_sums: bool = False, segments: int = 1
@@ -316,13 +320,31 @@ def conv2d(x: torch.Tensor, weight: torch.Tensor, stride: int = 1, want_sums: bo
     return y, (sums if want else None)
 
 
+def _eager(conv: nn.Module, bn: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor], relu: bool, fork: bool):
+    """An eligible convolution and its training-mode BatchNorm as one C++ autograd function: ``(y,)``, with ``fork`` ``(y, x)``;
+    None where that does not apply."""
+    host = _f.eager() if type(x) is torch.Tensor else None
+    if host is None:
+        return None
+    weight, stride = conv.weight, conv.stride[0]
+    n, h, w, _, cout, k, ho, wo = _geom(x, weight, stride)
+    segs = _bn.tracked_segments(bn, n * ho * wo, n, cout)
+    if segs == 0:
+        return None
+    return host.conv_bn_act(x, weight, _w16(weight), bn.weight, bn.bias, residual, bn.sum, bn.sum_squares, bn.count,
+                            bn.group.total, bn.eps, relu, stride, segs, _stats_ok(n, ho, wo, k, stride, segs), fork,
+                            _gemm._status_word(x.device))
+
+
 def conv_bn_act(conv: nn.Module, bn: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] = None,
                 relu: bool = False) -> torch.Tensor:
     """``relu(bn(conv(x)) + residual)``.  An eligible convolution runs on the tcgen05 implicit-GEMM kernel; in front
     of a training-mode BatchNorm its epilogue already produces the BatchNorm's statistics (one pass over the
     activation less).  Everything else is the library convolution followed by :func:`tspipe_b200.ops.bn.bn_act`."""
-    from . import bn as _bn
     if _IGEMM and torch.is_autocast_enabled() and igemm_eligible(conv, x):
+        out = _eager(conv, bn, x, residual, relu, False)
+        if out is not None:
+            return out[0]
         want = bool(bn.training)
         segs = _bn.current_segments() if want else 1
         y, sums = conv2d(x, conv.weight, conv.stride[0], want_sums=want, segments=segs)
@@ -334,10 +356,12 @@ def conv_bn_act_fork(conv: nn.Module, bn: nn.Module, x: torch.Tensor, relu: bool
                      ) -> Tuple[torch.Tensor, torch.Tensor]:
     """``(relu(bn(conv(x))), x)`` for the first convolution of a residual block: the second output is ``x`` for the
     block's other branch, whose gradient the convolution's data gradient takes along (see :class:`_Conv2dFork`)."""
-    from . import bn as _bn
     if not (_IGEMM and torch.is_grad_enabled() and x.requires_grad and torch.is_autocast_enabled()
             and igemm_eligible(conv, x) and (conv.kernel_size[0], conv.stride[0]) != (1, 2)):
         return conv_bn_act(conv, bn, x, relu=relu), x
+    out = _eager(conv, bn, x, None, relu, True)
+    if out is not None:
+        return out[0], out[1]
     want = bool(bn.training)
     segs = _bn.current_segments() if want else 1
     n, h, w, _, _, k, ho, wo = _geom(x, conv.weight, conv.stride[0])

@@ -7,6 +7,8 @@ library cannot be loaded on a CUDA machine.
 from __future__ import annotations
 
 import ctypes
+import sys
+import types
 import weakref
 from typing import Optional, Sequence
 
@@ -14,8 +16,9 @@ import torch
 
 from . import build as _build
 
-LAUNCHES = 0
+_launches = 0         # by the functions of this package; LAUNCHES adds those of the C++ functions
 _lib = None
+_host = None
 _c = ctypes
 
 
@@ -51,8 +54,34 @@ def set_sm_reserve(n: int) -> None:
 
 
 def _count(n: int = 1) -> None:
-    global LAUNCHES
-    LAUNCHES += n
+    global _launches
+    _launches += n
+
+
+class _Counting(types.ModuleType):
+    @property
+    def LAUNCHES(self) -> int:
+        return _launches + (0 if _host is None else _host.launches())
+
+    @LAUNCHES.setter
+    def LAUNCHES(self, n: int) -> None:
+        global _launches
+        _launches = n - (0 if _host is None else _host.launches())
+
+
+sys.modules[__name__].__class__ = _Counting
+
+
+def eager():
+    """The C++ autograd functions (``csrc/host/eager.cpp``) for a call that is made eagerly; None while a stage is being
+    recorded, whose backward adds small gradients in place, and under a trace, which sees the calls of the Python functions."""
+    global _host
+    if IN_CAPTURE or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling():
+        return None
+    if _host is None:
+        lib()
+        _host = _build.load_host()
+    return _host
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -475,6 +504,11 @@ class _ByolBoth(torch.autograd.Function):
 
 
 def byol_loss(o1, o2, t1, t2) -> torch.Tensor:
+    host = eager() if type(o1) is torch.Tensor and type(o2) is torch.Tensor else None
+    if host is not None:
+        loss = host.byol_pair(o1, o2, t2, t1)
+        if loss is not None:
+            return loss
     n = o1.shape[0]
     if all(t.dim() == 2 and t.shape == o1.shape and t.dtype == o1.dtype and t.device == o1.device
            and t.is_contiguous() for t in (o1, o2, t1, t2)) and o1.dtype in (torch.float32, torch.bfloat16) and n > 0:

@@ -349,6 +349,11 @@ def linear_qkv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    host = _f.eager() if _two_cta and type(x) is torch.Tensor else None
+    if host is not None:
+        y = host.linear(x, weight, _w16(weight), bias, _status_word(x.device))
+        if y is not None:
+            return y
     return _Linear.apply(x, weight, bias)
 
 
@@ -561,6 +566,11 @@ def info_nce_pair(q1: torch.Tensor, k1: torch.Tensor, q2: torch.Tensor, k2: torc
         if not (t.shape == q1.shape and t.dtype == q1.dtype and t.device == q1.device and t.is_contiguous()
                 and t.data_ptr() % 16 == 0):
             return None
+    host = _f.eager() if type(q1) is torch.Tensor and type(q2) is torch.Tensor else None
+    if host is not None:
+        loss = host.nce_pair(q1, q2, k1, k2, float(temp), *nce_pair_chunks(q1.shape[0]), _status_word(q1.device))
+        if loss is not None:
+            return loss
     k1, k2 = (t.detach() if t.requires_grad else t for t in (k1, k2))
     return _NCEPair.apply(q1, q2, k1, k2, float(temp))
 
