@@ -607,16 +607,7 @@ __host__ __device__ constexpr uint32_t lanes(uint32_t code) { return code << 8 |
 constexpr uint32_t kNoTap = lanes(0xff);
 __host__ __device__ constexpr uint32_t tap_code(int ky, int kx) { return lanes((uint32_t)((2 - ky) * 4 + 2 - kx)); }
 
-// Unsigned division of numbers below 2^31 by a constant of the launch: multiply-high and shift (Granlund and Montgomery).
-struct FastDiv {
-  uint32_t d, mul, shift;
-  explicit FastDiv(uint32_t div = 1) : d(div), mul(0), shift(0) {
-    while ((1ull << shift) < d) ++shift;
-    mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
-  }
-  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(mul, n) + n) >> shift; }
-};
-
+using tsp::FastDiv;
 struct PoolGeom {
   int n, h, w, c, ho, wo;      // images of one segment, extents
   int rows;                    // output rows of a strip, which a thread walks from top to bottom

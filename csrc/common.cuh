@@ -168,6 +168,21 @@ inline int row_stride_blocks(int64_t nvec, int cpv, int threads, int per_thread,
   return (int)((g + unit - 1) / unit * unit);
 }
 
+// Unsigned division of numbers below 2^31 by a constant of the launch: multiply-high and shift (Granlund and Montgomery).
+struct FastDiv {
+  uint32_t d, mul, shift;
+  FastDiv(uint32_t div = 1) : d(div), mul(0), shift(0) {
+    while ((1ull << shift) < d) ++shift;
+    mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(mul, n) + n) >> shift; }
+  __device__ __forceinline__ uint32_t div(uint32_t n, uint32_t& rest) const {
+    const uint32_t q = div(n);
+    rest = n - q * d;
+    return q;
+  }
+};
+
 // Hyperparameters of an optimizer's parameter groups for one launch.  They change from step to step (learning rates, bias
 // corrections), so they travel with the launch: a table in device memory would have to be copied before each step.  Few
 // groups go by value; a table serves more of them.  What does not change is a code per segment: group << 1 | adapt.

@@ -67,6 +67,9 @@ struct Geom {
   int tma_store;                            // forward kernel, flat pixel grid: the epilogue writes with TMA stores
   int n_fastest;                            // tile index = m_tile * tiles_n + n_tile (else n_tile * tiles_m + m_tile)
   unsigned long long wait_ns;               // give-up time of every mbarrier wait
+  // divisors that every role meets once or more per tile (a division by a number the compiler does not know is some thirty
+  // instructions, and the nine of a tile were more than half of what an epilogue warp issued for it)
+  tsp::FastDiv by_tiles_w, by_tiles_h, by_order, by_seg;      // by_order: channel tiles or pixel tiles, see split_tile
   int n_taps;
   int kc;                                   // channels per tap on the contraction side (forward) / on the M side (wgrad)
   int nc;                                   // channels on the N side
@@ -110,16 +113,26 @@ __device__ __forceinline__ int tile_begin(int num_tiles, unsigned cta) {
 // Split a tile index into (pixel tile, channel tile).  With statistics a CTA should stay on one channel block (one set
 // of accumulators, few flushes): channel-major.  Without, channel tiles run fastest: the CTAs that run together share
 // a pixel tile's input (fetched from DRAM once, then from L2) and sweep the weights, which stay in L2.
-__device__ __forceinline__ void split_tile(const Geom& g, int t, int tiles_m, int tiles_nn, int& tm, int& tn) {
-  if (g.n_fastest) { tm = t / tiles_nn; tn = t % tiles_nn; }
-  else { tm = t % tiles_m; tn = t / tiles_m; }
+__device__ __forceinline__ void split_tile(const Geom& g, int t, int& tm, int& tn) {
+  uint32_t rest;
+  const uint32_t q = g.by_order.div((uint32_t)t, rest);
+  tm = (int)(g.n_fastest ? q : rest);
+  tn = (int)(g.n_fastest ? rest : q);
+}
+// Of a geometry that is complete, for `tiles_nn` channel tiles.
+inline void set_divisors(Geom& g, int tiles_nn) {
+  g.by_tiles_w = tsp::FastDiv(g.tiles_w);
+  g.by_tiles_h = tsp::FastDiv(g.tiles_h);
+  g.by_order = tsp::FastDiv(g.n_fastest ? tiles_nn : g.tiles_w * g.tiles_h * g.tiles_n);
+  g.by_seg = tsp::FastDiv(g.rows_per_seg > 0 ? g.rows_per_seg : 1);
 }
 
 __device__ __forceinline__ void tile_origin(const Geom& g, int tm, int& w0, int& h0, int& n0) {
-  const int wb = tm % g.tiles_w, r = tm / g.tiles_w;
-  w0 = wb * g.box_w;
-  h0 = (r % g.tiles_h) * g.box_h;
-  n0 = (r / g.tiles_h) * g.box_n;
+  uint32_t wb, hb;
+  const uint32_t r = g.by_tiles_w.div((uint32_t)tm, wb), nb = g.by_tiles_h.div(r, hb);
+  w0 = (int)wb * g.box_w;
+  h0 = (int)hb * g.box_h;
+  n0 = (int)nb * g.box_n;
 }
 
 // Epilogue warps (from 2 on) of the forward / data-gradient kernels.  A tile has `n_sub` accumulators of 128 rows (SUBS
@@ -168,24 +181,29 @@ __device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int t
       }
     }
   };
+  // the lane's pixel of each accumulator within the box, far outside the image for a row that is none
+  int3 in_box[SUBS];
+#pragma unroll
+  for (int sub = 0; sub < SUBS; ++sub) {
+    const int p = sub * 128 + quarter * 32 + lane, r2 = p / g.row_pitch;
+    in_box[sub] = make_int3(p - r2 * g.row_pitch, r2 % g.box_h, r2 / g.box_h);
+    if (p >= g.pix || in_box[sub].x >= g.box_w) in_box[sub].x = 1 << 30;
+  }
   const int t_begin = tile_begin(num_tiles, blockIdx.x), t_end = tile_begin(num_tiles, blockIdx.x + 1);
   for (int t = t_begin; t < t_end && ok; ++t, ++lt) {
     int w0, h0, n0, tm, tn;
-    split_tile(g, t, tiles_m, (g.nc + BN - 1) / BN, tm, tn);
+    split_tile(g, t, tm, tn);
     tile_origin(g, tm, w0, h0, n0);
     const int c0 = tn * BN;
     const uint32_t acc = lt % ACC_BUFS, use = lt / ACC_BUFS;
     if (STATS) {
-      const int seg = (int)((((int64_t)n0 * g.out_h + h0) * g.out_w + w0) / g.rows_per_seg);
+      const int seg = (int)g.by_seg.div((uint32_t)((n0 * g.out_h + h0) * g.out_w + w0));       // (fewer than 2^31 pixels)
       if (c0 != cur_c0 || seg != cur_seg) { flush_stats(); cur_c0 = c0; cur_seg = seg; }
     }
     // a lane's pixel and where it is stored (units of 8 elements), -1 for rows that are not stored
     auto pixel_off = [&](int sub) -> int {
-      const int p = sub * 128 + quarter * 32 + lane;
-      const int bw = p % g.row_pitch, r2 = p / g.row_pitch;
-      const int w = w0 + bw, h = h0 + r2 % g.box_h, n = n0 + r2 / g.box_h;
-      return p < g.pix && bw < g.box_w && w < g.out_w && h < g.out_h && n < g.out_n
-                 ? n * g.out_sn + h * g.out_sh + w * g.out_sw : -1;
+      const int w = w0 + in_box[sub].x, h = h0 + in_box[sub].y, n = n0 + in_box[sub].z;
+      return w < g.out_w && h < g.out_h && n < g.out_n ? n * g.out_sn + h * g.out_sh + w * g.out_sw : -1;
     };
     const int pc = lane & 7;
     auto takes = [&](int sub) -> bool { return kShare == 1 || (int)((lt * n_sub + sub) % kShare) == group / kBlocks; };
@@ -343,7 +361,7 @@ __device__ __forceinline__ void add_epilogue(const Geom& g, int num_tiles, int t
   const int units = idle ? 0 : (t_end - t_begin) * kMine;
   auto place = [&](int u, int& col, int& row) {
     int w0, h0, n0, tm, tn;
-    split_tile(g, t_begin + u / kMine, tiles_m, (g.nc + BN - 1) / BN, tm, tn);
+    split_tile(g, t_begin + u / kMine, tm, tn);
     tile_origin(g, tm, w0, h0, n0);
     col = tn * BN + 64 * (kBlocks == 1 ? 0 : 2 * (u % kMine) + group);
     row = w0 + quarter * 32;
@@ -470,7 +488,7 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       const uint32_t tx = (uint32_t)(g.pix * 128 + C::kBBytes);     // a box is written in full, zero fill included
       for (int t = tile_begin(num_tiles, blockIdx.x); t < tile_begin(num_tiles, blockIdx.x + 1) && ok; ++t) {
         int w0, h0, n0, tm, tn;
-        split_tile(g, t, tiles_m, tiles_nn, tm, tn);
+        split_tile(g, t, tm, tn);
         tile_origin(g, tm, w0, h0, n0);
         const int c0 = tn * BN;
         for (int tap = 0; tap < g.n_taps && ok; ++tap) {
@@ -651,7 +669,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
       auto load_a = [&](int u) -> bool {
         const int t = t_first + u / kcb, cb = u % kcb;
         int w0, h0, n0, tm, tn;
-        split_tile(g, t, tiles_m, tiles_nn, tm, tn);
+        split_tile(g, t, tm, tn);
         tile_origin(g, tm, w0, h0, n0);
         const int s = u % C::kAStages;
         const uint32_t round = (uint32_t)u / C::kAStages;
@@ -666,7 +684,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         if (resident && u > 0) continue;
         const int t = t_first + u / kcb, cb = u % kcb;
         int tm, tn;
-        split_tile(g, t, tiles_m, tiles_nn, tm, tn);
+        split_tile(g, t, tm, tn);
         const int c0 = tn * BN;
         for (int tap = 0; tap < 9; ++tap, ++ib) {
           const int s = ib % C::kBStages;
@@ -1295,6 +1313,7 @@ int launch_fwd(const Plan& p, const CUtensorMap& wmap, void* out, const void* ad
   CUtensorMap omap = wmap, addmap = wmap;
   g.tma_store = 0;
   g.n_fastest = STATS ? 0 : 1;
+  set_divisors(g, (g.nc + BN - 1) / BN);
   if (g.out_h == 1 && g.out_n == 1 && g.out_sw * 8 == g.nc && g.box_w == 128) {
     const uint64_t dims[2] = {(uint64_t)g.nc, (uint64_t)g.out_w};
     const uint64_t strides[2] = {2, (uint64_t)g.nc * 2};
@@ -1356,6 +1375,7 @@ template <int BN, bool B_MN, bool STATS, bool ADD>
 int launch_halo(Geom& g, const CUtensorMap& amap, const CUtensorMap& wmap, void* out, const void* addend, float* col_sums,
                 int* status, cudaStream_t stream) {
   g.n_fastest = STATS ? 0 : 1;
+  set_divisors(g, (g.nc + BN - 1) / BN);
   auto kern = conv_halo_kernel<BN, B_MN, STATS, ADD>;
   static bool attr_set[64] = {};
   int dev = 0;
@@ -1406,7 +1426,8 @@ int launch_wgrad(const Plan& p, const CUtensorMap& dymap, float* dw, int* status
     if (e != cudaSuccess) return (int)e;
     attr_set[dev] = true;
   }
-  const Geom& g = p.g;
+  Geom g = p.g;
+  set_divisors(g, 1);
   const int m_tiles = (g.n_taps * (g.kc / 64) + 1) / 2, n_tiles = (g.nc + BN - 1) / BN;
   const int items = m_tiles * n_tiles * g.splits;
   const int n_sm = sm_count();
@@ -1422,6 +1443,7 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int n, int h, in
       !act_map(&dymap, dy, 64, w, h, n, 64, (int64_t)w * 64, (int64_t)h * w * 64, g.row_pitch, g.box_h, 1))
     return -6;
   for (int t = 0; t < 9; ++t) g.tap_off[t] = (t / 3) * g.row_pitch + t % 3;
+  set_divisors(g, 1);
   auto kern = conv_wgrad_halo_kernel;
   static bool attr_set[64] = {};
   int dev = 0;
