@@ -38,6 +38,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t addr, uint32_t parity) {
   return done != 0;
 }
 
+// Whether a phase is complete, without waiting.  An issuing warp that looks at the barrier of the next operands before it issues
+// the products of these has the some 250 clocks covered that a wait which is already over takes, from the look to the first product
+// behind it.  (Pays in conv_fwd_kernel only: the CTA-pair products and the bordered boxes have twice the products behind a wait.)
+__device__ __forceinline__ bool mbar_over(uint64_t* bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
 // A role whose wait ran out pauses before it leaves: what its CTA has in flight (copies into shared memory, products, all of
 // which take microseconds) lands before the barrier in front of the kernel's end lets the memory go to another block.
 __device__ __forceinline__ void drain_in_flight() {
