@@ -68,6 +68,8 @@ Tensor gradient_like(Tensor g, const Tensor& like) {
   return aligned(g) ? g : g.clone(at::MemoryFormat::Preserve);
 }
 
+bool owns_saved() { return !at::SavedTensorDefaultHooks::get_hooks().has_value(); }
+
 // The fp32 gradient of a leaf that a kernel can add to in place: the weight's elements in the order [rows][taps][columns].
 Tensor grad_target(const Tensor& weight) {
   if (!g_accumulate.load(std::memory_order_relaxed) || !weight.is_leaf()) return {};
@@ -181,7 +183,11 @@ struct ConvBnAct : Function<ConvBnAct> {
     const bool has_res = res.has_value();
     bn_apply(y, res.value_or(Tensor()), out, s, bn_w, bn_b, acc, g.pixels(), g.cout, eps, relu, (int)segs, st);
     ctx->set_materialize_grads(false);
-    ctx->save_for_backward({x, weight, bn_w, bn_b, y, sums, relu && has_res ? out : Tensor()});
+    // The convolution's output is for the first half of the backward alone and is let go behind it (hooks on saved tensors get
+    // it as all others).
+    const bool own = owns_saved();
+    if (own) ctx->saved_data["y"] = y;
+    ctx->save_for_backward({x, weight, bn_w, bn_b, own ? Tensor() : y, sums, relu && has_res ? out : Tensor()});
     ctx->saved_data["w16"] = w16;             // (not for hooks on saved tensors, which may hand back copies)
     ctx->saved_data["status"] = status;
     ctx->saved_data["o"] = std::vector<int64_t>{stride, segs, relu, has_res, fork};
@@ -199,8 +205,13 @@ struct ConvBnAct : Function<ConvBnAct> {
       return r;
     }
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &weight = saved[1], &bn_w = saved[2], &bn_b = saved[3], &y = saved[4], &sums = saved[5],
-                 &out = saved[6], w16 = ctx->saved_data["w16"].toTensor();
+    const Tensor &x = saved[0], &weight = saved[1], &bn_w = saved[2], &bn_b = saved[3], &sums = saved[5], &out = saved[6],
+                 w16 = ctx->saved_data["w16"].toTensor();
+    Tensor y = saved[4];
+    if (!y.defined()) {
+      y = ctx->saved_data["y"].toTensor();
+      if (!torch::autograd::get_current_graph_task_keep_graph()) ctx->saved_data.erase("y");
+    }
     int* word = ctx->saved_data["status"].toTensor().data_ptr<int>();
     const int segs = (int)o[1];
     const bool relu = o[2] != 0, has_res = o[3] != 0;
@@ -210,6 +221,7 @@ struct ConvBnAct : Function<ConvBnAct> {
     const ConvGeom g(x, weight, o[0]);
     const BnGrads b = bn_backward(gradient_like(grads[0], y), y, out, sums.data_ptr<float>() + (int64_t)segs * 2 * g.cout, bn_w,
                                   bn_b, relu, has_res, ctx->needs_input_grad(3) && ctx->needs_input_grad(4), g.pixels(), g.cout, segs, st);
+    y = Tensor();
     if (ctx->needs_input_grad(3)) r[3] = b.dw;
     if (ctx->needs_input_grad(4)) r[4] = b.db;
     r[5] = b.dres;
@@ -368,7 +380,6 @@ Tensor scaled(const Tensor& g, const Tensor& gout, bool own) {
   g_launches += 1;
   return out;
 }
-bool owns_saved() { return !at::SavedTensorDefaultHooks::get_hooks().has_value(); }
 
 // Both directions of a symmetric loss: forward leaves the loss and [2][n][d] gradients of the two students.
 variable_list pair_backward(AutogradContext* ctx, const variable_list& grads, int args) {
