@@ -107,12 +107,14 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
 #pragma unroll
     for (int e = 0; e < 8; ++e) { adw[k][e] = 0.f; adb[k][e] = 0.f; }
   for (int row = blockIdx.x * kLnBwdWarps + warp; row < rows; row += gridDim.x * kLnBwdWarps) {
-    tsp::Raw8<T> xr[NV], gr[NV];
+    tsp::Raw8<T> xr[NV], gr[NV], kr[ADD ? NV : 1];
 #pragma unroll
     for (int k = 0; k < NV; ++k)
       if (lane + 32 * k < nvec) {
-        tsp::ldraw(x + (int64_t)row * d, (int64_t)(lane + 32 * k) * 8, xr[k]);
-        tsp::ldraw(dy + (int64_t)row * d, (int64_t)(lane + 32 * k) * 8, gr[k]);
+        const int64_t at = (int64_t)row * d + (lane + 32 * k) * 8;
+        tsp::ldraw(x, at, xr[k]);
+        tsp::ldraw(dy, at, gr[k]);
+        if constexpr (ADD) tsp::ldraw(skip, at, kr[k]);
       }
     const float mu = mean[row], rs = rstd[row];
     float s1 = 0.f, s2 = 0.f;
@@ -148,7 +150,7 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
         for (int e = 0; e < 8; ++e) o[e] = rs * (gv[e] * wv[e] - s1 - (xv[e] - mu) * rs * s2);
         if constexpr (ADD) {
           float sv[8];
-          tsp::ld8(skip + (int64_t)row * d, (int64_t)vi * 8, sv);
+          tsp::cvt8(kr[k], sv);
           tsp::round_as<T>(o);
 #pragma unroll
           for (int e = 0; e < 8; ++e) o[e] += sv[e];
