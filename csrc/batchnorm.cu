@@ -53,7 +53,10 @@ __global__ void __launch_bounds__(kBlock, 2) bn_colsum_kernel(const T* __restric
                                                            int relu, int64_t m, int c, float* __restrict__ out) {
   tsp::let_next_start();
   __shared__ float sm[(kBlock + 4) * 16];
-  {   // blockIdx.z = segment: an independent group of m rows with its own statistics
+  if constexpr (MODE == 2) {     // blockIdx.z = one of up to three matrices (x, dy, y), whose sums lie side by side
+    if (blockIdx.z != 0) x = blockIdx.z == 1 ? dy : y;
+    out += (int64_t)blockIdx.z * c;
+  } else {   // blockIdx.z = segment: an independent group of m rows with its own statistics
     const int64_t so = (int64_t)blockIdx.z * m * c;
     x += so;
     if (dy != nullptr) dy += so;
@@ -1104,19 +1107,26 @@ int tsp_bn_stats(const void* x, int64_t m, int c, int dtype, float* sums, int se
 
 // sums [c] fp32 = (or, with `add`, +=) column sums of x [m, c] (the gradient of a bias).
 int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, int add, cudaStream_t stream) {
+  return tsp_col_sums_of(&x, 1, m, c, dtype, sums, add, stream);
+}
+
+// The same of n_src (at most three) matrices of m rows and c columns each, in one launch: sums [n_src][c].  The gradients of q, k and
+// v, 12608 rows of 768 columns each, B200, from memory: 22.5 us as three launches, 18.0 as one.
+int tsp_col_sums_of(const void* const* x, int n_src, int64_t m, int c, int dtype, float* sums, int add, cudaStream_t stream) {
   if (m <= 0) return 0;
-  if (c % 8 != 0 || c > 8192) return -3;
-  cudaError_t e = add ? cudaSuccess : cudaMemsetAsync(sums, 0, sizeof(float) * (size_t)c, stream);
+  if (c % 8 != 0 || c > 8192 || n_src < 1 || n_src > 3) return -3;
+  cudaError_t e = add ? cudaSuccess : cudaMemsetAsync(sums, 0, sizeof(float) * (size_t)c * n_src, stream);
   if (e != cudaSuccess) return (int)e;
   const Tile tl = make_tile(c / 8);
   const int slabs = (c / 8 + tl.tx_n - 1) / tl.tx_n;
-  const dim3 grid(row_blocks(m, tl.ty_n, (dtype == TSP_DTYPE_BF16 ? ColsumRows<__nv_bfloat16, 2>::value : ColsumRows<float, 2>::value), slabs, 1), slabs, 1);
-  if (dtype == TSP_DTYPE_BF16)
-    bn_colsum_kernel<__nv_bfloat16, 2><<<grid, kBlock, 0, stream>>>((const __nv_bfloat16*)x, nullptr, nullptr, nullptr,
-                                                                    nullptr, nullptr, nullptr, 0, m, c, sums);
-  else
-    bn_colsum_kernel<float, 2><<<grid, kBlock, 0, stream>>>((const float*)x, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                            nullptr, 0, m, c, sums);
+  const dim3 grid(row_blocks(m, tl.ty_n, (dtype == TSP_DTYPE_BF16 ? ColsumRows<__nv_bfloat16, 2>::value : ColsumRows<float, 2>::value), slabs, n_src), slabs, n_src);
+  const void *x1 = n_src > 1 ? x[1] : nullptr, *x2 = n_src > 2 ? x[2] : nullptr;
+  auto run = [&](auto kern, auto* p0, auto* p1, auto* p2) {
+    kern<<<grid, kBlock, 0, stream>>>(p0, p1, p2, nullptr, nullptr, nullptr, nullptr, 0, m, c, sums);
+  };
+  using B = __nv_bfloat16;
+  if (dtype == TSP_DTYPE_BF16) run(bn_colsum_kernel<B, 2>, (const B*)x[0], (const B*)x1, (const B*)x2);
+  else run(bn_colsum_kernel<float, 2>, (const float*)x[0], (const float*)x1, (const float*)x2);
   return TSP_LAUNCH_CHECK();
 }
 

@@ -65,6 +65,7 @@ int tsp_gelu_bwd_sums(const void* dy, const void* x, const float* bias, void* dx
 int tsp_bn_stats(const void* x, int64_t m, int c, int dtype, float* sums, int segs, cudaStream_t stream);
 int tsp_bn_stream_status(int reset);
 int tsp_col_sums(const void* x, int64_t m, int c, int dtype, float* sums, int add, cudaStream_t stream);
+int tsp_col_sums_of(const void* const* x, int n_src, int64_t m, int c, int dtype, float* sums, int add, cudaStream_t stream);
 int tsp_bn_apply(const void* x, const void* res, void* y, const float* sums, const float* fixed_mean_var,
                  const float* w, const float* b, float* save_mean_rstd, float* acc_sum, float* acc_sumsq,
                  float* acc_count, int64_t acc_seg_stride, int64_t m, int c, float eps, int relu, int dtype, int segs,

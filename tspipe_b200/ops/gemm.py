@@ -138,6 +138,21 @@ def _column_sums(dy2: torch.Tensor, out: Optional[torch.Tensor] = None, add_to: 
     return None if add_to is not None else sums
 
 
+def _column_sums_of(dys, out: torch.Tensor, add: bool) -> None:
+    """fp32 column sums of up to three bf16 matrices of one shape, side by side into ``out`` (``add``: on top of it)."""
+    m, n = dys[0].shape
+    if n % 8 or n > 8192 or m < 2:
+        for i, dy in enumerate(dys):
+            part = out[i * n: (i + 1) * n]
+            _column_sums(dy, *((None, part) if add else (part,)))
+        return
+    ptrs = (_c.c_void_p * len(dys))(*(t.data_ptr() for t in dys))
+    with _f.on_device(out.device):
+        _f._check(_f.lib().tsp_col_sums_of(ptrs, _c.c_int(len(dys)), _c.c_int64(m), _c.c_int(n), _c.c_int(_f._dt(dys[0])),
+                                           _f._ptr(out), _c.c_int(1 if add else 0), _f._stream()), "tsp_col_sums_of")
+    _f._count()
+
+
 def matmul_nn(a, b: torch.Tensor) -> torch.Tensor:
     """``[a_0 | a_1 | ..] @ b`` (bf16, fp32 accumulation): ``a`` = up to three ``[M, K_i]`` matrices of one width, ``b
     [K, N]`` read in place as MN-major tiles.  ``dX = dY @ W`` of a linear layer, or of layers that share their input."""
@@ -271,9 +286,7 @@ class _LinearQKV(torch.autograd.Function):
             gb = _f.recorded_grad(ctx.bias)
             if gb is None:
                 db = torch.empty(n, dtype=torch.float32, device=x2.device)
-            for i in range(3):
-                rows = slice(i * c, (i + 1) * c)
-                _column_sums(dy2[i], *((None, gb[rows]) if db is None else (db[rows],)))
+            _column_sums_of(dy2, db if db is not None else gb, db is None)
             db = None if db is None else db.to(ctx.dtypes[2])
         return dx, dw, db
 
