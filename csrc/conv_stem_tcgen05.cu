@@ -60,12 +60,17 @@ constexpr int kMBlockBytes = 128 * 128;   // 128 pixels x 64 channels of dY
 constexpr int kBBlockBytes = kCout * 128;
 constexpr int kBBytes = 4 * kBBlockBytes; // weights: 14 x 16 of the contraction, in blocks of 64
 constexpr int kStoreBufBytes = 32 * 128;
-constexpr int kEpiWarps = 8;
+// Epilogue warps: one per output row of a tile and TMEM lane quarter where statistics are formed and a CTA has tiles enough to make
+// up for its larger start (128 images of 224 x 224, B200: 76.8 us with eight, 69 with sixteen; 37 of 192 x 192 22.9 and 22.0, 16 of
+// 160 x 160 14.4 and 14.8, 8 of 96 x 96 9.1 and 10.2; without statistics 57 and 61), half of them with two rows each elsewhere.
+constexpr int kManyWarps = 16, kFewWarps = 8, kManyTiles = 5;
+constexpr int kWeightWarps = 8;          // of them, those that lay out the weights
+constexpr int kStagingBytes = 16 * kStoreBufBytes;
 constexpr int kTileRows = 4;
 constexpr int kAccs = 2;
 constexpr int kLoaders = 8;               // warps that fill the ring
-constexpr int kThreads = (kLoaders + 1 + kEpiWarps) * 32;
-constexpr int kSmemBytes = kBBytes + 2 * kEpiWarps * kStoreBufBytes + 2 * kRingBytes + 1024 + 256;
+__host__ __device__ constexpr int threads_with(int epi_warps) { return (kLoaders + 1 + epi_warps) * 32; }
+constexpr int kSmemBytes = kBBytes + kStagingBytes + 2 * kRingBytes + 1024 + 256;
 constexpr int kWgThreads = (kLoaders + 2) * 32;
 constexpr int kWgRows = kRows - 4 + 16;   // rows that a product may touch from the last tile start on
 constexpr int kDyStages = 2;
@@ -76,7 +81,7 @@ constexpr uint64_t kWaitNs = 2000000000ull;
 // which neither rows nor columns meet in a bank
 constexpr int kPartPitch = kCout + 4, kPartFloats = kK * kPartPitch, kPartAt = 9408;
 static_assert(kPartAt >= kCout * kK && (kPartAt + 2 * kPartFloats) * 4 <= kDyStages * kDyBytes, "sums and parts in two tiles of dY");
-static_assert(kCout * kKPad * 2 <= 2 * kEpiWarps * kStoreBufBytes, "the weights in the staging buffers");
+static_assert(kCout * kKPad * 2 <= kStagingBytes, "the weights in the staging buffers");
 
 using tc5::mbar_arrive;
 using tc5::mbar_expect_tx;
@@ -202,14 +207,16 @@ __device__ __forceinline__ void zero_margins(uint8_t* ring, int rows, int first,
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+template <int EPI>
+__global__ void __launch_bounds__(threads_with(EPI), 1)
 conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__ CUtensorMap tmap_y,
                  const __nv_bfloat16* __restrict__ x, int n_img, int h, int w, int oh_n, int ow_n, int imgs_per_seg,
                  float* __restrict__ sums, int* __restrict__ status) {
+  constexpr int kThreads = threads_with(EPI), kRowsEach = 16 / EPI;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* b_tile = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* store_bufs = b_tile + kBBytes;
-  uint8_t* ring = store_bufs + 2 * kEpiWarps * kStoreBufBytes;
+  uint8_t* ring = store_bufs + kStagingBytes;
   uint8_t* shifted = ring + kRingBytes;
   uint64_t* bars = (uint64_t*)(shifted + kRingBytes);
   uint64_t* full_bar = bars;                     // [kBatches]  rows -> MMA (one arrival per loading warp)
@@ -228,9 +235,9 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
 
   if (tid == 0) {
     for (int b = 0; b < kBatches; ++b) { mbar_init(full_bar + b, kLoaders); mbar_init(empty_bar + b, 1); }
-    for (int a = 0; a < kAccs; ++a) { mbar_init(tmem_full_bar + a, 1); mbar_init(tmem_empty_bar + a, kEpiWarps); }
+    for (int a = 0; a < kAccs; ++a) { mbar_init(tmem_full_bar + a, 1); mbar_init(tmem_empty_bar + a, EPI); }
     mbar_init(weight_bar, 1);
-    mbar_init(ready_bar, kEpiWarps);
+    mbar_init(ready_bar, kWeightWarps);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_expect_tx(weight_bar, kCout * kKPad * 2);
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(store_bufs)),
@@ -311,9 +318,9 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
     // First the weights as the products take them, while the loaders fill the ring: step 2 kh + half, element 4 * tap + channel, taps
     // 0..3 and 3..6 (128-byte swizzle), from a copy in the staging buffers.  (By all warps before their roles began, from
     // memory element by element, they made every call 2 us longer: 8 images of 96 x 96 10.8 us, 9.1 this way.)
-    tc5::mbar_wait(weight_bar, 0, status, 6, kWaitNs);
     const __nv_bfloat16* raw = reinterpret_cast<const __nv_bfloat16*>(store_bufs);
-    {
+    if (warp <= kLoaders + kWeightWarps) {
+      tc5::mbar_wait(weight_bar, 0, status, 6, kWaitNs);
       const int e = tid - (kLoaders + 1) * 32, kh = (e >> 3) & 7, half = (e >> 2) & 1, tap = 3 * half + (e & 3);
       const int step = 2 * kh + half, piece = 2 * (step & 3) + ((e >> 1) & 1);
       const __nv_bfloat16* at = raw + kh * 21 + tap * 3;
@@ -340,12 +347,12 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
           *reinterpret_cast<uint2*>(to + (co0 + 4 * k) * 128 + ((piece ^ ((co0 + 4 * k) & 7)) << 4)) =
               make_uint2(*reinterpret_cast<const uint32_t*>(&v[k][0]), *reinterpret_cast<const uint32_t*>(&v[k][1]));
       }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ready_bar);
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) mbar_arrive(ready_bar);
     const int quarter = warp & 3, group = (warp - kLoaders - 1) >> 2;
-    uint8_t* bufs = store_bufs + (warp - kLoaders - 1) * 2 * kStoreBufBytes;
+    uint8_t* bufs = store_bufs + (warp - kLoaders - 1) * kRowsEach * kStoreBufBytes;      // a staging block per row
     tc5::ColSums cs;
     cs.clear();
     int cur_seg = -1;
@@ -365,8 +372,8 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
     uint32_t stores = 0;
     bool ok = true;
     for (int t = t_begin; t < t_end && ok; ++t) {
-      const uint32_t it = t - t_begin;
-      const int n = t / per_image, oh = (t - n * per_image) * kTileRows + 2 * group;
+      const uint32_t it = t - t_begin, first_store = stores;
+      const int n = t / per_image, oh = (t - n * per_image) * kTileRows + kRowsEach * group;
       const int seg = n / imgs_per_seg;                    // statistics are kept per group of images
       if (seg != cur_seg) { flush_sums(); cur_seg = seg; }
       const uint32_t acc = it % kAccs;
@@ -374,10 +381,14 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-      for (int j = 0; j < 2 && oh + j < oh_n; ++j) {
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (acc * 2 + group) * 2 * kCout + (j == 0 ? kCout : 0);
-        uint8_t* buf = bufs + (stores++ & 1) * kStoreBufBytes;
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");    // the store before the last has read it
+      for (int j = 0; j < kRowsEach && oh + j < oh_n; ++j) {
+        const int row = kRowsEach * group + j;             // of the tile: columns 64..127 of its pair's accumulator are the first one's
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (acc * 2 + (row >> 1)) * 2 * kCout + ((row & 1) == 0 ? kCout : 0);
+        uint8_t* buf = bufs + stores++ % kRowsEach * kStoreBufBytes;
+        if (lane == 0) {                                   // the last store from it has read it
+          if (kRowsEach == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        }
         __syncwarp();
         uint8_t* my_row = buf + lane * 128;
         const bool keep = row0 + lane < ow_n;              // (the products' rows past the output row hold what lies there)
@@ -404,11 +415,12 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
           if (row0 < ow_n) tma_store_3d(&tmap_y, buf, 0, row0, n * oh_n + oh + j);
           else asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
-        if (sums != nullptr) cs.add(buf, lane);            // statistics of the rounded outputs
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(tmem_empty_bar + acc);
+      if (sums != nullptr)                                 // statistics of the rounded outputs, the accumulator being free again
+        for (int j = 0; j < kRowsEach && oh + j < oh_n; ++j) cs.add(bufs + (first_store + j) % kRowsEach * kStoreBufBytes, lane);
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     __syncwarp();
@@ -426,11 +438,11 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
   if (sums != nullptr && tid < 2 * kCout) {
     // (additions to one sector are serialised: 8 warps x 2 instructions from each of 148 CTAs cost some 30 us)
     const float* st = reinterpret_cast<const float*>(store_bufs);
-    constexpr int kWarpFloats = 2 * kStoreBufBytes / 4;
+    constexpr int kWarpFloats = kRowsEach * kStoreBufBytes / 4;
     const int seg = __float_as_int(st[2 * kCout]);
     bool same = seg >= 0;
     float v = 0.f;
-    for (int q = 0; q < kEpiWarps; ++q) {
+    for (int q = 0; q < EPI; ++q) {
       v += st[q * kWarpFloats + tid];
       same = same && __float_as_int(st[q * kWarpFloats + 2 * kCout]) == seg;      // (else a wait ran out)
     }
@@ -686,7 +698,9 @@ int tsp_conv_stem_fwd(const void* x, const void* wmat, void* y, float* sums, int
   cudaGetDevice(&dev);
   dev &= 63;
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(conv_stem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(conv_stem_kernel<kFewWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(conv_stem_kernel<kManyWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     cudaDeviceGetAttribute(&n_sm[dev], cudaDevAttrMultiProcessorCount, dev);
     if (n_sm[dev] <= 0) n_sm[dev] = 148;
@@ -695,7 +709,12 @@ int tsp_conv_stem_fwd(const void* x, const void* wmat, void* y, float* sums, int
   const int tiles = n * ((oh + kTileRows - 1) / kTileRows);
   const int usable = n_sm[dev] - g_tsp_sm_reserve > 8 ? n_sm[dev] - g_tsp_sm_reserve : 8;
   const int grid = tiles < usable ? tiles : usable;
-  conv_stem_kernel<<<grid, kThreads, kSmemBytes, stream>>>((const __nv_bfloat16*)wmat, ty, (const __nv_bfloat16*)x, n, h, w, oh, ow, n / segs, sums, status);
+  auto run = [&](auto kern, int threads) {
+    kern<<<grid, threads, kSmemBytes, stream>>>((const __nv_bfloat16*)wmat, ty, (const __nv_bfloat16*)x, n, h, w, oh, ow, n / segs,
+                                                sums, status);
+  };
+  if (sums != nullptr && tiles >= kManyTiles * usable) run(conv_stem_kernel<kManyWarps>, threads_with(kManyWarps));
+  else run(conv_stem_kernel<kFewWarps>, threads_with(kFewWarps));
   return TSP_LAUNCH_CHECK();
 }
 

@@ -34,7 +34,7 @@ def test_stem_conv_matches_fp32_reference(n, h, w):
     torch.testing.assert_close(weight.grad, wr.grad, rtol=5e-2, atol=5e-2 * wr.grad.abs().max().item())
 
 
-@pytest.mark.parametrize("n,h,w", [(1, 8, 8), (2, 10, 16), (3, 50, 200), (37, 18, 224), (1, 600, 24)])
+@pytest.mark.parametrize("n,h,w", [(1, 8, 8), (2, 10, 16), (3, 50, 200), (37, 18, 224), (1, 600, 24), (250, 18, 40), (372, 10, 16)])
 def test_stem_conv_rows_and_runs(n, h, w):
     """Widths whose rows end inside a product, odd numbers of output rows, CTAs that begin and end inside an image; infinite and
     NaN pixels reach the outputs whose window holds them and no other."""
