@@ -236,8 +236,7 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const T* __restrict__ x, 
       if (i + u * stride < nv) {
         float v[8];
         tsp::cvt8(raw[u], v);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = tsp::gelu_f<T>(v[e] + b[e]);
+        tsp::gelu_all<T>(v, b);
         tsp::st8(y, (i + u * stride) * 8, v);
       }
   }
@@ -265,8 +264,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const T* __restrict__ dy,
         float v[8], g[8];
         tsp::cvt8(xr[u], v);
         tsp::cvt8(gr[u], g);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) g[e] *= tsp::gelu_grad_f<T>(v[e] + b[e]);
+        tsp::times_gelu_grad<T>(g, v, b);
         tsp::st8(dx, (i + u * stride) * 8, g);
       }
   }
@@ -301,8 +299,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_sums_kernel(const T* __restrict_
         float v[8], g[8];
         tsp::cvt8(xr[u], v);
         tsp::cvt8(gr[u], g);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) g[e] *= tsp::gelu_grad_f<T>(v[e] + b[e]);
+        tsp::times_gelu_grad<T>(g, v, b);
         tsp::round_as<T>(g);
         tsp::st8(dx, (r + u * step) * d + col, g);
 #pragma unroll

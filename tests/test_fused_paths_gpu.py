@@ -428,6 +428,25 @@ def test_gelu_special_values_and_wide_bias(dtype):
             assert _rel(a, w) < 2 * EPS[dtype] + 1e-6
 
 
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gelu_of_every_bf16_argument(shift):
+    """Two values share an instruction: each is its own GELU, in either place, over all arguments with a finite result."""
+    from tspipe_b200.ops import fused
+    x = torch.arange(-32768, 32768, device=DEV).to(torch.int16).view(torch.bfloat16)
+    x = x[x.isfinite()]
+    x = x[: x.numel() // 8 * 8].roll(shift)
+    y, swapped = fused.gelu(x.view(-1, 8)).view(-1).double(), fused.gelu(x.flip(0).contiguous().view(-1, 8)).view(-1).flip(0).double()
+    assert torch.equal(y, swapped)
+    v = x.double()
+    ref = v * torch.special.ndtr(v)
+    # the rounding to bf16; the tail's rational form, 0.75e-7 absolute (Abramowitz & Stegun 7.1.26 has 1.5e-7 for erf), which is
+    # an exact zero behind |x| = 16; its fp32 arithmetic and approximate exponential, whose argument is rounded at up to 2^7; a
+    # subnormal flushed
+    tail = torch.special.ndtr(-v.abs())
+    err = (y - ref).abs() - ref.abs() * 2.0 ** -8 - v.abs().clamp_max(16) * (0.75e-7 + tail * 2.0 ** -16) - 2.0 ** -126
+    assert err.max() <= 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,d", [(1, 8), (17, 256), (16, 264), (4800, 520), (33, 776), (5000, 1024)])
 def test_layer_norm_widths(rows, d, dtype):
