@@ -35,8 +35,7 @@ constexpr int UMMA_K = 16;
 constexpr uint64_t kWaitNs = 2000000000ull;   // every mbarrier wait gives up after two seconds
 constexpr int kGroup = 2;                       // stages released per tcgen05.commit
 constexpr int kABytes = BM * BK * 2;
-constexpr int kStoreBufBytes = 32 * 128;                        // 32 rows x 128 bytes of C, one TMA store
-constexpr int kStoreBytes = 8 * kStoreBufBytes;                 // two buffers per epilogue warp, or one for each of eight
+constexpr int kStoreBytes = 8 * 32 * 128;                       // two 32 x 128 byte blocks per epilogue warp, or 16 of 32 x 64
 // BN = tile columns (256, 128 or 64); each CTA stages BN / 2 rows of B
 template <int BN> struct Cfg {
   static constexpr int kStages = BN == 256 ? 6 : 8;
@@ -145,9 +144,14 @@ enum Kind {
   kRed = 2      // C += A[k, m]^T B[k, n]     gradient of the weight: fp32, split along k, added in L2 by the TMA unit; A may
                 //                            be up to three matrices side by side along m
 };
-// Epilogue warps: two per TMEM lane quarter where the epilogue computes (256 GELUs per row and tile would take one longer
-// than the tile's products), with one staging buffer each instead of two.
-__host__ __device__ constexpr int epi_warps(int kind) { return kind == kGelu ? 8 : 4; }
+// Epilogue warps: four per TMEM lane quarter where the epilogue computes.  The GELUs of a tile are about as many issue slots as
+// the products of a K = 768 tile are clocks, so that the warps of a scheduler have to cover each other's waits for TMEM, the
+// reciprocal and the exponential; with two per quarter they did not.  Each stages 32 x 32 blocks in a buffer of its own, which
+// keeps the staging at 32 KB.  B200, 12608 x 3072 x 768, both outputs: 74.8 us with two -> 70.7, 16384 rows and one output
+// 83.0 -> 78.8.
+__host__ __device__ constexpr int epi_warps(int kind) { return kind == kGelu ? 16 : 4; }
+// bytes of a row of C that a warp stages and stores at a time
+__host__ __device__ constexpr int block_bytes(int kind) { return kind == kGelu ? 64 : 128; }
 constexpr int kMaxASrc = 3;
 struct AMaps {
   CUtensorMap m[kMaxASrc];
@@ -323,12 +327,12 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
     }
   } else {
     // ---------------- epilogue (both CTAs): this CTA's 128 rows, all BN columns ----------------
-    // Per warp: 32 accumulator rows.  Blocks of 128 output bytes per row (64 bf16 or 32 fp32 columns) go
+    // Per warp: 32 accumulator rows.  Blocks of 128 output bytes per row (64 bf16 or 32 fp32 columns; kGelu 64 bytes) go
     // TMEM -> registers -> (bias, GELU, convert) -> swizzled shared memory -> one TMA store; two staging
-    // buffers per warp, so the store of block i overlaps the conversion of block i + 1.  Without a usable
+    // buffers per warp, so the store of block i overlaps the conversion of block i + 1 (kGelu one).  Without a usable
     // tensor map for C (unaligned base or row pitch) every thread stores its own row directly.
-    constexpr int kCols = 128 / (int)sizeof(OutT);
-    constexpr int kBufs = 8 / epi_warps(KIND);         // staging buffers per warp
+    constexpr int kRowBytes = block_bytes(KIND), kStoreBufBytes = 32 * kRowBytes, kCols = kRowBytes / (int)sizeof(OutT);
+    constexpr int kBufs = kStoreBytes / kStoreBufBytes / epi_warps(KIND);         // staging buffers per warp
     const int quarter = warp & 3, group = (warp - 2) >> 2;
     uint8_t* my_bufs = store_bufs + (warp - 2) * kBufs * kStoreBufBytes;
     uint32_t lt = 0, nstore = 0;
@@ -377,11 +381,12 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
           }
           __syncwarp();
         }
-        uint8_t* my_row = buf + lane * 128;
+        uint8_t* my_row = buf + lane * kRowBytes;
+        const int swizzle = kRowBytes == 128 ? lane & 7 : (lane >> 1) & 3;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {   // 16-byte piece j of this row sits at piece (j ^ (row & 7))
+        for (int j = 0; j < kRowBytes / 16; ++j) {   // 16-byte piece j of this row sits at piece (j ^ swizzle)
           uint4 q;
-          if constexpr (kCols == 64) {
+          if constexpr (sizeof(OutT) == 2) {
             q.x = pack_bf16x2(v[8 * j + 0], v[8 * j + 1]);
             q.y = pack_bf16x2(v[8 * j + 2], v[8 * j + 3]);
             q.z = pack_bf16x2(v[8 * j + 4], v[8 * j + 5]);
@@ -392,7 +397,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ AMaps tmap_a, int a_per, const 
             q.z = __float_as_uint(v[4 * j + 2]);
             q.w = __float_as_uint(v[4 * j + 3]);
           }
-          *reinterpret_cast<uint4*>(my_row + ((j ^ (lane & 7)) << 4)) = q;
+          *reinterpret_cast<uint4*>(my_row + ((j ^ swizzle) << 4)) = q;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -511,12 +516,13 @@ bool make_map(CUtensorMap* map, const void* ptr, int rows, int cols, int ld, int
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
-bool make_store_map(CUtensorMap* map, void* ptr, int rows, int cols, int ld, bool bf16) {
+bool make_store_map(CUtensorMap* map, void* ptr, int rows, int cols, int ld, bool bf16, int row_bytes) {
   const int esz = bf16 ? 2 : 4;
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * esz};
-  const cuuint32_t box[2] = {(cuuint32_t)(128 / esz), 32};
+  const cuuint32_t box[2] = {(cuuint32_t)(row_bytes / esz), 32};
   return tc5::encode_tiled(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, ptr, 2, dims,
-                           strides, box, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+                           strides, box, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                           row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 // About the clocks that a pair needs for 64 rows of a weight gradient's contraction, and what an item costs besides: its
@@ -595,7 +601,7 @@ int launch_bn(const Args& p, int dev, int max_pairs, cudaStream_t stream) {
     if (c == nullptr) c = p.c[1];                       // (kGelu without C0)
     tc.m[i] = tb;               // placeholder when C cannot be described (the kernel then stores directly)
     if ((((uintptr_t)c & 15) != 0) || ((p.ldc * (int)sizeof(OutT)) % 16 != 0) ||
-        !make_store_map(&tc.m[i], c, p.m, n_per, p.ldc, sizeof(OutT) == 2))
+        !make_store_map(&tc.m[i], c, p.m, n_per, p.ldc, sizeof(OutT) == 2, block_bytes(KIND)))
       tma_store = 0;
   }
   // statistics come from the staged blocks, sums and several destinations need the TMA unit
@@ -680,7 +686,7 @@ int tsp_gemm_bf16_tn_2cta(const void* a, const void* b, void* c, const float* bi
 
 // h[m,n] (bf16, optional) = A[m,k] * B[n,k]^T, act[m,n] (bf16) = gelu(h + bias[n]) of the rounded h: a linear layer and its
 // activation in one pass.  n a multiple of 64, bias 16-byte aligned.  B200: 12608 x 3072 x 768 with
-// both outputs 75 us against 54 + 34 for product and activation, 16384 rows without h 83 against 65 + 43.
+// both outputs 71 us against 54 + 34 for product and activation, 16384 rows without h 79 against 65 + 43.
 int tsp_gemm_bf16_tn_gelu_2cta(const void* a, const void* b, void* h, void* act, const float* bias, int m, int n, int k,
                                int lda, int ldb, int ldc, int* status, cudaStream_t stream) {
   if (m <= 0 || n <= 0 || k <= 0) return 0;

@@ -310,14 +310,15 @@ inline EncodeTiledFn get_encode() {
 
 // Tensor map with a 128-byte swizzle and zeros out of range.
 inline bool encode_tiled(CUtensorMap* map, CUtensorMapDataType type, const void* base, int rank, const cuuint64_t* dims,
-                         const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapL2promotion promotion) {
+                         const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapL2promotion promotion,
+                         CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn enc = get_encode();
   if (enc == nullptr) return false;
   const cuuint32_t e[4] = {1, 1, 1, 1};
   CUresult r = CUDA_ERROR_UNKNOWN;
   for (int attempt = 0; attempt < 2; ++attempt) {
     r = enc(map, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     // The encoder is a driver call and wants a current context.  A thread that has not made a runtime call yet (an
     // autograd worker calling straight into this library) has none: bind the device's primary context and retry.
     if (r == CUDA_SUCCESS) break;

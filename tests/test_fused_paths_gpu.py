@@ -623,6 +623,20 @@ def test_linear_gelu_epilogue_equals_the_separate_kernel(m, n, k, grad):
         gemm.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 64, 8), (33, 128, 72), (257, 320, 64), (300, 448, 200), (9733, 512, 64)])
+def test_linear_gelu_at_the_edges_of_tiles_and_blocks(m, n, k):
+    """The epilogue's 32 x 32 blocks past the last row, in a cut tile and in pieces of tiles (the last case): bit for bit."""
+    from tspipe_b200.ops import fused, gemm
+    torch.manual_seed(41)
+    x, w = torch.randn(m, k, device=DEV).bfloat16(), torch.randn(n, k, device=DEV) / math.sqrt(k)
+    b = torch.randn(n, device=DEV)
+    h = gemm.linear(x, w, None)
+    assert torch.equal(gemm.linear_gelu(x, w, b), fused.gelu(h, b))
+    y = gemm.linear_gelu(x.clone().requires_grad_(), w, b)          # which keeps h as well
+    gemm.check_status()
+    assert torch.equal(y.detach(), fused.gelu(h, b))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,d", [(1, 8), (17, 264), (16, 256), (128, 3072), (5000, 1000), (20000, 8200)])
 def test_gelu_backward_with_the_bias_gradient(rows, d, dtype):
