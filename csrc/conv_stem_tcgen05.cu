@@ -314,7 +314,7 @@ conv_stem_kernel(const __nv_bfloat16* __restrict__ wmat, const __grid_constant__
       }
     }
   } else {
-    // ---------------- epilogue: warps 9 .. 16, TMEM lanes 32*(warp%4) .. +31; group g takes the g-th pair of a tile's rows ----------------
+    // ---------------- epilogue: warps from 9 on, TMEM lanes 32*(warp%4) .. +31; group g takes the g-th kRowsEach of a tile's rows ----------------
     // First the weights as the products take them, while the loaders fill the ring: step 2 kh + half, element 4 * tap + channel, taps
     // 0..3 and 3..6 (128-byte swizzle), from a copy in the staging buffers.  (By all warps before their roles began, from
     // memory element by element, they made every call 2 us longer: 8 images of 96 x 96 10.8 us, 9.1 this way.)
