@@ -100,6 +100,18 @@ __device__ __forceinline__ void ldraw(const float* p, int64_t i, Raw8<float>& r)
 __device__ __forceinline__ void ldraw(const __nv_bfloat16* p, int64_t i, Raw8<__nv_bfloat16>& r) {
   r.a = *reinterpret_cast<const uint4*>(p + i);
 }
+// the same where ONCE, with evict-first hints: what is not read again soon
+template <bool ONCE>
+__device__ __forceinline__ void ldraw(const float* p, int64_t i, Raw8<float>& r) {
+  if constexpr (!ONCE) return ldraw(p, i, r);
+  r.a = __ldcs(reinterpret_cast<const float4*>(p + i));
+  r.b = __ldcs(reinterpret_cast<const float4*>(p + i + 4));
+}
+template <bool ONCE>
+__device__ __forceinline__ void ldraw(const __nv_bfloat16* p, int64_t i, Raw8<__nv_bfloat16>& r) {
+  if constexpr (!ONCE) return ldraw(p, i, r);
+  r.a = __ldcs(reinterpret_cast<const uint4*>(p + i));
+}
 __device__ __forceinline__ void cvt8(const Raw8<float>& r, float (&v)[8]) {
   v[0] = r.a.x; v[1] = r.a.y; v[2] = r.a.z; v[3] = r.a.w; v[4] = r.b.x; v[5] = r.b.y; v[6] = r.b.z; v[7] = r.b.w;
 }

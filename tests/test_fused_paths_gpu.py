@@ -428,6 +428,31 @@ def test_gelu_special_values_and_wide_bias(dtype):
             assert _rel(a, w) < 2 * EPS[dtype] + 1e-6
 
 
+@pytest.mark.parametrize("res", [False, True])
+def test_batchnorm_apply_on_both_sides_of_the_cache_size(res):
+    """The rows that a tensor of 126 MB and one above it have in common, which are read with and without hints."""
+    from tspipe_b200.ops import bn
+    torch.manual_seed(42)
+    c, m = 64, (126 << 20) // 128
+    x = torch.randn(m + 8, c, device=DEV).bfloat16()
+    r = torch.randn_like(x) if res else None
+    w, b, mean, var = (torch.rand(c, device=DEV) + 0.5 for _ in range(4))
+
+    def apply(n):
+        y, f = torch.empty_like(x[:n]), bn._f
+        k = f._c
+        fixed = torch.cat([mean, var])
+        assert f.lib().tsp_bn_apply(f._ptr(x), f._ptr(r), f._ptr(y), None, f._ptr(fixed), f._ptr(w), f._ptr(b), None, None, None, None,
+                                    k.c_int64(0), k.c_int64(n), k.c_int(c), k.c_float(1e-5), k.c_int(1), k.c_int(f._dt(x)), k.c_int(1),
+                                    f._stream()) == 0
+        return y
+    small, large = apply(m), apply(m + 8)
+    assert torch.equal(small, large[:m])
+    want = (x[-4096:].double() - mean) * (var.double() + 1e-5).rsqrt() * w + b + (r[-4096:].double() if res else 0)
+    # a rounding to bf16 behind a handful in fp32 of terms below 32
+    assert ((large[-4096:].double() - want.relu()).abs() <= want.abs() * 2.0 ** -8 + 32 * 2.0 ** -21).all()
+
+
 @pytest.mark.parametrize("shift", [0, 1])
 def test_gelu_of_every_bf16_argument(shift):
     """Two values share an instruction: each is its own GELU, in either place, over all arguments with a finite result."""
