@@ -272,7 +272,9 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const T* __restrict__ dy,
 
 // The same with the column sums of dx (the gradient of the bias), of the values as they are stored: 32 lanes = 256 columns of a
 // row, eight warps = eight rows, blocks stacked over the rows, so that a thread keeps its columns' sums in registers and a
-// block adds one number per column.  [12608, 3072] bf16: 41 us and a pass of 16 for the sums, 48 this way.
+// block adds one number per column.  [12608, 3072] bf16: 41 us and a pass of 16 for the sums, 48 this way.  x and dy are read with
+// evict-first hints, so that dx is in the L2 cache for the two products that follow; with a reader of dx behind it 75.8 us without
+// hints and 67.6 with, [12608, 4096] 108.6 and 94.2, [4000, 3072] 40.1 and 38.7, [50432, 3072] 250 both.
 constexpr int kGeluSumRows = 8, kGeluSumVecs = 2;
 
 template <typename T>
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_sums_kernel(const T* __restrict_
     tsp::Raw8<T> xr[U], gr[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (r + u * step < rows) { tsp::ldraw(x, (r + u * step) * d + col, xr[u]); tsp::ldraw(dy, (r + u * step) * d + col, gr[u]); }
+      if (r + u * step < rows) { tsp::ldraw<true>(x, (r + u * step) * d + col, xr[u]); tsp::ldraw<true>(dy, (r + u * step) * d + col, gr[u]); }
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (r + u * step < rows) {
