@@ -1496,8 +1496,8 @@ int tsp_bounded_wait_probe(int limit_ms, int code, int* status, cudaStream_t str
 // y[n, ho, wo, cout] = conv(x[n, h, w, cin], wgt[cout][k][k][cin]), stride s, padding (k - 1) / 2; all bf16,
 // channels-last, 16-byte aligned, cin and cout multiples of 64.  col_sums (optional, zeroed by the caller):
 // [segs][2 * cout] fp32 receives per-channel sum and sum of squares of y over each of `segs` equal groups of
-// consecutive images (n divisible by segs; for a 1x1 stride-1 convolution the pixels per group must be a multiple of
-// 128).  `status`: one zeroed int in device memory; non-zero afterwards = a bounded wait ran out, y is not valid.
+// consecutive images (n divisible by segs; for a 1x1 stride-1 convolution of several groups the pixels per group must be a
+// multiple of 128).  `status`: one zeroed int in device memory; non-zero afterwards = a bounded wait ran out, y is not valid.
 int tsp_conv_fprop(const void* x, const void* wgt, void* y, float* col_sums, int segs, int n, int h, int w, int cin,
                    int cout, int k, int s, int* status, cudaStream_t stream) {
   if (!shape_ok(n, h, w, cin, cout, k, s)) return -3;
@@ -1535,7 +1535,7 @@ int tsp_conv_fprop(const void* x, const void* wgt, void* y, float* col_sums, int
   if (col_sums != nullptr) {
     if (segs < 1 || n % segs) return -3;
     const int64_t rows = (int64_t)n * ho * wo / segs;
-    if (flat && rows % 128) return -3;
+    if (flat && segs > 1 && rows % 128) return -3;
     if (!flat && g.box_n > 1 && (n / segs) % g.box_n) return -3;
     g.rows_per_seg = (int)rows;
   }

@@ -188,6 +188,28 @@ def test_igemm_convolution_forward_backward_and_statistics(shape, cout, k, strid
     torch.testing.assert_close(m.weight.grad, 2 * wr.grad, rtol=5e-2, atol=1e-1 * wr.grad.abs().max().item())
 
 
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 1, 1, 64, 64), (1, 7, 7, 64, 128), (3, 10, 10, 128, 64), (37, 14, 14, 256, 1024),
+                                            (64, 7, 7, 512, 2048), (64, 7, 7, 2048, 512)])
+def test_statistics_of_one_group_with_a_ragged_last_tile(n, h, w, cin, cout):
+    """1x1: the rows that the last tile of 128 pixels lacks count as zeros, also where a weight is infinite."""
+    from tspipe_b200.ops import conv, gemm
+    torch.manual_seed(43)
+    dev = torch.device("cuda", 0)
+    x = torch.rand(n, cin, h, w, device=dev).add(0.5).to(dtype=torch.bfloat16, memory_format=torch.channels_last)
+    weight = (torch.randn(cout, cin, 1, 1, device=dev) / cin ** 0.5).to(memory_format=torch.channels_last)
+    weight[3, 5] = float("inf")
+    conv.clear_weight_cache()
+    y, sums = conv.conv2d(x, weight, 1, want_sums=True)
+    gemm.check_status()
+    terms = y.double()
+    assert terms[:, 3].eq(float("inf")).all()
+    for got, part in zip(sums.view(2, cout).double(), (terms, terms * terms)):
+        want, size = part.sum((0, 2, 3)), part.abs().sum((0, 2, 3))
+        assert got[3] == float("inf")
+        keep = torch.arange(cout, device=dev) != 3
+        assert ((got - want).abs() <= 2.0 ** -16 * size)[keep].all()     # fp32 sums of some hundred terms each, added up
+
+
 # (images, height, width, cin, cout, kernel): the pixel tiles around the numbers where the channel tile changes its width (74
 # tiles of 256 channels run at once in halves on 148 SMs, 37 in quarters), and grids of several tiles per block
 TILE_CASES = [(37, 16, 16, 256, 256, 1), (75, 16, 8, 256, 256, 1), (37, 16, 8, 256, 256, 1), (19, 16, 16, 256, 256, 3),

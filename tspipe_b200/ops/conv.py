@@ -204,8 +204,11 @@ def _geom(x: torch.Tensor, weight: torch.Tensor, stride: int):
 def _stats_ok(n: int, ho: int, wo: int, k: int, stride: int, segs: int) -> bool:
     if n % segs:
         return False
+    # Flat tiles of 128 pixels, which must not straddle two views; the rows that the last one lacks count as zeros.  Convolution,
+    # statistics and normalisation on a B200, with a pass of its own for the statistics and with the epilogue's: 64 images of 7 x 7,
+    # 512 -> 2048 42.4 and 36.2 us, 37 of 14 x 14, 256 -> 1024 40.2 and 34.0, one of 7 x 7, 64 -> 64 25.4 and 24.5.
     if k == 1 and stride == 1:
-        return (n // segs * ho * wo) % 128 == 0
+        return segs == 1 or (n // segs * ho * wo) % 128 == 0
     if ho * wo <= 64:                          # several images per pixel box: a box must not straddle two views
         per_box = 128 // (ho * wo)
         tiles = -(-n // per_box)
