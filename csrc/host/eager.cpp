@@ -70,9 +70,18 @@ Tensor gradient_like(Tensor g, const Tensor& like) {
 
 bool owns_saved() { return !at::SavedTensorDefaultHooks::get_hooks().has_value(); }
 
-// The fp32 gradient of a leaf that a kernel can add to in place: the weight's elements in the order [rows][taps][columns].
-Tensor grad_target(const Tensor& weight) {
-  if (!g_accumulate.load(std::memory_order_relaxed) || !weight.is_leaf()) return {};
+// Whether autograd's accumulation of p's gradient runs on `st`.  Autograd orders the accumulation, and the caller of backward()
+// behind it, by the stream on which the accumulating node was made, and for the gradients that this node is handed; an
+// addition that a backward launches itself is in that order on that very stream and on no other.
+bool accumulates_on(const Tensor& p, cudaStream_t st) {
+  const auto node = torch::autograd::impl::try_get_grad_accumulator(p);
+  const auto own = node ? node->stream() : std::nullopt;
+  return own.has_value() && own->device() == p.device() && c10::cuda::CUDAStream(*own).stream() == st;
+}
+
+// The fp32 gradient of a leaf that a kernel on `st` can add to in place: the weight's elements in the order [rows][taps][columns].
+Tensor grad_target(const Tensor& weight, cudaStream_t st) {
+  if (!g_accumulate.load(std::memory_order_relaxed) || !weight.is_leaf() || !accumulates_on(weight, st)) return {};
   const Tensor& g = weight.grad();
   if (!g.defined() || g.scalar_type() != at::kFloat || g.sizes() != weight.sizes() || g.layout() != at::kStrided || !g.is_cuda())
     return {};
@@ -80,10 +89,11 @@ Tensor grad_target(const Tensor& weight) {
   return g.is_contiguous() && aligned(g) ? g : Tensor();
 }
 
-// The fp32 gradient of a vector parameter that a backward may add to itself, in place of the node that accumulates it: in a
+// The fp32 gradient of a vector parameter that a backward may add to itself on `st`, in place of the node that accumulates it: in a
 // backward() over the whole graph (one that was asked for gradients by name lists what to execute), without a recorded graph of
-// its own, for a leaf with a gradient whose hooks want to see nothing.
-Tensor accumulated(const Tensor& p) {
+// its own, for a leaf with a gradient whose hooks want to see nothing, on the stream of the accumulation.  (The kernels read, add and
+// write: two of them on two streams would lose one's sums.)
+Tensor accumulated(const Tensor& p, cudaStream_t st) {
   namespace ag = torch::autograd;
   const auto* listed = ag::get_current_graph_task_exec_info();
   if (listed == nullptr || !listed->empty() || at::GradMode::is_enabled() || !p.is_leaf() || !p.requires_grad()) return {};
@@ -95,7 +105,7 @@ Tensor accumulated(const Tensor& p) {
   if (const auto node = ag::impl::try_get_grad_accumulator(p);
       node && !(node->pre_hooks().empty() && node->post_hooks().empty() && node->tensor_pre_hooks().empty()))
     return {};
-  return g;
+  return accumulates_on(p, st) ? g : Tensor();
 }
 
 struct ConvGeom {
@@ -131,7 +141,7 @@ struct BnGrads {
 BnGrads bn_backward(const Tensor& dy, const Tensor& x, const Tensor& y, const float* mean_rstd, const Tensor& w, const Tensor& b,
                     bool relu, bool has_res, bool params, int64_t m, int c, int segs, cudaStream_t st) {
   BnGrads g;
-  Tensor add_w = params ? accumulated(w) : Tensor(), add_b = params ? accumulated(b) : Tensor();
+  Tensor add_w = params ? accumulated(w, st) : Tensor(), add_b = params ? accumulated(b, st) : Tensor();
   const bool add = add_w.defined() && add_b.defined();
   g.dx = at::empty_like(x);
   const bool masked = has_res && relu;
@@ -235,7 +245,7 @@ struct ConvBnAct : Function<ConvBnAct> {
       r[0] = dskip.defined() && !fits ? dx + dskip : dx;
     }
     if (ctx->needs_input_grad(1)) {
-      Tensor target = grad_target(weight);
+      Tensor target = grad_target(weight, st);
       if (!target.defined()) {
         target = zeroed_f32((int64_t)g.cout * g.k * g.k * g.cin, x, st);
         r[1] = target.view({g.cout, g.k, g.k, g.cin}).permute({0, 3, 1, 2});
@@ -340,7 +350,7 @@ struct LinearBias : Function<LinearBias> {
       r[0] = want == at::kBFloat16 ? dx : dx.to(want);
     }
     if (ctx->needs_input_grad(1)) {
-      Tensor target = grad_target(weight);
+      Tensor target = grad_target(weight, st);
       if (!target.defined()) {
         target = zeroed_f32(n * k, x2, st).view({n, k});
         r[1] = target;
@@ -355,7 +365,7 @@ struct LinearBias : Function<LinearBias> {
       if (n % 8 != 0 || n > 8192 || m < 2) {
         r[3] = dy.sum(0, false, at::kFloat);
       } else {
-        const Tensor add = accumulated(ctx->saved_data["bias"].toTensor()), out = add.defined() ? add : at::empty({n}, f32_like(x2));
+        const Tensor add = accumulated(ctx->saved_data["bias"].toTensor(), st), out = add.defined() ? add : at::empty({n}, f32_like(x2));
         check(tsp_col_sums(ptr(dy), m, (int)n, TSP_DTYPE_BF16, out.data_ptr<float>(), add.defined() ? 1 : 0, st), "tsp_col_sums");
         g_launches += 1;
         if (!add.defined()) r[3] = out;

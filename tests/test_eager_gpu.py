@@ -259,3 +259,63 @@ def test_pair_losses(monkeypatch, kind, dtype):
     ts = make()
     with pytest.raises(Exception):              # (teachers have no gradient)
         torch.autograd.grad(fused.byol_loss(*ts) if kind == "byol" else gemm.info_nce_pair(ts[0], ts[3], ts[1], ts[2], 0.2), [ts[2]])
+
+
+def _additions(call):
+    """In-place additions that autograd has made during ``call`` (a gradient that a kernel adds itself is none)."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        call()
+    return sum(e.count for e in prof.key_averages() if e.key == "aten::add_")
+
+
+def _three_layers():
+    """A linear layer, a BatchNorm and a convolution with one, with gradient buffers: forward of all, parameters, gradients."""
+    from tspipe_b200.ops import bn as fbn
+    from tspipe_b200.ops import conv as fconv
+    from tspipe_b200.ops import gemm
+    lin, conv = nn.Linear(64, 128).to(DEV), nn.Conv2d(64, 64, 1, bias=False).to(DEV, memory_format=torch.channels_last)
+    bns = nn.ModuleList([DeferredBatchNorm(128), DeferredBatchNorm(64)]).to(DEV)
+    group = BatchNormGroup(bns, chunks=100)
+    xs = torch.randn(256, 64, device=DEV).bfloat16(), torch.randn(256, 128, device=DEV).bfloat16(), _cl(4, 64, 8, 8)
+    gs = torch.randn(256, 128, device=DEV).bfloat16(), torch.randn(256, 128, device=DEV).bfloat16(), _cl(4, 64, 8, 8)
+    ps = [*lin.parameters(), *conv.parameters(), *bns.parameters()]
+    for p in ps:
+        p.grad = torch.ones_like(p)
+
+    def forward():
+        with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False):
+            return [gemm.linear(xs[0], lin.weight, lin.bias), fbn.bn_act(bns[0], xs[1], None, True),
+                    fconv.conv_bn_act(conv, bns[1], xs[2], relu=True)]
+    return forward, ps, gs, group
+
+
+@pytest.mark.parametrize("where", ["here", "side", "held", "both"])
+def test_gradients_of_layers_on_other_streams(monkeypatch, where):
+    """A kernel adds to a gradient itself only on the stream of the accumulation: not where the accumulating nodes were made on
+    another one than the layer's (``held``), and of two uses on two streams in one graph (``both``) on one of them.  The caller's stream
+    reads the gradients behind backward() without a wait of its own, while the side stream is busy."""
+    def call(forward, ps, gs, group):
+        here, native = torch.cuda.current_stream(), fused.eager() is not None
+        side = torch.cuda.Stream() if native else here          # (the reference on one stream)
+        held = [p.expand_as(p).grad_fn.next_functions[0][0] for p in ps] if where == "held" else None
+        ys = forward() if where in ("here", "both") else []
+        side.wait_stream(here)
+        if where != "here":
+            with torch.cuda.stream(side):
+                ys += forward()
+                here.wait_stream(side)
+                torch.cuda._sleep(10_000_000)
+        outs = []
+
+        def backward():
+            torch.autograd.backward(ys, gs * (len(ys) // 3))
+            outs.extend(p.grad.clone() for p in ps)
+        added = _additions(backward)
+        torch.cuda.synchronize()
+        if native:
+            assert added == {"here": 0, "side": 0, "held": len(ps), "both": len(ps)}[where]
+        del held
+        return outs
+    a, b = _both(monkeypatch, _three_layers, call)
+    for p, q in zip(a, b):
+        _same(p, q)
