@@ -96,6 +96,7 @@ Tensor grad_target(const Tensor& weight, cudaStream_t st) {
 Tensor accumulated(const Tensor& p, cudaStream_t st) {
   namespace ag = torch::autograd;
   const auto* listed = ag::get_current_graph_task_exec_info();
+  if (!g_accumulate.load(std::memory_order_relaxed)) return {};
   if (listed == nullptr || !listed->empty() || at::GradMode::is_enabled() || !p.is_leaf() || !p.requires_grad()) return {};
   const Tensor& g = p.grad();
   if (!g.defined() || !plain(g) || g.scalar_type() != at::kFloat || g.sizes() != p.sizes() || !g.is_contiguous() ||

@@ -319,3 +319,21 @@ def test_gradients_of_layers_on_other_streams(monkeypatch, where):
     a, b = _both(monkeypatch, _three_layers, call)
     for p, q in zip(a, b):
         _same(p, q)
+
+
+def test_every_gradient_goes_to_autograd_where_in_place_addition_is_off(monkeypatch):
+    from tspipe_b200.ops import conv as fconv
+
+    def call(forward, ps, gs, group):
+        native = fused.eager() is not None
+        fconv.set_accumulate_in_place(False)
+        try:
+            ys = forward()
+            added = _additions(lambda: torch.autograd.backward(ys, gs))
+        finally:
+            fconv.set_accumulate_in_place(True)
+        assert added == len(ps) or not native
+        return [p.grad for p in ps]
+    a, b = _both(monkeypatch, _three_layers, call)
+    for p, q in zip(a, b):
+        _same(p, q)

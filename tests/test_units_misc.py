@@ -235,3 +235,30 @@ def test_lars_order_updates_after_the_norms_of_the_whole_tensor(lag):
         assert pos > max(p for p, s, _ in at[0].values() if s == seg)
         mine = norms.index(at[0][begin][0])
         assert pos > norms[min(mine + lag, len(norms) - 1)]
+
+
+def test_in_place_setting_loads_nothing_and_reaches_the_extension(monkeypatch):
+    """The setting is kept for an extension that is loaded later, and passed on to one that is there."""
+    from tspipe_b200.ops import build, conv, fused
+
+    class Host:
+        seen = []
+
+        def set_accumulate(self, on):
+            self.seen.append(on)
+
+    def unavailable():
+        raise RuntimeError("no compiler")
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(build, "load", unavailable)
+    monkeypatch.setattr(build, "load_host", unavailable)
+    monkeypatch.setattr(fused, "_host", None)
+    try:
+        conv.set_accumulate_in_place(False)
+        monkeypatch.setattr(build, "load_host", Host)
+        monkeypatch.setattr(fused, "lib", lambda: None)
+        assert isinstance(fused.eager(), Host) and Host.seen == [False]
+        conv.set_accumulate_in_place(True)
+        assert Host.seen == [False, True]
+    finally:
+        conv.set_accumulate_in_place(True)

@@ -303,13 +303,12 @@ _ACCUMULATE_IN_PLACE = True
 
 
 def set_accumulate_in_place(flag: bool) -> None:
-    """Let the weight-gradient kernel add straight into an existing fp32 ``weight.grad`` of matching layout (default)
-    instead of handing autograd a fresh tensor to accumulate."""
+    """Let the kernels of weight gradients, and in eager calls those of bias and BatchNorm gradients, add straight into an
+    existing fp32 ``grad`` of matching layout (default) instead of handing autograd a fresh tensor to accumulate."""
     global _ACCUMULATE_IN_PLACE
     _ACCUMULATE_IN_PLACE = bool(flag)
-    if torch.cuda.is_available():
-        _f.lib()
-        _f._build.load_host().set_accumulate(_ACCUMULATE_IN_PLACE)
+    if _f._host is not None:                   # (one that is loaded later takes the setting then)
+        _f._host.set_accumulate(_ACCUMULATE_IN_PLACE)
 
 
 def conv2d(x: torch.Tensor, weight: torch.Tensor, stride: int = 1, want_sums: bool = False, segments: int = 1

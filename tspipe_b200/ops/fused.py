@@ -79,8 +79,10 @@ def eager():
     if IN_CAPTURE or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling():
         return None
     if _host is None:
+        from . import conv
         lib()
         _host = _build.load_host()
+        _host.set_accumulate(conv._ACCUMULATE_IN_PLACE)
     return _host
 
 
