@@ -91,15 +91,15 @@ Tensor grad_target(const Tensor& weight, cudaStream_t st) {
 
 // The fp32 gradient of a vector parameter that a backward may add to itself on `st`, in place of the node that accumulates it: in a
 // backward() over the whole graph (one that was asked for gradients by name lists what to execute), without a recorded graph of
-// its own, for a leaf with a gradient whose hooks want to see nothing, on the stream of the accumulation.  (The kernels read, add and
-// write: two of them on two streams would lose one's sums.)
+// its own, for a leaf with a gradient whose hooks want to see nothing and no search for NaN, on the stream of the accumulation.  (The
+// kernels read, add and write: two of them on two streams would lose one's sums.)  The caller bumps its version, as the node would have.
 Tensor accumulated(const Tensor& p, cudaStream_t st) {
   namespace ag = torch::autograd;
   const auto* listed = ag::get_current_graph_task_exec_info();
-  if (!g_accumulate.load(std::memory_order_relaxed)) return {};
+  if (!g_accumulate.load(std::memory_order_relaxed) || ag::AnomalyMode::is_enabled()) return {};
   if (listed == nullptr || !listed->empty() || at::GradMode::is_enabled() || !p.is_leaf() || !p.requires_grad()) return {};
   const Tensor& g = p.grad();
-  if (!g.defined() || !plain(g) || g.scalar_type() != at::kFloat || g.sizes() != p.sizes() || !g.is_contiguous() ||
+  if (!g.defined() || !plain(g) || g.layout() != at::kStrided || g.scalar_type() != at::kFloat || g.sizes() != p.sizes() || !g.is_contiguous() ||
       g.get_device() != p.get_device())
     return {};
   if (!ag::impl::hooks(p).empty() || ag::impl::post_acc_grad_hooks(p) != nullptr) return {};
@@ -144,6 +144,10 @@ BnGrads bn_backward(const Tensor& dy, const Tensor& x, const Tensor& y, const fl
   BnGrads g;
   Tensor add_w = params ? accumulated(w, st) : Tensor(), add_b = params ? accumulated(b, st) : Tensor();
   const bool add = add_w.defined() && add_b.defined();
+  if (add) {
+    torch::autograd::impl::bump_version(add_w);
+    torch::autograd::impl::bump_version(add_b);
+  }
   g.dx = at::empty_like(x);
   const bool masked = has_res && relu;
   if (masked) g.dres = at::empty_like(x);
@@ -366,7 +370,9 @@ struct LinearBias : Function<LinearBias> {
       if (n % 8 != 0 || n > 8192 || m < 2) {
         r[3] = dy.sum(0, false, at::kFloat);
       } else {
-        const Tensor add = accumulated(ctx->saved_data["bias"].toTensor(), st), out = add.defined() ? add : at::empty({n}, f32_like(x2));
+        const Tensor add = accumulated(ctx->saved_data["bias"].toTensor(), st);
+        if (add.defined()) torch::autograd::impl::bump_version(add);
+        const Tensor out = add.defined() ? add : at::empty({n}, f32_like(x2));
         check(tsp_col_sums(ptr(dy), m, (int)n, TSP_DTYPE_BF16, out.data_ptr<float>(), add.defined() ? 1 : 0, st), "tsp_col_sums");
         g_launches += 1;
         if (!add.defined()) r[3] = out;

@@ -337,3 +337,20 @@ def test_every_gradient_goes_to_autograd_where_in_place_addition_is_off(monkeypa
     a, b = _both(monkeypatch, _three_layers, call)
     for p, q in zip(a, b):
         _same(p, q)
+
+
+@pytest.mark.parametrize("anomaly", [False, True])
+def test_vector_gradients_in_place_count_as_written(anomaly):
+    """A gradient that a graph has saved is refused behind a backward() that added to it, and a search for NaN sees all of them."""
+    forward, ps, gs, group = _three_layers()
+    vectors = [p for p in ps if p.dim() == 1]
+    kept = [p.grad * torch.ones_like(p, requires_grad=True) for p in vectors]
+    ys = forward()
+    if anomaly:
+        with pytest.raises(RuntimeError, match="returned nan values"), torch.autograd.detect_anomaly():
+            ys[0].backward(torch.full_like(gs[0], float("nan")))
+    else:
+        torch.autograd.backward(ys, gs)
+        for k in kept:
+            with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+                k.sum().backward()
