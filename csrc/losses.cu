@@ -544,11 +544,11 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
           if (has_ce) {                                 // (the row once more, from L2)
             const uint4 q = __ldg(sr + i);
             const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-            const Pair ms2(ms, ms), e2(kLog2e, kLog2e), l2(l1, l1), wc(w_ce, w_ce);
+            const Pair ms2(ms, ms), e2(kLog2e, kLog2e), minus_l2(-l1, -l1), wc(w_ce, w_ce);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const Pair d = unpack2(w[j]) - ms2;
-              Pair p = ex2(d * e2 - l2);
+              Pair p = ex2(fma2(d, e2, minus_l2));
               if (i * 4 + j == (id.y >> 1)) {
                 float d0, d1;
                 d.split(d0, d1);
@@ -581,8 +581,10 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
             }
           }
         }
-        part = tsp::warp_sum(part);
-        if (lane == 0) atomicAdd(&block_part, (double)wt * (double)part);
+        double wide = part;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) wide += __shfl_xor_sync(0xffffffffu, wide, o);
+        if (lane == 0) atomicAdd(&block_part, (double)wt * wide);
       }
     }
   }
