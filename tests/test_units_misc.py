@@ -262,3 +262,30 @@ def test_in_place_setting_loads_nothing_and_reaches_the_extension(monkeypatch):
         assert Host.seen == [False, True]
     finally:
         conv.set_accumulate_in_place(True)
+
+
+@pytest.mark.parametrize("left", ["nothing", "a stale module", "a compiler that fails"])
+def test_eager_calls_go_on_without_the_extension(monkeypatch, tmp_path, left):
+    """Without a module that fits, or a compiler, the Python functions take the calls, which is said once."""
+    import subprocess
+    import warnings
+
+    from tspipe_b200.ops import build, fused
+    path = tmp_path / "tspipe_eager.so"
+    if left == "a stale module":
+        path.write_bytes(b"of another torch")
+        (tmp_path / "tspipe_eager.so.srchash").write_text("0")
+    monkeypatch.setattr(build, "HOST_PATH", str(path))
+    monkeypatch.setattr(build, "load", lambda: None)
+    monkeypatch.setattr(build, "build", lambda: None)
+    monkeypatch.setattr(build, "_host", None)
+    monkeypatch.setattr(build, "_no_host", False, raising=False)
+    monkeypatch.setattr(build.shutil, "which", lambda name: None if left != "a compiler that fails" else name)
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **k: subprocess.CompletedProcess(cmd, 1, "", "no header"))
+    monkeypatch.setattr(fused, "_host", None)
+    monkeypatch.setattr(fused, "lib", lambda: None)
+    with pytest.warns(RuntimeWarning, match="Python functions"):
+        assert fused.eager() is None
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert fused.eager() is None

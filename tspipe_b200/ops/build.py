@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import threading
+import warnings
 from typing import List, Optional
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -32,6 +33,7 @@ HOST_PATH = os.path.join(LIB_DIR, HOST_NAME + ".so")
 _lock = threading.Lock()
 _lib: Optional[ctypes.CDLL] = None
 _host = None
+_no_host = False        # building or loading it has failed
 
 
 def sources() -> List[str]:
@@ -158,15 +160,18 @@ def build_host() -> str:
 
 
 def load_host():
-    """The extension module of the eager calls, built first when it is missing or stale (as :func:`load`)."""
-    global _host
-    if _host is None:
-        load()
+    """The extension module of the eager calls, built first when it is missing or stale; None where that cannot be done, with a
+    warning the first time: their Python functions launch the same kernels, at a higher cost to the host.  A stale module is
+    not loaded, since it is bound to the C++ interface of the torch that it was built against."""
+    global _host, _no_host
+    if _host is not None or _no_host:
+        return _host
+    load()
+    try:
         if not host_is_fresh():
-            if shutil.which("g++") is not None:
-                build_host()
-            elif not os.path.exists(HOST_PATH):
-                raise RuntimeError(f"{HOST_PATH} is missing and g++ is unavailable; run __graft_entry__.build()")
+            if shutil.which("g++") is None:
+                raise RuntimeError(f"{HOST_PATH} is missing or stale and g++ is unavailable")
+            build_host()
         import importlib.util
         with _lock:
             if _host is None:
@@ -174,4 +179,7 @@ def load_host():
                 module = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(module)
                 _host = module
+    except (RuntimeError, ImportError, OSError) as e:
+        _no_host = True
+        warnings.warn(f"eager calls stay with their Python functions: {e}", RuntimeWarning, stacklevel=2)
     return _host

@@ -74,7 +74,8 @@ sys.modules[__name__].__class__ = _Counting
 
 def eager():
     """The C++ autograd functions (``csrc/host/eager.cpp``) for a call that is made eagerly; None while a stage is being
-    recorded, whose backward adds small gradients in place, and under a trace, which sees the calls of the Python functions."""
+    recorded, whose backward adds small gradients in place, under a trace, which sees the calls of the Python functions, and where
+    they cannot be built."""
     global _host
     if IN_CAPTURE or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling():
         return None
@@ -82,7 +83,8 @@ def eager():
         from . import conv
         lib()
         _host = _build.load_host()
-        _host.set_accumulate(conv._ACCUMULATE_IN_PLACE)
+        if _host is not None:
+            _host.set_accumulate(conv._ACCUMULATE_IN_PLACE)
     return _host
 
 
