@@ -1233,9 +1233,10 @@ static int pool_geom(int n, int h, int w, int c, int segs, PoolGeom* g) {
   const int ho = (h + 1) / 2, wo = (w + 1) / 2;
   if ((int64_t)n * (h + 1) * (w + 1) >= 0x7fffffff || (int64_t)w * c >= 0x7fffffff) return -3;
   // strips of four rows where they give an SM four blocks, of fewer rows on smaller tensors
-  int rows = 4;
+  int rows = 4, sms = 0;
+  if (cudaError_t e = tsp::usable_sms(sms); e != cudaSuccess) return (int)e;
   const int64_t blocks = (int64_t)segs * n * ho * wo * (c / 8) / kBlock;
-  while (rows > 1 && blocks / rows < 148 * 4) rows /= 2;
+  while (rows > 1 && blocks / rows < sms * 4) rows /= 2;
   const int strips = (ho + rows - 1) / rows;
   *g = {n, h, w, c, ho, wo, rows, FastDiv(wo), FastDiv(strips), (uint32_t)((int64_t)n * strips * wo)};
   return 0;

@@ -274,7 +274,7 @@ constexpr int kRowQueue = 4;                                    // rows that the
 static_assert(kRing < kRowQueue * 2 && kRowSmem <= 227 * 1024, "a row in the ring is two pieces at least");
 constexpr uint64_t kRowWaitNs = 2000000000ull;                  // a wait gives up after two seconds
 constexpr int kStreamMin = (kRowVecs - 1) * kPieceElems + 1;    // elements of a row: only the last vector is partly filled
-constexpr int kStreamRows = 4 * 148;                            // rows: four per SM
+constexpr int kStreamRows = 4;                                  // rows per SM that the kernel may use
 
 using tsp::Pair;
 using tsp::fma2;
@@ -754,15 +754,17 @@ static int launch_kd_ce(const void* s, const void* t, const int64_t* labels, con
                         cudaStream_t stream) {
   const bool vec = rows_of_8(c, s, t, gs);
   if (vec && t != nullptr && w_kd != 0.f && s_dtype == TSP_DTYPE_BF16 && t_dtype == TSP_DTYPE_BF16 &&
-      n >= kStreamRows && c >= kStreamMin && c <= kRowVecs * kPieceElems) {
+      c >= kStreamMin && c <= kRowVecs * kPieceElems) {
     int sms = 0;
-    cudaError_t e = tsp::usable_sms(sms);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kd_ce_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmem);
-    if (e != cudaSuccess) return (int)e;
-    kd_ce_stream_kernel<<<n < sms ? n : sms, kRowThreads + 32, kRowSmem, stream>>>(
-        (const __nv_bfloat16*)s, (const __nv_bfloat16*)t, labels, row_mask, n, c, temp, w_ce, w_kd, sum, loss,
-        (__nv_bfloat16*)gs);
-    return TSP_LAUNCH_CHECK();
+    if (cudaError_t e = tsp::usable_sms(sms); e != cudaSuccess) return (int)e;
+    if (n >= kStreamRows * sms) {
+      cudaError_t e = cudaFuncSetAttribute(kd_ce_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmem);
+      if (e != cudaSuccess) return (int)e;
+      kd_ce_stream_kernel<<<sms, kRowThreads + 32, kRowSmem, stream>>>(
+          (const __nv_bfloat16*)s, (const __nv_bfloat16*)t, labels, row_mask, n, c, temp, w_ce, w_kd, sum, loss,
+          (__nv_bfloat16*)gs);
+      return TSP_LAUNCH_CHECK();
+    }
   }
   // at least four accesses per thread and sweep on long rows, one warp of latency on short ones
   const int parts = vec ? c / 8 : c;

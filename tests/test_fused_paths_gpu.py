@@ -154,6 +154,24 @@ def test_kd_ce_long_rows_leave_reserved_sms(reserve):
     assert abs(float(loss)) < 1e-4
 
 
+@pytest.mark.parametrize("reserve", [0, 8])
+def test_kd_ce_long_rows_from_four_per_usable_sm(reserve):
+    from tspipe_b200.ops import fused as f
+    usable, c = torch.cuda.get_device_properties(DEV).multi_processor_count - reserve, 24584
+    s = torch.randn(4 * usable, c, device=DEV).bfloat16()
+    total, loss = torch.empty(3, dtype=torch.float64, device=DEV), torch.empty((), device=DEV)
+    for n in (4 * usable - 1, 4 * usable):
+        f.set_sm_reserve(reserve)
+        try:
+            assert f.lib().tsp_kd_ce_loss(s.data_ptr(), s.data_ptr(), None, None, n, c, 1, 1, 2.0, 0.0, 1.0, total.data_ptr(),
+                                          loss.data_ptr(), None, f._raw_stream()) == 0
+        finally:
+            f.set_sm_reserve(0)
+        tickets, blocks = total[1:2].view(torch.int32).tolist()          # (none drawn by the kernel for fewer rows)
+        assert (tickets, blocks) == ((n + usable, usable) if n == 4 * usable else (0, 0))
+        assert abs(float(loss)) < 1e-4
+
+
 @pytest.mark.parametrize("off", [-math.inf, torch.finfo(torch.bfloat16).min])
 def test_kd_ce_long_rows_with_classes_switched_off_for_the_student_alone(off):
     """Many rows give what few rows do, whose kernel forms the divergence from the probabilities: where the student's lowest
