@@ -49,10 +49,11 @@ bool plain(const Tensor& t) {
   return t.defined() && t.is_cuda() && !t.key_set().has_any(wrapped);
 }
 
-// [N, C, H, W] with channels innermost
+// [N, C, H, W] with channels innermost, which a single pixel's are in either format
 bool nhwc(const Tensor& t) {
   if (t.dim() != 4) return false;
   const int64_t c = t.size(1), h = t.size(2), w = t.size(3);
+  if (h * w == 1 && t.is_contiguous()) return true;
   return t.stride(1) == 1 && t.stride(3) == c && t.stride(2) == w * c && t.stride(0) == h * w * c;
 }
 // (rows, channels) of a matrix with channels innermost, or (0, 0)

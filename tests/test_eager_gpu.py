@@ -354,3 +354,22 @@ def test_vector_gradients_in_place_count_as_written(anomaly):
         for k in kept:
             with pytest.raises(RuntimeError, match="modified by an inplace operation"):
                 k.sum().backward()
+
+
+@pytest.mark.parametrize("fmt", [torch.channels_last, torch.contiguous_format])
+def test_fork_of_single_pixels_takes_the_other_gradient_along(monkeypatch, fmt):
+    """Images of one pixel are channels-last in either format: the data gradient adds the other branch's, in one rounding."""
+    from tspipe_b200.ops import conv as fconv
+
+    def call(conv, bn, group, x, r, gy, gx, views, fork):
+        native = fused.eager() is not None
+        gx = gx.clone(memory_format=fmt)
+        with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False):
+            y, skip = fconv.conv_bn_act_fork(conv, bn, x, relu=True)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+            dx, dw = torch.autograd.grad([y, skip], [x, conv.weight], [gy, gx])
+        assert not native or not any(e.key == "aten::add" for e in prof.key_averages())
+        return [dx, dw]
+    a, b = _both(monkeypatch, lambda: _conv_block(1, 1, 64, 64, 64, 1, 1, False, True), call)
+    for p, q in zip(a, b):
+        _same(p, q)
