@@ -535,27 +535,59 @@ def test_add_layer_norm_equals_the_separate_passes(rows, d, with_a, dtype):
                                          ((8, 64, 137, 139), 1), ((16, 64, 137, 139), 2)])
 def test_batchnorm_relu_maxpool_equals_the_separate_passes(shape, views, dtype):
     """Odd extents (last window of two rows or columns), strips of one, two and four rows that end early, channel counts off
-    the block size, more channels than a block takes."""
+    the block size, more channels than a block takes.  Both sides are handed the same statistics, with sums of zero, whose variance
+    is one product however it is contracted: their activations are the same bits, and ties are the same ties."""
     from tspipe_b200.batchnorm import BatchNormGroup, DeferredBatchNorm
     from tspipe_b200.ops import bn as fbn
     from tspipe_b200.ops.pool import MaxPool3x3s2
     torch.manual_seed(8)
+    n, c, h, w = shape
     x = _cl(*shape, dtype=dtype).requires_grad_()
+    variance = torch.linspace(0.5, 4, c, device=DEV)
+    stats = torch.stack([torch.zeros_like(variance), variance * (n // views * h * w)]).repeat(views, 1, 1).reshape(-1)
     outs = []
     for fused in (True, False):
-        mod = DeferredBatchNorm(shape[1]).to(DEV)
+        mod = DeferredBatchNorm(c).to(DEV)
         with torch.no_grad():
-            mod.weight.copy_(torch.linspace(-1, 2, shape[1]))
-            mod.bias.copy_(torch.linspace(0.5, -0.5, shape[1]))
+            mod.weight.copy_(torch.linspace(-1, 2, c))
+            mod.bias.copy_(torch.linspace(0.5, -0.5, c))
         group = BatchNormGroup(mod, chunks=10)
         with fbn.segments(views):
-            y = fbn.bn_relu_pool(mod, x) if fused else MaxPool3x3s2()(fbn.bn_act(mod, x, None, True))
-        assert y is not None
+            if fused:
+                y = fbn.bn_relu_pool(mod, x, stats.clone())
+                _, idx, won = y.grad_fn.saved_tensors[:3]
+            else:
+                act = fbn.bn_act(mod, x, None, True, stats.clone())
+                y = MaxPool3x3s2()(act)
         torch.manual_seed(9)
         g = _cl(*y.shape, dtype=dtype)
-        outs.append([y.detach(), *torch.autograd.grad(y, [x, mod.weight, mod.bias], g), group._acc])
-    for a, b in zip(outs[0], outs[1]):                 # same roundings, sums in another order
-        assert _rel(a, b) < EPS[dtype] + 1e-5
+        outs.append([y.detach(), *torch.autograd.grad(y, [x, mod.weight, mod.bias] + ([] if fused else [act]), g), group._acc])
+    (y, dx, dw, db, acc), (y2, dx2, dw2, db2, dact, acc2) = outs
+    assert torch.equal(y, y2) and torch.equal(acc, acc2)
+    # the winners: x and the activation at the tap that the code names (a code is larger for an earlier tap)
+    code = idx.view(n, y.shape[2], y.shape[3], c).permute(0, 3, 1, 2).long()
+    live = code != 255
+    assert torch.equal(live, y > 0)
+    code = code.where(live, torch.full_like(code, 5))                   # (any tap that exists)
+    iy = 2 * torch.arange(y.shape[2], device=DEV).view(-1, 1) - 1 + 2 - code // 4
+    ix = 2 * torch.arange(y.shape[3], device=DEV) - 1 + 2 - code % 4
+    assert bool(((iy >= 0) & (iy < h) & (ix >= 0) & (ix < w))[live].all())
+    at = iy * w + ix
+
+    def taken(t):
+        return t.detach().reshape(n, c, h * w).gather(2, at.reshape(n, c, -1)).view_as(y)
+    assert torch.equal(taken(x)[live], won[live]) and torch.equal(taken(act)[live], y[live])
+    # dx = A (dact - mean(dact) - xhat mean(dact xhat)) with A = weight / std: dact and dx are rounded to the type, on one side perhaps to
+    # the neighbour of the other's (two units of 2^-8 or 2^-23); the means are of the rounded dact on one side and of what its windows
+    # give on the other; terms add up in another order
+    per = lambda t: t.double().reshape(views, n // views, c, h, w)                                      # noqa: E731
+    a = (torch.linspace(-1, 2, c, device=DEV).abs() * variance.rsqrt()).view(-1, 1, 1)
+    xhat, d = per(x.detach()).abs() * variance.rsqrt().view(-1, 1, 1), per(dact).abs()
+    means = d.mean((1, 3, 4), True) + xhat * (d * xhat).mean((1, 3, 4), True)
+    off = (per(dx) - per(dx2)).abs() - EPS[dtype] * (2 * per(dx2).abs() + a * (2 * d + means))
+    assert float(off.max()) <= 1e-5
+    for p, q in ((dw, dw2), (db, db2)):
+        assert _rel(p, q) < EPS[dtype] + 1e-5
 
 
 @pytest.mark.parametrize("widths", [(8,), (64, 8, 256, 2048)])
