@@ -490,6 +490,29 @@ def test_gelu_of_every_bf16_argument(shift):
     assert err.max() <= 0
 
 
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gelu_gradient_of_every_bf16_argument(shift):
+    """As above for the derivative, times one: within a bf16 rounding and the tail's error, also where a gradient of two follows."""
+    from tspipe_b200.ops import fused
+    x = torch.arange(-32768, 32768, device=DEV).to(torch.int16).view(torch.bfloat16)
+    x = x[x.isfinite()]
+    x = x[: x.numel() // 8 * 8].roll(shift)
+
+    def grad(v, g):
+        v = v.reshape(-1, 8).clone().requires_grad_()
+        return torch.autograd.grad(fused.gelu(v), v, torch.full_like(v, g))[0].view(-1)
+    g = grad(x, 1.0)
+    assert torch.equal(g, grad(x.flip(0), 1.0).flip(0)) and torch.equal(grad(x, 2.0), 2 * g)
+    v = x.double()
+    density = torch.exp(-0.5 * v * v) * 0.3989422804014327
+    ref = torch.special.ndtr(v) + v * density
+    # the rounding to bf16; the tail's rational form, 0.75e-7 absolute; its fp32 arithmetic and the approximate exponential, whose argument
+    # is rounded at up to 2^7 (2^-17 times ln 2 of it, and as much for its product with the constants); a subnormal flushed
+    tail = torch.special.ndtr(-v.abs())
+    err = (g.double() - ref).abs() - ref.abs() * 2.0 ** -8 - 0.75e-7 - (tail + v.abs() * density) * 2.0 ** -16 - 2.0 ** -126
+    assert err.max() <= 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,d", [(1, 8), (17, 256), (16, 264), (4800, 520), (33, 776), (5000, 1024)])
 def test_layer_norm_widths(rows, d, dtype):
