@@ -145,7 +145,7 @@ __device__ __forceinline__ void tile_origin(const Geom& g, int tm, int& w0, int&
 // (STATS) and coalesced 16-byte stores, 8 lanes per pixel.
 // ADD: `addend` has the output's layout and is added to the rounded result, as the sum of two bf16 gradients would be.
 template <int BN, int SUBS, int ACC_BUFS, int GROUPS, bool STATS, bool ADD>
-__device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int tiles_m, int n_sub, uint32_t tmem_base,
+__device__ __forceinline__ void fwd_epilogue(const Geom& g, int num_tiles, int n_sub, uint32_t tmem_base,
                                              uint64_t* tmem_full_bar, uint64_t* tmem_empty_bar, uint8_t* store_bufs,
                                              __nv_bfloat16* __restrict__ out,
                                              const __nv_bfloat16* __restrict__ addend, float* __restrict__ col_sums,
@@ -348,7 +348,7 @@ __device__ __forceinline__ void flush_cta_stats(const Geom& g, const uint8_t* st
 // 96 KB per SM are in flight whatever the tile is waiting for.  Read by the threads instead, one tile ahead in registers, the
 // gradient of [256, 56, 56, 256] took 223 us, 157 this way (141 at the rate of a copy).
 template <int BN>
-__device__ __forceinline__ void add_epilogue(const Geom& g, int num_tiles, int tiles_m, uint32_t tmem_base,
+__device__ __forceinline__ void add_epilogue(const Geom& g, int num_tiles, uint32_t tmem_base,
                                              uint64_t* tmem_full_bar, uint64_t* tmem_empty_bar, uint8_t* store_bufs,
                                              uint64_t* add_bars, const CUtensorMap* __restrict__ omap,
                                              const CUtensorMap* __restrict__ amap, int* __restrict__ status, int warp, int lane) {
@@ -527,8 +527,9 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
       const uint32_t tiles_addr = smem_u32(tiles);
       uint32_t it = 0, lt = 0;
       // The next operands and the next accumulator, looked at ahead (mbar_over), where the contraction is long: 64 images, B200,
-      // 512 -> 512 3x3 at 7 x 7 26.2 us without, 23.7 with, 512 -> 128 at 28 x 28 18.4 and 18.0, 3x3 of stride 2 30.8 and 29.0; 256 -> 512
-      // of stride 2 26.4 and 26.9.
+      // 512 -> 512 3x3 at 7 x 7 26.2 us without, 23.7 with, 512 -> 128 1x1 at 28 x 28 (8 blocks) 18.4 and 18.0, 256 -> 256 3x3 of
+      // stride 2 at 28 x 28 29.5 and 25.1, 256 -> 512 3x3 of stride 2 at 56 x 56 119.4 and 120.5; with 4 blocks 256 -> 512 1x1 of stride
+      // 2 at 56 x 56 27.0 and 27.8.
       const bool ahead = num_kb >= 8;
       bool ok = true, there = false, room = false;
       for (int t = tile_begin(num_tiles, blockIdx.x); t < tile_begin(num_tiles, blockIdx.x + 1) && ok; ++t, ++lt) {
@@ -565,10 +566,10 @@ conv_fwd_kernel(const __grid_constant__ ActMaps amaps, const __grid_constant__ C
     }
   } else {
     if constexpr (ADD == 2)
-      add_epilogue<BN>(g, num_tiles, tiles_m, tmem_base, tmem_full_bar, tmem_empty_bar, store_bufs, add_bars, &omap, &addmap,
+      add_epilogue<BN>(g, num_tiles, tmem_base, tmem_full_bar, tmem_empty_bar, store_bufs, add_bars, &omap, &addmap,
                        status, warp, lane);
     else
-      fwd_epilogue<BN, 1, C::kAccBufs, GROUPS, STATS, ADD == 1>(g, num_tiles, tiles_m, 1, tmem_base, tmem_full_bar,
+      fwd_epilogue<BN, 1, C::kAccBufs, GROUPS, STATS, ADD == 1>(g, num_tiles, 1, tmem_base, tmem_full_bar,
                                                                        tmem_empty_bar, store_bufs, out, addend, col_sums, status, warp,
                                                                        lane, &omap);
   }
@@ -784,7 +785,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
       }
     }
   } else {
-    fwd_epilogue<BN, 2, C::kAccBufs, 2, STATS, ADD>(g, num_tiles, tiles_m, n_sub, tmem_base, tmem_full_bar, tmem_empty_bar,
+    fwd_epilogue<BN, 2, C::kAccBufs, 2, STATS, ADD>(g, num_tiles, n_sub, tmem_base, tmem_full_bar, tmem_empty_bar,
                                                  store_bufs, out, addend, col_sums, status, warp, lane);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -148,7 +148,8 @@ enum Kind {
 // the products of a K = 768 tile are clocks, so that the warps of a scheduler have to cover each other's waits for TMEM, the
 // reciprocal and the exponential; with two per quarter they did not.  Each stages 32 x 32 blocks in a buffer of its own, which
 // keeps the staging at 32 KB.  B200, 12608 x 3072 x 768, both outputs: 74.8 us with two -> 70.7, 16384 rows and one output
-// 83.0 -> 78.8.
+// 83.0 -> 78.8.  With few tiles the larger start costs nothing that shows: 128 rows 15.4 and 15.4, 788 21.5 and 20.5, 1576 25.5 and 23.6; 4096
+// x 1024 of 128 rows 16.5 both, of 788 23.5 and 22.6; 1536 x 384 13.3 and 13.3, 15.3 and 15.3.
 __host__ __device__ constexpr int epi_warps(int kind) { return kind == kGelu ? 16 : 4; }
 // bytes of a row of C that a warp stages and stores at a time
 __host__ __device__ constexpr int block_bytes(int kind) { return kind == kGelu ? 64 : 128; }

@@ -330,7 +330,7 @@ kd_ce_stream_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __
   __shared__ float part[2][6][32];
   __shared__ int failed[2];                           // by row, as `part`: a wait of a computing warp ran out
   __shared__ double block_part;                       // the block's share of the loss
-  __shared__ float2 refs[kRowWarps][kRowVecs];        // the maxima that a warp's exponentials refer to, of s and t
+  __shared__ float2 refs[kRowWarps][kRowVecs];        // what a warp's exponentials refer to (see above), of s and t
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nv = c / 8;
   unsigned* counters = reinterpret_cast<unsigned*>(sum + 1);      // [0] ticket, [1] blocks that are done

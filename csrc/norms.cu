@@ -88,7 +88,8 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const T* __restrict__ x, co
 // memory.  A lane keeps its columns' dw / db sums in registers over all rows of its warp and holds the row as loaded (16
 // bits where the activation has 16 bits), so that 16 warps fit an SM; an earlier one-kernel form with the row in fp32 took
 // 176 registers and ran at 1.45 TB/s, and separate dx and dw / db kernels read everything twice.  [12608, 768] bf16,
-// B200: 40 us as separate kernels, 20 this way, with a residual gradient 30 where that was loaded behind the sums and 23 now.  (Requesting the next row ahead of the current one: 36, fewer warps fit.)
+// B200, with its reduction (3): 40 us as separate kernels, 23 this way, with a residual's gradient 26, and 33 where that was loaded
+// behind the sums.  (Requesting the next row ahead of the current one: 36, fewer warps fit.)
 // partial layout: [gridDim.x][2][d] fp32 (scratch memory owned by the caller), summed by ln_bwd_reduce_kernel.
 constexpr int kLnBwdWarps = 8;
 // ADD: `skip` (the gradient that reaches the row on a residual connection) is added to the rounded dx.
