@@ -558,7 +558,7 @@ int pick_splits(int m, int n, int k, int bn, int pairs) {
 // Pieces of a tile's columns in the last round of tiles, where it leaves at least half of the pairs idle: as many as `most` and
 // as run at once.  A step of a narrow piece takes less time, and the sums are formed in the same order.  12608 x 768 (150 tiles on 74
 // pairs), B200: K = 3072 56.5 us with whole tiles in the third round, 47.8 in quarters; in halves (MN-major B) 53.8.  Within a
-// ViT-B block, whose products run at the power limit, 880 us and 877.
+// ViT-B block 880 us and 877.
 int last_round_pieces(int tiles, int pairs, int most) {
   const int left = tiles % pairs;
   int pieces = 1;

@@ -119,9 +119,9 @@ class DeferredBatchNorm(_BatchNorm):
 
 class BatchNormGroup:
     """All :class:`DeferredBatchNorm` layers of one partition with their statistics re-homed into flat
-    buffers, so that the per-mini-batch commit is a handful of launches for the whole partition instead
-    of eight per layer (53 layers in a ResNet-50), and so that nothing on the per-microbatch path depends
-    on host-side counters: the kernels accumulate ``sum``, ``sum_squares`` and the per-channel element
+    buffers, so that the per-mini-batch commit is one launch for the whole partition instead of eight per layer
+    (53 layers in a ResNet-50; a handful of library calls with cumulative averages or on a CPU), and so that nothing
+    on the per-microbatch path depends on host-side counters: the kernels accumulate ``sum``, ``sum_squares`` and the per-channel element
     ``count`` on the device.  The owner calls :meth:`step` once per partition forward."""
 
     def __init__(self, module: nn.Module, chunks: Optional[int] = None):
